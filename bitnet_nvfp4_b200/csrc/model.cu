@@ -855,7 +855,8 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
         const size_t Er = static_cast<size_t>(W) * V;
         A_(tok_ident, V); A_(emb_a, Er * H / 2); A_(emb_sf, sf_bytes(static_cast<int>(Er), H)); A_(emb_t, Er * r); A_(y_emb, Er * H);
     }
-    A_(qkv, Mr * m->FC); A_(y, Mr * H); A_(bb_eff, static_cast<size_t>(L) * W); A_(ce_partial, static_cast<size_t>(W) * 16); A_(losses, W);
+    // the logits (V columns) share the q | k | v | beta buffer: a model narrower than its vocabulary needs the wider of the two
+    A_(qkv, Mr * std::max(m->FC, V)); A_(y, Mr * H); A_(bb_eff, static_cast<size_t>(L) * W); A_(ce_partial, static_cast<size_t>(W) * 16); A_(losses, W);
     A_(t_a, Mr * 4 * r); A_(t_f, Mr * r);
     if (m->dense) {
         const DenseLayout lay = dense_layout(*m);
