@@ -1,0 +1,494 @@
+// EFLA / DeltaNet recurrence of a whole sequence of at most 128 tokens as dense contractions, for heads of any width.
+//
+// With a zero initial state the recurrence of efla.cu has a closed form that never builds the hd x hd state. Let
+// k_t = n_t k^_t (n_t = |k_t|), w_t = alpha_t n_t (v_t - n_t k^_t . S_{t-1}), so that S_t = S_{t-1} + k^_t w_t^T. Then
+//     (I + diag(a) strict(G)) w = diag(b) v,   G = K^ K^^T,  a_t = alpha_t n_t^2,  b_t = alpha_t n_t
+//     y = P~ v,   P~ = lower(Q^ K^^T) (I + diag(a) strict(G))^-1 diag(b)
+// P~ is a T x T lower-triangular matrix shared by all columns of the head, so one CTA per (sequence, head) computes it once and
+// multiplies it with V: 2 T^2 hd multiply-adds per sequence instead of the 3 T hd^2 of the state form (six times fewer at
+// T = 128, hd = 512), every input read once, no state, no scratch.
+//
+// Precision: every operand is split into two fp16 terms (x = hi + mid, 22 significant bits; rows are normalised and scaled by powers of
+// two first so that neither term under- or overflows) and the products hi hi + hi mid + mid hi accumulate in fp32. Nothing is
+// rounded to fp16 between tokens, so the result lies closer to exact arithmetic than the per-token form's fp16 state.
+//
+// One CTA of 16 warps per (sequence, head):
+//   1. norms of q and k and the per-token scalars (one warp per row),
+//   2. G and X = Q^ K^^T over 64-column blocks of K and Q (fp32 -> two halves -> shared memory, double-buffered, the next block's
+//      loads in flight behind the MMAs). Warp (pair, G or X, column half) owns row blocks p and nb - 1 - p, so the lower
+//      triangles are spread evenly,
+//   3. inverses of the 16 x 16 diagonal blocks of I + diag(a) strict(G) by forward substitution in fp32,
+//   4. P~ by block back substitution from the right, one warp per 16-row block (rows are independent, no barriers),
+//   5. y = P~ V over 64-column tiles of V.
+// What bounds it: the MMAs of steps 2 and 5 (about 40 k tensor cycles per sequence at T = 128, hd = 512; the legacy mma.sync path, since
+// the triangular solve between the contractions needs its operands in registers). 1024 sequences of 128 tokens, one head of 512:
+// 0.58 ms, against 75 ms for the per-token kernel (whose state passes through shared memory twice per token).
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "kernels.h"
+
+namespace bnf4 {
+
+namespace {
+
+constexpr int kSeqMaxT = 128;
+constexpr int kSeqThreads = 512;
+constexpr int kSqStride = 72;                      // halves per row of the K / Q / V blocks: conflict-free ldmatrix rows
+constexpr int kSqTile = kSeqMaxT * kSqStride * 2;  // bytes of one 128 x 64 block of halves
+constexpr int kSqStage = 4 * kSqTile;              // K hi, K mid, Q hi, Q mid
+constexpr int kSqLStride = 136;                    // halves per row of L hi / L mid
+constexpr int kSqXStride = 140;                    // floats per row of X; the row then holds P~ hi (272 bytes) and P~ mid
+constexpr int kSqPMid = 272;                       // byte offset of P~ mid inside a row
+constexpr int kSqTStride = 24;                     // halves per row of a diagonal block's inverse
+constexpr int kSqDiag = 2 * kSqStage;                            // fp32 diagonal blocks of L [8][16][17]
+constexpr int kSqInv = kSqDiag + 8 * 16 * 17 * 4;                // their inverses, hi and mid [2][8][16][kSqTStride]
+constexpr int kSqScal = kSqInv + 2 * 8 * 16 * kSqTStride * 2;    // q scale, k scale, a, b [4][128] floats
+constexpr int kSqRed = kSqScal + 4 * kSeqMaxT * 4;               // reduction scratch [2][16] + broadcast
+constexpr int kSqSmem = kSqRed + 256;
+static_assert(2 * kSeqMaxT * kSqLStride * 2 <= kSqStage && kSeqMaxT * kSqXStride * 4 <= kSqStage && 4 * kSqTile <= kSqStage, "overlaid regions");
+static_assert(kSqDiag % 16 == 0 && kSqInv % 16 == 0 && kSqScal % 16 == 0, "16-byte aligned regions");
+constexpr float kSqUp = 256.0f;                    // power-of-two scale of every normalised operand
+
+__device__ __forceinline__ void sq_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void sq_ldm(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void sq_ldm_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// x0, x1 -> packed (hi, hi) and (mid, mid) halves with x = hi + mid to 22 bits
+__device__ __forceinline__ void sq_split(float x0, float x1, uint32_t& hi, uint32_t& mid) {
+    const __half2 h = __floats2half2_rn(x0, x1);
+    const float2 hf = __half22float2(h);
+    const __half2 m = __floats2half2_rn(x0 - hf.x, x1 - hf.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    mid = *reinterpret_cast<const uint32_t*>(&m);
+}
+// largest power of two that keeps |x| <= m below kSqUp (1 for m == 0)
+__device__ __forceinline__ float sq_pow2_scale(float m) {
+    if (!(m > 0.0f)) return 1.0f;
+    const int e = static_cast<int>((__float_as_uint(m) >> 23) & 0xffu) - 127;  // 2^e <= m < 2^(e+1)
+    return __uint_as_float(static_cast<uint32_t>(min(max(7 - e + 127, 1), 254)) << 23);
+}
+
+__global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaParams p) {
+    extern __shared__ __align__(16) uint8_t sm[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int T = p.T, hd = p.hidden / p.heads;
+    const unsigned unit = blockIdx.x;
+    const unsigned seq = unit / static_cast<unsigned>(p.heads);
+    const int h = static_cast<int>(unit - seq * static_cast<unsigned>(p.heads));
+    const int nb = (T + 15) >> 4;  // 16-token blocks
+    const size_t row0 = static_cast<size_t>(seq) * T;
+    const float* qg = static_cast<const float*>(p.q) + row0 * p.ld_qkv + h * hd;
+    const float* kg = static_cast<const float*>(p.k) + row0 * p.ld_qkv + h * hd;
+    const float* vg = static_cast<const float*>(p.v) + row0 * p.ld_qkv + h * hd;
+    float* og = static_cast<float*>(p.out) + row0 * p.ld_out + h * hd;
+
+    float* qs_sh = reinterpret_cast<float*>(sm + kSqScal);
+    float* ks_sh = qs_sh + kSeqMaxT;
+    float* a_sh = ks_sh + kSeqMaxT;
+    float* b_sh = a_sh + kSeqMaxT;
+    float* red = reinterpret_cast<float*>(sm + kSqRed);
+    const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
+
+    // ---------------- 1. norms and scalars ----------------
+    for (int t = warp; t < kSeqMaxT; t += 16) {
+        float qss = 0.0f, kss = 0.0f;
+        if (t < T) {
+            const float4* q4 = reinterpret_cast<const float4*>(qg + static_cast<size_t>(t) * p.ld_qkv);
+            const float4* k4 = reinterpret_cast<const float4*>(kg + static_cast<size_t>(t) * p.ld_qkv);
+            for (int i = lane; i < (hd >> 2); i += 32) {
+                const float4 a = q4[i], b = k4[i];
+                qss = fmaf(a.x, a.x, qss); qss = fmaf(a.y, a.y, qss); qss = fmaf(a.z, a.z, qss); qss = fmaf(a.w, a.w, qss);
+                kss = fmaf(b.x, b.x, kss); kss = fmaf(b.y, b.y, kss); kss = fmaf(b.z, b.z, kss); kss = fmaf(b.w, b.w, kss);
+            }
+        }
+        qss = warp_sum_f(qss);
+        kss = warp_sum_f(kss);
+        if (lane == 0) { qs_sh[t] = qss; ks_sh[t] = kss; }
+    }
+    __syncthreads();
+    if (tid < kSeqMaxT) {
+        const int t = tid;
+        const float qss = qs_sh[t], kss = ks_sh[t];
+        float a = 0.0f, b = 0.0f, kinv = 0.0f, qinv = 0.0f;
+        if (t < T) {
+            const float bias = p.beta_bias_seq != nullptr ? p.beta_bias_seq[seq / static_cast<unsigned>(p.seqs_per_bias)] : p.beta_bias;
+            const float beta = 1.0f / (1.0f + expf(-(p.beta_raw[(row0 + t) * p.ld_beta] + bias)));
+            const float lambda = kss < p.eps ? p.eps : kss;
+            qinv = rsqrtf(qss + p.eps);
+            kinv = kss > 0.0f ? rsqrtf(kss) : 0.0f;
+            const float n = kss * kinv;
+            if (p.method == 0) {
+                const float ksc = rsqrtf(lambda + p.eps);
+                a = beta * (n * ksc) * (n * ksc);
+                b = beta * (n * ksc);
+            } else {
+                const float alpha = -expm1f(-(beta * lambda)) / (lambda + p.eps);
+                a = alpha * kss;
+                b = alpha * n;
+            }
+        }
+        qs_sh[t] = kSqUp * qinv;
+        ks_sh[t] = kSqUp * kinv;
+        a_sh[t] = a;
+        b_sh[t] = b;
+        float m = b;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (lane == 0) red[warp] = m;
+    }
+    __syncthreads();
+    const float bscale = sq_pow2_scale(fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]))) * (1.0f / kSqUp);  // b * bscale <= 1
+
+    // ---------------- 2. G and X ----------------
+    const int pr = warp & 3, which = (warp >> 2) & 1, half = warp >> 3;
+    const int r1 = pr, r2 = nb - 1 - pr;  // this warp's row blocks (r1 < r2: both; equal: one; r1 > r2: none)
+    float acc1[4][4], acc2[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { acc2[j][i] = 0.0f; if (j < 4) acc1[j][i] = 0.0f; }
+
+    // staging: thread = (16-byte piece of a 64-column row block, row); four rows of K and of Q per thread
+    const int piece = tid & 15, srow = tid >> 4;
+    float4 kr[4], qr[4];
+    auto load_block = [&](int d0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = srow + 32 * i, c = d0 + 4 * piece;
+            kr[i] = qr[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (t < T && c < hd) {
+                kr[i] = *reinterpret_cast<const float4*>(kg + static_cast<size_t>(t) * p.ld_qkv + c);
+                qr[i] = *reinterpret_cast<const float4*>(qg + static_cast<size_t>(t) * p.ld_qkv + c);
+            }
+        }
+    };
+    auto store_block = [&](int buf) {
+        uint8_t* st = sm + buf * kSqStage;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = srow + 32 * i;
+            const float ks = ks_sh[t], qs = qs_sh[t];
+            const int o = (t * kSqStride + 4 * piece) * 2;
+            uint2 hi, mid;
+            sq_split(kr[i].x * ks, kr[i].y * ks, hi.x, mid.x);
+            sq_split(kr[i].z * ks, kr[i].w * ks, hi.y, mid.y);
+            *reinterpret_cast<uint2*>(st + o) = hi;
+            *reinterpret_cast<uint2*>(st + kSqTile + o) = mid;
+            sq_split(qr[i].x * qs, qr[i].y * qs, hi.x, mid.x);
+            sq_split(qr[i].z * qs, qr[i].w * qs, hi.y, mid.y);
+            *reinterpret_cast<uint2*>(st + 2 * kSqTile + o) = hi;
+            *reinterpret_cast<uint2*>(st + 3 * kSqTile + o) = mid;
+        }
+    };
+    // ldmatrix addresses inside a stage: A rows (lane % 16, column half lane / 16); B: eight K rows, matrices (hi, k 0-7), (hi, 8-15), (mid, ..), (mid, ..)
+    const uint32_t a_off = static_cast<uint32_t>((lane & 15) * kSqStride + (lane >> 4) * 8) * 2u + (which ? 2u * kSqTile : 0u);
+    const uint32_t b_off = static_cast<uint32_t>((half * 8 + (lane & 7)) * kSqStride + ((lane >> 3) & 1) * 8) * 2u + (lane >> 4) * static_cast<uint32_t>(kSqTile);
+    const int nd = (hd + 63) >> 6;
+    load_block(0);
+    store_block(0);
+    __syncthreads();
+    for (int db = 0; db < nd; ++db) {
+        if (db + 1 < nd) load_block((db + 1) * 64);
+        const uint32_t st = sm0 + (db & 1) * kSqStage;
+        const int nk = min(4, (hd - db * 64) >> 4);
+        if (r1 <= r2) {
+            for (int kk = 0; kk < nk; ++kk) {
+                uint32_t ah1[4], am1[4], ah2[4], am2[4];
+                const uint32_t ab = st + a_off + kk * 32;
+                sq_ldm(ah2, ab + r2 * (16 * kSqStride * 2));
+                sq_ldm(am2, ab + r2 * (16 * kSqStride * 2) + kSqTile);
+                sq_ldm(ah1, ab + r1 * (16 * kSqStride * 2));
+                sq_ldm(am1, ab + r1 * (16 * kSqStride * 2) + kSqTile);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (j <= r2) {
+                        uint32_t b[4];
+                        sq_ldm(b, st + b_off + kk * 32 + j * (16 * kSqStride * 2));
+                        sq_mma(acc2[j], ah2, b[0], b[1]);
+                        if (j < 4 && j <= r1) sq_mma(acc1[j & 3], ah1, b[0], b[1]);
+                        sq_mma(acc2[j], ah2, b[2], b[3]);
+                        if (j < 4 && j <= r1) sq_mma(acc1[j & 3], ah1, b[2], b[3]);
+                        sq_mma(acc2[j], am2, b[0], b[1]);
+                        if (j < 4 && j <= r1) sq_mma(acc1[j & 3], am1, b[0], b[1]);
+                    }
+                }
+            }
+        }
+        if (db + 1 < nd) store_block((db + 1) & 1);
+        __syncthreads();
+    }
+
+    // ---------------- 3. L (two halves, stage 0), its diagonal blocks (fp32), X (fp32, stage 1) ----------------
+    const int g = lane >> 2, tq = lane & 3;
+    __half* Lh = reinterpret_cast<__half*>(sm);
+    __half* Lm = Lh + kSeqMaxT * kSqLStride;
+    float* X = reinterpret_cast<float*>(sm + kSqStage);
+    float* Ld = reinterpret_cast<float*>(sm + kSqDiag);
+    const float gdown = 1.0f / (kSqUp * kSqUp);
+    auto put_tile = [&](const float (&acc)[4], int r, int j) {
+        const int c0 = j * 16 + half * 8 + 2 * tq;
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+            const int t = r * 16 + g + 8 * hr;
+            float x0 = acc[2 * hr] * gdown, x1 = acc[2 * hr + 1] * gdown;
+            if (which == 0) {
+                const float at = a_sh[t];
+                x0 = c0 < t ? at * x0 : 0.0f;
+                x1 = c0 + 1 < t ? at * x1 : 0.0f;
+                uint32_t hi, mid;
+                sq_split(x0 * kSqUp, x1 * kSqUp, hi, mid);
+                *reinterpret_cast<uint32_t*>(Lh + t * kSqLStride + c0) = hi;
+                *reinterpret_cast<uint32_t*>(Lm + t * kSqLStride + c0) = mid;
+                if (r == j) {
+                    float* d = Ld + (r * 16 + g + 8 * hr) * 17 + half * 8 + 2 * tq;
+                    d[0] = x0;
+                    d[1] = x1;
+                }
+            } else {
+                *reinterpret_cast<float2*>(X + t * kSqXStride + c0) = make_float2(c0 <= t ? x0 : 0.0f, c0 + 1 <= t ? x1 : 0.0f);
+            }
+        }
+    };
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (r1 <= r2 && j <= r2) put_tile(acc2[j], r2, j);
+        if (j < 4 && r1 < r2 && j <= r1) put_tile(acc1[j & 3], r1, j);
+    }
+    __syncthreads();
+    // inverse of I + L_ii: lane c owns column c of a block, two blocks per warp
+    if (warp < 4) {
+        const int blk = 2 * warp + (lane >> 4), c = lane & 15;
+        if (blk < nb) {
+            const float* d = Ld + blk * 16 * 17;
+            float col[16];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                float x = t == c ? 1.0f : 0.0f;
+#pragma unroll
+                for (int s = 0; s < 16; ++s)
+                    if (s < t) x = fmaf(-d[t * 17 + s], col[s], x);
+                col[t] = x;
+            }
+            __half* ih = reinterpret_cast<__half*>(sm + kSqInv) + blk * 16 * kSqTStride + c;
+            __half* im = ih + 8 * 16 * kSqTStride;
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                const float x = col[t] * kSqUp;
+                const __half hi = __float2half_rn(x);
+                ih[t * kSqTStride] = hi;
+                im[t * kSqTStride] = __float2half_rn(x - __half2float(hi));
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---------------- 4. P~ M = X by block columns from the right; warp i owns rows 16 i .. 16 i + 15 ----------------
+    // ldmatrix addresses: A rows of P~ (stage 1), B = rows of L / inverse read transposed (matrices (k 0-7, n 0-7), (8-15, 0-7), (0-7, 8-15), (8-15, 8-15))
+    if (warp < nb) {
+        const int i = warp;
+        float xr[8][2][4];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j <= i) {
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    const float2 lo = *reinterpret_cast<const float2*>(X + (i * 16 + g) * kSqXStride + j * 16 + n * 8 + 2 * tq);
+                    const float2 hi = *reinterpret_cast<const float2*>(X + (i * 16 + g + 8) * kSqXStride + j * 16 + n * 8 + 2 * tq);
+                    xr[j][n][0] = lo.x; xr[j][n][1] = lo.y; xr[j][n][2] = hi.x; xr[j][n][3] = hi.y;
+                }
+            }
+        }
+        __syncwarp();  // the rows are in registers: P~ takes their place
+        uint8_t* prow = sm + kSqStage;
+        const uint32_t p_addr = sm0 + kSqStage + static_cast<uint32_t>((i * 16 + (lane & 15)) * (kSqXStride * 4) + (lane >> 4) * 16);
+        const uint32_t l_addr = sm0 + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqLStride + (lane >> 4) * 8) * 2u;
+        const uint32_t i_addr = sm0 + kSqInv + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqTStride + (lane >> 4) * 8) * 2u;
+        constexpr uint32_t kLMid = kSeqMaxT * kSqLStride * 2, kIMid = 8 * 16 * kSqTStride * 2;
+        const float down = 1.0f / (kSqUp * kSqUp);
+#pragma unroll
+        for (int j = 7; j >= 0; --j) {
+            if (j > i) continue;
+            float s[2][4], c[2][4];  // sum over k > j of P~_ik L_kj: the large products and the cross terms in two chains
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[n][e] = c[n][e] = 0.0f;
+            for (int k = j + 1; k <= i; ++k) {
+                uint32_t ph[4], pm[4], lh[4], lm[4];
+                sq_ldm(ph, p_addr + k * 32);
+                sq_ldm(pm, p_addr + kSqPMid + k * 32);
+                sq_ldm_trans(lh, l_addr + k * (16 * kSqLStride * 2) + j * 32);
+                sq_ldm_trans(lm, l_addr + kLMid + k * (16 * kSqLStride * 2) + j * 32);
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    sq_mma(s[n], ph, lh[2 * n], lh[2 * n + 1]);
+                    sq_mma(c[n], ph, lm[2 * n], lm[2 * n + 1]);
+                    sq_mma(c[n], pm, lh[2 * n], lh[2 * n + 1]);
+                }
+            }
+            // z = X_ij - sum, then P~_ij = z inv_jj
+            uint32_t zh[4], zm[4];
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                float z[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) z[e] = (xr[j][n][e] - (s[n][e] + c[n][e]) * down) * kSqUp;
+                sq_split(z[0], z[1], zh[2 * n], zm[2 * n]);
+                sq_split(z[2], z[3], zh[2 * n + 1], zm[2 * n + 1]);
+            }
+            uint32_t th[4], tm[4];
+            sq_ldm_trans(th, i_addr + j * (16 * kSqTStride * 2));
+            sq_ldm_trans(tm, i_addr + kIMid + j * (16 * kSqTStride * 2));
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                float o[4] = {0.0f, 0.0f, 0.0f, 0.0f}, oc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                sq_mma(o, zh, th[2 * n], th[2 * n + 1]);
+                sq_mma(oc, zh, tm[2 * n], tm[2 * n + 1]);
+                sq_mma(oc, zm, th[2 * n], th[2 * n + 1]);
+                const int c0 = j * 16 + n * 8 + 2 * tq;
+#pragma unroll
+                for (int hr = 0; hr < 2; ++hr) {
+                    uint32_t hi, mid;
+                    sq_split((o[2 * hr] + oc[2 * hr]) * (1.0f / kSqUp), (o[2 * hr + 1] + oc[2 * hr + 1]) * (1.0f / kSqUp), hi, mid);
+                    uint8_t* d = prow + (i * 16 + g + 8 * hr) * (kSqXStride * 4) + c0 * 2;
+                    *reinterpret_cast<uint32_t*>(d) = hi;
+                    *reinterpret_cast<uint32_t*>(d + kSqPMid) = mid;
+                }
+            }
+            __syncwarp();
+        }
+        // the columns' factors b_s, scaled to at most one: applied to the finished rows (exact powers of two aside, one more rounding)
+        for (int idx = lane; idx < 16 * (i + 1) * 8; idx += 32) {
+            const int rr = idx / ((i + 1) * 8), cc = (idx - rr * ((i + 1) * 8)) * 2;
+            uint8_t* d = prow + (i * 16 + rr) * (kSqXStride * 4) + cc * 2;
+            const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(d)), mf = __half22float2(*reinterpret_cast<const __half2*>(d + kSqPMid));
+            uint32_t hi, mid;
+            sq_split((hf.x + mf.x) * (b_sh[cc] * bscale), (hf.y + mf.y) * (b_sh[cc + 1] * bscale), hi, mid);
+            *reinterpret_cast<uint32_t*>(d) = hi;
+            *reinterpret_cast<uint32_t*>(d + kSqPMid) = mid;
+        }
+    }
+    __syncthreads();
+
+    // ---------------- 5. y = P~ V, 64 columns at a time ----------------
+    const int cg = warp >> 2;  // 16-column group of the tile
+    const uint32_t pa = sm0 + kSqStage + static_cast<uint32_t>((lane & 15) * (kSqXStride * 4) + (lane >> 4) * 16);
+    const uint32_t vb = sm0 + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqStride + cg * 16 + (lane >> 4) * 8) * 2u;
+    float4 vr[4];
+    auto load_v = [&](int c0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = srow + 32 * i, c = c0 + 4 * piece;
+            vr[i] = (t < T && c < hd) ? *reinterpret_cast<const float4*>(vg + static_cast<size_t>(t) * p.ld_qkv + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    load_v(0);
+    for (int ct = 0; ct < nd; ++ct) {
+        // the tile's own power-of-two scale keeps both halves of its values in range
+        float m = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m = fmaxf(fmaxf(fmaxf(m, fabsf(vr[i].x)), fmaxf(fabsf(vr[i].y), fabsf(vr[i].z))), fabsf(vr[i].w));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        float* redb = red + 16 * (ct & 1);
+        if (lane == 0) redb[warp] = m;
+        __syncthreads();  // also: everyone is done with the tile before the previous one
+        m = redb[lane & 15];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const float vs = sq_pow2_scale(m);
+        uint8_t* st = sm + (ct & 1) * (2 * kSqTile);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int o = ((srow + 32 * i) * kSqStride + 4 * piece) * 2;
+            uint2 hi, mid;
+            sq_split(vr[i].x * vs, vr[i].y * vs, hi.x, mid.x);
+            sq_split(vr[i].z * vs, vr[i].w * vs, hi.y, mid.y);
+            *reinterpret_cast<uint2*>(st + o) = hi;
+            *reinterpret_cast<uint2*>(st + kSqTile + o) = mid;
+        }
+        if (ct + 1 < nd) load_v((ct + 1) * 64);
+        __syncthreads();
+        if (r1 <= r2) {
+            float y1[2][4], y2[2][4];
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) y1[n][e] = y2[n][e] = 0.0f;
+            const uint32_t vbt = vb + (ct & 1) * (2 * kSqTile);
+            for (int j = 0; j <= r2; ++j) {
+                uint32_t vh[4], vm[4], ah[4], am[4];
+                sq_ldm_trans(vh, vbt + j * (16 * kSqStride * 2));
+                sq_ldm_trans(vm, vbt + kSqTile + j * (16 * kSqStride * 2));
+                sq_ldm(ah, pa + r2 * (16 * kSqXStride * 4) + j * 32);
+                sq_ldm(am, pa + r2 * (16 * kSqXStride * 4) + kSqPMid + j * 32);
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    sq_mma(y2[n], ah, vh[2 * n], vh[2 * n + 1]);
+                    sq_mma(y2[n], ah, vm[2 * n], vm[2 * n + 1]);
+                    sq_mma(y2[n], am, vh[2 * n], vh[2 * n + 1]);
+                }
+                if (r1 < r2 && j <= r1) {
+                    sq_ldm(ah, pa + r1 * (16 * kSqXStride * 4) + j * 32);
+                    sq_ldm(am, pa + r1 * (16 * kSqXStride * 4) + kSqPMid + j * 32);
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) {
+                        sq_mma(y1[n], ah, vh[2 * n], vh[2 * n + 1]);
+                        sq_mma(y1[n], ah, vm[2 * n], vm[2 * n + 1]);
+                        sq_mma(y1[n], am, vh[2 * n], vh[2 * n + 1]);
+                    }
+                }
+            }
+            // undo the scales of P~ (2^8 and b's) and of V
+            const float ds = 1.0f / kSqUp / bscale / vs;
+            auto put = [&](const float (&y)[2][4], int r) {
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    const int c = ct * 64 + cg * 16 + n * 8 + 2 * tq;
+#pragma unroll
+                    for (int hr = 0; hr < 2; ++hr) {
+                        const int t = r * 16 + g + 8 * hr;
+                        if (t < T && c < hd)
+                            *reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c) = make_float2(y[n][2 * hr] * ds, y[n][2 * hr + 1] * ds);
+                    }
+                }
+            };
+            put(y2, r2);
+            if (r1 < r2) put(y1, r1);
+        }
+    }
+}
+
+}  // namespace
+
+bool efla_seq_applies(const EflaParams& p) {
+    const int hd = p.hidden / p.heads;
+    return p.state == nullptr && p.state_fp16 != 0 && !p.qkv_f16 && !p.out_f16 && hd % 32 == 0 && p.T <= kSeqMaxT &&
+           ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0 && p.ld_qkv % 4 == 0 &&
+           (reinterpret_cast<uintptr_t>(p.out) & 7) == 0 && p.ld_out % 2 == 0 && p.seqs * static_cast<long long>(p.heads) <= 0x7fffffffLL;
+}
+
+int efla_seq_launch(const EflaParams& p, cudaStream_t stream) {
+    static bool configured[64] = {};  // function attributes are per device
+    int dev = 0;
+    int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+    if (rc) return rc;
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        rc = check_cuda(cudaFuncSetAttribute(efla_seq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSqSmem), "cudaFuncSetAttribute(efla_seq_kernel)");
+        if (rc) return rc;
+        if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    efla_seq_kernel<<<static_cast<unsigned>(p.seqs * p.heads), kSeqThreads, kSqSmem, stream>>>(p);
+    return check_launch("efla_seq_kernel");
+}
+
+}  // namespace bnf4

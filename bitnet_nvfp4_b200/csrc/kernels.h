@@ -51,6 +51,9 @@ extern int g_gemm_allow_tma_store;
 using EflaParams = bnf4_efla_desc;
 int efla_launch(const EflaParams& p, cudaStream_t stream);
 extern int g_efla_chunked;
+// Whole sequences of at most 128 tokens from a zero state, any head_dim (efla_seq.cu).
+bool efla_seq_applies(const EflaParams& p);
+int efla_seq_launch(const EflaParams& p, cudaStream_t stream);
 
 // Rank-r noise sums Z of a table of matrices in one launch (es_kernels.cu).
 struct ZLowrankDesc {

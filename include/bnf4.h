@@ -263,12 +263,14 @@ typedef struct bnf4_efla_desc {
     void* out; /* fp32 (or halves, see out_f16): row r at out + r*ld_out */
     int ld_out;
     int variant; /* BNF4_EFLA_*: which kernel runs. AUTO: for heads of 64 with no HBM state, the chunked or the per-token
-                    register-state kernel as option "efla_chunked" says; the generic kernel otherwise. */
+                    register-state kernel as option "efla_chunked" says; for other head widths with no HBM state, an fp16 state, at
+                    most 128 tokens and "efla_chunked" on, the closed form of the whole sequence (nothing rounded to fp16 between
+                    tokens); the generic kernel otherwise. */
     int qkv_f16; /* 1: q, k, v are IEEE halves and ld_qkv counts halves (chunked kernel only; 16-byte aligned rows) */
     int out_f16; /* 1: out is IEEE halves and ld_out counts halves (chunked kernel only; 16-byte aligned rows) */
 } bnf4_efla_desc;
 #define BNF4_EFLA_AUTO 0
-#define BNF4_EFLA_GENERIC 1   /* any head_dim, state in shared memory (and in HBM between calls), per-token fp16 rounding */
+#define BNF4_EFLA_GENERIC 1   /* any head_dim up to 2048, state in registers (and in HBM between calls), per-token fp16 rounding */
 #define BNF4_EFLA_PER_TOKEN 2 /* heads of 64: state in registers, rounded to fp16 after every token like the reference */
 #define BNF4_EFLA_CHUNKED 3   /* heads of 64: 16 tokens per step as tensor-core contractions, state rounded to fp16 per chunk */
 
