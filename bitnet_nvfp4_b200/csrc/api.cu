@@ -40,6 +40,21 @@ int check_launch(const char* what) {
     return check_cuda(cudaGetLastError(), what);
 }
 
+int current_device(int* dev) {
+    const int rc = check_cuda(cudaGetDevice(dev), "cudaGetDevice");
+    if (rc) return rc;
+    if (*dev < 0 || *dev >= 64) return set_error(BNF4_ERR_INVALID, "device index %d out of range", *dev);
+    return BNF4_OK;
+}
+
+int multiprocessors(int dev) {
+    static std::atomic<int> count[64] = {};
+    int n = count[dev].load(std::memory_order_relaxed);
+    if (n == 0 && check_cuda(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute") == BNF4_OK)
+        count[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
+
 }  // namespace bnf4
 
 using namespace bnf4;

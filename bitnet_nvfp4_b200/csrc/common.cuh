@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstddef>
 #include <cstdint>
+#include <utility>
 
 // ---------------------------------------------------------------------------------------------
 // Error reporting. Every extern "C" entry point returns 0 on success or one of these codes and
@@ -26,6 +27,59 @@ namespace bnf4 {
 int set_error(int code, const char* fmt, ...);
 int check_cuda(cudaError_t e, const char* what);
 int check_launch(const char* what);
+int current_device(int* dev);       // cudaGetDevice with an error code and a range check (0..63)
+int multiprocessors(int dev);       // SM count of a device, looked up once (0 on failure)
+
+// ---------------------------------------------------------------------------------------------
+// Programmatic dependent launch. A step is a chain of short kernels on one stream; with the attribute below a kernel's blocks
+// may become resident (and run their prologue: barrier and TMEM set-up, table loads) while its predecessor drains, instead of
+// after a full grid-to-grid hand-over of one to two microseconds.
+//   pdl_wait()    first access to global memory that another kernel may write or still read comes after it: it returns when the
+//                 preceding kernel has completed and its writes are visible. Every kernel launched with launch_pdl calls it in
+//                 every thread that touches such memory, so completion is transitive along the stream.
+//   pdl_trigger() lets the successor's blocks be scheduled once every block of this kernel has called it or exited (exit counts
+//                 as a call). It belongs where the block is nearly done: blocks of a small grid that become resident early pile up on
+//                 the SMs the predecessor leaves free (a 119-block scan behind another one took 76 instead of 37 us). Only the row
+//                 quantisers call it at the top: what follows them is a GEMM, whose blocks fill an SM each and cannot pile up.
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Loads through read-only qualified pointers (const __restrict__, __ldg, __ldcs) are not ordered by the memory clobber above: the
+// compiler may take such data for constant. Their addresses are made to depend on something it cannot see before the wait: the
+// pointers themselves (after), or an index (opaque_zero, where the pointers should stay in the parameter bank).
+template <typename... T>
+__device__ __forceinline__ void after(T&... ptr) {  // pointer lvalues, restrict-qualified or not
+    (([&] { asm volatile("" : "+l"(ptr)); }()), ...);
+}
+__device__ __forceinline__ uint32_t opaque_zero() {
+    uint32_t z;
+    asm volatile("mov.u32 %0, 0;" : "=r"(z));
+    return z;
+}
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// `early` false launches in plain stream order. Streaming kernels that run for long after a kernel with much shared memory want
+// that: blocks that become resident early keep the predecessor's split between shared memory and L1 (the row quantisers of a
+// full-size wave lost 5-15 % that way), while the hand-over they would save is a microsecond or two.
+template <typename... KArgs, typename... Args>
+inline void launch_pdl_if(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);  // errors surface in check_launch (cudaGetLastError)
+}
+template <typename... KArgs, typename... Args>
+inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    launch_pdl_if(true, kernel, grid, block, smem, stream, std::forward<Args>(args)...);
+}
+// elements a streaming kernel may process and still gain from an early launch (about ten microseconds of work)
+constexpr long long kPdlStreamElems = 16ll << 20;
 
 // ---------------------------------------------------------------------------------------------
 // Counter-based rng (bit-compatible with the reference's src/rng.h:7-29 and

@@ -75,6 +75,7 @@ template <> struct StatePiece<float> {
 
 template <typename ST, int NPC, int NI>
 __global__ void __launch_bounds__(kGenThreads, (NI <= 16 ? 2 : 1)) efla_generic_kernel(const EflaParams p) {
+    pdl_wait();
     constexpr int PN = StatePiece<ST>::N;       // columns per piece
     constexpr int NC = NPC * PN;                // columns per CTA
     constexpr int RG = kGenThreads / NPC;       // row groups
@@ -254,7 +255,8 @@ int launch_generic(const EflaParams& p, cudaStream_t stream) {
     const size_t smem = sizeof(float) * (4 * static_cast<size_t>(hd) + 4 * (kGenThreads / 32) + 3 * (kGenThreads / 32) * NC);
     const long long ctas = p.seqs * static_cast<long long>(p.heads) * ((hd + NC - 1) / NC);
     if (ctas > 0x7fffffffLL) return set_error(BNF4_ERR_INVALID, "efla (generic kernel): too many sequences in one call");
-    efla_generic_kernel<ST, NPC, NI><<<static_cast<unsigned>(ctas), kGenThreads, smem, stream>>>(p);
+    const bool early = p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems;
+    launch_pdl_if(early, efla_generic_kernel<ST, NPC, NI>, static_cast<unsigned>(ctas), kGenThreads, smem, stream, p);
     return check_launch("efla_generic_kernel");
 }
 
@@ -338,6 +340,7 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 __global__ void __launch_bounds__(kScanWarps * 32, kScan2CtasPerSm) efla_scan64_mma2_kernel(const EflaParams p) {
+    pdl_wait();
     constexpr int HD = 64;
     extern __shared__ __align__(16) uint8_t scan_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -594,6 +597,7 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t saddr, uint32_t r0, u
 
 template <bool IN16, bool OUT16>
 __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const EflaParams p) {
+    pdl_wait();
     constexpr int HD = 64;
     extern __shared__ __align__(16) uint8_t scan_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -951,6 +955,7 @@ static_assert(kM1WarpBytes % 16 == 0 && kM1L % 16 == 0 && kM1T % 16 == 0 && kM1B
 
 template <bool OUT16>
 __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_m1_kernel(const EflaParams p) {
+    pdl_wait();
     constexpr int HD = 64;
     extern __shared__ __align__(16) uint8_t scan_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1264,6 +1269,7 @@ int efla_launch(const EflaParams& p, cudaStream_t stream) {
         return set_error(BNF4_ERR_INVALID, "efla: fp16 q, k, v or output are supported by the chunked kernel only");
     if ((p.variant == BNF4_EFLA_PER_TOKEN || p.variant == BNF4_EFLA_CHUNKED) && !regs_ok)
         return set_error(BNF4_ERR_INVALID, "efla: the register-state kernels need head_dim 64, no HBM state, an fp16 state and 16-byte aligned q, k, v");
+    const bool early = p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems;
     if (regs_ok && p.variant != BNF4_EFLA_GENERIC) {
         const bool chunked = p.variant == BNF4_EFLA_CHUNKED || (p.variant == BNF4_EFLA_AUTO && g_efla_chunked != 0);
         const long long units = p.seqs * static_cast<long long>(p.heads);
@@ -1292,20 +1298,19 @@ int efla_launch(const EflaParams& p, cudaStream_t stream) {
             if (p.out_f16 && (((p.ld_out % 8) != 0) || (reinterpret_cast<uintptr_t>(p.out) & 15))) return set_error(BNF4_ERR_INVALID, "efla: fp16 output needs 16-byte aligned rows");
             const unsigned grid = static_cast<unsigned>(ctas);
             if (p.qkv_f16 && p.method == 1) {  // the batched driver's case: raw-operand kernel, persistent warps (two CTAs per SM)
-                int sms = 0;
-                rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
-                if (rc) return rc;
+                const int sms = multiprocessors(dev);
+                if (sms <= 0) return BNF4_ERR_CUDA;
                 const unsigned pgrid = std::min(grid, static_cast<unsigned>(2 * sms));
-                if (p.out_f16) efla_chunk16_m1_kernel<true><<<pgrid, kChunkWarps * 32, kM1SmemBytes, stream>>>(p);
-                else efla_chunk16_m1_kernel<false><<<pgrid, kChunkWarps * 32, kM1SmemBytes, stream>>>(p);
-            } else if (p.qkv_f16 && p.out_f16) efla_chunk16_kernel<true, true><<<grid, kChunkWarps * 32, kCkSmemBytes, stream>>>(p);
-            else if (p.qkv_f16) efla_chunk16_kernel<true, false><<<grid, kChunkWarps * 32, kCkSmemBytes, stream>>>(p);
-            else if (p.out_f16) efla_chunk16_kernel<false, true><<<grid, kChunkWarps * 32, kCkSmemBytes, stream>>>(p);
-            else efla_chunk16_kernel<false, false><<<grid, kChunkWarps * 32, kCkSmemBytes, stream>>>(p);
+                if (p.out_f16) launch_pdl_if(early, efla_chunk16_m1_kernel<true>, pgrid, kChunkWarps * 32, kM1SmemBytes, stream, p);
+                else launch_pdl_if(early, efla_chunk16_m1_kernel<false>, pgrid, kChunkWarps * 32, kM1SmemBytes, stream, p);
+            } else if (p.qkv_f16 && p.out_f16) launch_pdl_if(early, efla_chunk16_kernel<true, true>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
+            else if (p.qkv_f16) launch_pdl_if(early, efla_chunk16_kernel<true, false>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
+            else if (p.out_f16) launch_pdl_if(early, efla_chunk16_kernel<false, true>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
+            else launch_pdl_if(early, efla_chunk16_kernel<false, false>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
             return check_launch("efla_chunk16_kernel");
         }
         if (p.qkv_f16 || p.out_f16) return set_error(BNF4_ERR_INVALID, "efla: fp16 q, k, v or output are supported by the chunked kernel only");
-        efla_scan64_mma2_kernel<<<static_cast<unsigned>(ctas), kScanWarps * 32, kScan2SmemBytes, stream>>>(p);
+        launch_pdl_if(early, efla_scan64_mma2_kernel, static_cast<unsigned>(ctas), kScanWarps * 32, kScan2SmemBytes, stream, p);
         return check_launch("efla_scan64_mma2_kernel");
     }
     if ((hd % 32) != 0) return set_error(BNF4_ERR_INVALID, "efla: head_dim=%d must be a multiple of 32", hd);

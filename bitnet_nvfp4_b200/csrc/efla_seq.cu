@@ -78,6 +78,7 @@ __device__ __forceinline__ float sq_pow2_scale(float m) {
 }
 
 __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaParams p) {
+    pdl_wait();
     extern __shared__ __align__(16) uint8_t sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int T = p.T, hd = p.hidden / p.heads;
@@ -487,7 +488,7 @@ int efla_seq_launch(const EflaParams& p, cudaStream_t stream) {
         if (rc) return rc;
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    efla_seq_kernel<<<static_cast<unsigned>(p.seqs * p.heads), kSeqThreads, kSqSmem, stream>>>(p);
+    launch_pdl_if(p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems, efla_seq_kernel, static_cast<unsigned>(p.seqs * p.heads), kSeqThreads, kSqSmem, stream, p);
     return check_launch("efla_seq_kernel");
 }
 

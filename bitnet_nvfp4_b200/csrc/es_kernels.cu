@@ -66,6 +66,8 @@ __global__ void __launch_bounds__(256) ce_step_kernel(const float* __restrict__ 
                                                       const float* __restrict__ bias_noise, float bns,
                                                       const uint8_t* __restrict__ targets_t, int token_stride, int vocab, int batch,
                                                       float* loss_accum) {
+    pdl_wait();
+    after(logits, bias, bias_noise, targets_t);
     __shared__ float part[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float acc = 0.0f;
@@ -88,6 +90,8 @@ __global__ void __launch_bounds__(256) ce_population_kernel(const float* __restr
                                                             const int8_t* __restrict__ bias_noise, float sigma,
                                                             const uint8_t* __restrict__ targets, int vocab, int rows_per_member,
                                                             float* __restrict__ partial) {
+    pdl_wait();
+    after(logits, bias, bias_noise, targets);
     __shared__ float part[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int member = blockIdx.y, chunk = blockIdx.x;
@@ -118,6 +122,8 @@ __global__ void __launch_bounds__(256) ce_population_vec_kernel(const float* __r
                                                                 const int8_t* __restrict__ bias_noise, float sigma,
                                                                 const uint8_t* __restrict__ targets, int vocab, int rows_per_member,
                                                                 float* __restrict__ partial) {
+    pdl_wait();
+    after(logits, bias, bias_noise, targets);
     __shared__ float part[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int member = blockIdx.y, chunk = blockIdx.x;
@@ -190,6 +196,8 @@ __global__ void __launch_bounds__(256) ce_population_vec_kernel(const float* __r
 }
 
 __global__ void ce_finalize_kernel(const float* __restrict__ partial, int members, int rows_per_member, float* __restrict__ loss_mean) {
+    pdl_wait();
+    after(partial);
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= members) return;
     double t = 0.0;
@@ -201,10 +209,13 @@ __global__ void ce_finalize_kernel(const float* __restrict__ partial, int member
 // Noise
 // ------------------------------------------------------------------------------------------------
 __global__ void fill_noise_kernel(int8_t* __restrict__ out, size_t n, uint64_t seed, int use_clt, int clt_k) {
+    pdl_wait();
     const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx < n) out[idx] = static_cast<int8_t>(noise_hash(seed, idx, use_clt != 0, clt_k));
 }
 __global__ void fill_noise_batched_kernel(const bnf4_noise_desc* __restrict__ descs, int num_desc, int use_clt, int clt_k) {
+    pdl_wait();
+    after(descs);
     const int di = blockIdx.y;
     if (di >= num_desc) return;
     const bnf4_noise_desc d = descs[di];
@@ -212,10 +223,12 @@ __global__ void fill_noise_batched_kernel(const bnf4_noise_desc* __restrict__ de
     if (idx < d.n) d.out[idx] = static_cast<int8_t>(noise_hash(d.seed, idx, use_clt != 0, clt_k));
 }
 __global__ void fill_float_noise_kernel(float* __restrict__ out, int n, uint64_t seed, int use_clt, int clt_k) {
+    pdl_wait();
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx < n) out[idx] = static_cast<float>(noise_hash(seed, static_cast<uint64_t>(idx), use_clt != 0, clt_k));
 }
 __global__ void pair_seeds_kernel(uint64_t base_seed, uint64_t epoch, int pairs, uint64_t* __restrict__ out) {
+    pdl_wait();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p < pairs) out[p] = mix_u64(base_seed, mix_u64(epoch, static_cast<uint64_t>(p)));
 }
@@ -224,6 +237,8 @@ __global__ void pair_seeds_kernel(uint64_t base_seed, uint64_t epoch, int pairs,
 // ES update
 // ------------------------------------------------------------------------------------------------
 __global__ void init_shadow_kernel(const int8_t* __restrict__ w, float* __restrict__ shadow, int n) {
+    pdl_wait();
+    after(w);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) shadow[i] = static_cast<float>(w[i]);
 }
@@ -232,6 +247,8 @@ __global__ void init_shadow_kernel(const int8_t* __restrict__ w, float* __restri
 // Elements idx0 .. idx0 + n - 1 of the vector (the hash is keyed by the element's index in the whole vector) go to Z[0 .. n).
 __global__ void __launch_bounds__(256) z_dense_kernel(const float* __restrict__ pair_weights, const uint64_t* __restrict__ pair_seeds,
                                                       uint64_t salt, int pairs, int idx0, int n, int use_clt, int clt_k, float* __restrict__ Z) {
+    pdl_wait();
+    after(pair_weights, pair_seeds);
     extern __shared__ uint8_t zsm[];
     uint64_t* seeds = reinterpret_cast<uint64_t*>(zsm);
     float* wts = reinterpret_cast<float*>(zsm + sizeof(uint64_t) * 256);
@@ -291,6 +308,8 @@ template <int RANK>
 __global__ void __launch_bounds__(kZThreads) z_lowrank_tiles_kernel(const float* __restrict__ pair_weights, const ZLowrankDesc* __restrict__ descs,
                                                                     int ndesc, const ZLowrankDesc single, int pairs, float cscale, int shard,
                                                                     int nshards) {
+    pdl_wait();
+    after(pair_weights);
     constexpr int PC = RANK <= 2 ? 16 : 8;  // pairs per chunk
     constexpr int TR = kZTileRows, TC = kZTileCols;
     constexpr int A_PER_THREAD = PC * TR * RANK / kZThreads;        // bytes of A per thread and chunk
@@ -418,6 +437,8 @@ __global__ void __launch_bounds__(kZThreads) z_lowrank_tiles_kernel(const float*
 
 // Sum of squares, stage 1: block b reduces Z[256b .. 256b+255] with the reference's shared-memory tree.
 __global__ void __launch_bounds__(256) sumsq_blocks_kernel(const float* __restrict__ Z, int n, float* __restrict__ partial) {
+    pdl_wait();
+    after(Z);
     __shared__ float sh[256];
     const int idx = blockIdx.x * 256 + threadIdx.x;
     const float z = idx < n ? Z[idx] : 0.0f;
@@ -432,6 +453,8 @@ __global__ void __launch_bounds__(256) sumsq_blocks_kernel(const float* __restri
 // stage 2: one warp adds the block partials in double (lane-contiguous ranges, then lanes in order) and
 // accumulates into *sumsq.
 __global__ void sumsq_final_kernel(const float* __restrict__ partial, int nblocks, float* sumsq) {
+    pdl_wait();
+    after(partial);
     __shared__ double lane_sum[32];
     const int lane = threadIdx.x;
     const int per = (nblocks + 31) / 32;
@@ -448,6 +471,8 @@ __global__ void sumsq_final_kernel(const float* __restrict__ partial, int nblock
 
 __global__ void inv_rms_kernel(const float* __restrict__ sumsq, float* __restrict__ rms_ema, int use_adaptive, float beta, float eps,
                                int n, float* __restrict__ inv_rms_out) {
+    pdl_wait();
+    after(sumsq);
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     float inv = 1.0f;
     if (use_adaptive) {
@@ -463,6 +488,8 @@ __global__ void inv_rms_kernel(const float* __restrict__ sumsq, float* __restric
 
 __global__ void update_shadow_kernel(int8_t* __restrict__ w, float* __restrict__ shadow, const float* __restrict__ Z, int n,
                                      const float* __restrict__ inv_rms_dev, float inv_rms_host, float lr, float thresh) {
+    pdl_wait();
+    after(Z, inv_rms_dev);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float inv = inv_rms_dev != nullptr ? inv_rms_dev[0] : inv_rms_host;
@@ -475,6 +502,8 @@ __global__ void update_shadow_kernel(int8_t* __restrict__ w, float* __restrict__
 
 __global__ void update_vector_kernel(float* __restrict__ v, const float* __restrict__ Z, int n, const float* __restrict__ inv_rms,
                                      float lr, float thresh) {
+    pdl_wait();
+    after(Z, inv_rms);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float g = __fmul_rn(inv_rms[0], Z[i]);
@@ -483,6 +512,8 @@ __global__ void update_vector_kernel(float* __restrict__ v, const float* __restr
 }
 
 __global__ void add_scaled_kernel(float* __restrict__ out, const float* __restrict__ noise, int n, float scale) {
+    pdl_wait();
+    after(noise);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = fmaf(scale, noise[i], out[i]);
 }
@@ -500,6 +531,7 @@ __device__ __forceinline__ int find_tensor(const UpdApplyDesc* __restrict__ d, i
     return lo;
 }
 __global__ void __launch_bounds__(256) sumsq_blocks_batched_kernel(const UpdApplyDesc* __restrict__ d, int ndesc, float* __restrict__ partial) {
+    pdl_wait();
     __shared__ float sh[256];
     __shared__ int ti;
     if (threadIdx.x == 0) ti = find_tensor(d, ndesc, static_cast<int>(blockIdx.x));
@@ -518,6 +550,8 @@ __global__ void __launch_bounds__(256) sumsq_blocks_batched_kernel(const UpdAppl
 // one warp per tensor; then its lane 0 turns the sum into inv_rms (and advances the tensor's RMS-EMA)
 __global__ void sumsq_final_inv_rms_batched_kernel(const UpdApplyDesc* __restrict__ d, const float* __restrict__ partial, int use_adaptive,
                                                    float beta, float eps, float* __restrict__ inv_rms_out) {
+    pdl_wait();
+    after(partial);
     __shared__ double lane_sum[32];
     const UpdApplyDesc& x = d[blockIdx.x];
     const int lane = threadIdx.x;
@@ -546,6 +580,8 @@ __global__ void sumsq_final_inv_rms_batched_kernel(const UpdApplyDesc* __restric
 }
 __global__ void __launch_bounds__(256) update_batched_kernel(const UpdApplyDesc* __restrict__ d, int ndesc, const float* __restrict__ inv_rms,
                                                              float lr, float thresh) {
+    pdl_wait();
+    after(inv_rms);
     __shared__ int ti;
     if (threadIdx.x == 0) ti = find_tensor(d, ndesc, static_cast<int>(blockIdx.x));
     __syncthreads();
@@ -598,7 +634,7 @@ int get_scratch(size_t floats, float** out) {
 int z_dense_launch(const float* pair_weights, const uint64_t* pair_seeds, uint64_t salt, int pairs, int idx0, int n, int use_clt, int clt_k,
                    float* Z, cudaStream_t st) {
     if (n <= 0) return BNF4_OK;
-    z_dense_kernel<<<(n + 255) / 256, 256, 256 * (sizeof(uint64_t) + sizeof(float)), st>>>(pair_weights, pair_seeds, salt, pairs, idx0, n, use_clt, clt_k, Z);
+    launch_pdl_if(static_cast<long long>(n) * pairs <= (1ll << 22), z_dense_kernel, (n + 255) / 256, 256, 256 * (sizeof(uint64_t) + sizeof(float)), st, pair_weights, pair_seeds, salt, pairs, idx0, n, use_clt, clt_k, Z);
     return check_launch("z_dense_kernel");
 }
 
@@ -607,13 +643,14 @@ int z_dense_launch(const float* pair_weights, const uint64_t* pair_seeds, uint64
 int update_apply_batched(const UpdApplyDesc* d_descs, int ndesc, int total_blocks, float* partial, float* inv_rms, int use_adaptive, float beta,
                          float eps, float lr, float thresh, cudaStream_t st) {
     if (ndesc <= 0 || total_blocks <= 0) return BNF4_OK;
-    sumsq_blocks_batched_kernel<<<total_blocks, 256, 0, st>>>(d_descs, ndesc, partial);
+    const bool early = total_blocks * 256ll <= kPdlStreamElems;
+    launch_pdl_if(early, sumsq_blocks_batched_kernel, total_blocks, 256, 0, st, d_descs, ndesc, partial);
     int rc = check_launch("sumsq_blocks_batched_kernel");
     if (rc) return rc;
-    sumsq_final_inv_rms_batched_kernel<<<ndesc, 32, 0, st>>>(d_descs, partial, use_adaptive, beta, eps, inv_rms);
+    launch_pdl(sumsq_final_inv_rms_batched_kernel, ndesc, 32, 0, st, d_descs, partial, use_adaptive, beta, eps, inv_rms);
     rc = check_launch("sumsq_final_inv_rms_batched_kernel");
     if (rc) return rc;
-    update_batched_kernel<<<total_blocks, 256, 0, st>>>(d_descs, ndesc, inv_rms, lr, thresh);
+    launch_pdl_if(early, update_batched_kernel, total_blocks, 256, 0, st, d_descs, ndesc, inv_rms, lr, thresh);
     return check_launch("update_batched_kernel");
 }
 
@@ -635,10 +672,10 @@ int z_lowrank_launch(const float* pair_weights, const ZLowrankDesc* d_descs, con
     const unsigned grid = static_cast<unsigned>(tiles);
     const ZLowrankDesc single = h_descs[0];
     switch (rank) {
-        case 1: z_lowrank_tiles_kernel<1><<<grid, kZThreads, 0, st>>>(pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
-        case 2: z_lowrank_tiles_kernel<2><<<grid, kZThreads, 0, st>>>(pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
-        case 3: z_lowrank_tiles_kernel<3><<<grid, kZThreads, 0, st>>>(pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
-        default: z_lowrank_tiles_kernel<4><<<grid, kZThreads, 0, st>>>(pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
+        case 1: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<1>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
+        case 2: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<2>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
+        case 3: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<3>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
+        default: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<4>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
     }
     return check_launch("z_lowrank_tiles_kernel");
 }
@@ -650,10 +687,10 @@ int sumsq_into(const float* Z, int n, float* sumsq, cudaStream_t st) {
     float* partial = nullptr;
     int rc = get_scratch(static_cast<size_t>(nblocks), &partial);
     if (rc) return rc;
-    sumsq_blocks_kernel<<<nblocks, 256, 0, st>>>(Z, n, partial);
+    launch_pdl(sumsq_blocks_kernel, nblocks, 256, 0, st, Z, n, partial);
     rc = check_launch("sumsq_blocks_kernel");
     if (rc) return rc;
-    sumsq_final_kernel<<<1, 32, 0, st>>>(partial, nblocks, sumsq);
+    launch_pdl(sumsq_final_kernel, 1, 32, 0, st, partial, nblocks, sumsq);
     return check_launch("sumsq_final_kernel");
 }
 
@@ -661,10 +698,10 @@ int sumsq_into(const float* Z, int n, float* sumsq, cudaStream_t st) {
 
 int sumsq_with_scratch(const float* Z, int n, float* partial, float* sumsq, cudaStream_t st) {
     const int nblocks = (n + 255) / 256;
-    sumsq_blocks_kernel<<<nblocks, 256, 0, st>>>(Z, n, partial);
+    launch_pdl(sumsq_blocks_kernel, nblocks, 256, 0, st, Z, n, partial);
     int rc = check_launch("sumsq_blocks_kernel");
     if (rc) return rc;
-    sumsq_final_kernel<<<1, 32, 0, st>>>(partial, nblocks, sumsq);
+    launch_pdl(sumsq_final_kernel, 1, 32, 0, st, partial, nblocks, sumsq);
     return check_launch("sumsq_final_kernel");
 }
 
@@ -680,7 +717,7 @@ int bnf4_cross_entropy_loss(const float* logits, const float* bias, const float*
     if (batch <= 0) return BNF4_OK;
     if (!logits || !targets_t || !loss_accum) return set_error(BNF4_ERR_INVALID, "cross_entropy_loss: null pointer");
     if (vocab <= 0 || vocab > 32 * kCeMaxPerLane) return set_error(BNF4_ERR_INVALID, "cross_entropy_loss: vocab=%d outside [1,%d]", vocab, 32 * kCeMaxPerLane);
-    ce_step_kernel<<<1, 256, 0, S(stream)>>>(logits, bias, bias_noise, bias_noise_scale, targets_t, token_stride, vocab, batch, loss_accum);
+    launch_pdl(ce_step_kernel, 1, 256, 0, S(stream), logits, bias, bias_noise, bias_noise_scale, targets_t, token_stride, vocab, batch, loss_accum);
     return check_launch("ce_step_kernel");
 }
 
@@ -692,53 +729,54 @@ int bnf4_cross_entropy_population(const float* logits, int ld, const float* bias
     if (vocab <= 0 || vocab > 32 * kCeMaxPerLane) return set_error(BNF4_ERR_INVALID, "cross_entropy_population: vocab=%d", vocab);
     if (members > 65535) return set_error(BNF4_ERR_INVALID, "cross_entropy_population: at most 65535 members per call");
     const dim3 grid(kCeChunks, members);
+    const bool early = static_cast<long long>(members) * rows_per_member * vocab <= kPdlStreamElems;
     const bool vec = (vocab % 4) == 0 && (ld % 4) == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(bias_noise) & 3) == 0;
     if (vec && vocab <= 128)
-        ce_population_vec_kernel<1, 4><<<grid, 256, 0, S(stream)>>>(logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
+        launch_pdl_if(early, ce_population_vec_kernel<1, 4>, grid, 256, 0, S(stream), logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
     else if (vec && vocab <= 256)
-        ce_population_vec_kernel<2, 4><<<grid, 256, 0, S(stream)>>>(logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
+        launch_pdl_if(early, ce_population_vec_kernel<2, 4>, grid, 256, 0, S(stream), logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
     else if (vec && vocab <= 512)
-        ce_population_vec_kernel<4, 2><<<grid, 256, 0, S(stream)>>>(logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
+        launch_pdl_if(early, ce_population_vec_kernel<4, 2>, grid, 256, 0, S(stream), logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
     else if (vec)
-        ce_population_vec_kernel<8, 1><<<grid, 256, 0, S(stream)>>>(logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
+        launch_pdl_if(early, ce_population_vec_kernel<8, 1>, grid, 256, 0, S(stream), logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
     else
-        ce_population_kernel<<<grid, 256, 0, S(stream)>>>(logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
+        launch_pdl_if(early, ce_population_kernel, grid, 256, 0, S(stream), logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
     int rc = check_launch("ce_population_kernel");
     if (rc) return rc;
-    ce_finalize_kernel<<<(members + 127) / 128, 128, 0, S(stream)>>>(partial, members, rows_per_member, loss_mean);
+    launch_pdl(ce_finalize_kernel, (members + 127) / 128, 128, 0, S(stream), partial, members, rows_per_member, loss_mean);
     return check_launch("ce_finalize_kernel");
 }
 
 int bnf4_fill_ternary_noise(int8_t* out, size_t n, uint64_t seed, int use_clt, int clt_k, void* stream) {
     if (n == 0) return BNF4_OK;
     if (!out) return set_error(BNF4_ERR_INVALID, "fill_ternary_noise: null pointer");
-    fill_noise_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, S(stream)>>>(out, n, seed, use_clt, clt_k);
+    launch_pdl(fill_noise_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0, S(stream), out, n, seed, use_clt, clt_k);
     return check_launch("fill_noise_kernel");
 }
 
 int bnf4_fill_ternary_noise_batched(const bnf4_noise_desc* descs, int num_desc, int max_blocks, int use_clt, int clt_k, void* stream) {
     if (num_desc <= 0 || max_blocks <= 0) return BNF4_OK;
     if (!descs) return set_error(BNF4_ERR_INVALID, "fill_ternary_noise_batched: null pointer");
-    fill_noise_batched_kernel<<<dim3(max_blocks, num_desc), 256, 0, S(stream)>>>(descs, num_desc, use_clt, clt_k);
+    launch_pdl(fill_noise_batched_kernel, dim3(max_blocks, num_desc), 256, 0, S(stream), descs, num_desc, use_clt, clt_k);
     return check_launch("fill_noise_batched_kernel");
 }
 
 int bnf4_fill_float_noise(float* out, int n, uint64_t seed, int use_clt, int clt_k, void* stream) {
     if (n <= 0) return BNF4_OK;
-    fill_float_noise_kernel<<<(n + 255) / 256, 256, 0, S(stream)>>>(out, n, seed, use_clt, clt_k);
+    launch_pdl(fill_float_noise_kernel, (n + 255) / 256, 256, 0, S(stream), out, n, seed, use_clt, clt_k);
     return check_launch("fill_float_noise_kernel");
 }
 
 int bnf4_init_shadow_from_weights(const int8_t* w, float* shadow, int n, void* stream) {
     if (n <= 0) return BNF4_OK;
-    init_shadow_kernel<<<(n + 255) / 256, 256, 0, S(stream)>>>(w, shadow, n);
+    launch_pdl(init_shadow_kernel, (n + 255) / 256, 256, 0, S(stream), w, shadow, n);
     return check_launch("init_shadow_kernel");
 }
 
 int bnf4_fill_pair_seeds(uint64_t base_seed, uint64_t epoch, int pairs, uint64_t* out, void* stream) {
     if (pairs <= 0) return BNF4_OK;
-    pair_seeds_kernel<<<(pairs + 255) / 256, 256, 0, S(stream)>>>(base_seed, epoch, pairs, out);
+    launch_pdl(pair_seeds_kernel, (pairs + 255) / 256, 256, 0, S(stream), base_seed, epoch, pairs, out);
     return check_launch("pair_seeds_kernel");
 }
 
@@ -746,7 +784,7 @@ int bnf4_compute_z_sumsq(const float* pair_weights, const uint64_t* pair_seeds, 
                          int clt_k, float* Z, float* sumsq, void* stream) {
     if (n <= 0) return BNF4_OK;
     if (!pair_weights || !pair_seeds || !Z || !sumsq) return set_error(BNF4_ERR_INVALID, "compute_z_sumsq: null pointer");
-    z_dense_kernel<<<(n + 255) / 256, 256, 256 * (sizeof(uint64_t) + sizeof(float)), S(stream)>>>(pair_weights, pair_seeds, salt, pairs, 0, n, use_clt, clt_k, Z);
+    launch_pdl_if(static_cast<long long>(n) * pairs <= (1ll << 22), z_dense_kernel, (n + 255) / 256, 256, 256 * (sizeof(uint64_t) + sizeof(float)), S(stream), pair_weights, pair_seeds, salt, pairs, 0, n, use_clt, clt_k, Z);
     const int rc = check_launch("z_dense_kernel");
     if (rc) return rc;
     return sumsq_into(Z, n, sumsq, S(stream));
@@ -779,7 +817,7 @@ int bnf4_compute_z_sumsq_lowrank(const float* pair_weights, const int8_t* A, lon
 int bnf4_update_inv_rms(const float* sumsq, float* rms_ema, int use_adaptive, float adaptive_beta, float adaptive_eps, int n,
                         float* inv_rms, void* stream) {
     if (!sumsq || !rms_ema || !inv_rms) return set_error(BNF4_ERR_INVALID, "update_inv_rms: null pointer");
-    inv_rms_kernel<<<1, 1, 0, S(stream)>>>(sumsq, rms_ema, use_adaptive, adaptive_beta, adaptive_eps, n, inv_rms);
+    launch_pdl(inv_rms_kernel, 1, 1, 0, S(stream), sumsq, rms_ema, use_adaptive, adaptive_beta, adaptive_eps, n, inv_rms);
     return check_launch("inv_rms_kernel");
 }
 
@@ -787,25 +825,25 @@ int bnf4_update_shadow_ternary_device(int8_t* w, float* shadow, const float* Z, 
                                       float thresh, void* stream) {
     if (n <= 0) return BNF4_OK;
     if (!inv_rms) return set_error(BNF4_ERR_INVALID, "update_shadow_ternary_device: null inv_rms");
-    update_shadow_kernel<<<(n + 255) / 256, 256, 0, S(stream)>>>(w, shadow, Z, n, inv_rms, 0.0f, lr, thresh);
+    launch_pdl(update_shadow_kernel, (n + 255) / 256, 256, 0, S(stream), w, shadow, Z, n, inv_rms, 0.0f, lr, thresh);
     return check_launch("update_shadow_kernel");
 }
 
 int bnf4_update_shadow_ternary(int8_t* w, float* shadow, const float* Z, int n, float inv_rms, float lr, float thresh, void* stream) {
     if (n <= 0) return BNF4_OK;
-    update_shadow_kernel<<<(n + 255) / 256, 256, 0, S(stream)>>>(w, shadow, Z, n, nullptr, inv_rms, lr, thresh);
+    launch_pdl(update_shadow_kernel, (n + 255) / 256, 256, 0, S(stream), w, shadow, Z, n, nullptr, inv_rms, lr, thresh);
     return check_launch("update_shadow_kernel");
 }
 
 int bnf4_update_vector_device(float* v, const float* Z, int n, const float* inv_rms, float lr, float thresh, void* stream) {
     if (n <= 0) return BNF4_OK;
-    update_vector_kernel<<<(n + 255) / 256, 256, 0, S(stream)>>>(v, Z, n, inv_rms, lr, thresh);
+    launch_pdl(update_vector_kernel, (n + 255) / 256, 256, 0, S(stream), v, Z, n, inv_rms, lr, thresh);
     return check_launch("update_vector_kernel");
 }
 
 int bnf4_add_scaled(float* out, const float* noise, int n, float scale, void* stream) {
     if (n <= 0) return BNF4_OK;
-    add_scaled_kernel<<<(n + 255) / 256, 256, 0, S(stream)>>>(out, noise, n, scale);
+    launch_pdl(add_scaled_kernel, (n + 255) / 256, 256, 0, S(stream), out, noise, n, scale);
     return check_launch("add_scaled_kernel");
 }
 
@@ -865,7 +903,7 @@ extern "C" int bnf4_compute_z_sumsq_static(const float* pair_weights, const uint
     int rc = static_partials(&partial);
     if (rc) return rc;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
-    z_dense_kernel<<<(n + 255) / 256, 256, 256 * (sizeof(uint64_t) + sizeof(float)), st>>>(pair_weights, pair_seeds, salt, pairs, 0, n, use_clt, clt_k, Z);
+    launch_pdl_if(static_cast<long long>(n) * pairs <= (1ll << 22), z_dense_kernel, (n + 255) / 256, 256, 256 * (sizeof(uint64_t) + sizeof(float)), st, pair_weights, pair_seeds, salt, pairs, 0, n, use_clt, clt_k, Z);
     rc = check_launch("z_dense_kernel");
     if (rc) return rc;
     // Every partial the final kernel reads (indices 0 .. ceil(n/256)-1) is written by the block kernel of this same

@@ -21,6 +21,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -266,6 +267,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_gen;
+    pdl_wait();  // the set-up above overlaps the predecessor's tail; everything below reads what it wrote
 
     if (warp == 0) {
         // ------------------------------ producer ------------------------------
@@ -307,6 +309,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     if (++s == kStages) { s = 0; empty_parity ^= 1u; }
                 }
             }
+            pdl_trigger();  // every operand is on its way: what is left of this CTA is its last tile
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer ------------------------------
@@ -410,7 +413,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         // Members are visited in ascending order, so when tiles never straddle members (rows_per_member a multiple of the
         // tile height) the member of the next tile is tracked with comparisons instead of a division per row.
         const bool tile_uniform_member = p.rows_per_member > 0 && (p.rows_per_member % BM) == 0;
-        int trk_member = 0;
+        int trk_member = static_cast<int>(opaque_zero());  // (the pair's vectors are loaded read-only: their addresses depend on this)
         long long trk_end = p.rows_per_member;  // first row of member trk_member + 1
         const uint32_t group_magic = args.group_magic;  // ceil(2^32 / group_cols): exact quotients for columns below 65536
         auto fetch_ctx = [&](const TileIdx& t, bool valid, LoraCtx& cx) {
@@ -446,22 +449,22 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             if (row_ < p.m && col0_ < p.n) {
                 const int g = p.group_cols > 0 ? static_cast<int>(__umulhi(static_cast<uint32_t>(col0_), group_magic)) : 0;
                 const int* tp = p.lora_t + static_cast<size_t>(row_) * p.t_stride + g * p.rank;
-                cx.tr[0] = __ldg(tp);
+                cx.tr[0] = tp[0];
                 if (p.rank > 1) {
-                    cx.tr[1] = __ldg(tp + 1);
-                    if (p.rank > 2) cx.tr[2] = __ldg(tp + 2);
-                    if (p.rank > 3) cx.tr[3] = __ldg(tp + 3);
+                    cx.tr[1] = tp[1];
+                    if (p.rank > 2) cx.tr[2] = tp[2];
+                    if (p.rank > 3) cx.tr[3] = tp[3];
                 }
             }
             cx.a_staged = (pair_first == pair_last);
             const int n = col0_ + lane;
             if (cx.a_staged && n < p.n) {
                 const int8_t* Ag = p.lora_A + static_cast<size_t>(pair_first) * p.lora_A_pair_stride + static_cast<size_t>(n) * p.rank;
-                cx.aval[0] = __ldg(Ag);
+                cx.aval[0] = Ag[0];
                 if (p.rank > 1) {
-                    cx.aval[1] = __ldg(Ag + 1);
-                    if (p.rank > 2) cx.aval[2] = __ldg(Ag + 2);
-                    if (p.rank > 3) cx.aval[3] = __ldg(Ag + 3);
+                    cx.aval[1] = Ag[1];
+                    if (p.rank > 2) cx.aval[2] = Ag[2];
+                    if (p.rank > 3) cx.aval[3] = Ag[3];
                 }
             }
         };
@@ -482,7 +485,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             cx.pair = trk_member >> 1;
             if ((R1 || m0_ + row_in_tile < p.m) && col0_ < p.n) {
                 const int g = p.group_cols > 0 ? static_cast<int>(__umulhi(static_cast<uint32_t>(col0_), group_magic)) : 0;
-                cx.tr[0] = __ldg(t_row + static_cast<size_t>(m0_) * p.t_stride + g);
+                cx.tr[0] = t_row[static_cast<size_t>(m0_) * p.t_stride + g];
                 cx.lsign = (trk_member & 1) ? -p.lora_scale : p.lora_scale;
             }
             if (col0_ + lane < p.n) cx.aval[0] = __ldg(p.lora_A + static_cast<size_t>(cx.pair) * p.lora_A_pair_stride + col0_ + lane);
@@ -908,8 +911,35 @@ EncodeTiledFn get_encode_fn() {
     return fn;
 }
 
+// Encoding a tensor map costs about half a microsecond of host time, as much as the rest of a launch's preparation, and callers
+// keep their buffers: each thread keeps the maps of its last calls (direct-mapped, 256 entries, no device memory). A map is a
+// pure function of its key.
+struct MapKey {
+    const void* base;
+    uint64_t dim0, dim1, stride1;
+    uint32_t box0, box1;
+    int dt, swizzle;
+    bool operator==(const MapKey& o) const {
+        return base == o.base && dim0 == o.dim0 && dim1 == o.dim1 && stride1 == o.stride1 && box0 == o.box0 && box1 == o.box1 && dt == o.dt && swizzle == o.swizzle;
+    }
+};
+struct MapSlot {
+    MapKey key;
+    CUtensorMap map;
+};
+constexpr unsigned kMapSlots = 256;
+
 int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t dim0, uint64_t dim1, uint64_t stride1_bytes,
                 uint32_t box0, uint32_t box1, const char* what, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
+    static thread_local std::vector<MapSlot> cache;
+    if (cache.empty()) cache.resize(kMapSlots, MapSlot{});
+    const MapKey key{base, dim0, dim1, stride1_bytes, box0, box1, static_cast<int>(dt), static_cast<int>(swizzle)};
+    const uint64_t hash = mix_u64(reinterpret_cast<uint64_t>(base), mix_u64(dim0 ^ (static_cast<uint64_t>(box1) << 48), dim1 ^ (stride1_bytes << 24)));
+    MapSlot& slot = cache[hash % kMapSlots];
+    if (base != nullptr && slot.key == key) {
+        *map = slot.map;
+        return BNF4_OK;
+    }
     EncodeTiledFn fn = get_encode_fn();
     if (fn == nullptr) return set_error(BNF4_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     const cuuint64_t dims[2] = {dim0, dim1};
@@ -919,22 +949,22 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint
     const CUresult r = fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(BNF4_ERR_CUDA, "cuTensorMapEncodeTiled(%s) failed with %d", what, static_cast<int>(r));
+    slot.key = key;
+    slot.map = *map;
     return BNF4_OK;
 }
 
 template <int EPI, int RK>
-int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, const KernelArgs& args, dim3 grid,
+int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, const KernelArgs& args, dim3 grid, int dev,
              cudaStream_t stream) {
-    // function attributes are per device: set once for each device this process uses
-    static bool configured[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return check_cuda(cudaGetLastError(), "cudaGetDevice");
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
+    static bool configured[64] = {};  // function attributes are per device: set once for each device this process uses
+    if (!configured[dev]) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_nvfp4_kernel<EPI, RK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlloc);
         if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(gemm_nvfp4_kernel)");
-        if (dev >= 0 && dev < 64) configured[dev] = true;
+        configured[dev] = true;
     }
-    gemm_nvfp4_kernel<EPI, RK><<<grid, kThreads, kSmemAlloc, stream>>>(ma, mb, md, args);
+    // (an early launch pays while the kernel is short: a dozen tiles per SM)
+    launch_pdl_if(args.total_tiles <= 12 * static_cast<int>(grid.x), gemm_nvfp4_kernel<EPI, RK>, grid, kThreads, kSmemAlloc, stream, ma, mb, md, args);
     return check_launch("gemm_nvfp4_kernel");
 }
 
@@ -1011,21 +1041,21 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     const long long tiles = static_cast<long long>(args.n_tiles) * ((p.m + BM - 1) / BM);
     if (tiles > 0x7fffffffLL) return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: too many tiles");
     args.total_tiles = static_cast<int>(tiles);
-    int dev = 0, sms = 0;
-    rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+    int dev = 0;
+    rc = current_device(&dev);
     if (rc) return rc;
-    rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
-    if (rc) return rc;
+    const int sms = multiprocessors(dev);
+    if (sms <= 0) return BNF4_ERR_CUDA;
     const dim3 grid(static_cast<unsigned>(std::min<long long>(tiles, sms)), 1, 1);
     const bool gelu = p.epilogue == EPI_GELU_FP4 || p.epilogue == EPI_GELU_I8;
     const bool gelu_plain = !gelu || (p.act_scale <= 700.0f && (p.n % 32) == 0 && (p.epilogue == EPI_GELU_FP4 ? (p.next_nvec == 1 && p.d_i8 == nullptr) : p.next_nvec <= 1));
     const int rk = p.rank == 4 ? 4 : ((p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1)) ? 1 : 0);
     switch (p.epilogue) {
-        case EPI_F32: return rk == 4 ? launch_t<EPI_F32, 4>(ma, mb, md, args, grid, stream) : (rk == 1 ? launch_t<EPI_F32, 1>(ma, mb, md, args, grid, stream) : launch_t<EPI_F32, 0>(ma, mb, md, args, grid, stream));
-        case EPI_GELU_I8: return rk == 4 ? launch_t<EPI_GELU_I8, 4>(ma, mb, md, args, grid, stream) : (rk == 1 ? launch_t<EPI_GELU_I8, 1>(ma, mb, md, args, grid, stream) : launch_t<EPI_GELU_I8, 0>(ma, mb, md, args, grid, stream));
-        case EPI_GELU_FP4: return rk == 4 ? launch_t<EPI_GELU_FP4, 4>(ma, mb, md, args, grid, stream) : (rk == 1 ? launch_t<EPI_GELU_FP4, 1>(ma, mb, md, args, grid, stream) : launch_t<EPI_GELU_FP4, 0>(ma, mb, md, args, grid, stream));
-        case EPI_ADD_I8: return rk == 4 ? launch_t<EPI_ADD_I8, 4>(ma, mb, md, args, grid, stream) : (rk == 1 ? launch_t<EPI_ADD_I8, 1>(ma, mb, md, args, grid, stream) : launch_t<EPI_ADD_I8, 0>(ma, mb, md, args, grid, stream));
-        case EPI_F16: return rk == 4 ? launch_t<EPI_F16, 4>(ma, mb, md, args, grid, stream) : (rk == 1 ? launch_t<EPI_F16, 1>(ma, mb, md, args, grid, stream) : launch_t<EPI_F16, 0>(ma, mb, md, args, grid, stream));
+        case EPI_F32: return rk == 4 ? launch_t<EPI_F32, 4>(ma, mb, md, args, grid, dev, stream) : (rk == 1 ? launch_t<EPI_F32, 1>(ma, mb, md, args, grid, dev, stream) : launch_t<EPI_F32, 0>(ma, mb, md, args, grid, dev, stream));
+        case EPI_GELU_I8: return rk == 4 ? launch_t<EPI_GELU_I8, 4>(ma, mb, md, args, grid, dev, stream) : (rk == 1 ? launch_t<EPI_GELU_I8, 1>(ma, mb, md, args, grid, dev, stream) : launch_t<EPI_GELU_I8, 0>(ma, mb, md, args, grid, dev, stream));
+        case EPI_GELU_FP4: return rk == 4 ? launch_t<EPI_GELU_FP4, 4>(ma, mb, md, args, grid, dev, stream) : (rk == 1 ? launch_t<EPI_GELU_FP4, 1>(ma, mb, md, args, grid, dev, stream) : launch_t<EPI_GELU_FP4, 0>(ma, mb, md, args, grid, dev, stream));
+        case EPI_ADD_I8: return rk == 4 ? launch_t<EPI_ADD_I8, 4>(ma, mb, md, args, grid, dev, stream) : (rk == 1 ? launch_t<EPI_ADD_I8, 1>(ma, mb, md, args, grid, dev, stream) : launch_t<EPI_ADD_I8, 0>(ma, mb, md, args, grid, dev, stream));
+        case EPI_F16: return rk == 4 ? launch_t<EPI_F16, 4>(ma, mb, md, args, grid, dev, stream) : (rk == 1 ? launch_t<EPI_F16, 1>(ma, mb, md, args, grid, dev, stream) : launch_t<EPI_F16, 0>(ma, mb, md, args, grid, dev, stream));
     }
     return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: unknown epilogue %d", p.epilogue);
 }

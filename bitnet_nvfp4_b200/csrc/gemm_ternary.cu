@@ -24,6 +24,8 @@ constexpr int TKW = 64;  // 32-bit words (=256 int8 columns, one scale group) pe
 __global__ void __launch_bounds__(256) gemm_ternary_f_kernel(const int8_t* __restrict__ x, const int8_t* __restrict__ w,
                                                              const float* __restrict__ scale_x, float out_scale, int cols,
                                                              int rows, int batch, float* __restrict__ out) {
+    pdl_wait();
+    after(x, w, scale_x);
     __shared__ int xs[TB][TKW + 1];
     __shared__ int ws[TR][TKW + 1];
     const int b0 = blockIdx.y * TB, i0 = blockIdx.x * TR;
@@ -74,6 +76,8 @@ __global__ void __launch_bounds__(256) gemm_ternary_f_kernel(const int8_t* __res
 
 __global__ void lora_t_kernel(const int8_t* __restrict__ x, const int8_t* __restrict__ B, int cols, int batch, int rank,
                               int32_t* __restrict__ t) {
+    pdl_wait();
+    after(x, B);
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= batch * rank) return;
     const int b = warp / rank, r = warp - b * rank;
@@ -85,6 +89,8 @@ __global__ void lora_t_kernel(const int8_t* __restrict__ x, const int8_t* __rest
 
 __global__ void lora_add_kernel(const int32_t* __restrict__ t, const int8_t* __restrict__ A, int rows, int batch, int rank,
                                 float scale, float* __restrict__ out) {
+    pdl_wait();
+    after(t, A);
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     const int b = blockIdx.y;
     if (row >= rows || b >= batch) return;
@@ -96,6 +102,8 @@ __global__ void lora_add_kernel(const int32_t* __restrict__ t, const int8_t* __r
 
 __global__ void split_qkvb_kernel(const float* __restrict__ in, int batch, int hidden, int fused_cols, float* __restrict__ q,
                                   float* __restrict__ k, float* __restrict__ v, float* __restrict__ beta, float beta_bias) {
+    pdl_wait();
+    after(in);
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int b = blockIdx.y;
     if (b >= batch || c >= hidden) return;
@@ -121,21 +129,21 @@ int bnf4_gemm_ternary_f(const int8_t* x, const int8_t* w, const float* scale_x, 
     if (!x || !w || !out || cols <= 0) return set_error(BNF4_ERR_INVALID, "gemm_ternary_f: bad argument");
     if ((batch + TB - 1) / TB > 65535) return set_error(BNF4_ERR_INVALID, "gemm_ternary_f: batch too large");
     const dim3 grid((rows + TR - 1) / TR, (batch + TB - 1) / TB);
-    gemm_ternary_f_kernel<<<grid, 256, 0, S(stream)>>>(x, w, scale_x, out_scale, cols, rows, batch, out);
+    launch_pdl(gemm_ternary_f_kernel, grid, 256, 0, S(stream), x, w, scale_x, out_scale, cols, rows, batch, out);
     return check_launch("gemm_ternary_f_kernel");
 }
 
 int bnf4_lora_compute_t(const int8_t* x, const int8_t* B, int cols, int batch, int rank, int32_t* t, void* stream) {
     if (batch <= 0 || rank <= 0) return BNF4_OK;
     const int warps = batch * rank;
-    lora_t_kernel<<<(warps + 3) / 4, 128, 0, S(stream)>>>(x, B, cols, batch, rank, t);
+    launch_pdl(lora_t_kernel, (warps + 3) / 4, 128, 0, S(stream), x, B, cols, batch, rank, t);
     return check_launch("lora_t_kernel");
 }
 
 int bnf4_lora_add(const int32_t* t, const int8_t* A, int rows, int batch, int rank, float scale, float* out, void* stream) {
     if (batch <= 0 || rows <= 0) return BNF4_OK;
     if (batch > 65535) return set_error(BNF4_ERR_INVALID, "lora_add: batch too large");
-    lora_add_kernel<<<dim3((rows + 127) / 128, batch), 128, 0, S(stream)>>>(t, A, rows, batch, rank, scale, out);
+    launch_pdl(lora_add_kernel, dim3((rows + 127) / 128, batch), 128, 0, S(stream), t, A, rows, batch, rank, scale, out);
     return check_launch("lora_add_kernel");
 }
 
@@ -143,7 +151,7 @@ int bnf4_split_qkvb_fused(const float* in, int batch, int hidden, int fused_cols
                           float beta_bias, void* stream) {
     if (batch <= 0 || hidden <= 0) return BNF4_OK;
     if (batch > 65535) return set_error(BNF4_ERR_INVALID, "split_qkvb_fused: batch too large");
-    split_qkvb_kernel<<<dim3((hidden + 127) / 128, batch), 128, 0, S(stream)>>>(in, batch, hidden, fused_cols, q, k, v, beta, beta_bias);
+    launch_pdl(split_qkvb_kernel, dim3((hidden + 127) / 128, batch), 128, 0, S(stream), in, batch, hidden, fused_cols, q, k, v, beta, beta_bias);
     return check_launch("split_qkvb_kernel");
 }
 

@@ -44,6 +44,8 @@ struct GenDesc {
 // block_map[b] = (descriptor << 20) | block within that descriptor: every launched block has work.
 __global__ void gen_noise_kernel(const GenDesc* __restrict__ descs, const uint32_t* __restrict__ block_map, int block0, int pair0,
                                  const uint64_t* __restrict__ pair_seeds, int use_clt, int clt_k) {
+    pdl_wait();
+    after(pair_seeds);
     const uint32_t bm = block_map[block0 + blockIdx.x];
     const GenDesc d = descs[bm >> 20];
     const int pair = pair0 + blockIdx.y;
@@ -64,6 +66,8 @@ __global__ void gen_noise_kernel(const GenDesc* __restrict__ descs, const uint32
 // beta_bias_eff[l][member] = beta_bias[l] + ns(member) * noise[pair][l]   (reference: src/train_efla_lm.cpp:2912-2917)
 __global__ void beta_bias_kernel(const float* __restrict__ beta_bias, const int8_t* __restrict__ noise, int layers, int members,
                                  float sigma, float* __restrict__ out) {
+    pdl_wait();
+    after(beta_bias, noise);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= layers * members) return;
     const int l = i / members, m = i - l * members;
@@ -243,7 +247,7 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
     {   // per-member beta bias for every layer
         const int n = L * nm;
         TimedScope ts(m, KC_BETA_BIAS, st);
-        beta_bias_kernel<<<(n + 127) / 128, 128, 0, st>>>(m.beta_bias, m.bb_noise + P0 * L, L, nm, sigma, m.bb_eff);
+        launch_pdl(beta_bias_kernel, (n + 127) / 128, 128, 0, st, m.beta_bias, m.bb_noise + P0 * L, L, nm, sigma, m.bb_eff);
         TRY(check_launch("beta_bias_kernel"));
         ++launches;
     }
@@ -528,7 +532,7 @@ int run_pair_dense(Model& m, int pair, float* losses_out, cudaStream_t st) {
     }
     {
         TimedScope ts(m, KC_BETA_BIAS, st);
-        beta_bias_kernel<<<(2 * L + 127) / 128, 128, 0, st>>>(m.beta_bias, m.bb_noise + static_cast<size_t>(pair) * L, L, 2, sigma, m.bb_eff);
+        launch_pdl(beta_bias_kernel, (2 * L + 127) / 128, 128, 0, st, m.beta_bias, m.bb_noise + static_cast<size_t>(pair) * L, L, 2, sigma, m.bb_eff);
         TRY(check_launch("beta_bias_kernel"));
     }
     // base product into d, then the two members' noise products added in place (alpha = +-sigma * alpha_base, beta = 1)
@@ -1054,12 +1058,12 @@ int bnf4_model_prepare_step_range(void* handle, uint64_t seed, uint64_t epoch, i
     TimedScope ts(m, KC_GEN_NOISE, S(stream), 3);
     // rank-r factors of all pairs (the update reads them all; the dense mode has none) ...
     if (!m.dense) {
-        gen_noise_kernel<<<dim3(m.gen_blocks_factors, pairs), 256, 0, S(stream)>>>(m.gen_descs, m.gen_block_map, 0, 0, m.pair_seeds, m.cfg.use_clt, m.cfg.clt_k);
+        launch_pdl_if(pairs * static_cast<long long>(m.gen_blocks_factors) <= 8192, gen_noise_kernel, dim3(m.gen_blocks_factors, pairs), 256, 0, S(stream), m.gen_descs, m.gen_block_map, 0, 0, m.pair_seeds, m.cfg.use_clt, m.cfg.clt_k);
         TRY(check_launch("gen_noise_kernel"));
     }
     // ... and the per-pair vectors only for the pairs this process evaluates
     if (eval_count > 0) {
-        gen_noise_kernel<<<dim3(m.gen_blocks - m.gen_blocks_factors, eval_count), 256, 0, S(stream)>>>(m.gen_descs, m.gen_block_map, m.gen_blocks_factors,
+        launch_pdl_if(eval_count * static_cast<long long>(m.gen_blocks - m.gen_blocks_factors) <= 8192, gen_noise_kernel, dim3(m.gen_blocks - m.gen_blocks_factors, eval_count), 256, 0, S(stream), m.gen_descs, m.gen_block_map, m.gen_blocks_factors,
                                                                                                         eval_begin, m.pair_seeds, m.cfg.use_clt, m.cfg.clt_k);
         TRY(check_launch("gen_noise_kernel"));
     }

@@ -12,6 +12,8 @@ namespace {
 
 __global__ void quant_direct_f32_kernel(const float* __restrict__ in, int rows, int k_in, int k_out, long long ld_in,
                                         uint8_t* __restrict__ codes, uint8_t* __restrict__ sf, int k_atoms) {
+    pdl_wait();
+    after(in);
     const int blocks_per_row = k_out >> 4;
     const long long gid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (gid >= static_cast<long long>(rows) * blocks_per_row) return;
@@ -58,7 +60,7 @@ extern "C" int bnf4_nvfp4_quantize_f32(const float* in, int rows, int k_in, int 
     if (reinterpret_cast<uintptr_t>(out) & 7) return set_error(BNF4_ERR_INVALID, "nvfp4_quantize_f32: codes must be 8-byte aligned");
     const long long blocks = static_cast<long long>(rows) * (k_out / 16);
     const int threads = 128;
-    quant_direct_f32_kernel<<<static_cast<unsigned>((blocks + threads - 1) / threads), threads, 0, static_cast<cudaStream_t>(stream)>>>(
+    launch_pdl(quant_direct_f32_kernel, static_cast<unsigned>((blocks + threads - 1) / threads), threads, 0, static_cast<cudaStream_t>(stream), 
         in, rows, k_in, k_out, k_in, static_cast<uint8_t*>(out), static_cast<uint8_t*>(sf), sf_k_atoms(k_out));
     return check_launch("quant_direct_f32_kernel");
 }

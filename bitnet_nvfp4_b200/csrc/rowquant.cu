@@ -19,6 +19,7 @@
 //   residual add + norm        src/cuda_kernels.cu:3033-3143
 
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -32,9 +33,11 @@ constexpr int kMaxBlocksPerLaneInt8 = 16;  // ... and 8192 for plain int8 rows (
 
 template <int FE, int NB>
 __global__ void __launch_bounds__(256) rowquant_kernel(const RowQuantParams p, const uint8_t* __restrict__ lut) {
+    pdl_trigger();
     const int warps_per_cta = blockDim.x >> 5;
     const int lane = threadIdx.x & 31;
-    const long long row = static_cast<long long>(blockIdx.x) * warps_per_cta + (threadIdx.x >> 5);
+    pdl_wait();
+    const long long row = static_cast<long long>(blockIdx.x + opaque_zero()) * warps_per_cta + (threadIdx.x >> 5);
     if (row >= p.rows) return;
 
     const int nblk = p.cols_out >> 4;
@@ -294,9 +297,11 @@ __device__ __forceinline__ uint2 lds_u64(uint32_t saddr) {
 // exactly NV projections; no int8 copy; the residual branch as halves), which carries none of the corresponding tests.
 template <int FE, int NB, int NV, bool MODEL = false>
 __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowquant_fast_kernel(const RowQuantParams p, const uint8_t* __restrict__ lut) {
+    pdl_trigger();
     __shared__ __align__(16) uint2 tab_s[128];  // per amax: {bits of fl(1 / scale), scale byte}
     if (threadIdx.x < 128) tab_s[threadIdx.x] = __ldg(reinterpret_cast<const uint2*>(lut + kQuantBlockTabOffset) + threadIdx.x);
     __syncthreads();
+    pdl_wait();  // the table is constant; the rows are the predecessor's
     // entry address from the bit pattern of (amax + kRoundBias): (bits - kRoundBiasBits) * 8, folded into one constant
     const uint32_t tab_c = static_cast<uint32_t>(__cvta_generic_to_shared(tab_s)) - (static_cast<uint32_t>(kRoundBiasBits) << 3);
     const float M = kRoundBias;
@@ -312,7 +317,7 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
     const bool pos_mod_pow2 = MODEL || (p.pos_mod > 0 && (p.pos_mod & (p.pos_mod - 1)) == 0);
     const int rpm_shift = (p.rows_per_member > 0 && (p.rows_per_member & (p.rows_per_member - 1)) == 0) ? __ffs(p.rows_per_member) - 1 : -1;
     const float inv_cols = 1.0f / static_cast<float>(p.cols_in);
-    for (unsigned row = blockIdx.x * 8u + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8u) {
+    for (unsigned row = (blockIdx.x + opaque_zero()) * 8u + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8u) {
         // rows per member is a power of two in every model configuration: a shift instead of a division per row
         const int member = (MODEL || p.rows_per_member > 0) ? static_cast<int>((MODEL || rpm_shift >= 0) ? row >> rpm_shift : row / static_cast<unsigned>(p.rows_per_member)) : 0;
         const int row_in_member = (MODEL || p.rows_per_member > 0) ? static_cast<int>(row - static_cast<unsigned>(member) * static_cast<unsigned>(p.rows_per_member)) : static_cast<int>(row);
@@ -633,6 +638,10 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
     }
 }
 
+// CTAs of a fast-kernel instance that fit one SM, per device (0 = not looked up yet)
+template <int FE, int NB, int NV, bool MODEL = false>
+std::atomic<int> resident_ctas[64] = {};
+
 template <int FE>
 int launch(const RowQuantParams& p, cudaStream_t stream) {
     if (p.rows <= 0 || p.cols_out <= 0) return BNF4_OK;
@@ -648,6 +657,7 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
     const int nblk = p.cols_out >> 4;
     const uint8_t* lut = get_quant_lut();
     if (lut == nullptr) return BNF4_ERR_CUDA;
+    const bool early = static_cast<long long>(p.rows) * p.cols_out <= kPdlStreamElems;
     if constexpr (FE == FE_EMBED_LOWRANK || FE == FE_POS_GELU_ABSMEAN || FE == FE_ADD_ABSMEAN || FE == FE_ABSMEAN) {
         auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
         bool fast = p.cols_in == p.cols_out && nblk <= 128 && (p.out_q == nullptr || p.vec_ok_q) && al16(p.inout_i8 ? p.inout_i8 : nullptr);
@@ -659,17 +669,22 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
         if (FE == FE_EMBED_LOWRANK)
             fast = fast && al16(p.emb_w) && p.rank >= 0 && p.rank <= 4 && (p.sigma == 0.0f || (al16(p.embB) && (p.embB_pair_stride % 16) == 0));
         if (fast) {
-            int dev = 0, sms = 0;
-            int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
-            if (!rc) rc = check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+            int dev = 0;
+            int rc = current_device(&dev);
             if (rc) return rc;
+            const int sms = multiprocessors(dev);
+            if (sms <= 0) return BNF4_ERR_CUDA;
             // persistent CTAs: exactly as many as are resident at once (each loads its 1 KB copy of the table once)
-            auto run = [&](auto kernel) -> int {
-                int per_sm = 0;
-                int rc2 = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, 0), "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-                if (rc2) return rc2;
-                const unsigned grid = std::min(ctas, static_cast<unsigned>(sms) * static_cast<unsigned>(std::max(per_sm, 1)));
-                kernel<<<grid, warps * 32, 0, stream>>>(p, lut);
+            auto run = [&](auto kernel, std::atomic<int>* resident) -> int {
+                int per_sm = resident[dev].load(std::memory_order_relaxed);
+                if (per_sm == 0) {  // looked up once per kernel and device
+                    const int rc2 = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, 0), "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+                    if (rc2) return rc2;
+                    per_sm = std::max(per_sm, 1);
+                    resident[dev].store(per_sm, std::memory_order_relaxed);
+                }
+                const unsigned grid = std::min(ctas, static_cast<unsigned>(sms) * static_cast<unsigned>(per_sm));
+                launch_pdl_if(early, kernel, grid, warps * 32, 0, stream, p, lut);
                 return BNF4_OK;
             };
             // the batched driver's calls at hidden <= 512: see MODEL above
@@ -680,30 +695,30 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
             if (FE == FE_POS_GELU_ABSMEAN) model = model && pow2(p.pos_mod) && (p.gather_rows <= 0 || pow2(p.row_mod));
             if constexpr (FE == FE_ADD_ABSMEAN || FE == FE_ABSMEAN || FE == FE_POS_GELU_ABSMEAN) {
                 if (model) {
-                    rc = p.nvec == 1 ? run(rowquant_fast_kernel<FE, 1, 1, true>) : run(rowquant_fast_kernel<FE, 1, 4, true>);
+                    rc = p.nvec == 1 ? run(rowquant_fast_kernel<FE, 1, 1, true>, resident_ctas<FE, 1, 1, true>) : run(rowquant_fast_kernel<FE, 1, 4, true>, resident_ctas<FE, 1, 4, true>);
                     if (rc) return rc;
                     return check_launch("rowquant_fast_kernel");
                 }
             }
             if (p.nvec <= 4) {
-                if (nblk <= 32) rc = run(rowquant_fast_kernel<FE, 1, 4>);
-                else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, 4>);
-                else rc = run(rowquant_fast_kernel<FE, 4, 4>);
+                if (nblk <= 32) rc = run(rowquant_fast_kernel<FE, 1, 4>, resident_ctas<FE, 1, 4>);
+                else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, 4>, resident_ctas<FE, 2, 4>);
+                else rc = run(rowquant_fast_kernel<FE, 4, 4>, resident_ctas<FE, 4, 4>);
             } else {
-                if (nblk <= 32) rc = run(rowquant_fast_kernel<FE, 1, kMaxTVec>);
-                else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, kMaxTVec>);
-                else rc = run(rowquant_fast_kernel<FE, 4, kMaxTVec>);
+                if (nblk <= 32) rc = run(rowquant_fast_kernel<FE, 1, kMaxTVec>, resident_ctas<FE, 1, kMaxTVec>);
+                else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, kMaxTVec>, resident_ctas<FE, 2, kMaxTVec>);
+                else rc = run(rowquant_fast_kernel<FE, 4, kMaxTVec>, resident_ctas<FE, 4, kMaxTVec>);
             }
             if (rc) return rc;
             return check_launch("rowquant_fast_kernel");
         }
     }
-    if (nblk <= 32) rowquant_kernel<FE, 1><<<ctas, warps * 32, 0, stream>>>(p, lut);
-    else if (nblk <= 64) rowquant_kernel<FE, 2><<<ctas, warps * 32, 0, stream>>>(p, lut);
-    else if (nblk <= 128) rowquant_kernel<FE, 4><<<ctas, warps * 32, 0, stream>>>(p, lut);
-    else if (nblk <= 256) rowquant_kernel<FE, 8><<<ctas, warps * 32, 0, stream>>>(p, lut);
+    if (nblk <= 32) launch_pdl_if(early, rowquant_kernel<FE, 1>, ctas, warps * 32, 0, stream, p, lut);
+    else if (nblk <= 64) launch_pdl_if(early, rowquant_kernel<FE, 2>, ctas, warps * 32, 0, stream, p, lut);
+    else if (nblk <= 128) launch_pdl_if(early, rowquant_kernel<FE, 4>, ctas, warps * 32, 0, stream, p, lut);
+    else if (nblk <= 256) launch_pdl_if(early, rowquant_kernel<FE, 8>, ctas, warps * 32, 0, stream, p, lut);
     else {
-        if constexpr (FE == FE_INT8) rowquant_kernel<FE, 16><<<ctas, warps * 32, 0, stream>>>(p, lut);
+        if constexpr (FE == FE_INT8) launch_pdl_if(early, rowquant_kernel<FE, 16>, ctas, warps * 32, 0, stream, p, lut);
     }
     return check_launch("rowquant_kernel");
 }

@@ -24,8 +24,7 @@ def c_rank(rank: int) -> float:
     return 0.0 if rank <= 0 else float(np.float32(C_RANK_BASE) / np.sqrt(np.float32(rank)))
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+_stream = _l.stream
 
 
 def _p(t):
@@ -33,17 +32,21 @@ def _p(t):
 
 
 def sf_bytes(rows: int, k: int) -> int:
-    return _l.load().bnf4_nvfp4_sfa_bytes(rows, 1, k)
+    """bnf4_nvfp4_sfa_bytes: whole atoms of 128 rows x 64 elements, one byte per 16 elements."""
+    return -(-rows // 128) * 128 * (-(-(-(-k // 16)) // 4) * 4)
 
 
 def matrix_bytes(rows: int, cols: int) -> int:
-    return _l.load().bnf4_nvfp4_matrix_bytes(rows, cols)
+    """bnf4_nvfp4_matrix_bytes: two elements per byte."""
+    return (rows * cols * 4 + 7) // 8
 
 
 def _alloc_q(rows: int, cols: int, device, want_q=True):
-    q = torch.zeros((rows, cols), dtype=torch.int8, device=device) if want_q else None
-    codes = torch.zeros(matrix_bytes(rows, cols), dtype=torch.uint8, device=device)
-    sf = torch.zeros(sf_bytes(rows, cols), dtype=torch.uint8, device=device)
+    """Outputs of a quantiser. It writes every int8 value and code and the scale byte of every block; only the padding of a
+    ragged scale array (rows to 128, columns to 64) has to be cleared."""
+    q = torch.empty((rows, cols), dtype=torch.int8, device=device) if want_q else None
+    codes = torch.empty(matrix_bytes(rows, cols), dtype=torch.uint8, device=device)
+    sf = (torch.zeros if rows % 128 or cols % 64 else torch.empty)(sf_bytes(rows, cols), dtype=torch.uint8, device=device)
     return q, codes, sf
 
 

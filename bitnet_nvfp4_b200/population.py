@@ -120,8 +120,7 @@ class Config:
                 "ff1": (L, F, H), "ff2": (L, H, F), "head": (V, H), "head_bias": (V,), "beta_bias": (L,), "pos": (T, H)}
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+_stream = _l.stream
 
 
 class PopulationModel:
