@@ -11,6 +11,7 @@
 // (the reference uses unordered float atomics).
 
 #include <algorithm>
+#include <cstring>
 #include <mutex>
 
 #include "common.cuh"
@@ -211,7 +212,7 @@ __global__ void ce_finalize_kernel(const float* __restrict__ partial, int member
 __global__ void fill_noise_kernel(int8_t* __restrict__ out, size_t n, uint64_t seed, int use_clt, int clt_k) {
     pdl_wait();
     const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx < n) out[idx] = static_cast<int8_t>(noise_hash(seed, idx, use_clt != 0, clt_k));
+    if (idx < n) out[idx] = static_cast<int8_t>(use_clt != 0 && clt_k == 4 ? noise_clt4(noise_seed(seed), idx) : noise_hash(seed, idx, use_clt != 0, clt_k));
 }
 __global__ void fill_noise_batched_kernel(const bnf4_noise_desc* __restrict__ descs, int num_desc, int use_clt, int clt_k) {
     pdl_wait();
@@ -220,7 +221,8 @@ __global__ void fill_noise_batched_kernel(const bnf4_noise_desc* __restrict__ de
     if (di >= num_desc) return;
     const bnf4_noise_desc d = descs[di];
     const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx < d.n) d.out[idx] = static_cast<int8_t>(noise_hash(d.seed, idx, use_clt != 0, clt_k));
+    if (idx < d.n)
+        d.out[idx] = static_cast<int8_t>(use_clt != 0 && clt_k == 4 ? noise_clt4(noise_seed(d.seed), idx) : noise_hash(d.seed, idx, use_clt != 0, clt_k));
 }
 __global__ void fill_float_noise_kernel(float* __restrict__ out, int n, uint64_t seed, int use_clt, int clt_k) {
     pdl_wait();
@@ -245,31 +247,32 @@ __global__ void init_shadow_kernel(const int8_t* __restrict__ w, float* __restri
 
 // Z for the dense (full-matrix noise) form; 256 threads per block, one element each.
 // Elements idx0 .. idx0 + n - 1 of the vector (the hash is keyed by the element's index in the whole vector) go to Z[0 .. n).
-__global__ void __launch_bounds__(256) z_dense_kernel(const float* __restrict__ pair_weights, const uint64_t* __restrict__ pair_seeds,
-                                                      uint64_t salt, int pairs, int idx0, int n, int use_clt, int clt_k, float* __restrict__ Z) {
-    pdl_wait();
-    after(pair_weights, pair_seeds);
-    extern __shared__ uint8_t zsm[];
-    uint64_t* seeds = reinterpret_cast<uint64_t*>(zsm);
-    float* wts = reinterpret_cast<float*>(zsm + sizeof(uint64_t) * 256);
-    const int idx = blockIdx.x * 256 + threadIdx.x;
+// CLT4: the noise every model uses (sum of four ternary draws).
+template <bool CLT4>
+__device__ __forceinline__ void z_dense_block(const float* pair_weights, const uint64_t* pair_seeds, uint64_t salt, int pairs, int idx, bool active,
+                                              int use_clt, int clt_k, float* out) {
+    __shared__ NoiseSeed seeds[256];
+    __shared__ float wts[256];
     float z = 0.0f;
     for (int p0 = 0; p0 < pairs; p0 += 256) {
         __syncthreads();
         if (p0 + threadIdx.x < pairs) {
-            seeds[threadIdx.x] = mix_u64(pair_seeds[p0 + threadIdx.x], salt);
+            seeds[threadIdx.x] = noise_seed(mix_u64(pair_seeds[p0 + threadIdx.x], salt));
             wts[threadIdx.x] = pair_weights[p0 + threadIdx.x];
         }
         __syncthreads();
         const int cnt = min(256, pairs - p0);
-        if (idx < n) {
-            // four independent hash chains in flight; the multiply-adds stay in pair order (pairs of weight zero are skipped,
-            // like in the reference)
+        if (active) {
+            // independent hash chains in flight; the multiply-adds stay in pair order (pairs of weight zero are skipped, like in the
+            // reference)
+            auto noise = [&](int p) {
+                return static_cast<float>(CLT4 ? noise_clt4(seeds[p], static_cast<uint64_t>(idx)) : noise_hash(seeds[p].a, static_cast<uint64_t>(idx), use_clt != 0, clt_k));
+            };
             int p = 0;
             for (; p + 4 <= cnt; p += 4) {
                 float e[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) e[q] = static_cast<float>(noise_hash(seeds[p + q], static_cast<uint64_t>(idx0 + idx), use_clt != 0, clt_k));
+                for (int q = 0; q < 4; ++q) e[q] = noise(p + q);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float w = wts[p + q];
@@ -278,12 +281,62 @@ __global__ void __launch_bounds__(256) z_dense_kernel(const float* __restrict__ 
             }
             for (; p < cnt; ++p) {
                 const float w = wts[p];
-                if (w == 0.0f) continue;
-                z = fmaf(w, static_cast<float>(noise_hash(seeds[p], static_cast<uint64_t>(idx0 + idx), use_clt != 0, clt_k)), z);
+                if (w != 0.0f) z = fmaf(w, noise(p), z);
             }
         }
     }
-    if (idx < n) Z[idx] = z;
+    if (active) *out = z;
+}
+template <bool CLT4>
+__global__ void __launch_bounds__(256) z_dense_kernel(const float* __restrict__ pair_weights, const uint64_t* __restrict__ pair_seeds,
+                                                      uint64_t salt, int pairs, int idx0, int n, int use_clt, int clt_k, float* __restrict__ Z) {
+    pdl_wait();
+    after(pair_weights, pair_seeds);
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    z_dense_block<CLT4>(pair_weights, pair_seeds, salt, pairs, idx0 + i, i < n, use_clt, clt_k, Z + i);
+}
+// The same for a table of tensors (the fp32 vectors of a model; in the dense mode also its matrices) in one launch: block b finds
+// its tensor by walking the table. With nshards > 1 a tensor that is computed in shards covers this shard's elements only.
+template <bool CLT4>
+__global__ void __launch_bounds__(256) z_dense_table_kernel(const float* __restrict__ pair_weights, const uint64_t* __restrict__ pair_seeds,
+                                                            const ZDenseDesc* __restrict__ descs, int ndesc, int pairs, int use_clt, int clt_k,
+                                                            int use_noise_tables, int shard, int nshards, float* __restrict__ z_all) {
+    pdl_wait();
+    after(pair_weights, pair_seeds);
+    int block = static_cast<int>(blockIdx.x), idx0 = 0, n = 0;
+    ZDenseDesc d = {};
+    for (int t = 0; t < ndesc; ++t) {
+        d = descs[t];
+        z_dense_range(d, shard, nshards, idx0, n);
+        const int blocks = (n + 255) / 256;
+        if (block < blocks) break;
+        block -= blocks;
+    }
+    const int i = block * 256 + threadIdx.x;
+    float* out = z_all + d.zoff + idx0 + i;
+    if (use_noise_tables && d.noise != nullptr) {  // one byte per pair instead of one hash; same values, same order
+        if (i >= n) return;
+        const int8_t* src = d.noise + idx0 + i;
+        float z = 0.0f;
+        int p = 0;
+        for (; p + 16 <= pairs; p += 16) {
+            int8_t e[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) e[q] = src[static_cast<size_t>(p + q) * d.n];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const float w = pair_weights[p + q];
+                if (w != 0.0f) z = fmaf(w, static_cast<float>(e[q]), z);
+            }
+        }
+        for (; p < pairs; ++p) {
+            const float w = pair_weights[p];
+            if (w != 0.0f) z = fmaf(w, static_cast<float>(src[static_cast<size_t>(p) * d.n]), z);
+        }
+        *out = z;
+        return;
+    }
+    z_dense_block<CLT4>(pair_weights, pair_seeds, d.salt, pairs, idx0 + i, i < n, use_clt, clt_k, out);
 }
 
 // Rank-r form of Z: Z[i][j] = cscale * sum_p w_p * (sum_r A[p][i][r] * B[p][r][j]), pairs in ascending order with one fused
@@ -435,38 +488,53 @@ __global__ void __launch_bounds__(kZThreads) z_lowrank_tiles_kernel(const float*
     }
 }
 
-// Sum of squares, stage 1: block b reduces Z[256b .. 256b+255] with the reference's shared-memory tree.
+// Sum of squares, stage 1: the squares of 256 consecutive elements are added in the order of the reference's shared-memory tree
+// (strides 128, 64, .. 1). One warp per 256 elements: lane l holds elements l, l + 32, .. so that the strides down to 32 are
+// register additions and the rest shuffles; no barriers, eight loads in flight per lane.
+__device__ __forceinline__ float sumsq_256(const float* Z, int first, int n) {
+    const int lane = threadIdx.x & 31;
+    float e[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int i = first + lane + 32 * j;
+        const float z = i < n ? Z[i] : 0.0f;
+        e[j] = __fmul_rn(z, z);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) e[j] += e[j + 4];
+    e[0] += e[2];
+    e[1] += e[3];
+    e[0] += e[1];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e[0] += __shfl_down_sync(0xffffffffu, e[0], o);
+    return e[0];  // lane 0
+}
 __global__ void __launch_bounds__(256) sumsq_blocks_kernel(const float* __restrict__ Z, int n, float* __restrict__ partial) {
     pdl_wait();
     after(Z);
-    __shared__ float sh[256];
-    const int idx = blockIdx.x * 256 + threadIdx.x;
-    const float z = idx < n ? Z[idx] : 0.0f;
-    sh[threadIdx.x] = __fmul_rn(z, z);
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
+    const int block = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (block * 256ll >= n) return;
+    const float t = sumsq_256(Z, block * 256, n);
+    if ((threadIdx.x & 31) == 0) partial[block] = t;
 }
-// stage 2: one warp adds the block partials in double (lane-contiguous ranges, then lanes in order) and
-// accumulates into *sumsq.
-__global__ void sumsq_final_kernel(const float* __restrict__ partial, int nblocks, float* sumsq) {
+// stage 2: the block partials in double, in a fixed order (256 strided chains, then a tree). Result in thread 0.
+__device__ __forceinline__ double sumsq_total(const float* partial, int nblocks) {
+    __shared__ double warp_sum[8];
+    double t = 0.0;
+    for (int b = threadIdx.x; b < nblocks; b += 256) t += static_cast<double>(partial[b]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < 8; ++w) t += warp_sum[w];
+    return t;
+}
+__global__ void __launch_bounds__(256) sumsq_final_kernel(const float* __restrict__ partial, int nblocks, float* sumsq) {
     pdl_wait();
     after(partial);
-    __shared__ double lane_sum[32];
-    const int lane = threadIdx.x;
-    const int per = (nblocks + 31) / 32;
-    double t = 0.0;
-    for (int b = lane * per; b < min(nblocks, (lane + 1) * per); ++b) t += static_cast<double>(partial[b]);
-    lane_sum[lane] = t;
-    __syncwarp();
-    if (lane == 0) {
-        double tot = 0.0;
-        for (int l = 0; l < 32; ++l) tot += lane_sum[l];
-        sumsq[0] += static_cast<float>(tot);
-    }
+    const double tot = sumsq_total(partial, nblocks);
+    if (threadIdx.x == 0) sumsq[0] += static_cast<float>(tot);
 }
 
 __global__ void inv_rms_kernel(const float* __restrict__ sumsq, float* __restrict__ rms_ema, int use_adaptive, float beta, float eps,
@@ -518,81 +586,173 @@ __global__ void add_scaled_kernel(float* __restrict__ out, const float* __restri
     if (i < n) out[i] = fmaf(scale, noise[i], out[i]);
 }
 
-// ---- the apply phase of the ES update for a table of tensors: four launches instead of five per tensor -------------------
-// Same arithmetic, block structure and summation order as sumsq_blocks / sumsq_final / inv_rms / update_shadow /
-// update_vector above, so the bits are those of the per-tensor calls. Block b of the grid belongs to the tensor whose
-// [block0, block0 + ceil(n / 256)) contains it.
+// Fitness shaping on the device, bit for bit the host function bnf4_shape_pair_weights (api.cu): f_p = -(loss+ - loss-), then sign,
+// z-score or centered rank followed by the z-score with clipping. Ranks come from counting (ties by index, as the stable sort
+// orders them); mean and variance are sums in index order, one thread each way, because that is the order the host adds in (1024
+// pairs: about 5 us, against a stream synchronisation, two copies and an idle GPU between evaluation and update).
+constexpr int kShapeMaxPairs = 4096;
+__global__ void __launch_bounds__(1024) shape_fitness_kernel(const float* __restrict__ losses, int n, int mode, float clip, float* __restrict__ out) {
+    pdl_wait();
+    after(losses);
+    __shared__ float f[kShapeMaxPairs], r[kShapeMaxPairs];
+    __shared__ float mean_s, std_s;
+    for (int i = threadIdx.x; i < n; i += 1024) f[i] = -__fsub_rn(losses[2 * i], losses[2 * i + 1]);
+    __syncthreads();
+    if (mode == BNF4_FITNESS_SIGN) {
+        for (int i = threadIdx.x; i < n; i += 1024) out[i] = f[i] > 0.0f ? 1.0f : (f[i] < 0.0f ? -1.0f : 0.0f);
+        return;
+    }
+    for (int i = threadIdx.x; i < n; i += 1024) {
+        float v = f[i];
+        if (mode == BNF4_FITNESS_CENTERED_RANK) {
+            int rank = 0;
+            for (int j = 0; j < n; ++j) rank += (f[j] < v || (j < i && !(v < f[j]))) ? 1 : 0;
+            v = n == 1 ? 0.0f : __fsub_rn(__fdiv_rn(static_cast<float>(rank), static_cast<float>(n - 1)), 0.5f);
+        }
+        r[i] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float mean = 0.0f;
+#pragma unroll 16
+        for (int i = 0; i < n; ++i) mean = __fadd_rn(mean, r[i]);
+        mean = __fdiv_rn(mean, static_cast<float>(n));
+        mean_s = mean;
+    }
+    __syncthreads();
+    const float mean = mean_s;
+    for (int i = threadIdx.x; i < n; i += 1024) {
+        const float d = __fsub_rn(r[i], mean);
+        r[i] = d;
+        f[i] = __fmul_rn(d, d);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float var = 0.0f;
+#pragma unroll 16
+        for (int i = 0; i < n; ++i) var = __fadd_rn(var, f[i]);
+        std_s = __fadd_rn(__fsqrt_rn(__fdiv_rn(var, static_cast<float>(n))), 1e-6f);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += 1024) {
+        float d = __fdiv_rn(r[i], std_s);
+        if (d > clip) d = clip;
+        if (d < -clip) d = -clip;
+        out[i] = d;
+    }
+}
+
+// ---- the apply phase of the ES update for a table of tensors: three launches for all of them ----------------------------------
+// Same arithmetic and summation order as sumsq_blocks / sumsq_final / inv_rms / update_shadow / update_vector above, so the bits are
+// those of the per-tensor calls. The tensor of a block is found by binary search over the running block counts.
+template <bool UPDATE_BLOCKS>
 __device__ __forceinline__ int find_tensor(const UpdApplyDesc* __restrict__ d, int ndesc, int block) {
     int lo = 0, hi = ndesc - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (d[mid].block0 <= block) lo = mid; else hi = mid - 1;
+        if ((UPDATE_BLOCKS ? d[mid].ublock0 : d[mid].block0) <= block) lo = mid; else hi = mid - 1;
     }
     return lo;
 }
-__global__ void __launch_bounds__(256) sumsq_blocks_batched_kernel(const UpdApplyDesc* __restrict__ d, int ndesc, float* __restrict__ partial) {
+__global__ void __launch_bounds__(256) sumsq_blocks_batched_kernel(const UpdApplyDesc* __restrict__ d, int ndesc, int total_blocks,
+                                                                   const float* __restrict__ z_all, float* __restrict__ partial) {
     pdl_wait();
-    __shared__ float sh[256];
-    __shared__ int ti;
-    if (threadIdx.x == 0) ti = find_tensor(d, ndesc, static_cast<int>(blockIdx.x));
-    __syncthreads();
-    const UpdApplyDesc& x = d[ti];
-    const int idx = (static_cast<int>(blockIdx.x) - x.block0) * 256 + threadIdx.x;
-    const float z = idx < x.n ? x.Z[idx] : 0.0f;
-    sh[threadIdx.x] = __fmul_rn(z, z);
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) partial[blockIdx.x] = sh[0];
+    after(z_all);
+    const int block = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (block >= total_blocks) return;
+    const UpdApplyDesc& x = d[find_tensor<false>(d, ndesc, block)];
+    const float t = sumsq_256(z_all + x.zoff, (block - x.block0) * 256, x.n);
+    if ((threadIdx.x & 31) == 0) partial[block] = t;
 }
-// one warp per tensor; then its lane 0 turns the sum into inv_rms (and advances the tensor's RMS-EMA)
-__global__ void sumsq_final_inv_rms_batched_kernel(const UpdApplyDesc* __restrict__ d, const float* __restrict__ partial, int use_adaptive,
-                                                   float beta, float eps, float* __restrict__ inv_rms_out) {
+// one CTA per tensor; its thread 0 turns the sum into inv_rms (and advances the tensor's RMS-EMA)
+__global__ void __launch_bounds__(256) sumsq_final_inv_rms_batched_kernel(const UpdApplyDesc* __restrict__ d, const float* __restrict__ partial, int use_adaptive,
+                                                                          float beta, float eps, float* __restrict__ inv_rms_out) {
     pdl_wait();
     after(partial);
-    __shared__ double lane_sum[32];
     const UpdApplyDesc& x = d[blockIdx.x];
-    const int lane = threadIdx.x;
-    const int nblocks = (x.n + 255) / 256;
-    const float* part = partial + x.block0;
-    const int per = (nblocks + 31) / 32;
-    double t = 0.0;
-    for (int b = lane * per; b < min(nblocks, (lane + 1) * per); ++b) t += static_cast<double>(part[b]);
-    lane_sum[lane] = t;
-    __syncwarp();
-    if (lane == 0) {
-        double tot = 0.0;
-        for (int l = 0; l < 32; ++l) tot += lane_sum[l];
-        const float sumsq = static_cast<float>(tot);
-        float inv = 1.0f;
-        if (use_adaptive) {
-            const float ms = __fdiv_rn(sumsq, static_cast<float>(x.n));
-            float ema = x.ema[0];
-            if (ema == 0.0f) ema = ms;
-            ema = fmaf(beta, ema, __fmul_rn(1.0f - beta, ms));
-            x.ema[0] = ema;
-            inv = __fdiv_rn(1.0f, __fsqrt_rn(ema + eps));
-        }
-        inv_rms_out[blockIdx.x] = inv;
+    const double tot = sumsq_total(partial + x.block0, (x.n + 255) / 256);
+    if (threadIdx.x != 0) return;
+    float inv = 1.0f;
+    if (use_adaptive) {
+        const float ms = __fdiv_rn(static_cast<float>(tot), static_cast<float>(x.n));
+        float ema = x.ema[0];
+        if (ema == 0.0f) ema = ms;
+        ema = fmaf(beta, ema, __fmul_rn(1.0f - beta, ms));
+        x.ema[0] = ema;
+        inv = __fdiv_rn(1.0f, __fsqrt_rn(ema + eps));
     }
+    inv_rms_out[blockIdx.x] = inv;
 }
-__global__ void __launch_bounds__(256) update_batched_kernel(const UpdApplyDesc* __restrict__ d, int ndesc, const float* __restrict__ inv_rms,
-                                                             float lr, float thresh) {
+// Gated update of four consecutive elements per thread (16-byte accesses, a warp covers 512 contiguous bytes of Z and shadow) and,
+// in the same pass, the NVFP4 copy of the new weights: the four threads of a 16-element scale block agree on its maximum with two
+// shuffles. Memory bound: 14 bytes per weight read and written plus 0.56 of NVFP4, against a second pass over the weights by one
+// quantiser launch per matrix. UPDATE false: the NVFP4 copies of the present weights only.
+template <bool UPDATE>
+__global__ void __launch_bounds__(256) update_batched_kernel(const UpdApplyDesc* __restrict__ d, int ndesc, const float* __restrict__ z_all,
+                                                             const float* __restrict__ inv_rms, float lr, float thresh, const uint2* __restrict__ tab) {
     pdl_wait();
-    after(inv_rms);
-    __shared__ int ti;
-    if (threadIdx.x == 0) ti = find_tensor(d, ndesc, static_cast<int>(blockIdx.x));
-    __syncthreads();
+    after(z_all, inv_rms);
+    const int ti = find_tensor<true>(d, ndesc, static_cast<int>(blockIdx.x));
     const UpdApplyDesc& x = d[ti];
-    const int i = (static_cast<int>(blockIdx.x) - x.block0) * 256 + threadIdx.x;
-    if (i >= x.n) return;
-    const float g = __fmul_rn(inv_rms[ti], x.Z[i]);
-    if (fabsf(g) < thresh) return;
-    const float s = fmaf(lr, g, x.target[i]);
-    x.target[i] = s;
-    if (x.w != nullptr) x.w[i] = static_cast<int8_t>(clip_ternary(__float2int_rn(s)));
+    const int i0 = (static_cast<int>(blockIdx.x) - x.ublock0) * 1024 + static_cast<int>(threadIdx.x) * 4;
+    const int n = x.n;
+    int8_t* w = x.w;
+    uint32_t wq = 0;  // the four weights as bytes
+    const bool whole = i0 + 4 <= n;
+    if constexpr (UPDATE) {
+        const float* Z = z_all + x.zoff;
+        float* target = x.target;
+        const float inv = inv_rms[ti];
+        if (whole && ((reinterpret_cast<uintptr_t>(Z) | reinterpret_cast<uintptr_t>(target)) & 15) == 0) {
+            const float4 z4 = *reinterpret_cast<const float4*>(Z + i0);
+            float4 s4 = *reinterpret_cast<const float4*>(target + i0);
+            uint32_t old = w != nullptr ? *reinterpret_cast<const uint32_t*>(w + i0) : 0u;
+            const float zz[4] = {z4.x, z4.y, z4.z, z4.w};
+            float ss[4] = {s4.x, s4.y, s4.z, s4.w};
+            bool any = false;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float g = __fmul_rn(inv, zz[e]);
+                if (!(fabsf(g) < thresh)) {
+                    any = true;
+                    ss[e] = fmaf(lr, g, ss[e]);
+                    old = (old & ~(0xffu << (8 * e))) | (static_cast<uint32_t>(clip_ternary(__float2int_rn(ss[e])) & 0xff) << (8 * e));
+                }
+            }
+            if (any) {
+                *reinterpret_cast<float4*>(target + i0) = make_float4(ss[0], ss[1], ss[2], ss[3]);
+                if (w != nullptr) *reinterpret_cast<uint32_t*>(w + i0) = old;
+            }
+            wq = old;
+        } else {
+            for (int i = i0; i < min(n, i0 + 4); ++i) {
+                const float g = __fmul_rn(inv, Z[i]);
+                if (!(fabsf(g) < thresh)) {
+                    const float s = fmaf(lr, g, target[i]);
+                    target[i] = s;
+                    if (w != nullptr) w[i] = static_cast<int8_t>(clip_ternary(__float2int_rn(s)));
+                }
+                if (w != nullptr) wq |= static_cast<uint32_t>(static_cast<uint8_t>(w[i])) << (8 * (i - i0));
+            }
+        }
+    } else {
+        if (w != nullptr && whole) wq = *reinterpret_cast<const uint32_t*>(w + i0);
+    }
+    if (x.codes == nullptr) return;  // (uniform in the CTA; matrices with a copy have n a multiple of 16)
+    float f[4];
+    bytes4_to_float(wq, f);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f[e] = fmaxf(f[e], -127.0f);  // -128 is treated as -127, as by the row quantisers
+    float am = fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3])));
+    am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
+    am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
+    if (i0 >= n) return;
+    const uint2 ent = __ldg(tab + x.scaled * 128 + static_cast<int>(am));
+    const float n8[8] = {f[0], f[1], f[2], f[3], 0.0f, 0.0f, 0.0f, 0.0f};
+    const uint32_t codes = e2m1x8_int(n8, __uint_as_float(ent.x));
+    const int row = i0 / x.cols, col = i0 - row * x.cols;
+    *reinterpret_cast<uint16_t*>(x.codes + (static_cast<size_t>(x.row0 + row) * x.cols + col) / 2) = static_cast<uint16_t>(codes);
+    if ((col & 15) == 0) x.sf[sf_offset(x.row0 + row, col >> 4, sf_k_atoms(x.cols))] = static_cast<uint8_t>(ent.y);
 }
 
 // library-owned scratch for the block partials of sum(Z^2), one per device
@@ -630,27 +790,75 @@ int get_scratch(size_t floats, float** out) {
 
 }  // namespace
 
-// Dense-noise Z of elements idx0 .. idx0 + n - 1 of a vector into Z[0 .. n).
-int z_dense_launch(const float* pair_weights, const uint64_t* pair_seeds, uint64_t salt, int pairs, int idx0, int n, int use_clt, int clt_k,
-                   float* Z, cudaStream_t st) {
-    if (n <= 0) return BNF4_OK;
-    launch_pdl_if(static_cast<long long>(n) * pairs <= (1ll << 22), z_dense_kernel, (n + 255) / 256, 256, 256 * (sizeof(uint64_t) + sizeof(float)), st, pair_weights, pair_seeds, salt, pairs, idx0, n, use_clt, clt_k, Z);
-    return check_launch("z_dense_kernel");
+bool shape_fitness_applies(int pairs, int mode) { return pairs <= kShapeMaxPairs && mode >= BNF4_FITNESS_SIGN && mode <= BNF4_FITNESS_CENTERED_RANK; }
+int shape_fitness_launch(const float* losses, int pairs, int mode, float clip, float* weights, cudaStream_t st) {
+    launch_pdl(shape_fitness_kernel, 1, 1024, 0, st, losses, pairs, mode, clip, weights);
+    return check_launch("shape_fitness_kernel");
 }
 
-// Apply phase for a table of tensors (block0 filled by the caller: running sum of ceil(n / 256)); partial holds one float
-// per block, inv_rms one per tensor.
-int update_apply_batched(const UpdApplyDesc* d_descs, int ndesc, int total_blocks, float* partial, float* inv_rms, int use_adaptive, float beta,
-                         float eps, float lr, float thresh, cudaStream_t st) {
+namespace {
+// 524288 elements x 1024 pairs: 2.87 ms with the generic hash (branches on the noise kind, a loop over the draws), 2.22 ms with the
+// specialised one; both are bound by the integer pipes.
+int z_dense_single(const float* pair_weights, const uint64_t* pair_seeds, uint64_t salt, int pairs, int n, int use_clt, int clt_k, float* Z, cudaStream_t st) {
+    const bool early = static_cast<long long>(n) * pairs <= (1ll << 22);
+    const dim3 grid((n + 255) / 256);
+    if (use_clt != 0 && clt_k == 4) launch_pdl_if(early, z_dense_kernel<true>, grid, 256, 0, st, pair_weights, pair_seeds, salt, pairs, 0, n, use_clt, clt_k, Z);
+    else launch_pdl_if(early, z_dense_kernel<false>, grid, 256, 0, st, pair_weights, pair_seeds, salt, pairs, 0, n, use_clt, clt_k, Z);
+    return check_launch("z_dense_kernel");
+}
+}  // namespace
+
+int z_dense_table_launch(const float* pair_weights, const uint64_t* pair_seeds, const ZDenseDesc* d_descs, const ZDenseDesc* h_descs, int ndesc, int pairs,
+                         int use_clt, int clt_k, int use_noise_tables, int shard, int nshards, float* z_all, cudaStream_t st) {
+    long long blocks = 0, elems = 0;
+    for (int i = 0; i < ndesc; ++i) {
+        int i0 = 0, cnt = 0;
+        z_dense_range(h_descs[i], shard, nshards, i0, cnt);
+        blocks += (cnt + 255) / 256;
+        elems += cnt;
+    }
+    if (blocks <= 0) return BNF4_OK;
+    const bool early = elems * pairs <= (1ll << 22);
+    const dim3 grid(static_cast<unsigned>(blocks));
+    if (use_clt != 0 && clt_k == 4)
+        launch_pdl_if(early, z_dense_table_kernel<true>, grid, 256, 0, st, pair_weights, pair_seeds, d_descs, ndesc, pairs, use_clt, clt_k, use_noise_tables, shard, nshards, z_all);
+    else
+        launch_pdl_if(early, z_dense_table_kernel<false>, grid, 256, 0, st, pair_weights, pair_seeds, d_descs, ndesc, pairs, use_clt, clt_k, use_noise_tables, shard, nshards, z_all);
+    return check_launch("z_dense_table_kernel");
+}
+
+void update_quant_table(float row_scale, uint2 (&tab)[256]) {
+    for (int scaled = 0; scaled < 2; ++scaled)
+        for (int amax = 0; amax < 128; ++amax) {  // the arithmetic of quant_block16, IEEE on host and device alike
+            float scale = amax > 0 ? static_cast<float>(amax) / 6.0f : 1.0f;
+            if (scaled) scale *= row_scale;
+            uint32_t sq = ue4m3_encode_host(scale);
+            float sf = ue4m3_decode(sq);
+            if (sf == 0.0f) { sq = 0x38u; sf = 1.0f; }
+            const float rcp = 1.0f / sf;
+            uint2 e;
+            memcpy(&e.x, &rcp, 4);
+            e.y = sq;
+            tab[scaled * 128 + amax] = e;
+        }
+}
+
+// Apply phase for a table of tensors; partial holds one float per 256-element block, inv_rms one per tensor.
+int update_apply_batched(const UpdApplyDesc* d_descs, int ndesc, int total_blocks, int total_ublocks, const float* z_all, const uint2* tab, float* partial,
+                         float* inv_rms, int use_adaptive, float beta, float eps, float lr, float thresh, cudaStream_t st) {
     if (ndesc <= 0 || total_blocks <= 0) return BNF4_OK;
     const bool early = total_blocks * 256ll <= kPdlStreamElems;
-    launch_pdl_if(early, sumsq_blocks_batched_kernel, total_blocks, 256, 0, st, d_descs, ndesc, partial);
+    launch_pdl_if(early, sumsq_blocks_batched_kernel, (total_blocks + 7) / 8, 256, 0, st, d_descs, ndesc, total_blocks, z_all, partial);
     int rc = check_launch("sumsq_blocks_batched_kernel");
     if (rc) return rc;
-    launch_pdl(sumsq_final_inv_rms_batched_kernel, ndesc, 32, 0, st, d_descs, partial, use_adaptive, beta, eps, inv_rms);
+    launch_pdl(sumsq_final_inv_rms_batched_kernel, ndesc, 256, 0, st, d_descs, partial, use_adaptive, beta, eps, inv_rms);
     rc = check_launch("sumsq_final_inv_rms_batched_kernel");
     if (rc) return rc;
-    launch_pdl_if(early, update_batched_kernel, total_blocks, 256, 0, st, d_descs, ndesc, inv_rms, lr, thresh);
+    launch_pdl_if(early, update_batched_kernel<true>, total_ublocks, 256, 0, st, d_descs, ndesc, z_all, inv_rms, lr, thresh, tab);
+    return check_launch("update_batched_kernel");
+}
+int requantize_batched(const UpdApplyDesc* d_descs, int ndesc, int total_ublocks, const uint2* tab, cudaStream_t st) {
+    launch_pdl(update_batched_kernel<false>, total_ublocks, 256, 0, st, d_descs, ndesc, nullptr, nullptr, 0.0f, 0.0f, tab);
     return check_launch("update_batched_kernel");
 }
 
@@ -687,10 +895,10 @@ int sumsq_into(const float* Z, int n, float* sumsq, cudaStream_t st) {
     float* partial = nullptr;
     int rc = get_scratch(static_cast<size_t>(nblocks), &partial);
     if (rc) return rc;
-    launch_pdl(sumsq_blocks_kernel, nblocks, 256, 0, st, Z, n, partial);
+    launch_pdl(sumsq_blocks_kernel, (nblocks + 7) / 8, 256, 0, st, Z, n, partial);
     rc = check_launch("sumsq_blocks_kernel");
     if (rc) return rc;
-    launch_pdl(sumsq_final_kernel, 1, 32, 0, st, partial, nblocks, sumsq);
+    launch_pdl(sumsq_final_kernel, 1, 256, 0, st, partial, nblocks, sumsq);
     return check_launch("sumsq_final_kernel");
 }
 
@@ -698,10 +906,10 @@ int sumsq_into(const float* Z, int n, float* sumsq, cudaStream_t st) {
 
 int sumsq_with_scratch(const float* Z, int n, float* partial, float* sumsq, cudaStream_t st) {
     const int nblocks = (n + 255) / 256;
-    launch_pdl(sumsq_blocks_kernel, nblocks, 256, 0, st, Z, n, partial);
+    launch_pdl(sumsq_blocks_kernel, (nblocks + 7) / 8, 256, 0, st, Z, n, partial);
     int rc = check_launch("sumsq_blocks_kernel");
     if (rc) return rc;
-    launch_pdl(sumsq_final_kernel, 1, 32, 0, st, partial, nblocks, sumsq);
+    launch_pdl(sumsq_final_kernel, 1, 256, 0, st, partial, nblocks, sumsq);
     return check_launch("sumsq_final_kernel");
 }
 
@@ -784,8 +992,7 @@ int bnf4_compute_z_sumsq(const float* pair_weights, const uint64_t* pair_seeds, 
                          int clt_k, float* Z, float* sumsq, void* stream) {
     if (n <= 0) return BNF4_OK;
     if (!pair_weights || !pair_seeds || !Z || !sumsq) return set_error(BNF4_ERR_INVALID, "compute_z_sumsq: null pointer");
-    launch_pdl_if(static_cast<long long>(n) * pairs <= (1ll << 22), z_dense_kernel, (n + 255) / 256, 256, 256 * (sizeof(uint64_t) + sizeof(float)), S(stream), pair_weights, pair_seeds, salt, pairs, 0, n, use_clt, clt_k, Z);
-    const int rc = check_launch("z_dense_kernel");
+    const int rc = z_dense_single(pair_weights, pair_seeds, salt, pairs, n, use_clt, clt_k, Z, S(stream));
     if (rc) return rc;
     return sumsq_into(Z, n, sumsq, S(stream));
 }
@@ -903,8 +1110,7 @@ extern "C" int bnf4_compute_z_sumsq_static(const float* pair_weights, const uint
     int rc = static_partials(&partial);
     if (rc) return rc;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
-    launch_pdl_if(static_cast<long long>(n) * pairs <= (1ll << 22), z_dense_kernel, (n + 255) / 256, 256, 256 * (sizeof(uint64_t) + sizeof(float)), st, pair_weights, pair_seeds, salt, pairs, 0, n, use_clt, clt_k, Z);
-    rc = check_launch("z_dense_kernel");
+    rc = z_dense_single(pair_weights, pair_seeds, salt, pairs, n, use_clt, clt_k, Z, st);
     if (rc) return rc;
     // Every partial the final kernel reads (indices 0 .. ceil(n/256)-1) is written by the block kernel of this same
     // call first, so stale contents left by an earlier call are never observed and nothing needs clearing.

@@ -27,7 +27,11 @@ enum RowFrontEnd : int {
 
 constexpr int kMaxTVec = 16;  // rank-r projections per row (4 stacked groups x rank 4)
 
-using RowQuantParams = bnf4_rowquant_desc;
+struct RowQuantParams : bnf4_rowquant_desc {
+    RowQuantParams(const bnf4_rowquant_desc& d) : bnf4_rowquant_desc(d) {}
+    int32_t* zero_t = nullptr;  // FE_ADD_ABSMEAN: clears [rows][zero_n] words, the projections the GEMM after next accumulates with atomics
+    int zero_n = 0;
+};
 int rowquant_dispatch(int front_end, RowQuantParams p, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------------------------
@@ -67,19 +71,49 @@ struct ZLowrankDesc {
 int z_lowrank_launch(const float* pair_weights, const ZLowrankDesc* d_descs, const ZLowrankDesc* h_descs, int ndesc, int pairs, int rank,
                      float cscale, int shard, int nshards, cudaStream_t stream);
 
-// Apply phase of the ES update over a table of tensors (es_kernels.cu).
+// Apply phase of the ES update over a table of tensors (es_kernels.cu). The table does not change during a model's life: Z is given by
+// an offset into the launch's Z buffer.
 struct UpdApplyDesc {
     int8_t* w;       // ternary weights (nullptr for an fp32 vector)
     float* target;   // fp32 shadow of a matrix, or the vector itself
-    const float* Z;  // noise sum
     float* ema;      // the tensor's RMS-EMA slot
+    uint8_t* codes;  // NVFP4 copy of the weights (nullptr: none), row `row0` of its operand onwards
+    uint8_t* sf;
+    long long zoff;  // floats
     int n;
-    int block0;      // first 256-element block of this tensor in the launch
+    int cols;        // of a matrix with an NVFP4 copy (a multiple of 16)
+    int row0;        // first row inside the stacked operand
+    int scaled;      // 1: the row scale of the stacked projection is folded into the scale bytes (second half of the quantiser table)
+    int block0;      // first 256-element block of this tensor in the sum-of-squares launch
+    int ublock0;     // first 1024-element block in the update launch
 };
-int update_apply_batched(const UpdApplyDesc* d_descs, int ndesc, int total_blocks, float* partial, float* inv_rms, int use_adaptive, float beta,
-                         float eps, float lr, float thresh, cudaStream_t stream);
-int z_dense_launch(const float* pair_weights, const uint64_t* pair_seeds, uint64_t salt, int pairs, int idx0, int n, int use_clt, int clt_k,
-                   float* Z, cudaStream_t stream);
+// tab: {1 / scale, scale byte} per block maximum, 128 entries unscaled and 128 with the row scale (update_quant_table).
+void update_quant_table(float row_scale, uint2 (&tab)[256]);
+int update_apply_batched(const UpdApplyDesc* d_descs, int ndesc, int total_blocks, int total_ublocks, const float* z_all, const uint2* tab, float* partial,
+                         float* inv_rms, int use_adaptive, float beta, float eps, float lr, float thresh, cudaStream_t stream);
+// The NVFP4 copies alone, from the present weights.
+int requantize_batched(const UpdApplyDesc* d_descs, int ndesc, int total_ublocks, const uint2* tab, cudaStream_t stream);
+
+// Dense-noise Z of a table of tensors in one launch. noise != nullptr: the table of the step's noise [pair][n] that prepare_step left in
+// memory for all pairs; otherwise the values are hashed.
+struct ZDenseDesc {
+    uint64_t salt;
+    const int8_t* noise;
+    long long zoff;
+    int n;
+    int rows;  // of a matrix: sharded by rows when they divide; 0 for a vector: sharded when it is long enough
+};
+__host__ __device__ inline void z_dense_range(const ZDenseDesc& d, int shard, int nshards, int& i0, int& cnt) {
+    const bool split = nshards > 1 && (d.rows > 0 ? d.rows >= nshards && d.rows % nshards == 0 : d.n >= 4096 && d.n % nshards == 0);
+    cnt = split ? d.n / nshards : d.n;
+    i0 = split ? shard * cnt : 0;
+}
+int z_dense_table_launch(const float* pair_weights, const uint64_t* pair_seeds, const ZDenseDesc* d_descs, const ZDenseDesc* h_descs, int ndesc, int pairs,
+                         int use_clt, int clt_k, int use_noise_tables, int shard, int nshards, float* z_all, cudaStream_t stream);
+
+// Fitness shaping of all pairs on the device, from the losses of their members (es_kernels.cu).
+bool shape_fitness_applies(int pairs, int mode);
+int shape_fitness_launch(const float* losses, int pairs, int mode, float clip, float* weights, cudaStream_t stream);
 
 void count_launch();
 

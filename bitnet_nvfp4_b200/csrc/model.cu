@@ -19,6 +19,7 @@ namespace bnf4 {
 
 namespace {
 
+constexpr size_t kWeightStageBytes = 2u << 20;  // largest weight set that get_weights stages in pinned memory
 constexpr float kCRankBase = 0.6123724356957945f;  // sqrt(3/8)
 
 // Kernel classes for the optional timing breakdown (bnf4_model_get_timing).
@@ -41,20 +42,22 @@ struct GenDesc {
     int transposed;   // store element (major, r) at r*n_major + major instead of major*rank + r
 };
 
-// block_map[b] = (descriptor << 20) | block within that descriptor: every launched block has work.
-__global__ void gen_noise_kernel(const GenDesc* __restrict__ descs, const uint32_t* __restrict__ block_map, int block0, int pair0,
-                                 const uint64_t* __restrict__ pair_seeds, int use_clt, int clt_k) {
-    pdl_wait();
-    after(pair_seeds);
+// block_map[b] = (descriptor << 20) | block within that descriptor: every launched block has work. The pair's seed is
+// mix(seed, mix(epoch, pair)); the first block of a pair also stores it for the update (seeds_out).
+__global__ void __launch_bounds__(256) gen_noise_kernel(const GenDesc* __restrict__ descs, const uint32_t* __restrict__ block_map, int block0, int pair0, uint64_t seed0,
+                                                        uint64_t epoch, int use_clt, int clt_k, uint64_t* __restrict__ seeds_out) {
     const uint32_t bm = block_map[block0 + blockIdx.x];
     const GenDesc d = descs[bm >> 20];
     const int pair = pair0 + blockIdx.y;
+    const uint64_t pair_seed = mix_u64(seed0, mix_u64(epoch, static_cast<uint64_t>(pair)));
     const long long n = static_cast<long long>(d.n_major) * d.rank;
     const long long idx = static_cast<long long>(bm & 0xfffffu) * blockDim.x + threadIdx.x;
-    if (idx >= n) return;
-    uint64_t seed = mix_u64(pair_seeds[pair], d.salt);
+    uint64_t seed = mix_u64(pair_seed, d.salt);
     if (d.factor != 0) seed = mix_u64(seed, d.factor);
-    const int v = noise_hash(seed, static_cast<uint64_t>(idx), use_clt != 0, clt_k);
+    const int v = use_clt != 0 && clt_k == 4 ? noise_clt4(noise_seed(seed), static_cast<uint64_t>(idx)) : noise_hash(seed, static_cast<uint64_t>(idx), use_clt != 0, clt_k);
+    pdl_wait();  // everything above is computed from constants
+    if (seeds_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) seeds_out[pair] = pair_seed;
+    if (idx >= n) return;
     long long o = idx;
     if (d.transposed) {
         const long long major = idx / d.rank, r = idx - major * d.rank;
@@ -116,13 +119,18 @@ struct Model {
     float* y_emb;
     int32_t *t_a, *t_f;
     // update scratch
-    float *Z, *Z_all, *sumsq, *inv_rms;
-    UpdApplyDesc* upd_descs;  // table, block partials and inv_rms of the batched apply phase
+    float* Z_all;
+    UpdApplyDesc* upd_descs;  // table (matrices, head bias, beta bias, positional table), block partials and inv_rms of the batched apply phase
+    uint2* upd_tab;           // the block quantiser's table for the weights
+    int num_upd = 0, upd_blocks = 0, upd_ublocks = 0, upd_blocks_nopos = 0, upd_ublocks_nopos = 0;
     float *upd_partial, *upd_inv;
+    ZDenseDesc* zdense;       // tensors whose Z comes from dense noise: the vectors, in the dense mode the matrices too
+    std::vector<ZDenseDesc> h_zdense;
     ZLowrankDesc *zdesc, *zdesc_ext;  // device tables of the update's matrices: Z inside Z_all / inside a caller's buffer
     int launches_per_wave = 0;
+    uint8_t* h_weights = nullptr;  // pinned staging of get_weights (small models only)
     float* h_step = nullptr;    // bnf4_model_es_step: pinned losses [2 * max_pairs] + pair weights [max_pairs]
-    float* d_step_w = nullptr;  // ... and the shaped pair weights on the device
+    float* d_step_w;            // ... and the shaped pair weights on the device
     // dense (rank 0) mode: the reference driver's own perturbation, one materialised noise matrix per weight matrix and pair,
     // applied as a second GEMM with beta = 1 (src/train_efla_lm.cpp:2359-2367). One pair per wave.
     bool dense = false;
@@ -171,19 +179,27 @@ struct Model {
         return e;
     }
 
+    // Buffers are requested first and carved out of one zeroed allocation afterwards: sixty allocations cost tens of milliseconds.
+    struct Request { void** slot; size_t bytes; };
+    std::vector<Request> requests;
     template <typename Tp>
-    int alloc(Tp** p, size_t count, bool zero = true) {
-        void* ptr = nullptr;
-        const size_t bytes = ((count * sizeof(Tp) + 255) / 256) * 256;
-        int rc = check_cuda(cudaMalloc(&ptr, bytes), "cudaMalloc(model)");
+    void want(Tp** p, size_t count) {
+        *p = nullptr;
+        requests.push_back({reinterpret_cast<void**>(p), (std::max<size_t>(count, 1) * sizeof(Tp) + 1023) / 1024 * 1024});
+    }
+    int commit() {
+        size_t total = 0;
+        for (const Request& r : requests) total += r.bytes;
+        void* base = nullptr;
+        int rc = check_cuda(cudaMalloc(&base, total), "cudaMalloc(model)");
         if (rc) return rc;
-        allocs.push_back(ptr);
-        device_bytes += bytes;
-        if (zero) {
-            rc = check_cuda(cudaMemset(ptr, 0, bytes), "cudaMemset(model)");
-            if (rc) return rc;
-        }
-        *p = static_cast<Tp*>(ptr);
+        allocs.push_back(base);
+        device_bytes += total;
+        rc = check_cuda(cudaMemset(base, 0, total), "cudaMemset(model)");
+        if (rc) return rc;
+        uint8_t* at = static_cast<uint8_t*>(base);
+        for (const Request& r : requests) { *r.slot = at; at += r.bytes; }
+        requests.clear();
         return BNF4_OK;
     }
 };
@@ -214,25 +230,7 @@ struct TimedScope {
     } while (0)
 
 int quantize_base(Model& m, cudaStream_t st) {
-    auto plain = [&](const int8_t* w, int rows, int cols, uint8_t* codes, uint8_t* sf) {
-        bnf4_rowquant_desc p = {};
-        p.rows = rows; p.cols_in = cols; p.cols_out = cols; p.in_i8 = w; p.ld_in = cols; p.out_codes = codes; p.out_sf = sf;
-        return rowquant_dispatch(FE_INT8, p, st);
-    };
-    TRY(plain(m.win, m.H, m.H, m.q_win, m.sfq_win));
-    TRY(plain(m.head, m.V, m.H, m.q_head, m.sfq_head));
-    const size_t hh = static_cast<size_t>(m.H) * m.H, hf = static_cast<size_t>(m.H) * m.F;
-    for (int l = 0; l < m.L; ++l) {
-        bnf4_rowquant_desc p = {};
-        p.rows = 3 * m.H + 1; p.cols_in = m.H; p.cols_out = m.H;
-        p.wq = m.wq + l * hh; p.wk = m.wk + l * hh; p.wv = m.wv + l * hh; p.wb = m.wbeta + static_cast<size_t>(l) * m.H;
-        p.q_scale = p.k_scale = p.v_scale = p.b_scale = m.s_h;
-        p.out_codes = m.q_qkv[l]; p.out_sf = m.sfq_qkv[l];
-        TRY(rowquant_dispatch(FE_WQKV, p, st));
-        TRY(plain(m.ff1 + l * hf, m.F, m.H, m.q_ff1[l], m.sfq_ff1[l]));
-        TRY(plain(m.ff2 + l * hf, m.H, m.F, m.q_ff2[l], m.sfq_ff2[l]));
-    }
-    return BNF4_OK;
+    return requantize_batched(m.upd_descs, m.num_upd, m.upd_ublocks, m.upd_tab, st);
 }
 
 // One wave: members [0, nm) of the wave correspond to pairs [p0, p0 + nm/2). sigma == 0 evaluates the base model.
@@ -360,12 +358,13 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
             p.add_scale = m.cfg.residual_scale; p.norm_scale = m.cfg.ln_scale;
             p.out_codes = m.a_h; p.out_sf = m.sf_h;
             if (pert) { p.tvec = m.tB_ff1[l] + P0 * r * H; p.tvec_pair_stride = static_cast<long long>(r) * H; p.nvec = r; p.t_out = m.t_a; }
-            TRY(rowquant_dispatch(FE_ADD_ABSMEAN, p, st));
+            RowQuantParams pz(p);
+            if (pert) { pz.zero_t = m.t_f; pz.zero_n = r; }  // ff1 accumulates the projections for ff2 there
+            TRY(rowquant_dispatch(FE_ADD_ABSMEAN, pz, st));
             ++launches;
         }
         {   // ff1 with GELU -> int8 -> FP4 epilogue, projections for ff2
             TimedScope ts(m, KC_GEMM_FF1, st);
-            if (pert) TRY(check_cuda(cudaMemsetAsync(m.t_f, 0, static_cast<size_t>(rows) * r * sizeof(int32_t), st), "cudaMemsetAsync(t_f)"));
             bnf4_gemm_desc g = {};
             g.a = m.a_h; g.b = m.q_ff1[l]; g.sfa = m.sf_h; g.sfb = m.sfq_ff1[l]; g.m = rows; g.n = F; g.k = H; g.alpha = m.s_h;
             g.epilogue = EPI_GELU_FP4; g.act_scale = m.cfg.mlp_act_scale; g.d_codes = m.a_f; g.d_sf = m.sf_f;
@@ -677,11 +676,6 @@ std::vector<UpdVector> update_vectors(Model& m) {
 }
 // A vector is computed in element ranges by the ranks only when that saves real work.
 inline bool vector_sharded(int n, int nshards) { return nshards > 1 && n >= 4096 && (n % nshards) == 0; }
-long long z_matrix_elems(Model& m) {
-    long long n = 0;
-    for (const UpdMatrix& x : update_matrices(m)) n += static_cast<long long>(x.rows) * x.cols;
-    return n;
-}
 
 // Device table of the matrices with Z laid out back to back from z_base (the order of update_matrices).
 std::vector<ZLowrankDesc> z_descs(Model& m, float* z_base) {
@@ -704,69 +698,75 @@ int update_z(Model& m, const float* pair_weights, int shard, int nshards, float*
         dtab = m.zdesc_ext;
     }
     float* zb = z_ext != nullptr ? z_ext : m.Z_all;
-    TimedScope ts(m, KC_UPDATE_Z, st, 4);
-    if (m.dense) {
-        // Z[i] = sum_p w_p noise(mix(seed_p, salt), i) per matrix: the reference's compute_z_sumsq (src/efla_lm_kernels.cu:1854-1890),
-        // rows of a sharded matrix by element range
-        const int L = m.L;
-        std::vector<uint64_t> salts = {kSaltEmb, kSaltWin};
-        for (int l = 0; l < L; ++l)
-            for (uint64_t sl : {kSaltWq, kSaltWk, kSaltWv, kSaltWbeta, kSaltFf1, kSaltFf2}) salts.push_back(mix_u64(static_cast<uint64_t>(l), sl));
-        salts.push_back(kSaltHead);
-        long long zo = 0;
-        for (size_t i = 0; i < h.size(); ++i) {
-            const long long n = static_cast<long long>(h[i].rows) * h[i].cols;
-            long long i0 = 0, cnt = n;
-            if (nshards > 1 && h[i].rows >= nshards && (h[i].rows % nshards) == 0) { cnt = n / nshards; i0 = shard * cnt; }
-            TRY(z_dense_launch(pair_weights, m.pair_seeds, salts[i], m.pairs_step, static_cast<int>(i0), static_cast<int>(cnt), m.cfg.use_clt, m.cfg.clt_k,
-                               zb + zo + i0, st));
-            zo += n;
-        }
-    } else {
-        TRY(z_lowrank_launch(pair_weights, dtab, h.data(), static_cast<int>(h.size()), m.pairs_step, m.r, m.c_r, shard, nshards, st));
-    }
-    long long off = z_matrix_elems(m);
-    for (const UpdVector& x : update_vectors(m)) {
-        int i0 = 0, cnt = x.n;
-        if (vector_sharded(x.n, nshards)) { cnt = x.n / nshards; i0 = shard * cnt; }
-        TRY(z_dense_launch(pair_weights, m.pair_seeds, x.salt, m.pairs_step, i0, cnt, m.cfg.use_clt, m.cfg.clt_k, zb + off + i0, st));
-        off += x.n;
-    }
-    return BNF4_OK;
+    TimedScope ts(m, KC_UPDATE_Z, st, 2);
+    if (!m.dense) TRY(z_lowrank_launch(pair_weights, dtab, h.data(), static_cast<int>(h.size()), m.pairs_step, m.r, m.c_r, shard, nshards, st));
+    // the fp32 vectors (in the dense mode the matrices too: Z[i] = sum_p w_p noise(mix(seed_p, salt), i), the reference's
+    // compute_z_sumsq, src/efla_lm_kernels.cu:1854-1890); the vectors' noise lies in memory when this process evaluated every pair
+    const int tables = m.eval_begin == 0 && m.eval_end == m.pairs_step;
+    return z_dense_table_launch(pair_weights, m.pair_seeds, m.zdense, m.h_zdense.data(), static_cast<int>(m.h_zdense.size()), m.pairs_step, m.cfg.use_clt,
+                                m.cfg.clt_k, tables, shard, nshards, zb, st);
 }
 
-// Applies the precomputed Z of every tensor (sum of squares, RMS-EMA, gated update: four launches for all of them) and
-// re-quantises the base weights.
+// Applies the precomputed Z of every tensor (sum of squares, RMS-EMA, gated update) and renews the NVFP4 copies of the weights: three
+// launches for all of them.
 int update_apply(Model& m, const float* pair_weights, const float* z_all, const bnf4_update_cfg* u, cudaStream_t st) {
     (void)pair_weights;
-    const int P = m.pairs_step;
-    const int L = m.L;
-    const float thresh = u->thresh * std::sqrt(static_cast<float>(P));
+    const float thresh = u->thresh * std::sqrt(static_cast<float>(m.pairs_step));
+    const bool pos = u->train_pos != 0;  // the positional table is the last tensor
+    TimedScope ts(m, KC_UPDATE_APPLY, st, 3);
+    return update_apply_batched(m.upd_descs, pos ? m.num_upd : m.num_upd - 1, pos ? m.upd_blocks : m.upd_blocks_nopos, pos ? m.upd_ublocks : m.upd_ublocks_nopos, z_all,
+                                m.upd_tab, m.upd_partial, m.upd_inv, u->use_adaptive, u->adaptive_beta, u->adaptive_eps, u->lr, thresh, st);
+}
+
+// The static tables of the update: every tensor's weights, shadow and NVFP4 copy; the tensors with dense noise. Called once, after
+// the buffers exist.
+int build_update_tables(Model& m) {
     std::vector<UpdApplyDesc> h;
-    int slot = 0, block0 = 0;
+    int slot = 0;
     long long off = 0;
-    for (const UpdMatrix& x : update_matrices(m)) {
-        const int n = x.rows * x.cols;
-        h.push_back({x.w, x.shadow, z_all + off, m.rms_ema + (slot++), n, block0});
-        block0 += (n + 255) / 256;
+    auto add = [&](int8_t* w, float* target, int n, int cols, uint8_t* codes, uint8_t* sf, int row0, int scaled) {
+        UpdApplyDesc d = {};
+        d.w = w; d.target = target; d.ema = m.rms_ema + (slot++); d.codes = codes; d.sf = sf; d.zoff = off; d.n = n; d.cols = cols; d.row0 = row0;
+        d.scaled = scaled; d.block0 = m.upd_blocks; d.ublock0 = m.upd_ublocks;
+        h.push_back(d);
         off += n;
+        m.upd_blocks += (n + 255) / 256;
+        m.upd_ublocks += (n + 1023) / 1024;
+    };
+    const std::vector<UpdMatrix> mats = update_matrices(m);
+    for (size_t i = 0; i < mats.size(); ++i) {
+        const UpdMatrix& x = mats[i];
+        uint8_t *codes = nullptr, *sf = nullptr;  // (the embedding is looked up, it has no NVFP4 copy)
+        int row0 = 0, scaled = 0;
+        if (i == 1) { codes = m.q_win; sf = m.sfq_win; }
+        else if (i + 1 == mats.size()) { codes = m.q_head; sf = m.sfq_head; }
+        else if (i >= 2) {
+            const int l = static_cast<int>(i - 2) / 6, g = static_cast<int>(i - 2) % 6;
+            if (g < 4) { codes = m.q_qkv[l]; sf = m.sfq_qkv[l]; row0 = g * m.H; scaled = 1; }
+            else if (g == 4) { codes = m.q_ff1[l]; sf = m.sfq_ff1[l]; }
+            else { codes = m.q_ff2[l]; sf = m.sfq_ff2[l]; }
+        }
+        add(x.w, x.shadow, x.rows * x.cols, x.cols, codes, sf, row0, scaled);
     }
+    std::vector<uint64_t> salts = {kSaltEmb, kSaltWin};
+    for (int l = 0; l < m.L; ++l)
+        for (uint64_t sl : {kSaltWq, kSaltWk, kSaltWv, kSaltWbeta, kSaltFf1, kSaltFf2}) salts.push_back(mix_u64(static_cast<uint64_t>(l), sl));
+    salts.push_back(kSaltHead);
+    if (m.dense)
+        for (size_t i = 0; i < mats.size(); ++i) m.h_zdense.push_back({salts[i], nullptr, h[i].zoff, h[i].n, mats[i].rows});
+    const int8_t* noise[3] = {m.hb_noise, m.bb_noise, m.pos_noise};
+    int v = 0;
     for (const UpdVector& x : update_vectors(m)) {
-        const float* Z = z_all + off;
-        off += x.n;
-        if (x.v == m.pos && !u->train_pos) continue;
-        h.push_back({nullptr, x.v, Z, m.rms_ema + (slot++), x.n, block0});
-        block0 += (x.n + 255) / 256;
+        if (x.v == m.pos) { m.upd_blocks_nopos = m.upd_blocks; m.upd_ublocks_nopos = m.upd_ublocks; }
+        m.h_zdense.push_back({x.salt, noise[v++], off, x.n, 0});
+        add(nullptr, x.v, x.n, 0, nullptr, nullptr, 0, 0);
     }
-    {
-        TimedScope ts(m, KC_UPDATE_APPLY, st, 3);
-        // pageable source: the copy is staged before the call returns
-        TRY(check_cuda(cudaMemcpyAsync(m.upd_descs, h.data(), h.size() * sizeof(UpdApplyDesc), cudaMemcpyHostToDevice, st), "cudaMemcpyAsync(upd_descs)"));
-        TRY(update_apply_batched(m.upd_descs, static_cast<int>(h.size()), block0, m.upd_partial, m.upd_inv, u->use_adaptive, u->adaptive_beta,
-                                 u->adaptive_eps, u->lr, thresh, st));
-    }
-    TimedScope ts(m, KC_REQUANTIZE, st, 2 + 3 * L);
-    return quantize_base(m, st);
+    m.num_upd = static_cast<int>(h.size());
+    uint2 tab[256];
+    update_quant_table(m.s_h, tab);
+    TRY(check_cuda(cudaMemcpy(m.upd_descs, h.data(), h.size() * sizeof(UpdApplyDesc), cudaMemcpyHostToDevice), "cudaMemcpy(upd_descs)"));
+    TRY(check_cuda(cudaMemcpy(m.zdense, m.h_zdense.data(), m.h_zdense.size() * sizeof(ZDenseDesc), cudaMemcpyHostToDevice), "cudaMemcpy(zdense)"));
+    return check_cuda(cudaMemcpy(m.upd_tab, tab, sizeof(tab), cudaMemcpyHostToDevice), "cudaMemcpy(upd_tab)");
 }
 
 }  // namespace
@@ -781,7 +781,7 @@ int bnf4_model_destroy(void* handle) {
     if (m->cap_stream) cudaStreamDestroy(m->cap_stream);
     for (void* p : m->allocs) cudaFree(p);
     if (m->h_step) cudaFreeHost(m->h_step);
-    if (m->d_step_w) cudaFree(m->d_step_w);
+    if (m->h_weights) cudaFreeHost(m->h_weights);
     for (cudaEvent_t e : m->free_events) cudaEventDestroy(e);
     for (const Model::Span& sp : m->spans) { cudaEventDestroy(sp.a); cudaEventDestroy(sp.b); }
     delete m;
@@ -829,7 +829,7 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     const int V = m->V, H = m->H, F = m->F, L = m->L, T = m->T, r = m->r, P = cfg->max_pairs;
     const size_t hh = static_cast<size_t>(H) * H, hf = static_cast<size_t>(H) * F;
     int rc = 0;
-#define A_(ptr, count) if (!rc) rc = m->alloc(&m->ptr, (count))
+#define A_(ptr, count) m->want(&m->ptr, (count))
     A_(emb, static_cast<size_t>(V) * H); A_(win, hh); A_(wq, L * hh); A_(wk, L * hh); A_(wv, L * hh); A_(wbeta, static_cast<size_t>(L) * H);
     A_(ff1, L * hf); A_(ff2, L * hf); A_(head, static_cast<size_t>(V) * H);
     A_(head_bias, V); A_(beta_bias, L); A_(pos, static_cast<size_t>(T) * H);
@@ -839,7 +839,7 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     A_(q_win, hh / 2); A_(sfq_win, sf_bytes(H, H)); A_(q_head, static_cast<size_t>(V) * H / 2); A_(sfq_head, sf_bytes(V, H));
     m->q_qkv.resize(L); m->sfq_qkv.resize(L); m->q_ff1.resize(L); m->sfq_ff1.resize(L); m->q_ff2.resize(L); m->sfq_ff2.resize(L);
     m->A_qkv.resize(L); m->tB_qkv.resize(L); m->A_ff1.resize(L); m->tB_ff1.resize(L); m->A_ff2.resize(L); m->tB_ff2.resize(L);
-    for (int l = 0; l < L && !rc; ++l) {
+    for (int l = 0; l < L; ++l) {
         A_(q_qkv[l], static_cast<size_t>(m->FC) * H / 2); A_(sfq_qkv[l], sf_bytes(m->FC, H));
         A_(q_ff1[l], hf / 2); A_(sfq_ff1[l], sf_bytes(F, H)); A_(q_ff2[l], hf / 2); A_(sfq_ff2[l], sf_bytes(H, F));
         A_(A_qkv[l], static_cast<size_t>(P) * (3 * H + 1) * r); A_(tB_qkv[l], static_cast<size_t>(P) * 4 * r * H);
@@ -867,24 +867,35 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
         A_(E_all, lay.total);
         A_(qe_win, hh / 2); A_(sfe_win, sf_bytes(H, H)); A_(qe_head, static_cast<size_t>(V) * H / 2); A_(sfe_head, sf_bytes(V, H));
         m->qe_qkv.resize(L); m->sfe_qkv.resize(L); m->qe_ff1.resize(L); m->sfe_ff1.resize(L); m->qe_ff2.resize(L); m->sfe_ff2.resize(L);
-        for (int l = 0; l < L && !rc; ++l) {
+        for (int l = 0; l < L; ++l) {
             A_(qe_qkv[l], static_cast<size_t>(m->FC) * H / 2); A_(sfe_qkv[l], sf_bytes(m->FC, H));
             A_(qe_ff1[l], hf / 2); A_(sfe_ff1[l], sf_bytes(F, H)); A_(qe_ff2[l], hf / 2); A_(sfe_ff2[l], sf_bytes(H, F));
         }
         A_(noise_descs, 3 + 6 * static_cast<size_t>(L));
         A_(ff1_f, Mr * F); A_(ff1_q, Mr * F);
     }
-    A_(Z, static_cast<size_t>(T) * H + V + L); A_(sumsq, 1); A_(inv_rms, 1);
+    const size_t nmat = 3 + 6 * static_cast<size_t>(L);  // emb, win, head and six per layer
     {
-        size_t zn = static_cast<size_t>(V) + L + static_cast<size_t>(T) * H;
-        for (const UpdMatrix& x : update_matrices(*m)) zn += static_cast<size_t>(x.rows) * x.cols;
-        const size_t nd = update_matrices(*m).size();
-        A_(Z_all, zn); A_(zdesc, nd); A_(zdesc_ext, nd);
-        size_t nblk = (static_cast<size_t>(V) + 255) / 256 + (static_cast<size_t>(L) + 255) / 256 + (static_cast<size_t>(T) * H + 255) / 256;
-        for (const UpdMatrix& x : update_matrices(*m)) nblk += (static_cast<size_t>(x.rows) * x.cols + 255) / 256;
-        A_(upd_descs, nd + 3); A_(upd_partial, nblk); A_(upd_inv, nd + 3);
+        const size_t mat_elems[] = {static_cast<size_t>(V) * H, hh, static_cast<size_t>(V) * H};
+        const size_t layer_elems[] = {hh, hh, hh, static_cast<size_t>(H), hf, hf};
+        const size_t vec_elems[] = {static_cast<size_t>(V), static_cast<size_t>(L), static_cast<size_t>(T) * H};
+        size_t zn = 0, nblk = 0;
+        auto count = [&](size_t n, size_t times) { zn += times * n; nblk += times * ((n + 255) / 256); };
+        for (size_t n : mat_elems) count(n, 1);
+        for (size_t n : layer_elems) count(n, L);
+        for (size_t n : vec_elems) count(n, 1);
+        A_(Z_all, zn); A_(zdesc, nmat); A_(zdesc_ext, nmat); A_(upd_descs, nmat + 3); A_(upd_partial, nblk); A_(upd_inv, nmat + 3); A_(upd_tab, 256);
+        A_(zdense, nmat + 3); A_(d_step_w, P);
+        // noise table: two factors per matrix and three vectors
+        auto nb = [](size_t n) { return (n + 255) / 256; };
+        const size_t bV = nb(static_cast<size_t>(V) * r), bH = nb(static_cast<size_t>(H) * r), bF = nb(static_cast<size_t>(F) * r), b1 = nb(r);
+        A_(gen_descs, 2 * nmat + 3);
+        A_(gen_block_map, 2 * (bV + bH) + 2 * bH + L * (6 * bH + b1 + bH + 2 * (bF + bH)) + nb(static_cast<size_t>(T) * H) + nb(V) + nb(L));
     }
 #undef A_
+    rc = m->commit();
+    if (rc) { bnf4_model_destroy(m); return rc; }
+    rc = build_update_tables(*m);
     if (rc) { bnf4_model_destroy(m); return rc; }
     {
         const std::vector<ZLowrankDesc> zd = z_descs(*m, m->Z_all);
@@ -932,11 +943,14 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
         for (long long b = 0; b < nb; ++b) bmap.push_back(static_cast<uint32_t>(i << 20) | static_cast<uint32_t>(b));
     }
     m->gen_blocks = static_cast<int>(bmap.size());
-    rc = m->alloc(&m->gen_descs, gd.size());
-    if (!rc) rc = check_cuda(cudaMemcpy(m->gen_descs, gd.data(), gd.size() * sizeof(GenDesc), cudaMemcpyHostToDevice), "cudaMemcpy(gen_descs)");
-    if (!rc) rc = m->alloc(&m->gen_block_map, bmap.size());
+    rc = check_cuda(cudaMemcpy(m->gen_descs, gd.data(), gd.size() * sizeof(GenDesc), cudaMemcpyHostToDevice), "cudaMemcpy(gen_descs)");
     if (!rc) rc = check_cuda(cudaMemcpy(m->gen_block_map, bmap.data(), bmap.size() * sizeof(uint32_t), cudaMemcpyHostToDevice), "cudaMemcpy(gen_block_map)");
     if (rc) { bnf4_model_destroy(m); return rc; }
+    const size_t span = static_cast<size_t>(reinterpret_cast<const uint8_t*>(m->pos) - reinterpret_cast<const uint8_t*>(m->emb)) + static_cast<size_t>(T) * H * sizeof(float);
+    if (span <= kWeightStageBytes) {
+        rc = check_cuda(cudaMallocHost(&m->h_weights, span), "cudaMallocHost(weights)");
+        if (rc) { bnf4_model_destroy(m); return rc; }
+    }
     *handle = m;
     return BNF4_OK;
 }
@@ -1022,13 +1036,23 @@ int bnf4_model_set_optimizer_state(void* handle, const float* h_shadow, const fl
 int bnf4_model_get_weights(void* handle, bnf4_model_weights* w) {
     if (!handle || !w) return set_error(BNF4_ERR_INVALID, "model_get_weights: null argument");
     Model& m = *M(handle);
-    TRY(check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize"));
     const size_t vh = static_cast<size_t>(m.V) * m.H, hh = static_cast<size_t>(m.H) * m.H, hf = static_cast<size_t>(m.H) * m.F;
     struct Item { const void* d; void* h; size_t bytes; };
     const Item items[] = {{m.emb, w->emb, vh}, {m.win, w->win, hh}, {m.wq, w->wq, m.L * hh}, {m.wk, w->wk, m.L * hh}, {m.wv, w->wv, m.L * hh},
                           {m.wbeta, w->wbeta, static_cast<size_t>(m.L) * m.H}, {m.ff1, w->ff1, m.L * hf}, {m.ff2, w->ff2, m.L * hf},
                           {m.head, w->head, vh}, {m.head_bias, w->head_bias, m.V * sizeof(float)}, {m.beta_bias, w->beta_bias, m.L * sizeof(float)},
                           {m.pos, w->pos, static_cast<size_t>(m.T) * m.H * sizeof(float)}};
+    TRY(check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize"));
+    // The twelve arrays lie back to back on the device (create requests them first, in this order). Small models come over in one
+    // copy through a pinned buffer: twelve copies to pageable memory cost more than the smallest step. Large ones go directly.
+    if (m.h_weights != nullptr) {
+        const uint8_t* first = reinterpret_cast<const uint8_t*>(m.emb);
+        const size_t span = static_cast<size_t>(reinterpret_cast<const uint8_t*>(m.pos) - first) + items[11].bytes;
+        TRY(check_cuda(cudaMemcpy(m.h_weights, first, span, cudaMemcpyDeviceToHost), "cudaMemcpy(weights)"));
+        for (const Item& it : items)
+            if (it.h) std::memcpy(it.h, m.h_weights + (static_cast<const uint8_t*>(it.d) - first), it.bytes);
+        return BNF4_OK;
+    }
     for (const Item& it : items)
         if (it.h) TRY(check_cuda(cudaMemcpy(it.h, it.d, it.bytes, cudaMemcpyDeviceToHost), "cudaMemcpy(weights)"));
     return BNF4_OK;
@@ -1054,20 +1078,21 @@ int bnf4_model_prepare_step_range(void* handle, uint64_t seed, uint64_t epoch, i
     m.eval_end = eval_begin + eval_count;
     m.step_seed = seed;
     m.step_epoch = epoch;
-    TRY(bnf4_fill_pair_seeds(seed, epoch, pairs, m.pair_seeds, stream));
-    TimedScope ts(m, KC_GEN_NOISE, S(stream), 3);
-    // rank-r factors of all pairs (the update reads them all; the dense mode has none) ...
-    if (!m.dense) {
-        launch_pdl_if(pairs * static_cast<long long>(m.gen_blocks_factors) <= 8192, gen_noise_kernel, dim3(m.gen_blocks_factors, pairs), 256, 0, S(stream), m.gen_descs, m.gen_block_map, 0, 0, m.pair_seeds, m.cfg.use_clt, m.cfg.clt_k);
-        TRY(check_launch("gen_noise_kernel"));
+    TimedScope ts(m, KC_GEN_NOISE, S(stream), 2);
+    auto gen = [&](int block0, int blocks, int pair0, int count, uint64_t* seeds_out) -> int {
+        if (blocks <= 0 || count <= 0) return BNF4_OK;
+        launch_pdl_if(count * static_cast<long long>(blocks) <= 8192, gen_noise_kernel, dim3(blocks, count), 256, 0, S(stream), m.gen_descs, m.gen_block_map, block0,
+                      pair0, seed, epoch, m.cfg.use_clt, m.cfg.clt_k, seeds_out);
+        return check_launch("gen_noise_kernel");
+    };
+    if (m.dense) {  // no rank-r factors
+        TRY(bnf4_fill_pair_seeds(seed, epoch, pairs, m.pair_seeds, stream));
+        return gen(m.gen_blocks_factors, m.gen_blocks - m.gen_blocks_factors, eval_begin, eval_count, nullptr);
     }
-    // ... and the per-pair vectors only for the pairs this process evaluates
-    if (eval_count > 0) {
-        launch_pdl_if(eval_count * static_cast<long long>(m.gen_blocks - m.gen_blocks_factors) <= 8192, gen_noise_kernel, dim3(m.gen_blocks - m.gen_blocks_factors, eval_count), 256, 0, S(stream), m.gen_descs, m.gen_block_map, m.gen_blocks_factors,
-                                                                                                        eval_begin, m.pair_seeds, m.cfg.use_clt, m.cfg.clt_k);
-        TRY(check_launch("gen_noise_kernel"));
-    }
-    return BNF4_OK;
+    if (eval_count == pairs) return gen(0, m.gen_blocks, 0, pairs, m.pair_seeds);
+    // rank-r factors of all pairs (the update reads them all), the per-pair vectors only for the pairs this process evaluates
+    TRY(gen(0, m.gen_blocks_factors, 0, pairs, m.pair_seeds));
+    return gen(m.gen_blocks_factors, m.gen_blocks - m.gen_blocks_factors, eval_begin, eval_count, nullptr);
 }
 
 int bnf4_model_prepare_step(void* handle, uint64_t seed, uint64_t epoch, int pairs, void* stream) {
@@ -1097,8 +1122,7 @@ int bnf4_model_eval_pairs(void* handle, int pair_begin, int pair_count, float* l
 int bnf4_model_eval_base(void* handle, float* loss, void* stream) {
     if (!handle || !loss) return set_error(BNF4_ERR_INVALID, "model_eval_base: null argument");
     Model& m = *M(handle);
-    TRY(run_wave_cached(m, 0, 2, 0.0f, m.losses, S(stream)));
-    return check_cuda(cudaMemcpyAsync(loss, m.losses, sizeof(float), cudaMemcpyDeviceToDevice, S(stream)), "cudaMemcpyAsync(loss)");
+    return run_wave_cached(m, 0, 1, 0.0f, loss, S(stream));  // one unperturbed member
 }
 
 int bnf4_model_update(void* handle, const float* pair_weights, const bnf4_update_cfg* u, void* stream) {
@@ -1167,18 +1191,20 @@ int bnf4_model_es_step(void* handle, const bnf4_es_step_cfg* cfg, const bnf4_col
     TRY(bnf4_model_eval_pairs(handle, begin, count, d_losses_all + 2 * static_cast<size_t>(begin), stream));
     if (world > 1 && coll->allgather_inplace(coll->ctx, d_losses_all, 2 * static_cast<size_t>(count) * sizeof(float), stream) != 0)
         return set_error(BNF4_ERR_CUDA, "model_es_step: the all-gather of the losses failed");
-    // fitness shaping on the host, like the reference (src/train_efla_lm.cpp:5466, 5476): f_p = -(loss+ - loss-)
-    if (m.h_step == nullptr) {
-        TRY(check_cuda(cudaMallocHost(&m.h_step, 3 * static_cast<size_t>(m.cfg.max_pairs) * sizeof(float)), "cudaMallocHost(es_step)"));
-        TRY(check_cuda(cudaMalloc(&m.d_step_w, static_cast<size_t>(m.cfg.max_pairs) * sizeof(float)), "cudaMalloc(es_step)"));
+    // fitness shaping (reference: src/train_efla_lm.cpp:5466, 5476): f_p = -(loss+ - loss-), on the device where the population is small enough
+    // for its counting sort -- the step then runs without a host round trip -- and on the host otherwise, with the same bits
+    if (shape_fitness_applies(pairs, cfg->fitness_mode)) {
+        TRY(shape_fitness_launch(d_losses_all, pairs, cfg->fitness_mode, cfg->fitness_clip, m.d_step_w, st));
+    } else {
+        if (m.h_step == nullptr) TRY(check_cuda(cudaMallocHost(&m.h_step, 3 * static_cast<size_t>(m.cfg.max_pairs) * sizeof(float)), "cudaMallocHost(es_step)"));
+        float* h_losses = m.h_step;
+        float* h_w = m.h_step + 2 * static_cast<size_t>(m.cfg.max_pairs);
+        TRY(check_cuda(cudaMemcpyAsync(h_losses, d_losses_all, 2 * static_cast<size_t>(pairs) * sizeof(float), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync(losses)"));
+        TRY(check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize"));
+        for (int p = 0; p < pairs; ++p) h_w[p] = -(h_losses[2 * p] - h_losses[2 * p + 1]);
+        TRY(bnf4_shape_pair_weights(h_w, pairs, cfg->fitness_mode, cfg->fitness_clip));
+        TRY(check_cuda(cudaMemcpyAsync(m.d_step_w, h_w, static_cast<size_t>(pairs) * sizeof(float), cudaMemcpyHostToDevice, st), "cudaMemcpyAsync(pair weights)"));
     }
-    float* h_losses = m.h_step;
-    float* h_w = m.h_step + 2 * static_cast<size_t>(m.cfg.max_pairs);
-    TRY(check_cuda(cudaMemcpyAsync(h_losses, d_losses_all, 2 * static_cast<size_t>(pairs) * sizeof(float), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync(losses)"));
-    TRY(check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize"));
-    for (int p = 0; p < pairs; ++p) h_w[p] = -(h_losses[2 * p] - h_losses[2 * p + 1]);
-    TRY(bnf4_shape_pair_weights(h_w, pairs, cfg->fitness_mode, cfg->fitness_clip));
-    TRY(check_cuda(cudaMemcpyAsync(m.d_step_w, h_w, static_cast<size_t>(pairs) * sizeof(float), cudaMemcpyHostToDevice, st), "cudaMemcpyAsync(pair weights)"));
     if (world == 1) {
         TRY(update_z(m, m.d_step_w, 0, 1, nullptr, st));
         return update_apply(m, m.d_step_w, m.Z_all, &cfg->update, st);

@@ -51,6 +51,10 @@ __global__ void __launch_bounds__(256) rowquant_kernel(const RowQuantParams p, c
     int xw[NB][4];  // stage-1 int8 values of this lane's blocks, four per word
     int sum_abs = 0;
 
+    if constexpr (FE == FE_ADD_ABSMEAN) {
+        if (p.zero_t != nullptr && lane < p.zero_n) p.zero_t[static_cast<size_t>(row) * p.zero_n + lane] = 0;
+    }
+
     // ---------------- stage 1: produce integer values ----------------
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
@@ -341,6 +345,10 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
                     }
                 }
             }
+        }
+
+        if constexpr (FE == FE_ADD_ABSMEAN) {
+            if (p.zero_t != nullptr && lane < p.zero_n) p.zero_t[static_cast<size_t>(row) * p.zero_n + lane] = 0;
         }
 
         // ---------------- stage 1: integer values of the row as floats ----------------

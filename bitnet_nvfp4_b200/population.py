@@ -170,7 +170,7 @@ class PopulationModel:
 
     def get_weights(self) -> dict:
         shapes = self.cfg.weight_shapes()
-        arrays = {n: np.zeros(shapes[n], np.float32 if n in ("head_bias", "beta_bias", "pos") else np.int8) for n in WEIGHT_NAMES}
+        arrays = {n: np.empty(shapes[n], np.float32 if n in ("head_bias", "beta_bias", "pos") else np.int8) for n in WEIGHT_NAMES}
         _l.check(self.lib.bnf4_model_get_weights(self.h, C.byref(self._weights_struct(arrays))))
         return arrays
 
@@ -356,6 +356,8 @@ def es_step(model, seed: int, epoch: int, pairs_total: int, rank: int = 0, world
     `spans`: optional list that receives (name, start event, end event) around every collective (CUDA devices only).
     `marks`: optional dict that receives the host-clock durations "eval_s" (noise + evaluation + loss gather, the reference's
     eval_s) and "update_s" (shaping + update); asking for them adds two device synchronisations."""
+    if world == 1 and marks is None and isinstance(model, PopulationModel):  # one call, no host round trip
+        return es_step_native(model, seed, epoch, pairs_total, lr=lr, thresh=thresh, fitness_mode=fitness_mode, fitness_clip=fitness_clip, **update_kw)
     import time
     import torch.distributed as dist
 
@@ -444,6 +446,7 @@ def es_step_native(model: "PopulationModel", seed: int, epoch: int, pairs_total:
     losses = losses_out if losses_out is not None else torch.empty(2 * pairs_total, dtype=torch.float32, device="cuda")
     cfg = EsStepCfg(seed, epoch, pairs_total, rank, world, fitness_mode, fitness_clip,
                     UpdateCfg(lr, thresh, int(use_adaptive), adaptive_beta, adaptive_eps, int(train_pos)))
+    model.pairs = pairs_total
     coll, keep = (torch_collectives(rank, world, group) if world > 1 else (None, None))
     _l.check(model.lib.bnf4_model_es_step(model.h, C.byref(cfg), C.byref(coll) if coll is not None else None, losses.data_ptr(), _stream()))
     del keep

@@ -498,8 +498,8 @@ int bnf4_model_update_apply(void* handle, const float* pair_weights, const float
 /* The whole ES step of one rank in ONE call, for hosts that run one process per GPU (what population.es_step does over
  * torch.distributed, and what replaces the body of the reference's epoch loop between eval_worker and the vector updates,
  * src/train_efla_lm.cpp:5344-5657): noise for the step -> this rank's pairs [rank * pairs / world, (rank + 1) * pairs / world)
- * -> all-gather of the per-member losses -> f_p = -(loss+ - loss-) shaped on the host (bnf4_shape_pair_weights; one stream
- * synchronisation and a round trip of 8 * pairs bytes, as the reference) -> noise sums Z by rows over the ranks -> in-place
+ * -> all-gather of the per-member losses -> f_p = -(loss+ - loss-) shaped like bnf4_shape_pair_weights (on the device, stream-ordered, for
+ * up to 4096 pairs; on the host with one stream synchronisation beyond, same bits) -> noise sums Z by rows over the ranks -> in-place
  * all-gather of every sharded Z -> apply. The library links no communication library: the caller supplies the two
  * collectives as callbacks over its own communicator (NCCL: ncclAllGather with sendbuff = recv + rank * bytes_per_rank).
  * Every rank must make the call with the same cfg except `rank`; all ranks end with identical weights, bit-identical to

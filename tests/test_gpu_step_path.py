@@ -1,0 +1,81 @@
+"""The step's device-side path: fitness shaping, noise sums from the noise tables, the update that renews the NVFP4 copies in the
+same pass, single-member validation, and a model narrower than its vocabulary. Integer and shaping results are compared bit for bit."""
+import numpy as np
+import pytest
+
+import oracle_lib as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def make(seed=3, **kw):
+    import torch
+    from bitnet_nvfp4_b200 import population, synth
+    assert torch.cuda.is_available()
+    cfg = population.Config(**kw)
+    w = synth.init_weights(cfg)
+    tok, tgt = synth.sample_batch(synth.zipf_corpus(1 << 14, 1.1, 123), cfg.batch, cfg.seq, seed)
+    model = population.PopulationModel(cfg)
+    model.set_weights(w)
+    model.set_tokens(tok, tgt)
+    return cfg, w, tok, tgt, model
+
+
+def oracle_loss(cfg, w, tok, tgt):
+    ocfg = {k: getattr(cfg, k) for k in "vocab hidden layers mlp_mult seq batch heads rank sigma_shift use_clt clt_k method act_scale "
+                                        "mlp_act_scale ln_scale residual_scale mlp_residual_scale eps".split()}
+    return orc.OracleModel(ocfg, w).forward(tok, tgt, 0, 0)
+
+
+def state(model):
+    w = model.get_weights()
+    shadow, ema = model.get_optimizer_state()
+    return [w[n] for n in sorted(w)] + [shadow, ema]
+
+
+SMALL = dict(hidden=128, layers=1, seq=16, batch=4, heads=2)
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("pairs", [1, 2, 37, 1030])  # 1030: more than one element per thread of the shaping kernel
+def test_device_shaping_equals_the_host_function(mode, pairs):
+    """marks asks for the composed step, whose shaping is the host function; without it the step shapes on the device."""
+    from bitnet_nvfp4_b200 import population
+    results = []
+    for marks in (None, {}):
+        _, _, _, _, m = make(max_pairs=pairs, **SMALL)
+        losses = [population.es_step(m, 5, e, pairs, fitness_mode=mode, fitness_clip=1.5, marks=marks).cpu().numpy() for e in range(2)]
+        results.append(losses + state(m))
+    for a, b in zip(*results):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("pairs", [3, 17, 40])
+def test_noise_sums_from_tables_equal_the_hashed_ones(pairs):
+    """A process that evaluated every pair finds the vectors' noise in memory; one that evaluated none hashes it."""
+    import torch
+    w = torch.linspace(-0.5, 0.5, pairs, device="cuda")
+    w[pairs // 2] = 0.0
+    out = []
+    for count in (pairs, 0):
+        _, _, _, _, m = make(max_pairs=pairs, **SMALL)
+        m.prepare_step_range(9, 1, pairs, 0, count)
+        m.update(w, lr=0.7, thresh=0.001)
+        out.append(state(m))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("kw", [dict(SMALL), dict(hidden=192, layers=2, mlp_mult=3, seq=9, batch=3, heads=3, rank=2), dict(hidden=64, layers=1, seq=32, batch=9, heads=1, rank=4)])
+def test_validation_after_an_update_matches_the_oracle(kw):
+    """The update renews the NVFP4 copies of the weights itself: the next forward (one unperturbed member) is the oracle's at the updated
+    weights. The last case is narrower than its vocabulary of 256."""
+    from bitnet_nvfp4_b200 import host, population
+    cfg, w, tok, tgt, m = make(max_pairs=6, **kw)
+    assert abs(m.eval_base().item() - oracle_loss(cfg, w, tok, tgt)) <= 1e-4 * 6
+    population.es_step(m, 1, 0, 6, lr=1.5, thresh=0.004)
+    after = m.get_weights()
+    assert any(not np.array_equal(after[n], w[n]) for n in ("wq", "ff1", "head"))
+    ref = oracle_loss(cfg, after, tok, tgt)
+    assert abs(m.eval_base().item() - ref) <= 1e-4 * abs(ref)
+    assert host.device_error() == 0
