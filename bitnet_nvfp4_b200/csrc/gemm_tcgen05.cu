@@ -15,12 +15,13 @@
 //   warps 2..17 epilogue: tcgen05.ld the accumulator (four warps per TMEM lane quadrant, 32 columns each), apply
 //               alpha/beta/rank-r/GELU, and store (TMA store through swizzled staging, or direct)
 // The kernel is persistent (one CTA per SM, tiles assigned round-robin): the producer runs up to four k-blocks
-// ahead, and two TMEM accumulators let the MMAs of tile i+1 overlap the epilogue of tile i. Every mbarrier wait is bounded: on expiry the kernel records an error
+// ahead (long K: CTA pairs on 256 x 256 tiles, see PAIR below), and two TMEM accumulators let the MMAs of tile i+1 overlap the epilogue of tile i. Every mbarrier wait is bounded: on expiry the kernel records an error
 // word, leaves its role loop, frees TMEM and returns.
 
 #include <cuda.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -54,6 +55,20 @@ constexpr int kSmemLora = kSmemEpi + kEpiWarps * kEpiBufBytes;
 constexpr int kSmemBar = kSmemLora + kEpiWarps * 4 * 32 * 4;  // per epilogue warp: [4][32] floats of the pair's A factor
 constexpr int kSmemTotal = kSmemBar + 128;
 constexpr int kSmemAlloc = kSmemTotal + 1024;  // slack for manual 1024-byte alignment
+
+// CTA-pair instances (PAIR): two CTAs of a cluster share one 256 x 256 tile. Per stage a CTA holds its 128 rows of A, its half of
+// the 256 B rows, the scale atoms of its A rows and those of all 256 B rows.
+constexpr int kPairStageBBytes = 2 * 64 * 128;
+constexpr int kPairStageSfbBytes = 2 * kStageSfBytes;
+constexpr int kPairSmemSfa = kSmemB + kStages * kPairStageBBytes;
+constexpr int kPairSmemSfb = kPairSmemSfa + kStages * kStageSfBytes;
+constexpr int kPairSmemEpi = kPairSmemSfb + kStages * kPairStageSfbBytes;
+constexpr int kPairSmemLora = kPairSmemEpi + kEpiWarps * kEpiBufBytes;
+constexpr int kPairSmemBar = kPairSmemLora + kEpiWarps * 4 * 32 * 4;
+constexpr int kPairSmemAlloc = kPairSmemBar + 128 + 1024;
+constexpr int kPairAcc = 3;                 // accumulator blocks of 128 columns: even tiles fill the first two, odd ones the last two
+constexpr int kPairSfCol = kPairAcc * 128;  // two scale slots of 16 (A) + 32 (B) columns behind them
+static_assert(kPairSmemAlloc <= 232448 && kSmemAlloc <= 232448, "shared memory of one SM");
 
 constexpr long long kWaitCycles = 2000000000LL;  // ~1 s bound on every mbarrier wait
 
@@ -158,6 +173,55 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
+// ---- CTA-pair forms (cta_group::2): issued by the leading CTA (rank 0), they act on both CTAs of the pair
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// the address of the same shared-memory location in the leading CTA
+__device__ __forceinline__ uint32_t map_to_leader(uint32_t addr) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// a tile into this CTA's shared memory, counted by the leading CTA's barrier
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t leader_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(leader_bar)
+        : "memory");
+}
+// (no memory travels with this arrival: it hands back TMEM columns, ordered by tcgen05.fence)
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// arrives at this barrier of both CTAs
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
+}
+__device__ __forceinline__ void tc_cp_sf_pair(uint32_t taddr, uint64_t sdesc) {
+    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+}
+__device__ __forceinline__ void tc_mma_nvf4_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t tsfa, uint32_t tsfb,
+                                                 uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
 // prmt.b32 in its default mode: a selector nibble with bit 3 set replicates the sign of the selected byte
 __device__ __forceinline__ uint32_t prmt_b32(uint32_t a, uint32_t b, uint32_t sel) {
     uint32_t d;
@@ -197,6 +261,15 @@ constexpr uint32_t kLayoutNone = 0, kLayoutSw128 = 2;
 // K-major A and B, N>>3 at bit 17, ue4m3 scales (bit 23 = 0), M>>4 at bit 24, scale ids 0, dense K = 64.
 constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(BM >> 4) << 24);
 
+constexpr uint32_t kIdescPairM = (1u << 7) | (1u << 10) | (static_cast<uint32_t>(2 * BM >> 4) << 24);                 // M 256 ...
+constexpr uint32_t kIdescPair256 = kIdescPairM | (256u >> 3 << 17), kIdescPair128 = kIdescPairM | (128u >> 3 << 17);  // ... x N 256 / N 128
+
+// Scale atoms as rows of 512 bytes (the pair instances fetch them with tiled copies, which can signal the leading CTA's barrier).
+struct PairMaps {
+    CUtensorMap sfa, sfb;
+};
+struct NoMaps {};
+
 struct KernelArgs {
     GemmParams p;
     int use_tma_store;
@@ -204,7 +277,7 @@ struct KernelArgs {
     uint32_t group_magic;  // ceil(2^32 / group_cols) (0 when group_cols == 0)
     const uint8_t* lut;  // table of the block quantiser (EPI_GELU_FP4)
     int total_tiles;
-    int n_tiles;  // tiles along N; blockIdx.x = m_tile * n_tiles + n_tile (N fastest: CTAs that share A rows run together)
+    int n_tiles;  // tiles along N (of 256 columns in the pair instances); blockIdx.x = m_tile * n_tiles + n_tile (N fastest: CTAs that share A rows run together)
 };
 
 // One lane of a converged warp (the same one every time in practice). The role loops below run in all 32 lanes with
@@ -226,11 +299,20 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // RK: 4 = the instance for rank-4 perturbation terms (its epilogue applies the four factors with packed multiply-adds);
 // 1 = the instance for the batched driver's common case (rank 1, no C operand, every 128-row tile inside one member), which carries
 // none of the general paths; 0 = everything else.
-template <int EPI, int RK>
+// PAIR: the instance for operands with many K blocks. On the in-order pipe a scale copy costs about 44 cycles and an M 128 x N 128 MMA
+// 64 (measured, one CTA): 8 copies and 4 MMAs per 256-element K block of a 128 x 128 tile take 560 cycles before any operand
+// traffic, 860 with it. A CTA pair (cta_group::2) on a 256 x 256 tile needs 12 copies and 4 MMAs of N 256 for four times the work; the
+// long MMAs hide most of the copies: 718 cycles (968 with twice as many N 128 MMAs), and each CTA loads 38 instead of 68 KB.
+// Accumulators: even tiles use the 128-column blocks 0 and 1, odd tiles 1 and 2, and the epilogue drains block 1 first, so that the
+// next tile starts as soon as the shared block has been read. The epilogue code sees a sequence of 128 x 128 sub-tiles.
+template <int EPI, int RK, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                  const __grid_constant__ CUtensorMap map_b,
                                                                  const __grid_constant__ CUtensorMap map_d,
+                                                                 const __grid_constant__ std::conditional_t<PAIR, PairMaps, NoMaps> maps_sf,
                                                                  const KernelArgs args) {
+    constexpr int kAcc = PAIR ? kPairAcc : 2;  // TMEM accumulators
+    constexpr int oSmemEpi = PAIR ? kPairSmemEpi : kSmemEpi, oSmemLora = PAIR ? kPairSmemLora : kSmemLora, oSmemBar = PAIR ? kPairSmemBar : kSmemBar;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -241,35 +323,148 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
     const int num_ks = (p.k + BK - 1) / BK;
     const int total_tiles = args.total_tiles;
 
-    const uint32_t bar_full = smem_base + kSmemBar;               // kStages x 8 bytes
+    const uint32_t bar_full = smem_base + oSmemBar;               // kStages x 8 bytes (PAIR: the leading CTA's count for both)
     const uint32_t bar_empty = bar_full + 8 * kStages;            // kStages x 8 bytes
-    const uint32_t bar_acc_full = bar_empty + 8 * kStages;        // 2 x 8 bytes
-    const uint32_t bar_acc_empty = bar_acc_full + 16;             // 2 x 8 bytes
-    const uint32_t tmem_slot = bar_acc_empty + 16;                // 4 bytes
-    volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(smem_gen + kSmemBar + 16 * kStages + 32);
+    const uint32_t bar_acc_full = bar_empty + 8 * kStages;        // kAcc x 8 bytes
+    const uint32_t bar_acc_empty = bar_acc_full + 8 * kAcc;       // kAcc x 8 bytes (PAIR: likewise)
+    const uint32_t tmem_slot = bar_acc_empty + 8 * kAcc;          // 4 bytes
+    volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(smem_gen + oSmemBar + 16 * kStages + 16 * kAcc);
+    uint32_t rank = 0;  // of this CTA in its pair
+    if constexpr (PAIR) rank = cluster_rank();
+    // the tiles this CTA (or pair) walks: unit, unit + units, ..
+    const unsigned unit = PAIR ? blockIdx.x >> 1 : blockIdx.x, units = PAIR ? gridDim.x >> 1 : gridDim.x;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(bar_full + 8 * s, 1);
             mbar_init(bar_empty + 8 * s, 1);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < kAcc; ++b) {
             mbar_init(bar_acc_full + 8 * b, 1);
-            mbar_init(bar_acc_empty + 8 * b, kEpiWarps);
+            mbar_init(bar_acc_empty + 8 * b, PAIR ? 2 * kEpiWarps : kEpiWarps);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        tmem_alloc(tmem_slot, kTmemCols);
-        tmem_relinquish();
+        if constexpr (PAIR) {
+            tmem_alloc_pair(tmem_slot, kTmemCols);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(tmem_slot, kTmemCols);
+            tmem_relinquish();
+        }
     }
     tc_fence_before();
-    __syncthreads();
+    if constexpr (PAIR) cluster_sync();  // the peer's barriers exist before anything signals them
+    else __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot_gen;
     pdl_wait();  // the set-up above overlaps the predecessor's tail; everything below reads what it wrote
 
-    if (warp == 0) {
+    if (PAIR && warp == 0) {
+        // ------------------------------ producer of one half of a pair ------------------------------
+        if constexpr (PAIR) {
+            int kc = 0, s = 0;
+            uint32_t empty_parity = 1;
+            bool ok = true;
+            for (unsigned tile = unit; tile < static_cast<unsigned>(total_tiles) && ok; tile += units) {
+                const int mt = static_cast<int>(tile / static_cast<unsigned>(args.n_tiles)), nt = static_cast<int>(tile - static_cast<unsigned>(mt) * static_cast<unsigned>(args.n_tiles));
+                const bool two = nt * 256 + 128 < p.n;  // the second half has columns
+                // each CTA holds half of the B rows of the pair's MMA: 128 of 256, or 64 of 128
+                const int my = mt * 256 + static_cast<int>(rank) * BM, ny = nt * 256 + static_cast<int>(rank) * (two ? 128 : 64);
+                const int sfa_row = (my >> 7) * args.k_atoms, sfb_row = nt * 2 * args.k_atoms;
+                const uint32_t bytes = 2u * (kStageABytes + kStageSfBytes + (two ? 2u : 1u) * (64 * 128 + kStageSfBytes));
+                for (int ks = 0; ks < num_ks; ++ks, ++kc) {
+                    if (kc >= kStages) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, empty_parity, 1));
+                        if (!ok) break;
+                    }
+                    if (elect_one()) {
+                        const uint32_t bar = map_to_leader(bar_full + 8 * s);
+                        if (rank == 0) mbar_expect_tx(bar_full + 8 * s, bytes);
+                        tma_load_2d_pair(smem_base + kSmemA + s * kStageABytes, &map_a, ks * 128, my, bar);
+                        tma_load_2d_pair(smem_base + kSmemB + s * kPairStageBBytes, &map_b, ks * 128, ny, bar);
+                        tma_load_2d_pair(smem_base + kPairSmemSfa + s * kStageSfBytes, &maps_sf.sfa, 0, sfa_row + 4 * ks, bar);
+                        tma_load_2d_pair(smem_base + kPairSmemSfb + s * kPairStageSfbBytes, &maps_sf.sfb, 0, sfb_row + 4 * ks, bar);
+                        if (two) {
+                            tma_load_2d_pair(smem_base + kSmemB + s * kPairStageBBytes + 64 * 128, &map_b, ks * 128, ny + 64, bar);
+                            tma_load_2d_pair(smem_base + kPairSmemSfb + s * kPairStageSfbBytes + kStageSfBytes, &maps_sf.sfb, 0, sfb_row + args.k_atoms + 4 * ks, bar);
+                        }
+                    }
+                    __syncwarp();
+                    if (++s == kStages) { s = 0; empty_parity ^= 1u; }
+                }
+            }
+            // the last stages' releases arrive from the leading CTA: wait for them, so that none is in flight towards a CTA that has left
+            for (int i = 0; i < min(kc, kStages) && ok; ++i) {
+                if (kc < kStages) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * i, 0, 1));
+                else {
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, empty_parity, 1));
+                    if (++s == kStages) { s = 0; empty_parity ^= 1u; }
+                }
+            }
+        }
+    } else if (PAIR && warp == 1) {
+        // ------------------------------ MMA issuer: the leading CTA's warp works for both ------------------------------
+        if constexpr (PAIR) {
+            const uint64_t adesc0 = smem_desc(smem_base + kSmemA, 16, 1024, kLayoutSw128);
+            const uint64_t bdesc0 = smem_desc(smem_base + kSmemB, 16, 1024, kLayoutSw128);
+            const uint64_t sfadesc0 = smem_desc(smem_base + kPairSmemSfa, 0, 128, kLayoutNone);
+            const uint64_t sfbdesc0 = smem_desc(smem_base + kPairSmemSfb, 0, 128, kLayoutNone);
+            int s = 0;
+            uint32_t full_parity = 0, kc = 0, odd = 0;
+            uint32_t empty_par = 0, used = 0;  // per accumulator block (bit): parity of the drain to wait for next; whether it was used before
+            bool ok = rank == 0;
+            for (unsigned tile = unit; tile < static_cast<unsigned>(total_tiles) && ok; tile += units, odd ^= 1u) {
+                const int nt = static_cast<int>(tile % static_cast<unsigned>(args.n_tiles));
+                const bool two = nt * 256 + 128 < p.n;
+                // both CTAs' epilogues must have drained the blocks
+                for (uint32_t b = odd; b <= odd + (two ? 1u : 0u) && ok; ++b) {
+                    if ((used >> b) & 1u) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty + 8 * b, (empty_par >> b) & 1u, 4));
+                        empty_par ^= 1u << b;
+                    }
+                    used |= 1u << b;
+                }
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t acc = tmem_base + odd * 128, idesc = two ? kIdescPair256 : kIdescPair128;
+                for (int ks = 0; ks < num_ks; ++ks, ++kc) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * s, full_parity, 2));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const int nk = min(4, (p.k - ks * BK) / UMMA_K);
+                    const uint32_t t_sfa = tmem_base + kPairSfCol + (kc & 1u) * 48, t_sfb = t_sfa + 16;  // the pipe is in order: two slots suffice
+                    const uint64_t sfa_d = sfadesc0 + static_cast<uint64_t>(s * (kStageSfBytes >> 4)), sfb_d = sfbdesc0 + static_cast<uint64_t>(s * (kPairStageSfbBytes >> 4));
+                    const uint64_t a_d = adesc0 + static_cast<uint64_t>(s * (kStageABytes >> 4)), b_d = bdesc0 + static_cast<uint64_t>(s * (kPairStageBBytes >> 4));
+                    if (elect_one()) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            if (j < nk) {
+                                tc_cp_sf_pair(t_sfa + 4 * j, sfa_d + static_cast<uint64_t>(j * (512 >> 4)));
+                                tc_cp_sf_pair(t_sfb + 8 * j, sfb_d + static_cast<uint64_t>(j * (512 >> 4)));
+                                if (two) tc_cp_sf_pair(t_sfb + 8 * j + 4, sfb_d + static_cast<uint64_t>((kStageSfBytes + j * 512) >> 4));
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            if (j < nk) {
+                                const uint64_t kj = static_cast<uint64_t>(j * (32 >> 4));
+                                tc_mma_nvf4_pair(acc, a_d + kj, b_d + kj, idesc, t_sfa + 4 * j, t_sfb + 8 * j, ks > 0 || j > 0 ? 1u : 0u);
+                            }
+                        }
+                        tc_commit_pair(bar_empty + 8 * s);
+                        if (ks == num_ks - 1) {
+                            tc_commit_pair(bar_acc_full + 8 * odd);
+                            if (two) tc_commit_pair(bar_acc_full + 8 * odd + 8);
+                        }
+                    }
+                    __syncwarp();
+                    if (++s == kStages) { s = 0; full_parity ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == 0) {
         // ------------------------------ producer ------------------------------
         {
             // running indices instead of divisions, addresses advanced by constants
@@ -378,15 +573,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         const int ew = warp - 2;   // 0..15
         const int q = warp & 3;    // TMEM lane quadrant this warp may access
         const int c = ew >> 2;     // 32-column chunk of the tile handled by this warp
-        const uint32_t epi_buf = smem_base + kSmemEpi + ew * kEpiBufBytes;
-        uint8_t* epi_gen = smem_gen + kSmemEpi + ew * kEpiBufBytes;
+        const uint32_t epi_buf = smem_base + oSmemEpi + ew * kEpiBufBytes;
+        uint8_t* epi_gen = smem_gen + oSmemEpi + ew * kEpiBufBytes;
         bool ok = true;
         int it = 0;
         int stage_half = 0;  // EPI_F16: which half of the staging buffer the next store uses
         if constexpr (EPI == EPI_GELU_FP4) {
             // The block quantiser's table ({1 / scale, scale byte} per amax, 1 KB) lives in the staging area the fp32 epilogue would use.
             if (ew * 32 + lane < 128)
-                reinterpret_cast<uint2*>(smem_gen + kSmemEpi)[ew * 32 + lane] =
+                reinterpret_cast<uint2*>(smem_gen + oSmemEpi)[ew * 32 + lane] =
                     __ldg(reinterpret_cast<const uint2*>(args.lut + kQuantBlockTabOffset) + ew * 32 + lane);
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
         }
@@ -403,13 +598,33 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         };
         const int row_in_tile = q * 32 + lane;
         // Tile coordinates advance by additions (tiles are walked in steps of gridDim.x): no division per tile.
-        const int step_n = static_cast<int>(gridDim.x % static_cast<unsigned>(args.n_tiles)), step_m = static_cast<int>(gridDim.x / static_cast<unsigned>(args.n_tiles));
-        struct TileIdx { int m_tile, n_tile; };
-        auto advance = [&](TileIdx& t) {
-            t.n_tile += step_n;
-            t.m_tile += step_m;
-            if (t.n_tile >= args.n_tiles) { t.n_tile -= args.n_tiles; ++t.m_tile; }
+        const int step_n = static_cast<int>(units % static_cast<unsigned>(args.n_tiles)), step_m = static_cast<int>(units / static_cast<unsigned>(args.n_tiles));
+        // m_tile counts 128-row tiles (of a pair's tile: this CTA's), n_tile 128-column tiles; the halves of a pair's tile follow each other.
+        // PAIR: `odd` = parity of the tile, `last` = no further half follows in this tile.
+        struct TileIdx { int m_tile, n_tile, odd; bool last; };
+        auto first_half = [&](TileIdx& t, int nt) {  // of tile column nt: the half in the shared accumulator block
+            const bool two = nt * 256 + 128 < p.n;
+            t.n_tile = 2 * nt + (two && t.odd == 0 ? 1 : 0);
+            t.last = !two;
         };
+        auto advance = [&](TileIdx& t) {
+            if constexpr (PAIR) {
+                if (!t.last) { t.n_tile ^= 1; t.last = true; return; }
+                int nt = (t.n_tile >> 1) + step_n;
+                t.m_tile += 2 * step_m;
+                if (nt >= args.n_tiles) { nt -= args.n_tiles; t.m_tile += 2; }
+                t.odd ^= 1;
+                first_half(t, nt);
+            } else {
+                t.n_tile += step_n;
+                t.m_tile += step_m;
+                if (t.n_tile >= args.n_tiles) { t.n_tile -= args.n_tiles; ++t.m_tile; }
+            }
+        };
+        const int m_end = PAIR ? 2 * (total_tiles / args.n_tiles) : 0;  // first 128-row tile behind the matrix, pairs rounded up
+        auto in_range = [&](const TileIdx& t) { return t.m_tile < m_end; };
+        // a pair's second CTA may have no rows left in the last tile: it has nothing to fetch then
+        auto has_rows = [&](const TileIdx& t) { return t.m_tile < m_end && t.m_tile * BM < p.m; };
         // Members are visited in ascending order, so when tiles never straddle members (rows_per_member a multiple of the
         // tile height) the member of the next tile is tracked with comparisons instead of a division per row.
         const bool tile_uniform_member = p.rows_per_member > 0 && (p.rows_per_member % BM) == 0;
@@ -490,7 +705,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             }
             if (col0_ + lane < p.n) cx.aval[0] = __ldg(p.lora_A + static_cast<size_t>(cx.pair) * p.lora_A_pair_stride + col0_ + lane);
         };
-        TileIdx cur_t{static_cast<int>(blockIdx.x / static_cast<unsigned>(args.n_tiles)), static_cast<int>(blockIdx.x % static_cast<unsigned>(args.n_tiles))};
+        TileIdx cur_t{static_cast<int>(unit / static_cast<unsigned>(args.n_tiles)), static_cast<int>(unit % static_cast<unsigned>(args.n_tiles)), 0, true};
+        if constexpr (PAIR) {
+            cur_t.m_tile = 2 * cur_t.m_tile + static_cast<int>(rank);
+            first_half(cur_t, cur_t.n_tile);
+        }
         TileIdx nxt_t = cur_t;
         // EPI_ADD_I8 through TMA: this warp's 32 x 32-byte box of the residual stream is loaded one tile ahead into one of
         // three 1 KB buffers (each with its own mbarrier), updated in place and stored from there. A lane-per-row access to
@@ -521,18 +740,22 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     fence_async_smem();
                 }
                 __syncwarp();
-                issue_res_load(cur_t, static_cast<int>(blockIdx.x) < total_tiles);
+                issue_res_load(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles);
             }
         }
         LoraCtx nxt;
         nxt.tr[1] = nxt.tr[2] = nxt.tr[3] = 0;
         nxt.aval[1] = nxt.aval[2] = nxt.aval[3] = 0;
-        if (R1 || fast_ctx) fetch_fast(cur_t, static_cast<int>(blockIdx.x) < total_tiles, nxt);
-        else fetch_ctx(cur_t, static_cast<int>(blockIdx.x) < total_tiles, nxt);
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++it) {
-            const int buf = it & 1;
+        if (R1 || fast_ctx) fetch_fast(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles, nxt);
+        else fetch_ctx(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles, nxt);
+        uint32_t pfull = 0;  // PAIR: parities of the completions to wait for (bit per accumulator block)
+        uint32_t acc_empty_bar = bar_acc_empty;
+        if constexpr (PAIR) acc_empty_bar = map_to_leader(bar_acc_empty);
+        for (int tile = blockIdx.x; (PAIR ? in_range(nxt_t) : tile < total_tiles) && ok; tile += gridDim.x, ++it) {
             cur_t = nxt_t;
+            const int buf = PAIR ? (cur_t.n_tile & 1) + cur_t.odd : it & 1;
             advance(nxt_t);
+            const bool more = PAIR ? has_rows(nxt_t) : tile + static_cast<int>(gridDim.x) < total_tiles;
             const int m0 = cur_t.m_tile * BM, n0 = cur_t.n_tile * BN;
             const long long row = static_cast<long long>(m0) + row_in_tile;
             const bool row_ok = R1 || row < p.m;  // (the rank-1 instance runs with m a multiple of the tile height)
@@ -543,12 +766,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             const float lsign = nxt.lsign;
             float tr[4] = {static_cast<float>(nxt.tr[0]), 0.0f, 0.0f, 0.0f};
             const bool a_staged = nxt.a_staged;
-            float* loraA_sh = reinterpret_cast<float*>(smem_gen + kSmemLora) + ew * 4 * 32;  // this warp's [4][32]
+            float* loraA_sh = reinterpret_cast<float*>(smem_gen + oSmemLora) + ew * 4 * 32;  // this warp's [4][32]
             if (R1 || fast_ctx) {
                 __syncwarp();  // the previous tile's reads are done
                 loraA_sh[lane] = static_cast<float>(nxt.aval[0]);
                 __syncwarp();
-                fetch_fast(nxt_t, tile + static_cast<int>(gridDim.x) < total_tiles, nxt);
+                fetch_fast(nxt_t, more, nxt);
             } else if (p.rank > 0) {
                 tr[1] = static_cast<float>(nxt.tr[1]);
                 tr[2] = static_cast<float>(nxt.tr[2]);
@@ -560,7 +783,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                         if (r < p.rank) loraA_sh[r * 32 + lane] = static_cast<float>(nxt.aval[r]);
                 }
                 __syncwarp();
-                fetch_ctx(nxt_t, tile + static_cast<int>(gridDim.x) < total_tiles, nxt);
+                fetch_ctx(nxt_t, more, nxt);
             }
 
             // EPI_ADD_I8: this thread's 32 bytes of the residual stream, requested before the wait for the accumulator
@@ -570,7 +793,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 if (res_tma) {
                     have_cur = have_nxt;
                     rb_cur = rb_last;
-                    issue_res_load(nxt_t, tile + static_cast<int>(gridDim.x) < total_tiles);
+                    issue_res_load(nxt_t, more);
                 } else if (row_ok && chunk_ok) {
                     const int8_t* xr = p.resid + static_cast<size_t>(row) * p.ld_resid + col0;
                     res_vec = ((reinterpret_cast<uintptr_t>(xr) & 15) == 0) && (col0 + 32 <= p.n);
@@ -581,10 +804,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 }
             }
 
-            ok = mbar_wait(bar_acc_full + 8 * buf, (it >> 1) & 1, 3);
+            ok = mbar_wait(bar_acc_full + 8 * buf, PAIR ? (pfull >> buf) & 1u : (it >> 1) & 1, 3);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
+            if constexpr (PAIR) pfull ^= 1u << buf;
 
             uint32_t acc[32];
             tmem_ld32(tmem_base + kAccCol + buf * BN + (static_cast<uint32_t>(q * 32) << 16) + c * 32, acc);
@@ -592,7 +816,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             // this warp no longer needs the accumulator: hand it back to the MMA warp
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);
+            if (lane == 0) {
+                if constexpr (PAIR) mbar_arrive_remote(acc_empty_bar + 8 * buf);
+                else mbar_arrive(bar_acc_empty + 8 * buf);
+            }
             if (!chunk_ok) continue;
 
             float v[32];
@@ -793,7 +1020,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 // values still biased by 1.5 * 2^23: the low byte of the bit pattern is the int8.
                 const bool lower_clamp = !R1 && p.act_scale > 700.0f;  // gelu(x) >= -0.17 |x|: only a huge act_scale reaches -127 (those calls run the general instance)
                 // entry address from the bit pattern of (amax + kRoundBias): (bits - kRoundBiasBits) * 8, folded into one constant
-                const uint32_t tab_c = smem_base + kSmemEpi - (static_cast<uint32_t>(kRoundBiasBits) << 3);
+                const uint32_t tab_c = smem_base + oSmemEpi - (static_cast<uint32_t>(kRoundBiasBits) << 3);
                 int w[8];
                 uint32_t sfv[2] = {0u, 0u}, codes[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
@@ -883,10 +1110,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
     }
 
     tc_fence_before();
-    __syncthreads();
+    if constexpr (PAIR) cluster_sync();  // neither CTA leaves while the other may still signal or read it
+    else __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, kTmemCols);
+        if constexpr (PAIR) tmem_dealloc_pair(tmem_base, kTmemCols);
+        else tmem_dealloc(tmem_base, kTmemCols);
     }
 }
 
@@ -954,17 +1183,33 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint
     return BNF4_OK;
 }
 
-template <int EPI, int RK>
-int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, const KernelArgs& args, dim3 grid, int dev,
-             cudaStream_t stream) {
+template <int EPI, int RK, bool PAIR = false>
+int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, const std::conditional_t<PAIR, PairMaps, NoMaps>& msf, const KernelArgs& args,
+             dim3 grid, int dev, cudaStream_t stream) {
+    constexpr int smem = PAIR ? kPairSmemAlloc : kSmemAlloc;
     static bool configured[64] = {};  // function attributes are per device: set once for each device this process uses
     if (!configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_nvfp4_kernel<EPI, RK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAlloc);
+        const cudaError_t e = cudaFuncSetAttribute(gemm_nvfp4_kernel<EPI, RK, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(gemm_nvfp4_kernel)");
         configured[dev] = true;
     }
-    // (an early launch pays while the kernel is short: a dozen tiles per SM)
-    launch_pdl_if(args.total_tiles <= 12 * static_cast<int>(grid.x), gemm_nvfp4_kernel<EPI, RK>, grid, kThreads, kSmemAlloc, stream, ma, mb, md, args);
+    if constexpr (PAIR) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = grid;
+        cfg.blockDim = kThreads;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, gemm_nvfp4_kernel<EPI, RK, PAIR>, ma, mb, md, msf, args);
+    } else {
+        // (an early launch pays while the kernel is short: a dozen tiles per SM)
+        launch_pdl_if(args.total_tiles <= 12 * static_cast<int>(grid.x), gemm_nvfp4_kernel<EPI, RK, PAIR>, grid, kThreads, smem, stream, ma, mb, md, msf, args);
+    }
     return check_launch("gemm_nvfp4_kernel");
 }
 
@@ -1046,18 +1291,49 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     if (rc) return rc;
     const int sms = multiprocessors(dev);
     if (sms <= 0) return BNF4_ERR_CUDA;
-    const dim3 grid(static_cast<unsigned>(std::min<long long>(tiles, sms)), 1, 1);
     const bool gelu = p.epilogue == EPI_GELU_FP4 || p.epilogue == EPI_GELU_I8;
     const bool gelu_plain = !gelu || (p.act_scale <= 700.0f && (p.n % 32) == 0 && (p.epilogue == EPI_GELU_FP4 ? (p.next_nvec == 1 && p.d_i8 == nullptr) : p.next_nvec <= 1));
     const int rk = p.rank == 4 ? 4 : ((p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1)) ? 1 : 0);
-    switch (p.epilogue) {
-        case EPI_F32: return rk == 4 ? launch_t<EPI_F32, 4>(ma, mb, md, args, grid, dev, stream) : (rk == 1 ? launch_t<EPI_F32, 1>(ma, mb, md, args, grid, dev, stream) : launch_t<EPI_F32, 0>(ma, mb, md, args, grid, dev, stream));
-        case EPI_GELU_I8: return rk == 4 ? launch_t<EPI_GELU_I8, 4>(ma, mb, md, args, grid, dev, stream) : (rk == 1 ? launch_t<EPI_GELU_I8, 1>(ma, mb, md, args, grid, dev, stream) : launch_t<EPI_GELU_I8, 0>(ma, mb, md, args, grid, dev, stream));
-        case EPI_GELU_FP4: return rk == 4 ? launch_t<EPI_GELU_FP4, 4>(ma, mb, md, args, grid, dev, stream) : (rk == 1 ? launch_t<EPI_GELU_FP4, 1>(ma, mb, md, args, grid, dev, stream) : launch_t<EPI_GELU_FP4, 0>(ma, mb, md, args, grid, dev, stream));
-        case EPI_ADD_I8: return rk == 4 ? launch_t<EPI_ADD_I8, 4>(ma, mb, md, args, grid, dev, stream) : (rk == 1 ? launch_t<EPI_ADD_I8, 1>(ma, mb, md, args, grid, dev, stream) : launch_t<EPI_ADD_I8, 0>(ma, mb, md, args, grid, dev, stream));
-        case EPI_F16: return rk == 4 ? launch_t<EPI_F16, 4>(ma, mb, md, args, grid, dev, stream) : (rk == 1 ? launch_t<EPI_F16, 1>(ma, mb, md, args, grid, dev, stream) : launch_t<EPI_F16, 0>(ma, mb, md, args, grid, dev, stream));
+    // CTA pairs pay where the mainloop is longer than the epilogue and there is a tile for every pair. Measured at 65536 x 512 (us, single
+    // CTAs -> pairs): fp32 / half / residual epilogues, rank 1: K 512 33.9 -> 35.9, 25.6 -> 27.0, 29.0 -> 29.8; K 1024 42.7 -> 38.2,
+    // 33.1 -> 30.2, 36.1 -> 33.1; K 4096 107 -> 80, 96 -> 70, 98 -> 74. Rank 4 with the last two: K 1024 37.2 -> 39.2, 43.3 -> 45.4, K 1536
+    // 46.8 -> 43.3, 49.5 -> 47.4. GELU epilogues, whose math takes as long as K 1536: K 1536 52.7 -> 54.6, K 2048 63.8 -> 59.9, K 4096 105 -> 82.
+    const long long pair_tiles = static_cast<long long>((p.n + 255) / 256) * ((p.m + 255) / 256);
+    const int pair_k = gelu ? 2048 : (p.rank > 1 && p.epilogue != EPI_F32 ? 1536 : 1024);
+    const bool pair = p.k >= pair_k && pair_tiles >= sms / 2 && (rk != 1 || (p.m % 256) == 0);
+    // the epilogue (and with it the kernel) is a template argument
+    auto with_epilogue = [&](auto run) -> int {
+        switch (p.epilogue) {
+            case EPI_F32: return run(std::integral_constant<int, EPI_F32>());
+            case EPI_GELU_I8: return run(std::integral_constant<int, EPI_GELU_I8>());
+            case EPI_GELU_FP4: return run(std::integral_constant<int, EPI_GELU_FP4>());
+            case EPI_ADD_I8: return run(std::integral_constant<int, EPI_ADD_I8>());
+            case EPI_F16: return run(std::integral_constant<int, EPI_F16>());
+        }
+        return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: unknown epilogue %d", p.epilogue);
+    };
+    if (pair) {
+        PairMaps msf;
+        rc = make_map_2d(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.b, static_cast<uint64_t>(p.k) / 2, static_cast<uint64_t>(p.n), static_cast<uint64_t>(p.k) / 2, 128, 64, "B (pair)");
+        if (!rc) rc = make_map_2d(&msf.sfa, CU_TENSOR_MAP_DATA_TYPE_UINT32, p.sfa, 128, static_cast<uint64_t>((p.m + 127) / 128) * args.k_atoms, 512, 128, 4, "A scales", CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (!rc) rc = make_map_2d(&msf.sfb, CU_TENSOR_MAP_DATA_TYPE_UINT32, p.sfb, 128, static_cast<uint64_t>((p.n + 127) / 128) * args.k_atoms, 512, 128, 4, "B scales", CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (rc) return rc;
+        args.n_tiles = (p.n + 255) / 256;
+        args.total_tiles = static_cast<int>(pair_tiles);
+        const dim3 grid(2 * static_cast<unsigned>(std::min<long long>(pair_tiles, sms / 2)), 1, 1);
+        return with_epilogue([&](auto epi) -> int {
+            constexpr int E = decltype(epi)::value;
+            return rk == 4 ? launch_t<E, 4, true>(ma, mb, md, msf, args, grid, dev, stream)
+                           : (rk == 1 ? launch_t<E, 1, true>(ma, mb, md, msf, args, grid, dev, stream) : launch_t<E, 0, true>(ma, mb, md, msf, args, grid, dev, stream));
+        });
     }
-    return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: unknown epilogue %d", p.epilogue);
+    const dim3 grid(static_cast<unsigned>(std::min<long long>(tiles, sms)), 1, 1);
+    return with_epilogue([&](auto epi) -> int {
+        constexpr int E = decltype(epi)::value;
+        const NoMaps none;
+        return rk == 4 ? launch_t<E, 4>(ma, mb, md, none, args, grid, dev, stream)
+                       : (rk == 1 ? launch_t<E, 1>(ma, mb, md, none, args, grid, dev, stream) : launch_t<E, 0>(ma, mb, md, none, args, grid, dev, stream));
+    });
 }
 
 int gemm_nvfp4_device_error(cudaStream_t stream, int* out_code) {

@@ -277,7 +277,8 @@ __global__ void __launch_bounds__(256) rowquant_kernel(const RowQuantParams p, c
 
 // ------------------------------------------------------------------------------------------------
 // Float-domain fast path for the front-ends the population forward runs once or twice per layer
-// (embedding + rank-r noise, + pos / GELU / abs-mean norm, residual add + abs-mean norm, abs-mean norm of int8 rows).
+// (embedding + rank-r noise, + pos / GELU / abs-mean norm, residual add + abs-mean norm, abs-mean norm of int8 rows), and for plain int8
+// rows and fp32 activations (16384 x 512 fp32 with one projection: 20.3 us in rowquant_kernel, one row per warp and CTA launch).
 //
 // Same results as rowquant_kernel, fewer and cheaper instructions: int8 values travel as exact small integers in
 // fp32 ("v"), or biased by 1.5 * 2^23 ("t = v + M", whose low byte is the int8), so that
@@ -353,6 +354,7 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
 
         // ---------------- stage 1: integer values of the row as floats ----------------
         float vf[NB][16];
+        uint32_t raw_w[FE == FE_INT8 ? NB : 1][4];  // FE_INT8: the row's bytes
         uint32_t sum_abs = 0;  // sum of |value| over this lane's elements (exact integer)
         int tok = 0;
         float a_r[4] = {0.f, 0.f, 0.f, 0.f};
@@ -375,7 +377,43 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
                 for (int e = 0; e < 16; ++e) vf[i][e] = 0.0f;
                 continue;
             }
-            if constexpr (FE == FE_ABSMEAN) {
+            if constexpr (FE == FE_INT8) {
+                const int4 raw = *reinterpret_cast<const int4*>(p.in_i8 + static_cast<size_t>(row) * p.ld_in + k0);
+                const uint32_t rw[4] = {static_cast<uint32_t>(raw.x), static_cast<uint32_t>(raw.y), static_cast<uint32_t>(raw.z), static_cast<uint32_t>(raw.w)};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    raw_w[i][q] = rw[q];  // the int8 copy and the projections take the bytes as they are
+                    bytes4_to_float(rw[q], &vf[i][4 * q]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) vf[i][4 * q + j] = fmaxf(vf[i][4 * q + j], -127.0f);  // -128 is quantised as -127
+                }
+            } else if constexpr (FE == FE_ACT) {
+                const float* src = p.in_f32 + static_cast<size_t>(row) * p.ld_in + k0;
+                float4 f4[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) f4[q] = __ldcs(reinterpret_cast<const float4*>(src) + q);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    float x[4] = {f4[q].x, f4[q].y, f4[q].z, f4[q].w};
+                    if (p.act_mode == 3) {
+                        float worst = 0.0f, tb[4], fc[4];
+                        gelu_q8_fast2(x[0], x[1], p.act_scale, true, worst, tb[0], tb[1], fc[0], fc[1]);
+                        gelu_q8_fast2(x[2], x[3], p.act_scale, true, worst, tb[2], tb[3], fc[2], fc[3]);
+                        if (!(worst < kGeluSafe)) gelu_q8_exact4(x[0], x[1], x[2], x[3], p.act_scale, tb, fc);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) vf[i][4 * q + j] = tb[j] - M;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            float y = x[j];
+                            if (p.act_mode == 1) y = y < 0.0f ? 0.0f : y;
+                            else if (p.act_mode == 2) y = tanhf(__fdiv_rn(y, 127.0f)) * 127.0f;
+                            const float r = (fminf(fmaxf(y, -127.0f), 127.0f) + M) - M;  // clip8(rint(y))
+                            vf[i][4 * q + j] = y != y ? 0.0f : r;                        // (an integer conversion turns NaN into 0)
+                        }
+                    }
+                }
+            } else if constexpr (FE == FE_ABSMEAN) {
                 const int4 raw = *reinterpret_cast<const int4*>(p.in_i8 + static_cast<size_t>(row) * p.ld_in + k0);
                 const uint32_t rw[4] = {static_cast<uint32_t>(raw.x), static_cast<uint32_t>(raw.y), static_cast<uint32_t>(raw.z), static_cast<uint32_t>(raw.w)};
 #pragma unroll
@@ -553,7 +591,10 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
                     }
                 }
 #pragma unroll
-                for (int q = 0; q < 4; ++q) w[q] = biased4_to_bytes(tq[4 * q], tq[4 * q + 1], tq[4 * q + 2], tq[4 * q + 3]);
+                for (int q = 0; q < 4; ++q) {
+                    if constexpr (FE == FE_INT8) w[q] = raw_w[i][q];
+                    else w[q] = biased4_to_bytes(tq[4 * q], tq[4 * q + 1], tq[4 * q + 2], tq[4 * q + 3]);
+                }
                 if (!MODEL && p.out_q != nullptr)
                     *reinterpret_cast<int4*>(p.out_q + static_cast<size_t>(row) * p.ld_q + k0) =
                         make_int4(static_cast<int>(w[0]), static_cast<int>(w[1]), static_cast<int>(w[2]), static_cast<int>(w[3]));
@@ -666,10 +707,11 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
     const uint8_t* lut = get_quant_lut();
     if (lut == nullptr) return BNF4_ERR_CUDA;
     const bool early = static_cast<long long>(p.rows) * p.cols_out <= kPdlStreamElems;
-    if constexpr (FE == FE_EMBED_LOWRANK || FE == FE_POS_GELU_ABSMEAN || FE == FE_ADD_ABSMEAN || FE == FE_ABSMEAN) {
+    if constexpr (FE == FE_EMBED_LOWRANK || FE == FE_POS_GELU_ABSMEAN || FE == FE_ADD_ABSMEAN || FE == FE_ABSMEAN || FE == FE_ACT || FE == FE_INT8) {
         auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
         bool fast = p.cols_in == p.cols_out && nblk <= 128 && (p.out_q == nullptr || p.vec_ok_q) && al16(p.inout_i8 ? p.inout_i8 : nullptr);
-        if (FE == FE_ABSMEAN) fast = fast && p.vec_ok && p.in_i8 != nullptr;
+        if (FE == FE_ABSMEAN || FE == FE_INT8) fast = fast && p.vec_ok && p.in_i8 != nullptr;
+        if (FE == FE_ACT) fast = fast && p.vec_ok && p.in_f32 != nullptr;
         if (FE == FE_ADD_ABSMEAN) fast = fast && al16(p.in_f32) && (p.ld_in % (p.in_f16 ? 8 : 4)) == 0;
         if (FE == FE_ADD_ABSMEAN && p.in_f16 && !fast) return set_error(BNF4_ERR_INVALID, "rowquant: fp16 input needs 16-byte aligned rows and cols_in == cols_out <= 2048");
         if (FE == FE_POS_GELU_ABSMEAN)
