@@ -260,11 +260,144 @@ int launch_generic(const EflaParams& p, cudaStream_t stream) {
     return check_launch("efla_generic_kernel");
 }
 
+// ------------------------------------------------------------------------------------------------
+// Heads of 32: one warp owns one (sequence, head), lane n column n of the state as 32 floats in registers (rounded to ST after every
+// token), so no token needs a block-wide barrier. Tokens come in groups of four: the next group's q, k, v are in flight while the
+// current one is processed, the eight row norms share one butterfly, and lane j of each quad runs the scalar chain of token j.
+// k, alpha k and q^ of the group sit in shared memory and are read as broadcasts; multiply-adds are packed pairs. Issue bound, about
+// 140 instructions per token: 13200 sequences of 204 tokens in 0.4 ms, against 2.9 ms with the state in shared memory and 15 ms with
+// the generic kernel, whose 256 threads have nothing to do for a 32 x 32 state.
+// ------------------------------------------------------------------------------------------------
+constexpr int kH32Warps = 4;
+
+template <typename ST>
+__global__ void __launch_bounds__(kH32Warps * 32) efla_head32_kernel(const EflaParams p) {
+    constexpr bool kHalf = sizeof(ST) == 2;
+    __shared__ __align__(16) float vec[kH32Warps][3][4][32];  // [warp][k | alpha k | q^][token][d]
+    pdl_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned unit = blockIdx.x * kH32Warps + warp;
+    if (unit >= p.seqs * static_cast<long long>(p.heads)) return;
+    const unsigned seq = unit / static_cast<unsigned>(p.heads);
+    const int h = static_cast<int>(unit - seq * static_cast<unsigned>(p.heads));
+    const size_t row0 = static_cast<size_t>(seq) * p.T;
+    const float* qb = static_cast<const float*>(p.q) + row0 * p.ld_qkv + h * 32 + lane;
+    const float* kb = static_cast<const float*>(p.k) + row0 * p.ld_qkv + h * 32 + lane;
+    const float* vb = static_cast<const float*>(p.v) + row0 * p.ld_qkv + h * 32 + lane;
+    const float* bb = p.beta_raw + row0 * p.ld_beta;
+    float* ob = static_cast<float*>(p.out) + row0 * p.ld_out + h * 32 + lane;
+    const float beta_bias = p.beta_bias_seq != nullptr ? p.beta_bias_seq[seq / static_cast<unsigned>(p.seqs_per_bias)] : p.beta_bias;
+
+    float2 S[16];  // rows 2 i, 2 i + 1
+    ST* Sg = p.state != nullptr ? reinterpret_cast<ST*>(p.state) + static_cast<size_t>(unit) * 1024 + lane : nullptr;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        S[i] = Sg != nullptr ? make_float2(static_cast<float>(Sg[(2 * i) * 32]), static_cast<float>(Sg[(2 * i + 1) * 32])) : make_float2(0.0f, 0.0f);
+
+    float qn[4], kn[4], vn[4], bn;
+    auto fetch = [&](int t0) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const bool ok = t0 + j < p.T;
+            const size_t o = static_cast<size_t>(t0 + j) * p.ld_qkv;
+            qn[j] = ok ? qb[o] : 0.0f;
+            kn[j] = ok ? kb[o] : 0.0f;
+            vn[j] = ok ? vb[o] : 0.0f;
+        }
+        const int tj = t0 + (lane & 3);
+        bn = tj < p.T ? bb[static_cast<size_t>(tj) * p.ld_beta] : 0.0f;
+    };
+    fetch(0);
+    for (int t0 = 0; t0 < p.T; t0 += 4) {
+        float q[4], k[4], v[4], qs[4], ks[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { q[j] = qn[j]; k[j] = kn[j]; v[j] = vn[j]; }
+        const float braw = bn;
+        if (t0 + 4 < p.T) fetch(t0 + 4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            qs[j] = warp_sum_f(q[j] * q[j]);
+            ks[j] = warp_sum_f(k[j] * k[j]);
+        }
+        const int mj = lane & 3;
+        const float qt = mj == 0 ? qs[0] : (mj == 1 ? qs[1] : (mj == 2 ? qs[2] : qs[3]));
+        const float kt = mj == 0 ? ks[0] : (mj == 1 ? ks[1] : (mj == 2 ? ks[2] : ks[3]));
+        const float beta = sigmoidf_dev(braw + beta_bias);
+        const float lambda = kt < p.eps ? p.eps : kt;
+        float alpha, kscale = 1.0f;
+        if (p.method == 0) { alpha = beta; kscale = rsqrtf(lambda + p.eps); }
+        else alpha = -expm1f(-(beta * lambda)) / (lambda + p.eps);
+        const float q_inv = rsqrtf(qt + p.eps);
+        __syncwarp();  // the previous group's vectors have been read
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float kd = k[j] * __shfl_sync(0xffffffffu, kscale, j);
+            vec[warp][0][j][lane] = kd;
+            vec[warp][1][j][lane] = __shfl_sync(0xffffffffu, alpha, j) * kd;
+            vec[warp][2][j][lane] = q[j] * __shfl_sync(0xffffffffu, q_inv, j);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (t0 + j >= p.T) break;
+            const float4* kv = reinterpret_cast<const float4*>(vec[warp][0][j]);
+            const float4* av = reinterpret_cast<const float4*>(vec[warp][1][j]);
+            const float4* qv = reinterpret_cast<const float4*>(vec[warp][2][j]);
+            float2 c[4] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 x = kv[i];
+                c[2 * (i & 1)] = __ffma2_rn(make_float2(x.x, x.y), S[2 * i], c[2 * (i & 1)]);
+                c[2 * (i & 1) + 1] = __ffma2_rn(make_float2(x.z, x.w), S[2 * i + 1], c[2 * (i & 1) + 1]);
+            }
+            const float2 s01 = __fadd2_rn(__fadd2_rn(c[0], c[1]), __fadd2_rn(c[2], c[3]));
+            const float diff = v[j] - (s01.x + s01.y);
+            const float2 d2 = make_float2(diff, diff);
+            float2 y[4] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 a = av[i], x = qv[i];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    float2 s = __ffma2_rn(e == 0 ? make_float2(a.x, a.y) : make_float2(a.z, a.w), d2, S[2 * i + e]);
+                    if constexpr (kHalf) s = __half22float2(__floats2half2_rn(s.x, s.y));
+                    S[2 * i + e] = s;
+                    y[2 * (i & 1) + e] = __ffma2_rn(e == 0 ? make_float2(x.x, x.y) : make_float2(x.z, x.w), s, y[2 * (i & 1) + e]);
+                }
+            }
+            const float2 y01 = __fadd2_rn(__fadd2_rn(y[0], y[1]), __fadd2_rn(y[2], y[3]));
+            ob[static_cast<size_t>(t0 + j) * p.ld_out] = y01.x + y01.y;
+        }
+    }
+    if (Sg != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            if constexpr (kHalf) {
+                Sg[(2 * i) * 32] = __float2half_rn(S[i].x);  // (exact: the values are halves)
+                Sg[(2 * i + 1) * 32] = __float2half_rn(S[i].y);
+            } else {
+                Sg[(2 * i) * 32] = S[i].x;
+                Sg[(2 * i + 1) * 32] = S[i].y;
+            }
+        }
+    }
+}
+
+template <typename ST>
+int launch_head32(const EflaParams& p, cudaStream_t stream) {
+    const long long units = p.seqs * static_cast<long long>(p.heads);
+    if (units > 0x7fffffffLL) return set_error(BNF4_ERR_INVALID, "efla: more than 2^31 (sequence, head) units in one call");
+    launch_pdl_if(p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems, efla_head32_kernel<ST>, static_cast<unsigned>((units + kH32Warps - 1) / kH32Warps),
+                  kH32Warps * 32, 0, stream, p);
+    return check_launch("efla_head32_kernel");
+}
+
 // Split of a head's state: 128-byte row segments (NPC = 8) while a thread's share of the rows fits 16 registers quads and the
 // segment divides the row; 64-byte segments (half the columns, twice the row groups) beyond. NI follows from the width.
 template <typename ST>
 int launch_generic_for(const EflaParams& p, cudaStream_t stream) {
     const int hd = p.hidden / p.heads;
+    if (hd == 32) return launch_head32<ST>(p, stream);
     if (hd <= 512 && (hd % (8 * StatePiece<ST>::N)) == 0) {
         if (hd <= 128) return launch_generic<ST, 8, 4>(p, stream);
         if (hd <= 256) return launch_generic<ST, 8, 8>(p, stream);

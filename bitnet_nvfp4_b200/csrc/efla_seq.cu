@@ -471,9 +471,10 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
 
 }  // namespace
 
+// (heads of 32 are faster one warp each, token by token: efla_head32_kernel)
 bool efla_seq_applies(const EflaParams& p) {
     const int hd = p.hidden / p.heads;
-    return p.state == nullptr && p.state_fp16 != 0 && !p.qkv_f16 && !p.out_f16 && hd % 32 == 0 && p.T <= kSeqMaxT &&
+    return p.state == nullptr && p.state_fp16 != 0 && !p.qkv_f16 && !p.out_f16 && hd > 32 && hd % 32 == 0 && p.T <= kSeqMaxT &&
            ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0 && p.ld_qkv % 4 == 0 &&
            (reinterpret_cast<uintptr_t>(p.out) & 7) == 0 && p.ld_out % 2 == 0 && p.seqs * static_cast<long long>(p.heads) <= 0x7fffffffLL;
 }
