@@ -265,7 +265,7 @@ int launch_generic(const EflaParams& p, cudaStream_t stream) {
 // token), so no token needs a block-wide barrier. Tokens come in groups of four: the next group's q, k, v are in flight while the
 // current one is processed, the eight row norms share one butterfly, and lane j of each quad runs the scalar chain of token j.
 // k, alpha k and q^ of the group sit in shared memory and are read as broadcasts; multiply-adds are packed pairs. Issue bound, about
-// 140 instructions per token: 13200 sequences of 204 tokens in 0.4 ms, against 2.9 ms with the state in shared memory and 15 ms with
+// 140 instructions per token: 13200 units of 204 tokens in 0.81 ms, against 2.9 ms with the state in shared memory and 15 ms with
 // the generic kernel, whose 256 threads have nothing to do for a 32 x 32 state.
 // ------------------------------------------------------------------------------------------------
 constexpr int kH32Warps = 4;
@@ -1068,46 +1068,62 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const
 //       Y = diag(q_inv) (Q S0 + (Q K^T, lower triangle incl. diagonal) U~),        S += K^T U~
 // so K and Q enter the MMAs unscaled (ldmatrix straight from the raw tiles), alpha scales rows of G and columns of W^T, and the
 // query normalisation scales the finished output. No prepared operand tiles are written: the preparation phase only
-// computes the per-token scalars. The raw k tile is double-buffered because the state update at the end of a chunk still
-// reads it while the next chunk is being fetched.
+// computes the per-token scalars.
+//
+// Two warps share a unit: columns of the state are independent, so each keeps 32 of the 64 (state, W, U, Y, S update); the products
+// that do not depend on the state are divided between them (warp 0: G, alpha, the triangular solve; warp 1: Q K^T, the query norms).
+// One barrier of the pair per chunk when the tiles have arrived, one when T, P and the scalars are ready. Against one warp per unit a
+// chunk takes 1070 instead of 886 warp instructions, but its dependent chain is shorter and twice as many warps are resident (128
+// registers): 256 units, the size of a validation pass, 25.7 -> 20.0 us; 8192 sequences x 8 heads x 128 tokens 1.04 ms both ways
+// (tensor pipe 50 %, issue slots 49 %, 64 % of the copy bandwidth).
 // ------------------------------------------------------------------------------------------------
 constexpr int kM1Stride = 72;  // halves per row of the raw tiles: conflict-free for ldmatrix rows and for the 16-byte reads of eight rows
-constexpr int kM1RawQ = 0;
-constexpr int kM1RawK = kM1RawQ + kChunk * kM1Stride * 2;       // two buffers
-constexpr int kM1RawV = kM1RawK + 2 * kChunk * kM1Stride * 2;
-constexpr int kM1Y = kM1RawV + kChunk * kM1Stride * 2;          // output staging
-constexpr int kM1Beta = kM1Y + kChunk * kM1Stride * 2;
-constexpr int kM1Alpha = kM1Beta + kChunk * 4;
+constexpr int kM1YStride = 40; // halves per row of a warp's output staging tile (16 x 32)
+constexpr int kM1Tile = kChunk * kM1Stride * 2;
+constexpr int kM1RawQ = 0;                                      // two buffers each
+constexpr int kM1RawK = kM1RawQ + 2 * kM1Tile;
+constexpr int kM1RawV = kM1RawK + 2 * kM1Tile;
+constexpr int kM1Y = kM1RawV + 2 * kM1Tile;                     // output staging, one per warp
+constexpr int kM1Beta = kM1Y + 2 * kChunk * kM1YStride * 2;     // two buffers
+constexpr int kM1Alpha = kM1Beta + 2 * kChunk * 4;
 constexpr int kM1Qinv = kM1Alpha + kChunk * 4;
 constexpr int kM1L = kM1Qinv + kChunk * 4;
 constexpr int kM1T = kM1L + kChunk * kChunk * 4;
 constexpr int kM1P = kM1T + kChunk * kCkTStride * 2;
-constexpr int kM1WarpBytes = kM1P + kChunk * kCkTStride * 2;
-constexpr int kM1SmemBytes = kChunkWarps * kM1WarpBytes;
-static_assert(kM1WarpBytes % 16 == 0 && kM1L % 16 == 0 && kM1T % 16 == 0 && kM1Beta % 16 == 0, "16-byte aligned shared-memory regions");
+constexpr int kM1UnitBytes = kM1P + kChunk * kCkTStride * 2;
+constexpr int kM1Units = kChunkWarps / 2;                       // units per CTA
+constexpr int kM1CtasPerSm = 4;
+constexpr int kM1SmemBytes = kM1Units * kM1UnitBytes;
+static_assert(kM1UnitBytes % 16 == 0 && kM1L % 16 == 0 && kM1T % 16 == 0 && kM1Beta % 16 == 0 && kM1Y % 16 == 0, "16-byte aligned shared-memory regions");
 
 template <bool OUT16>
-__global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_m1_kernel(const EflaParams p) {
+__global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m1_kernel(const EflaParams p) {
     pdl_wait();
     constexpr int HD = 64;
     extern __shared__ __align__(16) uint8_t scan_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint8_t* wsm = scan_smem + warp * kM1WarpBytes;
-    __half* rawq = reinterpret_cast<__half*>(wsm + kM1RawQ);
-    __half* rawk = reinterpret_cast<__half*>(wsm + kM1RawK);   // + buffer * kChunk * kM1Stride
+    const int slot = warp >> 1, wp = warp & 1;  // unit of the CTA, warp of the unit: columns 32 wp .. 32 wp + 31
+    uint8_t* wsm = scan_smem + slot * kM1UnitBytes;
+    __half* rawq = reinterpret_cast<__half*>(wsm + kM1RawQ);   // each + buffer * kChunk * kM1Stride
+    __half* rawk = reinterpret_cast<__half*>(wsm + kM1RawK);
     __half* rawv = reinterpret_cast<__half*>(wsm + kM1RawV);
-    __half* y_sh = reinterpret_cast<__half*>(wsm + kM1Y);
+    __half* y_sh = reinterpret_cast<__half*>(wsm + kM1Y) + wp * kChunk * kM1YStride;
+    auto pair_sync = [&]() {  // constant barrier numbers: a variable one reserves all sixteen
+        static_assert(kM1Units == 2, "one barrier per unit of the CTA");
+        if (slot == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
+        else asm volatile("bar.sync 2, 64;" ::: "memory");
+    };
     float* beta_sh = reinterpret_cast<float*>(wsm + kM1Beta);
     float* alpha_sh = reinterpret_cast<float*>(wsm + kM1Alpha);
     float* qinv_sh = reinterpret_cast<float*>(wsm + kM1Qinv);
     float* L_sh = reinterpret_cast<float*>(wsm + kM1L);
     __half* t_sh = reinterpret_cast<__half*>(wsm + kM1T);
     __half* p_sh = reinterpret_cast<__half*>(wsm + kM1P);
-    // Persistent warps: each walks (sequence, head) units with a grid stride and fetches the first chunk of its next unit while the
-    // last chunk of the present one is computed, so that no unit starts with an exposed trip to DRAM.
+    // Persistent pairs of warps: each walks (sequence, head) units with a grid stride and fetches the first chunk of its next unit while
+    // the last chunk of the present one is computed, so that no unit starts with an exposed trip to DRAM.
     const unsigned total_units = static_cast<unsigned>(p.seqs * static_cast<long long>(p.heads));  // below 2^31 (checked by the host)
-    const unsigned unit_stride = gridDim.x * kChunkWarps;
-    unsigned unit = blockIdx.x * kChunkWarps + warp;
+    const unsigned unit_stride = gridDim.x * kM1Units;
+    unsigned unit = blockIdx.x * kM1Units + slot;
     if (unit >= total_units) return;
     const int g = lane >> 2, tq = lane & 3;
     // first row of a unit's sequence and its head (32-bit division: a 64-bit one costs more than a chunk's scalar work)
@@ -1123,28 +1139,29 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_m1_kernel(co
     // asynchronous copy of one chunk's q, k, v, beta rows (16-byte pieces, eight per 128-byte row); rows past the end of the
     // sequence are zero-filled so that everything derived from them stays finite
     auto issue_chunk = [&](const UnitAt& ua, int t0, int kbuf) {
-        const int piece = lane & 7, rsel = lane >> 3;
-        __half* rk = rawk + kbuf * kChunk * kM1Stride;
+        const int piece = lane & 7, rsel = 4 * wp + (lane >> 3);
+        const int bo = kbuf * kChunk * kM1Stride;
+        __half *rq = rawq + bo, *rk = rawk + bo, *rv = rawv + bo;
         const __half* qbh = static_cast<const __half*>(p.q) + ua.row0 * p.ld_qkv + ua.h * HD;
         const __half* kbh = static_cast<const __half*>(p.k) + ua.row0 * p.ld_qkv + ua.h * HD;
         const __half* vbh = static_cast<const __half*>(p.v) + ua.row0 * p.ld_qkv + ua.h * HD;
         const float* bb = p.beta_raw + ua.row0 * p.ld_beta;
 #pragma unroll
-        for (int j = 0; j < kChunk / 4; ++j) {
-            const int r = 4 * j + rsel;
+        for (int j = 0; j < kChunk / 8; ++j) {
+            const int r = 8 * j + rsel;
             if (t0 + r < p.T) {
                 const size_t o = static_cast<size_t>(t0 + r) * p.ld_qkv + 8 * piece;
-                cp_async16(rawq + r * kM1Stride + 8 * piece, qbh + o);
+                cp_async16(rq + r * kM1Stride + 8 * piece, qbh + o);
                 cp_async16(rk + r * kM1Stride + 8 * piece, kbh + o);
-                cp_async16(rawv + r * kM1Stride + 8 * piece, vbh + o);
+                cp_async16(rv + r * kM1Stride + 8 * piece, vbh + o);
             } else {
                 const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-                *reinterpret_cast<uint4*>(rawq + r * kM1Stride + 8 * piece) = z;
+                *reinterpret_cast<uint4*>(rq + r * kM1Stride + 8 * piece) = z;
                 *reinterpret_cast<uint4*>(rk + r * kM1Stride + 8 * piece) = z;
-                *reinterpret_cast<uint4*>(rawv + r * kM1Stride + 8 * piece) = z;
+                *reinterpret_cast<uint4*>(rv + r * kM1Stride + 8 * piece) = z;
             }
         }
-        if (lane < kChunk && t0 + lane < p.T) cp_async4(beta_sh + lane, bb + static_cast<size_t>(t0 + lane) * p.ld_beta);
+        if (wp == 0 && lane < kChunk && t0 + lane < p.T) cp_async4(beta_sh + kbuf * kChunk + lane, bb + static_cast<size_t>(t0 + lane) * p.ld_beta);
         cp_async_commit();
     };
 
@@ -1152,7 +1169,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_m1_kernel(co
     const int lm_j = lane >> 3, lm_r = lane & 7;
     // tiles stored [token][d]: matrices (tokens 0-7 | d 0-7), (0-7 | 8-15), (8-15 | 0-7), (8-15 | 8-15) of a 16-wide d block
     const uint32_t lm_tok_off = static_cast<uint32_t>(((lm_j >> 1) * 8 + lm_r) * kM1Stride + (lm_j & 1) * 8) * 2u;
-    const uint32_t q_addr = static_cast<uint32_t>(__cvta_generic_to_shared(rawq)) + lm_tok_off;
+    const uint32_t q_addr0 = static_cast<uint32_t>(__cvta_generic_to_shared(rawq)) + lm_tok_off;
     const uint32_t k_addr0 = static_cast<uint32_t>(__cvta_generic_to_shared(rawk)) + lm_tok_off;
     const uint32_t lm_ts_off = static_cast<uint32_t>(((lm_j >> 1) * 8 + lm_r) * kCkTStride + (lm_j & 1) * 8) * 2u;
     // T^T read transposed: matrices (s 0-7 | t 0-7), (s 8-15 | t 0-7), (s 0-7 | t 8-15), (s 8-15 | t 8-15)
@@ -1163,8 +1180,9 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_m1_kernel(co
     const uint32_t kt_addr0 = static_cast<uint32_t>(__cvta_generic_to_shared(rawk)) +
                               static_cast<uint32_t>(((lm_j & 1) * 8 + lm_r) * kM1Stride + (lm_j >> 1) * 8) * 2u;
     // V read and Y written through transposing matrix loads / stores (tokens 8 (j >> 1) .., columns 16 mt + 8 (j & 1) ..)
-    const uint32_t v_addr = static_cast<uint32_t>(__cvta_generic_to_shared(rawv)) + lm_tok_off;
-    const uint32_t y_addr = static_cast<uint32_t>(__cvta_generic_to_shared(y_sh)) + lm_tok_off;
+    const uint32_t v_addr0 = static_cast<uint32_t>(__cvta_generic_to_shared(rawv)) + lm_tok_off + wp * 64;
+    const uint32_t y_addr = static_cast<uint32_t>(__cvta_generic_to_shared(y_sh)) +
+                            static_cast<uint32_t>(((lm_j >> 1) * 8 + lm_r) * kM1YStride + (lm_j & 1) * 8) * 2u;
     constexpr uint32_t kKBufBytes = kChunk * kM1Stride * 2;
 
     int kbuf = 0;
@@ -1172,30 +1190,30 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_m1_kernel(co
     for (; unit < total_units; unit += unit_stride) {
     const UnitAt ua = unit_at(unit);
     const float beta_bias = p.beta_bias_seq != nullptr ? p.beta_bias_seq[ua.useq / static_cast<unsigned>(p.seqs_per_bias)] : p.beta_bias;
-    float* ob = static_cast<float*>(p.out) + ua.row0 * p.ld_out + ua.h * HD;
-    __half* obh = static_cast<__half*>(p.out) + ua.row0 * p.ld_out + ua.h * HD;
-    uint32_t Sh[4][4][4];  // state S^T as A fragments, as in efla_chunk16_kernel
+    float* ob = static_cast<float*>(p.out) + ua.row0 * p.ld_out + ua.h * HD + 32 * wp;
+    __half* obh = static_cast<__half*>(p.out) + ua.row0 * p.ld_out + ua.h * HD + 32 * wp;
+    uint32_t Sh[2][4][4];  // this warp's columns of the state S^T as A fragments, as in efla_chunk16_kernel
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
             for (int i = 0; i < 4; ++i) Sh[mt][ks][i] = 0u;
     for (int t0 = 0; t0 < p.T; t0 += kChunk, kbuf ^= 1) {
         cp_async_wait<0>();
-        __syncwarp();
+        pair_sync();  // both halves of the tiles have landed; both warps are done with the other buffers, T and P
+        if (t0 + kChunk < p.T) issue_chunk(ua, t0 + kChunk, kbuf ^ 1);
+        else if (unit + unit_stride < total_units) issue_chunk(unit_at(unit + unit_stride), 0, kbuf ^ 1);
+        const uint32_t bufo = kbuf * kKBufBytes;
         // ---------------- operand fragments straight from the raw tiles; W^T starts as -V^T ----------------
-        uint32_t kf[4][4], qf[4][4];  // per 16-wide d block: B fragments {b0, b1} for tokens 0-7 (regs 0, 1) and 8-15 (regs 2, 3)
+        uint32_t kf[4][4];  // per 16-wide d block: B fragments {b0, b1} for tokens 0-7 (regs 0, 1) and 8-15 (regs 2, 3)
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            ldmatrix_x4(kf[ks], k_addr0 + kbuf * kKBufBytes + ks * 32);
-            ldmatrix_x4(qf[ks], q_addr + ks * 32);
-        }
-        float Wc[4][2][4];  // -(V - K S0)^T = S0^T K^T - V^T
+        for (int ks = 0; ks < 4; ++ks) ldmatrix_x4(kf[ks], k_addr0 + bufo + ks * 32);
+        float Wc[2][2][4];  // -(V - K S0)^T = S0^T K^T - V^T
 #pragma unroll
-        for (int mt = 0; mt < 4; ++mt) {
+        for (int mt = 0; mt < 2; ++mt) {
             uint32_t vf[4];
-            ldmatrix_x4_trans(vf, v_addr + mt * 32);
+            ldmatrix_x4_trans(vf, v_addr0 + bufo + mt * 32);
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
                 const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&vf[2 * nt])), hi = __half22float2(*reinterpret_cast<const __half2*>(&vf[2 * nt + 1]));
@@ -1203,101 +1221,120 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_m1_kernel(co
                 Wc[mt][nt][2] = -hi.x; Wc[mt][nt][3] = -hi.y;
             }
         }
-        // The squared norms of k and q are the diagonals of K K^T and Q Q^T, which the tensor cores produce below. They land in
-        // the eight lanes with tq == g / 2 (tokens g and g + 8); each hands token g + 8 to its neighbour lane ^ 1, so sixteen
-        // lanes run the scalar chain for one token each. Those lanes take their beta now: the next chunk's copy overwrites it.
-        const bool diag_lane = tq == (g >> 1);
-        const bool helper_lane = (tq ^ 1) == (g >> 1);
-        const int my_tok = g + (helper_lane ? 8 : 0);
-        float braw = 0.0f;
-        if ((diag_lane || helper_lane) && t0 + my_tok < p.T) braw = beta_sh[my_tok];
-        __syncwarp();  // q, v and beta are consumed
-        if (t0 + kChunk < p.T) issue_chunk(ua, t0 + kChunk, kbuf ^ 1);
-        else if (unit + unit_stride < total_units) issue_chunk(unit_at(unit + unit_stride), 0, kbuf ^ 1);
-
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt)
+            for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt)
                     mma_f16_16816(Wc[mt][nt], Sh[mt][ks][0], Sh[mt][ks][1], Sh[mt][ks][2], Sh[mt][ks][3], kf[ks][2 * nt], kf[ks][2 * nt + 1]);
-        float Gc[2][4], Xc[2][4], Qc[2][4];  // rows t = g (+ 8 for i >= 2), columns s = 8 nt + 2 tq + (i & 1);  Xc = q_t . k_s, Qc = q_t . q_s
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) Gc[nt][i] = Xc[nt][i] = Qc[nt][i] = 0.0f;
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                mma_f16_16816(Gc[nt], kf[ks][0], kf[ks][2], kf[ks][1], kf[ks][3], kf[ks][2 * nt], kf[ks][2 * nt + 1]);
-                mma_f16_16816(Xc[nt], qf[ks][0], qf[ks][2], qf[ks][1], qf[ks][3], kf[ks][2 * nt], kf[ks][2 * nt + 1]);
-                mma_f16_16816(Qc[nt], qf[ks][0], qf[ks][2], qf[ks][1], qf[ks][3], qf[ks][2 * nt], qf[ks][2 * nt + 1]);
-            }
-        // ---------------- per-token scalars from the diagonals (exact fp16 products accumulated in fp32) ----------------
-        {
+        // The squared norms of k and q are the diagonals of K K^T and Q Q^T, which the tensor cores produce. They land in the eight
+        // lanes with tq == g / 2 (tokens g and g + 8); each hands token g + 8 to its neighbour lane ^ 1, so sixteen lanes run the
+        // scalar chain for one token each.
+        const bool diag_lane = tq == (g >> 1);
+        const bool helper_lane = (tq ^ 1) == (g >> 1);
+        const int my_tok = g + (helper_lane ? 8 : 0);
+        auto diagonal = [&](const float (&M)[2][4]) {  // of token my_tok, in the diagonal and helper lanes
             const int e = g & 1;
-            float kss = e ? Gc[0][1] : Gc[0][0], qss = e ? Qc[0][1] : Qc[0][0];              // token g (valid in the diagonal lanes)
-            const float kss_hi = e ? Gc[1][3] : Gc[1][2], qss_hi = e ? Qc[1][3] : Qc[1][2];  // token g + 8
-            const float k_from = __shfl_xor_sync(0xffffffffu, kss_hi, 1), q_from = __shfl_xor_sync(0xffffffffu, qss_hi, 1);
-            if (helper_lane) { kss = k_from; qss = q_from; }
-            if (diag_lane || helper_lane) {
-                const float lambda = kss < p.eps ? p.eps : kss;
-                // sigmoid and the final quotient with the fast exponential / division (about 2 ulp each: far below the fp16
-                // rounding of every operand alpha touches); expm1f keeps its accuracy for small beta * lambda
-                const float beta = __fdividef(1.0f, 1.0f + __expf(-(braw + beta_bias)));
-                alpha_sh[my_tok] = t0 + my_tok < p.T ? __fdividef(-expm1f(-(beta * lambda)), lambda + p.eps) : 0.0f;
-                qinv_sh[my_tok] = rsqrtf(qss + p.eps);
+            const float lo = e ? M[0][1] : M[0][0], hi = e ? M[1][3] : M[1][2];
+            const float from = __shfl_xor_sync(0xffffffffu, hi, 1);
+            return helper_lane ? from : lo;
+        };
+        if (wp == 0) {
+            float Gc[2][4];  // rows t = g (+ 8 for i >= 2), columns s = 8 nt + 2 tq + (i & 1)
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) Gc[nt][i] = 0.0f;
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) mma_f16_16816(Gc[nt], kf[ks][0], kf[ks][2], kf[ks][1], kf[ks][3], kf[ks][2 * nt], kf[ks][2 * nt + 1]);
+            // ---------------- alpha from the diagonal (exact fp16 products accumulated in fp32) ----------------
+            {
+                const float kss = diagonal(Gc);
+                if (diag_lane || helper_lane) {
+                    const bool valid = t0 + my_tok < p.T;
+                    const float braw = valid ? beta_sh[kbuf * kChunk + my_tok] : 0.0f;
+                    const float lambda = kss < p.eps ? p.eps : kss;
+                    // sigmoid and the final quotient with the fast exponential / division (about 2 ulp each: far below the fp16
+                    // rounding of every operand alpha touches); expm1f keeps its accuracy for small beta * lambda
+                    const float beta = __fdividef(1.0f, 1.0f + __expf(-(braw + beta_bias)));
+                    alpha_sh[my_tok] = valid ? __fdividef(-expm1f(-(beta * lambda)), lambda + p.eps) : 0.0f;
+                }
             }
-        }
-        __syncwarp();
-        // L[t][s] = a_t G[t][s] (s < t) in fp32 for the substitution; P[t][s] = q_t . k_s (s <= t) in fp16
-        {
-            const float a_lo = alpha_sh[g], a_hi = alpha_sh[g + 8];
+            __syncwarp();
+            // L[t][s] = a_t G[t][s] in fp32; the substitution reads it below the diagonal only: no mask needed
+            {
+                const float a_lo = alpha_sh[g], a_hi = alpha_sh[g + 8];
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    const int s0 = 8 * nt + 2 * tq;
+                    *reinterpret_cast<float2*>(L_sh + g * kChunk + s0) = make_float2(a_lo * Gc[nt][0], a_lo * Gc[nt][1]);
+                    *reinterpret_cast<float2*>(L_sh + (g + 8) * kChunk + s0) = make_float2(a_hi * Gc[nt][2], a_hi * Gc[nt][3]);
+                }
+            }
+            __syncwarp();
+            // ---------------- T = (I + L)^-1 by forward substitution, lane c owns column c ----------------
+            {
+                const int c = lane & 15;
+                float col[kChunk];
+#pragma unroll
+                for (int t = 0; t < kChunk; ++t) {
+                    float acc = t == c ? 1.0f : 0.0f;
+#pragma unroll
+                    for (int s4 = 0; s4 < t; s4 += 4) {
+                        const float4 lv = *reinterpret_cast<const float4*>(L_sh + t * kChunk + s4);
+                        acc = fmaf(-lv.x, col[s4], acc);
+                        if (s4 + 1 < t) acc = fmaf(-lv.y, col[s4 + 1], acc);
+                        if (s4 + 2 < t) acc = fmaf(-lv.z, col[s4 + 2], acc);
+                        if (s4 + 3 < t) acc = fmaf(-lv.w, col[s4 + 3], acc);
+                    }
+                    col[t] = acc;
+                }
+                if (lane < kChunk) {  // the column as one row of T^T: sixteen halves, two 16-byte stores
+                    uint32_t w[8];
+#pragma unroll
+                    for (int t = 0; t < kChunk; t += 2) w[t >> 1] = pack_half2(col[t], col[t + 1]);
+                    uint4* dst = reinterpret_cast<uint4*>(t_sh + c * kCkTStride);
+                    dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                    dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                }
+            }
+        } else {
+            uint32_t qf[4][4];
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) ldmatrix_x4(qf[ks], q_addr0 + bufo + ks * 32);
+            float Xc[2][4], Qc[2][4];  // Xc = q_t . k_s, Qc = q_t . q_s
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) Xc[nt][i] = Qc[nt][i] = 0.0f;
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    mma_f16_16816(Xc[nt], qf[ks][0], qf[ks][2], qf[ks][1], qf[ks][3], kf[ks][2 * nt], kf[ks][2 * nt + 1]);
+                    mma_f16_16816(Qc[nt], qf[ks][0], qf[ks][2], qf[ks][1], qf[ks][3], qf[ks][2 * nt], qf[ks][2 * nt + 1]);
+                }
+            const float qss = diagonal(Qc);
+            if (diag_lane || helper_lane) qinv_sh[my_tok] = rsqrtf(qss + p.eps);
+            // P[t][s] = q_t . k_s (s <= t) in fp16
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
                 const int s0 = 8 * nt + 2 * tq;
 #pragma unroll
                 for (int hr = 0; hr < 2; ++hr) {
                     const int t = g + 8 * hr;
-                    const float at = hr ? a_hi : a_lo;
-                    // the substitution reads L below the diagonal only: no mask needed there; P feeds an MMA and is masked
-                    const float l0 = at * Gc[nt][2 * hr], l1 = at * Gc[nt][2 * hr + 1];
-                    const float p0 = s0 <= t ? Xc[nt][2 * hr] : 0.0f, p1 = s0 + 1 <= t ? Xc[nt][2 * hr + 1] : 0.0f;
-                    *reinterpret_cast<float2*>(L_sh + t * kChunk + s0) = make_float2(l0, l1);
-                    *reinterpret_cast<uint32_t*>(p_sh + t * kCkTStride + s0) = pack_half2(p0, p1);
+                    *reinterpret_cast<uint32_t*>(p_sh + t * kCkTStride + s0) =
+                        pack_half2(s0 <= t ? Xc[nt][2 * hr] : 0.0f, s0 + 1 <= t ? Xc[nt][2 * hr + 1] : 0.0f);
                 }
             }
         }
-        __syncwarp();
-        // ---------------- T = (I + L)^-1 by forward substitution, lane c owns column c ----------------
-        {
-            const int c = lane & 15;
-            float col[kChunk];
+        pair_sync();  // T, P and the scalars are there
+        uint32_t qf[4][4];
 #pragma unroll
-            for (int t = 0; t < kChunk; ++t) {
-                float acc = t == c ? 1.0f : 0.0f;
-#pragma unroll
-                for (int s4 = 0; s4 < t; s4 += 4) {
-                    const float4 lv = *reinterpret_cast<const float4*>(L_sh + t * kChunk + s4);
-                    acc = fmaf(-lv.x, col[s4], acc);
-                    if (s4 + 1 < t) acc = fmaf(-lv.y, col[s4 + 1], acc);
-                    if (s4 + 2 < t) acc = fmaf(-lv.z, col[s4 + 2], acc);
-                    if (s4 + 3 < t) acc = fmaf(-lv.w, col[s4 + 3], acc);
-                }
-                col[t] = acc;
-            }
-            if (lane < kChunk) {  // the column as one row of T^T: sixteen halves, two 16-byte stores
-                uint32_t w[8];
-#pragma unroll
-                for (int t = 0; t < kChunk; t += 2) w[t >> 1] = pack_half2(col[t], col[t + 1]);
-                uint4* dst = reinterpret_cast<uint4*>(t_sh + c * kCkTStride);
-                dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-            }
-        }
-        __syncwarp();
+        for (int ks = 0; ks < 4; ++ks) ldmatrix_x4(qf[ks], q_addr0 + bufo + ks * 32);  // (warp 1 again: cheaper than keeping them)
         uint32_t tf[4], pf[4];
         ldmatrix_x4_trans(tf, tt_addr);  // T^T stored [s][t]: transposed on the way in, the fragments are those of T stored [t][s]
         ldmatrix_x4(pf, p_addr);
@@ -1310,9 +1347,9 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_m1_kernel(co
             na[nt][0] = -al.x; na[nt][1] = -al.y;
             qi[nt][0] = q2.x; qi[nt][1] = q2.y;
         }
-        uint32_t Up[4][4];
+        uint32_t Up[2][4];
 #pragma unroll
-        for (int mt = 0; mt < 4; ++mt) {
+        for (int mt = 0; mt < 2; ++mt) {
             // packed fp32 pairs (tokens 2 tq and 2 tq + 1): each half rounds like the scalar multiply
             const float2 na0 = make_float2(na[0][0], na[0][1]), na1 = make_float2(na[1][0], na[1][1]);
             const float2 x0 = __fmul2_rn(na0, make_float2(Wc[mt][0][0], Wc[mt][0][1])), x1 = __fmul2_rn(na0, make_float2(Wc[mt][0][2], Wc[mt][0][3]));
@@ -1326,7 +1363,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_m1_kernel(co
         }
         // ---------------- Y^T = (S0^T Q^T + U~^T P^T) diag(q_inv) ----------------
 #pragma unroll
-        for (int mt = 0; mt < 4; ++mt) {
+        for (int mt = 0; mt < 2; ++mt) {
             float Yc[2][4];
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) mma_f16_16816_zero(Yc[nt], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], pf[2 * nt], pf[2 * nt + 1]);
@@ -1361,25 +1398,25 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_m1_kernel(co
         if constexpr (OUT16) {
             __syncwarp();
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {  // 16 rows x 128 bytes: 16-byte pieces, eight per row
-                const int tl = 4 * j + (lane >> 3), piece = lane & 7;
+            for (int j = 0; j < 2; ++j) {  // 16 rows x 64 bytes: 16-byte pieces, four per row
+                const int tl = 8 * j + (lane >> 2), piece = lane & 3;
                 if (t0 + tl < p.T)
                     *reinterpret_cast<uint4*>(obh + static_cast<size_t>(t0 + tl) * p.ld_out + 8 * piece) =
-                        *reinterpret_cast<const uint4*>(y_sh + tl * kM1Stride + 8 * piece);
+                        *reinterpret_cast<const uint4*>(y_sh + tl * kM1YStride + 8 * piece);
             }
         }
         // ---------------- S^T += U~^T K: fp16 accumulators = the state registers, rounded once per chunk ----------------
 #pragma unroll
         for (int dp = 0; dp < 4; ++dp) {
             uint32_t af[4];
-            ldmatrix_x4_trans(af, kt_addr0 + kbuf * kKBufBytes + dp * 32);
+            ldmatrix_x4_trans(af, kt_addr0 + bufo + dp * 32);
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt) {
+            for (int mt = 0; mt < 2; ++mt) {
                 mma_f16acc_16816(Sh[mt][dp][0], Sh[mt][dp][1], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], af[0], af[1]);
                 mma_f16acc_16816(Sh[mt][dp][2], Sh[mt][dp][3], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], af[2], af[3]);
             }
         }
-        __syncwarp();  // the staging tile and this chunk's k buffer are free for the chunk after the next
+        __syncwarp();  // the staging tile is free
     }
     }
     cp_async_wait<0>();
@@ -1430,10 +1467,10 @@ int efla_launch(const EflaParams& p, cudaStream_t stream) {
             if (p.qkv_f16 && ((p.ld_qkv % 8) != 0)) return set_error(BNF4_ERR_INVALID, "efla: fp16 q, k, v need ld_qkv %% 8 == 0");
             if (p.out_f16 && (((p.ld_out % 8) != 0) || (reinterpret_cast<uintptr_t>(p.out) & 15))) return set_error(BNF4_ERR_INVALID, "efla: fp16 output needs 16-byte aligned rows");
             const unsigned grid = static_cast<unsigned>(ctas);
-            if (p.qkv_f16 && p.method == 1) {  // the batched driver's case: raw-operand kernel, persistent warps (two CTAs per SM)
+            if (p.qkv_f16 && p.method == 1) {  // the batched driver's case: raw-operand kernel, persistent pairs of warps
                 const int sms = multiprocessors(dev);
                 if (sms <= 0) return BNF4_ERR_CUDA;
-                const unsigned pgrid = std::min(grid, static_cast<unsigned>(2 * sms));
+                const unsigned pgrid = static_cast<unsigned>(std::min<long long>((units + kM1Units - 1) / kM1Units, kM1CtasPerSm * static_cast<long long>(sms)));
                 if (p.out_f16) launch_pdl_if(early, efla_chunk16_m1_kernel<true>, pgrid, kChunkWarps * 32, kM1SmemBytes, stream, p);
                 else launch_pdl_if(early, efla_chunk16_m1_kernel<false>, pgrid, kChunkWarps * 32, kM1SmemBytes, stream, p);
             } else if (p.qkv_f16 && p.out_f16) launch_pdl_if(early, efla_chunk16_kernel<true, true>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
