@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kGenThreads, (NI <= 16 ? 2 : 1)) efla_generic_
     const float* kb = static_cast<const float*>(p.k) + row0 * p.ld_qkv + h * hd;
     const float* vb = static_cast<const float*>(p.v) + row0 * p.ld_qkv + h * hd + col;
     float* ob = static_cast<float*>(p.out) + row0 * p.ld_out + h * hd + slice * NC;
-    const float beta_bias = p.beta_bias_seq != nullptr ? p.beta_bias_seq[seq / static_cast<unsigned>(p.seqs_per_bias)] : p.beta_bias;
+    const float beta_bias = efla_seq_bias(p, static_cast<unsigned>(seq));
 
     float qn[KQ], kn[KQ], vn[PN], bn;
     auto fetch = [&](int t) {  // the token's inputs, one token ahead of their use
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kH32Warps * 32) efla_head32_kernel(const EflaP
     const float* vb = static_cast<const float*>(p.v) + row0 * p.ld_qkv + h * 32 + lane;
     const float* bb = p.beta_raw + row0 * p.ld_beta;
     float* ob = static_cast<float*>(p.out) + row0 * p.ld_out + h * 32 + lane;
-    const float beta_bias = p.beta_bias_seq != nullptr ? p.beta_bias_seq[seq / static_cast<unsigned>(p.seqs_per_bias)] : p.beta_bias;
+    const float beta_bias = efla_seq_bias(p, static_cast<unsigned>(seq));
 
     float2 S[16];  // rows 2 i, 2 i + 1
     ST* Sg = p.state != nullptr ? reinterpret_cast<ST*>(p.state) + static_cast<size_t>(unit) * 1024 + lane : nullptr;
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kScanWarps * 32, kScan2CtasPerSm) efla_scan64_
     if (unit >= p.seqs * static_cast<long long>(p.heads)) return;
     const long long seq = unit / p.heads;
     const int h = static_cast<int>(unit - seq * p.heads);
-    const float beta_bias = p.beta_bias_seq != nullptr ? p.beta_bias_seq[seq / p.seqs_per_bias] : p.beta_bias;
+    const float beta_bias = efla_seq_bias(p, static_cast<unsigned>(seq));
     const int g = lane >> 2, tq = lane & 3;
 
     uint32_t Sh[4][4][4];  // [mt][ks][i]: the A fragment (i = 0: n = g, d pair 2tq; 1: n = g + 8; 2: n = g, d pair 2tq + 8; 3: n = g + 8)
@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const
     const unsigned useq = static_cast<unsigned>(unit) / static_cast<unsigned>(p.heads);
     const long long seq = useq;
     const int h = static_cast<int>(static_cast<unsigned>(unit) - useq * static_cast<unsigned>(p.heads));
-    const float beta_bias = p.beta_bias_seq != nullptr ? p.beta_bias_seq[useq / static_cast<unsigned>(p.seqs_per_bias)] : p.beta_bias;
+    const float beta_bias = efla_seq_bias(p, static_cast<unsigned>(useq));
     const int g = lane >> 2, tq = lane & 3;
 
     // state S^T as A fragments: Sh[mt][ks][i] holds S[d][n] for n = 16 mt + g (+ 8 for odd i), d = 16 ks + 2 tq + {0, 1} (+ 8 for i >= 2)
@@ -1189,7 +1189,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
     issue_chunk(unit_at(unit), 0, 0);
     for (; unit < total_units; unit += unit_stride) {
     const UnitAt ua = unit_at(unit);
-    const float beta_bias = p.beta_bias_seq != nullptr ? p.beta_bias_seq[ua.useq / static_cast<unsigned>(p.seqs_per_bias)] : p.beta_bias;
+    const float beta_bias = efla_seq_bias(p, static_cast<unsigned>(ua.useq));
     float* ob = static_cast<float*>(p.out) + ua.row0 * p.ld_out + ua.h * HD + 32 * wp;
     __half* obh = static_cast<__half*>(p.out) + ua.row0 * p.ld_out + ua.h * HD + 32 * wp;
     uint32_t Sh[2][4][4];  // this warp's columns of the state S^T as A fragments, as in efla_chunk16_kernel

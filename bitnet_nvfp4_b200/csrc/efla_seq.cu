@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         const float qss = qs_sh[t], kss = ks_sh[t];
         float a = 0.0f, b = 0.0f, kinv = 0.0f, qinv = 0.0f;
         if (t < T) {
-            const float bias = p.beta_bias_seq != nullptr ? p.beta_bias_seq[seq / static_cast<unsigned>(p.seqs_per_bias)] : p.beta_bias;
+            const float bias = efla_seq_bias(p, static_cast<unsigned>(seq));
             const float beta = 1.0f / (1.0f + expf(-(p.beta_raw[(row0 + t) * p.ld_beta] + bias)));
             const float lambda = kss < p.eps ? p.eps : kss;
             qinv = rsqrtf(qss + p.eps);

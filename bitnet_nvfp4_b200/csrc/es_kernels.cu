@@ -85,18 +85,41 @@ __global__ void __launch_bounds__(256) ce_step_kernel(const float* __restrict__ 
     }
 }
 
-// Population form: grid (16 chunks, members). partial[member*16 + chunk] = sum of the chunk's row losses.
+// Population form: grid (chunks, members). partial[member * chunks + chunk] = sum of the chunk's row losses. With a counter per member
+// (zero before the launch, zero again after it) the member's last block also forms the mean, in chunk order; without, ce_finalize_kernel
+// does.
 constexpr int kCeChunks = 16;
+__device__ __forceinline__ void ce_finish(float block_sum, float* partial, unsigned* counters, int rows_per_member, float* loss_mean) {
+    __shared__ bool last;
+    const int member = blockIdx.y, chunks = gridDim.x;
+    if (threadIdx.x == 0) {
+        partial[member * chunks + blockIdx.x] = block_sum;
+        last = false;
+        if (counters != nullptr) {
+            __threadfence();
+            last = atomicInc(counters + member, chunks - 1) == static_cast<unsigned>(chunks - 1);  // wraps to zero
+        }
+    }
+    if (counters == nullptr) return;
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return;
+    __threadfence();
+    double t = 0.0;
+    for (int c = threadIdx.x; c < chunks; c += 32) t += static_cast<double>(__ldcg(partial + member * chunks + c));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (threadIdx.x == 0) loss_mean[member] = static_cast<float>(t / static_cast<double>(rows_per_member));
+}
 __global__ void __launch_bounds__(256) ce_population_kernel(const float* __restrict__ logits, int ld, const float* __restrict__ bias,
                                                             const int8_t* __restrict__ bias_noise, float sigma,
                                                             const uint8_t* __restrict__ targets, int vocab, int rows_per_member,
-                                                            float* __restrict__ partial) {
+                                                            float* partial, unsigned* counters, float* loss_mean) {
     pdl_wait();
     after(logits, bias, bias_noise, targets);
     __shared__ float part[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int member = blockIdx.y, chunk = blockIdx.x;
-    const int per = (rows_per_member + kCeChunks - 1) / kCeChunks;
+    const int per = (rows_per_member + gridDim.x - 1) / gridDim.x;
     const int r0 = chunk * per, r1 = min(rows_per_member, r0 + per);
     const float bns = (member & 1) ? -sigma : sigma;
     const int8_t* nz = bias_noise != nullptr ? bias_noise + static_cast<size_t>(member >> 1) * vocab : nullptr;
@@ -107,11 +130,10 @@ __global__ void __launch_bounds__(256) ce_population_kernel(const float* __restr
     }
     if (lane == 0) part[warp] = acc;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
+    float t = 0.0f;
+    if (threadIdx.x == 0)
         for (int w = 0; w < 8; ++w) t += part[w];
-        partial[member * kCeChunks + chunk] = t;
-    }
+    ce_finish(t, partial, counters, rows_per_member, loss_mean);
 }
 
 // Streaming form of the same reduction for 16-byte aligned rows and vocab % 4 == 0: lane l owns the float4 groups
@@ -122,13 +144,13 @@ template <int NV4, int RPI>
 __global__ void __launch_bounds__(256) ce_population_vec_kernel(const float* __restrict__ logits, int ld, const float* __restrict__ bias,
                                                                 const int8_t* __restrict__ bias_noise, float sigma,
                                                                 const uint8_t* __restrict__ targets, int vocab, int rows_per_member,
-                                                                float* __restrict__ partial) {
+                                                                float* partial, unsigned* counters, float* loss_mean) {
     pdl_wait();
     after(logits, bias, bias_noise, targets);
     __shared__ float part[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int member = blockIdx.y, chunk = blockIdx.x;
-    const int per = (rows_per_member + kCeChunks - 1) / kCeChunks;
+    const int per = (rows_per_member + gridDim.x - 1) / gridDim.x;
     const int r0 = chunk * per, r1 = min(rows_per_member, r0 + per);
     const float bns = (member & 1) ? -sigma : sigma;
     const int groups = vocab >> 2;
@@ -189,11 +211,10 @@ __global__ void __launch_bounds__(256) ce_population_vec_kernel(const float* __r
     }
     if (lane == 0) part[warp] = acc;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.0f;
+    float t = 0.0f;
+    if (threadIdx.x == 0)
         for (int w = 0; w < 8; ++w) t += part[w];
-        partial[member * kCeChunks + chunk] = t;
-    }
+    ce_finish(t, partial, counters, rows_per_member, loss_mean);
 }
 
 __global__ void ce_finalize_kernel(const float* __restrict__ partial, int members, int rows_per_member, float* __restrict__ loss_mean) {
@@ -299,8 +320,8 @@ __global__ void __launch_bounds__(256) z_dense_kernel(const float* __restrict__ 
 // its tensor by walking the table. With nshards > 1 a tensor that is computed in shards covers this shard's elements only.
 template <bool CLT4>
 __global__ void __launch_bounds__(256) z_dense_table_kernel(const float* __restrict__ pair_weights, const uint64_t* __restrict__ pair_seeds,
-                                                            const ZDenseDesc* __restrict__ descs, int ndesc, int pairs, int use_clt, int clt_k,
-                                                            int use_noise_tables, int shard, int nshards, float* __restrict__ z_all) {
+                                                            const ZDenseDesc* __restrict__ descs, int ndesc, int pairs, int use_clt, int clt_k, int shard,
+                                                            int nshards, float* __restrict__ z_all) {
     pdl_wait();
     after(pair_weights, pair_seeds);
     int block = static_cast<int>(blockIdx.x), idx0 = 0, n = 0;
@@ -313,30 +334,7 @@ __global__ void __launch_bounds__(256) z_dense_table_kernel(const float* __restr
         block -= blocks;
     }
     const int i = block * 256 + threadIdx.x;
-    float* out = z_all + d.zoff + idx0 + i;
-    if (use_noise_tables && d.noise != nullptr) {  // one byte per pair instead of one hash; same values, same order
-        if (i >= n) return;
-        const int8_t* src = d.noise + idx0 + i;
-        float z = 0.0f;
-        int p = 0;
-        for (; p + 16 <= pairs; p += 16) {
-            int8_t e[16];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) e[q] = src[static_cast<size_t>(p + q) * d.n];
-#pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                const float w = pair_weights[p + q];
-                if (w != 0.0f) z = fmaf(w, static_cast<float>(e[q]), z);
-            }
-        }
-        for (; p < pairs; ++p) {
-            const float w = pair_weights[p];
-            if (w != 0.0f) z = fmaf(w, static_cast<float>(src[static_cast<size_t>(p) * d.n]), z);
-        }
-        *out = z;
-        return;
-    }
-    z_dense_block<CLT4>(pair_weights, pair_seeds, d.salt, pairs, idx0 + i, i < n, use_clt, clt_k, out);
+    z_dense_block<CLT4>(pair_weights, pair_seeds, d.salt, pairs, idx0 + i, i < n, use_clt, clt_k, z_all + d.zoff + idx0 + i);
 }
 
 // Rank-r form of Z: Z[i][j] = cscale * sum_p w_p * (sum_r A[p][i][r] * B[p][r][j]), pairs in ascending order with one fused
@@ -357,10 +355,45 @@ __device__ __forceinline__ void z_shard_rows(int rows, int shard, int nshards, i
     if (nshards > 1 && rows >= nshards && (rows % nshards) == 0) { nr = rows / nshards; r0 = shard * nr; }
 }
 
+// The first `table_blocks` blocks compute the tensors whose noise lies in memory as [pair][n] bytes (the step's fp32 vectors): one byte per
+// pair and element instead of one hash, same values, same order. They are few and latency-bound, so they start first.
+__device__ __forceinline__ void z_table_block(const float* __restrict__ pair_weights, const ZDenseDesc* __restrict__ descs, int ndesc, int block, int pairs, int shard,
+                                              int nshards, float* __restrict__ z_all) {
+    int idx0 = 0, n = 0;
+    ZDenseDesc d = {};
+    for (int t = 0; t < ndesc; ++t) {
+        d = descs[t];
+        z_dense_range(d, shard, nshards, idx0, n);
+        const int blocks = (n + kZThreads - 1) / kZThreads;
+        if (block < blocks) break;
+        block -= blocks;
+    }
+    const int i = block * kZThreads + static_cast<int>(threadIdx.x);
+    if (i >= n) return;
+    const int8_t* src = d.noise + idx0 + i;
+    float z = 0.0f;
+    int p = 0;
+    for (; p + 16 <= pairs; p += 16) {
+        int8_t e[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) e[q] = src[static_cast<size_t>(p + q) * d.n];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            const float w = pair_weights[p + q];
+            if (w != 0.0f) z = fmaf(w, static_cast<float>(e[q]), z);
+        }
+    }
+    for (; p < pairs; ++p) {
+        const float w = pair_weights[p];
+        if (w != 0.0f) z = fmaf(w, static_cast<float>(src[static_cast<size_t>(p) * d.n]), z);
+    }
+    z_all[d.zoff + idx0 + i] = z;
+}
+
 template <int RANK>
 __global__ void __launch_bounds__(kZThreads) z_lowrank_tiles_kernel(const float* __restrict__ pair_weights, const ZLowrankDesc* __restrict__ descs,
                                                                     int ndesc, const ZLowrankDesc single, int pairs, float cscale, int shard,
-                                                                    int nshards) {
+                                                                    int nshards, const ZTables tables) {
     pdl_wait();
     after(pair_weights);
     constexpr int PC = RANK <= 2 ? 16 : 8;  // pairs per chunk
@@ -371,9 +404,13 @@ __global__ void __launch_bounds__(kZThreads) z_lowrank_tiles_kernel(const float*
     __shared__ __align__(16) float b_sh[2][PC][RANK][TC];
     __shared__ float w_sh[2][PC];
 
+    if (static_cast<int>(blockIdx.x) < tables.blocks) {
+        z_table_block(pair_weights, tables.descs, tables.ndesc, static_cast<int>(blockIdx.x), pairs, shard, nshards, tables.z_all);
+        return;
+    }
     // which matrix, which tile
     ZLowrankDesc d = single;
-    int tile = static_cast<int>(blockIdx.x);
+    int tile = static_cast<int>(blockIdx.x) - tables.blocks;
     int r0 = 0, nr = d.rows;
     if (ndesc > 0) {
         int i = 0;
@@ -790,6 +827,25 @@ int get_scratch(size_t floats, float** out) {
 
 }  // namespace
 
+int cross_entropy_launch(const float* logits, int ld, const float* bias, const int8_t* bias_noise, float sigma, const uint8_t* targets, int vocab, int members,
+                         int rows_per_member, int chunks, float* partial, unsigned* counters, float* loss_mean, cudaStream_t st) {
+    const dim3 grid(chunks, members);
+    const bool early = static_cast<long long>(members) * rows_per_member * vocab <= kPdlStreamElems;
+    const bool vec = (vocab % 4) == 0 && (ld % 4) == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0 &&
+                     (reinterpret_cast<uintptr_t>(bias_noise) & 3) == 0;
+    if (vec && vocab <= 128)
+        launch_pdl_if(early, ce_population_vec_kernel<1, 4>, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean);
+    else if (vec && vocab <= 256)
+        launch_pdl_if(early, ce_population_vec_kernel<2, 4>, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean);
+    else if (vec && vocab <= 512)
+        launch_pdl_if(early, ce_population_vec_kernel<4, 2>, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean);
+    else if (vec)
+        launch_pdl_if(early, ce_population_vec_kernel<8, 1>, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean);
+    else
+        launch_pdl_if(early, ce_population_kernel, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean);
+    return check_launch("ce_population_kernel");
+}
+
 bool shape_fitness_applies(int pairs, int mode) { return pairs <= kShapeMaxPairs && mode >= BNF4_FITNESS_SIGN && mode <= BNF4_FITNESS_CENTERED_RANK; }
 int shape_fitness_launch(const float* losses, int pairs, int mode, float clip, float* weights, cudaStream_t st) {
     launch_pdl(shape_fitness_kernel, 1, 1024, 0, st, losses, pairs, mode, clip, weights);
@@ -809,7 +865,7 @@ int z_dense_single(const float* pair_weights, const uint64_t* pair_seeds, uint64
 }  // namespace
 
 int z_dense_table_launch(const float* pair_weights, const uint64_t* pair_seeds, const ZDenseDesc* d_descs, const ZDenseDesc* h_descs, int ndesc, int pairs,
-                         int use_clt, int clt_k, int use_noise_tables, int shard, int nshards, float* z_all, cudaStream_t st) {
+                         int use_clt, int clt_k, int shard, int nshards, float* z_all, cudaStream_t st) {
     long long blocks = 0, elems = 0;
     for (int i = 0; i < ndesc; ++i) {
         int i0 = 0, cnt = 0;
@@ -821,9 +877,9 @@ int z_dense_table_launch(const float* pair_weights, const uint64_t* pair_seeds, 
     const bool early = elems * pairs <= (1ll << 22);
     const dim3 grid(static_cast<unsigned>(blocks));
     if (use_clt != 0 && clt_k == 4)
-        launch_pdl_if(early, z_dense_table_kernel<true>, grid, 256, 0, st, pair_weights, pair_seeds, d_descs, ndesc, pairs, use_clt, clt_k, use_noise_tables, shard, nshards, z_all);
+        launch_pdl_if(early, z_dense_table_kernel<true>, grid, 256, 0, st, pair_weights, pair_seeds, d_descs, ndesc, pairs, use_clt, clt_k, shard, nshards, z_all);
     else
-        launch_pdl_if(early, z_dense_table_kernel<false>, grid, 256, 0, st, pair_weights, pair_seeds, d_descs, ndesc, pairs, use_clt, clt_k, use_noise_tables, shard, nshards, z_all);
+        launch_pdl_if(early, z_dense_table_kernel<false>, grid, 256, 0, st, pair_weights, pair_seeds, d_descs, ndesc, pairs, use_clt, clt_k, shard, nshards, z_all);
     return check_launch("z_dense_table_kernel");
 }
 
@@ -865,7 +921,7 @@ int requantize_batched(const UpdApplyDesc* d_descs, int ndesc, int total_ublocks
 // d_descs: the table in device memory (nullptr with ndesc == 0: the single matrix h_descs[0], passed by value).
 // h_descs: the same table in host memory, for the grid size.
 int z_lowrank_launch(const float* pair_weights, const ZLowrankDesc* d_descs, const ZLowrankDesc* h_descs, int ndesc, int pairs, int rank,
-                     float cscale, int shard, int nshards, cudaStream_t st) {
+                     float cscale, int shard, int nshards, ZTables tables, const ZDenseDesc* h_tables, cudaStream_t st) {
     if (rank < 1 || rank > 4) return set_error(BNF4_ERR_INVALID, "compute_z_lowrank: rank=%d outside [1,4]", rank);
     if (nshards < 1 || shard < 0 || shard >= nshards) return set_error(BNF4_ERR_INVALID, "compute_z_lowrank: shard %d of %d", shard, nshards);
     if (pairs <= 0) return set_error(BNF4_ERR_INVALID, "compute_z_lowrank: pairs=%d", pairs);
@@ -875,15 +931,22 @@ int z_lowrank_launch(const float* pair_weights, const ZLowrankDesc* d_descs, con
         if (ndesc > 0 && nshards > 1 && nr >= nshards && (nr % nshards) == 0) nr /= nshards;
         tiles += static_cast<long long>((nr + kZTileRows - 1) / kZTileRows) * ((h_descs[i].cols + kZTileCols - 1) / kZTileCols);
     }
+    tables.blocks = 0;
+    for (int i = 0; i < tables.ndesc; ++i) {
+        int i0 = 0, cnt = 0;
+        z_dense_range(h_tables[i], shard, nshards, i0, cnt);
+        tables.blocks += (cnt + kZThreads - 1) / kZThreads;
+    }
+    tiles += tables.blocks;
     if (tiles <= 0) return BNF4_OK;
     if (tiles > 0x7fffffffLL) return set_error(BNF4_ERR_INVALID, "compute_z_lowrank: too many tiles");
     const unsigned grid = static_cast<unsigned>(tiles);
     const ZLowrankDesc single = h_descs[0];
     switch (rank) {
-        case 1: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<1>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
-        case 2: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<2>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
-        case 3: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<3>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
-        default: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<4>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards); break;
+        case 1: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<1>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards, tables); break;
+        case 2: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<2>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards, tables); break;
+        case 3: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<3>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards, tables); break;
+        default: launch_pdl_if(grid <= 2048, z_lowrank_tiles_kernel<4>, grid, kZThreads, 0, st, pair_weights, d_descs, ndesc, single, pairs, cscale, shard, nshards, tables); break;
     }
     return check_launch("z_lowrank_tiles_kernel");
 }
@@ -936,21 +999,7 @@ int bnf4_cross_entropy_population(const float* logits, int ld, const float* bias
     if (!logits || !targets || !partial || !loss_mean) return set_error(BNF4_ERR_INVALID, "cross_entropy_population: null pointer");
     if (vocab <= 0 || vocab > 32 * kCeMaxPerLane) return set_error(BNF4_ERR_INVALID, "cross_entropy_population: vocab=%d", vocab);
     if (members > 65535) return set_error(BNF4_ERR_INVALID, "cross_entropy_population: at most 65535 members per call");
-    const dim3 grid(kCeChunks, members);
-    const bool early = static_cast<long long>(members) * rows_per_member * vocab <= kPdlStreamElems;
-    const bool vec = (vocab % 4) == 0 && (ld % 4) == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0 &&
-                     (reinterpret_cast<uintptr_t>(bias_noise) & 3) == 0;
-    if (vec && vocab <= 128)
-        launch_pdl_if(early, ce_population_vec_kernel<1, 4>, grid, 256, 0, S(stream), logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
-    else if (vec && vocab <= 256)
-        launch_pdl_if(early, ce_population_vec_kernel<2, 4>, grid, 256, 0, S(stream), logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
-    else if (vec && vocab <= 512)
-        launch_pdl_if(early, ce_population_vec_kernel<4, 2>, grid, 256, 0, S(stream), logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
-    else if (vec)
-        launch_pdl_if(early, ce_population_vec_kernel<8, 1>, grid, 256, 0, S(stream), logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
-    else
-        launch_pdl_if(early, ce_population_kernel, grid, 256, 0, S(stream), logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial);
-    int rc = check_launch("ce_population_kernel");
+    int rc = cross_entropy_launch(logits, ld, bias, bias_noise, sigma, targets, vocab, members, rows_per_member, kCeChunks, partial, nullptr, loss_mean, S(stream));
     if (rc) return rc;
     launch_pdl(ce_finalize_kernel, (members + 127) / 128, 128, 0, S(stream), partial, members, rows_per_member, loss_mean);
     return check_launch("ce_finalize_kernel");
@@ -1002,7 +1051,7 @@ int bnf4_compute_z_lowrank(const float* pair_weights, const int8_t* A, long long
     if (rows <= 0 || cols <= 0) return BNF4_OK;
     if (!pair_weights || !A || !B || !Z) return set_error(BNF4_ERR_INVALID, "compute_z_lowrank: null pointer");
     const ZLowrankDesc d = {A, A_pair_stride, B, B_pair_stride, Z, rows, cols};
-    return z_lowrank_launch(pair_weights, nullptr, &d, 0, pairs, rank, cscale, 0, 1, S(stream));
+    return z_lowrank_launch(pair_weights, nullptr, &d, 0, pairs, rank, cscale, 0, 1, ZTables{}, nullptr, S(stream));
 }
 
 int bnf4_sumsq(const float* Z, int n, float* sumsq, void* stream) {

@@ -52,7 +52,27 @@ int gemm_nvfp4_device_error(cudaStream_t stream, int* out_code);
 extern int g_gemm_allow_tma_store;
 
 // EFLA recurrence (efla.cu). Parameter block = the public bnf4_efla_desc.
-using EflaParams = bnf4_efla_desc;
+struct EflaParams : bnf4_efla_desc {
+    EflaParams() : bnf4_efla_desc{} {}
+    EflaParams(const bnf4_efla_desc& d) : bnf4_efla_desc(d) {}
+    // member_bias: the bias of sequence s is that of member m = s / seqs_per_bias, *beta_base + (+-bias_sigma) * bias_noise[(m / 2) * bias_stride]
+    // with the sign of the member's parity (the per-member perturbation of a scalar; bias_sigma 0: no noise is read)
+    int member_bias = 0;
+    const float* beta_base = nullptr;
+    const int8_t* bias_noise = nullptr;
+    int bias_stride = 0;
+    float bias_sigma = 0.0f;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ float efla_seq_bias(const EflaParams& p, unsigned seq) {
+    if (p.member_bias) {  // (reference: src/train_efla_lm.cpp:2912-2917)
+        const unsigned member = seq / static_cast<unsigned>(p.seqs_per_bias);
+        const float nz = p.bias_sigma != 0.0f ? static_cast<float>(p.bias_noise[static_cast<size_t>(member >> 1) * p.bias_stride]) : 0.0f;
+        return fmaf((member & 1u) ? -p.bias_sigma : p.bias_sigma, nz, *p.beta_base);
+    }
+    return p.beta_bias_seq != nullptr ? p.beta_bias_seq[seq / static_cast<unsigned>(p.seqs_per_bias)] : p.beta_bias;
+}
+#endif
 int efla_launch(const EflaParams& p, cudaStream_t stream);
 extern int g_efla_chunked;
 // Whole sequences of at most 128 tokens from a zero state, any head_dim (efla_seq.cu).
@@ -68,8 +88,27 @@ struct ZLowrankDesc {
     float* Z;         // [rows][cols]
     int rows, cols;
 };
+struct ZDenseDesc {
+    uint64_t salt;
+    const int8_t* noise;  // the step's noise [pair][n] in memory, for the table form
+    long long zoff;
+    int n;
+    int rows;  // of a matrix: sharded by rows when they divide; 0 for a vector: sharded when it is long enough
+};
+__host__ __device__ inline void z_dense_range(const ZDenseDesc& d, int shard, int nshards, int& i0, int& cnt) {
+    const bool split = nshards > 1 && (d.rows > 0 ? d.rows >= nshards && d.rows % nshards == 0 : d.n >= 4096 && d.n % nshards == 0);
+    cnt = split ? d.n / nshards : d.n;
+    i0 = split ? shard * cnt : 0;
+}
+// Tensors whose Z is formed from noise tables in the same launch (all have `noise` set, for all pairs).
+struct ZTables {
+    const ZDenseDesc* descs = nullptr;  // device
+    int ndesc = 0;
+    int blocks = 0;  // set by the launcher
+    float* z_all = nullptr;
+};
 int z_lowrank_launch(const float* pair_weights, const ZLowrankDesc* d_descs, const ZLowrankDesc* h_descs, int ndesc, int pairs, int rank,
-                     float cscale, int shard, int nshards, cudaStream_t stream);
+                     float cscale, int shard, int nshards, ZTables tables, const ZDenseDesc* h_tables, cudaStream_t stream);
 
 // Apply phase of the ES update over a table of tensors (es_kernels.cu). The table does not change during a model's life: Z is given by
 // an offset into the launch's Z buffer.
@@ -94,26 +133,18 @@ int update_apply_batched(const UpdApplyDesc* d_descs, int ndesc, int total_block
 // The NVFP4 copies alone, from the present weights.
 int requantize_batched(const UpdApplyDesc* d_descs, int ndesc, int total_ublocks, const uint2* tab, cudaStream_t stream);
 
-// Dense-noise Z of a table of tensors in one launch. noise != nullptr: the table of the step's noise [pair][n] that prepare_step left in
-// memory for all pairs; otherwise the values are hashed.
-struct ZDenseDesc {
-    uint64_t salt;
-    const int8_t* noise;
-    long long zoff;
-    int n;
-    int rows;  // of a matrix: sharded by rows when they divide; 0 for a vector: sharded when it is long enough
-};
-__host__ __device__ inline void z_dense_range(const ZDenseDesc& d, int shard, int nshards, int& i0, int& cnt) {
-    const bool split = nshards > 1 && (d.rows > 0 ? d.rows >= nshards && d.rows % nshards == 0 : d.n >= 4096 && d.n % nshards == 0);
-    cnt = split ? d.n / nshards : d.n;
-    i0 = split ? shard * cnt : 0;
-}
+// Dense-noise Z of a table of tensors in one launch, from the hash.
 int z_dense_table_launch(const float* pair_weights, const uint64_t* pair_seeds, const ZDenseDesc* d_descs, const ZDenseDesc* h_descs, int ndesc, int pairs,
-                         int use_clt, int clt_k, int use_noise_tables, int shard, int nshards, float* z_all, cudaStream_t stream);
+                         int use_clt, int clt_k, int shard, int nshards, float* z_all, cudaStream_t stream);
 
 // Fitness shaping of all pairs on the device, from the losses of their members (es_kernels.cu).
 bool shape_fitness_applies(int pairs, int mode);
 int shape_fitness_launch(const float* losses, int pairs, int mode, float clip, float* weights, cudaStream_t stream);
+
+// Mean cross-entropy of every member, `chunks` blocks per member (es_kernels.cu). partial: members * chunks floats. counters: one zeroed word per
+// member, zero again afterwards; nullptr: the partials only.
+int cross_entropy_launch(const float* logits, int ld, const float* bias, const int8_t* bias_noise, float sigma, const uint8_t* targets, int vocab, int members,
+                         int rows_per_member, int chunks, float* partial, unsigned* counters, float* loss_mean, cudaStream_t stream);
 
 void count_launch();
 

@@ -24,10 +24,10 @@ constexpr float kCRankBase = 0.6123724356957945f;  // sqrt(3/8)
 
 // Kernel classes for the optional timing breakdown (bnf4_model_get_timing).
 enum KernelClass : int {
-    KC_GEN_NOISE = 0, KC_BETA_BIAS, KC_EMBED, KC_GEMM_WIN, KC_POS_GELU_NORM, KC_GEMM_QKV, KC_EFLA, KC_ADD_NORM, KC_GEMM_FF1,
+    KC_GEN_NOISE = 0, KC_EMBED, KC_GEMM_WIN, KC_POS_GELU_NORM, KC_GEMM_QKV, KC_EFLA, KC_ADD_NORM, KC_GEMM_FF1,
     KC_GEMM_FF2, KC_GEMM_HEAD, KC_CROSS_ENTROPY, KC_UPDATE_Z, KC_UPDATE_APPLY, KC_REQUANTIZE, KC_NORM_QUANT, kNumClasses
 };
-const char* const kClassNames[kNumClasses] = {"gen_noise", "beta_bias", "embed_quant", "gemm_win", "pos_gelu_norm_quant", "gemm_qkv",
+const char* const kClassNames[kNumClasses] = {"gen_noise", "embed_quant", "gemm_win", "pos_gelu_norm_quant", "gemm_qkv",
                                               "efla_scan", "add_norm_quant", "gemm_ff1_gelu_fp4", "gemm_ff2", "gemm_head",
                                               "cross_entropy", "update_z_sumsq", "update_apply", "requantize_weights", "norm_quant"};
 
@@ -66,17 +66,15 @@ __global__ void __launch_bounds__(256) gen_noise_kernel(const GenDesc* __restric
     d.dst[static_cast<size_t>(pair) * d.pair_stride + o] = static_cast<int8_t>(v);
 }
 
-// beta_bias_eff[l][member] = beta_bias[l] + ns(member) * noise[pair][l]   (reference: src/train_efla_lm.cpp:2912-2917)
-__global__ void beta_bias_kernel(const float* __restrict__ beta_bias, const int8_t* __restrict__ noise, int layers, int members,
-                                 float sigma, float* __restrict__ out) {
+// tokens and targets from mapped host memory, both in one launch
+__global__ void __launch_bounds__(256) copy_tokens_kernel(const uint8_t* src_tokens, const uint8_t* src_targets, int n, uint8_t* tokens, uint8_t* targets) {
     pdl_wait();
-    after(beta_bias, noise);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= layers * members) return;
-    const int l = i / members, m = i - l * members;
-    const float ns = (m & 1) ? -sigma : sigma;
-    const float nz = sigma != 0.0f ? static_cast<float>(noise[static_cast<size_t>(m >> 1) * layers + l]) : 0.0f;
-    out[i] = fmaf(ns, nz, beta_bias[l]);
+    const int i = (blockIdx.x * 256 + threadIdx.x) * 16;
+    const uint8_t* src = blockIdx.y == 0 ? src_tokens : src_targets;
+    uint8_t* dst = blockIdx.y == 0 ? tokens : targets;
+    if (i + 16 <= n && (reinterpret_cast<uintptr_t>(src) & 15) == 0) *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(src + i);
+    else
+        for (int j = i; j < min(n, i + 16); ++j) dst[j] = src[j];
 }
 
 struct Model {
@@ -111,7 +109,9 @@ struct Model {
     // wave buffers
     int8_t* x_q;
     uint8_t *a_h, *sf_h, *a_f, *sf_f;
-    float *qkv, *y, *bb_eff, *ce_partial, *losses;
+    float *qkv, *y, *ce_partial, *losses;
+    unsigned* ce_count;  // arrivals of a member's cross-entropy blocks
+    int ce_chunks = 16;  // of a member's rows: a function of their number only, so that losses do not depend on the wave
     // input stage computed once per (member, distinct token) when the vocabulary is smaller than a member's rows
     bool dedup_input = false;
     uint8_t *tok_ident, *emb_a, *emb_sf;
@@ -242,13 +242,6 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
     const size_t P0 = static_cast<size_t>(p0);
     int launches = 0;
 
-    {   // per-member beta bias for every layer
-        const int n = L * nm;
-        TimedScope ts(m, KC_BETA_BIAS, st);
-        launch_pdl(beta_bias_kernel, (n + 127) / 128, 128, 0, st, m.beta_bias, m.bb_noise + P0 * L, L, nm, sigma, m.bb_eff);
-        TRY(check_launch("beta_bias_kernel"));
-        ++launches;
-    }
     // The embedding row and its input projection depend on (member, token) only. With a byte vocabulary there are V = 256
     // distinct tokens against R = B*T rows per member, so both are computed once per (member, token) (nm*V rows) and the
     // pos+GELU+norm stage gathers its input row by token. Same values as the row-by-row form, 1/16 of the work at R = 4096.
@@ -320,7 +313,7 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
         ++launches;
         {   // recurrence over the whole sequence -> y
             TimedScope ts(m, KC_EFLA, st);
-            bnf4_efla_desc e = {};
+            EflaParams e;
             e.state = nullptr; e.state_fp16 = 1;
             if (half_io) {
                 e.q = qkv16; e.k = qkv16 + H; e.v = qkv16 + 2 * H; e.beta_raw = beta16; e.ld_qkv = 3 * H; e.ld_beta = 1;
@@ -329,26 +322,12 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
                 e.q = m.qkv; e.k = m.qkv + H; e.v = m.qkv + 2 * H; e.beta_raw = m.qkv + 3 * H; e.ld_qkv = FC; e.ld_beta = FC;
                 e.out = m.y; e.ld_out = H;
             }
-            e.beta_bias_seq = m.bb_eff + static_cast<size_t>(l) * nm; e.seqs_per_bias = m.B;
+            e.member_bias = 1; e.beta_base = m.beta_bias + l; e.bias_noise = m.bb_noise + P0 * L + l; e.bias_stride = L; e.bias_sigma = sigma;
+            e.seqs_per_bias = m.B;
             e.hidden = H; e.heads = m.cfg.heads; e.seqs = static_cast<long long>(nm) * m.B; e.T = m.T; e.method = m.cfg.method;
             e.eps = m.cfg.eps;
-            // the generic kernel addresses sequences with blockIdx.z: split large waves
-            if (m.hd == 64) {
-                TRY(efla_launch(e, st));
-                ++launches;
-            } else {
-                for (long long s0 = 0; s0 < e.seqs; s0 += 32768) {
-                    bnf4_efla_desc ee = e;
-                    const long long cnt = std::min<long long>(32768, e.seqs - s0);
-                    const size_t ro = static_cast<size_t>(s0) * m.T;
-                    ee.q = m.qkv + ro * FC; ee.k = m.qkv + H + ro * FC; ee.v = m.qkv + 2 * H + ro * FC; ee.beta_raw = e.beta_raw + ro * FC;
-                    ee.out = m.y + ro * H; ee.seqs = cnt;
-                    if ((s0 % m.B) != 0) return set_error(BNF4_ERR_INVALID, "efla split not aligned to batch");
-                    ee.beta_bias_seq = e.beta_bias_seq + s0 / m.B;
-                    TRY(efla_launch(ee, st));
-                    ++launches;
-                }
-            }
+            TRY(efla_launch(e, st));
+            ++launches;
         }
         {   // residual add + abs-mean norm -> a_h; t for ff1
             TimedScope ts(m, KC_ADD_NORM, st);
@@ -403,10 +382,10 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
     // head -> logits (in the qkv buffer, leading dimension V), cross-entropy per member
     TRY(gemm(KC_GEMM_HEAD, m.a_h, m.sf_h, m.q_head, m.sfq_head, V, H, m.s_h, m.qkv, V, m.A_head + P0 * V * r, static_cast<long long>(V) * r, m.t_a, r, m.s_h, 0));
     ++launches;
-    TimedScope ts_ce(m, KC_CROSS_ENTROPY, st, 2);
-    TRY(bnf4_cross_entropy_population(m.qkv, V, m.head_bias, pert ? m.hb_noise + P0 * V : nullptr, sigma, m.targets, V, nm, R, m.ce_partial,
-                                      losses_out, st));
-    launches += 2;
+    TimedScope ts_ce(m, KC_CROSS_ENTROPY, st, 1);
+    TRY(cross_entropy_launch(m.qkv, V, m.head_bias, pert ? m.hb_noise + P0 * V : nullptr, sigma, m.targets, V, nm, R, m.ce_chunks, m.ce_partial, m.ce_count,
+                             losses_out, st));
+    ++launches;
     m.launches_per_wave = launches;
     return BNF4_OK;
 }
@@ -529,11 +508,6 @@ int run_pair_dense(Model& m, int pair, float* losses_out, cudaStream_t st) {
             TRY(plain(m.E_all + lay.ff2[l], H, F, m.qe_ff2[l], m.sfe_ff2[l]));
         }
     }
-    {
-        TimedScope ts(m, KC_BETA_BIAS, st);
-        launch_pdl(beta_bias_kernel, (2 * L + 127) / 128, 128, 0, st, m.beta_bias, m.bb_noise + static_cast<size_t>(pair) * L, L, 2, sigma, m.bb_eff);
-        TRY(check_launch("beta_bias_kernel"));
-    }
     // base product into d, then the two members' noise products added in place (alpha = +-sigma * alpha_base, beta = 1)
     auto noisy = [&](int cls, const uint8_t* a, const uint8_t* sfa, int a_k, const uint8_t* b, const uint8_t* sfb, const uint8_t* be, const uint8_t* sfbe,
                      int n, float alpha, float* d, int ldd) -> int {
@@ -575,9 +549,10 @@ int run_pair_dense(Model& m, int pair, float* losses_out, cudaStream_t st) {
         TRY(noisy(KC_GEMM_QKV, m.a_h, m.sf_h, H, m.q_qkv[l], m.sfq_qkv[l], m.qe_qkv[l], m.sfe_qkv[l], 3 * H + 1, 1.0f, m.qkv, FC));
         {
             TimedScope ts(m, KC_EFLA, st);
-            bnf4_efla_desc e = {};
+            EflaParams e;
             e.state = nullptr; e.state_fp16 = 1; e.q = m.qkv; e.k = m.qkv + H; e.v = m.qkv + 2 * H; e.beta_raw = m.qkv + 3 * H;
-            e.ld_qkv = FC; e.ld_beta = FC; e.beta_bias_seq = m.bb_eff + static_cast<size_t>(l) * 2; e.seqs_per_bias = m.B;
+            e.ld_qkv = FC; e.ld_beta = FC; e.seqs_per_bias = m.B;
+            e.member_bias = 1; e.beta_base = m.beta_bias + l; e.bias_noise = m.bb_noise + static_cast<size_t>(pair) * L + l; e.bias_stride = L; e.bias_sigma = sigma;
             e.hidden = H; e.heads = m.cfg.heads; e.seqs = 2LL * m.B; e.T = m.T; e.method = m.cfg.method; e.eps = m.cfg.eps;
             e.out = m.y; e.ld_out = H;
             TRY(efla_launch(e, st));
@@ -619,9 +594,9 @@ int run_pair_dense(Model& m, int pair, float* losses_out, cudaStream_t st) {
         }
     }
     TRY(noisy(KC_GEMM_HEAD, m.a_h, m.sf_h, H, m.q_head, m.sfq_head, m.qe_head, m.sfe_head, V, m.s_h, m.qkv, V));
-    TimedScope ts_ce(m, KC_CROSS_ENTROPY, st, 2);
-    return bnf4_cross_entropy_population(m.qkv, V, m.head_bias, m.hb_noise + static_cast<size_t>(pair) * V, sigma, m.targets, V, 2, R, m.ce_partial,
-                                         losses_out, st);
+    TimedScope ts_ce(m, KC_CROSS_ENTROPY, st, 1);
+    return cross_entropy_launch(m.qkv, V, m.head_bias, m.hb_noise + static_cast<size_t>(pair) * V, sigma, m.targets, V, 2, R, m.ce_chunks, m.ce_partial, m.ce_count,
+                                losses_out, st);
 }
 
 }  // namespace
@@ -699,12 +674,15 @@ int update_z(Model& m, const float* pair_weights, int shard, int nshards, float*
     }
     float* zb = z_ext != nullptr ? z_ext : m.Z_all;
     TimedScope ts(m, KC_UPDATE_Z, st, 2);
-    if (!m.dense) TRY(z_lowrank_launch(pair_weights, dtab, h.data(), static_cast<int>(h.size()), m.pairs_step, m.r, m.c_r, shard, nshards, st));
-    // the fp32 vectors (in the dense mode the matrices too: Z[i] = sum_p w_p noise(mix(seed_p, salt), i), the reference's
-    // compute_z_sumsq, src/efla_lm_kernels.cu:1854-1890); the vectors' noise lies in memory when this process evaluated every pair
-    const int tables = m.eval_begin == 0 && m.eval_end == m.pairs_step;
-    return z_dense_table_launch(pair_weights, m.pair_seeds, m.zdense, m.h_zdense.data(), static_cast<int>(m.h_zdense.size()), m.pairs_step, m.cfg.use_clt,
-                                m.cfg.clt_k, tables, shard, nshards, zb, st);
+    const int nz = static_cast<int>(m.h_zdense.size());
+    if (m.dense)  // Z[i] = sum_p w_p noise(mix(seed_p, salt), i): the reference's compute_z_sumsq, src/efla_lm_kernels.cu:1854-1890
+        return z_dense_table_launch(pair_weights, m.pair_seeds, m.zdense, m.h_zdense.data(), nz, m.pairs_step, m.cfg.use_clt, m.cfg.clt_k, shard, nshards, zb, st);
+    // the fp32 vectors' noise lies in memory when this process evaluated every pair of the step; otherwise it is hashed again
+    ZTables tables;
+    if (m.eval_begin == 0 && m.eval_end == m.pairs_step) { tables.descs = m.zdense; tables.ndesc = nz; tables.z_all = zb; }
+    TRY(z_lowrank_launch(pair_weights, dtab, h.data(), static_cast<int>(h.size()), m.pairs_step, m.r, m.c_r, shard, nshards, tables, m.h_zdense.data(), st));
+    if (tables.ndesc > 0) return BNF4_OK;
+    return z_dense_table_launch(pair_weights, m.pair_seeds, m.zdense, m.h_zdense.data(), nz, m.pairs_step, m.cfg.use_clt, m.cfg.clt_k, shard, nshards, zb, st);
 }
 
 // Applies the precomputed Z of every tensor (sum of squares, RMS-EMA, gated update) and renews the NVFP4 copies of the weights: three
@@ -826,6 +804,8 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     m->M = static_cast<long long>(W) * m->R;
     if (m->M > 0x7fffffffLL / 8) { delete m; return set_error(BNF4_ERR_INVALID, "model_create: wave of %d members is too large", W); }
 
+    // one block of eight warps per 64 rows of a member, 16 to 64 blocks: a validation pass has one member only
+    m->ce_chunks = std::min(64, std::max(16, m->R / 64));
     const int V = m->V, H = m->H, F = m->F, L = m->L, T = m->T, r = m->r, P = cfg->max_pairs;
     const size_t hh = static_cast<size_t>(H) * H, hf = static_cast<size_t>(H) * F;
     int rc = 0;
@@ -860,7 +840,7 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
         A_(tok_ident, V); A_(emb_a, Er * H / 2); A_(emb_sf, sf_bytes(static_cast<int>(Er), H)); A_(emb_t, Er * r); A_(y_emb, Er * H);
     }
     // the logits (V columns) share the q | k | v | beta buffer: a model narrower than its vocabulary needs the wider of the two
-    A_(qkv, Mr * std::max(m->FC, V)); A_(y, Mr * H); A_(bb_eff, static_cast<size_t>(L) * W); A_(ce_partial, static_cast<size_t>(W) * 16); A_(losses, W);
+    A_(qkv, Mr * std::max(m->FC, V)); A_(y, Mr * H); A_(ce_partial, static_cast<size_t>(W) * m->ce_chunks); A_(ce_count, W); A_(losses, W);
     A_(t_a, Mr * 4 * r); A_(t_f, Mr * r);
     if (m->dense) {
         const DenseLayout lay = dense_layout(*m);
@@ -1061,6 +1041,19 @@ int bnf4_model_get_weights(void* handle, bnf4_model_weights* w) {
 int bnf4_model_set_tokens(void* handle, const uint8_t* tokens, const uint8_t* targets, int on_device, void* stream) {
     if (!handle || !tokens || !targets) return set_error(BNF4_ERR_INVALID, "model_set_tokens: null argument");
     Model& m = *M(handle);
+    // Device memory and pinned host memory (which the device can read) are copied by one kernel: two copies through the copy engine
+    // cost several microseconds of stream time each. Pageable host memory goes through the runtime's staging.
+    auto device_address = [&](const uint8_t* ptr) -> const uint8_t* {
+        if (on_device) return ptr;
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, ptr) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        return at.type == cudaMemoryTypeHost ? static_cast<const uint8_t*>(at.devicePointer) : nullptr;
+    };
+    const uint8_t *dt = device_address(tokens), *dg = device_address(targets);
+    if (dt != nullptr && dg != nullptr) {
+        launch_pdl(copy_tokens_kernel, dim3((m.R + 4095) / 4096, 2), 256, 0, S(stream), dt, dg, m.R, m.tokens, m.targets);
+        return check_launch("copy_tokens_kernel");
+    }
     const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     TRY(check_cuda(cudaMemcpyAsync(m.tokens, tokens, m.R, kind, S(stream)), "cudaMemcpyAsync(tokens)"));
     return check_cuda(cudaMemcpyAsync(m.targets, targets, m.R, kind, S(stream)), "cudaMemcpyAsync(targets)");
