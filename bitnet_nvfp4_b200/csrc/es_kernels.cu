@@ -883,7 +883,7 @@ int z_dense_table_launch(const float* pair_weights, const uint64_t* pair_seeds, 
     return check_launch("z_dense_table_kernel");
 }
 
-void update_quant_table(float row_scale, uint2 (&tab)[256]) {
+void update_quant_table(float row_scale, float up, uint2 (&tab)[256]) {
     for (int scaled = 0; scaled < 2; ++scaled)
         for (int amax = 0; amax < 128; ++amax) {  // the arithmetic of quant_block16, IEEE on host and device alike
             float scale = amax > 0 ? static_cast<float>(amax) / 6.0f : 1.0f;
@@ -894,7 +894,7 @@ void update_quant_table(float row_scale, uint2 (&tab)[256]) {
             const float rcp = 1.0f / sf;
             uint2 e;
             memcpy(&e.x, &rcp, 4);
-            e.y = sq;
+            e.y = up == 1.0f ? sq : ue4m3_encode_host(sf * up);
             tab[scaled * 128 + amax] = e;
         }
 }

@@ -268,7 +268,9 @@ constexpr uint32_t kIdescPair256 = kIdescPairM | (256u >> 3 << 17), kIdescPair12
 struct PairMaps {
     CUtensorMap sfa, sfb;
 };
-struct NoMaps {};
+struct NoMaps {
+    CUtensorMap b2;  // the second B operand (GemmParams::b2)
+};
 
 struct KernelArgs {
     GemmParams p;
@@ -277,6 +279,7 @@ struct KernelArgs {
     uint32_t group_magic;  // ceil(2^32 / group_cols) (0 when group_cols == 0)
     const uint8_t* lut;  // table of the block quantiser (EPI_GELU_FP4)
     int total_tiles;
+    int ks_wrap;  // K blocks after which A starts again and B2 follows B (0: no second operand)
     int n_tiles;  // tiles along N (of 256 columns in the pair instances); blockIdx.x = m_tile * n_tiles + n_tile (N fastest: CTAs that share A rows run together)
 };
 
@@ -320,7 +323,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
     const GemmParams& p = args.p;
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int num_ks = (p.k + BK - 1) / BK;
+    const int num_ks = ((p.k + BK - 1) / BK) << (!PAIR && args.ks_wrap > 0 ? 1 : 0);  // K blocks of a tile (both B operands)
     const int total_tiles = args.total_tiles;
 
     const uint32_t bar_full = smem_base + oSmemBar;               // kStages x 8 bytes (PAIR: the leading CTA's count for both)
@@ -487,8 +490,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 const uint8_t* sfa_src = static_cast<const uint8_t*>(p.sfa) + static_cast<size_t>(m_tile) * args.k_atoms * 512;
                 const uint8_t* sfb_src = static_cast<const uint8_t*>(p.sfb) + static_cast<size_t>(n_tile) * args.k_atoms * 512;
                 const int my = m_tile * BM, ny = n_tile * BN;
-                int atoms_left = args.k_atoms;
-                for (int ks = 0; ks < num_ks; ++ks, ++kc) {
+                int atoms_left = args.k_atoms, x = 0, by = ny;
+                const CUtensorMap* bmap = &map_b;
+                for (int ks = 0; ks < num_ks; ++ks, ++kc, x += 128) {
+                    if constexpr (!PAIR) {
+                        if (ks > 0 && ks == args.ks_wrap) {
+                            const int member = my / p.rows_per_member;
+                            x = 0;
+                            by = member * p.b2_rows + ny;
+                            bmap = &maps_sf.b2;
+                            atoms_left = args.k_atoms;
+                            sfa_src = static_cast<const uint8_t*>(p.sfa) + static_cast<size_t>(m_tile) * args.k_atoms * 512;
+                            sfb_src = static_cast<const uint8_t*>(p.sfb2) + static_cast<size_t>(by >> 7) * args.k_atoms * 512;
+                        }
+                    }
                     if (kc >= kStages) {
                         ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, empty_parity, 1));
                         if (!ok) break;
@@ -498,8 +513,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     const uint32_t bar = bar_full + 8 * s;
                     if (elect_one()) {
                         mbar_expect_tx(bar, kStageABytes + kStageBBytes + 2 * sf_bytes_stage);
-                        tma_load_2d(smem_base + kSmemA + s * kStageABytes, &map_a, ks * 128, my, bar);
-                        tma_load_2d(smem_base + kSmemB + s * kStageBBytes, &map_b, ks * 128, ny, bar);
+                        tma_load_2d(smem_base + kSmemA + s * kStageABytes, &map_a, x, my, bar);
+                        tma_load_2d(smem_base + kSmemB + s * kStageBBytes, bmap, x, by, bar);
                         bulk_load_1d(smem_base + kSmemSfa + s * kStageSfBytes, sfa_src, sf_bytes_stage, bar);
                         bulk_load_1d(smem_base + kSmemSfb + s * kStageSfBytes, sfb_src, sf_bytes_stage, bar);
                     }
@@ -537,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * s, full_parity, 2));
                     if (!ok) break;
                     tc_fence_after();
-                    const int nk = min(4, (p.k - ks * BK) / UMMA_K);
+                    const int nk = min(4, (p.k - (ks >= args.ks_wrap ? ks - args.ks_wrap : ks) * BK) / UMMA_K);
                     const uint32_t t_sfa = tmem_base + kSfCol + s * 32;
                     const uint32_t t_sfb = t_sfa + 16;
                     const uint64_t sfa_d = sfadesc0 + static_cast<uint64_t>(s * (kStageSfBytes >> 4));
@@ -1266,6 +1281,7 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
         args.lut = get_quant_lut();
         if (args.lut == nullptr) return BNF4_ERR_CUDA;
     }
+    args.ks_wrap = p.b2 != nullptr ? (p.k + BK - 1) / BK : 0;
     args.use_tma_store = 0;
     if (p.epilogue == EPI_F32 && (reinterpret_cast<uintptr_t>(p.d) & 15) == 0 && (p.ldd % 4) == 0 && p.ldd >= p.n) {
         rc = make_map_2d(&md, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.d, static_cast<uint64_t>(p.n), static_cast<uint64_t>(p.m),
@@ -1305,7 +1321,7 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     // 46.8 -> 43.3, 49.5 -> 47.4. GELU epilogues, whose math takes as long as K 1536: K 1536 52.7 -> 54.6, K 2048 63.8 -> 59.9, K 4096 105 -> 82.
     const long long pair_tiles = static_cast<long long>((p.n + 255) / 256) * ((p.m + 255) / 256);
     const int pair_k = gelu ? 2048 : (p.rank > 1 && p.epilogue != EPI_F32 ? 1536 : 1024);
-    const bool pair = p.k >= pair_k && pair_tiles >= sms / 2 && (rk != 1 || (p.m % 256) == 0);
+    const bool pair = p.b2 == nullptr && p.k >= pair_k && pair_tiles >= sms / 2 && (rk != 1 || (p.m % 256) == 0);
     // the epilogue (and with it the kernel) is a template argument
     auto with_epilogue = [&](auto run) -> int {
         switch (p.epilogue) {
@@ -1333,9 +1349,17 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
         });
     }
     const dim3 grid(static_cast<unsigned>(std::min<long long>(tiles, sms)), 1, 1);
+    NoMaps none;
+    none.b2 = mb;  // unused
+    if (p.b2 != nullptr) {
+        if (p.sfb2 == nullptr || (p.b2_rows % 128) != 0 || p.b2_rows < p.n || p.rows_per_member <= 0 || (p.rows_per_member % BM) != 0)
+            return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: the second operand needs member rows and b2_rows in multiples of 128");
+        const uint64_t members = (static_cast<uint64_t>(p.m) + p.rows_per_member - 1) / p.rows_per_member;
+        rc = make_map_2d(&none.b2, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.b2, static_cast<uint64_t>(p.k) / 2, members * p.b2_rows, static_cast<uint64_t>(p.k) / 2, 128, BN, "B2");
+        if (rc) return rc;
+    }
     return with_epilogue([&](auto epi) -> int {
         constexpr int E = decltype(epi)::value;
-        const NoMaps none;
         return rk == 4 ? launch_t<E, 4>(ma, mb, md, none, args, grid, dev, stream)
                        : (rk == 1 ? launch_t<E, 1>(ma, mb, md, none, args, grid, dev, stream) : launch_t<E, 0>(ma, mb, md, none, args, grid, dev, stream));
     });

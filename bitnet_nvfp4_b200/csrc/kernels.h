@@ -45,7 +45,15 @@ enum GemmEpilogue : int {
     EPI_F16 = BNF4_EPI_F16,            // leading columns as IEEE halves, the rest fp32
 };
 
-using GemmParams = bnf4_gemm_desc;
+struct GemmParams : bnf4_gemm_desc {
+    GemmParams() : bnf4_gemm_desc{} {}
+    GemmParams(const bnf4_gemm_desc& d) : bnf4_gemm_desc(d) {}
+    // Second B operand, accumulated after the first one over the same A: D += alpha A B2_member^T. [members][b2_rows][K] codes and their scale
+    // atoms, b2_rows a multiple of 128; a member's rows (rows_per_member) are a multiple of 128.
+    const void* b2 = nullptr;
+    const void* sfb2 = nullptr;
+    int b2_rows = 0;
+};
 int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream);
 // Reads and clears the device-side error word of the GEMM kernels (0 = none). Synchronises the stream.
 int gemm_nvfp4_device_error(cudaStream_t stream, int* out_code);
@@ -127,7 +135,8 @@ struct UpdApplyDesc {
     int ublock0;     // first 1024-element block in the update launch
 };
 // tab: {1 / scale, scale byte} per block maximum, 128 entries unscaled and 128 with the row scale (update_quant_table).
-void update_quant_table(float row_scale, uint2 (&tab)[256]);
+// `up` (a power of two) is multiplied into the scale bytes only; whoever multiplies with the weights divides alpha by it.
+void update_quant_table(float row_scale, float up, uint2 (&tab)[256]);
 int update_apply_batched(const UpdApplyDesc* d_descs, int ndesc, int total_blocks, int total_ublocks, const float* z_all, const uint2* tab, float* partial,
                          float* inv_rms, int use_adaptive, float beta, float eps, float lr, float thresh, cudaStream_t stream);
 // The NVFP4 copies alone, from the present weights.

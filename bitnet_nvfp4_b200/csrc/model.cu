@@ -19,7 +19,6 @@ namespace bnf4 {
 
 namespace {
 
-constexpr size_t kWeightStageBytes = 2u << 20;  // largest weight set that get_weights stages in pinned memory
 constexpr float kCRankBase = 0.6123724356957945f;  // sqrt(3/8)
 
 // Kernel classes for the optional timing breakdown (bnf4_model_get_timing).
@@ -64,6 +63,65 @@ __global__ void __launch_bounds__(256) gen_noise_kernel(const GenDesc* __restric
         o = r * d.n_major + major;
     }
     d.dst[static_cast<size_t>(pair) * d.pair_stride + o] = static_cast<int8_t>(v);
+}
+
+// One noise matrix of the dense form as an operand of every member's GEMM.
+struct DenseGenDesc {
+    uint64_t salt;    // mixed with the pair seed
+    int8_t* raw;      // [pair][rows][cols] int8 (the embedding, which is looked up), or nullptr:
+    uint8_t* codes;   // [member][member_rows][cols] e2m1 (the - member's with flipped signs) ...
+    uint8_t* sf;      // ... and their scale atoms
+    long long n;
+    int cols, row0, member_rows, scaled;
+    int block0;       // first block of this matrix in the launch
+};
+
+// Noise of the matrices of pairs p0 .. p0 + gridDim.y - 1, quantised on the spot: a thread hashes one 16-element scale block and writes its
+// codes for both members. Bound by the hash (integer pipes); the noise itself never reaches memory.
+__global__ void __launch_bounds__(256) gen_dense_kernel(const DenseGenDesc* __restrict__ descs, int ndesc, uint64_t seed0, uint64_t epoch, int p0, int use_clt, int clt_k,
+                                                        const uint2* __restrict__ tab) {
+    int lo = 0, hi = ndesc - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (descs[mid].block0 <= static_cast<int>(blockIdx.x)) lo = mid; else hi = mid - 1;
+    }
+    const DenseGenDesc d = descs[lo];
+    const long long e0 = (static_cast<long long>(static_cast<int>(blockIdx.x) - d.block0) * 256 + threadIdx.x) * 16;
+    const int pair = blockIdx.y;
+    const NoiseSeed seed = noise_seed(mix_u64(mix_u64(seed0, mix_u64(epoch, static_cast<uint64_t>(p0 + pair))), d.salt));
+    float f[16];
+    float am = 0.0f;
+    if (e0 < d.n) {
+#pragma unroll 4
+        for (int e = 0; e < 16; ++e) {
+            const uint64_t idx = static_cast<uint64_t>(e0 + e);
+            f[e] = static_cast<float>(use_clt != 0 && clt_k == 4 ? noise_clt4(seed, idx) : static_cast<int8_t>(noise_hash(seed.a, idx, use_clt != 0, clt_k)));
+            am = fmaxf(am, fminf(fabsf(f[e]), 127.0f));
+        }
+    }
+    pdl_wait();  // everything above is computed from constants
+    if (e0 >= d.n) return;
+    if (d.raw != nullptr) {
+        uint32_t w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            w[q] = static_cast<uint32_t>(pack4_i8(static_cast<int>(f[4 * q]), static_cast<int>(f[4 * q + 1]), static_cast<int>(f[4 * q + 2]), static_cast<int>(f[4 * q + 3])));
+        *reinterpret_cast<uint4*>(d.raw + static_cast<size_t>(pair) * d.n + e0) = make_uint4(w[0], w[1], w[2], w[3]);
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < 16; ++e) f[e] = fmaxf(f[e], -127.0f);
+    const uint2 ent = tab[d.scaled * 128 + static_cast<int>(am)];
+    const uint32_t c0 = e2m1x8_int(f, __uint_as_float(ent.x)), c1 = e2m1x8_int(f + 8, __uint_as_float(ent.x));
+    const int row = static_cast<int>(e0 / d.cols), col = static_cast<int>(e0 - static_cast<long long>(row) * d.cols);
+    const size_t atoms = sf_k_atoms(d.cols);
+#pragma unroll
+    for (int neg = 0; neg < 2; ++neg) {
+        const size_t r = static_cast<size_t>(2 * pair + neg) * d.member_rows + d.row0 + row;
+        const uint32_t flip = neg ? 0x88888888u : 0u;
+        *reinterpret_cast<uint2*>(d.codes + (r * d.cols + col) / 2) = make_uint2(c0 ^ flip, c1 ^ flip);
+        d.sf[(r >> 7) * atoms * 512 + sf_offset(static_cast<int>(r & 127), col >> 4, static_cast<int>(atoms))] = static_cast<uint8_t>(ent.y);
+    }
 }
 
 // tokens and targets from mapped host memory, both in one launch
@@ -128,12 +186,21 @@ struct Model {
     std::vector<ZDenseDesc> h_zdense;
     ZLowrankDesc *zdesc, *zdesc_ext;  // device tables of the update's matrices: Z inside Z_all / inside a caller's buffer
     int launches_per_wave = 0;
-    uint8_t* h_weights = nullptr;  // pinned staging of get_weights (small models only)
     float* h_step = nullptr;    // bnf4_model_es_step: pinned losses [2 * max_pairs] + pair weights [max_pairs]
     float* d_step_w;            // ... and the shaped pair weights on the device
     // dense (rank 0) mode: the reference driver's own perturbation, one materialised noise matrix per weight matrix and pair,
     // applied as a second GEMM with beta = 1 (src/train_efla_lm.cpp:2359-2367). One pair per wave.
-    bool dense = false;
+    // dense_folded (sigma down to 2^-4): any number of pairs per wave; the noise operands of every member follow the base weights in the
+    // same GEMM (GemmParams::b2). sigma cannot scale part of an accumulation, so the base weights' scale bytes carry 2^sigma_shift (w_up,
+    // exact: a power of two, at most 448) and alpha its inverse. Smaller sigmas run one pair per wave with separate products.
+    bool dense = false, dense_folded = false;
+    float w_up = 1.0f;
+    struct NoiseOperand { uint8_t *codes, *sf; int rows; };
+    NoiseOperand nz_win{}, nz_head{};
+    std::vector<NoiseOperand> nz_qkv, nz_ff1, nz_ff2;
+    DenseGenDesc* dgen = nullptr;  // device table of the noise matrices
+    uint2* dgen_tab = nullptr;     // block quantiser table of the noise (scale bytes without w_up)
+    int num_dgen = 0, dgen_blocks = 0;
     uint64_t step_seed = 0, step_epoch = 0;
     int8_t* E_all = nullptr;                 // noise of one pair, all matrices back to back (order of update_matrices)
     uint8_t *qe_win, *sfe_win, *qe_head, *sfe_head;
@@ -238,9 +305,21 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
     const int H = m.H, F = m.F, L = m.L, V = m.V, R = m.R, FC = m.FC, r = m.r;
     const int rows = nm * R;
     const bool pert = sigma != 0.0f;
-    const int rank = pert ? r : 0;
+    const int rank = pert && !m.dense ? r : 0;
     const size_t P0 = static_cast<size_t>(p0);
+    const float w_down = 1.0f / m.w_up;
     int launches = 0;
+    if (pert && m.dense) {  // the noise matrices of the wave's pairs
+        TimedScope ts(m, KC_GEN_NOISE, st);
+        launch_pdl(gen_dense_kernel, dim3(m.dgen_blocks, nm / 2), 256, 0, st, m.dgen, m.num_dgen, m.step_seed, m.step_epoch, p0, m.cfg.use_clt, m.cfg.clt_k, m.dgen_tab);
+        TRY(check_launch("gen_dense_kernel"));
+        ++launches;
+    }
+    // adds a member's noise operand (dense form) to a GEMM
+    auto noise = [&](GemmParams& g, const Model::NoiseOperand& z) {
+        if (pert && m.dense) { g.b2 = z.codes; g.sfb2 = z.sf; g.b2_rows = z.rows; }
+    };
+    const Model::NoiseOperand no_noise{};
 
     // The embedding row and its input projection depend on (member, token) only. With a byte vocabulary there are V = 256
     // distinct tokens against R = B*T rows per member, so both are computed once per (member, token) (nm*V rows) and the
@@ -256,27 +335,29 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
         p.embA = m.embA + P0 * V * r; p.embB = m.embB + P0 * H * r; p.embA_pair_stride = static_cast<long long>(V) * r;
         p.embB_pair_stride = static_cast<long long>(H) * r; p.rank = r;
         p.out_codes = dedup ? m.emb_a : m.a_h; p.out_sf = dedup ? m.emb_sf : m.sf_h;
-        if (pert) { p.tvec = m.tB_win + P0 * H * r; p.tvec_pair_stride = static_cast<long long>(H) * r; p.nvec = r; p.t_out = dedup ? m.emb_t : m.t_a; }
-        TRY(rowquant_dispatch(FE_EMBED_LOWRANK, p, st));
+        if (rank > 0) { p.tvec = m.tB_win + P0 * H * r; p.tvec_pair_stride = static_cast<long long>(H) * r; p.nvec = r; p.t_out = dedup ? m.emb_t : m.t_a; }
+        if (m.dense) { p.emb_noise = pert ? m.E_all : nullptr; p.noise_pair_stride = static_cast<long long>(V) * H; }
+        TRY(rowquant_dispatch(m.dense ? FE_EMBED_DENSE : FE_EMBED_LOWRANK, p, st));
         ++launches;
     }
     auto gemm_rows = [&](int cls, int grows, int g_rpm, const uint8_t* a, const uint8_t* sfa, const uint8_t* b, const uint8_t* sfb, int n, int k,
                          float alpha, float* d, int ldd, const int8_t* A, long long A_stride, const int32_t* t, int t_stride, float out_scale,
-                         int group_cols) {
+                         int group_cols, const Model::NoiseOperand& z) {
         TimedScope ts(m, cls, st);
-        bnf4_gemm_desc g = {};
-        g.a = a; g.b = b; g.sfa = sfa; g.sfb = sfb; g.m = grows; g.n = n; g.k = k; g.alpha = alpha; g.d = d; g.ldd = ldd;
+        GemmParams g;
+        g.a = a; g.b = b; g.sfa = sfa; g.sfb = sfb; g.m = grows; g.n = n; g.k = k; g.alpha = alpha * w_down; g.d = d; g.ldd = ldd;
         g.epilogue = EPI_F32; g.rank = rank; g.rows_per_member = g_rpm; g.lora_t = t; g.t_stride = t_stride; g.lora_A = A;
         g.lora_A_pair_stride = A_stride; g.lora_scale = (sigma * out_scale) * m.c_r; g.group_cols = group_cols;
+        noise(g, z);
         return gemm_nvfp4_launch(g, st);
     };
     auto gemm = [&](int cls, const uint8_t* a, const uint8_t* sfa, const uint8_t* b, const uint8_t* sfb, int n, int k, float alpha, float* d,
-                    int ldd, const int8_t* A, long long A_stride, const int32_t* t, int t_stride, float out_scale, int group_cols) {
-        return gemm_rows(cls, rows, R, a, sfa, b, sfb, n, k, alpha, d, ldd, A, A_stride, t, t_stride, out_scale, group_cols);
+                    int ldd, const int8_t* A, long long A_stride, const int32_t* t, int t_stride, float out_scale, int group_cols, const Model::NoiseOperand& z) {
+        return gemm_rows(cls, rows, R, a, sfa, b, sfb, n, k, alpha, d, ldd, A, A_stride, t, t_stride, out_scale, group_cols, z);
     };
     // input projection -> y (per row) or y_emb (per member and token)
     TRY(gemm_rows(KC_GEMM_WIN, erows, e_rpm, dedup ? m.emb_a : m.a_h, dedup ? m.emb_sf : m.sf_h, m.q_win, m.sfq_win, H, H, m.s_h,
-                  dedup ? m.y_emb : m.y, H, m.A_win + P0 * H * r, static_cast<long long>(H) * r, dedup ? m.emb_t : m.t_a, r, m.s_h, 0));
+                  dedup ? m.y_emb : m.y, H, m.A_win + P0 * H * r, static_cast<long long>(H) * r, dedup ? m.emb_t : m.t_a, r, m.s_h, 0, m.dense ? m.nz_win : no_noise));
     ++launches;
     {   // + pos, GELU -> residual stream x_q; abs-mean norm -> a_h; t for qkv[0]
         TimedScope ts(m, KC_POS_GELU_NORM, st);
@@ -286,21 +367,21 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
         if (dedup) { p.gather_rows = V; p.tokens = m.tokens; p.token_stride = 1; p.row_mod = R; }
         p.pos_noise = pert ? m.pos_noise + P0 * m.T * H : nullptr; p.noise_pair_stride = static_cast<long long>(m.T) * H;
         p.act_scale = m.cfg.act_scale; p.norm_scale = m.cfg.ln_scale; p.out_codes = m.a_h; p.out_sf = m.sf_h;
-        if (pert) { p.tvec = m.tB_qkv[0] + P0 * 4 * r * H; p.tvec_pair_stride = static_cast<long long>(4) * r * H; p.nvec = 4 * r; p.t_out = m.t_a; }
+        if (rank > 0) { p.tvec = m.tB_qkv[0] + P0 * 4 * r * H; p.tvec_pair_stride = static_cast<long long>(4) * r * H; p.nvec = 4 * r; p.t_out = m.t_a; }
         TRY(rowquant_dispatch(FE_POS_GELU_ABSMEAN, p, st));
         ++launches;
     }
     // With heads of 64 and the chunked scan, q | k | v travel as IEEE halves (the scan rounds its operands to fp16 anyway) and
     // so does the scan's output: the projection writes [rows][3H] halves + [rows] fp32 beta_raw into the qkv buffer, the
     // scan writes [rows][H] halves into the y buffer. Otherwise everything stays fp32 (the reference's interface).
-    const bool half_io = m.hd == 64 && g_efla_chunked != 0;
+    const bool half_io = m.hd == 64 && g_efla_chunked != 0 && !m.dense;
     __half* qkv16 = reinterpret_cast<__half*>(m.qkv);
     float* beta16 = m.qkv + (static_cast<size_t>(rows) * 3 * H + 1) / 2;  // behind the halves
     for (int l = 0; l < L; ++l) {
         // fused QKV(+beta) projection; out_scale is folded into the weight scales (alpha = 1)
         if (half_io) {
             TimedScope ts(m, KC_GEMM_QKV, st);
-            bnf4_gemm_desc g = {};
+            GemmParams g;
             g.a = m.a_h; g.b = m.q_qkv[l]; g.sfa = m.sf_h; g.sfb = m.sfq_qkv[l]; g.m = rows; g.n = 3 * H + 1; g.k = H; g.alpha = 1.0f;
             g.epilogue = EPI_F16; g.d_f16 = qkv16; g.ld_f16 = 3 * H; g.n_f16 = 3 * H; g.d = beta16; g.ldd = 1;
             g.rank = rank; g.rows_per_member = R; g.lora_t = m.t_a; g.t_stride = 4 * r; g.lora_A = m.A_qkv[l] + P0 * (3 * H + 1) * r;
@@ -308,7 +389,7 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
             TRY(gemm_nvfp4_launch(g, st));
         } else {
             TRY(gemm(KC_GEMM_QKV, m.a_h, m.sf_h, m.q_qkv[l], m.sfq_qkv[l], 3 * H + 1, H, 1.0f, m.qkv, FC, m.A_qkv[l] + P0 * (3 * H + 1) * r,
-                     static_cast<long long>(3 * H + 1) * r, m.t_a, 4 * r, m.s_h, H));
+                     static_cast<long long>(3 * H + 1) * r, m.t_a, 4 * r, m.s_h, H, m.dense ? m.nz_qkv[l] : no_noise));
         }
         ++launches;
         {   // recurrence over the whole sequence -> y
@@ -336,30 +417,32 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
             p.inout_i8 = m.x_q; p.in_f32 = m.y; p.ld_in = H; p.in_f16 = half_io ? 1 : 0;
             p.add_scale = m.cfg.residual_scale; p.norm_scale = m.cfg.ln_scale;
             p.out_codes = m.a_h; p.out_sf = m.sf_h;
-            if (pert) { p.tvec = m.tB_ff1[l] + P0 * r * H; p.tvec_pair_stride = static_cast<long long>(r) * H; p.nvec = r; p.t_out = m.t_a; }
+            if (rank > 0) { p.tvec = m.tB_ff1[l] + P0 * r * H; p.tvec_pair_stride = static_cast<long long>(r) * H; p.nvec = r; p.t_out = m.t_a; }
             RowQuantParams pz(p);
-            if (pert) { pz.zero_t = m.t_f; pz.zero_n = r; }  // ff1 accumulates the projections for ff2 there
+            if (rank > 0) { pz.zero_t = m.t_f; pz.zero_n = r; }  // ff1 accumulates the projections for ff2 there
             TRY(rowquant_dispatch(FE_ADD_ABSMEAN, pz, st));
             ++launches;
         }
         {   // ff1 with GELU -> int8 -> FP4 epilogue, projections for ff2
             TimedScope ts(m, KC_GEMM_FF1, st);
-            bnf4_gemm_desc g = {};
-            g.a = m.a_h; g.b = m.q_ff1[l]; g.sfa = m.sf_h; g.sfb = m.sfq_ff1[l]; g.m = rows; g.n = F; g.k = H; g.alpha = m.s_h;
+            GemmParams g;
+            g.a = m.a_h; g.b = m.q_ff1[l]; g.sfa = m.sf_h; g.sfb = m.sfq_ff1[l]; g.m = rows; g.n = F; g.k = H; g.alpha = m.s_h * w_down;
             g.epilogue = EPI_GELU_FP4; g.act_scale = m.cfg.mlp_act_scale; g.d_codes = m.a_f; g.d_sf = m.sf_f;
             g.rank = rank; g.rows_per_member = R; g.lora_t = m.t_a; g.t_stride = r; g.lora_A = m.A_ff1[l] + P0 * F * r;
             g.lora_A_pair_stride = static_cast<long long>(F) * r; g.lora_scale = (sigma * m.s_h) * m.c_r;
-            if (pert) { g.next_tvec = m.tB_ff2[l] + P0 * r * F; g.next_tvec_pair_stride = static_cast<long long>(r) * F; g.next_nvec = r; g.next_t = m.t_f; }
+            if (m.dense) noise(g, m.nz_ff1[l]);
+            if (rank > 0) { g.next_tvec = m.tB_ff2[l] + P0 * r * F; g.next_tvec_pair_stride = static_cast<long long>(r) * F; g.next_nvec = r; g.next_t = m.t_f; }
             TRY(gemm_nvfp4_launch(g, st));
             ++launches;
         }
         {   // ff2, added into the residual stream by the epilogue: the fp32 product never leaves the SM
             TimedScope ts(m, KC_GEMM_FF2, st);
-            bnf4_gemm_desc g = {};
-            g.a = m.a_f; g.b = m.q_ff2[l]; g.sfa = m.sf_f; g.sfb = m.sfq_ff2[l]; g.m = rows; g.n = H; g.k = F; g.alpha = m.s_f;
+            GemmParams g;
+            g.a = m.a_f; g.b = m.q_ff2[l]; g.sfa = m.sf_f; g.sfb = m.sfq_ff2[l]; g.m = rows; g.n = H; g.k = F; g.alpha = m.s_f * w_down;
             g.epilogue = EPI_ADD_I8; g.resid = m.x_q; g.ld_resid = H; g.add_scale = m.cfg.mlp_residual_scale;
             g.rank = rank; g.rows_per_member = R; g.lora_t = m.t_f; g.t_stride = r; g.lora_A = m.A_ff2[l] + P0 * H * r;
             g.lora_A_pair_stride = static_cast<long long>(H) * r; g.lora_scale = (sigma * m.s_f) * m.c_r;
+            if (m.dense) noise(g, m.nz_ff2[l]);
             TRY(gemm_nvfp4_launch(g, st));
             ++launches;
         }
@@ -370,7 +453,7 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
             p.rows = rows; p.cols_in = H; p.cols_out = H; p.rows_per_member = R; p.sigma = sigma;
             p.in_i8 = m.x_q; p.ld_in = H; p.norm_scale = m.cfg.ln_scale;
             p.out_codes = m.a_h; p.out_sf = m.sf_h;
-            if (pert) {
+            if (rank > 0) {
                 if (last) { p.tvec = m.tB_head + P0 * r * H; p.tvec_pair_stride = static_cast<long long>(r) * H; p.nvec = r; }
                 else { p.tvec = m.tB_qkv[l + 1] + P0 * 4 * r * H; p.tvec_pair_stride = static_cast<long long>(4) * r * H; p.nvec = 4 * r; }
                 p.t_out = m.t_a;
@@ -380,7 +463,7 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
         }
     }
     // head -> logits (in the qkv buffer, leading dimension V), cross-entropy per member
-    TRY(gemm(KC_GEMM_HEAD, m.a_h, m.sf_h, m.q_head, m.sfq_head, V, H, m.s_h, m.qkv, V, m.A_head + P0 * V * r, static_cast<long long>(V) * r, m.t_a, r, m.s_h, 0));
+    TRY(gemm(KC_GEMM_HEAD, m.a_h, m.sf_h, m.q_head, m.sfq_head, V, H, m.s_h, m.qkv, V, m.A_head + P0 * V * r, static_cast<long long>(V) * r, m.t_a, r, m.s_h, 0, m.dense ? m.nz_head : no_noise));
     ++launches;
     TimedScope ts_ce(m, KC_CROSS_ENTROPY, st, 1);
     TRY(cross_entropy_launch(m.qkv, V, m.head_bias, pert ? m.hb_noise + P0 * V : nullptr, sigma, m.targets, V, nm, R, m.ce_chunks, m.ce_partial, m.ce_count,
@@ -391,9 +474,9 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
 }
 
 // run_wave, replayed from a captured graph when the model's graph mode is on (never while the timing breakdown records events:
-// events recorded during a capture cannot be read back). Results are those of the eager launches: same kernels, same arguments.
+// events recorded during a capture cannot be read back; never in the dense mode: its noise launch carries the step's seed). Results are those of the eager launches: same kernels, same arguments.
 int run_wave_cached(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStream_t st) {
-    if (!m.use_graph || m.timing) return run_wave(m, p0, nm, sigma, losses_out, st);
+    if (!m.use_graph || m.timing || m.dense) return run_wave(m, p0, nm, sigma, losses_out, st);
     const uint32_t sb = __builtin_bit_cast(uint32_t, sigma);
     Model::WaveGraph* e = nullptr;
     for (Model::WaveGraph& g : m.graphs)
@@ -459,7 +542,7 @@ DenseLayout dense_layout(const Model& m) {
     return d;
 }
 
-// One antithetic pair in the reference driver's own form: dense CLT noise matrices from the pair's seeds
+// One antithetic pair in the reference driver's own form, product by product (sigma below 2^-4; larger ones are folded into run_wave): dense CLT noise matrices from the pair's seeds
 // (set_noise_seeds, src/train_efla_lm.cpp:1946-2012), quantised to NVFP4 like the base weights, every projection as
 // D = alpha A W^T followed by D += (+-sigma alpha) A E^T (gemm_noisy :2349-2379, gemm_qkvb :2507-2523, gemm_ff1_gelu :2724-2747),
 // rows [0, R) = the + member, [R, 2R) = the - member. Layer-major over the tokens like the rank-r path.
@@ -741,10 +824,39 @@ int build_update_tables(Model& m) {
     }
     m.num_upd = static_cast<int>(h.size());
     uint2 tab[256];
-    update_quant_table(m.s_h, tab);
+    update_quant_table(m.s_h, m.w_up, tab);
     TRY(check_cuda(cudaMemcpy(m.upd_descs, h.data(), h.size() * sizeof(UpdApplyDesc), cudaMemcpyHostToDevice), "cudaMemcpy(upd_descs)"));
     TRY(check_cuda(cudaMemcpy(m.zdense, m.h_zdense.data(), m.h_zdense.size() * sizeof(ZDenseDesc), cudaMemcpyHostToDevice), "cudaMemcpy(zdense)"));
     return check_cuda(cudaMemcpy(m.upd_tab, tab, sizeof(tab), cudaMemcpyHostToDevice), "cudaMemcpy(upd_tab)");
+}
+
+// Table of the dense form's noise matrices (salts: set_noise_seeds, src/train_efla_lm.cpp:1946-2012).
+int build_dense_tables(Model& m) {
+    const long long H = m.H, F = m.F, V = m.V;
+    std::vector<DenseGenDesc> h;
+    auto add = [&](uint64_t salt, long long rows, int cols, const Model::NoiseOperand* z, int row0, int scaled) {
+        DenseGenDesc d = {};
+        d.salt = salt; d.n = rows * cols; d.cols = cols; d.row0 = row0; d.scaled = scaled; d.block0 = m.dgen_blocks;
+        if (z != nullptr) { d.codes = z->codes; d.sf = z->sf; d.member_rows = z->rows; }
+        else d.raw = m.E_all;
+        h.push_back(d);
+        m.dgen_blocks += static_cast<int>((d.n / 16 + 255) / 256);
+    };
+    add(kSaltEmb, V, m.H, nullptr, 0, 0);
+    add(kSaltWin, H, m.H, &m.nz_win, 0, 0);
+    for (int l = 0; l < m.L; ++l) {
+        const uint64_t lu = static_cast<uint64_t>(l);
+        const uint64_t gs[4] = {mix_u64(lu, kSaltWq), mix_u64(lu, kSaltWk), mix_u64(lu, kSaltWv), mix_u64(lu, kSaltWbeta)};
+        for (int g = 0; g < 4; ++g) add(gs[g], g < 3 ? H : 1, m.H, &m.nz_qkv[l], g * m.H, 1);
+        add(mix_u64(lu, kSaltFf1), F, m.H, &m.nz_ff1[l], 0, 0);
+        add(mix_u64(lu, kSaltFf2), H, m.F, &m.nz_ff2[l], 0, 0);
+    }
+    add(kSaltHead, V, m.H, &m.nz_head, 0, 0);
+    m.num_dgen = static_cast<int>(h.size());
+    uint2 tab[256];
+    update_quant_table(m.s_h, 1.0f, tab);
+    TRY(check_cuda(cudaMemcpy(m.dgen, h.data(), h.size() * sizeof(DenseGenDesc), cudaMemcpyHostToDevice), "cudaMemcpy(dgen)"));
+    return check_cuda(cudaMemcpy(m.dgen_tab, tab, sizeof(tab), cudaMemcpyHostToDevice), "cudaMemcpy(dgen_tab)");
 }
 
 }  // namespace
@@ -759,7 +871,6 @@ int bnf4_model_destroy(void* handle) {
     if (m->cap_stream) cudaStreamDestroy(m->cap_stream);
     for (void* p : m->allocs) cudaFree(p);
     if (m->h_step) cudaFreeHost(m->h_step);
-    if (m->h_weights) cudaFreeHost(m->h_weights);
     for (cudaEvent_t e : m->free_events) cudaEventDestroy(e);
     for (const Model::Span& sp : m->spans) { cudaEventDestroy(sp.a); cudaEventDestroy(sp.b); }
     delete m;
@@ -787,6 +898,8 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     m->V = cfg->vocab; m->H = cfg->hidden; m->F = cfg->hidden * cfg->mlp_mult; m->L = cfg->layers; m->T = cfg->seq; m->B = cfg->batch;
     m->R = m->B * m->T; m->FC = (3 * m->H + 1 + 31) & ~31; m->hd = m->H / cfg->heads;
     m->dense = cfg->rank == 0;
+    m->dense_folded = m->dense && cfg->sigma_shift <= 4;  // scale bytes of int8 weights are at most 127/6, 22 rounded: 352 of 448 with 2^4
+    if (m->dense_folded) m->w_up = static_cast<float>(1 << cfg->sigma_shift);
     m->r = m->dense ? 1 : cfg->rank;  // the rank-r tables are sized for rank 1 (and left unused) in the dense mode
     m->s_h = 1.0f / std::sqrt(static_cast<float>(m->H));
     m->s_f = 1.0f / std::sqrt(static_cast<float>(m->F));
@@ -797,7 +910,13 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     const double row_bytes = m->H * (1.0 + 0.5625 + 4.0) + m->F * 0.5625 + m->FC * 4.0 + 20.0 * m->r;
     const int w_auto = static_cast<int>(std::min(256.0, std::max(2.0, 12e9 / (row_bytes * static_cast<double>(m->R)))));
     int W = cfg->wave_members > 0 ? cfg->wave_members : w_auto;
-    if (m->dense) W = 2;  // one pair per wave: its noise matrices exist once
+    const int qkv_rows = (3 * m->H + 1 + 127) / 128 * 128;  // rows of a member's noise operands, whole scale atoms
+    auto pad128 = [](int n) { return (n + 127) / 128 * 128; };
+    if (m->dense_folded) {  // every member of a wave has noise operands of its own: at most 2 GB of them
+        const double per_member = 0.5625 * (static_cast<double>(pad128(m->H) + pad128(m->V)) * m->H +
+                                            m->L * (static_cast<double>(qkv_rows + pad128(m->F)) * m->H + static_cast<double>(pad128(m->H)) * m->F));
+        W = static_cast<int>(std::min<double>(W, std::max(2.0, 2e9 / per_member)));
+    } else if (m->dense) W = 2;  // one pair per wave: its noise matrices exist once
     W = std::min(W, 2 * cfg->max_pairs);
     W = std::max(2, W & ~1);
     m->W = W;
@@ -834,7 +953,7 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     A_(pos_noise, static_cast<size_t>(P) * T * H); A_(hb_noise, static_cast<size_t>(P) * V); A_(bb_noise, static_cast<size_t>(P) * L);
     const size_t Mr = static_cast<size_t>(m->M);
     A_(x_q, Mr * H); A_(a_h, Mr * H / 2); A_(sf_h, sf_bytes(static_cast<int>(Mr), H)); A_(a_f, Mr * F / 2); A_(sf_f, sf_bytes(static_cast<int>(Mr), F));
-    m->dedup_input = V <= 256 && V < m->R;
+    m->dedup_input = V <= 256 && V < m->R && (!m->dense || (m->dense_folded && V % 128 == 0));  // (a member's rows: whole tiles in the dense form)
     if (m->dedup_input) {
         const size_t Er = static_cast<size_t>(W) * V;
         A_(tok_ident, V); A_(emb_a, Er * H / 2); A_(emb_sf, sf_bytes(static_cast<int>(Er), H)); A_(emb_t, Er * r); A_(y_emb, Er * H);
@@ -842,7 +961,18 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     // the logits (V columns) share the q | k | v | beta buffer: a model narrower than its vocabulary needs the wider of the two
     A_(qkv, Mr * std::max(m->FC, V)); A_(y, Mr * H); A_(ce_partial, static_cast<size_t>(W) * m->ce_chunks); A_(ce_count, W); A_(losses, W);
     A_(t_a, Mr * 4 * r); A_(t_f, Mr * r);
-    if (m->dense) {
+    if (m->dense_folded) {
+        A_(E_all, static_cast<size_t>(W / 2) * V * H);  // the embedding's noise
+        auto operand = [&](Model::NoiseOperand& z, int n, int k) {
+            z.rows = pad128(n);
+            m->want(&z.codes, static_cast<size_t>(W) * z.rows * k / 2);
+            m->want(&z.sf, static_cast<size_t>(W) * sf_bytes(z.rows, k));
+        };
+        m->nz_qkv.resize(L); m->nz_ff1.resize(L); m->nz_ff2.resize(L);
+        operand(m->nz_win, H, H); operand(m->nz_head, V, H);
+        for (int l = 0; l < L; ++l) { operand(m->nz_qkv[l], 3 * H + 1, H); operand(m->nz_ff1[l], F, H); operand(m->nz_ff2[l], H, F); }
+        A_(dgen, 3 + 6 * static_cast<size_t>(L)); A_(dgen_tab, 256);
+    } else if (m->dense) {
         const DenseLayout lay = dense_layout(*m);
         A_(E_all, lay.total);
         A_(qe_win, hh / 2); A_(sfe_win, sf_bytes(H, H)); A_(qe_head, static_cast<size_t>(V) * H / 2); A_(sfe_head, sf_bytes(V, H));
@@ -876,6 +1006,7 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     rc = m->commit();
     if (rc) { bnf4_model_destroy(m); return rc; }
     rc = build_update_tables(*m);
+    if (!rc && m->dense_folded) rc = build_dense_tables(*m);
     if (rc) { bnf4_model_destroy(m); return rc; }
     {
         const std::vector<ZLowrankDesc> zd = z_descs(*m, m->Z_all);
@@ -926,11 +1057,6 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     rc = check_cuda(cudaMemcpy(m->gen_descs, gd.data(), gd.size() * sizeof(GenDesc), cudaMemcpyHostToDevice), "cudaMemcpy(gen_descs)");
     if (!rc) rc = check_cuda(cudaMemcpy(m->gen_block_map, bmap.data(), bmap.size() * sizeof(uint32_t), cudaMemcpyHostToDevice), "cudaMemcpy(gen_block_map)");
     if (rc) { bnf4_model_destroy(m); return rc; }
-    const size_t span = static_cast<size_t>(reinterpret_cast<const uint8_t*>(m->pos) - reinterpret_cast<const uint8_t*>(m->emb)) + static_cast<size_t>(T) * H * sizeof(float);
-    if (span <= kWeightStageBytes) {
-        rc = check_cuda(cudaMallocHost(&m->h_weights, span), "cudaMallocHost(weights)");
-        if (rc) { bnf4_model_destroy(m); return rc; }
-    }
     *handle = m;
     return BNF4_OK;
 }
@@ -1023,15 +1149,14 @@ int bnf4_model_get_weights(void* handle, bnf4_model_weights* w) {
                           {m.head, w->head, vh}, {m.head_bias, w->head_bias, m.V * sizeof(float)}, {m.beta_bias, w->beta_bias, m.L * sizeof(float)},
                           {m.pos, w->pos, static_cast<size_t>(m.T) * m.H * sizeof(float)}};
     TRY(check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize"));
-    // The twelve arrays lie back to back on the device (create requests them first, in this order). Small models come over in one
-    // copy through a pinned buffer: twelve copies to pageable memory cost more than the smallest step. Large ones go directly.
-    if (m.h_weights != nullptr) {
-        const uint8_t* first = reinterpret_cast<const uint8_t*>(m.emb);
-        const size_t span = static_cast<size_t>(reinterpret_cast<const uint8_t*>(m.pos) - first) + items[11].bytes;
-        TRY(check_cuda(cudaMemcpy(m.h_weights, first, span, cudaMemcpyDeviceToHost), "cudaMemcpy(weights)"));
-        for (const Item& it : items)
-            if (it.h) std::memcpy(it.h, m.h_weights + (static_cast<const uint8_t*>(it.d) - first), it.bytes);
-        return BNF4_OK;
+    // The twelve arrays lie back to back on the device (create requests them first, in this order, each rounded up to 1024 bytes). A caller
+    // whose host arrays lie the same way gets them in one copy: twelve copies cost more than the smallest step.
+    bool same = true;
+    for (const Item& it : items)
+        same = same && it.h != nullptr && static_cast<const uint8_t*>(it.h) - static_cast<const uint8_t*>(items[0].h) == static_cast<const uint8_t*>(it.d) - static_cast<const uint8_t*>(items[0].d);
+    if (same) {
+        const size_t span = static_cast<size_t>(static_cast<const uint8_t*>(items[11].d) - static_cast<const uint8_t*>(items[0].d)) + items[11].bytes;
+        return check_cuda(cudaMemcpy(items[0].h, items[0].d, span, cudaMemcpyDeviceToHost), "cudaMemcpy(weights)");
     }
     for (const Item& it : items)
         if (it.h) TRY(check_cuda(cudaMemcpy(it.h, it.d, it.bytes, cudaMemcpyDeviceToHost), "cudaMemcpy(weights)"));
@@ -1100,7 +1225,7 @@ int bnf4_model_eval_pairs(void* handle, int pair_begin, int pair_count, float* l
     if (pair_count > 0 && (pair_begin < m.eval_begin || pair_begin + pair_count > m.eval_end))
         return set_error(BNF4_ERR_INVALID, "model_eval_pairs: pairs [%d,%d) outside the range [%d,%d) the step was prepared for", pair_begin,
                          pair_begin + pair_count, m.eval_begin, m.eval_end);
-    if (m.dense) {
+    if (m.dense && !m.dense_folded) {
         for (int p = 0; p < pair_count; ++p) TRY(run_pair_dense(m, pair_begin + p, losses + 2 * static_cast<size_t>(p), S(stream)));
         return BNF4_OK;
     }

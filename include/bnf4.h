@@ -412,15 +412,16 @@ typedef struct bnf4_model_cfg {
     int batch;        /* B */
     int heads;        /* head_dim = H / heads; 1 reproduces the reference */
     int rank;         /* rank of the per-member perturbation, 1..4; 0 = the reference driver's dense form: one materialised CLT
-                         noise matrix per weight matrix and pair, applied as a second GEMM with beta = 1 (one pair per wave,
-                         batch * seq a multiple of 128; a reference-exact mode, not a fast one) */
+                         noise matrix per weight matrix and pair, quantised like the weights and multiplied with the same
+                         activations (batch * seq a multiple of 128) */
     int sigma_shift;  /* sigma = 2^-sigma_shift */
     int use_clt;
     int clt_k;
     int method;       /* 0 DeltaNet, 1 EFLA */
     float act_scale, mlp_act_scale, ln_scale, residual_scale, mlp_residual_scale, eps;
     int max_pairs;    /* pairs per ES step (population / 2) */
-    int wave_members; /* members evaluated per wave (even); 0 = library default: what fits ~12 GB of wave buffers, at most 256 */
+    int wave_members; /* members evaluated per wave (even); 0 = library default: what fits ~12 GB of wave buffers, at most 256
+                         (rank 0: also at most 2 GB of noise operands, whatever this says; one pair where sigma_shift > 4) */
 } bnf4_model_cfg;
 
 /* Host-side weight set (reference: EflaLmWeights src/train_efla_lm.cpp:419-431 plus the positional table). */

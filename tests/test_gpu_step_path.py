@@ -14,7 +14,7 @@ def make(seed=3, **kw):
     assert torch.cuda.is_available()
     cfg = population.Config(**kw)
     w = synth.init_weights(cfg)
-    tok, tgt = synth.sample_batch(synth.zipf_corpus(1 << 14, 1.1, 123), cfg.batch, cfg.seq, seed)
+    tok, tgt = (np.ascontiguousarray(np.minimum(x, cfg.vocab - 1)) for x in synth.sample_batch(synth.zipf_corpus(1 << 14, 1.1, 123), cfg.batch, cfg.seq, seed))
     model = population.PopulationModel(cfg)
     model.set_weights(w)
     model.set_tokens(tok, tgt)
@@ -79,3 +79,27 @@ def test_validation_after_an_update_matches_the_oracle(kw):
     ref = oracle_loss(cfg, after, tok, tgt)
     assert abs(m.eval_base().item() - ref) <= 1e-4 * abs(ref)
     assert host.device_error() == 0
+
+
+@pytest.mark.parametrize("kw", [
+    dict(hidden=128, layers=2, seq=64, batch=6, heads=2, max_pairs=5),                     # several pairs per wave, tokens de-duplicated
+    dict(hidden=192, layers=1, mlp_mult=3, seq=32, batch=4, heads=3, max_pairs=3, vocab=200),  # vocabulary that is no multiple of a tile, K remainder of 64
+    dict(hidden=128, layers=1, seq=32, batch=12, heads=1, max_pairs=2, sigma_shift=6),     # sigma too small for the folded form
+])
+def test_dense_noise_in_one_product(kw):
+    """rank 0: base weights and each member's noise operand in one accumulation (sigma >= 2^-4), product by product below: member losses
+    against the oracle's dense forward, and independence of the wave."""
+    from bitnet_nvfp4_b200 import host
+    cfg, w, tok, tgt, m = make(rank=0, **kw)
+    pairs = cfg.max_pairs
+    m.prepare_step(1, 3, pairs)
+    losses = m.eval_pairs(0, pairs).cpu().numpy()
+    assert host.device_error() == 0
+    ocfg = {k: getattr(cfg, k) for k in "vocab hidden layers mlp_mult seq batch heads rank sigma_shift use_clt clt_k method act_scale "
+                                        "mlp_act_scale ln_scale residual_scale mlp_residual_scale eps".split()}
+    om = orc.OracleModel(ocfg, w)
+    for p in range(pairs):
+        for s, anti in enumerate((1, -1)):
+            ref = om.forward(tok, tgt, orc.mix(1, orc.mix(3, p)), anti)
+            assert abs(losses[2 * p + s] - ref) <= 1e-4 * abs(ref), (p, anti)
+    assert np.array_equal(m.eval_pairs(1, pairs - 1).cpu().numpy(), losses[2:])
