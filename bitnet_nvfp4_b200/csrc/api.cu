@@ -94,6 +94,12 @@ size_t bnf4_nvfp4_sfa_bytes(int m, int /*n*/, int k) { return sf_bytes(m, k); }
 size_t bnf4_nvfp4_sfb_bytes(int /*m*/, int n, int k) { return sf_bytes(n, k); }
 
 // --------------------------------------------------------------------------------------------- quantisers
+// The single-matrix entry points own their whole scale array: they clear its padding too.
+static int quantise(int front_end, const bnf4_rowquant_desc& d, void* stream) {
+    RowQuantParams p(d);
+    p.pad_sf = (d.rows % 128) != 0 || (d.cols_out % 64) != 0;
+    return rowquant_dispatch(front_end, p, S(stream));
+}
 int bnf4_rowquant(int front_end, const bnf4_rowquant_desc* desc, void* stream) {
     if (!desc) return set_error(BNF4_ERR_INVALID, "bnf4_rowquant: null descriptor");
     return rowquant_dispatch(front_end, *desc, S(stream));
@@ -104,7 +110,7 @@ int bnf4_nvfp4_quantize_a(const int8_t* in, int m, int /*n*/, int k_in, int k_ou
     bnf4_rowquant_desc p = {};
     p.rows = m; p.cols_in = k_in; p.cols_out = k_out; p.in_i8 = in; p.ld_in = k_in;
     p.out_codes = static_cast<uint8_t*>(out); p.out_sf = static_cast<uint8_t*>(sfa);
-    return rowquant_dispatch(FE_INT8, p, S(stream));
+    return quantise(FE_INT8, p, stream);
 }
 
 int bnf4_nvfp4_quantize_b(const int8_t* in, int /*m*/, int n, int k_in, int k_out, void* out, void* sfb, void* stream) {
@@ -112,7 +118,7 @@ int bnf4_nvfp4_quantize_b(const int8_t* in, int /*m*/, int n, int k_in, int k_ou
     bnf4_rowquant_desc p = {};
     p.rows = n; p.cols_in = k_in; p.cols_out = k_out; p.in_i8 = in; p.ld_in = k_in;
     p.out_codes = static_cast<uint8_t*>(out); p.out_sf = static_cast<uint8_t*>(sfb);
-    return rowquant_dispatch(FE_INT8, p, S(stream));
+    return quantise(FE_INT8, p, stream);
 }
 
 int bnf4_nvfp4_quantize_wqkv_fused(const int8_t* wq, const int8_t* wk, const int8_t* wv, const int8_t* wb, int /*batch*/,
@@ -139,7 +145,7 @@ int bnf4_embedding_lookup_noise_quantize_nvfp4(const uint8_t* tokens_t, int toke
     p.tokens = tokens_t; p.token_stride = token_stride; p.emb_w = emb_w; p.emb_noise = emb_noise;
     p.sigma = noise_scale; p.anti_fixed = anti_sign;
     p.out_q = out_q; p.ld_q = hidden; p.out_codes = static_cast<uint8_t*>(out_nvfp4); p.out_sf = static_cast<uint8_t*>(sfa);
-    return rowquant_dispatch(FE_EMBED_DENSE, p, S(stream));
+    return quantise(FE_EMBED_DENSE, p, stream);
 }
 
 int bnf4_add_pos_gelu_quantize_nvfp4(const float* in, const float* pos_t, int hidden, int batch, float act_scale,
@@ -149,7 +155,7 @@ int bnf4_add_pos_gelu_quantize_nvfp4(const float* in, const float* pos_t, int hi
     p.rows = batch; p.cols_in = hidden; p.cols_out = hidden; p.in_f32 = in; p.ld_in = hidden;
     p.pos = pos_t; p.pos_mod = 0; p.act_scale = act_scale;
     p.out_q = out_q; p.ld_q = hidden; p.out_codes = static_cast<uint8_t*>(out_nvfp4); p.out_sf = static_cast<uint8_t*>(sfa);
-    return rowquant_dispatch(FE_POS_GELU, p, S(stream));
+    return quantise(FE_POS_GELU, p, stream);
 }
 
 int bnf4_activation_quantize_nvfp4(const float* in, int rows, int cols_in, int cols_out, int activation, int8_t* out_q,
@@ -159,7 +165,7 @@ int bnf4_activation_quantize_nvfp4(const float* in, int rows, int cols_in, int c
     p.rows = rows; p.cols_in = cols_in; p.cols_out = cols_out; p.in_f32 = in; p.ld_in = cols_in;
     p.act_mode = activation; p.act_scale = 1.0f;
     p.out_q = out_q; p.ld_q = cols_out; p.out_codes = static_cast<uint8_t*>(out_nvfp4); p.out_sf = static_cast<uint8_t*>(sfa);
-    return rowquant_dispatch(FE_ACT, p, S(stream));
+    return quantise(FE_ACT, p, stream);
 }
 
 int bnf4_gelu_quantize_nvfp4(const float* in, int rows, int cols_in, int cols_out, float act_scale, int8_t* out_q,
@@ -169,7 +175,7 @@ int bnf4_gelu_quantize_nvfp4(const float* in, int rows, int cols_in, int cols_ou
     p.rows = rows; p.cols_in = cols_in; p.cols_out = cols_out; p.in_f32 = in; p.ld_in = cols_in;
     p.act_mode = 3; p.act_scale = act_scale;
     p.out_q = out_q; p.ld_q = cols_out; p.out_codes = static_cast<uint8_t*>(out_nvfp4); p.out_sf = static_cast<uint8_t*>(sfa);
-    return rowquant_dispatch(FE_ACT, p, S(stream));
+    return quantise(FE_ACT, p, stream);
 }
 
 int bnf4_absmean_norm_q_nvfp4(const int8_t* in, int hidden, int batch, int cols_out, float scale, int8_t* out_q,
@@ -178,7 +184,7 @@ int bnf4_absmean_norm_q_nvfp4(const int8_t* in, int hidden, int batch, int cols_
     bnf4_rowquant_desc p = {};
     p.rows = batch; p.cols_in = hidden; p.cols_out = cols_out; p.in_i8 = in; p.ld_in = hidden; p.norm_scale = scale;
     p.out_q = out_q; p.ld_q = hidden; p.out_codes = static_cast<uint8_t*>(out_nvfp4); p.out_sf = static_cast<uint8_t*>(sfa);
-    return rowquant_dispatch(FE_ABSMEAN, p, S(stream));
+    return quantise(FE_ABSMEAN, p, stream);
 }
 
 int bnf4_add_scaled_to_int8_absmean_norm_q_nvfp4(int8_t* inout, const float* in, int hidden, int batch, int cols_out,
@@ -189,7 +195,7 @@ int bnf4_add_scaled_to_int8_absmean_norm_q_nvfp4(int8_t* inout, const float* in,
     p.rows = batch; p.cols_in = hidden; p.cols_out = cols_out; p.inout_i8 = inout; p.in_f32 = in; p.ld_in = hidden;
     p.add_scale = add_scale; p.norm_scale = norm_scale;
     p.out_q = out_q; p.ld_q = hidden; p.out_codes = static_cast<uint8_t*>(out_nvfp4); p.out_sf = static_cast<uint8_t*>(sfa);
-    return rowquant_dispatch(FE_ADD_ABSMEAN, p, S(stream));
+    return quantise(FE_ADD_ABSMEAN, p, stream);
 }
 
 // --------------------------------------------------------------------------------------------- GEMM

@@ -63,16 +63,16 @@ __device__ __forceinline__ float ce_row_loss(const float* lg, const float* bias,
 }
 
 // API form: a single CTA sums the rows of one token step in a fixed order and adds the total to *loss_accum.
-__global__ void __launch_bounds__(256) ce_step_kernel(const float* __restrict__ logits, const float* __restrict__ bias,
+__global__ void __launch_bounds__(1024) ce_step_kernel(const float* __restrict__ logits, const float* __restrict__ bias,
                                                       const float* __restrict__ bias_noise, float bns,
                                                       const uint8_t* __restrict__ targets_t, int token_stride, int vocab, int batch,
                                                       float* loss_accum) {
     pdl_wait();
     after(logits, bias, bias_noise, targets_t);
-    __shared__ float part[8];
+    __shared__ float part[32];  // a warp per row: 32 rows, the reference driver's batch, in one go
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float acc = 0.0f;
-    for (int b = warp; b < batch; b += 8) {
+    for (int b = warp; b < batch; b += 32) {
         const int y = static_cast<int>(targets_t[static_cast<size_t>(b) * token_stride]);
         acc += ce_row_loss(logits + static_cast<size_t>(b) * vocab, bias, bias_noise, nullptr, bns, vocab, y, lane);
     }
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(256) ce_step_kernel(const float* __restrict__ 
     __syncthreads();
     if (threadIdx.x == 0) {
         float t = 0.0f;
-        for (int w = 0; w < 8; ++w) t += part[w];
+        for (int w = 0; w < 32; ++w) t += part[w];
         loss_accum[0] += t;
     }
 }
@@ -988,7 +988,7 @@ int bnf4_cross_entropy_loss(const float* logits, const float* bias, const float*
     if (batch <= 0) return BNF4_OK;
     if (!logits || !targets_t || !loss_accum) return set_error(BNF4_ERR_INVALID, "cross_entropy_loss: null pointer");
     if (vocab <= 0 || vocab > 32 * kCeMaxPerLane) return set_error(BNF4_ERR_INVALID, "cross_entropy_loss: vocab=%d outside [1,%d]", vocab, 32 * kCeMaxPerLane);
-    launch_pdl(ce_step_kernel, 1, 256, 0, S(stream), logits, bias, bias_noise, bias_noise_scale, targets_t, token_stride, vocab, batch, loss_accum);
+    launch_pdl(ce_step_kernel, 1, 1024, 0, S(stream), logits, bias, bias_noise, bias_noise_scale, targets_t, token_stride, vocab, batch, loss_accum);
     return check_launch("ce_step_kernel");
 }
 

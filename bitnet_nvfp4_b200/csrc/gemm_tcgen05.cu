@@ -851,9 +851,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             }
             if (!R1 && p.beta != 0.0f && row_ok) {
                 const float* crow = p.c + static_cast<size_t>(row) * p.ldc + col0;
+                if (col0 + 32 <= p.n && (reinterpret_cast<uintptr_t>(crow) & 15) == 0) {
 #pragma unroll
-                for (int j = 0; j < 32; ++j)
-                    if (col0 + j < p.n) v[j] = fmaf(p.beta, crow[j], v[j]);
+                    for (int j = 0; j < 8; ++j) {
+                        const float4 c4 = reinterpret_cast<const float4*>(crow)[j];
+                        v[4 * j] = fmaf(p.beta, c4.x, v[4 * j]);
+                        v[4 * j + 1] = fmaf(p.beta, c4.y, v[4 * j + 1]);
+                        v[4 * j + 2] = fmaf(p.beta, c4.z, v[4 * j + 2]);
+                        v[4 * j + 3] = fmaf(p.beta, c4.w, v[4 * j + 3]);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j)
+                        if (col0 + j < p.n) v[j] = fmaf(p.beta, crow[j], v[j]);
+                }
             }
             if ((R1 || p.rank > 0) && row_ok) {
                 // sum_r t[r]*A[n][r] is an integer below 2^24: float products and sums are exact

@@ -31,6 +31,7 @@ struct RowQuantParams : bnf4_rowquant_desc {
     RowQuantParams(const bnf4_rowquant_desc& d) : bnf4_rowquant_desc(d) {}
     int32_t* zero_t = nullptr;  // FE_ADD_ABSMEAN: clears [rows][zero_n] words, the projections the GEMM after next accumulates with atomics
     int zero_n = 0;
+    int pad_sf = 0;              // also clears the padding of the scale array (rows to 128, columns to 64)
 };
 int rowquant_dispatch(int front_end, RowQuantParams p, cudaStream_t stream);
 

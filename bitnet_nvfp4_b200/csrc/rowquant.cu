@@ -31,12 +31,28 @@ namespace {
 constexpr int kMaxBlocksPerLane = 8;        // rows of up to 32*8*16 = 4096 columns ...
 constexpr int kMaxBlocksPerLaneInt8 = 16;  // ... and 8192 for plain int8 rows (weight matrices of wide MLPs)
 
+// Clears the scale bytes of the rows and columns that pad the last atoms, so that callers need not clear the array (a launch of its own).
+__device__ __forceinline__ void pad_scales(const RowQuantParams& p) {
+    const int nblk = p.cols_out >> 4, k_atoms = sf_k_atoms(p.cols_out), rows_pad = (p.rows + 127) & ~127;
+    const int tail = nblk & 3;  // first padding column of the last atom (0: none)
+    const int first = tail ? 0 : p.rows;
+    const int count = (rows_pad - first) * k_atoms;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const int row = first + i / k_atoms, a = i % k_atoms;
+        uint8_t* word = p.out_sf + sf_offset(row, 4 * a, k_atoms);
+        if (row >= p.rows) *reinterpret_cast<uint32_t*>(word) = 0u;
+        else if (tail && a == k_atoms - 1)
+            for (int b = tail; b < 4; ++b) word[b] = 0;
+    }
+}
+
 template <int FE, int NB>
 __global__ void __launch_bounds__(256) rowquant_kernel(const RowQuantParams p, const uint8_t* __restrict__ lut) {
     pdl_trigger();
     const int warps_per_cta = blockDim.x >> 5;
     const int lane = threadIdx.x & 31;
     pdl_wait();
+    if (p.pad_sf) pad_scales(p);
     const long long row = static_cast<long long>(blockIdx.x + opaque_zero()) * warps_per_cta + (threadIdx.x >> 5);
     if (row >= p.rows) return;
 
@@ -307,6 +323,7 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
     if (threadIdx.x < 128) tab_s[threadIdx.x] = __ldg(reinterpret_cast<const uint2*>(lut + kQuantBlockTabOffset) + threadIdx.x);
     __syncthreads();
     pdl_wait();  // the table is constant; the rows are the predecessor's
+    if (!MODEL && p.pad_sf) pad_scales(p);
     // entry address from the bit pattern of (amax + kRoundBias): (bits - kRoundBiasBits) * 8, folded into one constant
     const uint32_t tab_c = static_cast<uint32_t>(__cvta_generic_to_shared(tab_s)) - (static_cast<uint32_t>(kRoundBiasBits) << 3);
     const float M = kRoundBias;

@@ -41,13 +41,11 @@ def matrix_bytes(rows: int, cols: int) -> int:
     return (rows * cols * 4 + 7) // 8
 
 
-def _alloc_q(rows: int, cols: int, device, want_q=True):
-    """Outputs of a quantiser. It writes every int8 value and code and the scale byte of every block; only the padding of a
-    ragged scale array (rows to 128, columns to 64) has to be cleared."""
-    q = torch.empty((rows, cols), dtype=torch.int8, device=device) if want_q else None
-    codes = torch.empty(matrix_bytes(rows, cols), dtype=torch.uint8, device=device)
-    sf = (torch.zeros if rows % 128 or cols % 64 else torch.empty)(sf_bytes(rows, cols), dtype=torch.uint8, device=device)
-    return q, codes, sf
+def _alloc_q(like: torch.Tensor, rows: int, cols: int, want_q=True):
+    """Outputs of a quantiser on the device of `like`. Nothing is cleared: the library writes every int8 value, code and scale byte, the
+    padding of the scale array included."""
+    q = like.new_empty((rows, cols), dtype=torch.int8) if want_q else None
+    return q, like.new_empty(matrix_bytes(rows, cols), dtype=torch.uint8), like.new_empty(sf_bytes(rows, cols), dtype=torch.uint8)
 
 
 def device_error() -> int:
@@ -60,7 +58,7 @@ def device_error() -> int:
 def nvfp4_quantize_a(x: torch.Tensor, k_out: int | None = None):
     m, k_in = x.shape
     k_out = k_out or k_in
-    _, codes, sf = _alloc_q(m, k_out, x.device, want_q=False)
+    _, codes, sf = _alloc_q(x, m, k_out, want_q=False)
     _l.check(_l.load().bnf4_nvfp4_quantize_a(_p(x), m, 1, k_in, k_out, _p(codes), _p(sf), _stream()))
     return codes, sf
 
@@ -68,7 +66,7 @@ def nvfp4_quantize_a(x: torch.Tensor, k_out: int | None = None):
 def nvfp4_quantize_b(w: torch.Tensor, k_out: int | None = None):
     n, k_in = w.shape
     k_out = k_out or k_in
-    _, codes, sf = _alloc_q(n, k_out, w.device, want_q=False)
+    _, codes, sf = _alloc_q(w, n, k_out, want_q=False)
     _l.check(_l.load().bnf4_nvfp4_quantize_b(_p(w), 1, n, k_in, k_out, _p(codes), _p(sf), _stream()))
     return codes, sf
 
@@ -77,7 +75,9 @@ def nvfp4_quantize_f32(x: torch.Tensor, k_out: int | None = None):
     """fp32 rows straight to NVFP4 (no int8 stage)."""
     m, k_in = x.shape
     k_out = k_out or k_in
-    _, codes, sf = _alloc_q(m, k_out, x.device, want_q=False)
+    _, codes, sf = _alloc_q(x, m, k_out, want_q=False)
+    if m % 128 or k_out % 64:
+        sf.zero_()  # (this kernel leaves the padding alone)
     _l.check(_l.load().bnf4_nvfp4_quantize_f32(_p(x), m, k_in, k_out, _p(codes), _p(sf), _stream()))
     return codes, sf
 
@@ -91,7 +91,7 @@ def nvfp4_quantize_wqkv_fused(wq, wk, wv, wb, hidden: int, rows_total: int, scal
 
 
 def embedding_lookup_noise_quantize_nvfp4(tokens_t, token_stride, emb_w, emb_noise, hidden, batch, noise_scale, anti_sign):
-    q, codes, sf = _alloc_q(batch, hidden, emb_w.device)
+    q, codes, sf = _alloc_q(emb_w, batch, hidden)
     _l.check(_l.load().bnf4_embedding_lookup_noise_quantize_nvfp4(_p(tokens_t), token_stride, _p(emb_w), _p(emb_noise), hidden,
                                                                   batch, noise_scale, anti_sign, _p(q), _p(codes), _p(sf),
                                                                   _stream()))
@@ -100,7 +100,7 @@ def embedding_lookup_noise_quantize_nvfp4(tokens_t, token_stride, emb_w, emb_noi
 
 def add_pos_gelu_quantize_nvfp4(x, pos_t, act_scale):
     batch, hidden = x.shape
-    q, codes, sf = _alloc_q(batch, hidden, x.device)
+    q, codes, sf = _alloc_q(x, batch, hidden)
     _l.check(_l.load().bnf4_add_pos_gelu_quantize_nvfp4(_p(x), _p(pos_t), hidden, batch, act_scale, _p(q), _p(codes), _p(sf),
                                                         _stream()))
     return q, codes, sf
@@ -108,7 +108,7 @@ def add_pos_gelu_quantize_nvfp4(x, pos_t, act_scale):
 
 def activation_quantize_nvfp4(x, cols_out, activation):
     rows, cols_in = x.shape
-    q, codes, sf = _alloc_q(rows, cols_out, x.device)
+    q, codes, sf = _alloc_q(x, rows, cols_out)
     _l.check(_l.load().bnf4_activation_quantize_nvfp4(_p(x), rows, cols_in, cols_out, activation, _p(q), _p(codes), _p(sf),
                                                       _stream()))
     return q, codes, sf
@@ -116,21 +116,21 @@ def activation_quantize_nvfp4(x, cols_out, activation):
 
 def gelu_quantize_nvfp4(x, cols_out, act_scale):
     rows, cols_in = x.shape
-    q, codes, sf = _alloc_q(rows, cols_out, x.device)
+    q, codes, sf = _alloc_q(x, rows, cols_out)
     _l.check(_l.load().bnf4_gelu_quantize_nvfp4(_p(x), rows, cols_in, cols_out, act_scale, _p(q), _p(codes), _p(sf), _stream()))
     return q, codes, sf
 
 
 def absmean_norm_q_nvfp4(x8, scale):
     batch, hidden = x8.shape
-    q, codes, sf = _alloc_q(batch, hidden, x8.device)
+    q, codes, sf = _alloc_q(x8, batch, hidden)
     _l.check(_l.load().bnf4_absmean_norm_q_nvfp4(_p(x8), hidden, batch, hidden, scale, _p(q), _p(codes), _p(sf), _stream()))
     return q, codes, sf
 
 
 def add_scaled_to_int8_absmean_norm_q_nvfp4(x8_inout, y, add_scale, norm_scale):
     batch, hidden = x8_inout.shape
-    q, codes, sf = _alloc_q(batch, hidden, y.device)
+    q, codes, sf = _alloc_q(y, batch, hidden)
     _l.check(_l.load().bnf4_add_scaled_to_int8_absmean_norm_q_nvfp4(_p(x8_inout), _p(y), hidden, batch, hidden, add_scale,
                                                                     norm_scale, _p(q), _p(codes), _p(sf), _stream()))
     return q, codes, sf
@@ -148,13 +148,13 @@ def rowquant(front_end: int, **kw):
 # ------------------------------------------------------------------------------------------ GEMM
 def gemm_ternary_f_nvfp4(a, b, sfa, sfb, m, n, k, alpha, beta=0.0, c=None, d=None):
     if d is None:
-        d = torch.empty((m, n), dtype=torch.float32, device=a.device)
-    _l.check(_l.load().bnf4_gemm_ternary_f_nvfp4(_p(a), _p(b), _p(sfa), _p(sfb), m, n, k, alpha, beta, _p(c), _p(d), _stream()))
+        d = a.new_empty((m, n), dtype=torch.float32)
+    _l.check(_l.load().bnf4_gemm_ternary_f_nvfp4(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, k, alpha, beta, _p(c), d.data_ptr(), _stream()))
     return d
 
 
 def gemm_ternary_f_nvfp4_gelu_i8(a, b, sfa, sfb, m, n, k, alpha, beta, c, act_scale):
-    d = torch.empty((m, n), dtype=torch.int8, device=a.device)
+    d = a.new_empty((m, n), dtype=torch.int8)
     _l.check(_l.load().bnf4_gemm_ternary_f_nvfp4_gelu_i8(_p(a), _p(b), _p(sfa), _p(sfb), m, n, k, alpha, beta, _p(c), act_scale,
                                                          _p(d), _stream()))
     return d
@@ -209,14 +209,14 @@ def efla_scan(**kw):
 
 
 def efla_step_half_qkv_fused(S, qkv, fused_cols, beta_bias, hidden, batch, method, eps):
-    out = torch.empty((batch, hidden), dtype=torch.float32, device=qkv.device)
+    out = qkv.new_empty((batch, hidden))
     _l.check(_l.load().bnf4_efla_step_half_qkv_fused(_p(S), _p(qkv), fused_cols, beta_bias, hidden, batch, method, eps, _p(out),
                                                      _stream()))
     return out
 
 
 def efla_step_qkv_fused(S, qkv, fused_cols, beta_bias, hidden, batch, method, eps):
-    out = torch.empty((batch, hidden), dtype=torch.float32, device=qkv.device)
+    out = qkv.new_empty((batch, hidden))
     _l.check(_l.load().bnf4_efla_step_qkv_fused(_p(S), _p(qkv), fused_cols, beta_bias, hidden, batch, method, eps, _p(out),
                                                 _stream()))
     return out

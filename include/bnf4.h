@@ -62,7 +62,9 @@ size_t bnf4_nvfp4_sfb_bytes(int m, int n, int k);
 
 /* ---------------------------------------------------------------------------------------------
  * Quantisers: int8 / fp32 rows -> int8 copy + packed e2m1 codes + ue4m3 scale bytes.
- * Column counts must be multiples of 16 (the reference also handles ragged tails; unused by its driver).
+ * Column counts must be multiples of 16 (the reference also handles ragged tails; unused by its driver). The entry points for one
+ * int8 or fp32 matrix below also clear the padding of the scale array (rows to 128, columns to 64); bnf4_nvfp4_quantize_f32,
+ * bnf4_nvfp4_quantize_wqkv_fused and bnf4_rowquant write the scale bytes of existing blocks only.
  * ------------------------------------------------------------------------------------------- */
 /* reference: nvfp4_quantize_a src/cuda_kernels.cu:4013-4037 (kernel :1545-1625) */
 int bnf4_nvfp4_quantize_a(const int8_t* in, int m, int n, int k_in, int k_out, void* out, void* sfa, void* stream);
