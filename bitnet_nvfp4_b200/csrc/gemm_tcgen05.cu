@@ -277,6 +277,7 @@ struct KernelArgs {
     int use_tma_store;
     int k_atoms;  // scale atoms along K
     uint32_t group_magic;  // ceil(2^32 / group_cols) (0 when group_cols == 0)
+    uint32_t rpm_magic;    // floor(2^32 / rows_per_member), at most 2^32 - 1
     const uint8_t* lut;  // table of the block quantiser (EPI_GELU_FP4)
     int total_tiles;
     int ks_wrap;  // K blocks after which A starts again and B2 follows B (0: no second operand)
@@ -299,7 +300,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // CTAs working at the same time share rows of A through L2). Three roles run concurrently on different tiles:
 // the producer prefetches operands up to kStages k-blocks ahead, the MMA warp fills one of two TMEM
 // accumulators while the sixteen epilogue warps drain the other one.
-// RK: 4 = the instance for rank-4 perturbation terms (its epilogue applies the four factors with packed multiply-adds);
+// RK: 4 = the instance for rank-4 perturbation terms whose pairs start at multiples of 32 rows;
 // 1 = the instance for the batched driver's common case (rank 1, no C operand, every 128-row tile inside one member), which carries
 // none of the general paths; 0 = everything else.
 // PAIR: the instance for operands with many K blocks. On the in-order pipe a scale copy costs about 44 cycles and an M 128 x N 128 MMA
@@ -605,16 +606,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     __ldg(reinterpret_cast<const uint2*>(args.lut + kQuantBlockTabOffset) + ew * 32 + lane);
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
         }
-        // Perturbation context of one tile: this thread's row (projections t, sign, pair) and, when all rows of the tile
-        // belong to one pair (always true when rows_per_member is a multiple of 128), this thread's element of the
-        // pair's A factor for the tile's columns. It is fetched one tile ahead so that the global-load latency hides
-        // behind the previous tile's epilogue.
+        // Perturbation context of one tile: this thread's row (projections t, sign, pair) and this thread's element of the A factor
+        // of the warp's first pair for the tile's columns. It is fetched one tile ahead so that the global-load latency hides
+        // behind the previous tile's epilogue. A warp whose 32 rows reach into the next pair (members that are no multiple of the tile
+        // height) applies the pairs one after the other, each to its own rows.
         struct LoraCtx {
-            int pair;
-            float lsign;
+            int member;
             int tr[4];    // raw integers: converted to float only when the tile is processed, so that nothing waits
-            int aval[4];  // on these loads earlier;  aval[r] = A[pair][col0 + lane][r]
-            bool a_staged;
+            int aval[4];  // on these loads earlier;  aval[r] = A[pair of the warp's first row][col0 + lane][r]
         };
         const int row_in_tile = q * 32 + lane;
         // Tile coordinates advance by additions (tiles are walked in steps of gridDim.x): no division per tile.
@@ -651,36 +650,28 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         int trk_member = static_cast<int>(opaque_zero());  // (the pair's vectors are loaded read-only: their addresses depend on this)
         long long trk_end = p.rows_per_member;  // first row of member trk_member + 1
         const uint32_t group_magic = args.group_magic;  // ceil(2^32 / group_cols): exact quotients for columns below 65536
+        auto member_of = [&](unsigned row) {  // row / rows_per_member: the multiply-high is exact or one too small
+            if (p.rows_per_member <= 0) return 0;
+            const unsigned e = __umulhi(row, args.rpm_magic);
+            return static_cast<int>(row - e * static_cast<unsigned>(p.rows_per_member) >= static_cast<unsigned>(p.rows_per_member) ? e + 1 : e);
+        };
+        auto load_a = [&](int pr, int n, int (&aval)[4]) {
+            const int8_t* Ag = p.lora_A + static_cast<size_t>(pr) * p.lora_A_pair_stride + static_cast<size_t>(n) * p.rank;
+            aval[0] = Ag[0];
+            if (p.rank > 1) {
+                aval[1] = Ag[1];
+                if (p.rank > 2) aval[2] = Ag[2];
+                if (p.rank > 3) aval[3] = Ag[3];
+            }
+        };
         auto fetch_ctx = [&](const TileIdx& t, bool valid, LoraCtx& cx) {
-            cx.pair = 0;
-            cx.lsign = 0.0f;
+            cx.member = 0;
             cx.tr[0] = cx.tr[1] = cx.tr[2] = cx.tr[3] = 0;
             cx.aval[0] = cx.aval[1] = cx.aval[2] = cx.aval[3] = 0;
-            cx.a_staged = false;
             if (p.rank <= 0 || !valid) return;
-            const int m0_ = t.m_tile * BM, n0_ = t.n_tile * BN;
-            const long long row_ = static_cast<long long>(m0_) + row_in_tile;
-            const int col0_ = n0_ + c * 32;
-            int pair_first, pair_last;
-            if (tile_uniform_member) {
-                while (m0_ >= trk_end) { ++trk_member; trk_end += p.rows_per_member; }
-                pair_first = pair_last = trk_member >> 1;
-                if (row_ < p.m) {
-                    cx.pair = pair_first;
-                    cx.lsign = (trk_member & 1) ? -p.lora_scale : p.lora_scale;
-                }
-            } else {
-                // rows fit 31 bits (p.m is an int): 32-bit divisions
-                const unsigned rpm = static_cast<unsigned>(p.rows_per_member);
-                if (row_ < p.m) {
-                    const int member = p.rows_per_member > 0 ? static_cast<int>(static_cast<unsigned>(row_) / rpm) : 0;
-                    cx.pair = member >> 1;
-                    cx.lsign = (member & 1) ? -p.lora_scale : p.lora_scale;
-                }
-                const unsigned last_row = static_cast<unsigned>(min(static_cast<long long>(p.m), static_cast<long long>(m0_) + BM) - 1);
-                pair_first = p.rows_per_member > 0 ? static_cast<int>(static_cast<unsigned>(m0_) / rpm) >> 1 : 0;
-                pair_last = p.rows_per_member > 0 ? static_cast<int>(last_row / rpm) >> 1 : 0;
-            }
+            const int m0_ = t.m_tile * BM, col0_ = t.n_tile * BN + c * 32;
+            const int row_ = m0_ + row_in_tile;  // (rows fit 31 bits: p.m is an int)
+            cx.member = member_of(static_cast<unsigned>(min(row_, p.m - 1)));  // (rows past m are never stored)
             if (row_ < p.m && col0_ < p.n) {
                 const int g = p.group_cols > 0 ? static_cast<int>(__umulhi(static_cast<uint32_t>(col0_), group_magic)) : 0;
                 const int* tp = p.lora_t + static_cast<size_t>(row_) * p.t_stride + g * p.rank;
@@ -691,17 +682,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     if (p.rank > 3) cx.tr[3] = tp[3];
                 }
             }
-            cx.a_staged = (pair_first == pair_last);
-            const int n = col0_ + lane;
-            if (cx.a_staged && n < p.n) {
-                const int8_t* Ag = p.lora_A + static_cast<size_t>(pair_first) * p.lora_A_pair_stride + static_cast<size_t>(n) * p.rank;
-                cx.aval[0] = Ag[0];
-                if (p.rank > 1) {
-                    cx.aval[1] = Ag[1];
-                    if (p.rank > 2) cx.aval[2] = Ag[2];
-                    if (p.rank > 3) cx.aval[3] = Ag[3];
-                }
-            }
+            const int first = __shfl_sync(0xffffffffu, cx.member, 0) >> 1;
+            if (col0_ + lane < p.n) load_a(first, col0_ + lane, cx.aval);
         };
         // The common case (rank 1, tiles inside one member) with as few instructions as possible: this phase sits on the serial
         // path of every tile.
@@ -709,21 +691,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         const bool fast_ctx = R1 || (p.rank == 1 && tile_uniform_member);
         const int* t_row = p.rank > 0 ? p.lora_t + static_cast<size_t>(row_in_tile) * p.t_stride : nullptr;
         auto fetch_fast = [&](const TileIdx& t, bool valid, LoraCtx& cx) {
-            cx.pair = 0;
-            cx.lsign = 0.0f;
+            cx.member = 0;
             cx.tr[0] = 0;
             cx.aval[0] = 0;
-            cx.a_staged = true;
             if (!valid) return;
             const int m0_ = t.m_tile * BM, col0_ = t.n_tile * BN + c * 32;
             while (m0_ >= trk_end) { ++trk_member; trk_end += p.rows_per_member; }
-            cx.pair = trk_member >> 1;
+            cx.member = trk_member;
             if ((R1 || m0_ + row_in_tile < p.m) && col0_ < p.n) {
                 const int g = p.group_cols > 0 ? static_cast<int>(__umulhi(static_cast<uint32_t>(col0_), group_magic)) : 0;
                 cx.tr[0] = t_row[static_cast<size_t>(m0_) * p.t_stride + g];
-                cx.lsign = (trk_member & 1) ? -p.lora_scale : p.lora_scale;
             }
-            if (col0_ + lane < p.n) cx.aval[0] = __ldg(p.lora_A + static_cast<size_t>(cx.pair) * p.lora_A_pair_stride + col0_ + lane);
+            if (col0_ + lane < p.n) cx.aval[0] = __ldg(p.lora_A + static_cast<size_t>(trk_member >> 1) * p.lora_A_pair_stride + col0_ + lane);
         };
         TileIdx cur_t{static_cast<int>(unit / static_cast<unsigned>(args.n_tiles)), static_cast<int>(unit % static_cast<unsigned>(args.n_tiles)), 0, true};
         if constexpr (PAIR) {
@@ -782,10 +761,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             const int col0 = n0 + c * 32;
             const bool chunk_ok = col0 < p.n;  // warp-uniform
 
-            const int pair = nxt.pair;
-            const float lsign = nxt.lsign;
+            const int member = nxt.member, pair = member >> 1;
             float tr[4] = {static_cast<float>(nxt.tr[0]), 0.0f, 0.0f, 0.0f};
-            const bool a_staged = nxt.a_staged;
             float* loraA_sh = reinterpret_cast<float*>(smem_gen + oSmemLora) + ew * 4 * 32;  // this warp's [4][32]
             if (R1 || fast_ctx) {
                 __syncwarp();  // the previous tile's reads are done
@@ -797,11 +774,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 tr[2] = static_cast<float>(nxt.tr[2]);
                 tr[3] = static_cast<float>(nxt.tr[3]);
                 __syncwarp();  // the previous tile's reads are done
-                if (a_staged) {
 #pragma unroll
-                    for (int r = 0; r < 4; ++r)
-                        if (r < p.rank) loraA_sh[r * 32 + lane] = static_cast<float>(nxt.aval[r]);
-                }
+                for (int r = 0; r < 4; ++r)
+                    if (r < p.rank) loraA_sh[r * 32 + lane] = static_cast<float>(nxt.aval[r]);
                 __syncwarp();
                 fetch_ctx(nxt_t, more, nxt);
             }
@@ -866,74 +841,52 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                         if (col0 + j < p.n) v[j] = fmaf(p.beta, crow[j], v[j]);
                 }
             }
-            if ((R1 || p.rank > 0) && row_ok) {
-                // sum_r t[r]*A[n][r] is an integer below 2^24: float products and sums are exact
-                if constexpr (R4) {
-                    if (a_staged) {
-                        const float2 ls2 = make_float2(lsign, lsign);
-                        const float2 t0 = make_float2(tr[0], tr[0]), t1 = make_float2(tr[1], tr[1]), t2 = make_float2(tr[2], tr[2]), t3 = make_float2(tr[3], tr[3]);
+            const float lsign = (member & 1) ? -p.lora_scale : p.lora_scale;
+            if constexpr (R1) {
+                // t * A is an integer below 2^24: float products are exact
+                const float2 tr2 = make_float2(tr[0], tr[0]), ls2 = make_float2(lsign, lsign);
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float4 a0 = *reinterpret_cast<const float4*>(loraA_sh + 4 * j), a1 = *reinterpret_cast<const float4*>(loraA_sh + 32 + 4 * j);
-                            const float4 a2 = *reinterpret_cast<const float4*>(loraA_sh + 64 + 4 * j), a3 = *reinterpret_cast<const float4*>(loraA_sh + 96 + 4 * j);
-                            float2 lo = __fmul2_rn(t0, make_float2(a0.x, a0.y)), hi = __fmul2_rn(t0, make_float2(a0.z, a0.w));
-                            lo = __ffma2_rn(t1, make_float2(a1.x, a1.y), lo); hi = __ffma2_rn(t1, make_float2(a1.z, a1.w), hi);
-                            lo = __ffma2_rn(t2, make_float2(a2.x, a2.y), lo); hi = __ffma2_rn(t2, make_float2(a2.z, a2.w), hi);
-                            lo = __ffma2_rn(t3, make_float2(a3.x, a3.y), lo); hi = __ffma2_rn(t3, make_float2(a3.z, a3.w), hi);
-                            lo = __ffma2_rn(ls2, lo, make_float2(v[4 * j + 0], v[4 * j + 1]));
-                            hi = __ffma2_rn(ls2, hi, make_float2(v[4 * j + 2], v[4 * j + 3]));
-                            v[4 * j + 0] = lo.x; v[4 * j + 1] = lo.y; v[4 * j + 2] = hi.x; v[4 * j + 3] = hi.y;
-                        }
-                    } else {
-                        const int8_t* Ap = p.lora_A + static_cast<size_t>(pair) * p.lora_A_pair_stride + static_cast<size_t>(col0) * 4;
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            if (col0 + j < p.n) {
-                                float pert = 0.0f;
-#pragma unroll
-                                for (int r = 0; r < 4; ++r) pert = fmaf(tr[r], static_cast<float>(Ap[j * 4 + r]), pert);
-                                v[j] = fmaf(lsign, pert, v[j]);
-                            }
-                        }
-                    }
-                } else if (R1 || (a_staged && p.rank == 1)) {
-                    const float2 tr2 = make_float2(tr[0], tr[0]), ls2 = make_float2(lsign, lsign);
+                for (int j = 0; j < 8; ++j) {
+                    const float4 a4 = *reinterpret_cast<const float4*>(loraA_sh + 4 * j);
+                    const float2 lo = __ffma2_rn(ls2, __fmul2_rn(tr2, make_float2(a4.x, a4.y)), make_float2(v[4 * j + 0], v[4 * j + 1]));
+                    const float2 hi = __ffma2_rn(ls2, __fmul2_rn(tr2, make_float2(a4.z, a4.w)), make_float2(v[4 * j + 2], v[4 * j + 3]));
+                    v[4 * j + 0] = lo.x; v[4 * j + 1] = lo.y; v[4 * j + 2] = hi.x; v[4 * j + 3] = hi.y;
+                }
+            } else if (p.rank > 0) {
+                // sum_r t[r]*A[n][r] is an integer below 2^24: float products and sums are exact. Rows of another pair (and rows past m)
+                // take part with a zero factor.
+                const int pair_hi = R4 ? 0 : __shfl_sync(0xffffffffu, pair, 31);  // (the rank-4 instance runs with 32 rows inside one pair)
+                for (int pr = R4 ? 0 : __shfl_sync(0xffffffffu, pair, 0);; ++pr) {
+                    const float ls = R4 || pair == pr ? lsign : 0.0f;
+                    const float2 ls2 = make_float2(ls, ls);
+                    const float2 t0 = make_float2(tr[0], tr[0]), t1 = make_float2(tr[1], tr[1]), t2 = make_float2(tr[2], tr[2]), t3 = make_float2(tr[3], tr[3]);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float4 a4 = *reinterpret_cast<const float4*>(loraA_sh + 4 * j);
-                        const float2 lo = __ffma2_rn(ls2, __fmul2_rn(tr2, make_float2(a4.x, a4.y)), make_float2(v[4 * j + 0], v[4 * j + 1]));
-                        const float2 hi = __ffma2_rn(ls2, __fmul2_rn(tr2, make_float2(a4.z, a4.w)), make_float2(v[4 * j + 2], v[4 * j + 3]));
+                        const float4 a0 = *reinterpret_cast<const float4*>(loraA_sh + 4 * j);
+                        float2 lo = __fmul2_rn(t0, make_float2(a0.x, a0.y)), hi = __fmul2_rn(t0, make_float2(a0.z, a0.w));
+                        auto add = [&](const float2 tt, int r) {
+                            const float4 a = *reinterpret_cast<const float4*>(loraA_sh + 32 * r + 4 * j);
+                            lo = __ffma2_rn(tt, make_float2(a.x, a.y), lo);
+                            hi = __ffma2_rn(tt, make_float2(a.z, a.w), hi);
+                        };
+                        if constexpr (R4) { add(t1, 1); add(t2, 2); add(t3, 3); }
+                        else {
+                            if (p.rank > 1) add(t1, 1);
+                            if (p.rank > 2) add(t2, 2);
+                            if (p.rank > 3) add(t3, 3);
+                        }
+                        lo = __ffma2_rn(ls2, lo, make_float2(v[4 * j + 0], v[4 * j + 1]));
+                        hi = __ffma2_rn(ls2, hi, make_float2(v[4 * j + 2], v[4 * j + 3]));
                         v[4 * j + 0] = lo.x; v[4 * j + 1] = lo.y; v[4 * j + 2] = hi.x; v[4 * j + 3] = hi.y;
                     }
-                } else if (a_staged) {
+                    if (R4 || pr >= pair_hi) break;
+                    __syncwarp();  // the next pair's factor takes the place of this one's
+                    int av[4] = {0, 0, 0, 0};
+                    if (col0 + lane < p.n) load_a(pr + 1, col0 + lane, av);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        float4 pert = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                        for (int r = 0; r < p.rank; ++r) {
-                            const float trr = r == 0 ? tr[0] : (r == 1 ? tr[1] : (r == 2 ? tr[2] : tr[3]));
-                            const float4 a4 = *reinterpret_cast<const float4*>(loraA_sh + r * 32 + 4 * j);
-                            pert.x = fmaf(trr, a4.x, pert.x);
-                            pert.y = fmaf(trr, a4.y, pert.y);
-                            pert.z = fmaf(trr, a4.z, pert.z);
-                            pert.w = fmaf(trr, a4.w, pert.w);
-                        }
-                        v[4 * j + 0] = fmaf(lsign, pert.x, v[4 * j + 0]);
-                        v[4 * j + 1] = fmaf(lsign, pert.y, v[4 * j + 1]);
-                        v[4 * j + 2] = fmaf(lsign, pert.z, v[4 * j + 2]);
-                        v[4 * j + 3] = fmaf(lsign, pert.w, v[4 * j + 3]);
-                    }
-                } else {
-                    const int8_t* Ap = p.lora_A + static_cast<size_t>(pair) * p.lora_A_pair_stride + static_cast<size_t>(col0) * p.rank;
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        if (col0 + j < p.n) {
-                            float pert = 0.0f;
-#pragma unroll
-                            for (int r = 0; r < 4; ++r)
-                                if (r < p.rank) pert = fmaf(tr[r], static_cast<float>(Ap[static_cast<size_t>(j) * p.rank + r]), pert);
-                            v[j] = fmaf(lsign, pert, v[j]);
-                        }
-                    }
+                    for (int r = 0; r < 4; ++r)
+                        if (r < p.rank) loraA_sh[r * 32 + lane] = static_cast<float>(av[r]);
+                    __syncwarp();
                 }
             }
 
@@ -1285,6 +1238,7 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     KernelArgs args;
     args.p = p;
     args.k_atoms = sf_k_atoms(p.k);
+    args.rpm_magic = p.rows_per_member > 0 ? static_cast<uint32_t>(std::min<unsigned long long>((1ull << 32) / static_cast<unsigned long long>(p.rows_per_member), 0xffffffffull)) : 0u;
     args.group_magic = p.group_cols > 0 ? static_cast<uint32_t>(((1ull << 32) + static_cast<unsigned long long>(p.group_cols) - 1) / static_cast<unsigned long long>(p.group_cols)) : 0u;
     if (p.group_cols > 0 && p.n >= 65536) return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: column groups need n < 65536");
     args.lut = nullptr;
@@ -1325,7 +1279,7 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     if (sms <= 0) return BNF4_ERR_CUDA;
     const bool gelu = p.epilogue == EPI_GELU_FP4 || p.epilogue == EPI_GELU_I8;
     const bool gelu_plain = !gelu || (p.act_scale <= 700.0f && (p.n % 32) == 0 && (p.epilogue == EPI_GELU_FP4 ? (p.next_nvec == 1 && p.d_i8 == nullptr) : p.next_nvec <= 1));
-    const int rk = p.rank == 4 ? 4 : ((p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1)) ? 1 : 0);
+    const int rk = p.rank == 4 && (p.rows_per_member % 16) == 0 ? 4 : ((p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1)) ? 1 : 0);
     // CTA pairs pay where the mainloop is longer than the epilogue and there is a tile for every pair. Measured at 65536 x 512 (us, single
     // CTAs -> pairs): fp32 / half / residual epilogues, rank 1: K 512 33.9 -> 35.9, 25.6 -> 27.0, 29.0 -> 29.8; K 1024 42.7 -> 38.2,
     // 33.1 -> 30.2, 36.1 -> 33.1; K 4096 107 -> 80, 96 -> 70, 98 -> 74. Rank 4 with the last two: K 1024 37.2 -> 39.2, 43.3 -> 45.4, K 1536

@@ -923,8 +923,8 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     m->M = static_cast<long long>(W) * m->R;
     if (m->M > 0x7fffffffLL / 8) { delete m; return set_error(BNF4_ERR_INVALID, "model_create: wave of %d members is too large", W); }
 
-    // one block of eight warps per 64 rows of a member, 16 to 64 blocks: a validation pass has one member only
-    m->ce_chunks = std::min(64, std::max(16, m->R / 64));
+    // one block of eight warps per 128 rows of a member, 16 to 64 blocks: a validation pass has one member only
+    m->ce_chunks = std::min(64, std::max(16, m->R / 128));
     const int V = m->V, H = m->H, F = m->F, L = m->L, T = m->T, r = m->r, P = cfg->max_pairs;
     const size_t hh = static_cast<size_t>(H) * H, hf = static_cast<size_t>(H) * F;
     int rc = 0;
