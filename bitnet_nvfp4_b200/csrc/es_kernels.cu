@@ -412,7 +412,16 @@ __global__ void __launch_bounds__(kZThreads) z_lowrank_tiles_kernel(const float*
     ZLowrankDesc d = single;
     int tile = static_cast<int>(blockIdx.x) - tables.blocks;
     int r0 = 0, nr = d.rows;
-    if (ndesc > 0) {
+    if (ndesc > 0 && nshards == 1) {
+        int lo = 0, hi = ndesc - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (descs[mid].tile0 <= tile) lo = mid; else hi = mid - 1;
+        }
+        d = descs[lo];
+        tile -= d.tile0;
+        nr = d.rows;
+    } else if (ndesc > 0) {
         int i = 0;
         for (;;) {
             d = descs[i];

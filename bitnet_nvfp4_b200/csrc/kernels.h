@@ -96,7 +96,9 @@ struct ZLowrankDesc {
     long long B_ps;
     float* Z;         // [rows][cols]
     int rows, cols;
+    int tile0;        // first 32 x 64 tile of this matrix in an unsharded launch over the table
 };
+inline int z_lowrank_tiles(int rows, int cols) { return ((rows + 31) / 32) * ((cols + 63) / 64); }
 struct ZDenseDesc {
     uint64_t salt;
     const int8_t* noise;  // the step's noise [pair][n] in memory, for the table form

@@ -739,8 +739,10 @@ inline bool vector_sharded(int n, int nshards) { return nshards > 1 && n >= 4096
 std::vector<ZLowrankDesc> z_descs(Model& m, float* z_base) {
     std::vector<ZLowrankDesc> d;
     long long off = 0;
+    int tile0 = 0;
     for (const UpdMatrix& x : update_matrices(m)) {
-        d.push_back({x.A, x.A_stride, x.Bt, x.B_stride, z_base + off, x.rows, x.cols});
+        d.push_back({x.A, x.A_stride, x.Bt, x.B_stride, z_base + off, x.rows, x.cols, tile0});
+        tile0 += z_lowrank_tiles(x.rows, x.cols);
         off += static_cast<long long>(x.rows) * x.cols;
     }
     return d;
