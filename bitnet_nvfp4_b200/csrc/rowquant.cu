@@ -314,10 +314,83 @@ __device__ __forceinline__ uint2 lds_u64(uint32_t saddr) {
 }
 // Element ownership as in rowquant_kernel: lane l owns the 16-element scale blocks l, l + 32, ... (NB of them).
 // NV = upper bound of p.nvec this instance handles (4 or kMaxTVec): the projection loops carry no tests beyond it.
+// More than four projections (NV = kMaxTVec): reading each row's sixteen vectors of up to 2 KB through L1 is what bounds the row loop, and
+// their accumulators push the row out of the registers. A warp therefore quantises p.batch (four) consecutive rows, keeping their int8
+// values in shared memory (each lane its own blocks), and then takes four vectors at a time against all four rows: a quarter of the
+// vector reads, 64 dp4a per eight 16-byte loads. The sums of 4 rows x 4 vectors are folded over the warp together (every exchange
+// halves the values a lane holds). p.batch is 1 where the rows would not give every resident warp a batch.
 // MODEL: the instance for the calls of the batched driver (power-of-two columns, rows per member, token and position counts;
 // exactly NV projections; no int8 copy; the residual branch as halves), which carries none of the corresponding tests.
+constexpr int kBatchRows = 4;
+constexpr int batch_smem(int nb) { return 8 * kBatchRows * nb * 32 * 16; }
+
+// t[row0 + r][v] of up to R rows staged by this warp (stage: [R][NB][32] 16-byte pieces). Warp-wide.
+template <int NB, int R>
+__device__ __forceinline__ void project_rows(const RowQuantParams& p, const uint4* stage, unsigned row0, unsigned nrows, int nblk, int lane) {
+    const unsigned rpm = static_cast<unsigned>(p.rows_per_member);
+    const unsigned pair_rows = 2u * rpm;
+    for (unsigned r0 = 0; r0 < nrows;) {  // rows r0 .. r1 - 1 belong to one pair
+        const unsigned pair = rpm > 0 ? (row0 + r0) / pair_rows : 0u;
+        const unsigned r1 = rpm > 0 ? min(nrows, (pair + 1u) * pair_rows - row0) : nrows;
+        const int8_t* tv = p.tvec + static_cast<size_t>(pair) * p.tvec_pair_stride + 16 * lane;
+        for (int v0 = 0; v0 < p.nvec; v0 += 4) {
+            int acc[R][4];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[r][j] = 0;
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                if (lane + 32 * i >= nblk) continue;
+                int4 b[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)  // the last group may be short: its tail repeats the last vector and is not stored
+                    b[j] = *reinterpret_cast<const int4*>(tv + static_cast<size_t>(min(v0 + j, p.nvec - 1)) * p.cols_out + 512 * i);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const uint4 w = stage[(r * NB + i) * 32 + lane];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        int a = acc[r][j];
+                        a = __dp4a(static_cast<int>(w.x), b[j].x, a);
+                        a = __dp4a(static_cast<int>(w.y), b[j].y, a);
+                        a = __dp4a(static_cast<int>(w.z), b[j].z, a);
+                        acc[r][j] = __dp4a(static_cast<int>(w.w), b[j].w, a);
+                    }
+                }
+            }
+            if constexpr (R == 1) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int tot = __reduce_add_sync(0xffffffffu, acc[0][j]);
+                    if (lane == 0 && v0 + j < p.nvec) p.t_out[static_cast<size_t>(row0) * p.nvec + v0 + j] = tot;
+                }
+            } else {
+                // sixteen sums over 32 lanes: lane l ends with the sum of value l / 2 (row l / 8, vector (l / 2) % 4)
+                int x[8], y[4], z[2];
+                const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int lo = acc[q >> 2][q & 3], hi = acc[2 + (q >> 2)][q & 3];
+                    x[q] = (h16 ? hi : lo) + __shfl_xor_sync(0xffffffffu, h16 ? lo : hi, 16);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) y[q] = (h8 ? x[4 + q] : x[q]) + __shfl_xor_sync(0xffffffffu, h8 ? x[q] : x[4 + q], 8);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) z[q] = (h4 ? y[2 + q] : y[q]) + __shfl_xor_sync(0xffffffffu, h4 ? y[q] : y[2 + q], 4);
+                int tot = (h2 ? z[1] : z[0]) + __shfl_xor_sync(0xffffffffu, h2 ? z[0] : z[1], 2);
+                tot += __shfl_xor_sync(0xffffffffu, tot, 1);
+                const unsigned r = lane >> 3;
+                const int v = v0 + ((lane >> 1) & 3);
+                if (!(lane & 1) && r >= r0 && r < r1 && v < p.nvec) p.t_out[static_cast<size_t>(row0 + r) * p.nvec + v] = tot;
+            }
+        }
+        r0 = r1;
+    }
+}
+
 template <int FE, int NB, int NV, bool MODEL = false>
-__global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowquant_fast_kernel(const RowQuantParams p, const uint8_t* __restrict__ lut) {
+__global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1))) rowquant_fast_kernel(const RowQuantParams p, const uint8_t* __restrict__ lut) {
     pdl_trigger();
     __shared__ __align__(16) uint2 tab_s[128];  // per amax: {bits of fl(1 / scale), scale byte}
     if (threadIdx.x < 128) tab_s[threadIdx.x] = __ldg(reinterpret_cast<const uint2*>(lut + kQuantBlockTabOffset) + threadIdx.x);
@@ -339,7 +412,17 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
     const bool pos_mod_pow2 = MODEL || (p.pos_mod > 0 && (p.pos_mod & (p.pos_mod - 1)) == 0);
     const int rpm_shift = (p.rows_per_member > 0 && (p.rows_per_member & (p.rows_per_member - 1)) == 0) ? __ffs(p.rows_per_member) - 1 : -1;
     const float inv_cols = 1.0f / static_cast<float>(p.cols_in);
-    for (unsigned row = (blockIdx.x + opaque_zero()) * 8u + (threadIdx.x >> 5); row < rows; row += gridDim.x * 8u) {
+    constexpr bool BATCH = NV > 4;
+    const unsigned batch = BATCH ? static_cast<unsigned>(p.batch) : 1u;
+    uint4* stage = nullptr;
+    if constexpr (BATCH) {
+        extern __shared__ __align__(16) uint4 batch_stage[];
+        stage = batch_stage + (threadIdx.x >> 5) * (kBatchRows * NB * 32);
+    }
+    unsigned in_batch = 0;  // rows of the current batch before this one
+    unsigned next_row;
+    for (unsigned row = ((blockIdx.x + opaque_zero()) * 8u + (threadIdx.x >> 5)) * batch; row < rows; row = next_row) {
+        next_row = BATCH && in_batch + 1 < batch ? row + 1 : row - in_batch + gridDim.x * 8u * batch;
         // rows per member is a power of two in every model configuration: a shift instead of a division per row
         const int member = (MODEL || p.rows_per_member > 0) ? static_cast<int>((MODEL || rpm_shift >= 0) ? row >> rpm_shift : row / static_cast<unsigned>(p.rows_per_member)) : 0;
         const int row_in_member = (MODEL || p.rows_per_member > 0) ? static_cast<int>(row - static_cast<unsigned>(member) * static_cast<unsigned>(p.rows_per_member)) : static_cast<int>(row);
@@ -349,17 +432,16 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
         // The row this warp takes next starts its trip from DRAM to L2 now: a warp holds one row's loads at a time, too few
         // bytes in flight to cover the DRAM latency with the narrow inputs (int8 rows, a branch travelling as halves).
         if constexpr (FE == FE_ADD_ABSMEAN || FE == FE_ABSMEAN) {
-            const unsigned nrow = row + gridDim.x * 8u;
-            if (nrow < rows) {
+            if (next_row < rows) {
 #pragma unroll
                 for (int i = 0; i < NB; ++i) {
                     const int k0 = (lane + 32 * i) << 4;
                     if (k0 >= p.cols_in) continue;
                     if constexpr (FE == FE_ABSMEAN) {
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.in_i8 + static_cast<size_t>(nrow) * p.ld_in + k0));
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.in_i8 + static_cast<size_t>(next_row) * p.ld_in + k0));
                     } else if (MODEL || p.in_f16) {
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.inout_i8 + static_cast<size_t>(nrow) * p.cols_in + k0));
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const __half*>(p.in_f32) + static_cast<size_t>(nrow) * p.ld_in + k0));
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.inout_i8 + static_cast<size_t>(next_row) * p.cols_in + k0));
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const __half*>(p.in_f32) + static_cast<size_t>(next_row) * p.ld_in + k0));
                     }
                 }
             }
@@ -575,9 +657,9 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
         }
 
         // ---------------- stage 3: int8 copy, codes, scales, rank-r projections ----------------
-        int tacc[NV];
+        int tacc[BATCH ? 1 : NV];
 #pragma unroll
-        for (int v = 0; v < NV; ++v) tacc[v] = 0;
+        for (int v = 0; v < (BATCH ? 1 : NV); ++v) tacc[v] = 0;
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
             const int kb = lane + 32 * i;
@@ -646,24 +728,20 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
                         tacc[v] = a;
                     }
                 }
+            } else if constexpr (BATCH) {
+                if (active) stage[(in_batch * NB + i) * 32 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
             } else if (p.nvec > 0 && active) {
                 const int8_t* tv = p.tvec + static_cast<size_t>(pair) * p.tvec_pair_stride + k0;
 #pragma unroll
-                for (int vg = 0; vg < NV / 4; ++vg) {
-                    if (4 * vg < p.nvec) {  // warp-uniform; projections come in groups of four or fewer
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int v = 4 * vg + j;
-                            if (v < p.nvec) {
-                                const int4 bv = *reinterpret_cast<const int4*>(tv + static_cast<size_t>(v) * p.cols_out);
-                                int a = tacc[v];
-                                a = __dp4a(static_cast<int>(w[0]), bv.x, a);
-                                a = __dp4a(static_cast<int>(w[1]), bv.y, a);
-                                a = __dp4a(static_cast<int>(w[2]), bv.z, a);
-                                a = __dp4a(static_cast<int>(w[3]), bv.w, a);
-                                tacc[v] = a;
-                            }
-                        }
+                for (int v = 0; v < NV; ++v) {
+                    if (v < p.nvec) {
+                        const int4 bv = *reinterpret_cast<const int4*>(tv + static_cast<size_t>(v) * p.cols_out);
+                        int a = tacc[v];
+                        a = __dp4a(static_cast<int>(w[0]), bv.x, a);
+                        a = __dp4a(static_cast<int>(w[1]), bv.y, a);
+                        a = __dp4a(static_cast<int>(w[2]), bv.z, a);
+                        a = __dp4a(static_cast<int>(w[3]), bv.w, a);
+                        tacc[v] = a;
                     }
                 }
             }
@@ -680,23 +758,26 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 ? 2 : 1))) rowqua
                     if (lane == 0) p.t_out[static_cast<size_t>(row) * NV + v] = tot;
                 }
             }
+        } else if constexpr (BATCH) {
+            if (in_batch + 1 == batch || row + 1 == rows) {
+                if (batch == kBatchRows) project_rows<NB, kBatchRows>(p, stage, row - in_batch, in_batch + 1, nblk, lane);
+                else project_rows<NB, 1>(p, stage, row, 1, nblk, lane);
+                if (row + 1 == rows) break;
+                in_batch = 0;
+            } else {
+                ++in_batch;
+            }
         } else if (p.nvec > 0) {
+            if (p.nvec == 4 && (reinterpret_cast<uintptr_t>(p.t_out) & 15) == 0) {  // the four column groups of the fused q | k | v | beta projection: one 16-byte store
+                const int t0 = __reduce_add_sync(0xffffffffu, tacc[0]), t1 = __reduce_add_sync(0xffffffffu, tacc[1]);
+                const int t2 = __reduce_add_sync(0xffffffffu, tacc[2]), t3 = __reduce_add_sync(0xffffffffu, tacc[3]);
+                if (lane == 0) *reinterpret_cast<int4*>(p.t_out + static_cast<size_t>(row) * 4) = make_int4(t0, t1, t2, t3);
+            } else {
 #pragma unroll
-            for (int vg = 0; vg < NV / 4; ++vg) {
-                if (4 * vg < p.nvec) {
-                    if (p.nvec == 4 && vg == 0 && (reinterpret_cast<uintptr_t>(p.t_out) & 15) == 0) {  // the four column groups of the fused q | k | v | beta projection: one 16-byte store
-                        const int t0 = __reduce_add_sync(0xffffffffu, tacc[0]), t1 = __reduce_add_sync(0xffffffffu, tacc[1]);
-                        const int t2 = __reduce_add_sync(0xffffffffu, tacc[2]), t3 = __reduce_add_sync(0xffffffffu, tacc[3]);
-                        if (lane == 0) *reinterpret_cast<int4*>(p.t_out + static_cast<size_t>(row) * 4) = make_int4(t0, t1, t2, t3);
-                        continue;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int v = 4 * vg + j;
-                        if (v < p.nvec) {
-                            const int tot = __reduce_add_sync(0xffffffffu, tacc[v]);
-                            if (lane == 0) p.t_out[static_cast<size_t>(row) * p.nvec + v] = tot;
-                        }
+                for (int v = 0; v < NV; ++v) {
+                    if (v < p.nvec) {
+                        const int tot = __reduce_add_sync(0xffffffffu, tacc[v]);
+                        if (lane == 0) p.t_out[static_cast<size_t>(row) * p.nvec + v] = tot;
                     }
                 }
             }
@@ -742,16 +823,24 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
             const int sms = multiprocessors(dev);
             if (sms <= 0) return BNF4_ERR_CUDA;
             // persistent CTAs: exactly as many as are resident at once (each loads its 1 KB copy of the table once)
-            auto run = [&](auto kernel, std::atomic<int>* resident) -> int {
+            auto run = [&](auto kernel, std::atomic<int>* resident, int smem = 0) -> int {
                 int per_sm = resident[dev].load(std::memory_order_relaxed);
                 if (per_sm == 0) {  // looked up once per kernel and device
-                    const int rc2 = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, 0), "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+                    int rc2 = smem > 48 * 1024 ? check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute(rowquant_fast_kernel)") : BNF4_OK;
+                    if (!rc2) rc2 = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem), "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
                     if (rc2) return rc2;
                     per_sm = std::max(per_sm, 1);
                     resident[dev].store(per_sm, std::memory_order_relaxed);
                 }
-                const unsigned grid = std::min(ctas, static_cast<unsigned>(sms) * static_cast<unsigned>(per_sm));
-                launch_pdl_if(early, kernel, grid, warps * 32, 0, stream, p, lut);
+                unsigned work = ctas;
+                const unsigned fit = static_cast<unsigned>(sms) * static_cast<unsigned>(per_sm);
+                RowQuantParams q = p;
+                q.batch = 1;
+                if (smem > 0 && ctas >= kBatchRows * fit) {  // a batch of rows for every resident warp
+                    q.batch = kBatchRows;
+                    work = (ctas + kBatchRows - 1) / kBatchRows;
+                }
+                launch_pdl_if(early, kernel, std::min(work, fit), warps * 32, smem, stream, q, lut);
                 return BNF4_OK;
             };
             // the batched driver's calls at hidden <= 512: see MODEL above
@@ -772,9 +861,9 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
                 else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, 4>, resident_ctas<FE, 2, 4>);
                 else rc = run(rowquant_fast_kernel<FE, 4, 4>, resident_ctas<FE, 4, 4>);
             } else {
-                if (nblk <= 32) rc = run(rowquant_fast_kernel<FE, 1, kMaxTVec>, resident_ctas<FE, 1, kMaxTVec>);
-                else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, kMaxTVec>, resident_ctas<FE, 2, kMaxTVec>);
-                else rc = run(rowquant_fast_kernel<FE, 4, kMaxTVec>, resident_ctas<FE, 4, kMaxTVec>);
+                if (nblk <= 32) rc = run(rowquant_fast_kernel<FE, 1, kMaxTVec>, resident_ctas<FE, 1, kMaxTVec>, batch_smem(1));
+                else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, kMaxTVec>, resident_ctas<FE, 2, kMaxTVec>, batch_smem(2));
+                else rc = run(rowquant_fast_kernel<FE, 4, kMaxTVec>, resident_ctas<FE, 4, kMaxTVec>, batch_smem(4));
             }
             if (rc) return rc;
             return check_launch("rowquant_fast_kernel");

@@ -1,0 +1,41 @@
+"""Row quantisers with more than four projections: several rows per warp, whose projections are taken together."""
+import numpy as np
+import pytest
+
+import oracle_lib as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,hid,nvec,rpm", [
+    (19011, 320, 16, 17),     # pairs end inside a batch of four rows; the last batch has three; idle lanes
+    (19009, 512, 7, 1),       # two rows per pair; a last batch of one row; a short last group of vectors
+    (19600, 1024, 8, 4900),   # two blocks per lane
+    (9602, 2048, 5, 4801),    # four blocks per lane, a group of one vector
+    (19008, 16, 12, 0),       # one block per row, one set of vectors for all rows
+    (50, 512, 12, 3),         # too few rows for batches
+])
+def test_more_than_four_projections(rows, hid, nvec, rpm):
+    import torch
+    from bitnet_nvfp4_b200 import host as H
+    rng = np.random.default_rng(rows + hid)
+    pairs = (rows + 2 * rpm - 1) // (2 * rpm) if rpm else 1
+    x = rng.integers(-127, 128, (rows, hid)).astype(np.int8)
+    tvec = rng.integers(-127, 128, (pairs, nvec, hid)).astype(np.int8)
+    xd, tv = torch.from_numpy(x).cuda(), torch.from_numpy(tvec).cuda()
+    yq = torch.zeros((rows, hid), dtype=torch.int8, device="cuda")
+    codes = torch.zeros(rows * hid // 2, dtype=torch.uint8, device="cuda")
+    sf = torch.zeros(H.sf_bytes(rows, hid), dtype=torch.uint8, device="cuda")
+    t = torch.full((rows + 1, nvec), -7, dtype=torch.int32, device="cuda")
+    H.rowquant(H.FE_ABSMEAN, rows=rows, cols_in=hid, cols_out=hid, rows_per_member=rpm, in_i8=xd, ld_in=hid, norm_scale=40.0, out_q=yq,
+               ld_q=hid, out_codes=codes, out_sf=sf, tvec=tv, tvec_pair_stride=nvec * hid, nvec=nvec, t_out=t)
+    q, c, s = orc.absmean_norm_q(x.copy(), None, 0.0, 40.0)
+    assert np.array_equal(yq.cpu().numpy(), q)
+    assert np.array_equal(codes.cpu().numpy(), np.asarray(c).reshape(-1)) and np.array_equal(sf.cpu().numpy(), np.asarray(s).reshape(-1))
+    pair = np.arange(rows) // (2 * rpm) if rpm else np.zeros(rows, int)
+    ref = np.empty((rows, nvec), np.int32)
+    for p in range(pairs):
+        ref[pair == p] = q[pair == p].astype(np.int32) @ tvec[p].astype(np.int32).T
+    got = t.cpu().numpy()
+    assert np.array_equal(got[:rows], ref)
+    assert (got[rows] == -7).all()
