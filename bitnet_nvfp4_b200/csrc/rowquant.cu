@@ -314,58 +314,64 @@ __device__ __forceinline__ uint2 lds_u64(uint32_t saddr) {
 }
 // Element ownership as in rowquant_kernel: lane l owns the 16-element scale blocks l, l + 32, ... (NB of them).
 // NV = upper bound of p.nvec this instance handles (4 or kMaxTVec): the projection loops carry no tests beyond it.
-// More than four projections (NV = kMaxTVec): reading each row's sixteen vectors of up to 2 KB through L1 is what bounds the row loop, and
-// their accumulators push the row out of the registers. A warp therefore quantises p.batch (four) consecutive rows, keeping their int8
-// values in shared memory (each lane its own blocks), and then takes four vectors at a time against all four rows: a quarter of the
-// vector reads, 64 dp4a per eight 16-byte loads. The sums of 4 rows x 4 vectors are folded over the warp together (every exchange
-// halves the values a lane holds). p.batch is 1 where the rows would not give every resident warp a batch.
-// MODEL: the instance for the calls of the batched driver (power-of-two columns, rows per member, token and position counts;
-// exactly NV projections; no int8 copy; the residual branch as halves), which carries none of the corresponding tests.
-constexpr int kBatchRows = 4;
-constexpr int batch_smem(int nb) { return 8 * kBatchRows * nb * 32 * 16; }
+// BATCH (more than four projections): a 16-byte load per block and vector, one dp4a per four bytes, a warp reduction (8 cycles) per sum and
+// sixteen accumulators cost more than the quantisation itself. A warp therefore quantises p.batch consecutive rows, keeping their int8
+// values in shared memory, and reads each vector once for all of them. Rows of up to 1024 columns: eight rows, integer matrix instructions
+// (vectors as rows of A, staged rows as columns of B: 4096 products in 8 cycles, no reduction over lanes). Wider rows: four rows (eight would
+// leave one block per SM), where half of B would be empty; four vectors at a time with dp4a, whose 4 x 4 sums are folded over the warp
+// together, are faster there (262144 x 2048, 16 projections: 559 us, 619 us with matrix instructions, 997 us one row at a time).
+// 88800 x 320 with eight projections: 80 us one row at a time, 43 us with dp4a on four rows, 34 us here. With four projections (the
+// batched driver's instance, 1048576 x 512) one row at a time stays ahead: 337 us against 390 us.
+// p.batch is 1 where the rows would not give every resident warp a batch.
+__host__ __device__ constexpr int batch_rows(int nb) { return nb >= 4 ? 4 : 8; }
+__host__ __device__ constexpr int batch_smem(int nb) { return 8 * batch_rows(nb) * nb * 32 * 16; }
+// 16-byte piece c of staged row r: odd rows swap the halves of 128-byte lines, so that two rows' reads share no bank
+__device__ __forceinline__ int stage_piece(int r, int c, int nb) { return r * (nb * 32) + (c ^ ((r & 1) << 2)); }
 
-// t[row0 + r][v] of up to R rows staged by this warp (stage: [R][NB][32] 16-byte pieces). Warp-wide.
-template <int NB, int R>
-__device__ __forceinline__ void project_rows(const RowQuantParams& p, const uint4* stage, unsigned row0, unsigned nrows, int nblk, int lane) {
-    const unsigned rpm = static_cast<unsigned>(p.rows_per_member);
-    const unsigned pair_rows = 2u * rpm;
+__device__ __forceinline__ void mma_s8_16832(int (&d)[4], int a0, int a1, int a2, int a3, int b0, int b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// t[row0 + r][v] of the rows staged by this warp. Lane (g, tq) supplies 16 contiguous bytes of vectors g and g + 8 and of row g: which of the
+// 64 columns of a step meet in which instruction does not matter for the sum, as long as both sides agree.
+template <int NB>
+__device__ __forceinline__ void project_rows(const RowQuantParams& p, const int4* stage, unsigned row0, unsigned nrows, int nblk, int lane) {
+    const int g = lane >> 2, tq = lane & 3;
+    const unsigned pair_rows = 2u * static_cast<unsigned>(p.rows_per_member);
     for (unsigned r0 = 0; r0 < nrows;) {  // rows r0 .. r1 - 1 belong to one pair
-        const unsigned pair = rpm > 0 ? (row0 + r0) / pair_rows : 0u;
-        const unsigned r1 = rpm > 0 ? min(nrows, (pair + 1u) * pair_rows - row0) : nrows;
-        const int8_t* tv = p.tvec + static_cast<size_t>(pair) * p.tvec_pair_stride + 16 * lane;
-        for (int v0 = 0; v0 < p.nvec; v0 += 4) {
-            int acc[R][4];
+        const unsigned pair = pair_rows > 0 ? (row0 + r0) / pair_rows : 0u;
+        const unsigned r1 = pair_rows > 0 ? min(nrows, (pair + 1u) * pair_rows - row0) : nrows;
+        const int8_t* tv = p.tvec + static_cast<size_t>(pair) * p.tvec_pair_stride;
+        if constexpr (NB >= 4) {
+            constexpr int R = batch_rows(NB);
+            for (int v0 = 0; v0 < p.nvec; v0 += 4) {
+                int acc[R][4];
 #pragma unroll
-            for (int r = 0; r < R; ++r)
+                for (int r = 0; r < R; ++r)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[r][j] = 0;
+                    for (int j = 0; j < 4; ++j) acc[r][j] = 0;
 #pragma unroll
-            for (int i = 0; i < NB; ++i) {
-                if (lane + 32 * i >= nblk) continue;
-                int4 b[4];
+                for (int i = 0; i < NB; ++i) {
+                    if (lane + 32 * i >= nblk) continue;
+                    int4 b[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j)  // the last group may be short: its tail repeats the last vector and is not stored
-                    b[j] = *reinterpret_cast<const int4*>(tv + static_cast<size_t>(min(v0 + j, p.nvec - 1)) * p.cols_out + 512 * i);
+                    for (int j = 0; j < 4; ++j)  // the last group may be short: its tail repeats the last vector and is not stored
+                        b[j] = *reinterpret_cast<const int4*>(tv + 16 * lane + static_cast<size_t>(min(v0 + j, p.nvec - 1)) * p.cols_out + 512 * i);
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const uint4 w = stage[(r * NB + i) * 32 + lane];
+                    for (int r = 0; r < R; ++r) {
+                        const int4 w = stage[stage_piece(r, lane + 32 * i, NB)];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        int a = acc[r][j];
-                        a = __dp4a(static_cast<int>(w.x), b[j].x, a);
-                        a = __dp4a(static_cast<int>(w.y), b[j].y, a);
-                        a = __dp4a(static_cast<int>(w.z), b[j].z, a);
-                        acc[r][j] = __dp4a(static_cast<int>(w.w), b[j].w, a);
+                        for (int j = 0; j < 4; ++j) {
+                            int a = acc[r][j];
+                            a = __dp4a(w.x, b[j].x, a);
+                            a = __dp4a(w.y, b[j].y, a);
+                            a = __dp4a(w.z, b[j].z, a);
+                            acc[r][j] = __dp4a(w.w, b[j].w, a);
+                        }
                     }
                 }
-            }
-            if constexpr (R == 1) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int tot = __reduce_add_sync(0xffffffffu, acc[0][j]);
-                    if (lane == 0 && v0 + j < p.nvec) p.t_out[static_cast<size_t>(row0) * p.nvec + v0 + j] = tot;
-                }
-            } else {
                 // sixteen sums over 32 lanes: lane l ends with the sum of value l / 2 (row l / 8, vector (l / 2) % 4)
                 int x[8], y[4], z[2];
                 const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
@@ -383,6 +389,26 @@ __device__ __forceinline__ void project_rows(const RowQuantParams& p, const uint
                 const unsigned r = lane >> 3;
                 const int v = v0 + ((lane >> 1) & 3);
                 if (!(lane & 1) && r >= r0 && r < r1 && v < p.nvec) p.t_out[static_cast<size_t>(row0 + r) * p.nvec + v] = tot;
+            }
+        } else {
+            const int8_t* tg = tv + static_cast<size_t>(g) * p.cols_out + 16 * tq;
+            int d[4] = {0, 0, 0, 0}, d2[4] = {0, 0, 0, 0};  // two chains
+#pragma unroll 4
+            for (int c0 = 0; c0 < nblk; c0 += 4) {
+                int4 lo = make_int4(0, 0, 0, 0), hi = lo, w = lo;
+                if (c0 + tq < nblk) {
+                    if (g < p.nvec) lo = *reinterpret_cast<const int4*>(tg + 16 * c0);
+                    if (g + 8 < p.nvec) hi = *reinterpret_cast<const int4*>(tg + 8 * static_cast<size_t>(p.cols_out) + 16 * c0);
+                    if (g < batch_rows(NB)) w = stage[stage_piece(g, c0 + tq, NB)];
+                }
+                mma_s8_16832(d, lo.x, hi.x, lo.y, hi.y, w.x, w.y);
+                mma_s8_16832(d2, lo.z, hi.z, lo.w, hi.w, w.z, w.w);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const unsigned r = 2 * tq + (e & 1);
+                const int v = g + 8 * (e >> 1);
+                if (r >= r0 && r < r1 && v < p.nvec) p.t_out[static_cast<size_t>(row0 + r) * p.nvec + v] = d[e] + d2[e];
             }
         }
         r0 = r1;
@@ -414,10 +440,10 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
     const float inv_cols = 1.0f / static_cast<float>(p.cols_in);
     constexpr bool BATCH = NV > 4;
     const unsigned batch = BATCH ? static_cast<unsigned>(p.batch) : 1u;
-    uint4* stage = nullptr;
+    int4* stage = nullptr;
     if constexpr (BATCH) {
-        extern __shared__ __align__(16) uint4 batch_stage[];
-        stage = batch_stage + (threadIdx.x >> 5) * (kBatchRows * NB * 32);
+        extern __shared__ __align__(16) int4 batch_stage[];
+        stage = batch_stage + (threadIdx.x >> 5) * (batch_rows(NB) * NB * 32);
     }
     unsigned in_batch = 0;  // rows of the current batch before this one
     unsigned next_row;
@@ -714,7 +740,11 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
             // eight sectors a word store would
             if (active) p.out_sf[sf_offset(static_cast<int>(row), kb, k_atoms)] = static_cast<uint8_t>(sfb);
 
-            if constexpr (MODEL) {
+            if constexpr (BATCH) {
+                if (active)
+                    stage[stage_piece(static_cast<int>(in_batch), kb, NB)] =
+                        make_int4(static_cast<int>(w[0]), static_cast<int>(w[1]), static_cast<int>(w[2]), static_cast<int>(w[3]));
+            } else if constexpr (MODEL) {
                 if (active) {
                     const int8_t* tv = p.tvec + static_cast<size_t>(pair) * p.tvec_pair_stride + k0;
 #pragma unroll
@@ -728,8 +758,6 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                         tacc[v] = a;
                     }
                 }
-            } else if constexpr (BATCH) {
-                if (active) stage[(in_batch * NB + i) * 32 + lane] = make_uint4(w[0], w[1], w[2], w[3]);
             } else if (p.nvec > 0 && active) {
                 const int8_t* tv = p.tvec + static_cast<size_t>(pair) * p.tvec_pair_stride + k0;
 #pragma unroll
@@ -746,7 +774,17 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                 }
             }
         }
-        if constexpr (MODEL) {
+        if constexpr (BATCH) {
+            if (in_batch + 1 == batch || row + 1 == rows) {
+                __syncwarp();
+                project_rows<NB>(p, stage, row - in_batch, in_batch + 1, nblk, lane);
+                if (row + 1 == rows) break;
+                __syncwarp();
+                in_batch = 0;
+            } else {
+                ++in_batch;
+            }
+        } else if constexpr (MODEL) {
             if constexpr (NV == 4) {
                 const int t0 = __reduce_add_sync(0xffffffffu, tacc[0]), t1 = __reduce_add_sync(0xffffffffu, tacc[1]);
                 const int t2 = __reduce_add_sync(0xffffffffu, tacc[2]), t3 = __reduce_add_sync(0xffffffffu, tacc[3]);
@@ -757,15 +795,6 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                     const int tot = __reduce_add_sync(0xffffffffu, tacc[v]);
                     if (lane == 0) p.t_out[static_cast<size_t>(row) * NV + v] = tot;
                 }
-            }
-        } else if constexpr (BATCH) {
-            if (in_batch + 1 == batch || row + 1 == rows) {
-                if (batch == kBatchRows) project_rows<NB, kBatchRows>(p, stage, row - in_batch, in_batch + 1, nblk, lane);
-                else project_rows<NB, 1>(p, stage, row, 1, nblk, lane);
-                if (row + 1 == rows) break;
-                in_batch = 0;
-            } else {
-                ++in_batch;
             }
         } else if (p.nvec > 0) {
             if (p.nvec == 4 && (reinterpret_cast<uintptr_t>(p.t_out) & 15) == 0) {  // the four column groups of the fused q | k | v | beta projection: one 16-byte store
@@ -823,7 +852,7 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
             const int sms = multiprocessors(dev);
             if (sms <= 0) return BNF4_ERR_CUDA;
             // persistent CTAs: exactly as many as are resident at once (each loads its 1 KB copy of the table once)
-            auto run = [&](auto kernel, std::atomic<int>* resident, int smem = 0) -> int {
+            auto run = [&](auto kernel, std::atomic<int>* resident, int smem = 0, int batch = 1) -> int {
                 int per_sm = resident[dev].load(std::memory_order_relaxed);
                 if (per_sm == 0) {  // looked up once per kernel and device
                     int rc2 = smem > 48 * 1024 ? check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "cudaFuncSetAttribute(rowquant_fast_kernel)") : BNF4_OK;
@@ -836,9 +865,9 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
                 const unsigned fit = static_cast<unsigned>(sms) * static_cast<unsigned>(per_sm);
                 RowQuantParams q = p;
                 q.batch = 1;
-                if (smem > 0 && ctas >= kBatchRows * fit) {  // a batch of rows for every resident warp
-                    q.batch = kBatchRows;
-                    work = (ctas + kBatchRows - 1) / kBatchRows;
+                if (batch > 1 && ctas >= batch * fit) {  // a batch of rows for every resident warp
+                    q.batch = batch;
+                    work = (ctas + batch - 1) / batch;
                 }
                 launch_pdl_if(early, kernel, std::min(work, fit), warps * 32, smem, stream, q, lut);
                 return BNF4_OK;
@@ -861,9 +890,9 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
                 else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, 4>, resident_ctas<FE, 2, 4>);
                 else rc = run(rowquant_fast_kernel<FE, 4, 4>, resident_ctas<FE, 4, 4>);
             } else {
-                if (nblk <= 32) rc = run(rowquant_fast_kernel<FE, 1, kMaxTVec>, resident_ctas<FE, 1, kMaxTVec>, batch_smem(1));
-                else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, kMaxTVec>, resident_ctas<FE, 2, kMaxTVec>, batch_smem(2));
-                else rc = run(rowquant_fast_kernel<FE, 4, kMaxTVec>, resident_ctas<FE, 4, kMaxTVec>, batch_smem(4));
+                if (nblk <= 32) rc = run(rowquant_fast_kernel<FE, 1, kMaxTVec>, resident_ctas<FE, 1, kMaxTVec>, batch_smem(1), batch_rows(1));
+                else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, kMaxTVec>, resident_ctas<FE, 2, kMaxTVec>, batch_smem(2), batch_rows(2));
+                else rc = run(rowquant_fast_kernel<FE, 4, kMaxTVec>, resident_ctas<FE, 4, kMaxTVec>, batch_smem(4), batch_rows(4));
             }
             if (rc) return rc;
             return check_launch("rowquant_fast_kernel");

@@ -8,11 +8,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("rows,hid,nvec,rpm", [
-    (19011, 320, 16, 17),     # pairs end inside a batch of four rows; the last batch has three; idle lanes
-    (19009, 512, 7, 1),       # two rows per pair; a last batch of one row; a short last group of vectors
-    (19600, 1024, 8, 4900),   # two blocks per lane
-    (9602, 2048, 5, 4801),    # four blocks per lane, a group of one vector
-    (19008, 16, 12, 0),       # one block per row, one set of vectors for all rows
+    (37891, 320, 16, 17),     # pairs end inside a batch of eight rows; the last batch has three; a tail of the columns
+    (37889, 512, 7, 1),       # two rows per pair; a last batch of one row; one half of the vectors' operand empty
+    (28420, 1024, 9, 14210),  # two blocks per lane, one vector in the second half
+    (9602, 2048, 5, 4801),    # four rows per batch, a group of one vector
+    (9603, 1536, 13, 5),      # idle lanes in the last block; pairs end inside a batch; a last batch of three rows
+    (37888, 16, 12, 0),       # one block per row, one set of vectors for all rows
     (50, 512, 12, 3),         # too few rows for batches
 ])
 def test_more_than_four_projections(rows, hid, nvec, rpm):
