@@ -1,4 +1,4 @@
-"""In-tree build of libbnf4.so (sm_100a only) with nvcc.
+"""In-tree build of libbnf4.so (sm_100a only) with nvcc, and of _host.so (the Python-side call path over it) with g++.
 
     python -m bitnet_nvfp4_b200.build            # incremental
     python -m bitnet_nvfp4_b200.build --force    # rebuild everything
@@ -20,6 +20,7 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "libbnf4.so"
+HOST = PKG / "_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -82,7 +83,32 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link of libbnf4.so failed")
+    build_host(force)
     return LIB
+
+
+def build_host(force: bool = False) -> Path:
+    """_host.so: a CPython extension on torch's C++ tensors, linked to the libbnf4.so beside it."""
+    src = CSRC / "binding" / "host_calls.cpp"
+    if not force and not _newer(src, HOST, [ROOT / "include" / "bnf4.h"]):
+        return HOST
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    gxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+    cuda = Path(_nvcc()).resolve().parent.parent / "include"
+    torch_lib = Path(torch.__file__).resolve().parent / "lib"
+    cmd = [gxx, "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-isystem{d}" for d in [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], cuda]], f"-I{ROOT / 'include'}", str(src),
+           "-o", str(HOST), f"-L{PKG}", "-l:libbnf4.so", "-Wl,-rpath,$ORIGIN", f"-L{torch_lib}", "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
+           "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("build of _host.so failed")
+    return HOST
 
 
 if __name__ == "__main__":

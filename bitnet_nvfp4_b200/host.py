@@ -3,6 +3,9 @@ the reference's src/cuda_kernels.h and src/efla_lm_kernels.h), on torch device t
 
 Function names and argument meaning follow the reference; every call goes through the C ABI of
 libbnf4.so on the current CUDA stream. torch is used for device memory and streams only.
+
+The functions that a token loop calls dozens of times per token go through _host.so, which converts arguments, allocates the
+outputs and calls the library natively (8.5 us per call through ctypes, more than the kernels take).
 """
 from __future__ import annotations
 
@@ -25,6 +28,24 @@ def c_rank(rank: int) -> float:
 
 
 _stream = _l.stream
+_native = None
+
+
+def _n():
+    """The native call path. Raises if it has not been built, like lib.load()."""
+    global _native
+    if _native is None:
+        _l.load()
+        try:
+            from . import _host
+        except ImportError as e:
+            raise _l.Bnf4Error(f"_host.so cannot be loaded ({e}): build it with `python -m bitnet_nvfp4_b200.build`") from e
+        _host.set_error_class(_l.Bnf4Error)
+        codes = {C.c_void_p: "P", C.c_int: "i", C.c_float: "f", C.c_longlong: "q"}
+        for kind, desc in enumerate((_l.RowQuantDesc, _l.GemmDesc, _l.EflaDesc)):
+            _host.register_desc(kind, C.sizeof(desc), [(name, getattr(desc, name).offset, codes[t]) for name, t in desc._fields_])
+        _native = _host
+    return _native
 
 
 def _p(t):
@@ -56,11 +77,7 @@ def device_error() -> int:
 
 # ------------------------------------------------------------------------------------------ quantisers
 def nvfp4_quantize_a(x: torch.Tensor, k_out: int | None = None):
-    m, k_in = x.shape
-    k_out = k_out or k_in
-    _, codes, sf = _alloc_q(x, m, k_out, want_q=False)
-    _l.check(_l.load().bnf4_nvfp4_quantize_a(_p(x), m, 1, k_in, k_out, _p(codes), _p(sf), _stream()))
-    return codes, sf
+    return _n().quantize_a(x, k_out or x.shape[1])
 
 
 def nvfp4_quantize_b(w: torch.Tensor, k_out: int | None = None):
@@ -91,19 +108,11 @@ def nvfp4_quantize_wqkv_fused(wq, wk, wv, wb, hidden: int, rows_total: int, scal
 
 
 def embedding_lookup_noise_quantize_nvfp4(tokens_t, token_stride, emb_w, emb_noise, hidden, batch, noise_scale, anti_sign):
-    q, codes, sf = _alloc_q(emb_w, batch, hidden)
-    _l.check(_l.load().bnf4_embedding_lookup_noise_quantize_nvfp4(_p(tokens_t), token_stride, _p(emb_w), _p(emb_noise), hidden,
-                                                                  batch, noise_scale, anti_sign, _p(q), _p(codes), _p(sf),
-                                                                  _stream()))
-    return q, codes, sf
+    return _n().embedding_lookup_noise_quantize(tokens_t, token_stride, emb_w, emb_noise, hidden, batch, noise_scale, anti_sign)
 
 
 def add_pos_gelu_quantize_nvfp4(x, pos_t, act_scale):
-    batch, hidden = x.shape
-    q, codes, sf = _alloc_q(x, batch, hidden)
-    _l.check(_l.load().bnf4_add_pos_gelu_quantize_nvfp4(_p(x), _p(pos_t), hidden, batch, act_scale, _p(q), _p(codes), _p(sf),
-                                                        _stream()))
-    return q, codes, sf
+    return _n().add_pos_gelu_quantize(x, pos_t, act_scale)
 
 
 def activation_quantize_nvfp4(x, cols_out, activation):
@@ -122,50 +131,31 @@ def gelu_quantize_nvfp4(x, cols_out, act_scale):
 
 
 def absmean_norm_q_nvfp4(x8, scale):
-    batch, hidden = x8.shape
-    q, codes, sf = _alloc_q(x8, batch, hidden)
-    _l.check(_l.load().bnf4_absmean_norm_q_nvfp4(_p(x8), hidden, batch, hidden, scale, _p(q), _p(codes), _p(sf), _stream()))
-    return q, codes, sf
+    return _n().absmean_norm_q(x8, scale)
 
 
 def add_scaled_to_int8_absmean_norm_q_nvfp4(x8_inout, y, add_scale, norm_scale):
-    batch, hidden = x8_inout.shape
-    q, codes, sf = _alloc_q(y, batch, hidden)
-    _l.check(_l.load().bnf4_add_scaled_to_int8_absmean_norm_q_nvfp4(_p(x8_inout), _p(y), hidden, batch, hidden, add_scale,
-                                                                    norm_scale, _p(q), _p(codes), _p(sf), _stream()))
-    return q, codes, sf
+    return _n().add_scaled_absmean_norm_q(x8_inout, y, add_scale, norm_scale)
 
 
 def rowquant(front_end: int, **kw):
     """Generic row quantiser (bnf4_rowquant); keyword names are the fields of bnf4_rowquant_desc,
     tensors are converted to device pointers."""
-    d = _l.RowQuantDesc()
-    for k, v in kw.items():
-        setattr(d, k, _p(v) if isinstance(v, torch.Tensor) else v)
-    _l.check(_l.load().bnf4_rowquant(front_end, C.byref(d), _stream()))
+    _n().desc_call(0, front_end, kw)
 
 
 # ------------------------------------------------------------------------------------------ GEMM
 def gemm_ternary_f_nvfp4(a, b, sfa, sfb, m, n, k, alpha, beta=0.0, c=None, d=None):
-    if d is None:
-        d = a.new_empty((m, n), dtype=torch.float32)
-    _l.check(_l.load().bnf4_gemm_ternary_f_nvfp4(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, k, alpha, beta, _p(c), d.data_ptr(), _stream()))
-    return d
+    return _n().gemm(a, b, sfa, sfb, m, n, k, alpha, beta, c, d)
 
 
 def gemm_ternary_f_nvfp4_gelu_i8(a, b, sfa, sfb, m, n, k, alpha, beta, c, act_scale):
-    d = a.new_empty((m, n), dtype=torch.int8)
-    _l.check(_l.load().bnf4_gemm_ternary_f_nvfp4_gelu_i8(_p(a), _p(b), _p(sfa), _p(sfb), m, n, k, alpha, beta, _p(c), act_scale,
-                                                         _p(d), _stream()))
-    return d
+    return _n().gemm_gelu_i8(a, b, sfa, sfb, m, n, k, alpha, beta, c, act_scale)
 
 
 def gemm_nvfp4_ex(**kw):
     """Full-form GEMM (bnf4_gemm_nvfp4_ex); keyword names are the fields of bnf4_gemm_desc."""
-    g = _l.GemmDesc()
-    for k, v in kw.items():
-        setattr(g, k, _p(v) if isinstance(v, torch.Tensor) else v)
-    _l.check(_l.load().bnf4_gemm_nvfp4_ex(C.byref(g), _stream()))
+    _n().desc_call(1, 0, kw)
 
 
 # ------------------------------------------------------------------------------------------ ternary GEMM / rank-r helpers
@@ -202,17 +192,11 @@ def split_qkvb_fused(qkv, hidden, beta_bias):
 # ------------------------------------------------------------------------------------------ EFLA
 def efla_scan(**kw):
     """Whole-sequence scan / generic recurrence (bnf4_efla_scan); keyword names are the fields of bnf4_efla_desc."""
-    d = _l.EflaDesc()
-    for k, v in kw.items():
-        setattr(d, k, _p(v) if isinstance(v, torch.Tensor) else v)
-    _l.check(_l.load().bnf4_efla_scan(C.byref(d), _stream()))
+    _n().desc_call(2, 0, kw)
 
 
 def efla_step_half_qkv_fused(S, qkv, fused_cols, beta_bias, hidden, batch, method, eps):
-    out = qkv.new_empty((batch, hidden))
-    _l.check(_l.load().bnf4_efla_step_half_qkv_fused(_p(S), _p(qkv), fused_cols, beta_bias, hidden, batch, method, eps, _p(out),
-                                                     _stream()))
-    return out
+    return _n().efla_step_half(S, qkv, fused_cols, beta_bias, hidden, batch, method, eps)
 
 
 def efla_step_qkv_fused(S, qkv, fused_cols, beta_bias, hidden, batch, method, eps):
@@ -224,9 +208,7 @@ def efla_step_qkv_fused(S, qkv, fused_cols, beta_bias, hidden, batch, method, ep
 
 # ------------------------------------------------------------------------------------------ loss / noise / update
 def cross_entropy_loss(logits, bias, bias_noise, bias_noise_scale, targets_t, token_stride, loss_accum):
-    batch, vocab = logits.shape
-    _l.check(_l.load().bnf4_cross_entropy_loss(_p(logits), _p(bias), _p(bias_noise), bias_noise_scale, _p(targets_t),
-                                               token_stride, vocab, batch, _p(loss_accum), _stream()))
+    _n().cross_entropy(logits, bias, bias_noise, bias_noise_scale, targets_t, token_stride, loss_accum)
 
 
 def cross_entropy_population(logits, ld, bias, bias_noise_i8, sigma, targets, vocab, members, rows_per_member):

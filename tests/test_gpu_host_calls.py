@@ -1,0 +1,90 @@
+"""The native per-call path behind host.py: conversions, outputs, errors and threads, against direct calls of the C ABI."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def H():
+    import torch
+    from bitnet_nvfp4_b200 import host
+    assert torch.cuda.is_available()
+    return host
+
+
+def test_outputs_match_the_c_abi(H):
+    import torch
+    from bitnet_nvfp4_b200 import lib
+    x = torch.from_numpy(np.random.default_rng(1).integers(-127, 128, (33, 80)).astype(np.int8)).cuda()
+    codes, sf = H.nvfp4_quantize_a(x, 96)
+    c2, s2 = torch.empty_like(codes), torch.empty_like(sf)
+    assert codes.numel() == H.matrix_bytes(33, 96) and sf.numel() == H.sf_bytes(33, 96) and codes.device == x.device
+    lib.check(lib.load().bnf4_nvfp4_quantize_a(x.data_ptr(), 33, 1, 80, 96, c2.data_ptr(), s2.data_ptr(), lib.stream()))
+    assert torch.equal(codes, c2) and torch.equal(sf, s2)
+    d = torch.zeros((33, 33), device="cuda")
+    assert H.gemm_ternary_f_nvfp4(codes[: H.matrix_bytes(33, 64)], codes[: H.matrix_bytes(33, 64)], sf, sf, np.int64(33), 33, 64, 1, d=d) is d
+    assert H.gemm_ternary_f_nvfp4(codes, codes, sf, sf, 33, 33, 64, 1.0).shape == (33, 33)
+
+
+def test_descriptor_fields_of_every_type(H):
+    """Pointers as tensors, integers and None, 32- and 64-bit integers, floats from ints; names that are no fields are ignored."""
+    import torch
+    from bitnet_nvfp4_b200 import lib
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randint(-127, 128, (8, 64), dtype=torch.int8, device="cuda", generator=g)
+    tv = torch.randint(-4, 5, (2, 1, 64), dtype=torch.int8, device="cuda", generator=g)
+    got = []
+    for native in (True, False):
+        codes, sf, t = torch.zeros(256, dtype=torch.uint8, device="cuda"), torch.zeros(512, dtype=torch.uint8, device="cuda"), torch.zeros(8, dtype=torch.int32, device="cuda")
+        kw = dict(rows=np.int32(8), cols_in=64, cols_out=64, rows_per_member=2, in_i8=x.data_ptr(), ld_in=64, norm_scale=3, out_q=None, out_codes=codes, out_sf=sf,
+                  tvec=tv, tvec_pair_stride=64, nvec=True, t_out=t)
+        if native:
+            H.rowquant(H.FE_ABSMEAN, no_such_field=1, **kw)
+        else:
+            d = lib.RowQuantDesc()
+            for k, v in kw.items():
+                setattr(d, k, v.data_ptr() if isinstance(v, torch.Tensor) else int(v) if isinstance(v, np.integer) else v)
+            lib.check(lib.load().bnf4_rowquant(H.FE_ABSMEAN, C.byref(d), lib.stream()))
+        got.append((codes, sf, t))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+def test_errors(H):
+    import torch
+    from bitnet_nvfp4_b200.lib import Bnf4Error
+    x = torch.zeros((4, 64), dtype=torch.int8, device="cuda")
+    with pytest.raises(Bnf4Error):
+        H.nvfp4_quantize_a(x, 72)            # no multiple of 16
+    with pytest.raises(ValueError):
+        H.absmean_norm_q_nvfp4(x.view(-1), 1.0)
+    with pytest.raises(TypeError):
+        H.absmean_norm_q_nvfp4(x, "1.0")
+    with pytest.raises(TypeError):
+        H.rowquant(H.FE_ABSMEAN, rows=1.5)
+    with pytest.raises(Bnf4Error):
+        H.gemm_nvfp4_ex(m=1, n=1, k=63)
+
+
+def test_threads_use_their_own_streams(H):
+    import torch
+    x = [torch.full((64, 512), i + 1, dtype=torch.int8, device="cuda") for i in range(4)]
+    ref = [H.absmean_norm_q_nvfp4(t, 8.0) for t in x]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(200):
+                out = H.absmean_norm_q_nvfp4(x[i], 8.0)
+            torch.cuda.current_stream().synchronize()
+            if not all(torch.equal(a[: 64 * 32], b[: 64 * 32]) for a, b in zip(out, ref[i])):
+                bad.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad
