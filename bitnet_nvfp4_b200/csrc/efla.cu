@@ -693,6 +693,9 @@ constexpr int kCkQKStride = 72;  // floats per row of the raw q / k tiles: 16-by
 constexpr int kCkVStride = 68;   // floats per row of the raw v tile: the accumulator-shaped reads are conflict-free
 constexpr int kCkHStride = 72;   // halves per row of the prepared operands (-K, Q^, a K): conflict-free ldmatrix rows
 constexpr int kCkTStride = 24;   // halves per row of T and P
+// the same tiles when q, k, v arrive as halves: strides in halves (160-byte q / k rows, 144-byte v rows)
+constexpr int kCkQKStrideH = 80;
+constexpr int kCkVStrideH = 72;
 constexpr int kCkYStrideH = 72;  // halves per row of the output staging tile (in the -K / Q^ region, dead once their fragments are loaded)
 constexpr int kCkRawQ = 0;
 constexpr int kCkRawK = kCkRawQ + kChunk * kCkQKStride * 4;
@@ -725,7 +728,7 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t saddr, uint32_t r0, u
     asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
 }
 
-template <bool OUT16>
+template <bool IN16, bool OUT16>
 __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const EflaParams p) {
     pdl_wait();
     constexpr int HD = 64;
@@ -764,24 +767,45 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const
             for (int i = 0; i < 4; ++i) Sh[mt][ks][i] = 0u;
 
     const size_t row0 = static_cast<size_t>(seq) * p.T;
+    // element type of q, k, v: fp32 or (IN16) halves; ld_qkv counts elements of that type
     const float* qb = static_cast<const float*>(p.q) + row0 * p.ld_qkv + h * HD;
     const float* kb = static_cast<const float*>(p.k) + row0 * p.ld_qkv + h * HD;
     const float* vb = static_cast<const float*>(p.v) + row0 * p.ld_qkv + h * HD;
+    const __half* qbh = static_cast<const __half*>(p.q) + row0 * p.ld_qkv + h * HD;
+    const __half* kbh = static_cast<const __half*>(p.k) + row0 * p.ld_qkv + h * HD;
+    const __half* vbh = static_cast<const __half*>(p.v) + row0 * p.ld_qkv + h * HD;
     const float* bb = p.beta_raw + row0 * p.ld_beta;
     float* ob = static_cast<float*>(p.out) + row0 * p.ld_out + h * HD;
     __half* obh = static_cast<__half*>(p.out) + row0 * p.ld_out + h * HD;
+    __half* rawqh = reinterpret_cast<__half*>(rawq);
+    __half* rawkh = reinterpret_cast<__half*>(rawk);
+    __half* rawvh = reinterpret_cast<__half*>(rawv);
 
     // asynchronous copy of one chunk's q, k, v, beta rows into the raw tiles (16-byte pieces)
     auto issue_chunk = [&](int t0) {
-        const int piece = lane & 15, rsel = lane >> 4;
+        if constexpr (IN16) {  // 8 pieces per 128-byte row: lane = piece within a group of four rows
+            const int piece = lane & 7, rsel = lane >> 3;
 #pragma unroll
-        for (int j = 0; j < kChunk / 2; ++j) {
-            const int r = 2 * j + rsel;
-            if (t0 + r < p.T) {
-                const size_t o = static_cast<size_t>(t0 + r) * p.ld_qkv + 4 * piece;
-                cp_async16(rawq + r * kCkQKStride + 4 * piece, qb + o);
-                cp_async16(rawk + r * kCkQKStride + 4 * piece, kb + o);
-                cp_async16(rawv + r * kCkVStride + 4 * piece, vb + o);
+            for (int j = 0; j < kChunk / 4; ++j) {
+                const int r = 4 * j + rsel;
+                if (t0 + r < p.T) {
+                    const size_t o = static_cast<size_t>(t0 + r) * p.ld_qkv + 8 * piece;
+                    cp_async16(rawqh + r * kCkQKStrideH + 8 * piece, qbh + o);
+                    cp_async16(rawkh + r * kCkQKStrideH + 8 * piece, kbh + o);
+                    cp_async16(rawvh + r * kCkVStrideH + 8 * piece, vbh + o);
+                }
+            }
+        } else {  // 16 pieces per 256-byte row: lane = piece within a pair of rows
+            const int piece = lane & 15, rsel = lane >> 4;
+#pragma unroll
+            for (int j = 0; j < kChunk / 2; ++j) {
+                const int r = 2 * j + rsel;
+                if (t0 + r < p.T) {
+                    const size_t o = static_cast<size_t>(t0 + r) * p.ld_qkv + 4 * piece;
+                    cp_async16(rawq + r * kCkQKStride + 4 * piece, qb + o);
+                    cp_async16(rawk + r * kCkQKStride + 4 * piece, kb + o);
+                    cp_async16(rawv + r * kCkVStride + 4 * piece, vb + o);
+                }
             }
         }
         if (lane < kChunk && t0 + lane < p.T) cp_async4(beta_sh + lane, bb + static_cast<size_t>(t0 + lane) * p.ld_beta);
@@ -801,8 +825,10 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const
     const uint32_t ak_addr = static_cast<uint32_t>(__cvta_generic_to_shared(ak_sh)) +
                              static_cast<uint32_t>(((lm_j & 1) * 8 + lm_r) * kCkHStride + (lm_j >> 1) * 8) * 2u;
 
-    // Y written through transposing matrix stores: matrix j = lane / 8 covers tokens 8 (j >> 1) .. + 7 and
+    // V read and Y written through transposing matrix loads / stores: matrix j = lane / 8 covers tokens 8 (j >> 1) .. + 7 and
     // columns 16 mt + 8 (j & 1) .. + 7; a thread's register pair is (column g, tokens 2 tq and 2 tq + 1): the accumulator layout
+    const uint32_t v_addr = static_cast<uint32_t>(__cvta_generic_to_shared(rawvh)) +
+                            static_cast<uint32_t>(((lm_j >> 1) * 8 + lm_r) * kCkVStrideH + (lm_j & 1) * 8) * 2u;
     const uint32_t y_addr = static_cast<uint32_t>(__cvta_generic_to_shared(y_sh)) +
                             static_cast<uint32_t>(((lm_j >> 1) * 8 + lm_r) * kCkYStrideH + (lm_j & 1) * 8) * 2u;
     issue_chunk(0);
@@ -813,14 +839,30 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const
         {
             const int tt = lane >> 1, hh = lane & 1;
             const bool valid = t0 + tt < p.T;
-            // the lane's 32 elements of q and of k: 16-byte pieces 2 j + hh
+            // the lane's 32 elements of q and of k: 16-byte pieces 2 j + hh (four fp32, or eight halves: elements
+            // 8 (2 j + hh) .. + 7); element e of the register array is column kcol(e)
             float qv[32], kv[32];
+            if constexpr (IN16) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float4 a = *reinterpret_cast<const float4*>(rawq + tt * kCkQKStride + (2 * j + hh) * 4);
-                const float4 b = *reinterpret_cast<const float4*>(rawk + tt * kCkQKStride + (2 * j + hh) * 4);
-                qv[4 * j] = valid ? a.x : 0.0f; qv[4 * j + 1] = valid ? a.y : 0.0f; qv[4 * j + 2] = valid ? a.z : 0.0f; qv[4 * j + 3] = valid ? a.w : 0.0f;
-                kv[4 * j] = valid ? b.x : 0.0f; kv[4 * j + 1] = valid ? b.y : 0.0f; kv[4 * j + 2] = valid ? b.z : 0.0f; kv[4 * j + 3] = valid ? b.w : 0.0f;
+                for (int j = 0; j < 4; ++j) {
+                    const uint4 a = *reinterpret_cast<const uint4*>(rawqh + tt * kCkQKStrideH + (2 * j + hh) * 8);
+                    const uint4 b = *reinterpret_cast<const uint4*>(rawkh + tt * kCkQKStrideH + (2 * j + hh) * 8);
+                    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&aw[e])), fb = __half22float2(*reinterpret_cast<const __half2*>(&bw[e]));
+                        qv[8 * j + 2 * e] = valid ? fa.x : 0.0f; qv[8 * j + 2 * e + 1] = valid ? fa.y : 0.0f;
+                        kv[8 * j + 2 * e] = valid ? fb.x : 0.0f; kv[8 * j + 2 * e + 1] = valid ? fb.y : 0.0f;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float4 a = *reinterpret_cast<const float4*>(rawq + tt * kCkQKStride + (2 * j + hh) * 4);
+                    const float4 b = *reinterpret_cast<const float4*>(rawk + tt * kCkQKStride + (2 * j + hh) * 4);
+                    qv[4 * j] = valid ? a.x : 0.0f; qv[4 * j + 1] = valid ? a.y : 0.0f; qv[4 * j + 2] = valid ? a.z : 0.0f; qv[4 * j + 3] = valid ? a.w : 0.0f;
+                    kv[4 * j] = valid ? b.x : 0.0f; kv[4 * j + 1] = valid ? b.y : 0.0f; kv[4 * j + 2] = valid ? b.z : 0.0f; kv[4 * j + 3] = valid ? b.w : 0.0f;
+                }
             }
             float qss = 0.0f, kss = 0.0f;
 #pragma unroll
@@ -838,7 +880,8 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const
             const float nks = -kscale, aks = alpha * kscale;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const int c0 = (2 * j + hh) * 4;  // columns of elements 4 j .. 4 j + 3
+                // register elements 4 j .. 4 j + 3 are four consecutive columns starting at c0
+                const int c0 = IN16 ? (2 * (j >> 1) + hh) * 8 + 4 * (j & 1) : (2 * j + hh) * 4;
                 const int o = tt * kCkHStride + c0;
                 uint2 wq, wk, wa;
                 wq.x = pack_half2(qv[4 * j] * q_inv, qv[4 * j + 1] * q_inv); wq.y = pack_half2(qv[4 * j + 2] * q_inv, qv[4 * j + 3] * q_inv);
@@ -851,18 +894,35 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const
         }
         // ---------------- W^T starts as V^T: element (n, token) of this lane's accumulator positions ----------------
         float Wc[4][2][4];
+        if constexpr (IN16) {
+            // rows past the end of the sequence may hold stale halves: their columns of W are never used (alpha = 0 masks
+            // them out of L and P, and their outputs are not written), but they must be finite
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
+            for (int mt = 0; mt < 4; ++mt) {
+                uint32_t vf[4];
+                ldmatrix_x4_trans(vf, v_addr + mt * 32);
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int tok = 8 * nt + 2 * tq + e;
-                const bool valid = t0 + tok < p.T;
-#pragma unroll
-                for (int mt = 0; mt < 4; ++mt) {
-                    Wc[mt][nt][e] = valid ? rawv[tok * kCkVStride + 16 * mt + g] : 0.0f;
-                    Wc[mt][nt][2 + e] = valid ? rawv[tok * kCkVStride + 16 * mt + 8 + g] : 0.0f;
+                for (int nt = 0; nt < 2; ++nt) {
+                    const bool valid0 = t0 + 8 * nt + 2 * tq < p.T, valid1 = t0 + 8 * nt + 2 * tq + 1 < p.T;
+                    const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&vf[2 * nt])), hi = __half22float2(*reinterpret_cast<const __half2*>(&vf[2 * nt + 1]));
+                    Wc[mt][nt][0] = valid0 ? lo.x : 0.0f; Wc[mt][nt][1] = valid1 ? lo.y : 0.0f;
+                    Wc[mt][nt][2] = valid0 ? hi.x : 0.0f; Wc[mt][nt][3] = valid1 ? hi.y : 0.0f;
                 }
             }
+        } else {
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int tok = 8 * nt + 2 * tq + e;
+                    const bool valid = t0 + tok < p.T;
+#pragma unroll
+                    for (int mt = 0; mt < 4; ++mt) {
+                        Wc[mt][nt][e] = valid ? rawv[tok * kCkVStride + 16 * mt + g] : 0.0f;
+                        Wc[mt][nt][2 + e] = valid ? rawv[tok * kCkVStride + 16 * mt + 8 + g] : 0.0f;
+                    }
+                }
+        }
         __syncwarp();  // the raw tiles are free, the prepared operands are visible
         issue_chunk(t0 + kChunk);
 
@@ -1001,16 +1061,12 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const
 
 
 // ------------------------------------------------------------------------------------------------
-// The chunked scan for the case the batched driver runs: q | k | v as halves. The chunk's recurrence (here for EFLA, k unscaled) is
-// rewritten so that every tensor-core operand is a tile as it arrived from global memory:
+// The chunked scan for the case the batched driver runs: method 1 (k is used unscaled), q | k | v as halves. The chunk's
+// recurrence is rewritten so that every tensor-core operand is a tile as it arrived from global memory:
 //   with  U~_t = a_t U_t  (U the per-token updates, a_t = alpha_t):
 //       (I + diag(a) G_strict) U~ = diag(a) W,     W = V - K S0,  G = K K^T
 //       Y = diag(q_inv) (Q S0 + (Q K^T, lower triangle incl. diagonal) U~),        S += K^T U~
-// DeltaNet (DELTA) scales k_t by c_t = 1 / sqrt(lambda_t + eps): with U~_t = beta_t c_t U_t the same equations hold for raw k, a_t = beta_t c_t^2
-// and diag(a) W = diag(beta c) V - diag(a) K S0. U~ saturates at the largest half where |k| is next to zero (its product with k is what counts), and
-// P is taken of the normalised query, so that no product of two large rows meets the range of fp16. 100 us -> 45 us on 37 pairs x 12
-// sequences x 5 heads x 100 tokens against the kernel that prepares scaled operands, which fp32 inputs still take.
-// So K and Q enter the MMAs unscaled (ldmatrix straight from the raw tiles), alpha scales rows of G and columns of W^T, and the
+// so K and Q enter the MMAs unscaled (ldmatrix straight from the raw tiles), alpha scales rows of G and columns of W^T, and the
 // query normalisation scales the finished output. No prepared operand tiles are written: the preparation phase only
 // computes the per-token scalars.
 //
@@ -1031,8 +1087,7 @@ constexpr int kM1Y = kM1RawV + 2 * kM1Tile;                     // output stagin
 constexpr int kM1Beta = kM1Y + 2 * kChunk * kM1YStride * 2;     // two buffers
 constexpr int kM1Alpha = kM1Beta + 2 * kChunk * 4;
 constexpr int kM1Qinv = kM1Alpha + kChunk * 4;
-constexpr int kM1Cv = kM1Qinv + kChunk * 4;   // DeltaNet: factors of V
-constexpr int kM1L = kM1Cv + kChunk * 4;
+constexpr int kM1L = kM1Qinv + kChunk * 4;
 constexpr int kM1T = kM1L + kChunk * kChunk * 4;
 constexpr int kM1P = kM1T + kChunk * kCkTStride * 2;
 constexpr int kM1UnitBytes = kM1P + kChunk * kCkTStride * 2;
@@ -1041,7 +1096,7 @@ constexpr int kM1CtasPerSm = 4;
 constexpr int kM1SmemBytes = kM1Units * kM1UnitBytes;
 static_assert(kM1UnitBytes % 16 == 0 && kM1L % 16 == 0 && kM1T % 16 == 0 && kM1Beta % 16 == 0 && kM1Y % 16 == 0, "16-byte aligned shared-memory regions");
 
-template <bool OUT16, bool DELTA>
+template <bool OUT16>
 __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m1_kernel(const EflaParams p) {
     pdl_wait();
     constexpr int HD = 64;
@@ -1061,7 +1116,6 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
     float* beta_sh = reinterpret_cast<float*>(wsm + kM1Beta);
     float* alpha_sh = reinterpret_cast<float*>(wsm + kM1Alpha);
     float* qinv_sh = reinterpret_cast<float*>(wsm + kM1Qinv);
-    float* cv_sh = reinterpret_cast<float*>(wsm + kM1Cv);
     float* L_sh = reinterpret_cast<float*>(wsm + kM1L);
     __half* t_sh = reinterpret_cast<__half*>(wsm + kM1T);
     __half* p_sh = reinterpret_cast<__half*>(wsm + kM1P);
@@ -1155,7 +1209,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
         uint32_t kf[4][4];  // per 16-wide d block: B fragments {b0, b1} for tokens 0-7 (regs 0, 1) and 8-15 (regs 2, 3)
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) ldmatrix_x4(kf[ks], k_addr0 + bufo + ks * 32);
-        float Wc[2][2][4];  // -(V - K S0)^T = S0^T K^T - V^T (DELTA: S0^T K^T alone)
+        float Wc[2][2][4];  // -(V - K S0)^T = S0^T K^T - V^T
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) {
             uint32_t vf[4];
@@ -1163,8 +1217,8 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
                 const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&vf[2 * nt])), hi = __half22float2(*reinterpret_cast<const __half2*>(&vf[2 * nt + 1]));
-                Wc[mt][nt][0] = DELTA ? 0.0f : -lo.x; Wc[mt][nt][1] = DELTA ? 0.0f : -lo.y;
-                Wc[mt][nt][2] = DELTA ? 0.0f : -hi.x; Wc[mt][nt][3] = DELTA ? 0.0f : -hi.y;
+                Wc[mt][nt][0] = -lo.x; Wc[mt][nt][1] = -lo.y;
+                Wc[mt][nt][2] = -hi.x; Wc[mt][nt][3] = -hi.y;
             }
         }
 #pragma unroll
@@ -1206,13 +1260,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
                     // sigmoid and the final quotient with the fast exponential / division (about 2 ulp each: far below the fp16
                     // rounding of every operand alpha touches); expm1f keeps its accuracy for small beta * lambda
                     const float beta = __fdividef(1.0f, 1.0f + __expf(-(braw + beta_bias)));
-                    if constexpr (DELTA) {
-                        const float c = rsqrtf(lambda + p.eps), bc = valid ? beta * c : 0.0f;
-                        alpha_sh[my_tok] = bc * c;
-                        cv_sh[my_tok] = bc;
-                    } else {
-                        alpha_sh[my_tok] = valid ? __fdividef(-expm1f(-(beta * lambda)), lambda + p.eps) : 0.0f;
-                    }
+                    alpha_sh[my_tok] = valid ? __fdividef(-expm1f(-(beta * lambda)), lambda + p.eps) : 0.0f;
                 }
             }
             __syncwarp();
@@ -1271,18 +1319,9 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
                 }
             const float qss = diagonal(Qc);
             if (diag_lane || helper_lane) qinv_sh[my_tok] = rsqrtf(qss + p.eps);
-            // P[t][s] = q_t . k_s (s <= t) in fp16 (DELTA: of the normalised query)
-            float q_lo = 1.0f, q_hi = 1.0f;
-            if constexpr (DELTA) {
-                __syncwarp();
-                q_lo = qinv_sh[g]; q_hi = qinv_sh[g + 8];
-            }
+            // P[t][s] = q_t . k_s (s <= t) in fp16
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                if constexpr (DELTA) {
-                    Xc[nt][0] *= q_lo; Xc[nt][1] *= q_lo;
-                    Xc[nt][2] *= q_hi; Xc[nt][3] *= q_hi;
-                }
                 const int s0 = 8 * nt + 2 * tq;
 #pragma unroll
                 for (int hr = 0; hr < 2; ++hr) {
@@ -1313,21 +1352,8 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
         for (int mt = 0; mt < 2; ++mt) {
             // packed fp32 pairs (tokens 2 tq and 2 tq + 1): each half rounds like the scalar multiply
             const float2 na0 = make_float2(na[0][0], na[0][1]), na1 = make_float2(na[1][0], na[1][1]);
-            float2 x0, x1, x2, x3;
-            if constexpr (DELTA) {
-                auto sat = [](float2 x) { return make_float2(fminf(fmaxf(x.x, -65504.0f), 65504.0f), fminf(fmaxf(x.y, -65504.0f), 65504.0f)); };
-                uint32_t vf[4];  // read again: cheaper than keeping it
-                ldmatrix_x4_trans(vf, v_addr0 + bufo + mt * 32);
-                auto v2 = [&](int i) { return __half22float2(*reinterpret_cast<const __half2*>(&vf[i])); };
-                const float2 cv0 = *reinterpret_cast<const float2*>(cv_sh + 2 * tq), cv1 = *reinterpret_cast<const float2*>(cv_sh + 8 + 2 * tq);
-                x0 = sat(__ffma2_rn(na0, make_float2(Wc[mt][0][0], Wc[mt][0][1]), __fmul2_rn(cv0, v2(0))));
-                x1 = sat(__ffma2_rn(na0, make_float2(Wc[mt][0][2], Wc[mt][0][3]), __fmul2_rn(cv0, v2(1))));
-                x2 = sat(__ffma2_rn(na1, make_float2(Wc[mt][1][0], Wc[mt][1][1]), __fmul2_rn(cv1, v2(2))));
-                x3 = sat(__ffma2_rn(na1, make_float2(Wc[mt][1][2], Wc[mt][1][3]), __fmul2_rn(cv1, v2(3))));
-            } else {
-                x0 = __fmul2_rn(na0, make_float2(Wc[mt][0][0], Wc[mt][0][1])); x1 = __fmul2_rn(na0, make_float2(Wc[mt][0][2], Wc[mt][0][3]));
-                x2 = __fmul2_rn(na1, make_float2(Wc[mt][1][0], Wc[mt][1][1])); x3 = __fmul2_rn(na1, make_float2(Wc[mt][1][2], Wc[mt][1][3]));
-            }
+            const float2 x0 = __fmul2_rn(na0, make_float2(Wc[mt][0][0], Wc[mt][0][1])), x1 = __fmul2_rn(na0, make_float2(Wc[mt][0][2], Wc[mt][0][3]));
+            const float2 x2 = __fmul2_rn(na1, make_float2(Wc[mt][1][0], Wc[mt][1][1])), x3 = __fmul2_rn(na1, make_float2(Wc[mt][1][2], Wc[mt][1][3]));
             const uint32_t w0 = pack_half2(x0.x, x0.y), w1 = pack_half2(x1.x, x1.y), w2 = pack_half2(x2.x, x2.y), w3 = pack_half2(x3.x, x3.y);
             float Uc[2][4];
 #pragma unroll
@@ -1339,28 +1365,19 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) {
             float Yc[2][4];
-            auto scale_by_qinv = [&] {
 #pragma unroll
-                for (int nt = 0; nt < 2; ++nt) {
-                    const float2 q2 = make_float2(qi[nt][0], qi[nt][1]);
-                    const float2 lo = __fmul2_rn(q2, make_float2(Yc[nt][0], Yc[nt][1])), hi = __fmul2_rn(q2, make_float2(Yc[nt][2], Yc[nt][3]));
-                    Yc[nt][0] = lo.x; Yc[nt][1] = lo.y; Yc[nt][2] = hi.x; Yc[nt][3] = hi.y;
-                }
-            };
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                if constexpr (DELTA) Yc[nt][0] = Yc[nt][1] = Yc[nt][2] = Yc[nt][3] = 0.0f;
-                else mma_f16_16816_zero(Yc[nt], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], pf[2 * nt], pf[2 * nt + 1]);
-            }
+            for (int nt = 0; nt < 2; ++nt) mma_f16_16816_zero(Yc[nt], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], pf[2 * nt], pf[2 * nt + 1]);
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt)
                     mma_f16_16816(Yc[nt], Sh[mt][ks][0], Sh[mt][ks][1], Sh[mt][ks][2], Sh[mt][ks][3], qf[ks][2 * nt], qf[ks][2 * nt + 1]);
-            scale_by_qinv();
-            if constexpr (DELTA)
 #pragma unroll
-                for (int nt = 0; nt < 2; ++nt) mma_f16_16816(Yc[nt], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], pf[2 * nt], pf[2 * nt + 1]);
+            for (int nt = 0; nt < 2; ++nt) {
+                const float2 q2 = make_float2(qi[nt][0], qi[nt][1]);
+                const float2 lo = __fmul2_rn(q2, make_float2(Yc[nt][0], Yc[nt][1])), hi = __fmul2_rn(q2, make_float2(Yc[nt][2], Yc[nt][3]));
+                Yc[nt][0] = lo.x; Yc[nt][1] = lo.y; Yc[nt][2] = hi.x; Yc[nt][3] = hi.y;
+            }
             if constexpr (OUT16) {
                 stmatrix_x4_trans(y_addr + mt * 32, pack_half2(Yc[0][0], Yc[0][1]), pack_half2(Yc[0][2], Yc[0][3]), pack_half2(Yc[1][0], Yc[1][1]),
                                   pack_half2(Yc[1][2], Yc[1][3]));
@@ -1437,12 +1454,12 @@ int efla_launch(const EflaParams& p, cudaStream_t stream) {
         if (dev < 0 || dev >= 64 || !configured[dev]) {
             rc = check_cuda(cudaFuncSetAttribute(efla_scan64_mma2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kScan2SmemBytes), "cudaFuncSetAttribute(efla_scan64_mma2_kernel)");
             if (rc) return rc;
-            rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCkSmemBytes), "cudaFuncSetAttribute(efla_chunk16_kernel)");
-            if (!rc) rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCkSmemBytes), "cudaFuncSetAttribute(efla_chunk16_kernel)");
-            if (!rc) rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_m1_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kM1SmemBytes), "cudaFuncSetAttribute(efla_chunk16_m1_kernel)");
-            if (!rc) rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_m1_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kM1SmemBytes), "cudaFuncSetAttribute(efla_chunk16_m1_kernel)");
-            if (!rc) rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_m1_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kM1SmemBytes), "cudaFuncSetAttribute(efla_chunk16_m1_kernel)");
-            if (!rc) rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_m1_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kM1SmemBytes), "cudaFuncSetAttribute(efla_chunk16_m1_kernel)");
+            rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCkSmemBytes), "cudaFuncSetAttribute(efla_chunk16_kernel)");
+            if (!rc) rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCkSmemBytes), "cudaFuncSetAttribute(efla_chunk16_kernel)");
+            if (!rc) rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCkSmemBytes), "cudaFuncSetAttribute(efla_chunk16_kernel)");
+            if (!rc) rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCkSmemBytes), "cudaFuncSetAttribute(efla_chunk16_kernel)");
+            if (!rc) rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_m1_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kM1SmemBytes), "cudaFuncSetAttribute(efla_chunk16_m1_kernel)");
+            if (!rc) rc = check_cuda(cudaFuncSetAttribute(efla_chunk16_m1_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kM1SmemBytes), "cudaFuncSetAttribute(efla_chunk16_m1_kernel)");
             if (rc) return rc;
             if (dev >= 0 && dev < 64) configured[dev] = true;
         }
@@ -1450,16 +1467,16 @@ int efla_launch(const EflaParams& p, cudaStream_t stream) {
             if (p.qkv_f16 && ((p.ld_qkv % 8) != 0)) return set_error(BNF4_ERR_INVALID, "efla: fp16 q, k, v need ld_qkv %% 8 == 0");
             if (p.out_f16 && (((p.ld_out % 8) != 0) || (reinterpret_cast<uintptr_t>(p.out) & 15))) return set_error(BNF4_ERR_INVALID, "efla: fp16 output needs 16-byte aligned rows");
             const unsigned grid = static_cast<unsigned>(ctas);
-            if (p.qkv_f16) {  // the batched driver's case: raw-operand kernel, persistent pairs of warps
+            if (p.qkv_f16 && p.method == 1) {  // the batched driver's case: raw-operand kernel, persistent pairs of warps
                 const int sms = multiprocessors(dev);
                 if (sms <= 0) return BNF4_ERR_CUDA;
                 const unsigned pgrid = static_cast<unsigned>(std::min<long long>((units + kM1Units - 1) / kM1Units, kM1CtasPerSm * static_cast<long long>(sms)));
-                auto run = [&](auto kernel) { launch_pdl_if(early, kernel, pgrid, kChunkWarps * 32, kM1SmemBytes, stream, p); };
-                if (p.method == 0) p.out_f16 ? run(efla_chunk16_m1_kernel<true, true>) : run(efla_chunk16_m1_kernel<false, true>);
-                else p.out_f16 ? run(efla_chunk16_m1_kernel<true, false>) : run(efla_chunk16_m1_kernel<false, false>);
-            }
-            else if (p.out_f16) launch_pdl_if(early, efla_chunk16_kernel<true>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
-            else launch_pdl_if(early, efla_chunk16_kernel<false>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
+                if (p.out_f16) launch_pdl_if(early, efla_chunk16_m1_kernel<true>, pgrid, kChunkWarps * 32, kM1SmemBytes, stream, p);
+                else launch_pdl_if(early, efla_chunk16_m1_kernel<false>, pgrid, kChunkWarps * 32, kM1SmemBytes, stream, p);
+            } else if (p.qkv_f16 && p.out_f16) launch_pdl_if(early, efla_chunk16_kernel<true, true>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
+            else if (p.qkv_f16) launch_pdl_if(early, efla_chunk16_kernel<true, false>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
+            else if (p.out_f16) launch_pdl_if(early, efla_chunk16_kernel<false, true>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
+            else launch_pdl_if(early, efla_chunk16_kernel<false, false>, grid, kChunkWarps * 32, kCkSmemBytes, stream, p);
             return check_launch("efla_chunk16_kernel");
         }
         if (p.qkv_f16 || p.out_f16) return set_error(BNF4_ERR_INVALID, "efla: fp16 q, k, v or output are supported by the chunked kernel only");

@@ -123,26 +123,3 @@ def test_generic_kernel_carries_the_state(H, hidden, fp16, offset):
     parts = np.concatenate([call(qkv[:, :T1], two, T1), call(qkv[:, T1:], two, T2)], axis=1)
     assert np.array_equal(whole, parts)
     assert torch.equal(one, two)
-
-
-@pytest.mark.parametrize("k_scale,q_scale", [(0.4, 0.4), (60.0, 60.0), (0.01, 3.0)])   # 60: q . k beyond the range of fp16; 0.01: 1 / |k| = 12
-@pytest.mark.parametrize("out16", [0, 1])
-@pytest.mark.parametrize("heads,seqs,T", [(5, 12, 100), (1, 1, 1), (2, 5, 17), (8, 160, 16)])   # one unit, a partial chunk, more units than one pass holds
-def test_deltanet_chunked_scan_on_halves(H, heads, seqs, T, out16, k_scale, q_scale):
-    """Method 0 with q | k | v as halves, against the recurrence in float64: half operands and a half state per 16 tokens, the bound
-    of the other fp16-state kernels."""
-    import torch
-    rng = np.random.default_rng(heads * 100 + T)
-    hidden = 64 * heads
-    qkv = make_qkv(rng, seqs * T, hidden, 3 * hidden + 1, 1.0)
-    qkv[:, :hidden] *= q_scale
-    qkv[:, hidden:2 * hidden] *= k_scale
-    qkv[:, :3 * hidden] = qkv[:, :3 * hidden].astype(np.float16).astype(np.float32)
-    bb = (rng.standard_normal(seqs) * 0.2 - 2.0).astype(np.float32)
-    q16 = dev(qkv[:, :3 * hidden].astype(np.float16))
-    out = torch.full((seqs * T, hidden), float("nan"), dtype=torch.float16 if out16 else torch.float32, device="cuda")
-    H.efla_scan(state=None, state_fp16=1, q=q16, k=q16[:, hidden:], v=q16[:, 2 * hidden:], beta_raw=dev(qkv[:, 3 * hidden]), ld_qkv=3 * hidden,
-                ld_beta=1, beta_bias_seq=dev(bb), seqs_per_bias=1, hidden=hidden, heads=heads, seqs=seqs, T=T, method=0, eps=1e-6, out=out,
-                ld_out=hidden, variant=3, qkv_f16=1, out_f16=out16)
-    ref = exact_scan(qkv.reshape(seqs, T, 3 * hidden + 1), bb, hidden, heads, 0)
-    assert np.abs(out.float().cpu().numpy().reshape(seqs, T, hidden) - ref).max() <= (SCAN_TOL + (2 ** -11 if out16 else 0)) * np.abs(ref).max()
