@@ -22,9 +22,12 @@
 //   5. y = P~ V over 64-column tiles of V.
 // What bounds it: the MMAs of steps 2 and 5 (about 40 k tensor cycles per sequence at T = 128, hd = 512; the legacy mma.sync path, since
 // the triangular solve between the contractions needs its operands in registers). 1024 sequences of 128 tokens, one head of 512:
-// 0.58 ms, against 75 ms for the per-token kernel (whose state passes through shared memory twice per token).
+// 0.57 ms, against 75 ms for the per-token kernel (whose state passes through shared memory twice per token). Of 150 k cycles per unit, step 1
+// takes 31 k (DRAM), step 2 63 k, steps 3 and 4 8 k, step 5 47 k. MMAs and the conversions around them add up rather than overlap: staggering them
+// between warps, more independent MMA chains and L2 prefetches of V and of the next unit changed nothing.
 
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -46,7 +49,9 @@ constexpr int kSqDiag = 2 * kSqStage;                            // fp32 diagona
 constexpr int kSqInv = kSqDiag + 8 * 16 * 17 * 4;                // their inverses, hi and mid [2][8][16][kSqTStride]
 constexpr int kSqScal = kSqInv + 2 * 8 * 16 * kSqTStride * 2;    // q scale, k scale, a, b [4][128] floats
 constexpr int kSqRed = kSqScal + 4 * kSeqMaxT * 4;               // reduction scratch [2][16] + broadcast
-constexpr int kSqSmem = kSqRed + 256;
+constexpr int kSqPart = kSqRed + 256;                            // a CTA's share of the squared norms [2][128] floats (read by its cluster)
+constexpr int kSqSmem = kSqPart + 2 * kSeqMaxT * 4;
+static_assert(48 * kSeqThreads * 4 <= 2 * kSqStage, "the exchanged accumulators fit the stages");
 static_assert(2 * kSeqMaxT * kSqLStride * 2 <= kSqStage && kSeqMaxT * kSqXStride * 4 <= kSqStage && 4 * kSqTile <= kSqStage, "overlaid regions");
 static_assert(kSqDiag % 16 == 0 && kSqInv % 16 == 0 && kSqScal % 16 == 0, "16-byte aligned regions");
 constexpr float kSqUp = 256.0f;                    // power-of-two scale of every normalised operand
@@ -77,12 +82,31 @@ __device__ __forceinline__ float sq_pow2_scale(float m) {
     return __uint_as_float(static_cast<uint32_t>(min(max(7 - e + 127, 1), 254)) << 23);
 }
 
+template <int CS>
+__device__ __forceinline__ void sq_cluster_sync() {
+    if constexpr (CS > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the float at this shared-memory address in CTA `rank` of the cluster
+__device__ __forceinline__ float sq_remote(uint32_t addr, int rank) {
+    uint32_t a;
+    float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// CS CTAs of a cluster share a unit: each takes its share of the 64-column blocks in steps 1, 2 (partial sums, exchanged through distributed
+// shared memory and added in rank order, so all hold the same bits) and 5; steps 3 and 4 are done by every one of them.
+template <int CS>
 __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaParams p) {
     pdl_wait();
     extern __shared__ __align__(16) uint8_t sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int T = p.T, hd = p.hidden / p.heads;
-    const unsigned unit = blockIdx.x;
+    const unsigned unit = blockIdx.x / CS;
+    const int rank = static_cast<int>(blockIdx.x % CS);
+    const int nd = (p.hidden / p.heads + 63) >> 6;
+    const int db0 = rank * nd / CS, db1 = (rank + 1) * nd / CS;  // this CTA's 64-column blocks
     const unsigned seq = unit / static_cast<unsigned>(p.heads);
     const int h = static_cast<int>(unit - seq * static_cast<unsigned>(p.heads));
     const int nb = (T + 15) >> 4;  // 16-token blocks
@@ -97,6 +121,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     float* a_sh = ks_sh + kSeqMaxT;
     float* b_sh = a_sh + kSeqMaxT;
     float* red = reinterpret_cast<float*>(sm + kSqRed);
+    float* part = reinterpret_cast<float*>(sm + kSqPart);
     const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
 
     // ---------------- 1. norms and scalars ----------------
@@ -105,7 +130,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         if (t < T) {
             const float4* q4 = reinterpret_cast<const float4*>(qg + static_cast<size_t>(t) * p.ld_qkv);
             const float4* k4 = reinterpret_cast<const float4*>(kg + static_cast<size_t>(t) * p.ld_qkv);
-            for (int i = lane; i < (hd >> 2); i += 32) {
+            for (int i = 16 * db0 + lane; i < min(hd >> 2, 16 * db1); i += 32) {
                 const float4 a = q4[i], b = k4[i];
                 qss = fmaf(a.x, a.x, qss); qss = fmaf(a.y, a.y, qss); qss = fmaf(a.z, a.z, qss); qss = fmaf(a.w, a.w, qss);
                 kss = fmaf(b.x, b.x, kss); kss = fmaf(b.y, b.y, kss); kss = fmaf(b.z, b.z, kss); kss = fmaf(b.w, b.w, kss);
@@ -113,12 +138,23 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         }
         qss = warp_sum_f(qss);
         kss = warp_sum_f(kss);
-        if (lane == 0) { qs_sh[t] = qss; ks_sh[t] = kss; }
+        if (lane == 0) { part[t] = qss; part[kSeqMaxT + t] = kss; }
     }
-    __syncthreads();
+    if constexpr (CS > 1) sq_cluster_sync<CS>();
+    else __syncthreads();
     if (tid < kSeqMaxT) {
         const int t = tid;
-        const float qss = qs_sh[t], kss = ks_sh[t];
+        float qss = 0.0f, kss = 0.0f;
+        if constexpr (CS > 1) {
+#pragma unroll
+            for (int r = 0; r < CS; ++r) {
+                qss += sq_remote(sm0 + kSqPart + t * 4, r);
+                kss += sq_remote(sm0 + kSqPart + (kSeqMaxT + t) * 4, r);
+            }
+        } else {
+            qss = part[t];
+            kss = part[kSeqMaxT + t];
+        }
         float a = 0.0f, b = 0.0f, kinv = 0.0f, qinv = 0.0f;
         if (t < T) {
             const float bias = efla_seq_bias(p, static_cast<unsigned>(seq));
@@ -193,13 +229,12 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     // ldmatrix addresses inside a stage: A rows (lane % 16, column half lane / 16); B: eight K rows, matrices (hi, k 0-7), (hi, 8-15), (mid, ..), (mid, ..)
     const uint32_t a_off = static_cast<uint32_t>((lane & 15) * kSqStride + (lane >> 4) * 8) * 2u + (which ? 2u * kSqTile : 0u);
     const uint32_t b_off = static_cast<uint32_t>((half * 8 + (lane & 7)) * kSqStride + ((lane >> 3) & 1) * 8) * 2u + (lane >> 4) * static_cast<uint32_t>(kSqTile);
-    const int nd = (hd + 63) >> 6;
-    load_block(0);
+    load_block(db0 * 64);
     store_block(0);
     __syncthreads();
-    for (int db = 0; db < nd; ++db) {
-        if (db + 1 < nd) load_block((db + 1) * 64);
-        const uint32_t st = sm0 + (db & 1) * kSqStage;
+    for (int db = db0; db < db1; ++db) {
+        if (db + 1 < db1) load_block((db + 1) * 64);
+        const uint32_t st = sm0 + ((db - db0) & 1) * kSqStage;
         const int nk = min(4, (hd - db * 64) >> 4);
         if (r1 <= r2) {
             for (int kk = 0; kk < nk; ++kk) {
@@ -224,8 +259,38 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
                 }
             }
         }
-        if (db + 1 < nd) store_block((db + 1) & 1);
+        if (db + 1 < db1) store_block((db + 1 - db0) & 1);
         __syncthreads();
+    }
+    if constexpr (CS > 1) {  // the partial sums of all CTAs, thread by thread
+        float* ex = reinterpret_cast<float*>(sm) + tid;
+        const uint32_t exa = sm0 + tid * 4;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (j <= r2) ex[(j * 4 + i) * kSeqThreads] = acc2[j][i];
+                if (j < 4 && j <= r1) ex[(32 + (j & 3) * 4 + i) * kSeqThreads] = acc1[j & 3][i];
+            }
+        sq_cluster_sync<CS>();
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (j <= r2) {
+                    float x = 0.0f;
+#pragma unroll
+                    for (int r = 0; r < CS; ++r) x += sq_remote(exa + (j * 4 + i) * (kSeqThreads * 4), r);
+                    acc2[j][i] = x;
+                }
+                if (j < 4 && j <= r1) {
+                    float x = 0.0f;
+#pragma unroll
+                    for (int r = 0; r < CS; ++r) x += sq_remote(exa + (32 + (j & 3) * 4 + i) * (kSeqThreads * 4), r);
+                    acc1[j & 3][i] = x;
+                }
+            }
+        sq_cluster_sync<CS>();  // everyone has read: the stages are free again (and nobody's shared memory is read from here on)
     }
 
     // ---------------- 3. L (two halves, stage 0), its diagonal blocks (fp32), X (fp32, stage 1) ----------------
@@ -392,8 +457,8 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
             vr[i] = (t < T && c < hd) ? *reinterpret_cast<const float4*>(vg + static_cast<size_t>(t) * p.ld_qkv + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     };
-    load_v(0);
-    for (int ct = 0; ct < nd; ++ct) {
+    load_v(db0 * 64);
+    for (int ct = db0; ct < db1; ++ct) {
         // the tile's own power-of-two scale keeps both halves of its values in range
         float m = 0.0f;
 #pragma unroll
@@ -417,7 +482,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
             *reinterpret_cast<uint2*>(st + o) = hi;
             *reinterpret_cast<uint2*>(st + kSqTile + o) = mid;
         }
-        if (ct + 1 < nd) load_v((ct + 1) * 64);
+        if (ct + 1 < db1) load_v((ct + 1) * 64);
         __syncthreads();
         if (r1 <= r2) {
             float y1[2][4], y2[2][4];
@@ -476,20 +541,67 @@ bool efla_seq_applies(const EflaParams& p) {
     const int hd = p.hidden / p.heads;
     return p.state == nullptr && p.state_fp16 != 0 && !p.qkv_f16 && !p.out_f16 && hd > 32 && hd % 32 == 0 && p.T <= kSeqMaxT &&
            ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0 && p.ld_qkv % 4 == 0 &&
-           (reinterpret_cast<uintptr_t>(p.out) & 7) == 0 && p.ld_out % 2 == 0 && p.seqs * static_cast<long long>(p.heads) <= 0x7fffffffLL;
+           (reinterpret_cast<uintptr_t>(p.out) & 7) == 0 && p.ld_out % 2 == 0 && p.seqs * static_cast<long long>(p.heads) <= 0x7fffffffLL / 4;
 }
 
+namespace {
+// Clusters of CS such CTAs that the device holds at once (a cluster stays inside one processing cluster of the chip: fewer than SMs / CS); 0 on error.
+template <int CS>
+int resident_clusters(int dev) {
+    static std::atomic<int> known[64] = {};
+    int n = dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (n > 0) return n;
+    if (check_cuda(cudaFuncSetAttribute(efla_seq_kernel<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSqSmem), "cudaFuncSetAttribute(efla_seq_kernel)")) return 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(CS);
+    cfg.blockDim = dim3(kSeqThreads);
+    cfg.dynamicSmemBytes = kSqSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (check_cuda(cudaOccupancyMaxActiveClusters(&n, efla_seq_kernel<CS>, &cfg), "cudaOccupancyMaxActiveClusters(efla_seq_kernel)")) return 0;
+    if (dev < 64 && n > 0) known[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
+}  // namespace
+
 int efla_seq_launch(const EflaParams& p, cudaStream_t stream) {
-    static bool configured[64] = {};  // function attributes are per device
     int dev = 0;
-    int rc = check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+    const int rc = current_device(&dev);
     if (rc) return rc;
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        rc = check_cuda(cudaFuncSetAttribute(efla_seq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSqSmem), "cudaFuncSetAttribute(efla_seq_kernel)");
-        if (rc) return rc;
-        if (dev >= 0 && dev < 64) configured[dev] = true;
+    const int one = resident_clusters<1>(dev), two = resident_clusters<2>(dev), four = resident_clusters<4>(dev);
+    if (one <= 0 || two <= 0 || four <= 0) return BNF4_ERR_CUDA;
+    const long long units = p.seqs * p.heads;
+    const int nd = (p.hidden / p.heads + 63) >> 6;
+    // Few units leave SMs idle: two or four CTAs share one as long as all units still run at once and every CTA has a block of columns. One head of
+    // 512, 32 sequences: 71 us with one, 48 with two, 40 with four; a second pass costs more than sharing gains (37 units: 73 us with four,
+    // 48 with two; 256 units: 161 / 204 / 329 us).
+    const int cs = units <= four && nd >= 4 ? 4 : units <= two && nd >= 2 ? 2 : 1;
+    const bool early = p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(units * cs));
+    cfg.blockDim = dim3(kSeqThreads);
+    cfg.dynamicSmemBytes = kSqSmem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (cs > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = static_cast<unsigned>(cs);
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
     }
-    launch_pdl_if(p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems, efla_seq_kernel, static_cast<unsigned>(p.seqs * p.heads), kSeqThreads, kSqSmem, stream, p);
+    if (early) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    cudaLaunchKernelEx(&cfg, cs == 4 ? efla_seq_kernel<4> : cs == 2 ? efla_seq_kernel<2> : efla_seq_kernel<1>, p);  // errors surface in check_launch
     return check_launch("efla_seq_kernel");
 }
 

@@ -72,7 +72,8 @@ def run(H, qkv, bb, per_bias, hidden, heads, seqs, T, method, variant, state=Non
 @pytest.mark.parametrize("scale", [0.3, 1000.0, 1e-3])   # 1000: k, q, v far outside fp16's comfortable range; 1e-3: lambda near eps
 @pytest.mark.parametrize("hidden,heads,seqs,T,method", [
     (512, 1, 3, 128, 1), (512, 1, 2, 100, 0), (256, 2, 3, 33, 1), (96, 1, 2, 17, 1), (320, 2, 2, 113, 0), (96, 1, 5, 1, 1), (256, 2, 2, 16, 1),
-    (512, 1, 2, 47, 1)])
+    (512, 1, 2, 47, 1),
+    (512, 1, 40, 33, 1), (192, 2, 30, 20, 0), (96, 1, 160, 18, 1), (320, 1, 150, 16, 1)])   # two CTAs per unit; one
 def test_closed_form_matches_the_exact_recurrence(H, hidden, heads, seqs, T, method, scale):
     rng = np.random.default_rng(hidden + T + method)
     fc = (3 * hidden + 1 + 31) & ~31
