@@ -90,12 +90,23 @@ at::Tensor empty_like_device(const at::Tensor& like, at::IntArrayRef sizes, at::
     if (like.is_cuda()) return at::detail::empty_cuda(sizes, dtype, like.device(), c10::nullopt);
     return at::empty(sizes, like.options().dtype(dtype));
 }
-struct Quantised {  // outputs of a quantiser (nothing is cleared: the library writes every value, code and scale byte, padding included)
+// Outputs of a quantiser: three tensors on one allocation, each from a 512-byte boundary (an allocation costs about as much as the rest of the
+// call's host work). Nothing is cleared: the library writes every value, code and scale byte, padding included.
+struct Quantised {
     at::Tensor q, codes, sf;
     Quantised(const at::Tensor& like, int64_t rows, int64_t cols, bool want_q) {
-        if (want_q) q = empty_like_device(like, {rows, cols}, at::kChar);
-        codes = empty_like_device(like, {(rows * cols * 4 + 7) / 8}, at::kByte);
-        sf = empty_like_device(like, {(rows + 127) / 128 * 128 * (((cols + 15) / 16 + 3) / 4 * 4)}, at::kByte);
+        const int64_t nq = want_q ? rows * cols : 0, nc = (rows * cols * 4 + 7) / 8, ns = (rows + 127) / 128 * 128 * (((cols + 15) / 16 + 3) / 4 * 4);
+        auto up = [](int64_t n) { return (n + 511) / 512 * 512; };
+        const at::Tensor base = empty_like_device(like, {up(nq) + up(nc) + ns}, at::kByte);
+        auto part = [&](int64_t offset, at::IntArrayRef sizes, at::ScalarType dtype) {
+            at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(base.storage()), base.key_set(), c10::scalarTypeToTypeMeta(dtype));
+            t.unsafeGetTensorImpl()->set_storage_offset(offset);  // elements of one byte
+            t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+            return t;
+        };
+        if (want_q) q = part(0, {rows, cols}, at::kChar);
+        codes = part(up(nq), {nc}, at::kByte);
+        sf = part(up(nq) + up(nc), {ns}, at::kByte);
     }
     template <typename T>
     T* values() { return static_cast<T*>(q.data_ptr()); }
