@@ -12,7 +12,7 @@
 //     the current one is processed. HBM traffic is the algorithmic minimum: read q,k,v,beta, write y.
 //   * generic kernel, any head_dim: one CTA owns a column slice of one (sequence, head) in registers;
 //     also serves the reference's single-step entry points (state loaded from / stored to HBM).
-//   * short sequences of other head widths from a zero state: the closed form of efla_seq.cu.
+//   * sequences of other head widths from a zero state: the closed form of efla_seq.cu.
 // heads == 1 reproduces the reference; beta is one scalar per row, q-norm / lambda / alpha are per head.
 
 #include "common.cuh"
@@ -1484,7 +1484,7 @@ int efla_launch(const EflaParams& p, cudaStream_t stream) {
         return check_launch("efla_scan64_mma2_kernel");
     }
     if ((hd % 32) != 0) return set_error(BNF4_ERR_INVALID, "efla: head_dim=%d must be a multiple of 32", hd);
-    // AUTO with the chunked forms allowed: short sequences from a zero state take the closed form (efla_seq.cu)
+    // AUTO with the chunked forms allowed: sequences from a zero state take the closed form (efla_seq.cu)
     if (p.variant == BNF4_EFLA_AUTO && g_efla_chunked != 0 && efla_seq_applies(p)) return efla_seq_launch(p, stream);
     return p.state_fp16 ? launch_generic_for<__half>(p, stream) : launch_generic_for<float>(p, stream);
 }

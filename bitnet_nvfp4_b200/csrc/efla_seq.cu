@@ -1,4 +1,5 @@
-// EFLA / DeltaNet recurrence of a whole sequence of at most 128 tokens as dense contractions, for heads of any width.
+// EFLA / DeltaNet recurrence of a whole sequence as dense contractions, for heads of any width: up to 128 tokens in one block, longer ones in
+// blocks of 128 (efla_long_kernel).
 //
 // With a zero initial state the recurrence of efla.cu has a closed form that never builds the hd x hd state. Let
 // k_t = n_t k^_t (n_t = |k_t|), w_t = alpha_t n_t (v_t - n_t k^_t . S_{t-1}), so that S_t = S_{t-1} + k^_t w_t^T. Then
@@ -82,6 +83,115 @@ __device__ __forceinline__ float sq_pow2_scale(float m) {
     return __uint_as_float(static_cast<uint32_t>(min(max(7 - e + 127, 1), 254)) << 23);
 }
 
+// beta's logit and the squared norms of a token -> 1 / |q|, 1 / |k|, a and b
+__device__ __forceinline__ void seq_scalars(const EflaParams& p, float logit, float qss, float kss, float& qinv, float& kinv, float& a, float& b) {
+    const float beta = 1.0f / (1.0f + expf(-logit));
+    const float lambda = kss < p.eps ? p.eps : kss;
+    qinv = rsqrtf(qss + p.eps);
+    kinv = kss > 0.0f ? rsqrtf(kss) : 0.0f;
+    const float n = kss * kinv;
+    if (p.method == 0) {
+        const float ksc = rsqrtf(lambda + p.eps);
+        a = beta * (n * ksc) * (n * ksc);
+        b = beta * (n * ksc);
+    } else {
+        const float alpha = -expm1f(-(beta * lambda)) / (lambda + p.eps);
+        a = alpha * kss;
+        b = alpha * n;
+    }
+}
+
+// inverses of I + (diagonal 16 x 16 blocks of L): lane c owns column c of a block, two blocks per warp, four warps. Two halves, scaled by kSqUp.
+__device__ __forceinline__ void seq_invert_diagonal(const float* Ld, __half* inv, int nb, int warp, int lane) {
+    if (warp < 4) {
+        const int blk = 2 * warp + (lane >> 4), c = lane & 15;
+        if (blk < nb) {
+            const float* d = Ld + blk * 16 * 17;
+            float col[16];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                float x = t == c ? 1.0f : 0.0f;
+#pragma unroll
+                for (int s = 0; s < 16; ++s)
+                    if (s < t) x = fmaf(-d[t * 17 + s], col[s], x);
+                col[t] = x;
+            }
+            __half* ih = inv + blk * 16 * kSqTStride + c;
+            __half* im = ih + 8 * 16 * kSqTStride;
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                const float x = col[t] * kSqUp;
+                const __half hi = __float2half_rn(x);
+                ih[t * kSqTStride] = hi;
+                im[t * kSqTStride] = __float2half_rn(x - __half2float(hi));
+            }
+        }
+    }
+}
+
+// One warp: rows 16 i .. 16 i + 15 of P with P (I + L) = X by block columns from the right; X in registers, L (two halves) at the start of
+// shared memory, the diagonal blocks' inverses at inv_off; P (two halves, scaled by kSqUp) at mat_off (prow: the same place).
+__device__ __forceinline__ void seq_solve_rows(uint32_t sm0, uint32_t mat_off, uint8_t* prow, uint32_t inv_off, int i, int lane, const float (&xr)[8][2][4]) {
+    const int g = lane >> 2, tq = lane & 3;
+    const uint32_t p_addr = sm0 + mat_off + static_cast<uint32_t>((i * 16 + (lane & 15)) * (kSqXStride * 4) + (lane >> 4) * 16);
+    const uint32_t l_addr = sm0 + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqLStride + (lane >> 4) * 8) * 2u;
+    const uint32_t i_addr = sm0 + inv_off + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqTStride + (lane >> 4) * 8) * 2u;
+    constexpr uint32_t kLMid = kSeqMaxT * kSqLStride * 2, kIMid = 8 * 16 * kSqTStride * 2;
+    const float down = 1.0f / (kSqUp * kSqUp);
+#pragma unroll
+    for (int j = 7; j >= 0; --j) {
+        if (j > i) continue;
+        float s[2][4], c[2][4];  // sum over k > j of P~_ik L_kj: the large products and the cross terms in two chains
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[n][e] = c[n][e] = 0.0f;
+        for (int k = j + 1; k <= i; ++k) {
+            uint32_t ph[4], pm[4], lh[4], lm[4];
+            sq_ldm(ph, p_addr + k * 32);
+            sq_ldm(pm, p_addr + kSqPMid + k * 32);
+            sq_ldm_trans(lh, l_addr + k * (16 * kSqLStride * 2) + j * 32);
+            sq_ldm_trans(lm, l_addr + kLMid + k * (16 * kSqLStride * 2) + j * 32);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                sq_mma(s[n], ph, lh[2 * n], lh[2 * n + 1]);
+                sq_mma(c[n], ph, lm[2 * n], lm[2 * n + 1]);
+                sq_mma(c[n], pm, lh[2 * n], lh[2 * n + 1]);
+            }
+        }
+        // z = X_ij - sum, then P~_ij = z inv_jj
+        uint32_t zh[4], zm[4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            float z[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) z[e] = (xr[j][n][e] - (s[n][e] + c[n][e]) * down) * kSqUp;
+            sq_split(z[0], z[1], zh[2 * n], zm[2 * n]);
+            sq_split(z[2], z[3], zh[2 * n + 1], zm[2 * n + 1]);
+        }
+        uint32_t th[4], tm[4];
+        sq_ldm_trans(th, i_addr + j * (16 * kSqTStride * 2));
+        sq_ldm_trans(tm, i_addr + kIMid + j * (16 * kSqTStride * 2));
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            float o[4] = {0.0f, 0.0f, 0.0f, 0.0f}, oc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            sq_mma(o, zh, th[2 * n], th[2 * n + 1]);
+            sq_mma(oc, zh, tm[2 * n], tm[2 * n + 1]);
+            sq_mma(oc, zm, th[2 * n], th[2 * n + 1]);
+            const int c0 = j * 16 + n * 8 + 2 * tq;
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) {
+                uint32_t hi, mid;
+                sq_split((o[2 * hr] + oc[2 * hr]) * (1.0f / kSqUp), (o[2 * hr + 1] + oc[2 * hr + 1]) * (1.0f / kSqUp), hi, mid);
+                uint8_t* d = prow + (i * 16 + g + 8 * hr) * (kSqXStride * 4) + c0 * 2;
+                *reinterpret_cast<uint32_t*>(d) = hi;
+                *reinterpret_cast<uint32_t*>(d + kSqPMid) = mid;
+            }
+        }
+        __syncwarp();
+    }
+}
+
 template <int CS>
 __device__ __forceinline__ void sq_cluster_sync() {
     if constexpr (CS > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -158,20 +268,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         float a = 0.0f, b = 0.0f, kinv = 0.0f, qinv = 0.0f;
         if (t < T) {
             const float bias = efla_seq_bias(p, static_cast<unsigned>(seq));
-            const float beta = 1.0f / (1.0f + expf(-(p.beta_raw[(row0 + t) * p.ld_beta] + bias)));
-            const float lambda = kss < p.eps ? p.eps : kss;
-            qinv = rsqrtf(qss + p.eps);
-            kinv = kss > 0.0f ? rsqrtf(kss) : 0.0f;
-            const float n = kss * kinv;
-            if (p.method == 0) {
-                const float ksc = rsqrtf(lambda + p.eps);
-                a = beta * (n * ksc) * (n * ksc);
-                b = beta * (n * ksc);
-            } else {
-                const float alpha = -expm1f(-(beta * lambda)) / (lambda + p.eps);
-                a = alpha * kss;
-                b = alpha * n;
-            }
+            seq_scalars(p, p.beta_raw[(row0 + t) * p.ld_beta] + bias, qss, kss, qinv, kinv, a, b);
         }
         qs_sh[t] = kSqUp * qinv;
         ks_sh[t] = kSqUp * kinv;
@@ -331,30 +428,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     }
     __syncthreads();
     // inverse of I + L_ii: lane c owns column c of a block, two blocks per warp
-    if (warp < 4) {
-        const int blk = 2 * warp + (lane >> 4), c = lane & 15;
-        if (blk < nb) {
-            const float* d = Ld + blk * 16 * 17;
-            float col[16];
-#pragma unroll
-            for (int t = 0; t < 16; ++t) {
-                float x = t == c ? 1.0f : 0.0f;
-#pragma unroll
-                for (int s = 0; s < 16; ++s)
-                    if (s < t) x = fmaf(-d[t * 17 + s], col[s], x);
-                col[t] = x;
-            }
-            __half* ih = reinterpret_cast<__half*>(sm + kSqInv) + blk * 16 * kSqTStride + c;
-            __half* im = ih + 8 * 16 * kSqTStride;
-#pragma unroll
-            for (int t = 0; t < 16; ++t) {
-                const float x = col[t] * kSqUp;
-                const __half hi = __float2half_rn(x);
-                ih[t * kSqTStride] = hi;
-                im[t * kSqTStride] = __float2half_rn(x - __half2float(hi));
-            }
-        }
-    }
+    seq_invert_diagonal(Ld, reinterpret_cast<__half*>(sm + kSqInv), nb, warp, lane);
     __syncthreads();
 
     // ---------------- 4. P~ M = X by block columns from the right; warp i owns rows 16 i .. 16 i + 15 ----------------
@@ -375,63 +449,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         }
         __syncwarp();  // the rows are in registers: P~ takes their place
         uint8_t* prow = sm + kSqStage;
-        const uint32_t p_addr = sm0 + kSqStage + static_cast<uint32_t>((i * 16 + (lane & 15)) * (kSqXStride * 4) + (lane >> 4) * 16);
-        const uint32_t l_addr = sm0 + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqLStride + (lane >> 4) * 8) * 2u;
-        const uint32_t i_addr = sm0 + kSqInv + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqTStride + (lane >> 4) * 8) * 2u;
-        constexpr uint32_t kLMid = kSeqMaxT * kSqLStride * 2, kIMid = 8 * 16 * kSqTStride * 2;
-        const float down = 1.0f / (kSqUp * kSqUp);
-#pragma unroll
-        for (int j = 7; j >= 0; --j) {
-            if (j > i) continue;
-            float s[2][4], c[2][4];  // sum over k > j of P~_ik L_kj: the large products and the cross terms in two chains
-#pragma unroll
-            for (int n = 0; n < 2; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s[n][e] = c[n][e] = 0.0f;
-            for (int k = j + 1; k <= i; ++k) {
-                uint32_t ph[4], pm[4], lh[4], lm[4];
-                sq_ldm(ph, p_addr + k * 32);
-                sq_ldm(pm, p_addr + kSqPMid + k * 32);
-                sq_ldm_trans(lh, l_addr + k * (16 * kSqLStride * 2) + j * 32);
-                sq_ldm_trans(lm, l_addr + kLMid + k * (16 * kSqLStride * 2) + j * 32);
-#pragma unroll
-                for (int n = 0; n < 2; ++n) {
-                    sq_mma(s[n], ph, lh[2 * n], lh[2 * n + 1]);
-                    sq_mma(c[n], ph, lm[2 * n], lm[2 * n + 1]);
-                    sq_mma(c[n], pm, lh[2 * n], lh[2 * n + 1]);
-                }
-            }
-            // z = X_ij - sum, then P~_ij = z inv_jj
-            uint32_t zh[4], zm[4];
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                float z[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) z[e] = (xr[j][n][e] - (s[n][e] + c[n][e]) * down) * kSqUp;
-                sq_split(z[0], z[1], zh[2 * n], zm[2 * n]);
-                sq_split(z[2], z[3], zh[2 * n + 1], zm[2 * n + 1]);
-            }
-            uint32_t th[4], tm[4];
-            sq_ldm_trans(th, i_addr + j * (16 * kSqTStride * 2));
-            sq_ldm_trans(tm, i_addr + kIMid + j * (16 * kSqTStride * 2));
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                float o[4] = {0.0f, 0.0f, 0.0f, 0.0f}, oc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                sq_mma(o, zh, th[2 * n], th[2 * n + 1]);
-                sq_mma(oc, zh, tm[2 * n], tm[2 * n + 1]);
-                sq_mma(oc, zm, th[2 * n], th[2 * n + 1]);
-                const int c0 = j * 16 + n * 8 + 2 * tq;
-#pragma unroll
-                for (int hr = 0; hr < 2; ++hr) {
-                    uint32_t hi, mid;
-                    sq_split((o[2 * hr] + oc[2 * hr]) * (1.0f / kSqUp), (o[2 * hr + 1] + oc[2 * hr + 1]) * (1.0f / kSqUp), hi, mid);
-                    uint8_t* d = prow + (i * 16 + g + 8 * hr) * (kSqXStride * 4) + c0 * 2;
-                    *reinterpret_cast<uint32_t*>(d) = hi;
-                    *reinterpret_cast<uint32_t*>(d + kSqPMid) = mid;
-                }
-            }
-            __syncwarp();
-        }
+        seq_solve_rows(sm0, kSqStage, prow, kSqInv, i, lane, xr);
         // the columns' factors b_s, scaled to at most one: applied to the finished rows (exact powers of two aside, one more rounding)
         for (int idx = lane; idx < 16 * (i + 1) * 8; idx += 32) {
             const int rr = idx / ((i + 1) * 8), cc = (idx - rr * ((i + 1) * 8)) * 2;
@@ -534,12 +552,305 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// The same closed form for sequences of more than 128 tokens, one CTA per (sequence, head), 128-token blocks. With r_I = diag(b) v_I -
+// sum_{J < I} L_IJ w_J the blocks of w = (I + L)^-1 diag(b) v follow one after the other, w_I = (I + L_II)^-1 r_I, and y_I = sum_{J <= I} X_IJ w_J.
+// w lives in the rows of the output until its block's y replaces it: blocks of y are formed from the last to the first, and y_I needs w_J of
+// J <= I only, so there is no scratch. Every block product goes through one gram routine (two blocks of rows over hd -> 128 x 128
+// matrix in shared memory, two halves per element) and one product routine (that matrix times a 128 x hd block, 64 columns at a time).
+// T^2 hd products on the tensor cores instead of T hd^2 on the CUDA cores, whose per-token form passes the whole state through the
+// registers' adders twice and needs two block-wide barriers per token. 400 sequences of 322 tokens, one head of 512: 17.5 ms token by
+// token, 2.4 ms here (bound by the MMAs and the conversions around them, like efla_seq_kernel).
+// ------------------------------------------------------------------------------------------------
+constexpr int kLgMaxT = 1024;
+constexpr int kLgMat = 4 * kSqTile;                               // the matrix [128][kSqXStride floats]: hi halves, mid halves at kSqPMid
+constexpr int kLgDiag = kLgMat + kSeqMaxT * kSqXStride * 4;
+constexpr int kLgInv = kLgDiag + 8 * 16 * 17 * 4;
+constexpr int kLgScal = kLgInv + 2 * 8 * 16 * kSqTStride * 2;     // q scale, k scale, a, b [4][T]
+constexpr int kLgRed = kLgScal + 4 * kLgMaxT * 4;
+constexpr int kLgSmem = kLgRed + 64;
+static_assert(2 * kSeqMaxT * kSqLStride * 2 <= 4 * kSqTile, "L takes the staging tiles' place while the diagonal block is inverted");
+static_assert(kLgMat % 16 == 0 && kLgDiag % 16 == 0 && kLgInv % 16 == 0 && kLgScal % 16 == 0 && kLgRed % 16 == 0, "16-byte aligned regions");
+
+enum LongOut { LO_WRITE, LO_FROM_V, LO_SUB, LO_ADD };  // out = D, out = b v - D, out -= D, out += D
+
+__global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaParams p) {
+    pdl_wait();
+    extern __shared__ __align__(16) uint8_t sm[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, tq = lane & 3;
+    const int T = p.T, hd = p.hidden / p.heads;
+    const unsigned unit = blockIdx.x;
+    const unsigned seq = unit / static_cast<unsigned>(p.heads);
+    const int h = static_cast<int>(unit - seq * static_cast<unsigned>(p.heads));
+    const int nblocks = (T + kSeqMaxT - 1) / kSeqMaxT, nd = (hd + 63) >> 6;
+    const size_t row0 = static_cast<size_t>(seq) * T;
+    const float* qg = static_cast<const float*>(p.q) + row0 * p.ld_qkv + h * hd;
+    const float* kg = static_cast<const float*>(p.k) + row0 * p.ld_qkv + h * hd;
+    const float* vg = static_cast<const float*>(p.v) + row0 * p.ld_qkv + h * hd;
+    float* og = static_cast<float*>(p.out) + row0 * p.ld_out + h * hd;
+    float* qs_sh = reinterpret_cast<float*>(sm + kLgScal);
+    float* ks_sh = qs_sh + kLgMaxT;
+    float* a_sh = ks_sh + kLgMaxT;
+    float* b_sh = a_sh + kLgMaxT;
+    float* red = reinterpret_cast<float*>(sm + kLgRed);
+    const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
+
+    // ---------------- norms and scalars of all tokens (as in efla_seq_kernel) ----------------
+    for (int t = warp; t < nblocks * kSeqMaxT; t += 16) {
+        float qss = 0.0f, kss = 0.0f;
+        if (t < T) {
+            const float4* q4 = reinterpret_cast<const float4*>(qg + static_cast<size_t>(t) * p.ld_qkv);
+            const float4* k4 = reinterpret_cast<const float4*>(kg + static_cast<size_t>(t) * p.ld_qkv);
+            for (int i = lane; i < (hd >> 2); i += 32) {
+                const float4 a = q4[i], b = k4[i];
+                qss = fmaf(a.x, a.x, qss); qss = fmaf(a.y, a.y, qss); qss = fmaf(a.z, a.z, qss); qss = fmaf(a.w, a.w, qss);
+                kss = fmaf(b.x, b.x, kss); kss = fmaf(b.y, b.y, kss); kss = fmaf(b.z, b.z, kss); kss = fmaf(b.w, b.w, kss);
+            }
+        }
+        qss = warp_sum_f(qss);
+        kss = warp_sum_f(kss);
+        if (lane == 0) { qs_sh[t] = qss; ks_sh[t] = kss; }
+    }
+    __syncthreads();
+    const float bias = efla_seq_bias(p, seq);
+    for (int t = tid; t < nblocks * kSeqMaxT; t += kSeqThreads) {
+        float a = 0.0f, b = 0.0f, ks = 0.0f, qs = 0.0f;
+        if (t < T) seq_scalars(p, p.beta_raw[(row0 + t) * p.ld_beta] + bias, qs_sh[t], ks_sh[t], qs, ks, a, b);
+        qs_sh[t] = kSqUp * qs;
+        ks_sh[t] = kSqUp * ks;
+        a_sh[t] = a;
+        b_sh[t] = b;
+    }
+    __syncthreads();
+
+    const int piece = tid & 15, srow = tid >> 4;  // staging: 16-byte piece of a 64-column row, rows srow + 32 i
+    const int wr = warp >> 1, wc = warp & 1;      // results: 16-row block, column half
+    auto load = [&](float4 (&r)[4], const float* base, int ld, int blk, int ct) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = blk * kSeqMaxT + srow + 32 * i, c = ct * 64 + 4 * piece;
+            r[i] = t < T && c < hd ? *reinterpret_cast<const float4*>(base + static_cast<size_t>(t) * ld + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+    auto store = [&](const float4 (&r)[4], int tile, const float* scale, float common) {  // two halves per value
+        uint8_t* st = sm + tile * kSqTile;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float f = scale != nullptr ? scale[srow + 32 * i] : common;
+            const int o = ((srow + 32 * i) * kSqStride + 4 * piece) * 2;
+            uint2 hi, mid;
+            sq_split(r[i].x * f, r[i].y * f, hi.x, mid.x);
+            sq_split(r[i].z * f, r[i].w * f, hi.y, mid.y);
+            *reinterpret_cast<uint2*>(st + o) = hi;
+            *reinterpret_cast<uint2*>(st + kSqTile + o) = mid;
+        }
+    };
+
+    // rows of block I of `rows` (normalised by rscale) times rows of block J of k; G (is_g: scaled by a, strictly lower on the diagonal) or
+    // X (lower on the diagonal). Into the matrix, or (G on the diagonal) L and its diagonal blocks for the inversion.
+    auto gram = [&](const float* rows, const float* rscale, bool is_g, int I, int J) {
+        float acc[8][4];
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[n][e] = 0.0f;
+        float4 ra[4], rb[4];
+        load(ra, rows, p.ld_qkv, I, 0);
+        load(rb, kg, p.ld_qkv, J, 0);
+        const bool used = I != J || wc == 0 || wr >= 4;  // the upper half of a diagonal block is not needed
+        const uint32_t aa = sm0 + static_cast<uint32_t>((wr * 16 + (lane & 15)) * kSqStride + (lane >> 4) * 8) * 2u;
+        const uint32_t ba = sm0 + 2u * kSqTile + static_cast<uint32_t>((wc * 64 + (lane & 7)) * kSqStride + ((lane >> 3) & 1) * 8) * 2u + (lane >> 4) * static_cast<uint32_t>(kSqTile);
+        for (int db = 0; db < nd; ++db) {
+            store(ra, 0, rscale + I * kSeqMaxT, 0.0f);
+            store(rb, 2, ks_sh + J * kSeqMaxT, 0.0f);
+            __syncthreads();
+            if (db + 1 < nd) {
+                load(ra, rows, p.ld_qkv, I, db + 1);
+                load(rb, kg, p.ld_qkv, J, db + 1);
+            }
+            if (used) {
+                const int nk = min(4, (hd - db * 64) >> 4);
+                for (int kk = 0; kk < nk; ++kk) {
+                    uint32_t ah[4], am[4];
+                    sq_ldm(ah, aa + kk * 32);
+                    sq_ldm(am, aa + kSqTile + kk * 32);
+#pragma unroll
+                    for (int n = 0; n < 8; n += 2) {
+                        uint32_t b[4], c[4];
+                        sq_ldm(b, ba + kk * 32 + n * (8 * kSqStride * 2));
+                        sq_ldm(c, ba + kk * 32 + (n + 1) * (8 * kSqStride * 2));
+                        sq_mma(acc[n], ah, b[0], b[1]); sq_mma(acc[n + 1], ah, c[0], c[1]);
+                        sq_mma(acc[n], ah, b[2], b[3]); sq_mma(acc[n + 1], ah, c[2], c[3]);
+                        sq_mma(acc[n], am, b[0], b[1]); sq_mma(acc[n + 1], am, c[0], c[1]);
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        const float gdown = 1.0f / (kSqUp * kSqUp);
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {
+            const int c0 = wc * 64 + n * 8 + 2 * tq;
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) {
+                const int t = wr * 16 + g + 8 * hr;
+                const float f = is_g ? gdown * a_sh[I * kSeqMaxT + t] : gdown;
+                const int last = I != J ? kSeqMaxT : is_g ? t - 1 : t;  // last column kept
+                const float x0 = c0 <= last ? acc[n][2 * hr] * f : 0.0f, x1 = c0 + 1 <= last ? acc[n][2 * hr + 1] * f : 0.0f;
+                uint32_t hi, mid;
+                sq_split(x0 * kSqUp, x1 * kSqUp, hi, mid);
+                if (is_g && I == J) {
+                    *reinterpret_cast<uint32_t*>(sm + (t * kSqLStride + c0) * 2) = hi;
+                    *reinterpret_cast<uint32_t*>(sm + (kSeqMaxT * kSqLStride + t * kSqLStride + c0) * 2) = mid;
+                    if ((c0 >> 4) == wr) {
+                        float* d = reinterpret_cast<float*>(sm + kLgDiag) + t * 17 + (c0 & 15);
+                        d[0] = x0;
+                        d[1] = x1;
+                    }
+                } else {
+                    uint8_t* d = sm + kLgMat + t * (kSqXStride * 4) + c0 * 2;
+                    *reinterpret_cast<uint32_t*>(d) = hi;
+                    *reinterpret_cast<uint32_t*>(d + kSqPMid) = mid;
+                }
+            }
+        }
+        __syncthreads();
+    };
+
+    // out block I (op) matrix times block J of src (rows scaled by b where src is v); lower: only the lower triangle of blocks is read
+    auto product = [&](const float* src, int ld, bool scale_b, int I, int J, bool lower, LongOut op) {
+        float4 r[4];
+        auto fetch = [&](int ct) {
+            load(r, src, ld, J, ct);
+            if (scale_b) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float f = b_sh[J * kSeqMaxT + srow + 32 * i];
+                    r[i].x *= f; r[i].y *= f; r[i].z *= f; r[i].w *= f;
+                }
+            }
+        };
+        fetch(0);
+        const uint32_t pa = sm0 + kLgMat + static_cast<uint32_t>((wr * 16 + (lane & 15)) * (kSqXStride * 4) + (lane >> 4) * 16);
+        const uint32_t vb = sm0 + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqStride + wc * 32 + (lane >> 4) * 8) * 2u;
+        for (int ct = 0; ct < nd; ++ct) {
+            float m = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) m = fmaxf(fmaxf(fmaxf(m, fabsf(r[i].x)), fmaxf(fabsf(r[i].y), fabsf(r[i].z))), fabsf(r[i].w));
+            m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));  // non-negative floats order like their bits
+            if (lane == 0) red[warp] = m;
+            __syncthreads();  // also: everyone is done with the previous tile
+            const float vs = sq_pow2_scale(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(red[lane & 15]))));
+            store(r, 0, nullptr, vs);
+            if (ct + 1 < nd) fetch(ct + 1);
+            __syncthreads();
+            float y[4][4];
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) y[n][e] = 0.0f;
+            const int last = lower ? wr : 7;
+            for (int j = 0; j <= last; ++j) {
+                uint32_t ah[4], am[4];
+                sq_ldm(ah, pa + j * 32);
+                sq_ldm(am, pa + kSqPMid + j * 32);
+#pragma unroll
+                for (int np = 0; np < 2; ++np) {
+                    uint32_t vh[4], vm[4];
+                    sq_ldm_trans(vh, vb + j * (16 * kSqStride * 2) + np * 32);
+                    sq_ldm_trans(vm, vb + kSqTile + j * (16 * kSqStride * 2) + np * 32);
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) sq_mma(y[2 * np + n], ah, vh[2 * n], vh[2 * n + 1]);
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) sq_mma(y[2 * np + n], ah, vm[2 * n], vm[2 * n + 1]);
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) sq_mma(y[2 * np + n], am, vh[2 * n], vh[2 * n + 1]);
+                }
+            }
+            const float ds = 1.0f / kSqUp / vs;
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                const int c = ct * 64 + wc * 32 + n * 8 + 2 * tq;
+#pragma unroll
+                for (int hr = 0; hr < 2; ++hr) {
+                    const int t = I * kSeqMaxT + wr * 16 + g + 8 * hr;
+                    if (t >= T || c >= hd) continue;
+                    float2* o = reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c);
+                    float2 x = make_float2(y[n][2 * hr] * ds, y[n][2 * hr + 1] * ds);
+                    if (op == LO_FROM_V) {
+                        const float2 v = *reinterpret_cast<const float2*>(vg + static_cast<size_t>(t) * p.ld_qkv + c);
+                        x = make_float2(fmaf(b_sh[t], v.x, -x.x), fmaf(b_sh[t], v.y, -x.y));
+                    } else if (op == LO_SUB || op == LO_ADD) {
+                        const float2 old = *o;
+                        x = op == LO_SUB ? make_float2(old.x - x.x, old.y - x.y) : make_float2(old.x + x.x, old.y + x.y);
+                    }
+                    *o = x;
+                }
+            }
+        }
+        __syncthreads();  // the block is complete, matrix and tile are free
+    };
+
+    // inverse of the unit lower triangular I + L of a diagonal block, from its 16 x 16 diagonal blocks outwards, into the matrix
+    auto invert = [&] {
+        seq_invert_diagonal(reinterpret_cast<const float*>(sm + kLgDiag), reinterpret_cast<__half*>(sm + kLgInv), 8, warp, lane);
+        __syncthreads();
+        if (warp < 8) {
+            float xr[8][2][4];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) xr[j][n][e] = j == warp && n * 8 + 2 * tq + (e & 1) == g + 8 * (e >> 1) ? 1.0f : 0.0f;
+            seq_solve_rows(sm0, kLgMat, sm + kLgMat, kLgInv, warp, lane, xr);
+        }
+        __syncthreads();
+    };
+
+    for (int I = 0; I < nblocks; ++I) {
+        for (int J = 0; J < I; ++J) {
+            gram(kg, ks_sh, true, I, J);
+            product(og, p.ld_out, false, I, J, false, J == 0 ? LO_FROM_V : LO_SUB);
+        }
+        gram(kg, ks_sh, true, I, I);
+        invert();
+        if (I == 0) product(vg, p.ld_qkv, true, 0, 0, true, LO_WRITE);
+        else product(og, p.ld_out, false, I, I, true, LO_WRITE);
+    }
+    for (int I = nblocks - 1; I >= 0; --I) {
+        gram(qg, qs_sh, false, I, I);
+        product(og, p.ld_out, false, I, I, true, LO_WRITE);
+        for (int J = 0; J < I; ++J) {
+            gram(qg, qs_sh, false, I, J);
+            product(og, p.ld_out, false, I, J, false, LO_ADD);
+        }
+    }
+}
+
 }  // namespace
+
+// The closed form's work per token grows with the sequence, the per-token kernel's does not, but the latter spreads a unit over several SMs. One head of
+// 512: 322 tokens 0.69 / 1.16 ms (closed form / per token) for 4 sequences, 2.4 / 17.5 ms for 400; 1000 tokens 4.4 / 3.6 ms for 4, 5.1 / 8.3 ms for 40.
+static bool seq_long_pays(const EflaParams& p) {
+    if (p.T > 768 && (p.T > kLgMaxT || p.seqs * static_cast<long long>(p.heads) < 32)) return false;
+    // the output holds w before all of q, k and v have been read: it must not lie among them
+    if (p.seqs <= 0) return true;
+    const size_t last = static_cast<size_t>(p.seqs) * p.T - 1;
+    const char* o = static_cast<const char*>(p.out);
+    const char* o_end = o + (last * p.ld_out + p.hidden) * sizeof(float);
+    for (const void* in : {static_cast<const void*>(p.q), static_cast<const void*>(p.k), static_cast<const void*>(p.v)}) {
+        const char* a = static_cast<const char*>(in);
+        if (o < a + (last * p.ld_qkv + p.hidden) * sizeof(float) && a < o_end) return false;
+    }
+    return true;
+}
 
 // (heads of 32 are faster one warp each, token by token: efla_head32_kernel)
 bool efla_seq_applies(const EflaParams& p) {
     const int hd = p.hidden / p.heads;
-    return p.state == nullptr && p.state_fp16 != 0 && !p.qkv_f16 && !p.out_f16 && hd > 32 && hd % 32 == 0 && p.T <= kSeqMaxT &&
+    return p.state == nullptr && p.state_fp16 != 0 && !p.qkv_f16 && !p.out_f16 && hd > 32 && hd % 32 == 0 && (p.T <= kSeqMaxT || (seq_long_pays(p) && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0 && p.ld_out % 4 == 0)) &&
            ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v)) & 15) == 0 && p.ld_qkv % 4 == 0 &&
            (reinterpret_cast<uintptr_t>(p.out) & 7) == 0 && p.ld_out % 2 == 0 && p.seqs * static_cast<long long>(p.heads) <= 0x7fffffffLL / 4;
 }
@@ -575,6 +886,16 @@ int efla_seq_launch(const EflaParams& p, cudaStream_t stream) {
     const int one = resident_clusters<1>(dev), two = resident_clusters<2>(dev), four = resident_clusters<4>(dev);
     if (one <= 0 || two <= 0 || four <= 0) return BNF4_ERR_CUDA;
     const long long units = p.seqs * p.heads;
+    if (p.T > kSeqMaxT) {
+        static std::atomic<bool> configured[64] = {};  // function attributes are per device
+        if (dev >= 64 || !configured[dev].load(std::memory_order_relaxed)) {
+            const int rc2 = check_cuda(cudaFuncSetAttribute(efla_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLgSmem), "cudaFuncSetAttribute(efla_long_kernel)");
+            if (rc2) return rc2;
+            if (dev < 64) configured[dev].store(true, std::memory_order_relaxed);
+        }
+        launch_pdl_if(false, efla_long_kernel, static_cast<unsigned>(units), kSeqThreads, kLgSmem, stream, p);
+        return check_launch("efla_long_kernel");
+    }
     const int nd = (p.hidden / p.heads + 63) >> 6;
     // Few units leave SMs idle: two or four CTAs share one as long as all units still run at once and every CTA has a block of columns. One head of
     // 512, 32 sequences: 71 us with one, 48 with two, 40 with four; a second pass costs more than sharing gains (37 units: 73 us with four,

@@ -85,7 +85,7 @@ __device__ __forceinline__ float efla_seq_bias(const EflaParams& p, unsigned seq
 #endif
 int efla_launch(const EflaParams& p, cudaStream_t stream);
 extern int g_efla_chunked;
-// Whole sequences of at most 128 tokens from a zero state, any head_dim (efla_seq.cu).
+// Whole sequences from a zero state, any head_dim (efla_seq.cu).
 bool efla_seq_applies(const EflaParams& p);
 int efla_seq_launch(const EflaParams& p, cudaStream_t stream);
 

@@ -1,4 +1,4 @@
-"""EFLA scan for head widths other than 64: the closed form of a whole sequence (zero state, at most 128 tokens) and the
+"""EFLA scan for head widths other than 64: the closed form of a whole sequence (zero state) and the
 generic per-token kernel's column / row splits.
 
 The closed form rounds nothing to fp16 between tokens, so it is held to the recurrence in float64. Its operands carry 22
@@ -124,3 +124,34 @@ def test_generic_kernel_carries_the_state(H, hidden, fp16, offset):
     parts = np.concatenate([call(qkv[:, :T1], two, T1), call(qkv[:, T1:], two, T2)], axis=1)
     assert np.array_equal(whole, parts)
     assert torch.equal(one, two)
+
+
+@pytest.mark.parametrize("scale", [0.3, 1000.0, 1e-3])
+@pytest.mark.parametrize("hidden,heads,seqs,T,method", [
+    (512, 1, 2, 129, 1), (512, 1, 3, 322, 0), (96, 1, 2, 256, 1), (320, 2, 2, 257, 1), (128, 1, 150, 140, 0), (160, 1, 1, 768, 1),
+    (96, 1, 32, 1024, 1)])   # (the per-token kernel has 1024 tokens of fewer units)
+def test_closed_form_of_long_sequences(H, hidden, heads, seqs, T, method, scale):
+    """More than one block of 128 tokens: one token in the last block, full blocks, more units than SMs, the longest of few and of many
+    units. Every block product adds the error that the one-block form is allowed, so the bound grows with the number of blocks."""
+    rng = np.random.default_rng(hidden + T + method)
+    fc = (3 * hidden + 1 + 31) & ~31
+    qkv = make_qkv(rng, seqs * T, hidden, fc, scale)
+    bb = (rng.standard_normal((seqs + 1) // 2) * 0.2 - 2.0).astype(np.float32)
+    bb_seq = np.repeat(bb, 2)[:seqs]
+    got = run(H, qkv, bb, 2, hidden, heads, seqs, T, method, 0)
+    ref = exact_scan(qkv.reshape(seqs, T, fc), bb_seq, hidden, heads, method)
+    assert np.abs(got - ref).max() <= 2e-5 * ((T + 127) // 128) * np.abs(ref).max()
+
+
+def test_long_sequence_into_its_own_queries(H):
+    """An output that overlays q keeps the per-token kernel, which reads a token before it writes it."""
+    import torch
+    rng = np.random.default_rng(3)
+    hidden, T, fc = 96, 150, 320
+    qkv = make_qkv(rng, T, hidden, fc, 0.4)
+    bb = np.full(1, -2.0, np.float32)
+    ref = run(H, qkv, bb, 1, hidden, 1, 1, T, 1, 0)
+    qd = dev(qkv)
+    H.efla_scan(state=None, state_fp16=1, q=qd, k=qd[:, hidden:], v=qd[:, 2 * hidden:], beta_raw=dev(qkv[:, 3 * hidden]), ld_qkv=fc, ld_beta=1,
+                beta_bias_seq=dev(bb), seqs_per_bias=1, hidden=hidden, heads=1, seqs=1, T=T, method=1, eps=1e-6, out=qd, ld_out=fc, variant=0)
+    assert np.abs(qd[:, :hidden].cpu().numpy() - ref[0]).max() <= SCAN_TOL * np.abs(ref).max()
