@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Benchmark of the population-evaluation ES step (BASELINE.json metric: population tokens/s per ES step).
+"""Benchmark of the population-evaluation ES step (population tokens/s per ES step).
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--pop P] [--stress] [--exact-scan]
     python bench.py --sweep                      # perturbed-NVFP4 GEMM sweep M x (K = N) with FP4 utilisation, one JSON line
@@ -185,7 +185,7 @@ def _gemm_operands(H, m, n, k, rank, rows_per_member, seed=0):
 
 
 def run_sweep(args):
-    """BASELINE config 4's standalone sweep: D = alpha A B^T + rank-r term, fp32 out, M x (K = N)."""
+    """Standalone GEMM sweep: D = alpha A B^T + rank-r term, fp32 out, M x (K = N)."""
     import numpy as np
     import torch
     from bitnet_nvfp4_b200 import host as H
