@@ -86,7 +86,7 @@ def test_closed_form_matches_the_exact_recurrence(H, hidden, heads, seqs, T, met
 
 
 @pytest.mark.parametrize("hidden,heads,seqs,T,method", [(96, 1, 3, 20, 1), (160, 1, 2, 9, 1), (1024, 1, 2, 5, 1), (256, 8, 4, 12, 0), (1280, 1, 1, 3, 1),
-                                                        (512, 2, 3, 150, 1), (384, 1, 2, 140, 0), (128, 4, 3, 33, 1), (32, 1, 5, 1, 1), (96, 3, 7, 130, 0)])
+                                                        (512, 2, 3, 150, 1), (384, 1, 2, 140, 0), (512, 1, 3, 12, 1), (320, 1, 2, 9, 0), (512, 1, 20, 5, 1), (128, 4, 3, 33, 1), (32, 1, 5, 1, 1), (96, 3, 7, 130, 0)])
 def test_generic_kernel_splits_match_the_oracle(H, hidden, heads, seqs, T, method):
     """Every split of the generic kernel (piece counts and rows per thread), and AUTO beyond 128 tokens."""
     rng = np.random.default_rng(hidden * 7 + T)
