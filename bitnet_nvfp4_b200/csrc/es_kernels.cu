@@ -85,30 +85,82 @@ __global__ void __launch_bounds__(1024) ce_step_kernel(const float* __restrict__
     }
 }
 
-// Population form: grid (chunks, members). partial[member * chunks + chunk] = sum of the chunk's row losses. With a counter per member
-// (zero before the launch, zero again after it) the member's last block also forms the mean, in chunk order; without, ce_finalize_kernel
-// does.
+// Population form. A member's rows form 16 groups of consecutive rows, a group eight chains: chain w adds rows w, w + 8, .. of its group in
+// order, the group adds its chains in order, the mean adds the groups in double. Every loss is a function of the logits alone: grid and
+// member count only say which warps compute the row losses. (1024 pairs rank losses that differ in the last place: another order of these
+// sums moves some across each other and with them the update.)
+// Grid (16 split, members), split 1, 2 or 4: `split` blocks share a group, `split` warps a chain. Member counters (zero before the launch, zero
+// again after it): the member's last block forms the mean; without them split is 1, partial[member * 16 + group] holds the groups'
+// sums and ce_finalize_kernel follows. With split > 1 partial holds the chains' sums, 128 per member.
 constexpr int kCeChunks = 16;
-__device__ __forceinline__ void ce_finish(float block_sum, float* partial, unsigned* counters, int rows_per_member, float* loss_mean) {
+struct CeRows {
+    int split, r0, r1, chain, j;  // this warp: rows r0 + chain + 8 (j + split k) below r1
+    __device__ explicit CeRows(int rows_per_member) {
+        const int warp = threadIdx.x >> 5, per = (rows_per_member + kCeChunks - 1) / kCeChunks;
+        split = static_cast<int>(gridDim.x) / kCeChunks;
+        const int group = static_cast<int>(blockIdx.x) / split, sub = static_cast<int>(blockIdx.x) - group * split;
+        r0 = group * per;
+        r1 = min(rows_per_member, r0 + per);
+        chain = sub * (8 / split) + warp / split;
+        j = warp % split;
+    }
+    __device__ int row(int k) const { return r0 + chain + 8 * (j + split * k); }
+    __device__ int passes(int rpi) const { return (r1 - r0 + 8 * split * rpi - 1) / (8 * split * rpi); }  // (uniform in the block)
+};
+// adds the row losses l[i] of rows row(k0 + i) to the chain's sum (kept by its first warp)
+template <int RPI>
+__device__ __forceinline__ void ce_add(const CeRows& rr, int pass, const float (&l)[RPI], float& acc) {
+    if (rr.split == 1) {
+#pragma unroll
+        for (int i = 0; i < RPI; ++i) acc += l[i];
+        return;
+    }
+    __shared__ float rows[2][8][RPI];
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int i = 0; i < RPI; ++i) rows[pass & 1][warp][i] = l[i];
+    __syncthreads();
+    if (rr.j == 0)
+#pragma unroll
+        for (int i = 0; i < RPI; ++i)
+            for (int q = 0; q < rr.split; ++q) acc += rows[pass & 1][warp + q][i];
+}
+__device__ __forceinline__ void ce_finish(const CeRows& rr, float acc, float* partial, unsigned* counters, int rows_per_member, float* loss_mean) {
+    __shared__ float part[8];
     __shared__ bool last;
-    const int member = blockIdx.y, chunks = gridDim.x;
+    const int member = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0 && rr.j == 0) part[warp / rr.split] = acc;
+    __syncthreads();
     if (threadIdx.x == 0) {
-        partial[member * chunks + blockIdx.x] = block_sum;
+        if (rr.split == 1) {
+            float t = 0.0f;
+            for (int w = 0; w < 8; ++w) t += part[w];
+            partial[member * kCeChunks + blockIdx.x] = t;
+        } else {
+            const int chains = 8 / rr.split;
+            for (int w = 0; w < chains; ++w) partial[member * (8 * kCeChunks) + blockIdx.x * chains + w] = part[w];
+        }
         last = false;
         if (counters != nullptr) {
             __threadfence();
-            last = atomicInc(counters + member, chunks - 1) == static_cast<unsigned>(chunks - 1);  // wraps to zero
+            last = atomicInc(counters + member, gridDim.x - 1) == gridDim.x - 1;  // wraps to zero
         }
     }
     if (counters == nullptr) return;
     __syncthreads();
     if (!last || threadIdx.x >= 32) return;
     __threadfence();
-    double t = 0.0;
-    for (int c = threadIdx.x; c < chunks; c += 32) t += static_cast<double>(__ldcg(partial + member * chunks + c));
+    float group = 0.0f;
+    if (lane < kCeChunks) {
+        if (rr.split == 1) group = __ldcg(partial + member * kCeChunks + lane);
+        else
+            for (int w = 0; w < 8; ++w) group += __ldcg(partial + member * (8 * kCeChunks) + 8 * lane + w);
+    }
+    double t = static_cast<double>(group);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    if (threadIdx.x == 0) loss_mean[member] = static_cast<float>(t / static_cast<double>(rows_per_member));
+    if (lane == 0) loss_mean[member] = static_cast<float>(t / static_cast<double>(rows_per_member));
 }
 __global__ void __launch_bounds__(256) ce_population_kernel(const float* __restrict__ logits, int ld, const float* __restrict__ bias,
                                                             const int8_t* __restrict__ bias_noise, float sigma,
@@ -116,24 +168,20 @@ __global__ void __launch_bounds__(256) ce_population_kernel(const float* __restr
                                                             float* partial, unsigned* counters, float* loss_mean) {
     pdl_wait();
     after(logits, bias, bias_noise, targets);
-    __shared__ float part[8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int member = blockIdx.y, chunk = blockIdx.x;
-    const int per = (rows_per_member + gridDim.x - 1) / gridDim.x;
-    const int r0 = chunk * per, r1 = min(rows_per_member, r0 + per);
+    const CeRows rr(rows_per_member);
+    const int lane = threadIdx.x & 31, member = blockIdx.y;
     const float bns = (member & 1) ? -sigma : sigma;
     const int8_t* nz = bias_noise != nullptr ? bias_noise + static_cast<size_t>(member >> 1) * vocab : nullptr;
     float acc = 0.0f;
-    for (int r = r0 + warp; r < r1; r += 8) {
-        const size_t row = static_cast<size_t>(member) * rows_per_member + r;
-        acc += ce_row_loss(logits + row * ld, bias, nullptr, nz, bns, vocab, static_cast<int>(targets[r]), lane);
+    const int passes = rr.passes(1);
+    for (int k = 0; k < passes; ++k) {
+        const int r = rr.row(k);
+        float l[1] = {0.0f};
+        if (r < rr.r1)
+            l[0] = ce_row_loss(logits + (static_cast<size_t>(member) * rows_per_member + r) * ld, bias, nullptr, nz, bns, vocab, static_cast<int>(targets[r]), lane);
+        ce_add<1>(rr, k, l, acc);
     }
-    if (lane == 0) part[warp] = acc;
-    __syncthreads();
-    float t = 0.0f;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < 8; ++w) t += part[w];
-    ce_finish(t, partial, counters, rows_per_member, loss_mean);
+    ce_finish(rr, acc, partial, counters, rows_per_member, loss_mean);
 }
 
 // Streaming form of the same reduction for 16-byte aligned rows and vocab % 4 == 0: lane l owns the float4 groups
@@ -147,11 +195,8 @@ __global__ void __launch_bounds__(256) ce_population_vec_kernel(const float* __r
                                                                 float* partial, unsigned* counters, float* loss_mean) {
     pdl_wait();
     after(logits, bias, bias_noise, targets);
-    __shared__ float part[8];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int member = blockIdx.y, chunk = blockIdx.x;
-    const int per = (rows_per_member + gridDim.x - 1) / gridDim.x;
-    const int r0 = chunk * per, r1 = min(rows_per_member, r0 + per);
+    const CeRows rr(rows_per_member);
+    const int lane = threadIdx.x & 31, member = blockIdx.y, r1 = rr.r1;
     const float bns = (member & 1) ? -sigma : sigma;
     const int groups = vocab >> 2;
     float4 bv[NV4], nv[NV4];
@@ -168,12 +213,14 @@ __global__ void __launch_bounds__(256) ce_population_vec_kernel(const float* __r
         }
     }
     float acc = 0.0f;
-    for (int rb = r0 + warp; rb < r1; rb += 8 * RPI) {
+    const int passes = rr.passes(RPI);
+    for (int pass = 0; pass < passes; ++pass) {
+        float l[RPI];
         float4 x[RPI][NV4];
         int y[RPI];
 #pragma unroll
         for (int i = 0; i < RPI; ++i) {
-            const int r = rb + 8 * i;
+            const int r = rr.row(pass * RPI + i);
             y[i] = r < r1 ? static_cast<int>(targets[r]) : 0;
             const float* lg = logits + (static_cast<size_t>(member) * rows_per_member + min(r, r1 - 1)) * ld;
 #pragma unroll
@@ -202,19 +249,15 @@ __global__ void __launch_bounds__(256) ce_population_vec_kernel(const float* __r
             for (int j = 0; j < NV4; ++j) sum += (expf(x[i][j].x - mx) + expf(x[i][j].y - mx)) + (expf(x[i][j].z - mx) + expf(x[i][j].w - mx));
             sum = warp_sum_f(sum);
             // the target's logit is re-read (one broadcast load per row) and perturbed with the same two operations
-            const int r = min(rb + 8 * i, r1 - 1);
+            const int r = min(rr.row(pass * RPI + i), r1 - 1);
             float vy = logits[(static_cast<size_t>(member) * rows_per_member + r) * ld + y[i]];
             if (bias != nullptr) vy += bias[y[i]];
             if (bias_noise != nullptr) vy = fmaf(bns, static_cast<float>(bias_noise[static_cast<size_t>(member >> 1) * vocab + y[i]]), vy);
-            if (rb + 8 * i < r1) acc += -(vy - mx - logf(sum + 1e-9f));
+            l[i] = rr.row(pass * RPI + i) < r1 ? -(vy - mx - logf(sum + 1e-9f)) : 0.0f;
         }
+        ce_add<RPI>(rr, pass, l, acc);
     }
-    if (lane == 0) part[warp] = acc;
-    __syncthreads();
-    float t = 0.0f;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < 8; ++w) t += part[w];
-    ce_finish(t, partial, counters, rows_per_member, loss_mean);
+    ce_finish(rr, acc, partial, counters, rows_per_member, loss_mean);
 }
 
 __global__ void ce_finalize_kernel(const float* __restrict__ partial, int members, int rows_per_member, float* __restrict__ loss_mean) {
@@ -837,8 +880,11 @@ int get_scratch(size_t floats, float** out) {
 }  // namespace
 
 int cross_entropy_launch(const float* logits, int ld, const float* bias, const int8_t* bias_noise, float sigma, const uint8_t* targets, int vocab, int members,
-                         int rows_per_member, int chunks, float* partial, unsigned* counters, float* loss_mean, cudaStream_t st) {
-    const dim3 grid(chunks, members);
+                         int rows_per_member, float* partial, unsigned* counters, float* loss_mean, cudaStream_t st) {
+    // few members (a validation pass has one): more blocks per member as long as the SMs are not filled and a warp keeps eight rows. Same bits.
+    int split = 1;
+    while (counters != nullptr && split < 4 && members * kCeChunks * split < 2 * 148 && rows_per_member >= 2 * split * 1024) split *= 2;
+    const dim3 grid(kCeChunks * split, members);
     const bool early = static_cast<long long>(members) * rows_per_member * vocab <= kPdlStreamElems;
     const bool vec = (vocab % 4) == 0 && (ld % 4) == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(bias_noise) & 3) == 0;
@@ -1008,7 +1054,7 @@ int bnf4_cross_entropy_population(const float* logits, int ld, const float* bias
     if (!logits || !targets || !partial || !loss_mean) return set_error(BNF4_ERR_INVALID, "cross_entropy_population: null pointer");
     if (vocab <= 0 || vocab > 32 * kCeMaxPerLane) return set_error(BNF4_ERR_INVALID, "cross_entropy_population: vocab=%d", vocab);
     if (members > 65535) return set_error(BNF4_ERR_INVALID, "cross_entropy_population: at most 65535 members per call");
-    int rc = cross_entropy_launch(logits, ld, bias, bias_noise, sigma, targets, vocab, members, rows_per_member, kCeChunks, partial, nullptr, loss_mean, S(stream));
+    int rc = cross_entropy_launch(logits, ld, bias, bias_noise, sigma, targets, vocab, members, rows_per_member, partial, nullptr, loss_mean, S(stream));
     if (rc) return rc;
     launch_pdl(ce_finalize_kernel, (members + 127) / 128, 128, 0, S(stream), partial, members, rows_per_member, loss_mean);
     return check_launch("ce_finalize_kernel");

@@ -154,10 +154,11 @@ int z_dense_table_launch(const float* pair_weights, const uint64_t* pair_seeds, 
 bool shape_fitness_applies(int pairs, int mode);
 int shape_fitness_launch(const float* losses, int pairs, int mode, float clip, float* weights, cudaStream_t stream);
 
-// Mean cross-entropy of every member, `chunks` blocks per member (es_kernels.cu). partial: members * chunks floats. counters: one zeroed word per
-// member, zero again afterwards; nullptr: the partials only.
+// Mean cross-entropy of every member (es_kernels.cu). partial: kCePartials floats per member (16 without counters). counters: one zeroed word per
+// member, zero again afterwards; nullptr: the 16 group sums of every member only.
+constexpr int kCePartials = 128;
 int cross_entropy_launch(const float* logits, int ld, const float* bias, const int8_t* bias_noise, float sigma, const uint8_t* targets, int vocab, int members,
-                         int rows_per_member, int chunks, float* partial, unsigned* counters, float* loss_mean, cudaStream_t stream);
+                         int rows_per_member, float* partial, unsigned* counters, float* loss_mean, cudaStream_t stream);
 
 void count_launch();
 

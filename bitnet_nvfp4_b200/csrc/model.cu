@@ -169,7 +169,6 @@ struct Model {
     uint8_t *a_h, *sf_h, *a_f, *sf_f;
     float *qkv, *y, *ce_partial, *losses;
     unsigned* ce_count;  // arrivals of a member's cross-entropy blocks
-    int ce_chunks = 16;  // of a member's rows: a function of their number only, so that losses do not depend on the wave
     // input stage computed once per (member, distinct token) when the vocabulary is smaller than a member's rows
     bool dedup_input = false;
     uint8_t *tok_ident, *emb_a, *emb_sf;
@@ -466,7 +465,7 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
     TRY(gemm(KC_GEMM_HEAD, m.a_h, m.sf_h, m.q_head, m.sfq_head, V, H, m.s_h, m.qkv, V, m.A_head + P0 * V * r, static_cast<long long>(V) * r, m.t_a, r, m.s_h, 0, m.dense ? m.nz_head : no_noise));
     ++launches;
     TimedScope ts_ce(m, KC_CROSS_ENTROPY, st, 1);
-    TRY(cross_entropy_launch(m.qkv, V, m.head_bias, pert ? m.hb_noise + P0 * V : nullptr, sigma, m.targets, V, nm, R, m.ce_chunks, m.ce_partial, m.ce_count,
+    TRY(cross_entropy_launch(m.qkv, V, m.head_bias, pert ? m.hb_noise + P0 * V : nullptr, sigma, m.targets, V, nm, R, m.ce_partial, m.ce_count,
                              losses_out, st));
     ++launches;
     m.launches_per_wave = launches;
@@ -678,7 +677,7 @@ int run_pair_dense(Model& m, int pair, float* losses_out, cudaStream_t st) {
     }
     TRY(noisy(KC_GEMM_HEAD, m.a_h, m.sf_h, H, m.q_head, m.sfq_head, m.qe_head, m.sfe_head, V, m.s_h, m.qkv, V));
     TimedScope ts_ce(m, KC_CROSS_ENTROPY, st, 1);
-    return cross_entropy_launch(m.qkv, V, m.head_bias, m.hb_noise + static_cast<size_t>(pair) * V, sigma, m.targets, V, 2, R, m.ce_chunks, m.ce_partial, m.ce_count,
+    return cross_entropy_launch(m.qkv, V, m.head_bias, m.hb_noise + static_cast<size_t>(pair) * V, sigma, m.targets, V, 2, R, m.ce_partial, m.ce_count,
                                 losses_out, st);
 }
 
@@ -925,8 +924,6 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
     m->M = static_cast<long long>(W) * m->R;
     if (m->M > 0x7fffffffLL / 8) { delete m; return set_error(BNF4_ERR_INVALID, "model_create: wave of %d members is too large", W); }
 
-    // one block of eight warps per 128 rows of a member, 16 to 64 blocks: a validation pass has one member only
-    m->ce_chunks = std::min(64, std::max(16, m->R / 128));
     const int V = m->V, H = m->H, F = m->F, L = m->L, T = m->T, r = m->r, P = cfg->max_pairs;
     const size_t hh = static_cast<size_t>(H) * H, hf = static_cast<size_t>(H) * F;
     int rc = 0;
@@ -961,7 +958,7 @@ int bnf4_model_create(const bnf4_model_cfg* cfg, void** handle) {
         A_(tok_ident, V); A_(emb_a, Er * H / 2); A_(emb_sf, sf_bytes(static_cast<int>(Er), H)); A_(emb_t, Er * r); A_(y_emb, Er * H);
     }
     // the logits (V columns) share the q | k | v | beta buffer: a model narrower than its vocabulary needs the wider of the two
-    A_(qkv, Mr * std::max(m->FC, V)); A_(y, Mr * H); A_(ce_partial, static_cast<size_t>(W) * m->ce_chunks); A_(ce_count, W); A_(losses, W);
+    A_(qkv, Mr * std::max(m->FC, V)); A_(y, Mr * H); A_(ce_partial, static_cast<size_t>(W) * kCePartials); A_(ce_count, W); A_(losses, W);
     A_(t_a, Mr * 4 * r); A_(t_f, Mr * r);
     if (m->dense_folded) {
         A_(E_all, static_cast<size_t>(W / 2) * V * H);  // the embedding's noise
