@@ -187,6 +187,8 @@ struct Model {
     int launches_per_wave = 0;
     float* h_step = nullptr;    // bnf4_model_es_step: pinned losses [2 * max_pairs] + pair weights [max_pairs]
     float* d_step_w;            // ... and the shaped pair weights on the device
+    cudaEvent_t tokens_read = nullptr;  // behind the copy of a batch out of pinned host memory
+    bool tokens_pending = false;        // bnf4_model_es_step has to wait for it
     // dense (rank 0) mode: the reference driver's own perturbation, one materialised noise matrix per weight matrix and pair,
     // applied as a second GEMM with beta = 1 (src/train_efla_lm.cpp:2359-2367). One pair per wave.
     // dense_folded (sigma down to 2^-4): any number of pairs per wave; the noise operands of every member follow the base weights in the
@@ -872,6 +874,7 @@ int bnf4_model_destroy(void* handle) {
     if (m->cap_stream) cudaStreamDestroy(m->cap_stream);
     for (void* p : m->allocs) cudaFree(p);
     if (m->h_step) cudaFreeHost(m->h_step);
+    if (m->tokens_read) cudaEventDestroy(m->tokens_read);
     for (cudaEvent_t e : m->free_events) cudaEventDestroy(e);
     for (const Model::Span& sp : m->spans) { cudaEventDestroy(sp.a); cudaEventDestroy(sp.b); }
     delete m;
@@ -1176,11 +1179,20 @@ int bnf4_model_set_tokens(void* handle, const uint8_t* tokens, const uint8_t* ta
     const uint8_t *dt = device_address(tokens), *dg = device_address(targets);
     if (dt != nullptr && dg != nullptr) {
         launch_pdl(copy_tokens_kernel, dim3((m.R + 4095) / 4096, 2), 256, 0, S(stream), dt, dg, m.R, m.tokens, m.targets);
-        return check_launch("copy_tokens_kernel");
+        TRY(check_launch("copy_tokens_kernel"));
+    } else {
+        const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+        TRY(check_cuda(cudaMemcpyAsync(m.tokens, tokens, m.R, kind, S(stream)), "cudaMemcpyAsync(tokens)"));
+        TRY(check_cuda(cudaMemcpyAsync(m.targets, targets, m.R, kind, S(stream)), "cudaMemcpyAsync(targets)"));
     }
-    const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    TRY(check_cuda(cudaMemcpyAsync(m.tokens, tokens, m.R, kind, S(stream)), "cudaMemcpyAsync(tokens)"));
-    return check_cuda(cudaMemcpyAsync(m.targets, targets, m.R, kind, S(stream)), "cudaMemcpyAsync(targets)");
+    if (on_device) return BNF4_OK;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    TRY(check_cuda(cudaStreamIsCapturing(S(stream), &capturing), "cudaStreamIsCapturing"));
+    if (capturing != cudaStreamCaptureStatusNone) return BNF4_OK;  // (a captured copy reads the buffer at every replay)
+    if (m.tokens_read == nullptr) TRY(check_cuda(cudaEventCreateWithFlags(&m.tokens_read, cudaEventDisableTiming), "cudaEventCreate(tokens)"));
+    TRY(check_cuda(cudaEventRecord(m.tokens_read, S(stream)), "cudaEventRecord(tokens)"));
+    m.tokens_pending = true;
+    return BNF4_OK;
 }
 
 int bnf4_model_prepare_step_range(void* handle, uint64_t seed, uint64_t epoch, int pairs, int eval_begin, int eval_count, void* stream) {
@@ -1295,7 +1307,7 @@ int bnf4_model_update_apply(void* handle, const float* pair_weights, const float
     return update_apply(m, pair_weights, z_all, u, S(stream));
 }
 
-int bnf4_model_es_step(void* handle, const bnf4_es_step_cfg* cfg, const bnf4_collectives* coll, float* d_losses_all, void* stream) {
+static int es_step(void* handle, const bnf4_es_step_cfg* cfg, const bnf4_collectives* coll, float* d_losses_all, void* stream) {
     if (!handle || !cfg || !d_losses_all) return set_error(BNF4_ERR_INVALID, "model_es_step: null argument");
     Model& m = *M(handle);
     const int world = cfg->world, rank = cfg->rank, pairs = cfg->pairs;
@@ -1343,6 +1355,19 @@ int bnf4_model_es_step(void* handle, const bnf4_es_step_cfg* cfg, const bnf4_col
     if (coll->group_end && coll->group_end(coll->ctx) != 0) failed = 1;
     if (failed) return set_error(BNF4_ERR_CUDA, "model_es_step: the all-gather of the noise sums failed");
     return update_apply(m, m.d_step_w, m.Z_all, &cfg->update, st);
+}
+
+int bnf4_model_es_step(void* handle, const bnf4_es_step_cfg* cfg, const bnf4_collectives* coll, float* d_losses_all, void* stream) {
+    const int rc = es_step(handle, cfg, coll, d_losses_all, stream);
+    if (!handle) return rc;
+    // The caller may refill the batch's host buffers after the step: a copy out of pinned memory that is still queued has to have read them.
+    // It is the first thing the step queued, so the wait costs the GPU nothing.
+    Model& m = *M(handle);
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (!m.tokens_pending || cudaStreamIsCapturing(S(stream), &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return rc;
+    m.tokens_pending = false;
+    const int rc2 = check_cuda(cudaEventSynchronize(m.tokens_read), "cudaEventSynchronize(tokens)");
+    return rc ? rc : rc2;
 }
 
 int bnf4_model_set_timing(void* handle, int enable) {

@@ -222,7 +222,8 @@ class PopulationModel:
         return int(z["epoch"])
 
     def set_tokens(self, tokens, targets):
-        """tokens/targets: uint8 [B][T], torch CUDA tensors or (pinned) host tensors / numpy arrays."""
+        """tokens/targets: uint8 [B][T], torch CUDA tensors or (pinned) host tensors / numpy arrays. Pinned tensors are read when the current stream
+        gets there: they may be refilled after the next es_step, or after the stream has been waited for."""
         def ptr(x):
             if isinstance(x, torch.Tensor):
                 assert x.dtype == torch.uint8 and x.is_contiguous()
@@ -233,6 +234,7 @@ class PopulationModel:
         (pt, dt), (pg, dg) = ptr(tokens), ptr(targets)
         assert dt == dg
         _l.check(self.lib.bnf4_model_set_tokens(self.h, pt, pg, int(dt), _stream()))
+        self._batch = None if dt else (tokens, targets)  # (a pinned block that is let go may be handed out again before it has been read)
         if getattr(self, "_keep", None):
             # numpy inputs were copied to temporaries: wait for the H2D copies before releasing them
             torch.cuda.current_stream().synchronize()

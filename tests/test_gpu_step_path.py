@@ -103,3 +103,30 @@ def test_dense_noise_in_one_product(kw):
             ref = om.forward(tok, tgt, orc.mix(1, orc.mix(3, p)), anti)
             assert abs(losses[2 * p + s] - ref) <= 1e-4 * abs(ref), (p, anti)
     assert np.array_equal(m.eval_pairs(1, pairs - 1).cpu().numpy(), losses[2:])
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_a_pinned_batch_may_be_refilled_after_the_step(native):
+    """The device is busy when the batch is set, so its copy is still queued when the host gets to the next one."""
+    import torch
+    from bitnet_nvfp4_b200 import population, synth
+    busy = torch.randn(8192, 8192, device="cuda", dtype=torch.bfloat16)
+    batches = [synth.sample_batch(synth.zipf_corpus(1 << 14, 1.1, 5), SMALL["batch"], SMALL["seq"], 20 + e) for e in range(4)]
+    results = []
+    for refill in (False, True):
+        _, _, _, _, m = make(max_pairs=6, **SMALL)
+        tok, tgt = (torch.empty(SMALL["batch"], SMALL["seq"], dtype=torch.uint8, pin_memory=True) for _ in range(2))
+        losses = []
+        for e, (a, b) in enumerate(batches):
+            tok.copy_(torch.from_numpy(a))
+            tgt.copy_(torch.from_numpy(b))
+            if refill:
+                for _ in range(40):
+                    torch.mm(busy, busy)
+            m.set_tokens(tok, tgt)
+            losses.append((population.es_step_native if native else population.es_step)(m, 5, e, 6))
+            if not refill:
+                torch.cuda.synchronize()
+        results.append([x.cpu().numpy() for x in losses] + state(m))
+    for a, b in zip(*results):
+        assert np.array_equal(a, b)
