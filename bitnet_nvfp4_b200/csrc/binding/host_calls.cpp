@@ -263,7 +263,11 @@ ENTRY(efla_step_half) {  // S, qkv, fused_cols, beta_bias, hidden, batch, method
     const float bias = x.real();
     const int hidden = x.integer(), batch = x.integer(), method = x.integer();
     const float eps = x.real();
-    at::Tensor out = empty_like_device(qkv, {batch, hidden}, qkv.scalar_type());
+    if (at::isFloatingType(qkv.scalar_type()) && qkv.scalar_type() != at::kFloat) {  // (raw bytes of floats are a caller's business)
+        PyErr_Format(PyExc_TypeError, "qkv must be float32, not %s", at::toString(qkv.scalar_type()));
+        throw Failed{};
+    }
+    at::Tensor out = empty_like_device(qkv, {batch, hidden}, at::kFloat);
     void *in = qkv.data_ptr(), *o = out.data_ptr(), *s = raw_stream();
     call([&] { return bnf4_efla_step_half_qkv_fused(as<uint16_t>(S), as<float>(in), fused, bias, hidden, batch, method, eps, as<float>(o), s); });
     return THPVariable_Wrap(std::move(out));

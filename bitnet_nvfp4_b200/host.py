@@ -200,7 +200,9 @@ def efla_step_half_qkv_fused(S, qkv, fused_cols, beta_bias, hidden, batch, metho
 
 
 def efla_step_qkv_fused(S, qkv, fused_cols, beta_bias, hidden, batch, method, eps):
-    out = qkv.new_empty((batch, hidden))
+    if qkv.is_floating_point() and qkv.dtype != torch.float32:
+        raise TypeError(f"qkv must be float32, not {qkv.dtype}")
+    out = qkv.new_empty((batch, hidden), dtype=torch.float32)
     _l.check(_l.load().bnf4_efla_step_qkv_fused(_p(S), _p(qkv), fused_cols, beta_bias, hidden, batch, method, eps, _p(out),
                                                 _stream()))
     return out

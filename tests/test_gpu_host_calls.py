@@ -88,3 +88,20 @@ def test_threads_use_their_own_streams(H):
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not bad
+
+
+@pytest.mark.parametrize("state_half", [True, False])
+def test_single_step_output_is_fp32_whatever_holds_the_inputs(H, state_half):
+    """The kernel writes 4 * batch * hidden bytes. Halves, which it would read as floats, are refused; raw bytes of floats are taken."""
+    import torch
+    step = H.efla_step_half_qkv_fused if state_half else H.efla_step_qkv_fused
+    qkv = torch.randn(4, 3 * 64 + 32, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2))
+    def state():
+        return torch.zeros(4, 64, 64, dtype=torch.float16 if state_half else torch.float32, device="cuda")
+    want = step(state(), qkv, 224, -2.0, 64, 4, 1, 1e-6)
+    for raw in (qkv.view(torch.uint8), qkv.view(torch.int32)):
+        got = step(state(), raw, 224, -2.0, 64, 4, 1, 1e-6)
+        assert got.dtype == torch.float32 and torch.equal(got, want)
+    for dt in (torch.float16, torch.bfloat16, torch.float64):
+        with pytest.raises(TypeError):
+            step(state(), qkv.to(dt), 224, -2.0, 64, 4, 1, 1e-6)
