@@ -40,3 +40,27 @@ def test_more_than_four_projections(rows, hid, nvec, rpm):
     got = t.cpu().numpy()
     assert np.array_equal(got[:rows], ref)
     assert (got[rows] == -7).all()
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+@pytest.mark.parametrize("scale", [1.0, 0.8, 1000.0])
+def test_non_finite_activations_do_not_depend_on_alignment(mode, scale):
+    """Rows on a 16-byte boundary take the vectorised kernel, others the general one; NaN becomes 0 in both."""
+    import torch
+    from bitnet_nvfp4_b200 import host
+    rows, cols = 40, 512
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(rows, cols, device="cuda", generator=g) * 3
+    special = torch.tensor([float("nan"), float("inf"), float("-inf"), 3e38, -3e38, 1e-40, -0.0, float("nan")], device="cuda")
+    at = torch.randperm(rows * cols, device="cuda", generator=g)[:400]
+    x.view(-1)[at] = special[torch.arange(400, device="cuda") % 8]
+    buf = torch.empty(rows * cols + 1, device="cuda")
+    buf[1:] = x.view(-1)
+    outs = []
+    for t in (x, buf[1:].view(rows, cols)):
+        q = torch.empty(rows, cols, dtype=torch.int8, device="cuda")
+        codes, sf = torch.zeros(host.matrix_bytes(rows, cols), dtype=torch.uint8, device="cuda"), torch.zeros(host.sf_bytes(rows, cols), dtype=torch.uint8, device="cuda")
+        host.rowquant(host.FE_ACT, rows=rows, cols_in=cols, cols_out=cols, in_f32=t, ld_in=cols, act_mode=mode, act_scale=scale, out_q=q, ld_q=cols, out_codes=codes, out_sf=sf)
+        outs.append((q, codes, sf))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+    assert not outs[0][0].view(-1)[at][torch.arange(400, device="cuda") % 8 == 0].any()
