@@ -74,7 +74,7 @@ template <> struct StatePiece<float> {
 };
 
 template <typename ST, int NPC, int NI>
-__global__ void __launch_bounds__(kGenThreads, (NPC == 4 && NI == 8 ? 3 : NI <= 16 ? 2 : 1)) efla_generic_kernel(const EflaParams p) {
+__global__ void __launch_bounds__(kGenThreads, (NI <= 16 ? 2 : 1)) efla_generic_kernel(const EflaParams p) {
     pdl_wait();
     constexpr int PN = StatePiece<ST>::N;       // columns per piece
     constexpr int NC = NPC * PN;                // columns per CTA
@@ -394,8 +394,6 @@ int launch_head32(const EflaParams& p, cudaStream_t stream) {
 
 // Split of a head's state: 128-byte row segments (NPC = 8) while a thread's share of the rows fits 16 registers quads and the
 // segment divides the row; 64-byte segments (half the columns, twice the row groups) beyond. NI follows from the width.
-// Few sequences of wide heads take 64-byte segments too, as long as each of the twice as many CTAs has an SM of its own: one token of 8 sequences with a 512 x 512
-// state 6.3 -> 5.1 us (16 sequences, where it does not, 6.4 -> 6.5 us; 32: 9.0 -> 12.0 us).
 template <typename ST>
 int launch_generic_for(const EflaParams& p, cudaStream_t stream) {
     const int hd = p.hidden / p.heads;
@@ -403,10 +401,6 @@ int launch_generic_for(const EflaParams& p, cudaStream_t stream) {
     if (hd <= 512 && (hd % (8 * StatePiece<ST>::N)) == 0) {
         if (hd <= 128) return launch_generic<ST, 8, 4>(p, stream);
         if (hd <= 256) return launch_generic<ST, 8, 8>(p, stream);
-        int dev = 0;
-        const int rc = current_device(&dev);
-        if (rc) return rc;
-        if (2 * p.seqs * p.heads * (hd / (8 * StatePiece<ST>::N)) <= multiprocessors(dev)) return launch_generic<ST, 4, 8>(p, stream);
         return launch_generic<ST, 8, 16>(p, stream);
     }
     if (hd <= 256) return launch_generic<ST, 4, 4>(p, stream);
