@@ -50,9 +50,8 @@ constexpr int kSqDiag = 2 * kSqStage;                            // fp32 diagona
 constexpr int kSqInv = kSqDiag + 8 * 16 * 17 * 4;                // their inverses, hi and mid [2][8][16][kSqTStride]
 constexpr int kSqScal = kSqInv + 2 * 8 * 16 * kSqTStride * 2;    // q scale, k scale, a, b [4][128] floats
 constexpr int kSqRed = kSqScal + 4 * kSeqMaxT * 4;               // reduction scratch [2][16] + broadcast
-constexpr int kSqPart = kSqRed + 256;                            // a CTA's share of the squared norms [2][128] floats (read by its cluster)
+constexpr int kSqPart = kSqRed + 256;                            // squared norms of a CTA's tokens [2][128] floats (read by its cluster)
 constexpr int kSqSmem = kSqPart + 2 * kSeqMaxT * 4;
-static_assert(48 * kSeqThreads * 4 <= 2 * kSqStage, "the exchanged accumulators fit the stages");
 static_assert(2 * kSeqMaxT * kSqLStride * 2 <= kSqStage && kSeqMaxT * kSqXStride * 4 <= kSqStage && 4 * kSqTile <= kSqStage, "overlaid regions");
 static_assert(kSqDiag % 16 == 0 && kSqInv % 16 == 0 && kSqScal % 16 == 0, "16-byte aligned regions");
 constexpr float kSqUp = 256.0f;                    // power-of-two scale of every normalised operand
@@ -194,6 +193,7 @@ __device__ __forceinline__ void seq_solve_rows(uint32_t sm0, uint32_t mat_off, u
 
 template <int CS>
 __device__ __forceinline__ void sq_cluster_sync() {
+    if constexpr (CS > 1) __syncwarp();
     if constexpr (CS > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // the float at this shared-memory address in CTA `rank` of the cluster
@@ -205,8 +205,18 @@ __device__ __forceinline__ float sq_remote(uint32_t addr, int rank) {
     return v;
 }
 
-// CS CTAs of a cluster share a unit: each takes its share of the 64-column blocks in steps 1, 2 (partial sums, exchanged through distributed
-// shared memory and added in rank order, so all hold the same bits) and 5; steps 3 and 4 are done by every one of them.
+// the 16 bytes at this shared-memory address in CTA `rank` of the cluster
+__device__ __forceinline__ uint4 sq_remote16(uint32_t addr, int rank) {
+    uint32_t a;
+    uint4 v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
+
+// CS CTAs of a cluster share a unit. No sum is split: a CTA takes some of the tokens in step 1, some of the 16-row blocks of G and X in step 2 (all of
+// K, its own rows of Q; finished rows are exchanged through distributed shared memory) and some of the 64-column blocks in step 5; steps 3
+// and 4 are done by every one. Every CS gives the same bits, so a sequence's outputs do not depend on how many share the launch.
 template <int CS>
 __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaParams p) {
     pdl_wait();
@@ -235,12 +245,12 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
 
     // ---------------- 1. norms and scalars ----------------
-    for (int t = warp; t < kSeqMaxT; t += 16) {
+    for (int t = warp * CS + rank; t < kSeqMaxT; t += 16 * CS) {
         float qss = 0.0f, kss = 0.0f;
         if (t < T) {
             const float4* q4 = reinterpret_cast<const float4*>(qg + static_cast<size_t>(t) * p.ld_qkv);
             const float4* k4 = reinterpret_cast<const float4*>(kg + static_cast<size_t>(t) * p.ld_qkv);
-            for (int i = 16 * db0 + lane; i < min(hd >> 2, 16 * db1); i += 32) {
+            for (int i = lane; i < (hd >> 2); i += 32) {
                 const float4 a = q4[i], b = k4[i];
                 qss = fmaf(a.x, a.x, qss); qss = fmaf(a.y, a.y, qss); qss = fmaf(a.z, a.z, qss); qss = fmaf(a.w, a.w, qss);
                 kss = fmaf(b.x, b.x, kss); kss = fmaf(b.y, b.y, kss); kss = fmaf(b.z, b.z, kss); kss = fmaf(b.w, b.w, kss);
@@ -256,11 +266,8 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         const int t = tid;
         float qss = 0.0f, kss = 0.0f;
         if constexpr (CS > 1) {
-#pragma unroll
-            for (int r = 0; r < CS; ++r) {
-                qss += sq_remote(sm0 + kSqPart + t * 4, r);
-                kss += sq_remote(sm0 + kSqPart + (kSeqMaxT + t) * 4, r);
-            }
+            qss = sq_remote(sm0 + kSqPart + t * 4, t % CS);
+            kss = sq_remote(sm0 + kSqPart + (kSeqMaxT + t) * 4, t % CS);
         } else {
             qss = part[t];
             kss = part[kSeqMaxT + t];
@@ -283,13 +290,15 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     const float bscale = sq_pow2_scale(fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]))) * (1.0f / kSqUp);  // b * bscale <= 1
 
     // ---------------- 2. G and X ----------------
-    const int pr = warp & 3, which = (warp >> 2) & 1, half = warp >> 3;
-    const int r1 = pr, r2 = nb - 1 - pr;  // this warp's row blocks (r1 < r2: both; equal: one; r1 > r2: none)
-    float acc1[4][4], acc2[8][4];
+    const int pr = rank + CS * ((warp & 3) % (4 / CS)), which = (warp >> 2) & 1, half = warp >> 3;
+    const int jq = (warp & 3) / (4 / CS);  // column blocks jq, jq + CS, ..
+    const int r1 = pr, r2 = nb - 1 - pr;   // this warp's row blocks (r1 < r2: both; equal: one; r1 > r2: none)
+    auto owner = [&](int block) { return min(block, nb - 1 - block) % CS; };  // the CTA that forms this row block
+    float acc1[4 / CS][4], acc2[8 / CS][4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 8 / CS; ++j)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) { acc2[j][i] = 0.0f; if (j < 4) acc1[j][i] = 0.0f; }
+        for (int i = 0; i < 4; ++i) { acc2[j][i] = 0.0f; if (j < 4 / CS) acc1[j % (4 / CS)][i] = 0.0f; }
 
     // staging: thread = (16-byte piece of a 64-column row block, row); four rows of K and of Q per thread
     const int piece = tid & 15, srow = tid >> 4;
@@ -301,7 +310,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
             kr[i] = qr[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (t < T && c < hd) {
                 kr[i] = *reinterpret_cast<const float4*>(kg + static_cast<size_t>(t) * p.ld_qkv + c);
-                qr[i] = *reinterpret_cast<const float4*>(qg + static_cast<size_t>(t) * p.ld_qkv + c);
+                if (CS == 1 || owner(t >> 4) == rank) qr[i] = *reinterpret_cast<const float4*>(qg + static_cast<size_t>(t) * p.ld_qkv + c);
             }
         }
     };
@@ -317,6 +326,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
             sq_split(kr[i].z * ks, kr[i].w * ks, hi.y, mid.y);
             *reinterpret_cast<uint2*>(st + o) = hi;
             *reinterpret_cast<uint2*>(st + kSqTile + o) = mid;
+            if (CS > 1 && owner(t >> 4) != rank) continue;
             sq_split(qr[i].x * qs, qr[i].y * qs, hi.x, mid.x);
             sq_split(qr[i].z * qs, qr[i].w * qs, hi.y, mid.y);
             *reinterpret_cast<uint2*>(st + 2 * kSqTile + o) = hi;
@@ -326,12 +336,12 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     // ldmatrix addresses inside a stage: A rows (lane % 16, column half lane / 16); B: eight K rows, matrices (hi, k 0-7), (hi, 8-15), (mid, ..), (mid, ..)
     const uint32_t a_off = static_cast<uint32_t>((lane & 15) * kSqStride + (lane >> 4) * 8) * 2u + (which ? 2u * kSqTile : 0u);
     const uint32_t b_off = static_cast<uint32_t>((half * 8 + (lane & 7)) * kSqStride + ((lane >> 3) & 1) * 8) * 2u + (lane >> 4) * static_cast<uint32_t>(kSqTile);
-    load_block(db0 * 64);
+    load_block(0);
     store_block(0);
     __syncthreads();
-    for (int db = db0; db < db1; ++db) {
-        if (db + 1 < db1) load_block((db + 1) * 64);
-        const uint32_t st = sm0 + ((db - db0) & 1) * kSqStage;
+    for (int db = 0; db < nd; ++db) {
+        if (db + 1 < nd) load_block((db + 1) * 64);
+        const uint32_t st = sm0 + (db & 1) * kSqStage;
         const int nk = min(4, (hd - db * 64) >> 4);
         if (r1 <= r2) {
             for (int kk = 0; kk < nk; ++kk) {
@@ -342,52 +352,24 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
                 sq_ldm(ah1, ab + r1 * (16 * kSqStride * 2));
                 sq_ldm(am1, ab + r1 * (16 * kSqStride * 2) + kSqTile);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int jj = 0; jj < 8 / CS; ++jj) {
+                    const int j = jq + CS * jj;
+                    constexpr int N1 = 4 / CS;
                     if (j <= r2) {
                         uint32_t b[4];
                         sq_ldm(b, st + b_off + kk * 32 + j * (16 * kSqStride * 2));
-                        sq_mma(acc2[j], ah2, b[0], b[1]);
-                        if (j < 4 && j <= r1) sq_mma(acc1[j & 3], ah1, b[0], b[1]);
-                        sq_mma(acc2[j], ah2, b[2], b[3]);
-                        if (j < 4 && j <= r1) sq_mma(acc1[j & 3], ah1, b[2], b[3]);
-                        sq_mma(acc2[j], am2, b[0], b[1]);
-                        if (j < 4 && j <= r1) sq_mma(acc1[j & 3], am1, b[0], b[1]);
+                        sq_mma(acc2[jj], ah2, b[0], b[1]);
+                        if (jj < N1 && j <= r1) sq_mma(acc1[jj % N1], ah1, b[0], b[1]);
+                        sq_mma(acc2[jj], ah2, b[2], b[3]);
+                        if (jj < N1 && j <= r1) sq_mma(acc1[jj % N1], ah1, b[2], b[3]);
+                        sq_mma(acc2[jj], am2, b[0], b[1]);
+                        if (jj < N1 && j <= r1) sq_mma(acc1[jj % N1], am1, b[0], b[1]);
                     }
                 }
             }
         }
-        if (db + 1 < db1) store_block((db + 1 - db0) & 1);
+        if (db + 1 < nd) store_block((db + 1) & 1);
         __syncthreads();
-    }
-    if constexpr (CS > 1) {  // the partial sums of all CTAs, thread by thread
-        float* ex = reinterpret_cast<float*>(sm) + tid;
-        const uint32_t exa = sm0 + tid * 4;
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (j <= r2) ex[(j * 4 + i) * kSeqThreads] = acc2[j][i];
-                if (j < 4 && j <= r1) ex[(32 + (j & 3) * 4 + i) * kSeqThreads] = acc1[j & 3][i];
-            }
-        sq_cluster_sync<CS>();
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (j <= r2) {
-                    float x = 0.0f;
-#pragma unroll
-                    for (int r = 0; r < CS; ++r) x += sq_remote(exa + (j * 4 + i) * (kSeqThreads * 4), r);
-                    acc2[j][i] = x;
-                }
-                if (j < 4 && j <= r1) {
-                    float x = 0.0f;
-#pragma unroll
-                    for (int r = 0; r < CS; ++r) x += sq_remote(exa + (32 + (j & 3) * 4 + i) * (kSeqThreads * 4), r);
-                    acc1[j & 3][i] = x;
-                }
-            }
-        sq_cluster_sync<CS>();  // everyone has read: the stages are free again (and nobody's shared memory is read from here on)
     }
 
     // ---------------- 3. L (two halves, stage 0), its diagonal blocks (fp32), X (fp32, stage 1) ----------------
@@ -422,11 +404,29 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         }
     };
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        if (r1 <= r2 && j <= r2) put_tile(acc2[j], r2, j);
-        if (j < 4 && r1 < r2 && j <= r1) put_tile(acc1[j & 3], r1, j);
+    for (int jj = 0; jj < 8 / CS; ++jj) {
+        const int j = jq + CS * jj;
+        if (r1 <= r2 && j <= r2) put_tile(acc2[jj], r2, j);
+        if (jj < 4 / CS && r1 < r2 && j <= r1) put_tile(acc1[jj % (4 / CS)], r1, j);
     }
-    __syncthreads();
+    if constexpr (CS > 1) {  // the other CTAs' rows: L hi and mid, X up to the diagonal block, and that block
+        sq_cluster_sync<CS>();
+        for (int t = warp; t < 16 * nb; t += 16) {
+            const int blk = t >> 4, o = owner(blk);
+            if (o == rank) continue;
+            const int n2 = 2 * (blk + 1);  // 16-byte pieces of a row of halves
+            for (int i = lane; i < 4 * n2; i += 32) {
+                const uint32_t at = i < n2 ? (t * kSqLStride) * 2 + i * 16 : i < 2 * n2 ? ((kSeqMaxT + t) * kSqLStride) * 2 + (i - n2) * 16
+                                                                                         : kSqStage + (t * kSqXStride) * 4 + (i - 2 * n2) * 16;
+                *reinterpret_cast<uint4*>(sm + at) = sq_remote16(sm0 + at, o);
+            }
+        }
+        for (int i = tid; i < nb * 68; i += kSeqThreads) {  // 16 x 17 floats a block
+            const int o = owner(i / 68);
+            if (o != rank) *reinterpret_cast<uint4*>(sm + kSqDiag + i * 16) = sq_remote16(sm0 + kSqDiag + i * 16, o);
+        }
+        sq_cluster_sync<CS>();  // everyone has read (and nobody's shared memory is read from here on)
+    } else __syncthreads();
     // inverse of I + L_ii: lane c owns column c of a block, two blocks per warp
     seq_invert_diagonal(Ld, reinterpret_cast<__half*>(sm + kSqInv), nb, warp, lane);
     __syncthreads();

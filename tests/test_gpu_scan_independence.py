@@ -22,3 +22,31 @@ def bits_of_groups(H, hidden, heads, seqs, T, method, variant, groups):
 @pytest.mark.parametrize("hidden,heads,method", [(512, 1, 1), (1024, 2, 0), (320, 1, 1), (96, 1, 1), (1280, 1, 0)])
 def test_per_token_kernel(H, hidden, heads, method):
     bits_of_groups(H, hidden, heads, 48, 5, method, 1, [(0, 1), (3, 8), (17, 19)])
+
+
+# clusters of four, two and one CTA per (sequence, head), for every number of 16-token blocks
+@pytest.mark.parametrize("hidden,heads,seqs,groups", [(512, 1, 160, [(0, 1), (5, 30), (40, 60)]), (320, 2, 90, [(3, 2), (10, 35)]), (96, 1, 160, [(7, 3)])])
+@pytest.mark.parametrize("T", [1, 16, 17, 40, 64, 77, 96, 100, 128])
+def test_closed_form(H, hidden, heads, seqs, groups, T):
+    bits_of_groups(H, hidden, heads, seqs, T, T % 2, 0, groups)
+
+
+@pytest.mark.parametrize("hidden,heads,method", [(96, 1, 1), (512, 8, 1), (128, 4, 0)])
+def test_other_scans(H, hidden, heads, method):
+    """One CTA (128-token blocks) or one warp per unit, whatever their number."""
+    bits_of_groups(H, hidden, heads, 40, 130, method, 0, [(0, 1), (11, 20)])
+
+
+def test_losses_of_a_population_do_not_depend_on_the_wave():
+    """Wide heads: 2, 6 and 18 members a wave take clusters of four, of two and single CTAs."""
+    import torch
+    from bitnet_nvfp4_b200 import population, synth
+    out = []
+    for wave in (2, 6, 18):
+        cfg = population.Config(hidden=256, heads=1, layers=1, seq=40, batch=9, max_pairs=9, wave_members=wave)
+        model = population.PopulationModel(cfg)
+        model.set_weights(synth.init_weights(cfg))
+        model.set_tokens(*synth.sample_batch(synth.zipf_corpus(1 << 14, 1.1, 123), 9, 40, 7))
+        model.prepare_step(3, 1, 9)
+        out.append(model.eval_pairs(0, 9))
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
