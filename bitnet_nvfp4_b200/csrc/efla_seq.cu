@@ -833,8 +833,9 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
 
 // The closed form's work per token grows with the sequence, the per-token kernel's does not, but the latter spreads a unit over several SMs. One head of
 // 512: 322 tokens 0.69 / 1.16 ms (closed form / per token) for 4 sequences, 2.4 / 17.5 ms for 400; 1000 tokens 4.4 / 3.6 ms for 4, 5.1 / 8.3 ms for 40.
+// The number of sequences has no say: the two round differently, and a member's loss must not depend on how many share its wave.
 static bool seq_long_pays(const EflaParams& p) {
-    if (p.T > 768 && (p.T > kLgMaxT || p.seqs * static_cast<long long>(p.heads) < 32)) return false;
+    if (p.T > kLgMaxT) return false;
     // the output holds w before all of q, k and v have been read: it must not lie among them
     if (p.seqs <= 0) return true;
     const size_t last = static_cast<size_t>(p.seqs) * p.T - 1;

@@ -266,7 +266,7 @@ typedef struct bnf4_efla_desc {
     int ld_out;
     int variant; /* BNF4_EFLA_*: which kernel runs. AUTO: for heads of 64 with no HBM state, the chunked or the per-token
                     register-state kernel as option "efla_chunked" says; for head widths above 32 other than 64 with no HBM state, an fp16 state, up to
-                    768 tokens (1024 from 32 sequence-heads on; beyond 128 only if out lies apart from q, k and v) and "efla_chunked" on,
+                    1024 tokens (beyond 128 only if out lies apart from q, k and v) and "efla_chunked" on,
                     the closed form of the whole sequence (nothing rounded to fp16 between tokens); the generic kernel otherwise. */
     int qkv_f16; /* 1: q, k, v are IEEE halves and ld_qkv counts halves (chunked kernel only; 16-byte aligned rows) */
     int out_f16; /* 1: out is IEEE halves and ld_out counts halves (chunked kernel only; 16-byte aligned rows) */

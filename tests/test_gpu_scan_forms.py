@@ -129,7 +129,7 @@ def test_generic_kernel_carries_the_state(H, hidden, fp16, offset):
 @pytest.mark.parametrize("scale", [0.3, 1000.0, 1e-3])
 @pytest.mark.parametrize("hidden,heads,seqs,T,method", [
     (512, 1, 2, 129, 1), (512, 1, 3, 322, 0), (96, 1, 2, 256, 1), (320, 2, 2, 257, 1), (128, 1, 150, 140, 0), (160, 1, 1, 768, 1),
-    (96, 1, 32, 1024, 1)])   # (the per-token kernel has 1024 tokens of fewer units)
+    (96, 1, 32, 1024, 1), (96, 1, 2, 1024, 0)])
 def test_closed_form_of_long_sequences(H, hidden, heads, seqs, T, method, scale):
     """More than one block of 128 tokens: one token in the last block, full blocks, more units than SMs, the longest of few and of many
     units. Every block product adds the error that the one-block form is allowed, so the bound grows with the number of blocks."""

@@ -37,6 +37,11 @@ def test_other_scans(H, hidden, heads, method):
     bits_of_groups(H, hidden, heads, 40, 130, method, 0, [(0, 1), (11, 20)])
 
 
+@pytest.mark.parametrize("T", [768, 769, 1024])
+def test_long_closed_form(H, T):
+    bits_of_groups(H, 96, 1, 34, T, 1, 0, [(0, 1), (2, 31)])
+
+
 def test_losses_of_a_population_do_not_depend_on_the_wave():
     """Wide heads: 2, 6 and 18 members a wave take clusters of four, of two and single CTAs."""
     import torch
