@@ -248,10 +248,35 @@ __global__ void __launch_bounds__(kGenThreads, (NI <= 16 ? 2 : 1)) efla_generic_
     }
 }
 
+// Do two blocks of rows of `width` floats share memory? Exact for equal row strides (columns of one matrix), else by their address ranges.
+bool rows_touch(const void* a, long long lda, const void* b, long long ldb, long long rows, long long width) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    if (x >= y + ((rows - 1) * ldb + width) * sizeof(float) || y >= x + ((rows - 1) * lda + width) * sizeof(float)) return false;
+    if (lda != ldb || lda < width) return true;
+    const long long apart = static_cast<long long>((x > y ? x - y : y - x) % (lda * sizeof(float)));
+    return apart < static_cast<long long>(width * sizeof(float)) || apart > static_cast<long long>((lda - width) * sizeof(float));
+}
+
 template <typename ST, int NPC, int NI>
 int launch_generic(const EflaParams& p, cudaStream_t stream) {
     constexpr int NC = NPC * StatePiece<ST>::N;
     const int hd = p.hidden / p.heads;
+    // Every slice of a head reads whole rows of q and k while the others write their columns: an output that lies on them goes through a buffer of its
+    // own. (In place of v, or in one slice, a CTA reads a row before it writes there.)
+    const long long rows = p.seqs * static_cast<long long>(p.T);
+    if (hd > NC && (rows_touch(p.out, p.ld_out, p.q, p.ld_qkv, rows, p.hidden) || rows_touch(p.out, p.ld_out, p.k, p.ld_qkv, rows, p.hidden) ||
+                    (rows_touch(p.out, p.ld_out, p.v, p.ld_qkv, rows, p.hidden) && !(p.out == p.v && p.ld_out == p.ld_qkv)))) {
+        EflaParams apart = p;
+        int rc = check_cuda(cudaMallocAsync(&apart.out, rows * p.hidden * sizeof(float), stream), "cudaMallocAsync(efla)");
+        if (rc) return rc;
+        apart.ld_out = p.hidden;
+        rc = launch_generic<ST, NPC, NI>(apart, stream);
+        if (!rc)
+            rc = check_cuda(cudaMemcpy2DAsync(p.out, p.ld_out * sizeof(float), apart.out, p.hidden * sizeof(float), p.hidden * sizeof(float), rows, cudaMemcpyDeviceToDevice, stream),
+                            "cudaMemcpy2DAsync(efla)");
+        const int rc2 = check_cuda(cudaFreeAsync(apart.out, stream), "cudaFreeAsync(efla)");
+        return rc ? rc : rc2;
+    }
     const size_t smem = sizeof(float) * (4 * static_cast<size_t>(hd) + 4 * (kGenThreads / 32) + 3 * (kGenThreads / 32) * NC);
     const long long ctas = p.seqs * static_cast<long long>(p.heads) * ((hd + NC - 1) / NC);
     if (ctas > 0x7fffffffLL) return set_error(BNF4_ERR_INVALID, "efla (generic kernel): too many sequences in one call");

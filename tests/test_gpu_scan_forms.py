@@ -143,8 +143,32 @@ def test_closed_form_of_long_sequences(H, hidden, heads, seqs, T, method, scale)
     assert np.abs(got - ref).max() <= 2e-5 * ((T + 127) // 128) * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("on,shift", [("q", 0), ("k", 0), ("v", 0), ("v", 8), ("apart", 0)])
+@pytest.mark.parametrize("hidden,seqs,T", [(96, 1, 150), (512, 300, 133), (1024, 40, 130)])
+def test_long_sequence_into_its_own_inputs(H, hidden, seqs, T, on, shift):
+    """An output that lies on q, k or v keeps the per-token kernel. The slices of a head (more CTAs than fit the device here) read whole rows
+    of q and k, so they must not see one another's outputs: the same bits as into a buffer of its own."""
+    import torch
+    rng = np.random.default_rng(3)
+    fc = 4 * hidden + 32
+    qkv = make_qkv(rng, seqs * T, hidden, fc, 0.4)
+    beta = dev(qkv[:, 3 * hidden])
+
+    def scan(qd, out, ld):
+        H.efla_scan(state=None, state_fp16=1, q=qd, k=qd[:, hidden:], v=qd[:, 2 * hidden:], beta_raw=beta, ld_qkv=fc, ld_beta=1, beta_bias=-2.0, hidden=hidden, heads=1,
+                    seqs=seqs, T=T, method=1, eps=1e-6, out=out, ld_out=ld, variant=1)
+
+    want = torch.empty(seqs * T, hidden, device="cuda")
+    scan(dev(qkv), want, hidden)
+    qd = dev(qkv)
+    col = {"q": 0, "k": hidden, "v": 2 * hidden, "apart": 3 * hidden + 32}[on] + shift
+    scan(qd, qd[:, col:], fc)
+    assert torch.equal(qd[:, col:col + hidden], want)
+    assert torch.equal(torch.cat([qd[:, :col], qd[:, col + hidden:]], 1), torch.cat([dev(qkv)[:, :col], dev(qkv)[:, col + hidden:]], 1))
+
+
 def test_long_sequence_into_its_own_queries(H):
-    """An output that overlays q keeps the per-token kernel, which reads a token before it writes it."""
+    """An output that overlays q keeps the per-token kernel."""
     import torch
     rng = np.random.default_rng(3)
     hidden, T, fc = 96, 150, 320
