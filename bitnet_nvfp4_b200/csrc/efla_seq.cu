@@ -13,6 +13,10 @@
 // two first so that neither term under- or overflows) and the products hi hi + hi mid + mid hi accumulate in fp32. Nothing is
 // rounded to fp16 between tokens, so the result lies closer to exact arithmetic than the per-token form's fp16 state.
 //
+// Values that are no numbers stay where the recurrence has them, although 0 x NaN is NaN in a contraction: from the first token on whose k or beta
+// makes the state NaN, the sequence is cut off (as if it ended there) and the rows behind it are NaN; a v that is no number is taken out
+// and its column is NaN from its token on; in q it only meets its own row.
+//
 // One CTA of 16 warps per (sequence, head):
 //   1. norms of q and k and the per-token scalars (one warp per row),
 //   2. G and X = Q^ K^^T over 64-column blocks of K and Q (fp32 -> two halves -> shared memory, double-buffered, the next block's
@@ -29,6 +33,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cfloat>
+#include <cmath>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -51,7 +57,8 @@ constexpr int kSqInv = kSqDiag + 8 * 16 * 17 * 4;                // their invers
 constexpr int kSqScal = kSqInv + 2 * 8 * 16 * kSqTStride * 2;    // q scale, k scale, a, b [4][128] floats
 constexpr int kSqRed = kSqScal + 4 * kSeqMaxT * 4;               // reduction scratch [2][16] + broadcast
 constexpr int kSqPart = kSqRed + 256;                            // squared norms of a CTA's tokens [2][128] floats (read by its cluster)
-constexpr int kSqSmem = kSqPart + 2 * kSeqMaxT * 4;
+constexpr int kSqBad = kSqPart + 2 * kSeqMaxT * 4;               // first token of each of 64 columns whose v is no number
+constexpr int kSqSmem = kSqBad + 64 * 4;
 static_assert(2 * kSeqMaxT * kSqLStride * 2 <= kSqStage && kSeqMaxT * kSqXStride * 4 <= kSqStage && 4 * kSqTile <= kSqStage, "overlaid regions");
 static_assert(kSqDiag % 16 == 0 && kSqInv % 16 == 0 && kSqScal % 16 == 0, "16-byte aligned regions");
 constexpr float kSqUp = 256.0f;                    // power-of-two scale of every normalised operand
@@ -89,16 +96,30 @@ __device__ __forceinline__ void seq_scalars(const EflaParams& p, float logit, fl
     qinv = rsqrtf(qss + p.eps);
     kinv = kss > 0.0f ? rsqrtf(kss) : 0.0f;
     const float n = kss * kinv;
-    if (p.method == 0) {
-        const float ksc = rsqrtf(lambda + p.eps);
+    const float ksc = p.method == 0 ? rsqrtf(lambda + p.eps) : 1.0f;
+    const float alpha = p.method == 0 ? beta : -expm1f(-(beta * lambda)) / (lambda + p.eps);
+    if (kss == INFINITY) {  // the norm of a finite k overflows: the recurrence leaves the state alone
+        a = b = alpha * (p.method == 0 ? ksc : 1.0f);
+    } else if (p.method == 0) {
         a = beta * (n * ksc) * (n * ksc);
         b = beta * (n * ksc);
     } else {
-        const float alpha = -expm1f(-(beta * lambda)) / (lambda + p.eps);
         a = alpha * kss;
         b = alpha * n;
     }
 }
+// The squared norm of a row (a warp's lanes hold its sum): infinite because of an infinite element (NaN then) or of an overflow?
+__device__ __forceinline__ float seq_infinite_norm(float kss, const float* row, int hd, int lane) {
+    if (kss != INFINITY) return kss;
+    bool bad = false;
+    for (int i = lane; i < hd; i += 32) bad = bad || !(fabsf(row[i]) <= FLT_MAX);
+    return __any_sync(0xffffffffu, bad) ? NAN : kss;
+}
+__device__ __forceinline__ uint32_t seq_abs_bits(const float4& x) {  // ordered like the magnitudes, infinities and NaN above all numbers
+    const uint32_t m = 0x7fffffffu;
+    return max(max(__float_as_uint(x.x) & m, __float_as_uint(x.y) & m), max(__float_as_uint(x.z) & m, __float_as_uint(x.w) & m));
+}
+constexpr uint32_t kSeqNonFinite = 0x7f800000u;
 
 // inverses of I + (diagonal 16 x 16 blocks of L): lane c owns column c of a block, two blocks per warp, four warps. Two halves, scaled by kSqUp.
 __device__ __forceinline__ void seq_invert_diagonal(const float* Ld, __half* inv, int nb, int warp, int lane) {
@@ -241,6 +262,8 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     float* a_sh = ks_sh + kSeqMaxT;
     float* b_sh = a_sh + kSeqMaxT;
     float* red = reinterpret_cast<float*>(sm + kSqRed);
+    int* red_bad = reinterpret_cast<int*>(red + 48);  // [4]
+    int* bad_col = reinterpret_cast<int*>(sm + kSqBad);
     float* part = reinterpret_cast<float*>(sm + kSqPart);
     const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
 
@@ -258,6 +281,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         }
         qss = warp_sum_f(qss);
         kss = warp_sum_f(kss);
+        if (t < T) kss = seq_infinite_norm(kss, kg + static_cast<size_t>(t) * p.ld_qkv, hd, lane);
         if (lane == 0) { part[t] = qss; part[kSeqMaxT + t] = kss; }
     }
     if constexpr (CS > 1) sq_cluster_sync<CS>();
@@ -284,9 +308,15 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         float m = b;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) red[warp] = m;
+        const uint32_t bad = __reduce_min_sync(0xffffffffu, static_cast<uint32_t>(a == a && b == b ? T : t));
+        if (lane == 0) { red[warp] = m; red_bad[warp] = static_cast<int>(bad); }
     }
     __syncthreads();
+    const int Te = min(min(red_bad[0], red_bad[1]), min(red_bad[2], red_bad[3]));  // tokens before the first one that makes the state NaN
+    if (Te < T) {
+        if (tid >= Te && tid < T) qs_sh[tid] = ks_sh[tid] = a_sh[tid] = b_sh[tid] = 0.0f;
+        __syncthreads();
+    }
     const float bscale = sq_pow2_scale(fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]))) * (1.0f / kSqUp);  // b * bscale <= 1
 
     // ---------------- 2. G and X ----------------
@@ -308,7 +338,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         for (int i = 0; i < 4; ++i) {
             const int t = srow + 32 * i, c = d0 + 4 * piece;
             kr[i] = qr[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (t < T && c < hd) {
+            if (t < Te && c < hd) {
                 kr[i] = *reinterpret_cast<const float4*>(kg + static_cast<size_t>(t) * p.ld_qkv + c);
                 if (CS == 1 || owner(t >> 4) == rank) qr[i] = *reinterpret_cast<const float4*>(qg + static_cast<size_t>(t) * p.ld_qkv + c);
             }
@@ -472,24 +502,42 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int t = srow + 32 * i, c = c0 + 4 * piece;
-            vr[i] = (t < T && c < hd) ? *reinterpret_cast<const float4*>(vg + static_cast<size_t>(t) * p.ld_qkv + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            vr[i] = (t < Te && c < hd) ? *reinterpret_cast<const float4*>(vg + static_cast<size_t>(t) * p.ld_qkv + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     };
     load_v(db0 * 64);
     for (int ct = db0; ct < db1; ++ct) {
         // the tile's own power-of-two scale keeps both halves of its values in range
-        float m = 0.0f;
+        uint32_t m = 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) m = fmaxf(fmaxf(fmaxf(m, fabsf(vr[i].x)), fmaxf(fabsf(vr[i].y), fabsf(vr[i].z))), fabsf(vr[i].w));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        float* redb = red + 16 * (ct & 1);
+        for (int i = 0; i < 4; ++i) m = max(m, seq_abs_bits(vr[i]));
+        m = __reduce_max_sync(0xffffffffu, m);
+        uint32_t* redb = reinterpret_cast<uint32_t*>(red) + 16 * (ct & 1);
         if (lane == 0) redb[warp] = m;
         __syncthreads();  // also: everyone is done with the tile before the previous one
-        m = redb[lane & 15];
+        m = __reduce_max_sync(0xffffffffu, redb[lane & 15]);
+        const bool tile_bad = m >= kSeqNonFinite;
+        if (tile_bad) {
+            if (tid < 64) bad_col[tid] = T;
+            __syncthreads();
+            m = 0;
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        const float vs = sq_pow2_scale(m);
+            for (int i = 0; i < 4; ++i) {
+                auto clear = [&](float& x, int e) {
+                    if (!(fabsf(x) <= FLT_MAX)) {
+                        atomicMin(bad_col + 4 * piece + e, srow + 32 * i);
+                        x = 0.0f;
+                    }
+                };
+                clear(vr[i].x, 0); clear(vr[i].y, 1); clear(vr[i].z, 2); clear(vr[i].w, 3);
+                m = max(m, seq_abs_bits(vr[i]));
+            }
+            m = __reduce_max_sync(0xffffffffu, m);
+            if (lane == 0) redb[warp] = m;  // (read by everyone before the barrier above)
+            __syncthreads();
+            m = __reduce_max_sync(0xffffffffu, redb[lane & 15]);
+        }
+        const float vs = sq_pow2_scale(__uint_as_float(m));
         uint8_t* st = sm + (ct & 1) * (2 * kSqTile);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -541,8 +589,12 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
 #pragma unroll
                     for (int hr = 0; hr < 2; ++hr) {
                         const int t = r * 16 + g + 8 * hr;
-                        if (t < T && c < hd)
-                            *reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c) = make_float2(y[n][2 * hr] * ds, y[n][2 * hr + 1] * ds);
+                        float2 x = make_float2(y[n][2 * hr] * ds, y[n][2 * hr + 1] * ds);
+                        if (tile_bad || Te < T) {
+                            if (t >= Te || (tile_bad && t >= bad_col[c & 63])) x.x = NAN;
+                            if (t >= Te || (tile_bad && t >= bad_col[(c & 63) + 1])) x.y = NAN;
+                        }
+                        if (t < T && c < hd) *reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c) = x;
                     }
                 }
             };
@@ -568,7 +620,8 @@ constexpr int kLgDiag = kLgMat + kSeqMaxT * kSqXStride * 4;
 constexpr int kLgInv = kLgDiag + 8 * 16 * 17 * 4;
 constexpr int kLgScal = kLgInv + 2 * 8 * 16 * kSqTStride * 2;     // q scale, k scale, a, b [4][T]
 constexpr int kLgRed = kLgScal + 4 * kLgMaxT * 4;
-constexpr int kLgSmem = kLgRed + 64;
+constexpr int kLgState = kLgRed + 64;
+constexpr int kLgSmem = kLgState + 16;
 static_assert(2 * kSeqMaxT * kSqLStride * 2 <= 4 * kSqTile, "L takes the staging tiles' place while the diagonal block is inverted");
 static_assert(kLgMat % 16 == 0 && kLgDiag % 16 == 0 && kLgInv % 16 == 0 && kLgScal % 16 == 0 && kLgRed % 16 == 0, "16-byte aligned regions");
 
@@ -593,7 +646,8 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
     float* ks_sh = qs_sh + kLgMaxT;
     float* a_sh = ks_sh + kLgMaxT;
     float* b_sh = a_sh + kLgMaxT;
-    float* red = reinterpret_cast<float*>(sm + kLgRed);
+    uint32_t* red = reinterpret_cast<uint32_t*>(sm + kLgRed);
+    int* state = reinterpret_cast<int*>(sm + kLgState);  // tokens in use; whether a v was no number
     const uint32_t sm0 = static_cast<uint32_t>(__cvta_generic_to_shared(sm));
 
     // ---------------- norms and scalars of all tokens (as in efla_seq_kernel) ----------------
@@ -610,8 +664,10 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
         }
         qss = warp_sum_f(qss);
         kss = warp_sum_f(kss);
+        if (t < T) kss = seq_infinite_norm(kss, kg + static_cast<size_t>(t) * p.ld_qkv, hd, lane);
         if (lane == 0) { qs_sh[t] = qss; ks_sh[t] = kss; }
     }
+    if (tid == 0) { state[0] = T; state[1] = 0; }
     __syncthreads();
     const float bias = efla_seq_bias(p, seq);
     for (int t = tid; t < nblocks * kSeqMaxT; t += kSeqThreads) {
@@ -621,8 +677,14 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
         ks_sh[t] = kSqUp * ks;
         a_sh[t] = a;
         b_sh[t] = b;
+        if (!(a == a && b == b)) atomicMin(state, t);
     }
     __syncthreads();
+    const int Te = state[0];  // tokens before the first one that makes the state NaN
+    if (Te < T) {
+        for (int t = Te + tid; t < T; t += kSeqThreads) qs_sh[t] = ks_sh[t] = a_sh[t] = b_sh[t] = 0.0f;
+        __syncthreads();
+    }
 
     const int piece = tid & 15, srow = tid >> 4;  // staging: 16-byte piece of a 64-column row, rows srow + 32 i
     const int wr = warp >> 1, wc = warp & 1;      // results: 16-row block, column half
@@ -630,7 +692,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int t = blk * kSeqMaxT + srow + 32 * i, c = ct * 64 + 4 * piece;
-            r[i] = t < T && c < hd ? *reinterpret_cast<const float4*>(base + static_cast<size_t>(t) * ld + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            r[i] = t < Te && c < hd ? *reinterpret_cast<const float4*>(base + static_cast<size_t>(t) * ld + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     };
     auto store = [&](const float4 (&r)[4], int tile, const float* scale, float common) {  // two halves per value
@@ -735,13 +797,29 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
         const uint32_t pa = sm0 + kLgMat + static_cast<uint32_t>((wr * 16 + (lane & 15)) * (kSqXStride * 4) + (lane >> 4) * 16);
         const uint32_t vb = sm0 + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqStride + wc * 32 + (lane >> 4) * 8) * 2u;
         for (int ct = 0; ct < nd; ++ct) {
-            float m = 0.0f;
+            uint32_t m = 0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) m = fmaxf(fmaxf(fmaxf(m, fabsf(r[i].x)), fmaxf(fabsf(r[i].y), fabsf(r[i].z))), fabsf(r[i].w));
-            m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));  // non-negative floats order like their bits
+            for (int i = 0; i < 4; ++i) m = max(m, seq_abs_bits(r[i]));
+            m = __reduce_max_sync(0xffffffffu, m);
             if (lane == 0) red[warp] = m;
             __syncthreads();  // also: everyone is done with the previous tile
-            const float vs = sq_pow2_scale(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(red[lane & 15]))));
+            m = __reduce_max_sync(0xffffffffu, red[lane & 15]);
+            if (scale_b && m >= kSeqNonFinite) {  // (v: w is finite)
+                __syncthreads();  // everyone has read red
+                m = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    for (float* x : {&r[i].x, &r[i].y, &r[i].z, &r[i].w})
+                        if (!(fabsf(*x) <= FLT_MAX)) *x = 0.0f;
+                    m = max(m, seq_abs_bits(r[i]));
+                }
+                m = __reduce_max_sync(0xffffffffu, m);
+                if (lane == 0) red[warp] = m;
+                state[1] = 1;
+                __syncthreads();
+                m = __reduce_max_sync(0xffffffffu, red[lane & 15]);
+            }
+            const float vs = sq_pow2_scale(__uint_as_float(m));
             store(r, 0, nullptr, vs);
             if (ct + 1 < nd) fetch(ct + 1);
             __syncthreads();
@@ -779,7 +857,13 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
                     float2* o = reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c);
                     float2 x = make_float2(y[n][2 * hr] * ds, y[n][2 * hr + 1] * ds);
                     if (op == LO_FROM_V) {
-                        const float2 v = *reinterpret_cast<const float2*>(vg + static_cast<size_t>(t) * p.ld_qkv + c);
+                        float2 v = *reinterpret_cast<const float2*>(vg + static_cast<size_t>(t) * p.ld_qkv + c);
+                        if (!(fmaxf(fabsf(v.x), fabsf(v.y)) <= FLT_MAX) || v.x != v.x || v.y != v.y) {
+                            if (!(fabsf(v.x) <= FLT_MAX)) v.x = 0.0f;
+                            if (!(fabsf(v.y) <= FLT_MAX)) v.y = 0.0f;
+                            state[1] = 1;
+                        }
+                        if (t >= Te) v = make_float2(0.0f, 0.0f);
                         x = make_float2(fmaf(b_sh[t], v.x, -x.x), fmaf(b_sh[t], v.y, -x.y));
                     } else if (op == LO_SUB || op == LO_ADD) {
                         const float2 old = *o;
@@ -825,6 +909,13 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
         for (int J = 0; J < I; ++J) {
             gram(qg, qs_sh, false, I, J);
             product(og, p.ld_out, false, I, J, false, LO_ADD);
+        }
+    }
+    if (Te < T || state[1] != 0) {  // (product ends with a barrier)
+        for (int c = tid; c < hd; c += kSeqThreads) {
+            int t = 0;
+            while (t < Te && fabsf(vg[static_cast<size_t>(t) * p.ld_qkv + c]) <= FLT_MAX) ++t;
+            for (; t < T; ++t) og[static_cast<size_t>(t) * p.ld_out + c] = NAN;
         }
     }
 }
