@@ -494,7 +494,8 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     __syncthreads();
 
     // ---------------- 5. y = P~ V, 64 columns at a time ----------------
-    const int cg = warp >> 2;  // 16-column group of the tile
+    const int cg = warp >> 2;                        // 16-column group of the tile
+    const int y1r = warp & 3, y2r = nb - 1 - y1r;    // this warp's row blocks, as r1 and r2 of one CTA per unit
     const uint32_t pa = sm0 + kSqStage + static_cast<uint32_t>((lane & 15) * (kSqXStride * 4) + (lane >> 4) * 16);
     const uint32_t vb = sm0 + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqStride + cg * 16 + (lane >> 4) * 8) * 2u;
     float4 vr[4];
@@ -550,28 +551,28 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         }
         if (ct + 1 < db1) load_v((ct + 1) * 64);
         __syncthreads();
-        if (r1 <= r2) {
+        if (y1r <= y2r) {
             float y1[2][4], y2[2][4];
 #pragma unroll
             for (int n = 0; n < 2; ++n)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) y1[n][e] = y2[n][e] = 0.0f;
             const uint32_t vbt = vb + (ct & 1) * (2 * kSqTile);
-            for (int j = 0; j <= r2; ++j) {
+            for (int j = 0; j <= y2r; ++j) {
                 uint32_t vh[4], vm[4], ah[4], am[4];
                 sq_ldm_trans(vh, vbt + j * (16 * kSqStride * 2));
                 sq_ldm_trans(vm, vbt + kSqTile + j * (16 * kSqStride * 2));
-                sq_ldm(ah, pa + r2 * (16 * kSqXStride * 4) + j * 32);
-                sq_ldm(am, pa + r2 * (16 * kSqXStride * 4) + kSqPMid + j * 32);
+                sq_ldm(ah, pa + y2r * (16 * kSqXStride * 4) + j * 32);
+                sq_ldm(am, pa + y2r * (16 * kSqXStride * 4) + kSqPMid + j * 32);
 #pragma unroll
                 for (int n = 0; n < 2; ++n) {
                     sq_mma(y2[n], ah, vh[2 * n], vh[2 * n + 1]);
                     sq_mma(y2[n], ah, vm[2 * n], vm[2 * n + 1]);
                     sq_mma(y2[n], am, vh[2 * n], vh[2 * n + 1]);
                 }
-                if (r1 < r2 && j <= r1) {
-                    sq_ldm(ah, pa + r1 * (16 * kSqXStride * 4) + j * 32);
-                    sq_ldm(am, pa + r1 * (16 * kSqXStride * 4) + kSqPMid + j * 32);
+                if (y1r < y2r && j <= y1r) {
+                    sq_ldm(ah, pa + y1r * (16 * kSqXStride * 4) + j * 32);
+                    sq_ldm(am, pa + y1r * (16 * kSqXStride * 4) + kSqPMid + j * 32);
 #pragma unroll
                     for (int n = 0; n < 2; ++n) {
                         sq_mma(y1[n], ah, vh[2 * n], vh[2 * n + 1]);
@@ -598,8 +599,8 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
                     }
                 }
             };
-            put(y2, r2);
-            if (r1 < r2) put(y1, r1);
+            put(y2, y2r);
+            if (y1r < y2r) put(y1, y1r);
         }
     }
 }
