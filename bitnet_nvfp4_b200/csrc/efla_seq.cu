@@ -82,11 +82,14 @@ __device__ __forceinline__ void sq_split(float x0, float x1, uint32_t& hi, uint3
     hi = *reinterpret_cast<const uint32_t*>(&h);
     mid = *reinterpret_cast<const uint32_t*>(&m);
 }
-// largest power of two that keeps |x| <= m below kSqUp (1 for m == 0)
+// largest power of two that keeps |x| <= m below 2^TOP (1 for m == 0). V takes the most of fp16's range (TOP 15): its tokens share a scale, and what is
+// 2^d below the largest of them keeps 22 bits up to d = 17 and 39 - d beyond. With 2^8 rows a factor of 1e7 smaller than later ones of
+// their tile were off by 4e-3, more than fp16 states cost them.
+template <int TOP>
 __device__ __forceinline__ float sq_pow2_scale(float m) {
     if (!(m > 0.0f)) return 1.0f;
     const int e = static_cast<int>((__float_as_uint(m) >> 23) & 0xffu) - 127;  // 2^e <= m < 2^(e+1)
-    return __uint_as_float(static_cast<uint32_t>(min(max(7 - e + 127, 1), 254)) << 23);
+    return __uint_as_float(static_cast<uint32_t>(min(max(TOP - 1 - e + 127, 1), 254)) << 23);
 }
 
 // beta's logit and the squared norms of a token -> 1 / |q|, 1 / |k|, a and b
@@ -317,7 +320,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         if (tid >= Te && tid < T) qs_sh[tid] = ks_sh[tid] = a_sh[tid] = b_sh[tid] = 0.0f;
         __syncthreads();
     }
-    const float bscale = sq_pow2_scale(fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]))) * (1.0f / kSqUp);  // b * bscale <= 1
+    const float bscale = sq_pow2_scale<6>(fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3])));  // b * bscale < 64: P~ below 2^14, also for V's sake
 
     // ---------------- 2. G and X ----------------
     const int pr = rank + CS * ((warp & 3) % (4 / CS)), which = (warp >> 2) & 1, half = warp >> 3;
@@ -480,7 +483,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         __syncwarp();  // the rows are in registers: P~ takes their place
         uint8_t* prow = sm + kSqStage;
         seq_solve_rows(sm0, kSqStage, prow, kSqInv, i, lane, xr);
-        // the columns' factors b_s, scaled to at most one: applied to the finished rows (exact powers of two aside, one more rounding)
+        // the columns' factors b_s, scaled to at most 64: applied to the finished rows (exact powers of two aside, one more rounding)
         for (int idx = lane; idx < 16 * (i + 1) * 8; idx += 32) {
             const int rr = idx / ((i + 1) * 8), cc = (idx - rr * ((i + 1) * 8)) * 2;
             uint8_t* d = prow + (i * 16 + rr) * (kSqXStride * 4) + cc * 2;
@@ -538,7 +541,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
             __syncthreads();
             m = __reduce_max_sync(0xffffffffu, redb[lane & 15]);
         }
-        const float vs = sq_pow2_scale(__uint_as_float(m));
+        const float vs = sq_pow2_scale<15>(__uint_as_float(m));
         uint8_t* st = sm + (ct & 1) * (2 * kSqTile);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -820,7 +823,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
                 __syncthreads();
                 m = __reduce_max_sync(0xffffffffu, red[lane & 15]);
             }
-            const float vs = sq_pow2_scale(__uint_as_float(m));
+            const float vs = sq_pow2_scale<15>(__uint_as_float(m));
             store(r, 0, nullptr, vs);
             if (ct + 1 < nd) fetch(ct + 1);
             __syncthreads();

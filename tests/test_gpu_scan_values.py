@@ -7,7 +7,7 @@ from test_gpu_scan_forms import H, exact_scan, make_qkv, run  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(512, 1, 2, 128), (96, 1, 170, 50), (320, 2, 40, 77), (96, 1, 2, 1), (512, 1, 3, 300), (96, 2, 2, 513)]
+SHAPES = [(512, 1, 2, 128), (96, 1, 170, 50), (320, 2, 40, 77), (96, 1, 2, 1), (512, 1, 3, 300), (192, 2, 2, 513)]
 
 
 @pytest.mark.parametrize("method", [1, 0])
@@ -55,3 +55,20 @@ def test_norms_that_overflow(H, T, method):
     ref = exact_scan(without, bb, hidden, 1, method)
     ref[1, T - 3] = 0.0
     assert np.abs(got - ref).max() <= 4e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("ratio", [1e2, 1e5, 1e7, 1e8])
+@pytest.mark.parametrize("hidden,T", [(512, 128), (96, 40), (96, 200)])
+def test_tokens_much_smaller_than_later_ones(H, hidden, T, ratio):
+    """Rows of small values before large ones of their tile: off by no more than the form with fp16 states has them, relative to themselves."""
+    rng = np.random.default_rng(int(ratio) + T)
+    fc, seqs, half = (3 * hidden + 1 + 31) & ~31, 4, min(T, 128) // 2
+    qkv = make_qkv(rng, seqs * T, hidden, fc, 0.3).reshape(seqs, T, fc)
+    qkv[:, :half, 2 * hidden:3 * hidden] *= np.float32(1e-2)
+    qkv[:, half:, 2 * hidden:3 * hidden] *= np.float32(1e-2 * ratio)
+    if ratio > 1e7:  # (within fp16's range for the other form)
+        qkv[:, :, 2 * hidden:3 * hidden] *= np.float32(0.1)
+    bb = np.full(seqs, -2.0, np.float32)
+    ref = exact_scan(qkv, bb, hidden, 1, 1)[:, :half]
+    err = [np.abs(run(H, qkv.reshape(-1, fc), bb, 1, hidden, 1, seqs, T, 1, variant)[:, :half] - ref).max() / np.abs(ref).max() for variant in (0, 1)]
+    assert err[0] <= max(err[1], 1e-6), err
