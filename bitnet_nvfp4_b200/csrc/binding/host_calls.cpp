@@ -7,6 +7,7 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Device.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -34,38 +35,55 @@ struct Args {
         }
         return a[i++];
     }
-    const at::Tensor& tensor() {
+    at::Tensor tensor() {
         PyObject* o = next();
-        if (!THPVariable_Check(o)) {
-            PyErr_Format(PyExc_TypeError, "argument %zd must be a tensor, not %s", i, Py_TYPE(o)->tp_name);
-            throw Failed{};
-        }
-        return THPVariable_Unpack(o);
+        return THPVariable_Check(o) ? THPVariable_Unpack(o) : described(o);
     }
-    const at::Tensor& matrix() {
-        const at::Tensor& t = tensor();
+    at::Tensor matrix() {
+        at::Tensor t = tensor();
         if (t.dim() != 2) {
             PyErr_Format(PyExc_ValueError, "argument %zd must have two dimensions, not %lld", i, static_cast<long long>(t.dim()));
             throw Failed{};
         }
         return t;
     }
+    at::Tensor described(PyObject* o);
     void* ptr();
     int integer();
-    float real() {
-        const double v = PyFloat_AsDouble(next());
-        if (v == -1.0 && PyErr_Occurred()) throw Failed{};
-        return static_cast<float>(v);
-    }
+    float real();
 };
 
+// the Python value of a ctypes number or pointer, which the fields of a ctypes structure take (a new reference); nullptr for other objects
+PyObject* ctypes_value(PyObject* o) {
+    if (PyIndex_Check(o) || PyFloat_Check(o)) return nullptr;
+    static PyObject* simple = [] {
+        PyObject* m = PyImport_ImportModule("ctypes");
+        PyObject* c = m ? PyObject_GetAttrString(m, "_SimpleCData") : nullptr;
+        Py_XDECREF(m);
+        return c;
+    }();
+    if (!simple || PyObject_IsInstance(o, simple) != 1) {
+        PyErr_Clear();
+        return nullptr;
+    }
+    return PyObject_GetAttrString(o, "value");
+}
+float to_real(PyObject* o) {
+    PyObject* held = PyFloat_Check(o) ? nullptr : ctypes_value(o);
+    const double v = PyFloat_AsDouble(held ? held : o);
+    Py_XDECREF(held);
+    if (v == -1.0 && PyErr_Occurred()) throw Failed{};
+    return static_cast<float>(v);
+}
 long long to_integer(PyObject* o) {
     if (PyLong_Check(o)) {
         const unsigned long long v = PyLong_AsUnsignedLongLongMask(o);
         if (v == ~0ull && PyErr_Occurred()) throw Failed{};
         return static_cast<long long>(v);
     }
-    PyObject* l = PyNumber_Index(o);
+    PyObject* held = ctypes_value(o);
+    PyObject* l = PyNumber_Index(held ? held : o);
+    Py_XDECREF(held);
     if (!l) throw Failed{};
     const unsigned long long v = PyLong_AsUnsignedLongLongMask(l);
     Py_DECREF(l);
@@ -76,14 +94,50 @@ void* to_pointer(PyObject* o) {
     if (o == Py_None) return nullptr;
     if (THPVariable_Check(o)) return THPVariable_Unpack(o).data_ptr();
     if (PyLong_Check(o)) return reinterpret_cast<void*>(to_integer(o));
-    PyObject* r = PyObject_CallMethod(o, "data_ptr", nullptr);
-    if (!r) throw Failed{};
-    void* p = PyLong_AsVoidPtr(r);
+    PyObject* r = PyObject_HasAttrString(o, "data_ptr") ? PyObject_CallMethod(o, "data_ptr", nullptr) : ctypes_value(o);
+    if (!r) {
+        if (!PyErr_Occurred()) PyErr_Format(PyExc_TypeError, "%s is no pointer", Py_TYPE(o)->tp_name);
+        throw Failed{};
+    }
+    void* p = r == Py_None ? nullptr : PyLong_AsVoidPtr(r);
     Py_DECREF(r);
     if (!p && PyErr_Occurred()) throw Failed{};
     return p;
 }
 void* Args::ptr() { return to_pointer(next()); }
+// An object that is no tensor but has data_ptr() and, where they are asked for, shape and device. (Bytes without an owner: the element type does
+// not matter, the entry points know it.)
+at::Tensor Args::described(PyObject* o) {
+    if (!PyObject_HasAttrString(o, "data_ptr")) {
+        PyErr_Format(PyExc_TypeError, "argument %zd must be a tensor, not %s", i, Py_TYPE(o)->tp_name);
+        throw Failed{};
+    }
+    void* p = to_pointer(o);
+    at::globalContext().lazyInitDevice(at::kCUDA);  // (the outputs are allocated by torch)
+    std::vector<int64_t> sizes;
+    if (PyObject* shape = PyObject_GetAttrString(o, "shape")) {
+        PyObject* seq = PySequence_Tuple(shape);
+        Py_DECREF(shape);
+        if (!seq) throw Failed{};
+        for (Py_ssize_t d = 0; d < PyTuple_GET_SIZE(seq); ++d) {
+            const Py_ssize_t n = PyNumber_AsSsize_t(PyTuple_GET_ITEM(seq, d), PyExc_OverflowError);
+            if (n == -1 && PyErr_Occurred()) {
+                Py_DECREF(seq);
+                throw Failed{};
+            }
+            sizes.push_back(n);
+        }
+        Py_DECREF(seq);
+    } else PyErr_Clear();
+    at::Device device(at::kCUDA, c10::cuda::current_device());
+    if (PyObject* dev = PyObject_GetAttrString(o, "device")) {
+        if (THPDevice_Check(dev)) device = reinterpret_cast<THPDevice*>(dev)->device;
+        Py_DECREF(dev);
+        if (device.is_cuda() && !device.has_index()) device.set_index(c10::cuda::current_device());
+    } else PyErr_Clear();
+    return at::for_blob(p, sizes).options(at::TensorOptions().dtype(at::kByte).device(device)).target_device(device).make_tensor();
+}
+float Args::real() { return to_real(next()); }
 int Args::integer() { return static_cast<int>(to_integer(next())); }
 
 at::Tensor empty_like_device(const at::Tensor& like, at::IntArrayRef sizes, at::ScalarType dtype) {
@@ -155,7 +209,7 @@ T* as(void* p) { return static_cast<T*>(p); }
     PyObject* name##_body(Args& x)
 
 ENTRY(quantize_a) {  // x, k_out
-    const at::Tensor& t = x.matrix();
+    const at::Tensor t = x.matrix();
     const int m = static_cast<int>(t.size(0)), k = static_cast<int>(t.size(1)), k_out = x.integer();
     Quantised o(t, m, k_out, false);
     const void* in = t.data_ptr();
@@ -167,7 +221,7 @@ ENTRY(quantize_a) {  // x, k_out
 ENTRY(embedding_lookup_noise_quantize) {  // tokens, token_stride, emb_w, emb_noise, hidden, batch, noise_scale, anti_sign
     void* tokens = x.ptr();
     const int stride = x.integer();
-    const at::Tensor& emb = x.tensor();
+    const at::Tensor emb = x.tensor();
     void* noise = x.ptr();
     const int hidden = x.integer(), batch = x.integer();
     const float scale = x.real();
@@ -182,7 +236,7 @@ ENTRY(embedding_lookup_noise_quantize) {  // tokens, token_stride, emb_w, emb_no
 }
 
 ENTRY(add_pos_gelu_quantize) {  // x, pos, act_scale
-    const at::Tensor& t = x.matrix();
+    const at::Tensor t = x.matrix();
     const int batch = static_cast<int>(t.size(0)), hidden = static_cast<int>(t.size(1));
     void* pos = x.ptr();
     const float act = x.real();
@@ -196,7 +250,7 @@ ENTRY(add_pos_gelu_quantize) {  // x, pos, act_scale
 }
 
 ENTRY(absmean_norm_q) {  // x8, scale
-    const at::Tensor& t = x.matrix();
+    const at::Tensor t = x.matrix();
     const int batch = static_cast<int>(t.size(0)), hidden = static_cast<int>(t.size(1));
     const float scale = x.real();
     Quantised o(t, batch, hidden, true);
@@ -209,9 +263,9 @@ ENTRY(absmean_norm_q) {  // x8, scale
 }
 
 ENTRY(add_scaled_absmean_norm_q) {  // x8_inout, y, add_scale, norm_scale
-    const at::Tensor& t = x.matrix();
+    const at::Tensor t = x.matrix();
     const int batch = static_cast<int>(t.size(0)), hidden = static_cast<int>(t.size(1));
-    const at::Tensor& y = x.tensor();
+    const at::Tensor y = x.tensor();
     const float add = x.real(), norm = x.real();
     Quantised o(y, batch, hidden, true);
     void *inout = t.data_ptr(), *yp = y.data_ptr(), *s = raw_stream();
@@ -223,7 +277,7 @@ ENTRY(add_scaled_absmean_norm_q) {  // x8_inout, y, add_scale, norm_scale
 }
 
 ENTRY(gemm) {  // a, b, sfa, sfb, m, n, k, alpha, beta, c, d
-    const at::Tensor& a = x.tensor();
+    const at::Tensor a = x.tensor();
     void *b = x.ptr(), *sfa = x.ptr(), *sfb = x.ptr();
     const int m = x.integer(), n = x.integer(), k = x.integer();
     const float alpha = x.real(), beta = x.real();
@@ -241,7 +295,7 @@ ENTRY(gemm) {  // a, b, sfa, sfb, m, n, k, alpha, beta, c, d
 }
 
 ENTRY(gemm_gelu_i8) {  // a, b, sfa, sfb, m, n, k, alpha, beta, c, act_scale
-    const at::Tensor& a = x.tensor();
+    const at::Tensor a = x.tensor();
     void *b = x.ptr(), *sfa = x.ptr(), *sfb = x.ptr();
     const int m = x.integer(), n = x.integer(), k = x.integer();
     const float alpha = x.real(), beta = x.real();
@@ -258,7 +312,7 @@ ENTRY(gemm_gelu_i8) {  // a, b, sfa, sfb, m, n, k, alpha, beta, c, act_scale
 
 ENTRY(efla_step_half) {  // S, qkv, fused_cols, beta_bias, hidden, batch, method, eps
     void* S = x.ptr();
-    const at::Tensor& qkv = x.tensor();
+    const at::Tensor qkv = x.tensor();
     const int fused = x.integer();
     const float bias = x.real();
     const int hidden = x.integer(), batch = x.integer(), method = x.integer();
@@ -274,7 +328,7 @@ ENTRY(efla_step_half) {  // S, qkv, fused_cols, beta_bias, hidden, batch, method
 }
 
 ENTRY(cross_entropy) {  // logits, bias, bias_noise, bias_noise_scale, targets, token_stride, loss
-    const at::Tensor& logits = x.matrix();
+    const at::Tensor logits = x.matrix();
     const int batch = static_cast<int>(logits.size(0)), vocab = static_cast<int>(logits.size(1));
     void *bias = x.ptr(), *noise = x.ptr();
     const float scale = x.real();
@@ -335,9 +389,7 @@ ENTRY(desc_call) {  // kind, front end (row quantiser), {field: value}
         }
         const Field f = d.fields[static_cast<size_t>(PyLong_AsLong(pos))];
         if (f.code == 'f') {
-            const double v = PyFloat_AsDouble(value);
-            if (v == -1.0 && PyErr_Occurred()) throw Failed{};
-            const float fv = static_cast<float>(v);
+            const float fv = to_real(value);
             std::memcpy(buf + f.offset, &fv, 4);
         } else if (f.code == 'P') {
             void* p = to_pointer(value);

@@ -65,8 +65,8 @@ def matrix_bytes(rows: int, cols: int) -> int:
 def _alloc_q(like: torch.Tensor, rows: int, cols: int, want_q=True):
     """Outputs of a quantiser on the device of `like`. Nothing is cleared: the library writes every int8 value, code and scale byte, the
     padding of the scale array included."""
-    q = like.new_empty((rows, cols), dtype=torch.int8) if want_q else None
-    return q, like.new_empty(matrix_bytes(rows, cols), dtype=torch.uint8), like.new_empty(sf_bytes(rows, cols), dtype=torch.uint8)
+    q = torch.empty((rows, cols), dtype=torch.int8, device=like.device) if want_q else None
+    return q, *(torch.empty(n, dtype=torch.uint8, device=like.device) for n in (matrix_bytes(rows, cols), sf_bytes(rows, cols)))
 
 
 def device_error() -> int:

@@ -105,3 +105,38 @@ def test_single_step_output_is_fp32_whatever_holds_the_inputs(H, state_half):
     for dt in (torch.float16, torch.bfloat16, torch.float64):
         with pytest.raises(TypeError):
             step(state(), qkv.to(dt), 224, -2.0, 64, 4, 1, 1e-6)
+
+
+class Raw:
+    """Device memory as another library hands it out: an address, a shape and a device."""
+
+    def __init__(self, t):
+        self.t, self.shape, self.device = t, tuple(t.shape), t.device
+
+    def data_ptr(self):
+        return self.t.data_ptr()
+
+
+def test_objects_that_are_no_tensors(H):
+    """Arguments are taken by their data_ptr(), descriptor fields also as ctypes values, as the ctypes structures take them."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randint(-127, 128, (32, 128), dtype=torch.int8, device="cuda", generator=g)
+    y = torch.randn(32, 128, device="cuda", generator=g)
+    for f, args in ((H.nvfp4_quantize_a, (x,)), (H.nvfp4_quantize_b, (x,)), (H.absmean_norm_q_nvfp4, (x, 1.0)), (H.add_pos_gelu_quantize_nvfp4, (y, y, 0.8)),
+                    (H.gelu_quantize_nvfp4, (y, 128, 0.8)), (H.activation_quantize_nvfp4, (y, 128, 1))):
+        want = f(*args)
+        got = f(*(Raw(a) if isinstance(a, torch.Tensor) else a for a in args))
+        assert all(b is None or (torch.equal(a, b) and a.device == x.device) for a, b in zip(got, want))
+    codes, sf = H.nvfp4_quantize_a(x)
+    d = torch.zeros(32, 32, device="cuda")
+    out = Raw(d)
+    assert H.gemm_ternary_f_nvfp4(Raw(codes), Raw(codes), Raw(sf), Raw(sf), 32, 32, 128, 1.0, d=out) is out
+    assert torch.equal(d, H.gemm_ternary_f_nvfp4(codes, codes, sf, sf, 32, 32, 128, 1.0)) and d.any()
+    c2, s2 = torch.zeros_like(codes), torch.zeros_like(sf)
+    H.rowquant(H.FE_INT8, rows=C.c_int(32), cols_in=128, cols_out=128, in_i8=C.c_void_p(x.data_ptr()), ld_in=128, out_codes=Raw(c2), out_sf=s2, out_q=C.c_void_p(),
+               norm_scale=C.c_float(1.0), tvec_pair_stride=C.c_longlong(0))
+    assert torch.equal(c2, codes) and torch.equal(s2, sf)
+    for bad in (dict(rows=1.5), dict(rows="8"), dict(in_i8=1.5), dict(in_i8=b"x"), dict(norm_scale="1")):
+        with pytest.raises(TypeError):
+            H.rowquant(H.FE_INT8, **{**dict(rows=32, cols_in=128, cols_out=128, in_i8=x, ld_in=128, out_codes=c2, out_sf=s2), **bad})
