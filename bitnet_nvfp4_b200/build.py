@@ -1,4 +1,4 @@
-"""In-tree build of libbnf4.so (sm_100a only) with nvcc, and of _host.so (the Python-side call path over it) with g++.
+"""In-tree build of libbnf4.so (sm_100a only) with nvcc, and of the host extension _host (the Python-side call path over it) with g++.
 
     python -m bitnet_nvfp4_b200.build            # incremental
     python -m bitnet_nvfp4_b200.build --force    # rebuild everything
@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -20,7 +21,7 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "libbnf4.so"
-HOST = PKG / "_host.so"
+HOST = PKG / f"_host{sysconfig.get_config_var('EXT_SUFFIX')}"  # (another interpreter does not take it for its own)
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -88,12 +89,9 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
 
 def build_host(force: bool = False) -> Path:
-    """_host.so: a CPython extension on torch's C++ tensors, linked to the libbnf4.so beside it."""
+    """The host extension: a CPython extension on torch's C++ tensors, linked to the libbnf4.so beside it. It holds for one torch and one
+    interpreter only, so both are noted with the command that built it, and it is built again when any of them changes."""
     src = CSRC / "binding" / "host_calls.cpp"
-    if not force and not _newer(src, HOST, [ROOT / "include" / "bnf4.h"]):
-        return HOST
-    import sysconfig
-
     import torch
     from torch.utils import cpp_extension
 
@@ -104,10 +102,17 @@ def build_host(force: bool = False) -> Path:
            *[f"-isystem{d}" for d in [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], cuda]], f"-I{ROOT / 'include'}", str(src),
            "-o", str(HOST), f"-L{PKG}", "-l:libbnf4.so", "-Wl,-rpath,$ORIGIN", f"-L{torch_lib}", "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10",
            "-lc10_cuda"]
+    stamp, built = OBJ / "_host.stamp", "\n".join([torch.__version__, sys.version, *cmd]).replace(str(ROOT), "")
+    if not force and not _newer(src, HOST, [ROOT / "include" / "bnf4.h"]) and stamp.exists() and stamp.read_text() == built:
+        return HOST
+    (PKG / "_host.so").unlink(missing_ok=True)  # the name it had before
+    stamp.unlink(missing_ok=True)
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
-        raise RuntimeError("build of _host.so failed")
+        raise RuntimeError(f"build of {HOST.name} failed")
+    OBJ.mkdir(exist_ok=True)
+    stamp.write_text(built)
     return HOST
 
 

@@ -4,7 +4,7 @@ the reference's src/cuda_kernels.h and src/efla_lm_kernels.h), on torch device t
 Function names and argument meaning follow the reference; every call goes through the C ABI of
 libbnf4.so on the current CUDA stream. torch is used for device memory and streams only.
 
-The functions that a token loop calls dozens of times per token go through _host.so, which converts arguments, allocates the
+The functions that a token loop calls dozens of times per token go through the extension _host, which converts arguments, allocates the
 outputs and calls the library natively (8.5 us per call through ctypes, more than the kernels take).
 """
 from __future__ import annotations
@@ -39,7 +39,7 @@ def _n():
         try:
             from . import _host
         except ImportError as e:
-            raise _l.Bnf4Error(f"_host.so cannot be loaded ({e}): build it with `python -m bitnet_nvfp4_b200.build`") from e
+            raise _l.Bnf4Error(f"the extension _host cannot be loaded ({e}): build it with `python -m bitnet_nvfp4_b200.build`") from e
         _host.set_error_class(_l.Bnf4Error)
         codes = {C.c_void_p: "P", C.c_int: "i", C.c_float: "f", C.c_longlong: "q"}
         for kind, desc in enumerate((_l.RowQuantDesc, _l.GemmDesc, _l.EflaDesc)):
