@@ -5,7 +5,8 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
-#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Device.h>
 #include <torch/csrc/Exceptions.h>
@@ -140,27 +141,27 @@ at::Tensor Args::described(PyObject* o) {
 float Args::real() { return to_real(next()); }
 int Args::integer() { return static_cast<int>(to_integer(next())); }
 
+// Uncleared, on the device of `like`, straight from the caching allocator (at::empty takes twice the time on top of it).
 at::Tensor empty_like_device(const at::Tensor& like, at::IntArrayRef sizes, at::ScalarType dtype) {
-    if (like.is_cuda()) return at::detail::empty_cuda(sizes, dtype, like.device(), c10::nullopt);
-    return at::empty(sizes, like.options().dtype(dtype));
+    int64_t n = 1;
+    for (const int64_t d : sizes) n = d < 0 || n < 0 ? -1 : n * d;
+    if (!like.is_cuda() || n < 0) return at::empty(sizes, like.options().dtype(dtype));  // (with its errors)
+    const size_t bytes = static_cast<size_t>(n) * c10::elementSize(dtype);
+    const c10::cuda::CUDAGuard guard(like.device());
+    c10::Allocator* from = c10::cuda::CUDACachingAllocator::get();
+    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(
+        c10::Storage(c10::make_intrusive<c10::StorageImpl>(c10::StorageImpl::use_byte_size_t(), bytes, from->allocate(bytes), from, /*resizable=*/true)),
+        c10::DispatchKeySet(c10::DispatchKey::CUDA), c10::scalarTypeToTypeMeta(dtype));
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+    return t;
 }
-// Outputs of a quantiser: three tensors on one allocation, each from a 512-byte boundary (an allocation costs about as much as the rest of the
-// call's host work). Nothing is cleared: the library writes every value, code and scale byte, padding included.
+// Outputs of a quantiser, each with a storage of its own. Nothing is cleared: the library writes every value, code and scale byte, padding included.
 struct Quantised {
     at::Tensor q, codes, sf;
     Quantised(const at::Tensor& like, int64_t rows, int64_t cols, bool want_q) {
-        const int64_t nq = want_q ? rows * cols : 0, nc = (rows * cols * 4 + 7) / 8, ns = (rows + 127) / 128 * 128 * (((cols + 15) / 16 + 3) / 4 * 4);
-        auto up = [](int64_t n) { return (n + 511) / 512 * 512; };
-        const at::Tensor base = empty_like_device(like, {up(nq) + up(nc) + ns}, at::kByte);
-        auto part = [&](int64_t offset, at::IntArrayRef sizes, at::ScalarType dtype) {
-            at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(base.storage()), base.key_set(), c10::scalarTypeToTypeMeta(dtype));
-            t.unsafeGetTensorImpl()->set_storage_offset(offset);  // elements of one byte
-            t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
-            return t;
-        };
-        if (want_q) q = part(0, {rows, cols}, at::kChar);
-        codes = part(up(nq), {nc}, at::kByte);
-        sf = part(up(nq) + up(nc), {ns}, at::kByte);
+        if (want_q) q = empty_like_device(like, {rows, cols}, at::kChar);
+        codes = empty_like_device(like, {(rows * cols * 4 + 7) / 8}, at::kByte);
+        sf = empty_like_device(like, {(rows + 127) / 128 * 128 * (((cols + 15) / 16 + 3) / 4 * 4)}, at::kByte);
     }
     template <typename T>
     T* values() { return static_cast<T*>(q.data_ptr()); }

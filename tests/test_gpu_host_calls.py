@@ -140,3 +140,25 @@ def test_objects_that_are_no_tensors(H):
     for bad in (dict(rows=1.5), dict(rows="8"), dict(in_i8=1.5), dict(in_i8=b"x"), dict(norm_scale="1")):
         with pytest.raises(TypeError):
             H.rowquant(H.FE_INT8, **{**dict(rows=32, cols_in=128, cols_out=128, in_i8=x, ld_in=128, out_codes=c2, out_sf=s2), **bad})
+
+
+def test_quantiser_outputs_have_their_own_storage(H):
+    """One of them can be kept, saved or grown without the others."""
+    import io
+
+    import torch
+    x = torch.randint(-127, 128, (33, 128), dtype=torch.int8, device="cuda")
+    q, codes, sf = H.absmean_norm_q_nvfp4(x, 1.0)
+    assert q.untyped_storage().nbytes() == q.numel() == 33 * 128 and q.storage_offset() == 0 and q.is_contiguous()
+    assert codes.untyped_storage().nbytes() == codes.numel() and sf.untyped_storage().nbytes() == sf.numel()
+    want, other = q.clone(), codes.clone()
+    buf = io.BytesIO()
+    torch.save(q, buf)
+    assert buf.tell() < q.numel() + 2048 and torch.equal(torch.load(io.BytesIO(buf.getvalue())), q)
+    q.resize_(100, 128)
+    q[33:].fill_(5)
+    assert torch.equal(q[:33], want) and torch.equal(codes, other)
+    q.record_stream(torch.cuda.Stream())
+    with torch.inference_mode():
+        assert H.nvfp4_quantize_a(x)[0].is_inference()
+    assert H.nvfp4_quantize_a(x[:0])[0].numel() == 0
