@@ -1151,18 +1151,21 @@ int bnf4_model_get_weights(void* handle, bnf4_model_weights* w) {
                           {m.head, w->head, vh}, {m.head_bias, w->head_bias, m.V * sizeof(float)}, {m.beta_bias, w->beta_bias, m.L * sizeof(float)},
                           {m.pos, w->pos, static_cast<size_t>(m.T) * m.H * sizeof(float)}};
     TRY(check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize"));
-    // The twelve arrays lie back to back on the device (create requests them first, in this order, each rounded up to 1024 bytes). A caller
-    // whose host arrays lie the same way gets them in one copy: twelve copies cost more than the smallest step.
-    bool same = true;
-    for (const Item& it : items)
-        same = same && it.h != nullptr && static_cast<const uint8_t*>(it.h) - static_cast<const uint8_t*>(items[0].h) == static_cast<const uint8_t*>(it.d) - static_cast<const uint8_t*>(items[0].d);
-    if (same) {
-        const size_t span = static_cast<size_t>(static_cast<const uint8_t*>(items[11].d) - static_cast<const uint8_t*>(items[0].d)) + items[11].bytes;
-        return check_cuda(cudaMemcpy(items[0].h, items[0].d, span, cudaMemcpyDeviceToHost), "cudaMemcpy(weights)");
-    }
     for (const Item& it : items)
         if (it.h) TRY(check_cuda(cudaMemcpy(it.h, it.d, it.bytes, cudaMemcpyDeviceToHost), "cudaMemcpy(weights)"));
     return BNF4_OK;
+}
+
+// The twelve arrays lie back to back on the device: create requests them first, in this order, each rounded up to 1024 bytes. Twelve copies cost more
+// than the smallest step.
+int bnf4_model_get_weights_block(void* handle, void* block, size_t bytes) {
+    if (!handle || !block) return set_error(BNF4_ERR_INVALID, "model_get_weights_block: null argument");
+    Model& m = *M(handle);
+    const uint8_t *first = reinterpret_cast<const uint8_t*>(m.emb), *last = reinterpret_cast<const uint8_t*>(m.pos);
+    const size_t span = static_cast<size_t>(last - first) + (static_cast<size_t>(m.T) * m.H * sizeof(float) + 1023) / 1024 * 1024;
+    if (bytes != span) return set_error(BNF4_ERR_INVALID, "model_get_weights_block: %zu bytes, the block has %zu", bytes, span);
+    TRY(check_cuda(cudaDeviceSynchronize(), "cudaDeviceSynchronize"));
+    return check_cuda(cudaMemcpy(block, first, span, cudaMemcpyDeviceToHost), "cudaMemcpy(weights)");
 }
 
 int bnf4_model_set_tokens(void* handle, const uint8_t* tokens, const uint8_t* targets, int on_device, void* stream) {

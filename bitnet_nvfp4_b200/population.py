@@ -63,6 +63,7 @@ _l.register({
     "bnf4_model_device_bytes": (C.c_size_t, [c_void_p]),
     "bnf4_model_set_weights": (c_int, [c_void_p, C.POINTER(ModelWeights)]),
     "bnf4_model_get_weights": (c_int, [c_void_p, C.POINTER(ModelWeights)]),
+    "bnf4_model_get_weights_block": (c_int, [c_void_p, c_void_p, C.c_size_t]),
     "bnf4_model_set_tokens": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p]),
     "bnf4_model_prepare_step": (c_int, [c_void_p, C.c_uint64, C.c_uint64, c_int, c_void_p]),
     "bnf4_model_prepare_step_range": (c_int, [c_void_p, C.c_uint64, C.c_uint64, c_int, c_int, c_int, c_void_p]),
@@ -186,13 +187,11 @@ class PopulationModel:
             # one copy straight into page-locked memory (from torch's cache, back to it when the arrays are dropped), without the page
             # faults of fresh pageable arrays: 8 MB 1.8 -> 0.2 ms
             buf = torch.empty(self._layout_bytes, dtype=torch.uint8, pin_memory=True)
-            flat, base = buf.numpy(), buf.data_ptr()
-            arrays = {n: np.ndarray(shape, dt, flat, at) for n, dt, shape, at, _ in self._layout}
-            w = ModelWeights(*[base + at for _, _, _, at, _ in self._layout])
-        else:
-            arrays = {n: np.empty(shape, dt) for n, dt, shape, _, _ in self._layout}
-            w = self._weights_struct(arrays)
-        _l.check(self.lib.bnf4_model_get_weights(self.h, C.byref(w)))
+            flat = buf.numpy()
+            _l.check(self.lib.bnf4_model_get_weights_block(self.h, buf.data_ptr(), self._layout_bytes))
+            return {n: np.ndarray(shape, dt, flat, at) for n, dt, shape, at, _ in self._layout}
+        arrays = {n: np.empty(shape, dt) for n, dt, shape, _, _ in self._layout}
+        _l.check(self.lib.bnf4_model_get_weights(self.h, C.byref(self._weights_struct(arrays))))
         return arrays
 
     def get_optimizer_state(self):

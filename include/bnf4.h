@@ -461,6 +461,9 @@ size_t bnf4_model_device_bytes(void* handle);
 int bnf4_model_set_weights(void* handle, const bnf4_model_weights* h_w);
 /* Copies the current int8 weights / fp32 vectors (and optionally the shadow weights) back to host arrays. Synchronises. */
 int bnf4_model_get_weights(void* handle, bnf4_model_weights* h_w);
+/* The twelve arrays of bnf4_model_weights in one copy: block holds them in the order of the structure's members, each from the next multiple of 1024
+ * bytes; bytes is its size, the last array rounded up likewise. Synchronises. */
+int bnf4_model_get_weights_block(void* handle, void* block, size_t bytes);
 /* tokens / targets: uint8 [B][T] (device pointers when on_device != 0, else host). Out of pinned host memory the copy is queued on the stream: the
  * buffers may be written again when the stream has passed it or bnf4_model_es_step has returned. */
 int bnf4_model_set_tokens(void* handle, const uint8_t* tokens, const uint8_t* targets, int on_device, void* stream);

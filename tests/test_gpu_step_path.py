@@ -130,3 +130,29 @@ def test_a_pinned_batch_may_be_refilled_after_the_step(native):
         results.append([x.cpu().numpy() for x in losses] + state(m))
     for a, b in zip(*results):
         assert np.array_equal(a, b)
+
+
+def test_weights_go_into_the_callers_arrays_and_nowhere_else():
+    """Host arrays that lie like the device's (1024-byte steps) with a caller's data between them, and the one-copy form."""
+    import ctypes as C
+
+    from bitnet_nvfp4_b200 import lib, population
+    cfg, w, _, _, m = make(max_pairs=1, **SMALL)
+    layout, at = [], 0
+    for n, shape in cfg.weight_shapes().items():
+        nbytes = int(np.prod(shape)) * (4 if n in ("head_bias", "beta_bias", "pos") else 1)
+        layout.append((n, shape, at, nbytes))
+        at += -(-nbytes // 1024) * 1024
+    assert any(nbytes % 1024 for _, _, _, nbytes in layout[:-1])
+    block = np.full(at, 0xA5, np.uint8)
+    lib.check(m.lib.bnf4_model_get_weights(m.h, C.byref(population.ModelWeights(*[block.ctypes.data + a for _, _, a, _ in layout]))))
+    one = np.zeros(at, np.uint8)
+    lib.check(m.lib.bnf4_model_get_weights_block(m.h, one.ctypes.data, at))
+    mine = np.ones(at, bool)
+    for n, shape, a, nbytes in layout:
+        want = np.frombuffer(np.ascontiguousarray(w[n]).tobytes(), np.uint8)
+        assert np.array_equal(block[a:a + nbytes], want) and np.array_equal(one[a:a + nbytes], want) and np.array_equal(m.get_weights()[n], w[n])
+        mine[a:a + nbytes] = False
+    assert (block[mine] == 0xA5).all()
+    with pytest.raises(lib.Bnf4Error):
+        lib.check(m.lib.bnf4_model_get_weights_block(m.h, one.ctypes.data, at - 1024))
