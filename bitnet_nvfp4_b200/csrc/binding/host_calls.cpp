@@ -141,7 +141,7 @@ at::Tensor Args::described(PyObject* o) {
 float Args::real() { return to_real(next()); }
 int Args::integer() { return static_cast<int>(to_integer(next())); }
 
-// Uncleared, on the device of `like`, straight from the caching allocator (at::empty takes twice the time on top of it).
+// Uncleared, on the device of `like`, straight from the caching allocator.
 at::Tensor empty_like_device(const at::Tensor& like, at::IntArrayRef sizes, at::ScalarType dtype) {
     int64_t n = 1;
     for (const int64_t d : sizes) n = d < 0 || n < 0 ? -1 : n * d;

@@ -367,6 +367,12 @@ def gather_z_shards(z_all: torch.Tensor, entries, rank: int, world: int, group=N
             dist.all_gather_into_tensor(full, full[rank * per:(rank + 1) * per], group=group)
 
 
+def _own_step(model) -> bool:
+    """Whether the step's phases are PopulationModel's, so that one call of the library may take their place."""
+    return isinstance(model, PopulationModel) and all(getattr(type(model), n) is getattr(PopulationModel, n) and n not in vars(model)
+                                                      for n in ("prepare_step", "eval_pairs", "update"))
+
+
 def es_step(model, seed: int, epoch: int, pairs_total: int, rank: int = 0, world: int = 1, group=None, lr: float = 0.8,
             thresh: float = 0.008, fitness_mode: int = 2, fitness_clip: float = 3.0, losses_out: torch.Tensor | None = None,
             shard_update: bool = True, spans: list | None = None, marks: dict | None = None, **update_kw) -> torch.Tensor:
@@ -378,7 +384,7 @@ def es_step(model, seed: int, epoch: int, pairs_total: int, rank: int = 0, world
     `spans`: optional list that receives (name, start event, end event) around every collective (CUDA devices only).
     `marks`: optional dict that receives the host-clock durations "eval_s" (noise + evaluation + loss gather, the reference's
     eval_s) and "update_s" (shaping + update); asking for them adds two device synchronisations."""
-    if world == 1 and marks is None and isinstance(model, PopulationModel):  # one call, no host round trip
+    if world == 1 and marks is None and _own_step(model):  # one call, no host round trip
         return es_step_native(model, seed, epoch, pairs_total, lr=lr, thresh=thresh, fitness_mode=fitness_mode, fitness_clip=fitness_clip, **update_kw)
     import time
     import torch.distributed as dist

@@ -120,3 +120,30 @@ def test_train_loop_equals_manual_steps():
     assert "val_loss" in recs[0] and "val_loss" not in recs[1] and "val_loss" in recs[2]
     assert all(math.isfinite(r["train_loss"]) and r["tok_s_eval"] > 0 for r in recs)
     a.close(); b.close()
+
+
+def test_a_model_with_phases_of_its_own_is_stepped_through_them():
+    """The one-call step stands in for PopulationModel's phases, not for those of a class or an object that replaced one."""
+    from bitnet_nvfp4_b200 import population
+
+    class Own(population.PopulationModel):
+        def __init__(self):  # (no device)
+            self.h, self.calls = None, []
+
+        def prepare_step(self, seed, epoch, pairs):
+            self.calls.append("prepare")
+
+        def eval_pairs(self, begin, count):
+            self.calls.append("eval")
+            return torch.arange(2 * count, dtype=torch.float32)
+
+        def update(self, weights, lr, thresh, **kw):
+            self.calls.append("update")
+
+    m = Own()
+    assert population.es_step(m, 1, 2, 4).tolist() == list(range(8)) and m.calls == ["prepare", "eval", "update"]
+    plain = object.__new__(population.PopulationModel)
+    plain.h = None
+    assert population._own_step(plain)
+    plain.eval_pairs = m.eval_pairs
+    assert not population._own_step(plain) and not population._own_step(FakeModel())
