@@ -763,9 +763,10 @@ int update_z(Model& m, const float* pair_weights, int shard, int nshards, float*
     const int nz = static_cast<int>(m.h_zdense.size());
     if (m.dense)  // Z[i] = sum_p w_p noise(mix(seed_p, salt), i): the reference's compute_z_sumsq, src/efla_lm_kernels.cu:1854-1890
         return z_dense_table_launch(pair_weights, m.pair_seeds, m.zdense, m.h_zdense.data(), nz, m.pairs_step, m.cfg.use_clt, m.cfg.clt_k, shard, nshards, zb, st);
-    // the fp32 vectors' noise lies in memory when this process evaluated every pair of the step; otherwise it is hashed again
+    // the fp32 vectors' noise lies in memory, as bytes, when this process evaluated every pair of the step; otherwise (and where a sum of draws may
+    // exceed a byte) it is hashed again
     ZTables tables;
-    if (m.eval_begin == 0 && m.eval_end == m.pairs_step) { tables.descs = m.zdense; tables.ndesc = nz; tables.z_all = zb; }
+    if (m.eval_begin == 0 && m.eval_end == m.pairs_step && (m.cfg.use_clt == 0 || m.cfg.clt_k <= 127)) { tables.descs = m.zdense; tables.ndesc = nz; tables.z_all = zb; }
     TRY(z_lowrank_launch(pair_weights, dtab, h.data(), static_cast<int>(h.size()), m.pairs_step, m.r, m.c_r, shard, nshards, tables, m.h_zdense.data(), st));
     if (tables.ndesc > 0) return BNF4_OK;
     return z_dense_table_launch(pair_weights, m.pair_seeds, m.zdense, m.h_zdense.data(), nz, m.pairs_step, m.cfg.use_clt, m.cfg.clt_k, shard, nshards, zb, st);

@@ -66,6 +66,21 @@ def test_noise_sums_from_tables_equal_the_hashed_ones(pairs):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("use_clt,clt_k", [(1, 127), (1, 128), (1, 20000), (0, 20000)])
+def test_noise_sums_of_draws_that_exceed_a_byte(use_clt, clt_k):
+    """20000 ternary draws sum to some 115: one in four sums does not fit the byte that the evaluation reads, and the update takes the sum itself."""
+    import torch
+    w = torch.tensor([0.5, -0.25, 0.125], device="cuda")
+    out = []
+    for count in (3, 0):
+        _, _, _, _, m = make(max_pairs=3, use_clt=use_clt, clt_k=clt_k, **SMALL)
+        m.prepare_step_range(9, 1, 3, 0, count)
+        m.update(w, lr=0.7, thresh=0.001)
+        out.append(state(m))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("kw", [dict(SMALL), dict(hidden=192, layers=2, mlp_mult=3, seq=9, batch=3, heads=3, rank=2), dict(hidden=64, layers=1, seq=32, batch=9, heads=1, rank=4)])
 def test_validation_after_an_update_matches_the_oracle(kw):
     """The update renews the NVFP4 copies of the weights itself: the next forward (one unperturbed member) is the oracle's at the updated
