@@ -8,6 +8,8 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
+import weakref
 from dataclasses import dataclass, asdict
 
 import numpy as np
@@ -88,8 +90,36 @@ _l.register({
     "bnf4_model_get_timing": (c_int, [c_void_p, C.POINTER(C.c_double), C.POINTER(C.c_longlong), c_int]),
 })
 
-# largest weight set that get_weights returns in page-locked memory (results may be kept: a bound on what that locks)
-_PINNED_WEIGHTS = 32 << 20
+# get_weights returns sets of up to _PINNED_WEIGHTS bytes in page-locked memory, as long as the sets in use hold no more than _PINNED_TOTAL (a caller
+# may keep as many as it likes; pageable memory then)
+_PINNED_WEIGHTS, _PINNED_TOTAL = 32 << 20, 128 << 20
+_pinned_lock = threading.RLock()  # (a release may run inside a take: garbage collection)
+_pinned_bytes = 0
+
+
+def _pinned_block(nbytes: int) -> torch.Tensor | None:
+    """Page-locked bytes that count towards _PINNED_TOTAL until the last view of them is dropped, or None."""
+    global _pinned_bytes
+    if nbytes > _PINNED_WEIGHTS:
+        return None
+    with _pinned_lock:
+        if _pinned_bytes + nbytes > _PINNED_TOTAL:
+            return None
+        _pinned_bytes += nbytes
+    try:
+        block = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True)
+    except Exception:
+        _pinned_release(nbytes)
+        raise
+    weakref.finalize(block, _pinned_release, nbytes).atexit = False
+    return block
+
+
+def _pinned_release(nbytes: int) -> None:
+    global _pinned_bytes
+    with _pinned_lock:
+        _pinned_bytes -= nbytes
+
 
 WEIGHT_NAMES = "emb win wq wk wv wbeta ff1 ff2 head head_bias beta_bias pos".split()
 
@@ -175,6 +205,8 @@ class PopulationModel:
         _l.check(self.lib.bnf4_model_set_weights(self.h, C.byref(self._weights_struct(arrays))))
 
     def get_weights(self) -> dict:
+        """The weights as host arrays. Small sets are views of one page-locked block: whoever keeps a single array for long keeps the block, and
+        copies it to avoid that."""
         if self._layout is None:  # (name, dtype, shape, offset, bytes) of the arrays, laid out as the device holds them
             self._layout, at = [], 0
             for n, shape in self.cfg.weight_shapes().items():
@@ -183,10 +215,10 @@ class PopulationModel:
                 self._layout.append((n, dt, shape, at, nbytes))
                 at += -(-nbytes // 1024) * 1024
             self._layout_bytes = at
-        if self._layout_bytes <= _PINNED_WEIGHTS:
+        buf = _pinned_block(self._layout_bytes)
+        if buf is not None:
             # one copy straight into page-locked memory (from torch's cache, back to it when the arrays are dropped), without the page
             # faults of fresh pageable arrays: 8 MB 1.8 -> 0.2 ms
-            buf = torch.empty(self._layout_bytes, dtype=torch.uint8, pin_memory=True)
             flat = buf.numpy()
             _l.check(self.lib.bnf4_model_get_weights_block(self.h, buf.data_ptr(), self._layout_bytes))
             return {n: np.ndarray(shape, dt, flat, at) for n, dt, shape, at, _ in self._layout}

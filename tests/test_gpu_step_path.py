@@ -171,3 +171,27 @@ def test_weights_go_into_the_callers_arrays_and_nowhere_else():
     assert (block[mine] == 0xA5).all()
     with pytest.raises(lib.Bnf4Error):
         lib.check(m.lib.bnf4_model_get_weights_block(m.h, one.ctypes.data, at - 1024))
+
+
+def test_kept_weights_do_not_pile_up_page_locked_memory(monkeypatch):
+    import gc
+
+    import torch
+    from bitnet_nvfp4_b200 import population
+    _, w, _, _, m = make(max_pairs=1, **SMALL)
+    gc.collect()
+    size = sum(-(-a.nbytes // 1024) * 1024 for a in m.get_weights().values())
+    gc.collect()
+    assert population._pinned_bytes == 0
+    monkeypatch.setattr(population, "_PINNED_TOTAL", 3 * size)
+    kept = [m.get_weights() for _ in range(5)]
+    assert population._pinned_bytes == 3 * size
+    assert [torch.from_numpy(k["emb"]).is_pinned() for k in kept] == [True] * 3 + [False] * 2
+    assert all(np.array_equal(k[n], w[n]) for k in kept for n in w)
+    one = kept[0]["head"]
+    del kept
+    gc.collect()
+    assert population._pinned_bytes == size
+    del one
+    gc.collect()
+    assert population._pinned_bytes == 0
