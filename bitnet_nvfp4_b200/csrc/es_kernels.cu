@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -93,24 +94,27 @@ __global__ void __launch_bounds__(1024) ce_step_kernel(const float* __restrict__
 // again after it): the member's last block forms the mean; without them split is 1, partial[member * 16 + group] holds the groups'
 // sums and ce_finalize_kernel follows. With split > 1 partial holds the chains' sums, 128 per member.
 constexpr int kCeChunks = 16;
+// SHARED false: the instance for split 1 (with the split as a variable the default model's 1048576 rows took 121 instead of 97 us).
+template <bool SHARED>
 struct CeRows {
     int split, r0, r1, chain, j;  // this warp: rows r0 + chain + 8 (j + split k) below r1
     __device__ explicit CeRows(int rows_per_member) {
         const int warp = threadIdx.x >> 5, per = (rows_per_member + kCeChunks - 1) / kCeChunks;
-        split = static_cast<int>(gridDim.x) / kCeChunks;
+        split = SHARED ? static_cast<int>(gridDim.x) / kCeChunks : 1;
         const int group = static_cast<int>(blockIdx.x) / split, sub = static_cast<int>(blockIdx.x) - group * split;
         r0 = group * per;
         r1 = min(rows_per_member, r0 + per);
         chain = sub * (8 / split) + warp / split;
         j = warp % split;
     }
-    __device__ int row(int k) const { return r0 + chain + 8 * (j + split * k); }
-    __device__ int passes(int rpi) const { return (r1 - r0 + 8 * split * rpi - 1) / (8 * split * rpi); }  // (uniform in the block)
+    __device__ int row(int k) const { return r0 + chain + 8 * (SHARED ? j + split * k : k); }
+    // whether a pass over rows row(k0), .. has any (of this warp; SHARED: of the block, which passes together)
+    __device__ bool more(int k0) const { return SHARED ? r0 + 8 * split * k0 < r1 : row(k0) < r1; }
 };
 // adds the row losses l[i] of rows row(k0 + i) to the chain's sum (kept by its first warp)
-template <int RPI>
-__device__ __forceinline__ void ce_add(const CeRows& rr, int pass, const float (&l)[RPI], float& acc) {
-    if (rr.split == 1) {
+template <bool SHARED, int RPI>
+__device__ __forceinline__ void ce_add(const CeRows<SHARED>& rr, int pass, const float (&l)[RPI], float& acc) {
+    if constexpr (!SHARED) {
 #pragma unroll
         for (int i = 0; i < RPI; ++i) acc += l[i];
         return;
@@ -126,14 +130,15 @@ __device__ __forceinline__ void ce_add(const CeRows& rr, int pass, const float (
         for (int i = 0; i < RPI; ++i)
             for (int q = 0; q < rr.split; ++q) acc += rows[pass & 1][warp + q][i];
 }
-__device__ __forceinline__ void ce_finish(const CeRows& rr, float acc, float* partial, unsigned* counters, int rows_per_member, float* loss_mean) {
+template <bool SHARED>
+__device__ __forceinline__ void ce_finish(const CeRows<SHARED>& rr, float acc, float* partial, unsigned* counters, int rows_per_member, float* loss_mean) {
     __shared__ float part[8];
     __shared__ bool last;
     const int member = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0 && rr.j == 0) part[warp / rr.split] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (rr.split == 1) {
+        if constexpr (!SHARED) {
             float t = 0.0f;
             for (int w = 0; w < 8; ++w) t += part[w];
             partial[member * kCeChunks + blockIdx.x] = t;
@@ -153,7 +158,7 @@ __device__ __forceinline__ void ce_finish(const CeRows& rr, float acc, float* pa
     __threadfence();
     float group = 0.0f;
     if (lane < kCeChunks) {
-        if (rr.split == 1) group = __ldcg(partial + member * kCeChunks + lane);
+        if (!SHARED) group = __ldcg(partial + member * kCeChunks + lane);
         else
             for (int w = 0; w < 8; ++w) group += __ldcg(partial + member * (8 * kCeChunks) + 8 * lane + w);
     }
@@ -162,24 +167,24 @@ __device__ __forceinline__ void ce_finish(const CeRows& rr, float acc, float* pa
     for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
     if (lane == 0) loss_mean[member] = static_cast<float>(t / static_cast<double>(rows_per_member));
 }
+template <bool SHARED>
 __global__ void __launch_bounds__(256) ce_population_kernel(const float* __restrict__ logits, int ld, const float* __restrict__ bias,
                                                             const int8_t* __restrict__ bias_noise, float sigma,
                                                             const uint8_t* __restrict__ targets, int vocab, int rows_per_member,
                                                             float* partial, unsigned* counters, float* loss_mean) {
     pdl_wait();
     after(logits, bias, bias_noise, targets);
-    const CeRows rr(rows_per_member);
+    const CeRows<SHARED> rr(rows_per_member);
     const int lane = threadIdx.x & 31, member = blockIdx.y;
     const float bns = (member & 1) ? -sigma : sigma;
     const int8_t* nz = bias_noise != nullptr ? bias_noise + static_cast<size_t>(member >> 1) * vocab : nullptr;
     float acc = 0.0f;
-    const int passes = rr.passes(1);
-    for (int k = 0; k < passes; ++k) {
+    for (int k = 0; rr.more(k); ++k) {
         const int r = rr.row(k);
         float l[1] = {0.0f};
         if (r < rr.r1)
             l[0] = ce_row_loss(logits + (static_cast<size_t>(member) * rows_per_member + r) * ld, bias, nullptr, nz, bns, vocab, static_cast<int>(targets[r]), lane);
-        ce_add<1>(rr, k, l, acc);
+        ce_add<SHARED, 1>(rr, k, l, acc);
     }
     ce_finish(rr, acc, partial, counters, rows_per_member, loss_mean);
 }
@@ -188,14 +193,14 @@ __global__ void __launch_bounds__(256) ce_population_kernel(const float* __restr
 // l, l + 32, ... of a row (NV4 groups), the member's bias and noise stay in registers for all rows, and RPI rows are in
 // flight per warp so that the load latency of one row hides behind the reductions of the others. The warps walk the
 // rows in the same order and add the row losses in the same order as ce_population_kernel.
-template <int NV4, int RPI>
+template <int NV4, int RPI, bool SHARED>
 __global__ void __launch_bounds__(256) ce_population_vec_kernel(const float* __restrict__ logits, int ld, const float* __restrict__ bias,
                                                                 const int8_t* __restrict__ bias_noise, float sigma,
                                                                 const uint8_t* __restrict__ targets, int vocab, int rows_per_member,
                                                                 float* partial, unsigned* counters, float* loss_mean) {
     pdl_wait();
     after(logits, bias, bias_noise, targets);
-    const CeRows rr(rows_per_member);
+    const CeRows<SHARED> rr(rows_per_member);
     const int lane = threadIdx.x & 31, member = blockIdx.y, r1 = rr.r1;
     const float bns = (member & 1) ? -sigma : sigma;
     const int groups = vocab >> 2;
@@ -213,8 +218,7 @@ __global__ void __launch_bounds__(256) ce_population_vec_kernel(const float* __r
         }
     }
     float acc = 0.0f;
-    const int passes = rr.passes(RPI);
-    for (int pass = 0; pass < passes; ++pass) {
+    for (int pass = 0; rr.more(pass * RPI); ++pass) {
         float l[RPI];
         float4 x[RPI][NV4];
         int y[RPI];
@@ -255,7 +259,7 @@ __global__ void __launch_bounds__(256) ce_population_vec_kernel(const float* __r
             if (bias_noise != nullptr) vy = fmaf(bns, static_cast<float>(bias_noise[static_cast<size_t>(member >> 1) * vocab + y[i]]), vy);
             l[i] = rr.row(pass * RPI + i) < r1 ? -(vy - mx - logf(sum + 1e-9f)) : 0.0f;
         }
-        ce_add<RPI>(rr, pass, l, acc);
+        ce_add<SHARED, RPI>(rr, pass, l, acc);
     }
     ce_finish(rr, acc, partial, counters, rows_per_member, loss_mean);
 }
@@ -888,16 +892,17 @@ int cross_entropy_launch(const float* logits, int ld, const float* bias, const i
     const bool early = static_cast<long long>(members) * rows_per_member * vocab <= kPdlStreamElems;
     const bool vec = (vocab % 4) == 0 && (ld % 4) == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(bias_noise) & 3) == 0;
-    if (vec && vocab <= 128)
-        launch_pdl_if(early, ce_population_vec_kernel<1, 4>, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean);
-    else if (vec && vocab <= 256)
-        launch_pdl_if(early, ce_population_vec_kernel<2, 4>, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean);
-    else if (vec && vocab <= 512)
-        launch_pdl_if(early, ce_population_vec_kernel<4, 2>, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean);
-    else if (vec)
-        launch_pdl_if(early, ce_population_vec_kernel<8, 1>, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean);
-    else
-        launch_pdl_if(early, ce_population_kernel, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean);
+    auto run = [&](auto kernel) { launch_pdl_if(early, kernel, grid, 256, 0, st, logits, ld, bias, bias_noise, sigma, targets, vocab, rows_per_member, partial, counters, loss_mean); };
+    auto pick = [&](auto shared) {
+        constexpr bool SH = decltype(shared)::value;
+        if (vec && vocab <= 128) run(ce_population_vec_kernel<1, 4, SH>);
+        else if (vec && vocab <= 256) run(ce_population_vec_kernel<2, 4, SH>);
+        else if (vec && vocab <= 512) run(ce_population_vec_kernel<4, 2, SH>);
+        else if (vec) run(ce_population_vec_kernel<8, 1, SH>);
+        else run(ce_population_kernel<SH>);
+    };
+    if (split > 1) pick(std::true_type());
+    else pick(std::false_type());
     return check_launch("ce_population_kernel");
 }
 
