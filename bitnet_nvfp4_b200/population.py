@@ -215,13 +215,12 @@ class PopulationModel:
                 self._layout.append((n, dt, shape, at, nbytes))
                 at += -(-nbytes // 1024) * 1024
             self._layout_bytes = at
-        buf = _pinned_block(self._layout_bytes)
-        if buf is not None:
+        block = _pinned_block(self._layout_bytes)
+        if block is not None:
             # one copy straight into page-locked memory (from torch's cache, back to it when the arrays are dropped), without the page
             # faults of fresh pageable arrays: 8 MB 1.8 -> 0.2 ms
-            flat = buf.numpy()
-            _l.check(self.lib.bnf4_model_get_weights_block(self.h, buf.data_ptr(), self._layout_bytes))
-            return {n: np.ndarray(shape, dt, flat, at) for n, dt, shape, at, _ in self._layout}
+            _l.check(self.lib.bnf4_model_get_weights_block(self.h, block.ctypes.data, self._layout_bytes))
+            return {n: np.ndarray(shape, dt, block, at) for n, dt, shape, at, _ in self._layout}
         arrays = {n: np.empty(shape, dt) for n, dt, shape, _, _ in self._layout}
         _l.check(self.lib.bnf4_model_get_weights(self.h, C.byref(self._weights_struct(arrays))))
         return arrays
