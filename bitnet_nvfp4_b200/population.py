@@ -97,7 +97,7 @@ _pinned_lock = threading.RLock()  # (a release may run inside a take: garbage co
 _pinned_bytes = 0
 
 
-def _pinned_block(nbytes: int) -> torch.Tensor | None:
+def _pinned_block(nbytes: int) -> np.ndarray | None:
     """Page-locked bytes that count towards _PINNED_TOTAL until the last view of them is dropped, or None."""
     global _pinned_bytes
     if nbytes > _PINNED_WEIGHTS:
@@ -107,7 +107,7 @@ def _pinned_block(nbytes: int) -> torch.Tensor | None:
             return None
         _pinned_bytes += nbytes
     try:
-        block = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True)
+        block = torch.empty(nbytes, dtype=torch.uint8, pin_memory=True).numpy()  # (views of it keep the array alive, not the tensor object)
     except Exception:
         _pinned_release(nbytes)
         raise
