@@ -268,9 +268,12 @@ constexpr uint32_t kIdescPair256 = kIdescPairM | (256u >> 3 << 17), kIdescPair12
 struct PairMaps {
     CUtensorMap sfa, sfb;
 };
-struct NoMaps {
+struct B2Map {
     CUtensorMap b2;  // the second B operand (GemmParams::b2)
 };
+struct NoMaps {};
+template <bool PAIR, bool B2>
+using ExtraMaps = std::conditional_t<PAIR, PairMaps, std::conditional_t<B2, B2Map, NoMaps>>;
 
 struct KernelArgs {
     GemmParams p;
@@ -302,18 +305,20 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 // accumulators while the sixteen epilogue warps drain the other one.
 // RK: 4 = the instance for rank-4 perturbation terms whose pairs start at multiples of 32 rows;
 // 1 = the instance for the batched driver's common case (rank 1, no C operand, every 128-row tile inside one member), which carries
-// none of the general paths; 0 = everything else.
+// none of the general paths; 0 = no rank term at all, 2 = every other one. (262144 x 1024 x 512 with GELU to FP4, no rank term: 303 us as a case
+// of the general instance, which spills, 256 us.)
+// B2: the instance with a second B operand (no rank term); the others carry no tests for one (rank 2 with GELU to FP4 446 -> 412 us).
 // PAIR: the instance for operands with many K blocks. On the in-order pipe a scale copy costs about 44 cycles and an M 128 x N 128 MMA
 // 64 (measured, one CTA): 8 copies and 4 MMAs per 256-element K block of a 128 x 128 tile take 560 cycles before any operand
 // traffic, 860 with it. A CTA pair (cta_group::2) on a 256 x 256 tile needs 12 copies and 4 MMAs of N 256 for four times the work; the
 // long MMAs hide most of the copies: 718 cycles (968 with twice as many N 128 MMAs), and each CTA loads 38 instead of 68 KB.
 // Accumulators: even tiles use the 128-column blocks 0 and 1, odd tiles 1 and 2, and the epilogue drains block 1 first, so that the
 // next tile starts as soon as the shared block has been read. The epilogue code sees a sequence of 128 x 128 sub-tiles.
-template <int EPI, int RK, bool PAIR>
+template <int EPI, int RK, bool PAIR, bool B2>
 __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                  const __grid_constant__ CUtensorMap map_b,
                                                                  const __grid_constant__ CUtensorMap map_d,
-                                                                 const __grid_constant__ std::conditional_t<PAIR, PairMaps, NoMaps> maps_sf,
+                                                                 const __grid_constant__ ExtraMaps<PAIR, B2> maps_sf,
                                                                  const KernelArgs args) {
     constexpr int kAcc = PAIR ? kPairAcc : 2;  // TMEM accumulators
     constexpr int oSmemEpi = PAIR ? kPairSmemEpi : kSmemEpi, oSmemLora = PAIR ? kPairSmemLora : kSmemLora, oSmemBar = PAIR ? kPairSmemBar : kSmemBar;
@@ -324,7 +329,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
     const GemmParams& p = args.p;
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int num_ks = ((p.k + BK - 1) / BK) << (!PAIR && args.ks_wrap > 0 ? 1 : 0);  // K blocks of a tile (both B operands)
+    const int num_ks = ((p.k + BK - 1) / BK) << (B2 ? 1 : 0);  // K blocks of a tile (both B operands)
     const int total_tiles = args.total_tiles;
 
     const uint32_t bar_full = smem_base + oSmemBar;               // kStages x 8 bytes (PAIR: the leading CTA's count for both)
@@ -494,8 +499,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 int atoms_left = args.k_atoms, x = 0, by = ny;
                 const CUtensorMap* bmap = &map_b;
                 for (int ks = 0; ks < num_ks; ++ks, ++kc, x += 128) {
-                    if constexpr (!PAIR) {
-                        if (ks > 0 && ks == args.ks_wrap) {
+                    if constexpr (B2) {
+                        if (ks == args.ks_wrap) {
                             const int member = my / p.rows_per_member;
                             x = 0;
                             by = member * p.b2_rows + ny;
@@ -553,7 +558,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * s, full_parity, 2));
                     if (!ok) break;
                     tc_fence_after();
-                    const int nk = min(4, (p.k - (ks >= args.ks_wrap ? ks - args.ks_wrap : ks) * BK) / UMMA_K);
+                    const int nk = min(4, (p.k - (B2 && ks >= args.ks_wrap ? ks - args.ks_wrap : ks) * BK) / UMMA_K);
                     const uint32_t t_sfa = tmem_base + kSfCol + s * 32;
                     const uint32_t t_sfb = t_sfa + 16;
                     const uint64_t sfa_d = sfadesc0 + static_cast<uint64_t>(s * (kStageSfBytes >> 4));
@@ -668,7 +673,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             cx.member = 0;
             cx.tr[0] = cx.tr[1] = cx.tr[2] = cx.tr[3] = 0;
             cx.aval[0] = cx.aval[1] = cx.aval[2] = cx.aval[3] = 0;
-            if (p.rank <= 0 || !valid) return;
+            if (!valid) return;
             const int m0_ = t.m_tile * BM, col0_ = t.n_tile * BN + c * 32;
             const int row_ = m0_ + row_in_tile;  // (rows fit 31 bits: p.m is an int)
             cx.member = member_of(static_cast<unsigned>(min(row_, p.m - 1)));  // (rows past m are never stored)
@@ -687,9 +692,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         };
         // The common case (rank 1, tiles inside one member) with as few instructions as possible: this phase sits on the serial
         // path of every tile.
-        constexpr bool R4 = RK == 4, R1 = RK == 1;
-        const bool fast_ctx = R1 || (p.rank == 1 && tile_uniform_member);
-        const int* t_row = p.rank > 0 ? p.lora_t + static_cast<size_t>(row_in_tile) * p.t_stride : nullptr;
+        constexpr bool R4 = RK == 4, R1 = RK == 1, R0 = RK == 0;
+        const bool fast_ctx = R1 || (RK == 2 && p.rank == 1 && tile_uniform_member);
+        const int* t_row = !R0 && p.rank > 0 ? p.lora_t + static_cast<size_t>(row_in_tile) * p.t_stride : nullptr;
         auto fetch_fast = [&](const TileIdx& t, bool valid, LoraCtx& cx) {
             cx.member = 0;
             cx.tr[0] = 0;
@@ -745,7 +750,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         LoraCtx nxt;
         nxt.tr[1] = nxt.tr[2] = nxt.tr[3] = 0;
         nxt.aval[1] = nxt.aval[2] = nxt.aval[3] = 0;
-        if (R1 || fast_ctx) fetch_fast(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles, nxt);
+        if constexpr (R0) nxt.member = 0;
+        else if (R1 || fast_ctx) fetch_fast(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles, nxt);
         else fetch_ctx(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles, nxt);
         uint32_t pfull = 0;  // PAIR: parities of the completions to wait for (bit per accumulator block)
         uint32_t acc_empty_bar = bar_acc_empty;
@@ -762,14 +768,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             const bool chunk_ok = col0 < p.n;  // warp-uniform
 
             const int member = nxt.member, pair = member >> 1;
-            float tr[4] = {static_cast<float>(nxt.tr[0]), 0.0f, 0.0f, 0.0f};
+            float tr[4] = {R0 ? 0.0f : static_cast<float>(nxt.tr[0]), 0.0f, 0.0f, 0.0f};
             float* loraA_sh = reinterpret_cast<float*>(smem_gen + oSmemLora) + ew * 4 * 32;  // this warp's [4][32]
-            if (R1 || fast_ctx) {
+            if (R0) {
+            } else if (R1 || fast_ctx) {
                 __syncwarp();  // the previous tile's reads are done
                 loraA_sh[lane] = static_cast<float>(nxt.aval[0]);
                 __syncwarp();
                 fetch_fast(nxt_t, more, nxt);
-            } else if (p.rank > 0) {
+            } else {
                 tr[1] = static_cast<float>(nxt.tr[1]);
                 tr[2] = static_cast<float>(nxt.tr[2]);
                 tr[3] = static_cast<float>(nxt.tr[3]);
@@ -852,7 +859,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     const float2 hi = __ffma2_rn(ls2, __fmul2_rn(tr2, make_float2(a4.z, a4.w)), make_float2(v[4 * j + 2], v[4 * j + 3]));
                     v[4 * j + 0] = lo.x; v[4 * j + 1] = lo.y; v[4 * j + 2] = hi.x; v[4 * j + 3] = hi.y;
                 }
-            } else if (p.rank > 0) {
+            } else if constexpr (!R0) {
                 // sum_r t[r]*A[n][r] is an integer below 2^24: float products and sums are exact. Rows of another pair (and rows past m)
                 // take part with a zero factor.
                 const int pair_hi = R4 ? 0 : __shfl_sync(0xffffffffu, pair, 31);  // (the rank-4 instance runs with 32 rows inside one pair)
@@ -1007,11 +1014,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 const uint32_t tab_c = smem_base + oSmemEpi - (static_cast<uint32_t>(kRoundBiasBits) << 3);
                 int w[8];
                 uint32_t sfv[2] = {0u, 0u}, codes[4] = {0u, 0u, 0u, 0u};
+                int4 nb0 = make_int4(0, 0, 0, 0), nb1 = nb0;  // R1: the next projection's vector
 #pragma unroll
                 for (int blk = 0; blk < 2; ++blk) {
                     float tb[16];
                     float am = 0.0f;  // max |value| of the block
                     uint32_t bad = 0;
+                    // (requested behind the second block's math: 262144 x 1024 x 512 277.9 us with the loads where they are used, 273 in front of both
+                    // blocks, 281 in front of the accumulator wait, 271 here)
+                    if constexpr (R1 && EPI == EPI_GELU_FP4) {
+                        if (blk == 1) {
+                            const int4* bv = reinterpret_cast<const int4*>(p.next_tvec + static_cast<size_t>(pair) * p.next_tvec_pair_stride + col0);
+                            nb0 = __ldg(bv);
+                            nb1 = __ldg(bv + 1);
+                        }
+                    }
 #pragma unroll
                     for (int g = 0; g < 4; ++g) {
                         const int j = 16 * blk + 4 * g;
@@ -1074,7 +1091,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                             const int nv_ = R1 ? 1 : p.next_nvec;  // (the rank-1 instance runs with at most one projection)
                             for (int vv = 0; vv < nv_; ++vv) {
                                 const int4* bv = reinterpret_cast<const int4*>(tv + static_cast<size_t>(vv) * p.n);
-                                const int4 b0 = __ldg(bv), b1 = __ldg(bv + 1);
+                                const int4 b0 = R1 ? nb0 : __ldg(bv), b1 = R1 ? nb1 : __ldg(bv + 1);
                                 int a = 0;
                                 a = __dp4a(w[0], b0.x, a); a = __dp4a(w[1], b0.y, a); a = __dp4a(w[2], b0.z, a); a = __dp4a(w[3], b0.w, a);
                                 a = __dp4a(w[4], b1.x, a); a = __dp4a(w[5], b1.y, a); a = __dp4a(w[6], b1.z, a); a = __dp4a(w[7], b1.w, a);
@@ -1167,13 +1184,13 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint
     return BNF4_OK;
 }
 
-template <int EPI, int RK, bool PAIR = false>
-int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, const std::conditional_t<PAIR, PairMaps, NoMaps>& msf, const KernelArgs& args,
+template <int EPI, int RK, bool PAIR, bool B2>
+int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, const ExtraMaps<PAIR, B2>& msf, const KernelArgs& args,
              dim3 grid, int dev, cudaStream_t stream) {
     constexpr int smem = PAIR ? kPairSmemAlloc : kSmemAlloc;
     static bool configured[64] = {};  // function attributes are per device: set once for each device this process uses
     if (!configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_nvfp4_kernel<EPI, RK, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t e = cudaFuncSetAttribute(gemm_nvfp4_kernel<EPI, RK, PAIR, B2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(gemm_nvfp4_kernel)");
         configured[dev] = true;
     }
@@ -1189,10 +1206,10 @@ int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md
         attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, gemm_nvfp4_kernel<EPI, RK, PAIR>, ma, mb, md, msf, args);
+        cudaLaunchKernelEx(&cfg, gemm_nvfp4_kernel<EPI, RK, PAIR, B2>, ma, mb, md, msf, args);
     } else {
         // (an early launch pays while the kernel is short: a dozen tiles per SM)
-        launch_pdl_if(args.total_tiles <= 12 * static_cast<int>(grid.x), gemm_nvfp4_kernel<EPI, RK, PAIR>, grid, kThreads, smem, stream, ma, mb, md, msf, args);
+        launch_pdl_if(args.total_tiles <= 12 * static_cast<int>(grid.x), gemm_nvfp4_kernel<EPI, RK, PAIR, B2>, grid, kThreads, smem, stream, ma, mb, md, msf, args);
     }
     return check_launch("gemm_nvfp4_kernel");
 }
@@ -1279,7 +1296,7 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     if (sms <= 0) return BNF4_ERR_CUDA;
     const bool gelu = p.epilogue == EPI_GELU_FP4 || p.epilogue == EPI_GELU_I8;
     const bool gelu_plain = !gelu || (p.act_scale <= 700.0f && (p.n % 32) == 0 && (p.epilogue == EPI_GELU_FP4 ? (p.next_nvec == 1 && p.d_i8 == nullptr) : p.next_nvec <= 1));
-    const int rk = p.rank == 4 && (p.rows_per_member % 16) == 0 ? 4 : ((p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1)) ? 1 : 0);
+    const int rk = p.rank == 4 && (p.rows_per_member % 16) == 0 ? 4 : ((p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1)) ? 1 : (p.rank > 0 ? 2 : 0));
     // CTA pairs pay where the mainloop is longer than the epilogue and there is a tile for every pair. Measured at 65536 x 512 (us, single
     // CTAs -> pairs): fp32 / half / residual epilogues, rank 1: K 512 33.9 -> 35.9, 25.6 -> 27.0, 29.0 -> 29.8; K 1024 42.7 -> 38.2,
     // 33.1 -> 30.2, 36.1 -> 33.1; K 4096 107 -> 80, 96 -> 70, 98 -> 74. Rank 4 with the last two: K 1024 37.2 -> 39.2, 43.3 -> 45.4, K 1536
@@ -1287,7 +1304,10 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     const long long pair_tiles = static_cast<long long>((p.n + 255) / 256) * ((p.m + 255) / 256);
     const int pair_k = gelu ? 2048 : (p.rank > 1 && p.epilogue != EPI_F32 ? 1536 : 1024);
     const bool pair = p.b2 == nullptr && p.k >= pair_k && pair_tiles >= sms / 2 && (rk != 1 || (p.m % 256) == 0);
-    // the epilogue (and with it the kernel) is a template argument
+    // the epilogue and the form of the rank term are template arguments
+    auto with_rank = [&](auto run) -> int {
+        return rk == 4 ? run(std::integral_constant<int, 4>()) : rk == 1 ? run(std::integral_constant<int, 1>()) : rk == 2 ? run(std::integral_constant<int, 2>()) : run(std::integral_constant<int, 0>());
+    };
     auto with_epilogue = [&](auto run) -> int {
         switch (p.epilogue) {
             case EPI_F32: return run(std::integral_constant<int, EPI_F32>());
@@ -1309,24 +1329,29 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
         const dim3 grid(2 * static_cast<unsigned>(std::min<long long>(pair_tiles, sms / 2)), 1, 1);
         return with_epilogue([&](auto epi) -> int {
             constexpr int E = decltype(epi)::value;
-            return rk == 4 ? launch_t<E, 4, true>(ma, mb, md, msf, args, grid, dev, stream)
-                           : (rk == 1 ? launch_t<E, 1, true>(ma, mb, md, msf, args, grid, dev, stream) : launch_t<E, 0, true>(ma, mb, md, msf, args, grid, dev, stream));
+            auto run = [&](auto r) { return launch_t<E, decltype(r)::value, true, false>(ma, mb, md, msf, args, grid, dev, stream); };
+            return with_rank(run);
         });
     }
     const dim3 grid(static_cast<unsigned>(std::min<long long>(tiles, sms)), 1, 1);
-    NoMaps none;
-    none.b2 = mb;  // unused
     if (p.b2 != nullptr) {
-        if (p.sfb2 == nullptr || (p.b2_rows % 128) != 0 || p.b2_rows < p.n || p.rows_per_member <= 0 || (p.rows_per_member % BM) != 0)
-            return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: the second operand needs member rows and b2_rows in multiples of 128");
+        if (p.sfb2 == nullptr || (p.b2_rows % 128) != 0 || p.b2_rows < p.n || p.rows_per_member <= 0 || (p.rows_per_member % BM) != 0 || p.rank > 0)
+            return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: the second operand needs member rows and b2_rows in multiples of 128 and takes no rank term");
+        B2Map b2;
         const uint64_t members = (static_cast<uint64_t>(p.m) + p.rows_per_member - 1) / p.rows_per_member;
-        rc = make_map_2d(&none.b2, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.b2, static_cast<uint64_t>(p.k) / 2, members * p.b2_rows, static_cast<uint64_t>(p.k) / 2, 128, BN, "B2");
+        rc = make_map_2d(&b2.b2, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.b2, static_cast<uint64_t>(p.k) / 2, members * p.b2_rows, static_cast<uint64_t>(p.k) / 2, 128, BN, "B2");
         if (rc) return rc;
+        switch (p.epilogue) {  // (the dense form's)
+            case EPI_F32: return launch_t<EPI_F32, 0, false, true>(ma, mb, md, b2, args, grid, dev, stream);
+            case EPI_GELU_FP4: return launch_t<EPI_GELU_FP4, 0, false, true>(ma, mb, md, b2, args, grid, dev, stream);
+            case EPI_ADD_I8: return launch_t<EPI_ADD_I8, 0, false, true>(ma, mb, md, b2, args, grid, dev, stream);
+        }
+        return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: no second operand with epilogue %d", p.epilogue);
     }
     return with_epilogue([&](auto epi) -> int {
         constexpr int E = decltype(epi)::value;
-        return rk == 4 ? launch_t<E, 4>(ma, mb, md, none, args, grid, dev, stream)
-                       : (rk == 1 ? launch_t<E, 1>(ma, mb, md, none, args, grid, dev, stream) : launch_t<E, 0>(ma, mb, md, none, args, grid, dev, stream));
+        auto run = [&](auto r) { return launch_t<E, decltype(r)::value, false, false>(ma, mb, md, NoMaps{}, args, grid, dev, stream); };
+        return with_rank(run);
     });
 }
 
