@@ -3,6 +3,8 @@
 Bars: per-member mean cross-entropy within 1e-4 relative of the oracle; after an update driven by the
 oracle's own fitness vector the int8 weights are bit-identical to the oracle's.
 """
+import functools
+
 import numpy as np
 import pytest
 
@@ -275,8 +277,8 @@ def test_checkpoint_resume_is_bit_identical(tmp_path):
 
 
 def test_single_call_es_step_equals_the_composed_calls():
-    """bnf4_model_es_step (noise, evaluation, host-side shaping, update in one C call) against population.es_step, which composes
-    the same phases from Python: losses and weights bit-identical over two steps."""
+    """bnf4_model_es_step (noise, evaluation, shaping, update in one C call) against the phases composed from Python, which population.es_step
+    does when it is asked for their durations (marks): losses and weights bit-identical over two steps."""
     from bitnet_nvfp4_b200 import population, synth
     cfg = population.Config(hidden=128, layers=2, seq=16, batch=4, heads=2, rank=1, max_pairs=8)
     w = synth.init_weights(cfg)
@@ -286,7 +288,7 @@ def test_single_call_es_step_equals_the_composed_calls():
         m = population.PopulationModel(cfg)
         m.set_weights(w)
         m.set_tokens(tok, tgt)
-        step = population.es_step_native if native else population.es_step
+        step = population.es_step_native if native else functools.partial(population.es_step, marks={})
         losses = [step(m, 3, e, 8, lr=0.5, thresh=0.004).cpu().numpy().copy() for e in range(2)]
         out.append((losses, m.get_weights(), m.get_optimizer_state()))
         m.close()
