@@ -141,27 +141,41 @@ at::Tensor Args::described(PyObject* o) {
 float Args::real() { return to_real(next()); }
 int Args::integer() { return static_cast<int>(to_integer(next())); }
 
-// Uncleared, on the device of `like`, straight from the caching allocator.
+// Uncleared bytes on a device, straight from the caching allocator, and a tensor on a part of them.
+c10::Storage device_bytes(const at::Device& device, int64_t bytes) {
+    c10::cuda::OptionalCUDAGuard guard;
+    if (device.index() != c10::cuda::current_device()) guard.set_device(device);
+    c10::Allocator* from = c10::cuda::CUDACachingAllocator::get();
+    return c10::Storage(c10::make_intrusive<c10::StorageImpl>(c10::StorageImpl::use_byte_size_t(), bytes, from->allocate(static_cast<size_t>(bytes)), from, /*resizable=*/true));
+}
+at::Tensor part(c10::Storage storage, int64_t offset, at::IntArrayRef sizes, at::ScalarType dtype) {  // offset in elements
+    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(std::move(storage), c10::DispatchKeySet(c10::DispatchKey::CUDA), c10::scalarTypeToTypeMeta(dtype));
+    t.unsafeGetTensorImpl()->set_storage_offset(offset);
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+    return t;
+}
 at::Tensor empty_like_device(const at::Tensor& like, at::IntArrayRef sizes, at::ScalarType dtype) {
     int64_t n = 1;
     for (const int64_t d : sizes) n = d < 0 || n < 0 ? -1 : n * d;
     if (!like.is_cuda() || n < 0) return at::empty(sizes, like.options().dtype(dtype));  // (with its errors)
-    const size_t bytes = static_cast<size_t>(n) * c10::elementSize(dtype);
-    const c10::cuda::CUDAGuard guard(like.device());
-    c10::Allocator* from = c10::cuda::CUDACachingAllocator::get();
-    at::Tensor t = at::detail::make_tensor<c10::TensorImpl>(
-        c10::Storage(c10::make_intrusive<c10::StorageImpl>(c10::StorageImpl::use_byte_size_t(), bytes, from->allocate(bytes), from, /*resizable=*/true)),
-        c10::DispatchKeySet(c10::DispatchKey::CUDA), c10::scalarTypeToTypeMeta(dtype));
-    t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
-    return t;
+    return part(device_bytes(like.device(), n * static_cast<int64_t>(c10::elementSize(dtype))), 0, sizes, dtype);
 }
-// Outputs of a quantiser, each with a storage of its own. Nothing is cleared: the library writes every value, code and scale byte, padding included.
+// Outputs of a quantiser: the int8 values, and the operand of a GEMM, whose codes and scale bytes share a storage (an allocation is half a
+// microsecond, a seventh of the call). Nothing is cleared: the library writes every value, code and scale byte, padding included.
 struct Quantised {
     at::Tensor q, codes, sf;
     Quantised(const at::Tensor& like, int64_t rows, int64_t cols, bool want_q) {
+        const int64_t nc = (rows * cols * 4 + 7) / 8, ns = (rows + 127) / 128 * 128 * (((cols + 15) / 16 + 3) / 4 * 4);
         if (want_q) q = empty_like_device(like, {rows, cols}, at::kChar);
-        codes = empty_like_device(like, {(rows * cols * 4 + 7) / 8}, at::kByte);
-        sf = empty_like_device(like, {(rows + 127) / 128 * 128 * (((cols + 15) / 16 + 3) / 4 * 4)}, at::kByte);
+        if (!like.is_cuda() || rows < 0 || cols < 0) {
+            codes = empty_like_device(like, {nc}, at::kByte);
+            sf = empty_like_device(like, {ns}, at::kByte);
+            return;
+        }
+        const int64_t at = (nc + 511) / 512 * 512;
+        c10::Storage operand = device_bytes(like.device(), at + ns);
+        codes = part(operand, 0, {nc}, at::kByte);
+        sf = part(std::move(operand), at, {ns}, at::kByte);
     }
     template <typename T>
     T* values() { return static_cast<T*>(q.data_ptr()); }

@@ -76,6 +76,7 @@ def device_error() -> int:
 
 
 # ------------------------------------------------------------------------------------------ quantisers
+# (of a quantiser's outputs, codes and scale bytes -- one operand of a GEMM -- may share a storage: keeping either keeps both)
 def nvfp4_quantize_a(x: torch.Tensor, k_out: int | None = None):
     return _n().quantize_a(x, k_out or x.shape[1])
 

@@ -142,15 +142,16 @@ def test_objects_that_are_no_tensors(H):
             H.rowquant(H.FE_INT8, **{**dict(rows=32, cols_in=128, cols_out=128, in_i8=x, ld_in=128, out_codes=c2, out_sf=s2), **bad})
 
 
-def test_quantiser_outputs_have_their_own_storage(H):
-    """One of them can be kept, saved or grown without the others."""
+def test_quantised_values_have_their_own_storage(H):
+    """They can be kept, saved or grown without the operand, whose codes and scale bytes share one."""
     import io
 
     import torch
     x = torch.randint(-127, 128, (33, 128), dtype=torch.int8, device="cuda")
     q, codes, sf = H.absmean_norm_q_nvfp4(x, 1.0)
     assert q.untyped_storage().nbytes() == q.numel() == 33 * 128 and q.storage_offset() == 0 and q.is_contiguous()
-    assert codes.untyped_storage().nbytes() == codes.numel() and sf.untyped_storage().nbytes() == sf.numel()
+    assert codes.untyped_storage().data_ptr() == sf.untyped_storage().data_ptr() != q.untyped_storage().data_ptr()
+    assert codes.untyped_storage().nbytes() < codes.numel() + sf.numel() + 512 and sf.data_ptr() >= codes.data_ptr() + codes.numel() and sf.data_ptr() % 512 == 0
     want, other = q.clone(), codes.clone()
     buf = io.BytesIO()
     torch.save(q, buf)
@@ -159,6 +160,7 @@ def test_quantiser_outputs_have_their_own_storage(H):
     q[33:].fill_(5)
     assert torch.equal(q[:33], want) and torch.equal(codes, other)
     q.record_stream(torch.cuda.Stream())
+    sf.record_stream(torch.cuda.Stream())
     with torch.inference_mode():
         assert H.nvfp4_quantize_a(x)[0].is_inference()
     assert H.nvfp4_quantize_a(x[:0])[0].numel() == 0
