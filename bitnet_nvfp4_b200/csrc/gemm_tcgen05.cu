@@ -1297,13 +1297,23 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     const bool gelu = p.epilogue == EPI_GELU_FP4 || p.epilogue == EPI_GELU_I8;
     const bool gelu_plain = !gelu || (p.act_scale <= 700.0f && (p.n % 32) == 0 && (p.epilogue == EPI_GELU_FP4 ? (p.next_nvec == 1 && p.d_i8 == nullptr) : p.next_nvec <= 1));
     const int rk = p.rank == 4 && (p.rows_per_member % 16) == 0 ? 4 : ((p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1)) ? 1 : (p.rank > 0 ? 2 : 0));
-    // CTA pairs pay where the mainloop is longer than the epilogue and there is a tile for every pair. Measured at 65536 x 512 (us, single
+    // CTA pairs pay where the mainloop is longer than the epilogue. Measured at 65536 x 512 (us, single
     // CTAs -> pairs): fp32 / half / residual epilogues, rank 1: K 512 33.9 -> 35.9, 25.6 -> 27.0, 29.0 -> 29.8; K 1024 42.7 -> 38.2,
     // 33.1 -> 30.2, 36.1 -> 33.1; K 4096 107 -> 80, 96 -> 70, 98 -> 74. Rank 4 with the last two: K 1024 37.2 -> 39.2, 43.3 -> 45.4, K 1536
     // 46.8 -> 43.3, 49.5 -> 47.4. GELU epilogues, whose math takes as long as K 1536: K 1536 52.7 -> 54.6, K 2048 63.8 -> 59.9, K 4096 105 -> 82.
     const long long pair_tiles = static_cast<long long>((p.n + 255) / 256) * ((p.m + 255) / 256);
     const int pair_k = gelu ? 2048 : (p.rank > 1 && p.epilogue != EPI_F32 ? 1536 : 1024);
-    const bool pair = p.b2 == nullptr && p.k >= pair_k && pair_tiles >= sms / 2 && (rk != 1 || (p.m % 256) == 0);
+    // Those are figures of many waves. In a few, whole waves of the larger tiles and the drain of their two epilogues decide: 10218 x 384 x 2240 took
+    // 15.1 us with single CTAs and 25.0 with pairs, 7668 x 576 x 2880 21.7 and 26.6. So the two are compared by what they cost in waves, in us: K blocks of 256
+    // at 0.44 and 0.6, epilogues of a sub-tile at 1.3 (GELU 1.9; 60 % more with the longer rank terms), 3 for starting a pair. Over 315 shapes of 0.5
+    // to 16 k rows, 64 to 4096 columns and K 1024 to 4096 the choice costs 0.2 % on average against the better of the two (by K and one tile per pair alone 6 %).
+    auto waves_us = [&](long long t, int slots, float block, float epi) {
+        const float nk = block * static_cast<float>((p.k + BK - 1) / BK);
+        return nk + static_cast<float>((t + slots - 1) / slots - 1) * std::max(nk, epi) + epi;
+    };
+    const float epi_us = (gelu ? 1.9f : 1.3f) * (rk >= 2 ? 1.6f : 1.0f);
+    const bool pair = p.b2 == nullptr && p.k >= pair_k && (rk != 1 || (p.m % 256) == 0) &&
+                      3.0f + waves_us(pair_tiles, std::max(1, sms / 2), 0.6f, 2.0f * epi_us) < waves_us(tiles, sms, 0.44f, epi_us);
     // the epilogue and the form of the rank term are template arguments
     auto with_rank = [&](auto run) -> int {
         return rk == 4 ? run(std::integral_constant<int, 4>()) : rk == 1 ? run(std::integral_constant<int, 1>()) : rk == 2 ? run(std::integral_constant<int, 2>()) : run(std::integral_constant<int, 0>());

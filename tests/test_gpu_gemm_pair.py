@@ -1,4 +1,4 @@
-"""CTA-pair instances of the block-scaled GEMM (long K, at least one 256 x 256 tile per pair of SMs) against the single-CTA instances.
+"""CTA-pair instances of the block-scaled GEMM (long K, enough waves of 256 x 256 tiles to pay) against the single-CTA instances.
 
 A call over all rows runs the pair instance; the same rows in slices too small for it run the single-CTA one, which the other GEMM
 tests hold to the oracle. Both accumulate the same MMAs in the same order and share the epilogue code: outputs are compared bit for
@@ -19,12 +19,12 @@ def H():
 
 # rows of a slice: whole pairs of members, multiples of 128 (scale atoms), too few for the pair instance
 @pytest.mark.parametrize("m,n,k,rank,rpm,slice_rows", [
-    (6912, 768, 1024, 1, 128, 1280),      # the model's instance: rank 1, tiles inside one member, m a multiple of 256
-    (6756, 640, 1088, 0, 0, 1280),        # ends in the first CTA's half; the last tile column is half a tile
-    (6860, 736, 1152, 2, 640, 1280),      # ends in the second CTA's half; 736 = 2 x 256 + 224; members straddle tiles
-    (19000, 257, 2112, 4, 320, 1280),     # one column in the second tile column (fp32 / half only)
-    (6912, 768, 2048, 1, 128, 1280),      # GELU's threshold
-    (19200, 256, 2112, 4, 640, 1280),
+    (69120, 768, 1024, 1, 128, 1280),     # the model's instance: rank 1, tiles inside one member, m a multiple of 256
+    (69220, 640, 1088, 0, 0, 1280),       # ends in the first CTA's half; the last tile column is half a tile
+    (68300, 736, 1600, 2, 640, 1280),     # ends in the second CTA's half; 736 = 2 x 256 + 224; members straddle tiles
+    (96200, 513, 2112, 4, 320, 1280),     # one column in the third tile column (fp32 / half only)
+    (37632, 768, 2048, 1, 128, 1280),     # GELU's threshold
+    (96000, 512, 2112, 4, 640, 1280),
 ])
 def test_pair_instance_equals_single_cta_instance(H, m, n, k, rank, rpm, slice_rows):
     import torch
