@@ -467,7 +467,7 @@ def main():
     def step(epoch: int, from_host: bool, spans=None):
         if from_host:
             model.set_tokens(tok_h, tgt_h)            # H2D of the step's inputs (pinned host memory)
-        # evaluate this rank's pairs, all-gather the losses (NCCL), shape (4 KB host round trip, as the reference), update
+        # evaluate this rank's pairs, all-gather the losses (NCCL), shape, update
         losses = population.es_step(model, 1, epoch, pairs_total, rank, world, lr=0.8, thresh=0.008, losses_out=losses_all, spans=spans)
         if from_host:
             losses_host.copy_(losses, non_blocking=True)  # D2H of the step's result

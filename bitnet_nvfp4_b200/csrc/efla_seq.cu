@@ -27,7 +27,7 @@
 //   5. y = P~ V over 64-column tiles of V.
 // What bounds it: the MMAs of steps 2 and 5 (about 40 k tensor cycles per sequence at T = 128, hd = 512; the legacy mma.sync path, since
 // the triangular solve between the contractions needs its operands in registers). 1024 sequences of 128 tokens, one head of 512:
-// 0.57 ms, against 75 ms for the per-token kernel (whose state passes through shared memory twice per token). Of 150 k cycles per unit, step 1
+// 0.56 ms, against 17.6 ms for the per-token kernel. Of 150 k cycles per unit, step 1
 // takes 31 k (DRAM), step 2 63 k, steps 3 and 4 8 k, step 5 47 k. MMAs and the conversions around them add up rather than overlap: staggering them
 // between warps, more independent MMA chains and L2 prefetches of V and of the next unit changed nothing.
 
@@ -927,7 +927,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
 }  // namespace
 
 // The closed form's work per token grows with the sequence, the per-token kernel's does not, but the latter spreads a unit over several SMs. One head of
-// 512: 322 tokens 0.69 / 1.16 ms (closed form / per token) for 4 sequences, 2.4 / 17.5 ms for 400; 1000 tokens 4.4 / 3.6 ms for 4, 5.1 / 8.3 ms for 40.
+// 512: 322 tokens 0.69 / 1.16 ms (closed form / per token) for 4 sequences, 2.4 / 17.5 ms for 400; 1000 tokens 4.4 / 3.6 ms for 4, 5.0 / 8.3 ms for 40.
 // The number of sequences has no say: the two round differently, and a member's loss must not depend on how many share its wave.
 static bool seq_long_pays(const EflaParams& p) {
     if (p.T > kLgMaxT) return false;
@@ -994,8 +994,8 @@ int efla_seq_launch(const EflaParams& p, cudaStream_t stream) {
     }
     const int nd = (p.hidden / p.heads + 63) >> 6;
     // Few units leave SMs idle: two or four CTAs share one as long as all units still run at once and every CTA has a block of columns. One head of
-    // 512, 32 sequences: 71 us with one, 48 with two, 40 with four; a second pass costs more than sharing gains (37 units: 73 us with four,
-    // 48 with two; 256 units: 161 / 204 / 329 us).
+    // 512, 32 sequences: 71 us with one, 55 with two, 41 with four; 37 and 70: 71 with one, 55 with two. (Every CTA stages all of K, so sums keep their order;
+    // with partial sums over shares of the columns two took 48 and four 39 us, and other bits.) A second pass costs more than sharing gains.
     const int cs = units <= four && nd >= 4 ? 4 : units <= two && nd >= 2 ? 2 : 1;
     const bool early = p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems;
     cudaLaunchConfig_t cfg = {};

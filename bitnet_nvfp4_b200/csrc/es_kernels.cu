@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(1024) ce_step_kernel(const float* __restrict__
 // again after it): the member's last block forms the mean; without them split is 1, partial[member * 16 + group] holds the groups'
 // sums and ce_finalize_kernel follows. With split > 1 partial holds the chains' sums, 128 per member.
 constexpr int kCeChunks = 16;
-// SHARED false: the instance for split 1 (with the split as a variable the default model's 1048576 rows took 121 instead of 97 us).
+// SHARED false: the instance for split 1 (with the split as a variable a full wave of the default model, 1048576 rows, took 484 instead of 397 us).
 template <bool SHARED>
 struct CeRows {
     int split, r0, r1, chain, j;  // this warp: rows r0 + chain + 8 (j + split k) below r1
@@ -314,7 +314,7 @@ __global__ void init_shadow_kernel(const int8_t* __restrict__ w, float* __restri
 }
 
 // Z for the dense (full-matrix noise) form; 256 threads per block, one element each.
-// Elements idx0 .. idx0 + n - 1 of the vector (the hash is keyed by the element's index in the whole vector) go to Z[0 .. n).
+// idx: the element's index in the whole vector, which keys the hash.
 // CLT4: the noise every model uses (sum of four ternary draws).
 template <bool CLT4>
 __device__ __forceinline__ void z_dense_block(const float* pair_weights, const uint64_t* pair_seeds, uint64_t salt, int pairs, int idx, bool active,
@@ -357,11 +357,11 @@ __device__ __forceinline__ void z_dense_block(const float* pair_weights, const u
 }
 template <bool CLT4>
 __global__ void __launch_bounds__(256) z_dense_kernel(const float* __restrict__ pair_weights, const uint64_t* __restrict__ pair_seeds,
-                                                      uint64_t salt, int pairs, int idx0, int n, int use_clt, int clt_k, float* __restrict__ Z) {
+                                                      uint64_t salt, int pairs, int n, int use_clt, int clt_k, float* __restrict__ Z) {
     pdl_wait();
     after(pair_weights, pair_seeds);
     const int i = blockIdx.x * 256 + threadIdx.x;
-    z_dense_block<CLT4>(pair_weights, pair_seeds, salt, pairs, idx0 + i, i < n, use_clt, clt_k, Z + i);
+    z_dense_block<CLT4>(pair_weights, pair_seeds, salt, pairs, i, i < n, use_clt, clt_k, Z + i);
 }
 // The same for a table of tensors (the fp32 vectors of a model; in the dense mode also its matrices) in one launch: block b finds
 // its tensor by walking the table. With nshards > 1 a tensor that is computed in shards covers this shard's elements only.
@@ -918,8 +918,8 @@ namespace {
 int z_dense_single(const float* pair_weights, const uint64_t* pair_seeds, uint64_t salt, int pairs, int n, int use_clt, int clt_k, float* Z, cudaStream_t st) {
     const bool early = static_cast<long long>(n) * pairs <= (1ll << 22);
     const dim3 grid((n + 255) / 256);
-    if (use_clt != 0 && clt_k == 4) launch_pdl_if(early, z_dense_kernel<true>, grid, 256, 0, st, pair_weights, pair_seeds, salt, pairs, 0, n, use_clt, clt_k, Z);
-    else launch_pdl_if(early, z_dense_kernel<false>, grid, 256, 0, st, pair_weights, pair_seeds, salt, pairs, 0, n, use_clt, clt_k, Z);
+    if (use_clt != 0 && clt_k == 4) launch_pdl_if(early, z_dense_kernel<true>, grid, 256, 0, st, pair_weights, pair_seeds, salt, pairs, n, use_clt, clt_k, Z);
+    else launch_pdl_if(early, z_dense_kernel<false>, grid, 256, 0, st, pair_weights, pair_seeds, salt, pairs, n, use_clt, clt_k, Z);
     return check_launch("z_dense_kernel");
 }
 }  // namespace

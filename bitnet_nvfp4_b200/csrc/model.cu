@@ -189,11 +189,10 @@ struct Model {
     float* d_step_w;            // ... and the shaped pair weights on the device
     cudaEvent_t tokens_read = nullptr;  // behind the copy of a batch out of pinned host memory
     bool tokens_pending = false;        // bnf4_model_es_step has to wait for it
-    // dense (rank 0) mode: the reference driver's own perturbation, one materialised noise matrix per weight matrix and pair,
-    // applied as a second GEMM with beta = 1 (src/train_efla_lm.cpp:2359-2367). One pair per wave.
-    // dense_folded (sigma down to 2^-4): any number of pairs per wave; the noise operands of every member follow the base weights in the
+    // dense (rank 0) mode: the reference driver's own perturbation, one materialised noise matrix per weight matrix and pair
+    // (src/train_efla_lm.cpp:2359-2367). dense_folded (sigma down to 2^-4): any number of pairs per wave; the noise operands of every member follow the base weights in the
     // same GEMM (GemmParams::b2). sigma cannot scale part of an accumulation, so the base weights' scale bytes carry 2^sigma_shift (w_up,
-    // exact: a power of two, at most 448) and alpha its inverse. Smaller sigmas run one pair per wave with separate products.
+    // exact: a power of two, at most 448) and alpha its inverse. Smaller sigmas run one pair per wave, the noise as a second product with beta = 1.
     bool dense = false, dense_folded = false;
     float w_up = 1.0f;
     struct NoiseOperand { uint8_t *codes, *sf; int rows; };
@@ -203,7 +202,7 @@ struct Model {
     uint2* dgen_tab = nullptr;     // block quantiser table of the noise (scale bytes without w_up)
     int num_dgen = 0, dgen_blocks = 0;
     uint64_t step_seed = 0, step_epoch = 0;
-    int8_t* E_all = nullptr;                 // noise of one pair, all matrices back to back (order of update_matrices)
+    int8_t* E_all = nullptr;                 // folded: the embedding noise of a wave's pairs; else one pair's, all matrices back to back (order of update_matrices)
     uint8_t *qe_win, *sfe_win, *qe_head, *sfe_head;
     std::vector<uint8_t*> qe_qkv, sfe_qkv, qe_ff1, sfe_ff1, qe_ff2, sfe_ff2;
     bnf4_noise_desc* noise_descs = nullptr;  // device table for the batched fill
@@ -774,8 +773,7 @@ int update_z(Model& m, const float* pair_weights, int shard, int nshards, float*
 
 // Applies the precomputed Z of every tensor (sum of squares, RMS-EMA, gated update) and renews the NVFP4 copies of the weights: three
 // launches for all of them.
-int update_apply(Model& m, const float* pair_weights, const float* z_all, const bnf4_update_cfg* u, cudaStream_t st) {
-    (void)pair_weights;
+int update_apply(Model& m, const float* z_all, const bnf4_update_cfg* u, cudaStream_t st) {
     const float thresh = u->thresh * std::sqrt(static_cast<float>(m.pairs_step));
     const bool pos = u->train_pos != 0;  // the positional table is the last tensor
     TimedScope ts(m, KC_UPDATE_APPLY, st, 3);
@@ -1263,7 +1261,7 @@ int bnf4_model_update(void* handle, const float* pair_weights, const bnf4_update
     Model& m = *M(handle);
     if (m.pairs_step <= 0) return set_error(BNF4_ERR_INVALID, "model_update: no prepared step");
     TRY(update_z(m, pair_weights, 0, 1, nullptr, S(stream)));
-    return update_apply(m, pair_weights, m.Z_all, u, S(stream));
+    return update_apply(m, m.Z_all, u, S(stream));
 }
 
 int bnf4_model_update_z_layout(void* handle, int nshards, int max_entries, long long* offsets, long long* elems, int* sharded,
@@ -1308,7 +1306,7 @@ int bnf4_model_update_apply(void* handle, const float* pair_weights, const float
     if (!handle || !pair_weights || !z_all || !u) return set_error(BNF4_ERR_INVALID, "model_update_apply: null argument");
     Model& m = *M(handle);
     if (m.pairs_step <= 0) return set_error(BNF4_ERR_INVALID, "model_update_apply: no prepared step");
-    return update_apply(m, pair_weights, z_all, u, S(stream));
+    return update_apply(m, z_all, u, S(stream));
 }
 
 static int es_step(void* handle, const bnf4_es_step_cfg* cfg, const bnf4_collectives* coll, float* d_losses_all, void* stream) {
@@ -1340,7 +1338,7 @@ static int es_step(void* handle, const bnf4_es_step_cfg* cfg, const bnf4_collect
     }
     if (world == 1) {
         TRY(update_z(m, m.d_step_w, 0, 1, nullptr, st));
-        return update_apply(m, m.d_step_w, m.Z_all, &cfg->update, st);
+        return update_apply(m, m.Z_all, &cfg->update, st);
     }
     // Z by rows over the ranks into the model's own buffer (the layout does not depend on the number of shards), gathered in place
     TRY(update_z(m, m.d_step_w, rank, world, m.Z_all, st));
@@ -1358,7 +1356,7 @@ static int es_step(void* handle, const bnf4_es_step_cfg* cfg, const bnf4_collect
     }
     if (coll->group_end && coll->group_end(coll->ctx) != 0) failed = 1;
     if (failed) return set_error(BNF4_ERR_CUDA, "model_es_step: the all-gather of the noise sums failed");
-    return update_apply(m, m.d_step_w, m.Z_all, &cfg->update, st);
+    return update_apply(m, m.Z_all, &cfg->update, st);
 }
 
 int bnf4_model_es_step(void* handle, const bnf4_es_step_cfg* cfg, const bnf4_collectives* coll, float* d_losses_all, void* stream) {
