@@ -526,9 +526,11 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                         float worst = 0.0f, tb[4], fc[4];
                         gelu_q8_fast2(x[0], x[1], p.act_scale, true, worst, tb[0], tb[1], fc[0], fc[1]);
                         gelu_q8_fast2(x[2], x[3], p.act_scale, true, worst, tb[2], tb[3], fc[2], fc[3]);
-                        if (!(worst < kGeluSafe)) gelu_q8_exact4(x[0], x[1], x[2], x[3], p.act_scale, tb, fc);
+                        // (`worst` does not see a NaN, the sum does; a select per value cost the other modes 2 % as well)
+                        const float any_nan = (x[0] + x[1]) + (x[2] + x[3]);
+                        if (!(worst < kGeluSafe) || any_nan != any_nan) gelu_q8_exact4(x[0], x[1], x[2], x[3], p.act_scale, tb, fc);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) vf[i][4 * q + j] = x[j] != x[j] ? 0.0f : tb[j] - M;  // (`worst` does not see a NaN; its integer is 0)
+                        for (int j = 0; j < 4; ++j) vf[i][4 * q + j] = tb[j] - M;
                     } else {
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
