@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "tcgen05.cuh"
 
 namespace bnf4 {
 
@@ -70,192 +71,9 @@ constexpr int kPairAcc = 3;                 // accumulator blocks of 128 columns
 constexpr int kPairSfCol = kPairAcc * 128;  // two scale slots of 16 (A) + 32 (B) columns behind them
 static_assert(kPairSmemAlloc <= 232448 && kSmemAlloc <= 232448, "shared memory of one SM");
 
-constexpr long long kWaitCycles = 2000000000LL;  // ~1 s bound on every mbarrier wait
-
-__device__ int g_gemm_error = 0;
 }  // namespace
 int g_gemm_allow_tma_store = 1;  // host toggle: 0 forces the direct-store epilogue
 namespace {
-
-// ------------------------------------------------------------------------------------------------
-// PTX wrappers
-// ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// One attempt: the thread may be suspended by the hardware for up to ~20 us and is woken as soon as the phase completes,
-// so a waiting role issues a handful of instructions per attempt instead of spinning through the issue slots the
-// epilogue warps need.
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(20000u)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait. Returns false (and records `code`) if the phase did not complete in time.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int code) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity)) {
-        if (clock64() - t0 > kWaitCycles) {
-            atomicCAS(&g_gemm_error, 0, code);
-            return false;
-        }
-    }
-    return true;
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
-__device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(x), "r"(y)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_cp_sf(uint32_t taddr, uint64_t sdesc) {
-    asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
-}
-__device__ __forceinline__ void tc_mma_nvf4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t tsfa,
-                                            uint32_t tsfb, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-}
-// ---- CTA-pair forms (cta_group::2): issued by the leading CTA (rank 0), they act on both CTAs of the pair
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// the address of the same shared-memory location in the leading CTA
-__device__ __forceinline__ uint32_t map_to_leader(uint32_t addr) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
-// a tile into this CTA's shared memory, counted by the leading CTA's barrier
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t leader_bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(leader_bar)
-        : "memory");
-}
-// (no memory travels with this arrival: it hands back TMEM columns, ordered by tcgen05.fence)
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// arrives at this barrier of both CTAs
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
-}
-__device__ __forceinline__ void tc_cp_sf_pair(uint32_t taddr, uint64_t sdesc) {
-    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
-}
-__device__ __forceinline__ void tc_mma_nvf4_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t tsfa, uint32_t tsfb,
-                                                 uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// prmt.b32 in its default mode: a selector nibble with bit 3 set replicates the sign of the selected byte
-__device__ __forceinline__ uint32_t prmt_b32(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t d;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
-// Four bytes of the int8 residual stream updated with four accumulators: clip8(old + rint(v * add_scale)). rint is the low 16
-// bits of the biased float (the product is clamped first so that the field cannot wrap), added to the sign-extended old
-// bytes and clipped with packed 16-bit integer operations, two elements per instruction.
-__device__ __forceinline__ uint32_t resid_add_word(uint32_t old4, float v0, float v1, float v2, float v3, float add_scale) {
-    const uint32_t t0 = __float_as_uint(fminf(fmaxf(__fmul_rn(v0, add_scale), -512.0f), 512.0f) + kRoundBias);
-    const uint32_t t1 = __float_as_uint(fminf(fmaxf(__fmul_rn(v1, add_scale), -512.0f), 512.0f) + kRoundBias);
-    const uint32_t t2 = __float_as_uint(fminf(fmaxf(__fmul_rn(v2, add_scale), -512.0f), 512.0f) + kRoundBias);
-    const uint32_t t3 = __float_as_uint(fminf(fmaxf(__fmul_rn(v3, add_scale), -512.0f), 512.0f) + kRoundBias);
-    const uint32_t r01 = __byte_perm(t0, t1, 0x5410), r23 = __byte_perm(t2, t3, 0x5410);
-    const uint32_t o01 = prmt_b32(old4, 0u, 0x9180u), o23 = prmt_b32(old4, 0u, 0xB3A2u);
-    const uint32_t s01 = __vmins2(__viaddmax_s16x2(r01, o01, 0xff81ff81u), 0x007f007fu);
-    const uint32_t s23 = __vmins2(__viaddmax_s16x2(r23, o23, 0xff81ff81u), 0x007f007fu);
-    return __byte_perm(s01, s23, 0x6420);
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Shared-memory matrix descriptor (sm_100 format): start address >> 4 in bits [0,14), leading byte
-// offset >> 4 in [16,30), stride byte offset >> 4 in [32,46), version 1 in [46,48), layout type in [61,64).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr & 0x3ffffu) >> 4);
-    d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3fffu) << 16;
-    d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3fffu) << 32;
-    d |= 1ull << 46;
-    d |= static_cast<uint64_t>(layout) << 61;
-    return d;
-}
-constexpr uint32_t kLayoutNone = 0, kLayoutSw128 = 2;
 
 // Instruction descriptor of kind::mxf4nvf4 (block-scaled): a/b format e2m1 (=1) at bits 7 and 10,
 // K-major A and B, N>>3 at bit 17, ue4m3 scales (bit 23 = 0), M>>4 at bit 24, scale ids 0, dense K = 64.
@@ -286,18 +104,6 @@ struct KernelArgs {
     int ks_wrap;  // K blocks after which A starts again and B2 follows B (0: no second operand)
     int n_tiles;  // tiles along N (of 256 columns in the pair instances); blockIdx.x = m_tile * n_tiles + n_tile (N fastest: CTAs that share A rows run together)
 };
-
-// One lane of a converged warp (the same one every time in practice). The role loops below run in all 32 lanes with
-// warp-uniform control flow and values, and only the issuing instructions sit under this predicate: addresses, descriptors and
-// counters then qualify for the uniform datapath instead of being moved there instruction by instruction from a divergent lane.
-__device__ __forceinline__ bool elect_one() {
-    uint32_t pred;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
-    return pred != 0;
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 
 // Persistent kernel: one CTA per SM walks the tile list (tile = m_tile * n_tiles + n_tile, N fastest so that
 // CTAs working at the same time share rows of A through L2). Three roles run concurrently on different tiles:
@@ -1155,8 +961,9 @@ struct MapSlot {
 };
 constexpr unsigned kMapSlots = 256;
 
+}  // namespace
 int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t dim0, uint64_t dim1, uint64_t stride1_bytes,
-                uint32_t box0, uint32_t box1, const char* what, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
+                uint32_t box0, uint32_t box1, const char* what, CUtensorMapSwizzle swizzle) {
     static thread_local std::vector<MapSlot> cache;
     if (cache.empty()) cache.resize(kMapSlots, MapSlot{});
     const MapKey key{base, dim0, dim1, stride1_bytes, box0, box1, static_cast<int>(dt), static_cast<int>(swizzle)};
@@ -1179,6 +986,8 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint
     slot.map = *map;
     return BNF4_OK;
 }
+
+namespace {
 
 template <int EPI, int RK, bool PAIR, bool B2>
 int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, const ExtraMaps<PAIR, B2>& msf, const KernelArgs& args,
@@ -1339,6 +1148,7 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
             return with_rank(run);
         });
     }
+    if (gemm_panel_applies(p, rk, sms)) return gemm_panel_launch(p, rk, ma, mb, md, args.group_magic, sms, dev, stream);
     const dim3 grid(static_cast<unsigned>(std::min<long long>(tiles, sms)), 1, 1);
     if (p.b2 != nullptr) {
         if (p.sfb2 == nullptr || (p.b2_rows % 128) != 0 || p.b2_rows < p.n || p.rows_per_member <= 0 || (p.rows_per_member % BM) != 0 || p.rank > 0)
@@ -1365,14 +1175,14 @@ int gemm_nvfp4_device_error(cudaStream_t stream, int* out_code) {
     int rc = check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     if (rc) return rc;
     int code = 0;
-    rc = check_cuda(cudaMemcpyFromSymbol(&code, g_gemm_error, sizeof(int)), "cudaMemcpyFromSymbol(g_gemm_error)");
-    if (rc) return rc;
-    if (code != 0) {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_gemm_error, &zero, sizeof(int));
+    for (auto take : {take_wait_error, gemm_panel_device_error}) {
+        int one = 0;
+        rc = take(&one);
+        if (rc) return rc;
+        if (code == 0) code = one;
     }
     if (out_code) *out_code = code;
-    if (code != 0) return set_error(BNF4_ERR_DEVICE, "gemm_nvfp4: a bounded wait expired in the kernel (role code %d)", code);
+    if (code != 0) return set_error(BNF4_ERR_DEVICE, "a bounded wait expired in a kernel (role code %d)", code);
     return BNF4_OK;
 }
 
