@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "mma_sync.cuh"
 
 namespace bnf4 {
 
@@ -458,24 +459,9 @@ constexpr int kScanWarps = 4;
 // Shared-memory order of a 64-vector ("permuted"): element d sits at ((d % 8) / 2) * 16 + (d / 16) * 4 + (d % 2) + 2 * ((d / 8) % 2),
 // so that the 16 values a lane needs (d = 16 ks + 2 tq + {0, 1, 8, 9}, ks = 0..3) are contiguous at tq * 16.
 
-__device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// d = a (16 x 16) * b (16 x 8): no accumulator input
-__device__ __forceinline__ void mma_f16_16816_zero(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
-}
 // c (16 x 8, fp16, in place) += a (16 x 8) * b (8 x 8): fp16 accumulators, one rounding to nearest of the exact sum
 __device__ __forceinline__ void mma_f16acc_1688(uint32_t& c0, uint32_t& c1, uint32_t a0, uint32_t a1, uint32_t b0) {
     asm("mma.sync.aligned.m16n8k8.row.col.f16.f16.f16.f16 {%0, %1}, {%2, %3}, {%4}, {%0, %1};" : "+r"(c0), "+r"(c1) : "r"(a0), "r"(a1), "r"(b0));
-}
-__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
-    const __half2 hv = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&hv);
 }
 
 constexpr int kScanRing = 12;                // ring of raw v per warp: three groups of four tokens
@@ -741,16 +727,6 @@ __device__ __forceinline__ void mma_f16acc_16816(uint32_t& c0, uint32_t& c1, uin
     asm("mma.sync.aligned.m16n8k16.row.col.f16.f16.f16.f16 {%0, %1}, {%2, %3, %4, %5}, {%6, %7}, {%0, %1};"
         : "+r"(c0), "+r"(c1)
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t saddr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr) : "memory");
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t saddr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr) : "memory");
-}
-
-__device__ __forceinline__ void stmatrix_x4_trans(uint32_t saddr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
 }
 
 template <bool IN16, bool OUT16>
@@ -1495,6 +1471,7 @@ int efla_launch(const EflaParams& p, cudaStream_t stream) {
             if (p.qkv_f16 && p.method == 1) {  // the batched driver's case: raw-operand kernel, persistent pairs of warps
                 const int sms = multiprocessors(dev);
                 if (sms <= 0) return BNF4_ERR_CUDA;
+                if (efla_tc_applies(p)) return efla_tc_launch(p, early, dev, sms, stream);
                 const unsigned pgrid = static_cast<unsigned>(std::min<long long>((units + kM1Units - 1) / kM1Units, kM1CtasPerSm * static_cast<long long>(sms)));
                 if (p.out_f16) launch_pdl_if(early, efla_chunk16_m1_kernel<true>, pgrid, kChunkWarps * 32, kM1SmemBytes, stream, p);
                 else launch_pdl_if(early, efla_chunk16_m1_kernel<false>, pgrid, kChunkWarps * 32, kM1SmemBytes, stream, p);

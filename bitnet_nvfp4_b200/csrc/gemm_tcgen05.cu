@@ -948,11 +948,11 @@ EncodeTiledFn get_encode_fn() {
 // pure function of its key.
 struct MapKey {
     const void* base;
-    uint64_t dim0, dim1, stride1;
-    uint32_t box0, box1;
+    uint64_t dim0, dim1, stride1, dim2, stride2;  // dim2 = 0: two dimensions
+    uint32_t box0, box1, box2;
     int dt, swizzle;
     bool operator==(const MapKey& o) const {
-        return base == o.base && dim0 == o.dim0 && dim1 == o.dim1 && stride1 == o.stride1 && box0 == o.box0 && box1 == o.box1 && dt == o.dt && swizzle == o.swizzle;
+        return base == o.base && dim0 == o.dim0 && dim1 == o.dim1 && stride1 == o.stride1 && dim2 == o.dim2 && stride2 == o.stride2 && box0 == o.box0 && box1 == o.box1 && box2 == o.box2 && dt == o.dt && swizzle == o.swizzle;
     }
 };
 struct MapSlot {
@@ -962,11 +962,11 @@ struct MapSlot {
 constexpr unsigned kMapSlots = 256;
 
 }  // namespace
-int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t dim0, uint64_t dim1, uint64_t stride1_bytes,
-                uint32_t box0, uint32_t box1, const char* what, CUtensorMapSwizzle swizzle) {
+int make_map_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t dim0, uint64_t dim1, uint64_t dim2, uint64_t stride1_bytes, uint64_t stride2_bytes,
+                uint32_t box0, uint32_t box1, uint32_t box2, const char* what, CUtensorMapSwizzle swizzle) {
     static thread_local std::vector<MapSlot> cache;
     if (cache.empty()) cache.resize(kMapSlots, MapSlot{});
-    const MapKey key{base, dim0, dim1, stride1_bytes, box0, box1, static_cast<int>(dt), static_cast<int>(swizzle)};
+    const MapKey key{base, dim0, dim1, stride1_bytes, dim2, stride2_bytes, box0, box1, box2, static_cast<int>(dt), static_cast<int>(swizzle)};
     const uint64_t hash = mix_u64(reinterpret_cast<uint64_t>(base), mix_u64(dim0 ^ (static_cast<uint64_t>(box1) << 48), dim1 ^ (stride1_bytes << 24)));
     MapSlot& slot = cache[hash % kMapSlots];
     if (base != nullptr && slot.key == key) {
@@ -975,18 +975,21 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint
     }
     EncodeTiledFn fn = get_encode_fn();
     if (fn == nullptr) return set_error(BNF4_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    const cuuint64_t dims[2] = {dim0, dim1};
-    const cuuint64_t strides[1] = {stride1_bytes};
-    const cuuint32_t box[2] = {box0, box1};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = fn(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint64_t dims[3] = {dim0, dim1, dim2};
+    const cuuint64_t strides[2] = {stride1_bytes, stride2_bytes};
+    const cuuint32_t box[3] = {box0, box1, box2};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    const CUresult r = fn(map, dt, dim2 == 0 ? 2 : 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(BNF4_ERR_CUDA, "cuTensorMapEncodeTiled(%s) failed with %d", what, static_cast<int>(r));
     slot.key = key;
     slot.map = *map;
     return BNF4_OK;
 }
-
+int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t dim0, uint64_t dim1, uint64_t stride1_bytes,
+                uint32_t box0, uint32_t box1, const char* what, CUtensorMapSwizzle swizzle) {
+    return make_map_3d(map, dt, base, dim0, dim1, 0, stride1_bytes, 0, box0, box1, 1, what, swizzle);
+}
 namespace {
 
 template <int EPI, int RK, bool PAIR, bool B2>
@@ -1175,7 +1178,7 @@ int gemm_nvfp4_device_error(cudaStream_t stream, int* out_code) {
     int rc = check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     if (rc) return rc;
     int code = 0;
-    for (auto take : {take_wait_error, gemm_panel_device_error}) {
+    for (auto take : {take_wait_error, gemm_panel_device_error, efla_tc_device_error}) {
         int one = 0;
         rc = take(&one);
         if (rc) return rc;

@@ -88,6 +88,9 @@ extern int g_efla_chunked;
 // Whole sequences from a zero state, any head_dim (efla_seq.cu).
 bool efla_seq_applies(const EflaParams& p);
 int efla_seq_launch(const EflaParams& p, cudaStream_t stream);
+// Whole sequences of up to 128 tokens with half inputs and output, heads of 64 (efla_tc.cu).
+bool efla_tc_applies(const EflaParams& p);
+int efla_tc_launch(const EflaParams& p, bool early, int dev, int sms, cudaStream_t stream);
 
 // Rank-r noise sums Z of a table of matrices in one launch (es_kernels.cu).
 struct ZLowrankDesc {

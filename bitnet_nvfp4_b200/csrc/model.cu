@@ -399,6 +399,9 @@ int run_wave(Model& m, int p0, int nm, float sigma, float* losses_out, cudaStrea
             if (half_io) {
                 e.q = qkv16; e.k = qkv16 + H; e.v = qkv16 + 2 * H; e.beta_raw = beta16; e.ld_qkv = 3 * H; e.ld_beta = 1;
                 e.qkv_f16 = 1; e.out_f16 = 1; e.out = m.y; e.ld_out = H;
+                // Members keep the chunked form and its roundings, whatever their wave: pairs are ranked by differences that a rounding of y can turn
+                // where it decides an int8 of the residual stream. The unperturbed model is compared with none of them and takes the quicker one.
+                if (sigma != 0.0f) e.variant = BNF4_EFLA_CHUNKED;
             } else {
                 e.q = m.qkv; e.k = m.qkv + H; e.v = m.qkv + 2 * H; e.beta_raw = m.qkv + 3 * H; e.ld_qkv = FC; e.ld_beta = FC;
                 e.out = m.y; e.ld_out = H;

@@ -214,7 +214,9 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// A two-dimensional tensor map (dim0 contiguous), from the calling thread's table of its last ones (gemm_tcgen05.cu).
+// A two- or three-dimensional tensor map (dim0 contiguous), from the calling thread's table of its last ones (gemm_tcgen05.cu).
+int make_map_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t dim0, uint64_t dim1, uint64_t dim2, uint64_t stride1_bytes, uint64_t stride2_bytes,
+                uint32_t box0, uint32_t box1, uint32_t box2, const char* what, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint64_t dim0, uint64_t dim1, uint64_t stride1_bytes,
                 uint32_t box0, uint32_t box1, const char* what, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B);
 
@@ -223,6 +225,8 @@ int make_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, uint
 bool gemm_panel_applies(const GemmParams& p, int rk, int sms);
 int gemm_panel_launch(const GemmParams& p, int rk, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, uint32_t group_magic, int sms, int dev,
                       cudaStream_t stream);
-int gemm_panel_device_error(int* code);  // its take_wait_error
+// take_wait_error of the other translation units with such waits
+int gemm_panel_device_error(int* code);
+int efla_tc_device_error(int* code);
 
 }  // namespace bnf4

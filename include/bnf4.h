@@ -265,7 +265,8 @@ typedef struct bnf4_efla_desc {
     void* out; /* fp32 (or halves, see out_f16): row r at out + r*ld_out */
     int ld_out;
     int variant; /* BNF4_EFLA_*: which kernel runs. AUTO: for heads of 64 with no HBM state, the chunked or the per-token
-                    register-state kernel as option "efla_chunked" says; for head widths above 32 other than 64 with no HBM state, an fp16 state, up to
+                    register-state kernel as option "efla_chunked" says (chunked, half inputs and output, method 1 and 33 to 128
+                    tokens: the closed form of the whole sequence instead); for head widths above 32 other than 64 with no HBM state, an fp16 state, up to
                     1024 tokens (beyond 128 only if out lies apart from q, k and v) and "efla_chunked" on,
                     the closed form of the whole sequence (nothing rounded to fp16 between tokens); the generic kernel otherwise. */
     int qkv_f16; /* 1: q, k, v are IEEE halves and ld_qkv counts halves (chunked kernel only; 16-byte aligned rows) */
