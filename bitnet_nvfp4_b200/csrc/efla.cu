@@ -704,6 +704,7 @@ constexpr int kCkQKStride = 72;  // floats per row of the raw q / k tiles: 16-by
 constexpr int kCkVStride = 68;   // floats per row of the raw v tile: the accumulator-shaped reads are conflict-free
 constexpr int kCkHStride = 72;   // halves per row of the prepared operands (-K, Q^, a K): conflict-free ldmatrix rows
 constexpr int kCkTStride = 24;   // halves per row of T and P
+constexpr int kCkLStride = 20;   // floats per column of L: the accumulator-shaped stores are conflict-free
 // the same tiles when q, k, v arrive as halves: strides in halves (160-byte q / k rows, 144-byte v rows)
 constexpr int kCkQKStrideH = 80;
 constexpr int kCkVStrideH = 72;
@@ -714,7 +715,7 @@ constexpr int kCkRawV = kCkRawK + kChunk * kCkQKStride * 4;
 constexpr int kCkBeta = kCkRawV + kChunk * kCkVStride * 4;
 constexpr int kCkAlpha = kCkBeta + kChunk * 4;
 constexpr int kCkL = kCkAlpha + kChunk * 4;
-constexpr int kCkNK = kCkL + kChunk * kChunk * 4;
+constexpr int kCkNK = kCkL + kChunk * kCkLStride * 4;
 constexpr int kCkQh = kCkNK + kChunk * kCkHStride * 2;
 constexpr int kCkAK = kCkQh + kChunk * kCkHStride * 2;
 constexpr int kCkT = kCkAK + kChunk * kCkHStride * 2;
@@ -727,6 +728,24 @@ __device__ __forceinline__ void mma_f16acc_16816(uint32_t& c0, uint32_t& c1, uin
     asm("mma.sync.aligned.m16n8k16.row.col.f16.f16.f16.f16 {%0, %1}, {%2, %3, %4, %5}, {%6, %7}, {%0, %1};"
         : "+r"(c0), "+r"(c1)
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Column c of (I + L)^-1, L strictly lower and stored by columns. A finished element goes into all later ones at once: each of these still takes its terms in
+// ascending order, with the roundings of a sum per row, but the chain is fifteen multiply-adds long instead of a hundred and twenty. (With the raw-operand
+// kernel's products that wait for nothing moved in front of its scalar chain and behind its outputs: 32 sequences of 8 heads x 128 tokens 13.8 -> 12.8 us, the same bits.)
+__device__ __forceinline__ void chunk_substitute(const float* L, int c, float (&col)[kChunk]) {
+#pragma unroll
+    for (int t = 0; t < kChunk; ++t) col[t] = t == c ? 1.0f : 0.0f;
+#pragma unroll
+    for (int s = 0; s + 1 < kChunk; ++s)
+#pragma unroll
+        for (int t4 = (s + 1) / 4 * 4; t4 < kChunk; t4 += 4) {
+            const float4 lv = *reinterpret_cast<const float4*>(L + s * kCkLStride + t4);
+            if (t4 > s) col[t4] = fmaf(-lv.x, col[s], col[t4]);
+            if (t4 + 1 > s) col[t4 + 1] = fmaf(-lv.y, col[s], col[t4 + 1]);
+            if (t4 + 2 > s) col[t4 + 2] = fmaf(-lv.z, col[s], col[t4 + 2]);
+            if (t4 + 3 > s) col[t4 + 3] = fmaf(-lv.w, col[s], col[t4 + 3]);
+        }
 }
 
 template <bool IN16, bool OUT16>
@@ -963,7 +982,8 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const
                 const int t = g + 8 * hr;
                 const float l0 = s0 < t ? al.x * Gc[nt][2 * hr] : 0.0f, l1 = s0 + 1 < t ? al.y * Gc[nt][2 * hr + 1] : 0.0f;
                 const float p0 = s0 <= t ? -al.x * Xc[nt][2 * hr] : 0.0f, p1 = s0 + 1 <= t ? -al.y * Xc[nt][2 * hr + 1] : 0.0f;
-                *reinterpret_cast<float2*>(L_sh + t * kChunk + s0) = make_float2(l0, l1);
+                L_sh[s0 * kCkLStride + t] = l0;
+                L_sh[(s0 + 1) * kCkLStride + t] = l1;
                 *reinterpret_cast<uint32_t*>(p_sh + t * kCkTStride + s0) = pack_half2(p0, p1);
             }
         }
@@ -972,19 +992,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, 2) efla_chunk16_kernel(const
         {
             const int c = lane & 15;
             float col[kChunk];
-#pragma unroll
-            for (int t = 0; t < kChunk; ++t) {
-                float acc = t == c ? 1.0f : 0.0f;
-#pragma unroll
-                for (int s4 = 0; s4 < t; s4 += 4) {
-                    const float4 lv = *reinterpret_cast<const float4*>(L_sh + t * kChunk + s4);
-                    acc = fmaf(-lv.x, col[s4], acc);
-                    if (s4 + 1 < t) acc = fmaf(-lv.y, col[s4 + 1], acc);
-                    if (s4 + 2 < t) acc = fmaf(-lv.z, col[s4 + 2], acc);
-                    if (s4 + 3 < t) acc = fmaf(-lv.w, col[s4 + 3], acc);
-                }
-                col[t] = acc;
-            }
+            chunk_substitute(L_sh, c, col);
             if (lane < kChunk) {
 #pragma unroll
                 for (int t = 0; t < kChunk; ++t) t_sh[t * kCkTStride + c] = __float2half_rn(col[t]);
@@ -1089,7 +1097,7 @@ constexpr int kM1Beta = kM1Y + 2 * kChunk * kM1YStride * 2;     // two buffers
 constexpr int kM1Alpha = kM1Beta + 2 * kChunk * 4;
 constexpr int kM1Qinv = kM1Alpha + kChunk * 4;
 constexpr int kM1L = kM1Qinv + kChunk * 4;
-constexpr int kM1T = kM1L + kChunk * kChunk * 4;
+constexpr int kM1T = kM1L + kChunk * kCkLStride * 4;
 constexpr int kM1P = kM1T + kChunk * kCkTStride * 2;
 constexpr int kM1UnitBytes = kM1P + kChunk * kCkTStride * 2;
 constexpr int kM1Units = kChunkWarps / 2;                       // units per CTA
@@ -1203,8 +1211,10 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
     for (int t0 = 0; t0 < p.T; t0 += kChunk, kbuf ^= 1) {
         cp_async_wait<0>();
         pair_sync();  // both halves of the tiles have landed; both warps are done with the other buffers, T and P
-        if (t0 + kChunk < p.T) issue_chunk(ua, t0 + kChunk, kbuf ^ 1);
-        else if (unit + unit_stride < total_units) issue_chunk(unit_at(unit + unit_stride), 0, kbuf ^ 1);
+        auto fetch_next = [&]() {
+            if (t0 + kChunk < p.T) issue_chunk(ua, t0 + kChunk, kbuf ^ 1);
+            else if (unit + unit_stride < total_units) issue_chunk(unit_at(unit + unit_stride), 0, kbuf ^ 1);
+        };
         const uint32_t bufo = kbuf * kKBufBytes;
         // ---------------- operand fragments straight from the raw tiles; W^T starts as -V^T ----------------
         uint32_t kf[4][4];  // per 16-wide d block: B fragments {b0, b1} for tokens 0-7 (regs 0, 1) and 8-15 (regs 2, 3)
@@ -1222,13 +1232,15 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
                 Wc[mt][nt][2] = -hi.x; Wc[mt][nt][3] = -hi.y;
             }
         }
+        auto state_products = [&]() {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
+            for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
-            for (int mt = 0; mt < 2; ++mt)
+                for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-                for (int nt = 0; nt < 2; ++nt)
-                    mma_f16_16816(Wc[mt][nt], Sh[mt][ks][0], Sh[mt][ks][1], Sh[mt][ks][2], Sh[mt][ks][3], kf[ks][2 * nt], kf[ks][2 * nt + 1]);
+                    for (int nt = 0; nt < 2; ++nt)
+                        mma_f16_16816(Wc[mt][nt], Sh[mt][ks][0], Sh[mt][ks][1], Sh[mt][ks][2], Sh[mt][ks][3], kf[ks][2 * nt], kf[ks][2 * nt + 1]);
+        };
         // The squared norms of k and q are the diagonals of K K^T and Q Q^T, which the tensor cores produce. They land in the eight
         // lanes with tq == g / 2 (tokens g and g + 8); each hands token g + 8 to its neighbour lane ^ 1, so sixteen lanes run the
         // scalar chain for one token each.
@@ -1253,26 +1265,30 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
                 for (int nt = 0; nt < 2; ++nt) mma_f16_16816(Gc[nt], kf[ks][0], kf[ks][2], kf[ks][1], kf[ks][3], kf[ks][2 * nt], kf[ks][2 * nt + 1]);
             // ---------------- alpha from the diagonal (exact fp16 products accumulated in fp32) ----------------
             {
+                // sigmoid and the final quotient with the fast exponential / division (about 2 ulp each: far below the fp16
+                // rounding of every operand alpha touches); expm1f keeps its accuracy for small beta * lambda
+                const bool valid = t0 + my_tok < p.T;
+                const float braw = valid ? beta_sh[kbuf * kChunk + my_tok] : 0.0f;
+                const float beta = __fdividef(1.0f, 1.0f + __expf(-(braw + beta_bias)));
+                state_products();
+                fetch_next();
                 const float kss = diagonal(Gc);
                 if (diag_lane || helper_lane) {
-                    const bool valid = t0 + my_tok < p.T;
-                    const float braw = valid ? beta_sh[kbuf * kChunk + my_tok] : 0.0f;
                     const float lambda = kss < p.eps ? p.eps : kss;
-                    // sigmoid and the final quotient with the fast exponential / division (about 2 ulp each: far below the fp16
-                    // rounding of every operand alpha touches); expm1f keeps its accuracy for small beta * lambda
-                    const float beta = __fdividef(1.0f, 1.0f + __expf(-(braw + beta_bias)));
                     alpha_sh[my_tok] = valid ? __fdividef(-expm1f(-(beta * lambda)), lambda + p.eps) : 0.0f;
                 }
             }
             __syncwarp();
-            // L[t][s] = a_t G[t][s] in fp32; the substitution reads it below the diagonal only: no mask needed
+            // L[t][s] = a_t G[t][s] in fp32, by columns; the substitution reads it below the diagonal only: no mask needed
             {
                 const float a_lo = alpha_sh[g], a_hi = alpha_sh[g + 8];
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt) {
-                    const int s0 = 8 * nt + 2 * tq;
-                    *reinterpret_cast<float2*>(L_sh + g * kChunk + s0) = make_float2(a_lo * Gc[nt][0], a_lo * Gc[nt][1]);
-                    *reinterpret_cast<float2*>(L_sh + (g + 8) * kChunk + s0) = make_float2(a_hi * Gc[nt][2], a_hi * Gc[nt][3]);
+                    float* lc = L_sh + (8 * nt + 2 * tq) * kCkLStride + g;
+                    lc[0] = a_lo * Gc[nt][0];
+                    lc[kCkLStride] = a_lo * Gc[nt][1];
+                    lc[8] = a_hi * Gc[nt][2];
+                    lc[kCkLStride + 8] = a_hi * Gc[nt][3];
                 }
             }
             __syncwarp();
@@ -1280,19 +1296,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
             {
                 const int c = lane & 15;
                 float col[kChunk];
-#pragma unroll
-                for (int t = 0; t < kChunk; ++t) {
-                    float acc = t == c ? 1.0f : 0.0f;
-#pragma unroll
-                    for (int s4 = 0; s4 < t; s4 += 4) {
-                        const float4 lv = *reinterpret_cast<const float4*>(L_sh + t * kChunk + s4);
-                        acc = fmaf(-lv.x, col[s4], acc);
-                        if (s4 + 1 < t) acc = fmaf(-lv.y, col[s4 + 1], acc);
-                        if (s4 + 2 < t) acc = fmaf(-lv.z, col[s4 + 2], acc);
-                        if (s4 + 3 < t) acc = fmaf(-lv.w, col[s4 + 3], acc);
-                    }
-                    col[t] = acc;
-                }
+                chunk_substitute(L_sh, c, col);
                 if (lane < kChunk) {  // the column as one row of T^T: sixteen halves, two 16-byte stores
                     uint32_t w[8];
 #pragma unroll
@@ -1303,6 +1307,8 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
                 }
             }
         } else {
+            state_products();
+            fetch_next();
             uint32_t qf[4][4];
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) ldmatrix_x4(qf[ks], q_addr0 + bufo + ks * 32);
@@ -1363,25 +1369,41 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
             Up[mt][2] = pack_half2(Uc[1][0], Uc[1][1]); Up[mt][3] = pack_half2(Uc[1][2], Uc[1][3]);
         }
         // ---------------- Y^T = (S0^T Q^T + U~^T P^T) diag(q_inv) ----------------
+        float Yc[2][2][4];
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            float Yc[2][4];
+        for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt) mma_f16_16816_zero(Yc[nt], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], pf[2 * nt], pf[2 * nt + 1]);
+            for (int nt = 0; nt < 2; ++nt) mma_f16_16816_zero(Yc[mt][nt], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], pf[2 * nt], pf[2 * nt + 1]);
 #pragma unroll
-            for (int ks = 0; ks < 4; ++ks)
+        for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt)
-                    mma_f16_16816(Yc[nt], Sh[mt][ks][0], Sh[mt][ks][1], Sh[mt][ks][2], Sh[mt][ks][3], qf[ks][2 * nt], qf[ks][2 * nt + 1]);
+                    mma_f16_16816(Yc[mt][nt], Sh[mt][ks][0], Sh[mt][ks][1], Sh[mt][ks][2], Sh[mt][ks][3], qf[ks][2 * nt], qf[ks][2 * nt + 1]);
+        // ---------------- S^T += U~^T K: fp16 accumulators = the state registers, rounded once per chunk ----------------
+#pragma unroll
+        for (int dp = 0; dp < 4; ++dp) {
+            uint32_t af[4];
+            ldmatrix_x4_trans(af, kt_addr0 + bufo + dp * 32);
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+                mma_f16acc_16816(Sh[mt][dp][0], Sh[mt][dp][1], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], af[0], af[1]);
+                mma_f16acc_16816(Sh[mt][dp][2], Sh[mt][dp][3], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], af[2], af[3]);
+            }
+        }
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
+                float (&Y)[4] = Yc[mt][nt];
                 const float2 q2 = make_float2(qi[nt][0], qi[nt][1]);
-                const float2 lo = __fmul2_rn(q2, make_float2(Yc[nt][0], Yc[nt][1])), hi = __fmul2_rn(q2, make_float2(Yc[nt][2], Yc[nt][3]));
-                Yc[nt][0] = lo.x; Yc[nt][1] = lo.y; Yc[nt][2] = hi.x; Yc[nt][3] = hi.y;
+                const float2 lo = __fmul2_rn(q2, make_float2(Y[0], Y[1])), hi = __fmul2_rn(q2, make_float2(Y[2], Y[3]));
+                Y[0] = lo.x; Y[1] = lo.y; Y[2] = hi.x; Y[3] = hi.y;
             }
+            const float (&Y)[2][4] = Yc[mt];
             if constexpr (OUT16) {
-                stmatrix_x4_trans(y_addr + mt * 32, pack_half2(Yc[0][0], Yc[0][1]), pack_half2(Yc[0][2], Yc[0][3]), pack_half2(Yc[1][0], Yc[1][1]),
-                                  pack_half2(Yc[1][2], Yc[1][3]));
+                stmatrix_x4_trans(y_addr + mt * 32, pack_half2(Y[0][0], Y[0][1]), pack_half2(Y[0][2], Y[0][3]), pack_half2(Y[1][0], Y[1][1]), pack_half2(Y[1][2], Y[1][3]));
             } else {
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt)
@@ -1390,8 +1412,8 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
                         const int tl = 8 * nt + 2 * tq + e;
                         if (t0 + tl < p.T) {
                             float* orow = ob + static_cast<size_t>(t0 + tl) * p.ld_out + 16 * mt + g;
-                            orow[0] = Yc[nt][e];
-                            orow[8] = Yc[nt][2 + e];
+                            orow[0] = Y[nt][e];
+                            orow[8] = Y[nt][2 + e];
                         }
                     }
             }
@@ -1404,17 +1426,6 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kM1CtasPerSm) efla_chunk16_m
                 if (t0 + tl < p.T)
                     *reinterpret_cast<uint4*>(obh + static_cast<size_t>(t0 + tl) * p.ld_out + 8 * piece) =
                         *reinterpret_cast<const uint4*>(y_sh + tl * kM1YStride + 8 * piece);
-            }
-        }
-        // ---------------- S^T += U~^T K: fp16 accumulators = the state registers, rounded once per chunk ----------------
-#pragma unroll
-        for (int dp = 0; dp < 4; ++dp) {
-            uint32_t af[4];
-            ldmatrix_x4_trans(af, kt_addr0 + bufo + dp * 32);
-#pragma unroll
-            for (int mt = 0; mt < 2; ++mt) {
-                mma_f16acc_16816(Sh[mt][dp][0], Sh[mt][dp][1], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], af[0], af[1]);
-                mma_f16acc_16816(Sh[mt][dp][2], Sh[mt][dp][3], Up[mt][0], Up[mt][1], Up[mt][2], Up[mt][3], af[2], af[3]);
             }
         }
         __syncwarp();  // the staging tile is free
