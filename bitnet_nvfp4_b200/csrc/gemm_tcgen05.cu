@@ -1178,7 +1178,7 @@ int gemm_nvfp4_device_error(cudaStream_t stream, int* out_code) {
     int rc = check_cuda(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     if (rc) return rc;
     int code = 0;
-    for (auto take : {take_wait_error, gemm_panel_device_error, efla_tc_device_error}) {
+    for (auto take : {take_wait_error, gemm_panel_device_error, efla_tc_device_error, efla_seq_device_error}) {
         int one = 0;
         rc = take(&one);
         if (rc) return rc;

@@ -228,5 +228,6 @@ int gemm_panel_launch(const GemmParams& p, int rk, const CUtensorMap& ma, const 
 // take_wait_error of the other translation units with such waits
 int gemm_panel_device_error(int* code);
 int efla_tc_device_error(int* code);
+int efla_seq_device_error(int* code);
 
 }  // namespace bnf4
