@@ -118,8 +118,9 @@ struct KernelArgs {
 // 64 (measured, one CTA): 8 copies and 4 MMAs per 256-element K block of a 128 x 128 tile take 560 cycles before any operand
 // traffic, 860 with it. A CTA pair (cta_group::2) on a 256 x 256 tile needs 12 copies and 4 MMAs of N 256 for four times the work; the
 // long MMAs hide most of the copies: 718 cycles (968 with twice as many N 128 MMAs), and each CTA loads 38 instead of 68 KB.
-// Each K step's copies stand directly in front of its MMA: behind the MMA of the step before they run under it, while twelve in a row in front of four MMAs do
-// not (262144 x 1024 x 4096, rank 1, residual epilogue 540 -> 494 us; 16384 x 4096 x 4096, rank 4, 164.7 -> 157.5).
+// There each K step's copies stand directly in front of its MMA: behind the MMA of the step before they run under it, while twelve in a row in front of four
+// MMAs do not (262144 x 1024 x 4096, rank 1, residual epilogue 540 -> 494 us; 16384 x 4096 x 4096, rank 4, 164.7 -> 157.5). A single CTA's N 128 MMAs are
+// too short for that: eight copies in a row overlap one another better (262144 x 1537 x 512 205 us, 213 with the copies in between; 48 small GEMMs of a token step 239.5, 242).
 // Accumulators: even tiles use the 128-column blocks 0 and 1, odd tiles 1 and 2, and the epilogue drains block 1 first, so that the
 // next tile starts as soon as the shared block has been read. The epilogue code sees a sequence of 128 x 128 sub-tiles.
 template <int EPI, int RK, bool PAIR, bool B2>
@@ -374,16 +375,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                             for (int j = 0; j < 4; ++j) {
                                 tc_cp_sf(t_sfa + 4 * j, sfa_d + static_cast<uint64_t>(j * (512 >> 4)));
                                 tc_cp_sf(t_sfb + 4 * j, sfb_d + static_cast<uint64_t>(j * (512 >> 4)));
-                                tc_mma_nvf4(acc_col, a_d + static_cast<uint64_t>(j * (32 >> 4)), b_d + static_cast<uint64_t>(j * (32 >> 4)), kIdesc,
-                                            t_sfa + 4 * j, t_sfb + 4 * j, ks > 0 || j > 0 ? 1u : 0u);
                             }
+                            tc_mma_nvf4(acc_col, a_d, b_d, kIdesc, t_sfa, t_sfb, ks > 0 ? 1u : 0u);
+#pragma unroll
+                            for (int j = 1; j < 4; ++j)
+                                tc_mma_nvf4(acc_col, a_d + static_cast<uint64_t>(j * (32 >> 4)), b_d + static_cast<uint64_t>(j * (32 >> 4)), kIdesc,
+                                            t_sfa + 4 * j, t_sfb + 4 * j, 1u);
                         } else {
                             for (int j = 0; j < nk; ++j) {
                                 tc_cp_sf(t_sfa + 4 * j, sfa_d + static_cast<uint64_t>(j * (512 >> 4)));
                                 tc_cp_sf(t_sfb + 4 * j, sfb_d + static_cast<uint64_t>(j * (512 >> 4)));
+                            }
+                            for (int j = 0; j < nk; ++j)
                                 tc_mma_nvf4(acc_col, a_d + static_cast<uint64_t>(j * (32 >> 4)), b_d + static_cast<uint64_t>(j * (32 >> 4)), kIdesc,
                                             t_sfa + 4 * j, t_sfb + 4 * j, (ks > 0 || j > 0) ? 1u : 0u);
-                            }
                         }
                         tc_commit(bar_empty + 8 * s);  // frees this smem stage once the MMAs above have read it
                         if (ks == num_ks - 1) tc_commit(bar_acc_full + 8 * buf);  // accumulator of this tile complete
