@@ -28,6 +28,9 @@ def H():
     (159872, 96, 512, 1, 128, 0),       # three chunks of one half
     (40832, 931, 512, 0, 128, 0),       # three fp32 columns
     (75776, 512, 448, 1, 256, 256),     # two whole panels, a group each
+    (75776, 480, 192, 1, 256, 160),     # three groups, and chunks of the last panel behind the third: t has no fourth column for them
+    (160000, 96, 64, 1, 128, 32),       # the same with a panel of one half
+    (160000, 160, 128, 1, 128, 32),     # a group per chunk, the last half has one of four
 ])
 def test_panel_form_equals_the_general_kernel(H, m, n, k, rank, rpm, group):
     import torch
