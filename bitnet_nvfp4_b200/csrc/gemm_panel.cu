@@ -263,8 +263,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_panel_kernel(const __grid_co
         const int z = static_cast<int>(opaque_zero());  // (read-only loads: their addresses depend on this)
         // projections: the group of a chunk is the CTA's for good
         auto group_of = [&](int col) { return p.group_cols > 0 ? static_cast<int>(__umulhi(static_cast<uint32_t>(col), args.group_magic)) : 0; };
-        const int g0 = (!R0 && chunk0 ? group_of(colh[0]) : 0) + z, g1 = (!R0 && chunk1 ? group_of(colh[1]) : 0) + z;  // (a chunk behind the last column has none)
-        const bool two_groups = !R0 && chunk1 && g0 != g1;
+        const int g0 = R0 ? 0 : group_of(min(colh[0], p.n - 1)) + z, g1 = R0 ? 0 : group_of(min(colh[1], p.n - 1)) + z;  // (chunks behind the last column have none of their own)
+        const bool two_groups = !R0 && two && g0 != g1;
         const bool tail_warp = tail && c == 0;
         const int g_tail = R0 || !tail_warp ? 0 : group_of(p.n - 1) + z;
         // the next tile's projections (both halves' and the tail column's) are requested one tile ahead
