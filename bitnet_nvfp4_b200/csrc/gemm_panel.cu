@@ -41,9 +41,7 @@ constexpr int kTailBytes = kTailRows * 128;
 constexpr int kEpiWarps = 16;
 constexpr int kEpiBufBytes = 2 * 32 * 32 * 2;  // two boxes of 32 x 32 halves
 constexpr int kThreads = 64 + kEpiWarps * 32;
-// Row tiles per CTA from which the panel pays (general / panel, us, rank 1): 1537 x 512 with 1 tile 6.6 / 6.2, 2 8.9 / 8.0, 4 13.5 / 12.1, 16 44.7 / 38.5; 512 x 512 with 1
-// 5.9 / 6.9, 2 8.6 / 8.5, 4 14.1 / 13.0, 40 105 / 86; 961 x 320 with 1 6.1 / 6.5, 2 8.5 / 7.9, 40 105 / 84.
-constexpr int kMinTiles = 3;
+constexpr int kEarlyTiles = 6;  // row tiles per CTA up to which an early launch pays
 
 constexpr int kSmemA = 0;
 constexpr int kSmemB = kSmemA + kStages * kStageABytes;        // [K block][half] of 128 rows
@@ -429,7 +427,7 @@ int launch_t(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mb
         configured[dev] = true;
     }
     // (an early launch pays while the kernel is short)
-    launch_pdl_if(args.m_tiles <= 6 * args.per, gemm_panel_kernel<RK>, dim3(static_cast<unsigned>(args.panels * args.per)), kThreads, kSmemAlloc, stream, ma, mb, mbt, md, args);
+    launch_pdl_if(args.m_tiles <= kEarlyTiles * args.per, gemm_panel_kernel<RK>, dim3(static_cast<unsigned>(args.panels * args.per)), kThreads, kSmemAlloc, stream, ma, mb, mbt, md, args);
     return check_launch("gemm_panel_kernel");
 }
 
@@ -439,10 +437,23 @@ int panels_of(const GemmParams& p) { return (p.n - tail_column(p) + kWidth - 1) 
 
 }  // namespace
 
+// The two forms give the same bits and are compared by what they cost, in us beyond the general kernel's start. A panel's CTA passes over 128 x 128 sub-tiles of its
+// row tiles, as many as a CTA of the widest panel has, whatever is left of the last panel and of the SMs that the number of panels does not divide; the general kernel takes waves of
+// tiles over all SMs. General / panel, measured: 262144 x 1537 x 512 204 / 174 (rank 1), 16384 x 1345 x 448 15.3 / 15.0, 8192 x 1537 x 512 9.9 / 10.1; last panel
+// nearly empty: 65536 x 577 x 192 22.8 / 24.2, 75776 x 288 x 128 12.3 / 16.5; idle SMs: 1024 x 19200 x 512 12.4 / 18.5, 2048 x 12800 x 512 14.9 / 18.6; one half: 151552 x 96 x
+// 512 11.1 / 14.5. Over 290 shapes of 384 to 568320 rows, 64 to 24576 columns and K 64 to 512 the choice costs 0.4 % on average against the better of the two, and 9 % at most where it
+// takes the panel (by three row tiles per CTA alone 2.5 % and 55 %).
 bool gemm_panel_applies(const GemmParams& p, int rk, int sms) {
     if (p.epilogue != EPI_F16 || p.k > kMaxK || p.b2 != nullptr || p.beta != 0.0f || rk > 1) return false;
     const int panels = panels_of(p);
-    return panels <= sms && (p.m + BM - 1) / BM >= kMinTiles * (sms / panels);
+    if (panels > sms) return false;
+    const int m_tiles = (p.m + BM - 1) / BM, per = sms / panels, tiles = (m_tiles + per - 1) / per;
+    const bool long_k = p.k > BK, halves = p.n - tail_column(p) > 128;
+    const long long waves = (static_cast<long long>(m_tiles) * ((p.n + 127) / 128) + sms - 1) / sms;
+    // (2 us where the launch is too long to start early; a panel's set-up; with one panel no two tiles of the general kernel share rows of A in time)
+    const float panel_us = 1.2f + (tiles > kEarlyTiles ? 2.0f : 0.0f) + static_cast<float>(tiles) * (halves ? (long_k ? 1.6f : 1.48f) : (long_k ? 1.05f : 0.85f));
+    const float general_us = (waves > 12 ? 2.0f : 0.0f) + static_cast<float>(waves) * (long_k ? 1.12f : panels == 1 ? 1.2f : 0.9f);
+    return panel_us < general_us;
 }
 
 int gemm_panel_launch(const GemmParams& p, int rk, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& md, uint32_t group_magic, int sms, int dev,
