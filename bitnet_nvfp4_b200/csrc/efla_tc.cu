@@ -10,6 +10,12 @@
 // blocks; mma.sync pipe 50 %), 4096 x 64 tokens 280 -> 196 us. Nothing is rounded to fp16 between chunks: the operands of the block products (a G, T - I, a V, U, P)
 // are halves and all sums are fp32, so the result is nearer to the recurrence in float64 (relative error at 128 tokens 4.3e-4 instead of 5.0e-4).
 //
+// Keys far from unit length would leave the halves' range: a G and P grow with the ratio of two keys' lengths, U falls with its key's square. Where |k_s|
+// is below 2^-6 or from 2^6 on, the unknown is s U_s with s a power of two next to |k_s|: rows of a G and a V take the factor s_t, columns of a G and of P 1 / s_s, all in
+// fp32 and exact, so that no coefficient exceeds 64 and s U is as large as y. Tokens in between have s = 1, and blocks of them skip the products. (128 tokens, relative error with s = 1
+// throughout: |k| near 8e-5 1.8e-3, near 800 1.2e-2, and infinities from |k| = 65504 on. What it costs keys of ordinary length: 32 sequences of 8 heads 7.4 -> 7.75 us,
+// 8192 sequences 911 -> 919, 4096 x 64 tokens the same; where all blocks are scaled 1170.)
+//
 // Sequences of at most 64 tokens share a tile: R = 8 / NB of them (NB blocks of 16 tokens each), whose products across sequences are not read.
 //
 // One CTA (288 threads, two per SM) walks units of R sequences of one head, three roles one behind the other:
@@ -21,6 +27,7 @@
 //              that U's accumulator fragments are the next products' A fragments; Y takes V's place in shared memory and leaves by TMA.
 
 #include <algorithm>
+#include <cfloat>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -45,9 +52,13 @@ constexpr int kSmemP = kSmemL + kTriBytes;
 constexpr int kDBlock = 272;                  // floats of a diagonal block of -a G, by columns (and 16 for the banks)
 constexpr int kSmemD = kSmemP + kTriBytes;
 constexpr int kSmemAlpha = kSmemD + kBlocks * kDBlock * 4;
-constexpr int kSmemBar = kSmemAlpha + kTok * 4;
+constexpr int kSmemKey = kSmemAlpha + kTok * 4;  // 1 / s of the tokens, and whether 32 of them have another s than 1
+constexpr int kSmemBar = kSmemKey + kTok * 4 + 16;
+constexpr int kBarTriFree = 96;               // of the barriers: see the kernel
 constexpr int kSmemAlloc = kSmemBar + 256 + 1024;
 static_assert(2 * (kSmemAlloc + 1024) <= 233472, "two CTAs per SM");
+
+constexpr float kKeyLow = 1.0f / 4096.0f, kKeyHigh = 4096.0f;  // squared lengths of keys with s = 1
 
 constexpr int kTmemCols = 256;  // G | Q K^T
 constexpr uint32_t kIdescF16 = (1u << 4) | (static_cast<uint32_t>(kTok >> 3) << 17) | (static_cast<uint32_t>(kTok >> 4) << 24);  // f16 x f16 -> fp32, K-major
@@ -74,9 +85,129 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_shared(uint32_t addr, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+
 // Blocks of 16 x 16 halves, block (i, j <= i) at tri(i, j): four 8 x 8 matrices of 128 bytes, (row half, column half) at 128 * row half + 256 * column
 // half. A row of eight halves is one 16-byte piece, so the token-per-lane stores and every ldmatrix phase touch 128 contiguous bytes.
 __device__ __forceinline__ uint32_t tri(int i, int j) { return static_cast<uint32_t>(i * (i + 1) / 2 + j) * 512u; }
+
+// What a token's thread leaves for the substitution, in its warp's 32 rows of L, T and P. FAR: columns take their keys' scales (in the chunks whose bit is set).
+struct TokenRows {
+    uint32_t smem_base, trow;  // the warp's lanes of tensor memory
+    int first_chunk;           // 32 columns at a time, from the one in which the warp's first sequence starts
+    uint32_t far, n;           // n: units before this one
+    float alpha, qinv;
+};
+// rg: the chunk of G on the diagonal. Returns false when a wait has expired.
+template <bool FAR>
+__device__ __forceinline__ bool token_rows(const TokenRows& a, uint32_t (&rg)[32]) {
+    const int w = static_cast<int>(threadIdx.x) >> 5, lane = threadIdx.x & 31, t = 32 * w + lane, half = lane >> 4;
+    const int bi = 2 * w + half;  // this token's block row
+    const uint32_t lrow = static_cast<uint32_t>((lane >> 3) & 1) * 128u + static_cast<uint32_t>(lane & 7) * 16u;  // this token's row in its blocks
+    const uint32_t l_row = a.smem_base + kSmemL + tri(bi, 0) + lrow, p_row = a.smem_base + kSmemP + tri(bi, 0) + lrow;
+    const uint32_t dcol = a.smem_base + kSmemD + static_cast<uint32_t>(bi * kDBlock * 4);  // the token's diagonal block of -a G by columns
+    const float alpha = a.alpha;
+    auto scale_columns = [&](uint32_t (&r)[32], int cc) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+            const float4 f = ld_shared_f4(a.smem_base + kSmemKey + 128 * cc + 4 * j);
+            r[j] = __float_as_uint(__uint_as_float(r[j]) * f.x);
+            r[j + 1] = __float_as_uint(__uint_as_float(r[j + 1]) * f.y);
+            r[j + 2] = __float_as_uint(__uint_as_float(r[j + 2]) * f.z);
+            r[j + 3] = __float_as_uint(__uint_as_float(r[j + 3]) * f.w);
+        }
+    };
+    // 32 scaled columns of this token's row as halves: four pieces of eight, from block column 2 cc on
+    auto store_row = [&](const float (&x)[32], uint32_t row, int cc, bool left, bool right) {
+#pragma unroll
+        for (int c8 = 0; c8 < 4; ++c8)
+            if (c8 < 2 ? left : right)
+                st_shared_v4(row + static_cast<uint32_t>(2 * cc + (c8 >> 1)) * 512u + (c8 & 1) * 256u, pack_half2(x[8 * c8], x[8 * c8 + 1]),
+                             pack_half2(x[8 * c8 + 2], x[8 * c8 + 3]), pack_half2(x[8 * c8 + 4], x[8 * c8 + 5]), pack_half2(x[8 * c8 + 6], x[8 * c8 + 7]));
+    };
+    auto scaled = [](float f, const uint32_t (&r)[32], float (&x)[32]) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+            const float2 y = __fmul2_rn(make_float2(f, f), make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])));
+            x[j] = y.x;
+            x[j + 1] = y.y;
+        }
+    };
+    if (FAR && ((a.far >> w) & 1u)) scale_columns(rg, w);
+    uint32_t left[8], hv[8];  // the left half of the diagonal chunk and T - I, as halves
+#pragma unroll
+    for (int j = 0; j < 8; ++j) left[j] = pack_half2(-alpha * __uint_as_float(rg[2 * j]), -alpha * __uint_as_float(rg[2 * j + 1]));
+    __syncwarp();  // (the previous unit's reads are done)
+#pragma unroll
+    for (int s = 0; s < 16; ++s) st_shared(dcol + 64 * s + 4 * (lane & 15), __float_as_uint(-alpha * __uint_as_float(half ? rg[16 + s] : rg[s])));
+    __syncwarp();
+    {
+        // T = (I + a G)^-1 of the token's block by forward substitution: lane c of a half owns column c; a finished element goes
+        // into all later ones at once
+        const int c = lane & 15;
+        float col[16];
+#pragma unroll
+        for (int s = 0; s < 16; ++s) col[s] = s == c ? 1.0f : 0.0f;
+#pragma unroll
+        for (int s = 0; s < 15; ++s)
+#pragma unroll
+            for (int t4 = (s + 1) / 4 * 4; t4 < 16; t4 += 4) {
+                const float4 lv = ld_shared_f4(dcol + 64 * s + 4 * t4);
+                if (t4 > s) col[t4] = fmaf(lv.x, col[s], col[t4]);
+                if (t4 + 1 > s) col[t4 + 1] = fmaf(lv.y, col[s], col[t4 + 1]);
+                if (t4 + 2 > s) col[t4 + 2] = fmaf(lv.z, col[s], col[t4 + 2]);
+                if (t4 + 3 > s) col[t4 + 3] = fmaf(lv.w, col[s], col[t4 + 3]);
+            }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) hv[e] = pack_half2(2 * e == c ? 0.0f : col[2 * e], 2 * e + 1 == c ? 0.0f : col[2 * e + 1]);
+    }
+    if (a.n > 0 && !__all_sync(0xffffffffu, mbar_wait(a.smem_base + kSmemBar + kBarTriFree + 8 * w, (a.n - 1) & 1u, 17))) return false;
+    st_shared(a.smem_base + kSmemAlpha + 4 * t, __float_as_uint(alpha));
+    const uint32_t d = l_row + static_cast<uint32_t>(bi) * 512u;  // row c of (T - I)^T
+    st_shared_v4(d, hv[0], hv[1], hv[2], hv[3]);
+    st_shared_v4(d + 256u, hv[4], hv[5], hv[6], hv[7]);
+    if (half == 1) {
+        st_shared_v4(d - 512u, left[0], left[1], left[2], left[3]);
+        st_shared_v4(d - 256u, left[4], left[5], left[6], left[7]);
+    }
+    for (int cc = a.first_chunk; cc < w; ++cc) {
+        uint32_t rc[32], rp[32];
+        float x[32];
+        tmem_ld32(a.trow + 32 * cc, rc);
+        tmem_ld32(a.trow + 128 + 32 * cc, rp);
+        tmem_ld_wait();
+        if (FAR && ((a.far >> cc) & 1u)) {
+            scale_columns(rc, cc);
+            scale_columns(rp, cc);
+        }
+        scaled(-alpha, rc, x);
+        store_row(x, l_row, cc, true, true);
+        scaled(a.qinv, rp, x);
+        store_row(x, p_row, cc, true, true);
+    }
+    uint32_t rp[32];
+    float x[32];
+    tmem_ld32(a.trow + 128 + 32 * w, rp);
+    tmem_ld_wait();
+    if (FAR && ((a.far >> w) & 1u)) scale_columns(rp, w);
+    scaled(a.qinv, rp, x);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) x[j] = j <= lane ? x[j] : 0.0f;
+    store_row(x, p_row, w, true, half == 1);
+    return true;
+}
+// (a function of its own: the products and their registers stay out of the usual path)
+__device__ __noinline__ bool token_rows_far(const TokenRows a) {
+    uint32_t rg[32];
+    tmem_ld32(a.trow + 32 * (threadIdx.x >> 5), rg);
+    tmem_ld_wait();
+    return token_rows<true>(a, rg);
+}
 
 template <int NB>
 __global__ void __launch_bounds__(kThreads, 2) efla_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -94,8 +225,9 @@ __global__ void __launch_bounds__(kThreads, 2) efla_tc_kernel(const __grid_const
     const uint32_t bar_prod = bar_v_free + 16;       // products complete
     const uint32_t bar_prod_free = bar_prod + 8;     // tensor memory has been read (4)
     const uint32_t bar_tri = bar_prod_free + 8;      // L, T, P and the step sizes of 32 tokens are there (4 barriers)
-    const uint32_t bar_tri_free = bar_tri + 32;      // and have been read (4 x 4)
-    const uint32_t tmem_slot = bar_tri_free + 32;
+    const uint32_t bar_tri_free = bar_qk + kBarTriFree;  // and have been read (4 x 4)
+    const uint32_t bar_key = bar_tri_free + 32;      // the keys' scales are there (the warps with tokens)
+    const uint32_t tmem_slot = bar_key + 8;
     volatile uint32_t* tmem_slot_gen = reinterpret_cast<volatile uint32_t*>(smem_gen + kSmemBar + (tmem_slot - bar_qk));
 
     if (threadIdx.x == 0) {
@@ -107,6 +239,7 @@ __global__ void __launch_bounds__(kThreads, 2) efla_tc_kernel(const __grid_const
         }
         mbar_init(bar_prod, 1);
         mbar_init(bar_prod_free, 4);
+        mbar_init(bar_key, (kBlocks / NB * NB + 1) / 2);
         for (int b = 0; b < 4; ++b) {
             mbar_init(bar_tri + 8 * b, 1);
             mbar_init(bar_tri_free + 8 * b, 4);
@@ -186,14 +319,10 @@ __global__ void __launch_bounds__(kThreads, 2) efla_tc_kernel(const __grid_const
         // ------------------------------ a thread per token ------------------------------
         const int w = warp, t = 32 * w + lane, half = lane >> 4;
         const bool rows = 2 * w < kUsed;  // this warp has tokens
-        const int bi = 2 * w + half;      // this token's block row
         const int tok = t % (16 * NB);    // and its place in its sequence
         const unsigned sub = static_cast<unsigned>(t / (16 * NB));
         const int first_chunk = (2 * w - 2 * w % NB) / 2;  // 32 columns at a time, from the one in which the warp's first sequence starts
-        const uint32_t lrow = static_cast<uint32_t>((lane >> 3) & 1) * 128u + static_cast<uint32_t>(lane & 7) * 16u;  // this token's row in its blocks
-        const uint32_t l_row = smem_base + kSmemL + tri(bi, 0) + lrow, p_row = smem_base + kSmemP + tri(bi, 0) + lrow;
-        float* dcol = reinterpret_cast<float*>(smem_gen + kSmemD) + bi * kDBlock;  // the token's diagonal block of -a G by columns
-        float* alpha_sh = reinterpret_cast<float*>(smem_gen + kSmemAlpha);
+        const uint32_t key_sh = smem_base + kSmemKey, far_sh = key_sh + kTok * 4;
         // ldmatrix rows of the two 16-token blocks (128B swizzle): matrices (tokens 0-7 | d 0-7), (0-7 | 8-15), (8-15 | 0-7), (8-15 | 8-15)
         const uint32_t lm = static_cast<uint32_t>(32 * w + (lane >> 4) * 8 + (lane & 7)) * 128u + static_cast<uint32_t>(((lane >> 3) & 1) ^ (lane & 7)) * 16u;
         // squared norms of this warp's 32 queries from the diagonals of Q Q^T, handed to the token's thread
@@ -224,22 +353,6 @@ __global__ void __launch_bounds__(kThreads, 2) efla_tc_kernel(const __grid_const
             }
             return mine;
         };
-        // 32 scaled columns of this token's row as halves: four pieces of eight, from block column 2 cc on
-        auto store_row = [&](const float (&x)[32], uint32_t row, int cc, bool left, bool right) {
-#pragma unroll
-            for (int c8 = 0; c8 < 4; ++c8)
-                if (c8 < 2 ? left : right)
-                    st_shared_v4(row + static_cast<uint32_t>(2 * cc + (c8 >> 1)) * 512u + (c8 & 1) * 256u, pack_half2(x[8 * c8], x[8 * c8 + 1]),
-                                 pack_half2(x[8 * c8 + 2], x[8 * c8 + 3]), pack_half2(x[8 * c8 + 4], x[8 * c8 + 5]), pack_half2(x[8 * c8 + 6], x[8 * c8 + 7]));
-        };
-        auto scaled = [](float f, const uint32_t (&r)[32], float (&x)[32]) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-                const float2 y = __fmul2_rn(make_float2(f, f), make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])));
-                x[j] = y.x;
-                x[j + 1] = y.y;
-            }
-        };
         uint32_t n = 0;
         float braw = 0.0f;
         auto fetch_beta = [&](unsigned u) {
@@ -260,84 +373,52 @@ __global__ void __launch_bounds__(kThreads, 2) efla_tc_kernel(const __grid_const
             if (!ok) break;
             tc_fence_after();
             const uint32_t trow = tmem_base + (static_cast<uint32_t>(32 * w) << 16);
-            float alpha = 0.0f;
-            uint32_t left[8], hv[8];  // the left half of the diagonal chunk and T - I, as halves
             if (rows) {
                 // the chunk of G on the diagonal: block (2 w + 1, 2 w) in its lower left and two diagonal blocks; G_tt is the key's squared norm
                 uint32_t rg[32];
                 tmem_ld32(trow + 32 * w, rg);
                 tmem_ld_wait();
-                uint32_t sel[16];
-#pragma unroll
-                for (int j = 0; j < 16; ++j) sel[j] = half ? rg[16 + j] : rg[j];  // the diagonal block's row
                 uint32_t pick[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) pick[j] = (lane & 8) ? sel[8 + j] : sel[j];
+                for (int j = 0; j < 8; ++j) {
+                    const uint32_t lo = half ? rg[16 + j] : rg[j], hi = half ? rg[24 + j] : rg[8 + j];
+                    pick[j] = (lane & 8) ? hi : lo;
+                }
 #pragma unroll
                 for (int k = 4; k > 0; k >>= 1)
 #pragma unroll
                     for (int j = 0; j < k; ++j) pick[j] = (lane & k) ? pick[j + k] : pick[j];
                 const float kss = __uint_as_float(pick[0]);
+                // the key's scale: the next unit's are written behind its products, which wait for every warp to have read this one's
+                const bool off = !(kss >= kKeyLow && kss < kKeyHigh) && kss > 0.0f && kss <= FLT_MAX;
+                uint32_t far = __any_sync(0xffffffffu, off) ? 1u << w : 0u;  // bit c: tokens 32 c .. have another s than 1
+                float key = 1.0f;
+                if (far) {
+                    float key_inv = 1.0f;
+                    if (off) {
+                        const int e = (static_cast<int>(__float_as_uint(kss) >> 23) - 127) >> 1;
+                        key = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+                        key_inv = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
+                    }
+                    st_shared(key_sh + 4 * t, __float_as_uint(key_inv));
+                }
+                if (lane == 0) st_shared(far_sh + 4 * w, far);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_key);
                 const float lambda = kss < p.eps ? p.eps : kss;
                 // sigmoid and the final quotient with the fast exponential / division (about 2 ulp each: far below the fp16
                 // rounding of every operand alpha touches); expm1f keeps its accuracy for small beta * lambda
                 const float beta = __fdividef(1.0f, 1.0f + __expf(-logit));
-                alpha = tok < p.T ? __fdividef(-expm1f(-(beta * lambda)), lambda + p.eps) : 0.0f;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) left[j] = pack_half2(-alpha * __uint_as_float(rg[2 * j]), -alpha * __uint_as_float(rg[2 * j + 1]));
-                __syncwarp();  // (the previous unit's reads are done)
-#pragma unroll
-                for (int s = 0; s < 16; ++s) dcol[16 * s + (lane & 15)] = -alpha * __uint_as_float(sel[s]);
-                __syncwarp();
-                // T = (I + a G)^-1 of the token's block by forward substitution: lane c of a half owns column c; a finished element goes
-                // into all later ones at once
-                const int c = lane & 15;
-                float col[16];
-#pragma unroll
-                for (int s = 0; s < 16; ++s) col[s] = s == c ? 1.0f : 0.0f;
-#pragma unroll
-                for (int s = 0; s < 15; ++s)
-#pragma unroll
-                    for (int t4 = (s + 1) / 4 * 4; t4 < 16; t4 += 4) {
-                        const float4 lv = *reinterpret_cast<const float4*>(dcol + 16 * s + t4);
-                        if (t4 > s) col[t4] = fmaf(lv.x, col[s], col[t4]);
-                        if (t4 + 1 > s) col[t4 + 1] = fmaf(lv.y, col[s], col[t4 + 1]);
-                        if (t4 + 2 > s) col[t4 + 2] = fmaf(lv.z, col[s], col[t4 + 2]);
-                        if (t4 + 3 > s) col[t4 + 3] = fmaf(lv.w, col[s], col[t4 + 3]);
-                    }
-#pragma unroll
-                for (int e = 0; e < 8; ++e) hv[e] = pack_half2(2 * e == c ? 0.0f : col[2 * e], 2 * e + 1 == c ? 0.0f : col[2 * e + 1]);
-            }
-            if (rows && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_tri_free + 8 * w, (n - 1) & 1u, 17));
-            if (!ok) break;
-            if (rows) {
-                alpha_sh[t] = alpha;
-                const uint32_t d = l_row + static_cast<uint32_t>(bi) * 512u;  // row c of (T - I)^T
-                st_shared_v4(d, hv[0], hv[1], hv[2], hv[3]);
-                st_shared_v4(d + 256u, hv[4], hv[5], hv[6], hv[7]);
-                if (half == 1) {
-                    st_shared_v4(d - 512u, left[0], left[1], left[2], left[3]);
-                    st_shared_v4(d - 256u, left[4], left[5], left[6], left[7]);
+                const float alpha = tok < p.T ? __fdividef(-expm1f(-(beta * lambda)), lambda + p.eps) * key : 0.0f;  // a s
+                if (w > 0) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_key, n & 1u, 20));
+                    if (!ok) break;
+                    const float4 f = ld_shared_f4(far_sh);
+                    far |= (__float_as_uint(f.x) | __float_as_uint(f.y) | __float_as_uint(f.z)) & ((1u << w) - 1u);
                 }
-                for (int cc = first_chunk; cc < w; ++cc) {
-                    uint32_t rg[32], rp[32];
-                    float x[32];
-                    tmem_ld32(trow + 32 * cc, rg);
-                    tmem_ld32(trow + 128 + 32 * cc, rp);
-                    tmem_ld_wait();
-                    scaled(-alpha, rg, x);
-                    store_row(x, l_row, cc, true, true);
-                    scaled(qinv, rp, x);
-                    store_row(x, p_row, cc, true, true);
-                }
-                uint32_t rp[32];
-                float x[32];
-                tmem_ld32(trow + 128 + 32 * w, rp);
-                tmem_ld_wait();
-                scaled(qinv, rp, x);
-#pragma unroll
-                for (int j = 0; j < 32; ++j) x[j] = j <= lane ? x[j] : 0.0f;
-                store_row(x, p_row, w, true, half == 1);
+                const TokenRows r = {smem_base, trow, first_chunk, far, n, alpha, qinv};
+                ok = __builtin_expect(far, 0) ? token_rows_far(r) : token_rows<false>(r, rg);
+                if (!ok) break;
             }
             tc_fence_before();
             __syncwarp();

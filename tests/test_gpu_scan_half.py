@@ -63,6 +63,36 @@ def test_closed_form(H, T, heads, seqs, scale):
         assert closed <= 1.03 * chunked
 
 
+@pytest.mark.parametrize("T", [48, 64, 100, 128])
+@pytest.mark.parametrize("q_scale,k_scale,v_scale,decades", [(1.0, 1e-5, 1000.0, 0), (1.0, 1e-4, 100.0, 0), (30.0, 100.0, 100.0, 0), (0.01, 1e3, 1e3, 0), (0.01, 1e4, 1e4, 0),
+                                                             (1.0, 10.0, 1.0, 3), (0.01, 10.0, 100.0, 3), (1.0, 0.1, 10.0, 3), (1.0, 100.0, 1e3, 2)])
+def test_keys_of_any_length(H, T, q_scale, k_scale, v_scale, decades):
+    """Coefficients and the solution are halves whatever the keys' lengths, the same for all tokens or spread over decades: the error is that of keys of
+    ordinary length. (Values keep y above fp16's smallest numbers.)"""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(20 * T, 3, 2, 64, device="cuda", generator=g) * torch.tensor([q_scale, k_scale, v_scale], device="cuda")[None, :, None, None]
+    x[:, 1] *= 10.0 ** ((torch.rand(20 * T, 1, 1, device="cuda", generator=g) * 2 - 1) * decades)
+    qkv = torch.nn.functional.pad(x.clamp(-65504, 65504).half().reshape(20 * T, -1), (0, 16))
+    beta = torch.randn(20 * T, device="cuda", generator=g) * 2
+    ref = exact(qkv, beta, 2, 20, T)
+    assert float((run(H, qkv, beta, 2, 20, T).double() - ref).norm() / ref.norm()) <= 6e-4
+
+
+@pytest.mark.parametrize("T", [48, 64])
+def test_a_sequence_does_not_depend_on_its_tile(H, T):
+    """Two sequences share a tile: one with keys of extreme lengths leaves the other's bits alone."""
+    import torch
+    qkv, beta = inputs(T, 2, 6, 0.3)
+    clean = run(H, qkv, beta, 2, 6, T).reshape(6, T, 128)
+    for s, factor in ((0, 1e4), (3, 1e-5), (5, 1e4)):
+        far = qkv.clone().reshape(6, T, -1)
+        far[s, :, 128:256] *= factor
+        got = run(H, far.reshape(6 * T, -1), beta, 2, 6, T).reshape(6, T, 128)
+        assert not torch.equal(got[s], clean[s])
+        assert all(torch.equal(got[i], clean[i]) for i in range(6) if i != s)
+
+
 @pytest.mark.parametrize("T", [33, 64, 100, 128])
 def test_a_sequence_does_not_depend_on_its_company(H, T):
     import torch
