@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         tmem_alloc(bar0 + 32, kSqTmemCols);
         tmem_relinquish();
     }
-    bool ok = true;  // no wait has expired
+    bool ok = true;  // no wait of this thread has expired; behind one that has there are no others, and what the thread would write stays unwritten
 
     // ---------------- 1. norms and scalars ----------------
     for (int t0 = 2 * warp; t0 < kSeqMaxT; t0 += 32) {  // two rows of each at a time: twice the loads in flight (a row's trip to DRAM paced this step)
@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     };
     auto gram_block = [&](KQ& x, int db) {  // (the next block but one is requested when this one has left the registers)
         const int buf = db & 1;
-        if (db >= 2) ok = mbar_wait(bar0 + 8 * buf, static_cast<uint32_t>(db / 2 - 1) & 1u, 21) && ok;  // the stage's last products have read it
+        if (db >= 2) ok = ok && mbar_wait(bar0 + 8 * buf, static_cast<uint32_t>(db / 2 - 1) & 1u, 21);  // the stage's last products have read it
         uint8_t* st = sm + buf * kSqStage + s_at;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
             if (db + 1 < nd) gram_block(odd, db + 1);
         }
     }
-    for (int db = max(0, nd - 2); db < nd; ++db) ok = mbar_wait(bar0 + 8 * (db & 1), static_cast<uint32_t>(db / 2) & 1u, 22) && ok;
+    for (int db = max(0, nd - 2); db < nd; ++db) ok = ok && mbar_wait(bar0 + 8 * (db & 1), static_cast<uint32_t>(db / 2) & 1u, 22);
     tc_fence_after();
     __syncthreads();  // (everyone has seen the products done before their operands' places are taken)
     struct VT { float4 v[4]; };
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     float* out = reinterpret_cast<float*>(sm + kSqOut);
     // rows t of 256 bytes, 16-byte piece ^ t % 16: the column group's rows go in, whole rows of the output come out, both without bank conflicts
     auto finish = [&](int l, float ds, bool tile_bad) {  // the CTA's l-th tile
-        ok = mbar_wait(bar0 + 16 + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 23) && ok;
+        ok = ok && mbar_wait(bar0 + 16 + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 23);
         tc_fence_after();
         float y[16];
         sq_tmem_ld16(t_lane + (l & 1) * 64 + 16 * cg, y);
@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
         __syncthreads();
         const int c = (ct0 + l) * 64 + 2 * lane;
         for (int t = warp; t < T; t += 16)
-            if (c < hd) *reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float2*>(out + t * 64 + (((lane >> 1) ^ (t & 15)) << 2) + 2 * (lane & 1));
+            if (ok && c < hd) *reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float2*>(out + t * 64 + (((lane >> 1) ^ (t & 15)) << 2) + 2 * (lane & 1));
     };
     float ds_prev = 0.0f;
     bool bad_prev = false;
@@ -609,7 +609,6 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     }
     __syncthreads();  // (the tile before it has left)
     finish(nct - 1, ds_prev, bad_prev);
-    (void)ok;
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {

@@ -85,6 +85,20 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+// Waits for the 128 threads that meet at barrier 1. Does x hold for all of them?
+__device__ __forceinline__ bool all_of_barrier1(bool x) {
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.and.pred q, 1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all)
+        : "r"(static_cast<uint32_t>(x))
+        : "memory");
+    return all != 0;
+}
+
 __device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
@@ -441,11 +455,10 @@ __global__ void __launch_bounds__(kThreads, 2) efla_tc_kernel(const __grid_const
         for (unsigned u = blockIdx.x; u < total && ok; u += gridDim.x, ++n) {
             const uint32_t buf = n & 1u;
             ok = __all_sync(0xffffffffu, mbar_wait(bar_v + 8 * buf, (n >> 1) & 1u, 18));
-            if (!ok) break;
             const uint32_t v_addr = v_lane + buf * kTileBytes;
             // The chain from one U to the next is two products; the sums over earlier blocks for the next X and for Y fill it.
             // Rows of L, T, P and the step sizes arrive and are given back 32 tokens at a time, so the next unit's follow while later rows of this one are
-            // still read. (A wait that expires lets the unit run on: its results are not used, and the loop ends behind it.)
+            // still read. (A wait that expires lets the unit run on, and the four warps agree behind it: its output stays unwritten, and all of them end their loop.)
             auto start_x = [&](int b, float (&X)[2][4]) {  // a V, transposed
                 if (b % 2 == 0) ok = __all_sync(0xffffffffu, mbar_wait(bar_tri + 8 * (b / 2), n & 1u, 19)) && ok;
                 uint32_t vf[4];
@@ -519,8 +532,8 @@ __global__ void __launch_bounds__(kThreads, 2) efla_tc_kernel(const __grid_const
                 }
             }
             fence_async_smem();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (warp == 4 && lane == 0) {
+            ok = all_of_barrier1(ok);
+            if (ok && warp == 4 && lane == 0) {
                 const unsigned su = u / heads;
                 const int seq = static_cast<int>(su * R), x = static_cast<int>(u - su * heads) * 64;
                 tma_store_3d(&map_o, smem_base + kSmemV + buf * kTileBytes, x, 0, seq);  // (clips at T and at the last sequence)
