@@ -292,6 +292,11 @@ class PopulationModel:
         _l.check(self.lib.bnf4_model_eval_base(self.h, out.data_ptr(), _stream()))
         return out
 
+    def check_device(self):
+        """Raises if a bounded wait has expired in a kernel since the last look (its outputs are not valid). Waits for the current stream."""
+        if getattr(self, "h", None):
+            _l.check(_l.load().bnf4_device_error(_stream(), None))
+
     def update(self, pair_weights: torch.Tensor, lr=0.8, thresh=0.008, use_adaptive=True, adaptive_beta=0.95, adaptive_eps=1e-3,
                train_pos=True):
         assert pair_weights.is_cuda and pair_weights.dtype == torch.float32 and pair_weights.numel() == self.pairs

@@ -68,7 +68,8 @@ def _loss_of(model, tokens: np.ndarray, targets: np.ndarray) -> float:
 
 def train(model, corpus: np.ndarray, cfg: TrainConfig, rank: int = 0, world: int = 1, group=None, log=None) -> list[dict]:
     """Runs cfg.epochs epochs on `model` (a population.PopulationModel) and returns one record per epoch with the reference's
-    log fields. Every rank must call it with the same arguments; `log` (rank 0) receives each record's line."""
+    log fields. Every rank must call it with the same arguments; `log` (rank 0) receives each record's line. Raises after an
+    epoch in which a kernel on this rank's device reported an error."""
     B, T = model.cfg.batch, model.cfg.seq
     data_seed = cfg.data_seed or cfg.seed
     on_gpu = torch.cuda.is_available()
@@ -110,6 +111,9 @@ def train(model, corpus: np.ndarray, cfg: TrainConfig, rank: int = 0, world: int
                 model.set_tokens(tokens, targets)
             val_s = time.perf_counter() - t0
         sync()
+        check = getattr(model, "check_device", None)
+        if check is not None:  # a kernel that gave up waiting leaves outputs unwritten: no further epoch on them
+            check()
         wall_s = time.perf_counter() - t_epoch
         tokens_eval = cfg.pairs * 2.0 * B * T
         tokens_total = tokens_eval + B * T + (B * T if do_val else 0)

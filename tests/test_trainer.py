@@ -91,6 +91,33 @@ def test_fixed_train_restores_the_training_batch():
     assert toks[3] == ("tokens", train_sum)
 
 
+def test_a_device_error_ends_the_loop():
+    """The epoch in which a kernel gave up waiting is the last one."""
+    corpus = synth.zipf_corpus(1 << 12, 1.1, 5)
+
+    class Failing(FakeModel):
+        def check_device(self):
+            self.calls.append(("check",))
+            if sum(c == ("check",) for c in self.calls) == 2:
+                raise RuntimeError("a bounded wait expired")
+
+    m, lines = Failing(), []
+    with pytest.raises(RuntimeError, match="bounded wait"):
+        trainer.train(m, corpus, trainer.TrainConfig(epochs=4, pairs=2, seed=3), log=lines.append)
+    assert len(lines) == 1 and sum(c[0] == "prepare" for c in m.calls) == 2
+
+
+@pytest.mark.gpu
+def test_the_model_reads_the_device_error_word(monkeypatch):
+    from bitnet_nvfp4_b200 import lib, population
+    model = population.PopulationModel(population.Config(hidden=128, layers=1, seq=16, batch=2, heads=2, max_pairs=2))
+    model.check_device()
+    monkeypatch.setattr(lib.load(), "bnf4_device_error", lambda stream, code: 4)  # (a fake of the call: no kernel is made to wait)
+    with pytest.raises(lib.Bnf4Error):
+        model.check_device()
+    model.close()
+
+
 @pytest.mark.gpu
 def test_train_loop_equals_manual_steps():
     from bitnet_nvfp4_b200 import population
