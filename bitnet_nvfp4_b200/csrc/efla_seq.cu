@@ -241,8 +241,9 @@ __device__ __forceinline__ void sq_tmem_ld16(uint32_t taddr, float (&r)[16]) {
         : "memory");
 }
 
-// cs CTAs share a unit: each does steps 1 to 4 (the same sums) and its share of the column tiles of step 5.
-__global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaParams p, const int cs) {
+// cs CTAs share a unit: each does steps 1 to 4 (the same sums) and its share of the column tiles of step 5. meet: they form a cluster, and none writes
+// before all have read q and k, where the output may lie.
+__global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaParams p, const int cs, const int meet) {
     pdl_wait();
     extern __shared__ uint8_t sm_raw[];
     uint8_t* sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
@@ -410,6 +411,7 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     for (int db = max(0, nd - 2); db < nd; ++db) ok = ok && mbar_wait(bar0 + 8 * (db & 1), static_cast<uint32_t>(db / 2) & 1u, 22);
     tc_fence_after();
     __syncthreads();  // (everyone has seen the products done before their operands' places are taken)
+    if (meet) cluster_sync();
     struct VT { float4 v[4]; };
     auto load_v = [&](VT& x, int c0) {
 #pragma unroll
@@ -935,24 +937,30 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
 
 }  // namespace
 
-// Does the output lie apart from q, k and v?
-static bool seq_output_apart(const EflaParams& p) {
+// Do the addresses from the output's first to its last lie apart from those of q, k or v?
+static bool seq_ranges_apart(const EflaParams& p, const void* in) {
     if (p.seqs <= 0) return true;
     const size_t last = static_cast<size_t>(p.seqs) * p.T - 1;
-    const char* o = static_cast<const char*>(p.out);
-    const char* o_end = o + (last * p.ld_out + p.hidden) * sizeof(float);
-    for (const void* in : {static_cast<const void*>(p.q), static_cast<const void*>(p.k), static_cast<const void*>(p.v)}) {
-        const char* a = static_cast<const char*>(in);
-        if (o < a + (last * p.ld_qkv + p.hidden) * sizeof(float) && a < o_end) return false;
-    }
-    return true;
+    const char *o = static_cast<const char*>(p.out), *a = static_cast<const char*>(in);
+    return o >= a + (last * p.ld_qkv + p.hidden) * sizeof(float) || a >= o + (last * p.ld_out + p.hidden) * sizeof(float);
+}
+// How the output lies to q, k or v: apart from it (also in other columns of the same rows), exactly in its place, or in some other way.
+enum SeqOverlap { SEQ_APART, SEQ_SAME, SEQ_ACROSS };
+static SeqOverlap seq_overlap(const EflaParams& p, const void* in) {
+    if (seq_ranges_apart(p, in)) return SEQ_APART;
+    if (p.ld_out != p.ld_qkv) return SEQ_ACROSS;
+    if (in == p.out) return SEQ_SAME;
+    const long long row = static_cast<long long>(p.ld_qkv) * sizeof(float), width = static_cast<long long>(p.hidden) * sizeof(float);
+    if (row < 2 * width) return SEQ_ACROSS;
+    const long long d = ((static_cast<long long>(reinterpret_cast<intptr_t>(p.out)) - static_cast<long long>(reinterpret_cast<intptr_t>(in))) % row + row) % row;
+    return d >= width && row - d >= width ? SEQ_APART : SEQ_ACROSS;
 }
 
 // The closed form's work per token grows with the sequence, the per-token kernel's does not, but the latter spreads a unit over several SMs. One head of
 // 512: 322 tokens 0.69 / 1.16 ms (closed form / per token) for 4 sequences, 2.4 / 17.5 ms for 400; 1000 tokens 4.4 / 3.6 ms for 4, 5.0 / 8.3 ms for 40.
 // The number of sequences has no say: the two round differently, and a member's loss must not depend on how many share its wave.
 static bool seq_long_pays(const EflaParams& p) {
-    return p.T <= kLgMaxT && seq_output_apart(p);  // (the output holds w before all of q, k and v have been read)
+    return p.T <= kLgMaxT && seq_ranges_apart(p, p.q) && seq_ranges_apart(p, p.k) && seq_ranges_apart(p, p.v);  // (the output holds w before all of them have been read)
 }
 
 // (heads of 32 are faster one warp each, token by token: efla_head32_kernel)
@@ -985,12 +993,31 @@ int efla_seq_launch(const EflaParams& p, cudaStream_t stream) {
         if (dev < 64) configured[dev].store(true, std::memory_order_relaxed);
     }
     // Few units leave SMs idle: two or four CTAs each take a share of a unit's column tiles, as long as all run at once (the sums before them are done by
-    // each) and none writes what another still reads. One head of 512, 128 tokens: 32 sequences
-    // 45 us with one CTA each, 34 with four; 70 sequences 45 with one, 39 with two.
+    // each). One head of 512, 128 tokens: 32 sequences 45 us with one CTA each, 34 with four; 70 sequences 45 with one, 39 with two. Where the output lies on q or k, the CTAs of
+    // a unit are a cluster; fours of them fit all SMs of a chip only in part (a processing cluster of 18 SMs holds four).
     const int sms = multiprocessors(dev), nd = (p.hidden / p.heads + 63) >> 6;
     if (sms <= 0) return BNF4_ERR_CUDA;
-    const int cs = !seq_output_apart(p) ? 1 : units * 4 <= sms && nd >= 4 ? 4 : units * 2 <= sms && nd >= 2 ? 2 : 1;
-    launch_pdl_if(p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems, efla_seq_kernel, static_cast<unsigned>(units * cs), kSeqThreads, kSqSmem, stream, p, cs);
+    const bool meet = seq_overlap(p, p.q) != SEQ_APART || seq_overlap(p, p.k) != SEQ_APART;
+    const int cs = seq_overlap(p, p.v) == SEQ_ACROSS ? 1 : units * 4 <= (meet ? sms * 7 / 8 : sms) && nd >= 4 ? 4 : units * 2 <= sms && nd >= 2 ? 2 : 1;
+    const bool early = p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems;
+    if (cs > 1 && meet) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(units * cs));
+        cfg.blockDim = dim3(kSeqThreads);
+        cfg.dynamicSmemBytes = kSqSmem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(cs);
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = early ? 2 : 1;
+        cudaLaunchKernelEx(&cfg, efla_seq_kernel, p, cs, 1);  // errors surface in check_launch
+    } else {
+        launch_pdl_if(early, efla_seq_kernel, static_cast<unsigned>(units * cs), kSeqThreads, kSqSmem, stream, p, cs, 0);
+    }
     return check_launch("efla_seq_kernel");
 }
 

@@ -1,5 +1,5 @@
 """A sequence's outputs are the same bits in whatever company it is scanned: members of a population are compared with one another, on one rank
-or several, in full waves and partial ones, so no choice of kernel, slices or clusters may show."""
+or several, in full waves and partial ones, so no choice of kernel, slices or CTAs may show."""
 import numpy as np
 import pytest
 
@@ -24,11 +24,34 @@ def test_per_token_kernel(H, hidden, heads, method):
     bits_of_groups(H, hidden, heads, 48, 5, method, 1, [(0, 1), (3, 8), (17, 19)])
 
 
-# clusters of four, two and one CTA per (sequence, head), for every number of 16-token blocks
+# four, two and one CTA per (sequence, head), for every number of 16-token blocks
 @pytest.mark.parametrize("hidden,heads,seqs,groups", [(512, 1, 160, [(0, 1), (5, 30), (40, 60)]), (320, 2, 90, [(3, 2), (10, 35)]), (96, 1, 160, [(7, 3)])])
 @pytest.mark.parametrize("T", [1, 16, 17, 40, 64, 77, 96, 100, 128])
 def test_closed_form(H, hidden, heads, seqs, groups, T):
     bits_of_groups(H, hidden, heads, seqs, T, T % 2, 0, groups)
+
+
+@pytest.mark.parametrize("where", [0, 1, 2, 3])  # on q, k, v, or in a fourth part of the same rows
+@pytest.mark.parametrize("hidden,heads,seqs,T", [(512, 1, 3, 128), (512, 1, 30, 100), (512, 1, 70, 33), (320, 2, 20, 77), (96, 1, 160, 128)])
+def test_closed_form_in_place(H, hidden, heads, seqs, T, where):
+    """Four, two and one CTA per unit, with an output that lies where they still read, for both layouts of q, k and v."""
+    import torch
+    rng = np.random.default_rng(hidden + T)
+    x = torch.from_numpy((rng.standard_normal((seqs * T, 4 * hidden)) * 0.3).astype(np.float32)).cuda()
+    beta = torch.from_numpy(rng.standard_normal(seqs * T).astype(np.float32)).cuda()
+
+    def scan(q, k, v, ld, out, ld_out):
+        H.efla_scan(state=None, state_fp16=1, q=q, k=k, v=v, beta_raw=beta, ld_qkv=ld, ld_beta=1, beta_bias=-2.0, seqs_per_bias=1, hidden=hidden, heads=heads,
+                    seqs=seqs, T=T, method=1, eps=1e-6, out=out, ld_out=ld_out, variant=0)
+        assert H.device_error() == 0
+        return out[:, :hidden].clone()
+
+    apart = scan(x, x[:, hidden:], x[:, 2 * hidden:], 4 * hidden, torch.empty(seqs * T, hidden, device="cuda"), hidden)
+    y = x.clone()
+    rows = scan(y, y[:, hidden:], y[:, 2 * hidden:], 4 * hidden, y[:, where * hidden:], 4 * hidden)
+    parts = [x[:, i * hidden:(i + 1) * hidden].contiguous() for i in range(4)]
+    buffers = scan(*parts[:3], hidden, parts[where], hidden)
+    assert torch.equal(rows, apart) and torch.equal(buffers, apart)
 
 
 @pytest.mark.parametrize("hidden,heads,method", [(96, 1, 1), (512, 8, 1), (128, 4, 0)])
@@ -43,7 +66,7 @@ def test_long_closed_form(H, T):
 
 
 def test_losses_of_a_population_do_not_depend_on_the_wave():
-    """Wide heads: 2, 6 and 18 members a wave take clusters of four, of two and single CTAs."""
+    """Wide heads: 2, 6 and 18 members a wave take four, two and one CTA per (sequence, head)."""
     import torch
     from bitnet_nvfp4_b200 import population, synth
     out = []
