@@ -164,8 +164,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_panel_kernel(const __grid_co
         for (int mt = mt0; mt < args.m_tiles && ok; mt += args.per, sfa_src += sfa_step) {
             int atoms_left = args.k_atoms;
             for (int ks = 0; ks < num_ks; ++ks, ++kc) {
-                if (kc >= kStages) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, empty_parity, 1));
-                else if (kc == kStages - 1) ok = __all_sync(0xffffffffu, mbar_wait(bar_sfb, 0, 6));  // the panel's scales have left this stage
+                if (kc >= kStages) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, empty_parity, 31));
+                else if (kc == kStages - 1) ok = __all_sync(0xffffffffu, mbar_wait(bar_sfb, 0, 36));  // the panel's scales have left this stage
                 if (!ok) break;
                 const uint32_t sf_bytes = static_cast<uint32_t>(min(4, atoms_left)) * 512u;
                 atoms_left -= 4;
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_panel_kernel(const __grid_co
         const uint64_t sfbdesc0 = smem_desc(smem_base + kSmemSfb, 0, 128, kLayoutNone);
         const uint32_t idesc = kIdescM128 | (static_cast<uint32_t>((width + 15) / 16 * 2) << 17);
         constexpr uint32_t idesc_tail = kIdescM128 | (static_cast<uint32_t>(kTailRows >> 3) << 17);
-        bool ok = __all_sync(0xffffffffu, mbar_wait(bar_panel, 0, 2));
+        bool ok = __all_sync(0xffffffffu, mbar_wait(bar_panel, 0, 32));
         tc_fence_after();
         if (ok && elect_one()) {
             for (int j = 0; j < args.k_atoms; ++j) {
@@ -205,20 +205,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_panel_kernel(const __grid_co
         for (int mt = mt0; mt < args.m_tiles && ok; mt += args.per, odd ^= 1u) {
             for (uint32_t b = odd; b <= odd + (two ? 1u : 0u) && ok; ++b) {  // the epilogue has drained the blocks
                 if ((used >> b) & 1u) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty + 8 * b, (empty_par >> b) & 1u, 4));
+                    ok = __all_sync(0xffffffffu, mbar_wait(bar_acc_empty + 8 * b, (empty_par >> b) & 1u, 34));
                     empty_par ^= 1u << b;
                 }
                 used |= 1u << b;
             }
             if (tail && ok) {
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_tail_empty, tail_par, 4));  // (parity 1 first: passes at once)
+                ok = __all_sync(0xffffffffu, mbar_wait(bar_tail_empty, tail_par, 35));  // (parity 1 first: passes at once)
                 tail_par ^= 1u;
             }
             if (!ok) break;
             tc_fence_after();
             const uint32_t acc = tmem_base + odd * 128;
             for (int ks = 0; ks < num_ks; ++ks) {
-                ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * s, full_parity, 2));
+                ok = __all_sync(0xffffffffu, mbar_wait(bar_full + 8 * s, full_parity, 37));
                 if (!ok) break;
                 tc_fence_after();
                 const int nk = min(4, args.k_atoms - 4 * ks);
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_panel_kernel(const __grid_co
             }
             const float lsign = (member & 1) ? -p.lora_scale : p.lora_scale;
 
-            ok = __all_sync(0xffffffffu, mbar_wait(bar_tile + 8 * odd, (tile_par >> odd) & 1u, 3));
+            ok = __all_sync(0xffffffffu, mbar_wait(bar_tile + 8 * odd, (tile_par >> odd) & 1u, 33));
             if (!ok) break;
             tile_par ^= 1u << odd;
             tc_fence_after();

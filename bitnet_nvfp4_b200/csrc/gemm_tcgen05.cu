@@ -1190,7 +1190,7 @@ int gemm_nvfp4_device_error(cudaStream_t stream, int* out_code) {
         if (code == 0) code = one;
     }
     if (out_code) *out_code = code;
-    if (code != 0) return set_error(BNF4_ERR_DEVICE, "a bounded wait expired in a kernel (role code %d)", code);
+    if (code != 0) return set_error(BNF4_ERR_DEVICE, "a bounded wait expired in a kernel (code %d: up to 9 block-scaled GEMM, 11 to 20 scan on halves, 21 to 29 scan of wide heads, 31 to 39 panel GEMM)", code);
     return BNF4_OK;
 }
 

@@ -11,7 +11,9 @@ namespace bnf4 {
 
 constexpr long long kWaitCycles = 2000000000LL;  // ~1 s bound on every mbarrier wait
 
-static __device__ int g_wait_error = 0;  // code of the first wait that expired in a kernel of this translation unit
+// Code of the first wait that expired in a kernel of this translation unit. Each has its own: up to 9 gemm_tcgen05.cu, 11 to 20 efla_tc.cu, 21 to 29
+// efla_seq.cu, 31 to 39 gemm_panel.cu.
+static __device__ int g_wait_error = 0;
 // Reads and clears it. Called once the stream's kernels have finished.
 static inline int take_wait_error(int* code) {
     int rc = check_cuda(cudaMemcpyFromSymbol(code, g_wait_error, sizeof(int)), "cudaMemcpyFromSymbol(g_wait_error)");

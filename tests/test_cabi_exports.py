@@ -97,3 +97,13 @@ def test_reference_driver_links_against_the_library():
     import oracle_lib as orc
     assert lib.ref_mix(1, 2) == orc.mix(1, 2)
     assert hasattr(lib, "ref_train")
+
+
+def test_wait_codes_name_their_kernel():
+    """The error word of an expired wait says whose it is: no two translation units share a code."""
+    codes = {}
+    for src in sorted((ROOT / "bitnet_nvfp4_b200" / "csrc").glob("*.cu")):
+        for c in re.findall(r"mbar_wait\([^;]*?, (\d+)\)", src.read_text()):
+            codes.setdefault(int(c), set()).add(src.name)
+    assert set.union(*codes.values()) == {"gemm_tcgen05.cu", "gemm_panel.cu", "efla_tc.cu", "efla_seq.cu"}
+    assert all(len(users) == 1 for users in codes.values()), codes
