@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kThreads, 2) efla_tc_kernel(const __grid_const
                     for (int j = 0; j < k; ++j) pick[j] = (lane & k) ? pick[j + k] : pick[j];
                 const float kss = __uint_as_float(pick[0]);
                 // the key's scale: the next unit's are written behind its products, which wait for every warp to have read this one's
-                const bool off = !(kss >= kKeyLow && kss < kKeyHigh) && kss > 0.0f && kss <= FLT_MAX;
+                const bool off = t < 16 * kUsed && !(kss >= kKeyLow && kss < kKeyHigh) && kss > 0.0f && kss <= FLT_MAX;  // (what lies behind the last block is no token)
                 uint32_t far = __any_sync(0xffffffffu, off) ? 1u << w : 0u;  // bit c: tokens 32 c .. have another s than 1
                 float key = 1.0f;
                 if (far) {
