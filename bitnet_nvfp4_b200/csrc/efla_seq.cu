@@ -37,6 +37,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "mma_sync.cuh"
 #include "tcgen05.cuh"
 
 namespace bnf4 {
@@ -72,17 +73,6 @@ static_assert(2 * kSeqMaxT * kSqLStride * 2 <= kSqStage && kSeqMaxT * kSqXStride
 static_assert(kSqDiag % 16 == 0 && kSqInv % 16 == 0 && kSqScal % 16 == 0, "16-byte aligned regions");
 constexpr float kSqUp = 256.0f;                    // power-of-two scale of every normalised operand
 
-__device__ __forceinline__ void sq_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void sq_ldm(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void sq_ldm_trans(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
 // x0, x1 -> packed (hi, hi) and (mid, mid) halves with x = hi + mid to 22 bits
 __device__ __forceinline__ void sq_split(float x0, float x1, uint32_t& hi, uint32_t& mid) {
     const __half2 h = __floats2half2_rn(x0, x1);
@@ -180,15 +170,15 @@ __device__ __forceinline__ void seq_solve_rows(uint32_t sm0, uint32_t mat_off, u
             for (int e = 0; e < 4; ++e) s[n][e] = c[n][e] = 0.0f;
         for (int k = j + 1; k <= i; ++k) {
             uint32_t ph[4], pm[4], lh[4], lm[4];
-            sq_ldm(ph, p_addr + k * 32);
-            sq_ldm(pm, p_addr + kSqPMid + k * 32);
-            sq_ldm_trans(lh, l_addr + k * (16 * kSqLStride * 2) + j * 32);
-            sq_ldm_trans(lm, l_addr + kLMid + k * (16 * kSqLStride * 2) + j * 32);
+            ldmatrix_x4(ph, p_addr + k * 32);
+            ldmatrix_x4(pm, p_addr + kSqPMid + k * 32);
+            ldmatrix_x4_trans(lh, l_addr + k * (16 * kSqLStride * 2) + j * 32);
+            ldmatrix_x4_trans(lm, l_addr + kLMid + k * (16 * kSqLStride * 2) + j * 32);
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
-                sq_mma(s[n], ph, lh[2 * n], lh[2 * n + 1]);
-                sq_mma(c[n], ph, lm[2 * n], lm[2 * n + 1]);
-                sq_mma(c[n], pm, lh[2 * n], lh[2 * n + 1]);
+                mma_f16_16816(s[n], ph, lh[2 * n], lh[2 * n + 1]);
+                mma_f16_16816(c[n], ph, lm[2 * n], lm[2 * n + 1]);
+                mma_f16_16816(c[n], pm, lh[2 * n], lh[2 * n + 1]);
             }
         }
         // z = X_ij - sum, then P~_ij = z inv_jj
@@ -202,14 +192,14 @@ __device__ __forceinline__ void seq_solve_rows(uint32_t sm0, uint32_t mat_off, u
             sq_split(z[2], z[3], zh[2 * n + 1], zm[2 * n + 1]);
         }
         uint32_t th[4], tm[4];
-        sq_ldm_trans(th, i_addr + j * (16 * kSqTStride * 2));
-        sq_ldm_trans(tm, i_addr + kIMid + j * (16 * kSqTStride * 2));
+        ldmatrix_x4_trans(th, i_addr + j * (16 * kSqTStride * 2));
+        ldmatrix_x4_trans(tm, i_addr + kIMid + j * (16 * kSqTStride * 2));
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
             float o[4] = {0.0f, 0.0f, 0.0f, 0.0f}, oc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            sq_mma(o, zh, th[2 * n], th[2 * n + 1]);
-            sq_mma(oc, zh, tm[2 * n], tm[2 * n + 1]);
-            sq_mma(oc, zm, th[2 * n], th[2 * n + 1]);
+            mma_f16_16816(o, zh, th[2 * n], th[2 * n + 1]);
+            mma_f16_16816(oc, zh, tm[2 * n], tm[2 * n + 1]);
+            mma_f16_16816(oc, zm, th[2 * n], th[2 * n + 1]);
             const int c0 = j * 16 + n * 8 + 2 * tq;
 #pragma unroll
             for (int hr = 0; hr < 2; ++hr) {
@@ -224,14 +214,6 @@ __device__ __forceinline__ void seq_solve_rows(uint32_t sm0, uint32_t mat_off, u
     }
 }
 
-__device__ __forceinline__ void sq_umma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 __device__ __forceinline__ void sq_tmem_ld16(uint32_t taddr, float (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -388,12 +370,12 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
             for (int kk = 0; kk < nk; ++kk) {  // hi hi + hi mid + mid hi
                 const uint64_t o = static_cast<uint64_t>(2 * kk);
                 const uint32_t more = db > 0 || kk > 0 ? 1u : 0u;
-                sq_umma(tmem, kh + o, kh + o, gram, more);
-                sq_umma(tmem + 128, qh + o, kh + o, gram, more);
-                sq_umma(tmem, kh + o, km + o, gram, 1u);
-                sq_umma(tmem + 128, qh + o, km + o, gram, 1u);
-                sq_umma(tmem, km + o, kh + o, gram, 1u);
-                sq_umma(tmem + 128, qm + o, kh + o, gram, 1u);
+                tc_mma_f16(tmem, kh + o, kh + o, gram, more);
+                tc_mma_f16(tmem + 128, qh + o, kh + o, gram, more);
+                tc_mma_f16(tmem, kh + o, km + o, gram, 1u);
+                tc_mma_f16(tmem + 128, qh + o, km + o, gram, 1u);
+                tc_mma_f16(tmem, km + o, kh + o, gram, 1u);
+                tc_mma_f16(tmem + 128, qm + o, kh + o, gram, 1u);
             }
             tc_commit(bar0 + 8 * buf);
         }
@@ -590,9 +572,9 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
             const uint32_t d = tmem + (l & 1) * 64;
             for (int kk = 0; kk < nb; ++kk) {  // sixteen tokens: 32 bytes of a row of P~, 16 rows of V
                 const uint64_t a = static_cast<uint64_t>((kk >> 2) * (kSqUTile >> 4) + (kk & 3) * 2), b = static_cast<uint64_t>(kk * (2048 >> 4));
-                sq_umma(d, ph + a, vh + b, kSqIdescY, kk > 0 ? 1u : 0u);
-                sq_umma(d, ph + a, vm + b, kSqIdescY, 1u);
-                sq_umma(d, pm + a, vh + b, kSqIdescY, 1u);
+                tc_mma_f16(d, ph + a, vh + b, kSqIdescY, kk > 0 ? 1u : 0u);
+                tc_mma_f16(d, ph + a, vm + b, kSqIdescY, 1u);
+                tc_mma_f16(d, pm + a, vh + b, kSqIdescY, 1u);
             }
             tc_commit(bar0 + 16 + 8 * (l & 1));
         }
@@ -750,16 +732,16 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
                 const int nk = min(4, (hd - db * 64) >> 4);
                 for (int kk = 0; kk < nk; ++kk) {
                     uint32_t ah[4], am[4];
-                    sq_ldm(ah, aa + kk * 32);
-                    sq_ldm(am, aa + kSqTile + kk * 32);
+                    ldmatrix_x4(ah, aa + kk * 32);
+                    ldmatrix_x4(am, aa + kSqTile + kk * 32);
 #pragma unroll
                     for (int n = 0; n < 8; n += 2) {
                         uint32_t b[4], c[4];
-                        sq_ldm(b, ba + kk * 32 + n * (8 * kSqStride * 2));
-                        sq_ldm(c, ba + kk * 32 + (n + 1) * (8 * kSqStride * 2));
-                        sq_mma(acc[n], ah, b[0], b[1]); sq_mma(acc[n + 1], ah, c[0], c[1]);
-                        sq_mma(acc[n], ah, b[2], b[3]); sq_mma(acc[n + 1], ah, c[2], c[3]);
-                        sq_mma(acc[n], am, b[0], b[1]); sq_mma(acc[n + 1], am, c[0], c[1]);
+                        ldmatrix_x4(b, ba + kk * 32 + n * (8 * kSqStride * 2));
+                        ldmatrix_x4(c, ba + kk * 32 + (n + 1) * (8 * kSqStride * 2));
+                        mma_f16_16816(acc[n], ah, b[0], b[1]); mma_f16_16816(acc[n + 1], ah, c[0], c[1]);
+                        mma_f16_16816(acc[n], ah, b[2], b[3]); mma_f16_16816(acc[n + 1], ah, c[2], c[3]);
+                        mma_f16_16816(acc[n], am, b[0], b[1]); mma_f16_16816(acc[n + 1], am, c[0], c[1]);
                     }
                 }
             }
@@ -846,19 +828,19 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
             const int last = lower ? wr : 7;
             for (int j = 0; j <= last; ++j) {
                 uint32_t ah[4], am[4];
-                sq_ldm(ah, pa + j * 32);
-                sq_ldm(am, pa + kSqPMid + j * 32);
+                ldmatrix_x4(ah, pa + j * 32);
+                ldmatrix_x4(am, pa + kSqPMid + j * 32);
 #pragma unroll
                 for (int np = 0; np < 2; ++np) {
                     uint32_t vh[4], vm[4];
-                    sq_ldm_trans(vh, vb + j * (16 * kSqStride * 2) + np * 32);
-                    sq_ldm_trans(vm, vb + kSqTile + j * (16 * kSqStride * 2) + np * 32);
+                    ldmatrix_x4_trans(vh, vb + j * (16 * kSqStride * 2) + np * 32);
+                    ldmatrix_x4_trans(vm, vb + kSqTile + j * (16 * kSqStride * 2) + np * 32);
 #pragma unroll
-                    for (int n = 0; n < 2; ++n) sq_mma(y[2 * np + n], ah, vh[2 * n], vh[2 * n + 1]);
+                    for (int n = 0; n < 2; ++n) mma_f16_16816(y[2 * np + n], ah, vh[2 * n], vh[2 * n + 1]);
 #pragma unroll
-                    for (int n = 0; n < 2; ++n) sq_mma(y[2 * np + n], ah, vm[2 * n], vm[2 * n + 1]);
+                    for (int n = 0; n < 2; ++n) mma_f16_16816(y[2 * np + n], ah, vm[2 * n], vm[2 * n + 1]);
 #pragma unroll
-                    for (int n = 0; n < 2; ++n) sq_mma(y[2 * np + n], am, vh[2 * n], vh[2 * n + 1]);
+                    for (int n = 0; n < 2; ++n) mma_f16_16816(y[2 * np + n], am, vh[2 * n], vh[2 * n + 1]);
                 }
             }
             const float ds = 1.0f / kSqUp / vs;
