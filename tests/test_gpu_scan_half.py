@@ -59,8 +59,7 @@ def test_closed_form(H, T, heads, seqs, scale):
     ref = exact(qkv, beta, heads, seqs, T)
     closed, chunked = (float((run(H, qkv, beta, heads, seqs, T, v).double() - ref).norm() / ref.norm()) for v in (0, 3))
     assert closed <= 6e-4
-    if seqs * heads * T > 2000:
-        assert closed <= 1.03 * chunked
+    assert closed <= (1.03 if seqs * heads * T > 2000 else 1.1) * chunked  # (fewer rows: a tenth for the norms' sampling error)
 
 
 @pytest.mark.parametrize("T", [48, 64, 100, 128])
@@ -91,6 +90,20 @@ def test_a_sequence_does_not_depend_on_its_tile(H, T):
         got = run(H, far.reshape(6 * T, -1), beta, 2, 6, T).reshape(6, T, 128)
         assert not torch.equal(got[s], clean[s])
         assert all(torch.equal(got[i], clean[i]) for i in range(6) if i != s)
+
+
+@pytest.mark.parametrize("where", [0, 1, 2])
+@pytest.mark.parametrize("T", [33, 64, 72, 128])
+def test_in_place(H, T, where):
+    """An output that lies on q, k or v, for tiles of one and of two sequences."""
+    import torch
+    qkv, beta = inputs(T, 3, 400, 0.3)
+    apart = run(H, qkv, beta, 3, 400, T)
+    x = qkv.clone()
+    out = x[:, where * 192:]
+    H.efla_scan(state=None, state_fp16=1, q=x, k=x[:, 192:], v=x[:, 384:], beta_raw=beta, ld_qkv=x.shape[1], ld_beta=1, beta_bias=-2.0, seqs_per_bias=1, hidden=192,
+                heads=3, seqs=400, T=T, method=1, eps=1e-6, out=out, ld_out=x.shape[1], variant=0, qkv_f16=1, out_f16=1)
+    assert H.device_error() == 0 and torch.equal(out[:, :192], apart)
 
 
 @pytest.mark.parametrize("T", [33, 64, 100, 128])
