@@ -225,10 +225,10 @@ def run_kernel(args):
     peaks, src = load_peaks()
     out = {"kernel": args.kernel, "peak_source": src}
     if args.kernel == "efla":
-        T, hidden, heads, fc = 128, 512, 8, 1568
+        T, hidden, heads, fc = 128, 512, args.heads, 1568
         seqs = args.seqs
         bb = torch.full((seqs // 32 + 1,), -2.0, device="cuda")
-        if args.half:   # q | k | v and the output as IEEE halves, beta_raw fp32: what the batched driver feeds the chunked kernel
+        if args.half:   # q | k | v and the output as IEEE halves, beta_raw fp32: what the batched driver feeds its scans
             qkv = (torch.randn(seqs * T, 3 * hidden, device="cuda") * 0.3).half()
             beta = torch.randn(seqs * T, device="cuda")
             y = torch.empty(seqs * T, hidden, device="cuda", dtype=torch.float16)
@@ -246,7 +246,7 @@ def run_kernel(args):
 
         ms = _event_ms(run, args.iters)
         gbs = seqs * T * row_bytes / ms / 1e6
-        out.update(case=f"seqs={seqs} T={T} heads={heads}x64 variant={args.variant} half_io={int(args.half)}", ms=ms, achieved=gbs, unit="GB/s",
+        out.update(case=f"seqs={seqs} T={T} heads={heads}x{hidden // heads} variant={args.variant} half_io={int(args.half)}", ms=ms, achieved=gbs, unit="GB/s",
                    frac=gbs / peaks["hbm_gbs"], algorithmic_bytes=seqs * T * row_bytes)
     elif args.kernel == "gemm":
         m, n, k, R = args.m, args.n, args.k, 4096
@@ -330,6 +330,7 @@ def main():
     ap.add_argument("--kernel", choices=["efla", "gemm", "rowquant"], help="time one kernel on a small case instead of the ES step")
     ap.add_argument("--iters", type=int, default=5)
     ap.add_argument("--seqs", type=int, default=512, help="--kernel efla: sequences")
+    ap.add_argument("--heads", type=int, default=8, help="--kernel efla: heads of the 512 columns")
     ap.add_argument("--variant", type=int, default=0, help="--kernel efla: 0 library default, 2 per-token, 3 chunked")
     ap.add_argument("--m", type=int, default=65536)
     ap.add_argument("--n", type=int, default=512)
