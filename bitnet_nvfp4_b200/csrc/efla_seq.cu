@@ -17,7 +17,7 @@
 // makes the state NaN, the sequence is cut off (as if it ended there) and the rows behind it are NaN; a v that is no number is taken out
 // and its column is NaN from its token on; in q it only meets its own row.
 //
-// One CTA of 16 warps per (sequence, head):
+// One CTA of 16 warps per (sequence, head), two or four where units leave SMs idle (each does steps 1 to 4 and a share of step 5):
 //   1. norms of q and k and the per-token scalars (one warp per two rows at a time),
 //   2. G and X = Q^ K^^T over 64-column blocks of K and Q (fp32 -> two halves -> operand tiles, double-buffered): six tcgen05 products of 128 x 128 per
 //      16 columns accumulate in tensor memory while the next block is converted and the one after it is on its way,
@@ -26,7 +26,7 @@
 //   5. y = P~ V over 64-column tiles of V (tcgen05, V's columns contiguous); a tile leaves while the next one's product runs.
 // No sum depends on which units share a launch.
 // What bounds it: trips through registers and shared memory between block-wide barriers (conversions of 64 columns at a time; one CTA per SM); the input and output
-// of a unit of 128 x 512 alone take 45 k cycles of an SM's share of DRAM. 1024 sequences of 128 tokens, one head of 512: 0.43 ms (0.56 with the products of steps
+// of a unit of 128 x 512 alone take 45 k cycles of an SM's share of DRAM. 1024 sequences of 128 tokens, one head of 512: 0.434 ms (0.56 with the products of steps
 // 2 and 5 on mma.sync, 17.6 token by token); 32 sequences 34 us, of 16 tokens 19 (40 and 22 with mma.sync and clusters of four that split rows). Two rows at a time
 // in step 1, and loads two blocks ahead in steps 2 and 5, are 450 -> 430 us of it.
 

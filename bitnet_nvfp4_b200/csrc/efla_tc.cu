@@ -6,8 +6,8 @@
 // (reference recurrence: src/efla_lm_kernels.cu:590-726). The two 128 x 128 x 64 products are one tcgen05 tile each; what is left for mma.sync
 // is the blocked forward substitution and Y = P U, 36 blocks of 16 x 16 each. The kernel that carries the 64 x 64 state from chunk to chunk
 // of 16 tokens is bound by the latency of a chunk's chain (4700 cycles, eight of them); here the chain between blocks is two products. 4 to 32 sequences of
-// 8 heads x 128 tokens 13.4 -> 6.4 and 13.8 -> 8.8 us, 8192 sequences 1.05 to 1.2 -> 0.93 ms (75 % of the shared-memory wavefronts: four warps each read all
-// blocks; mma.sync pipe 50 %), 4096 x 64 tokens 280 -> 196 us. Nothing is rounded to fp16 between chunks: the operands of the block products (a G, T - I, a V, U, P)
+// 8 heads x 128 tokens 13.4 -> 6.4 and 13.8 -> 8.8 us, 8192 sequences 1.05 to 1.2 -> 0.93 ms (69 % of the shared-memory wavefronts: four warps each read all
+// blocks; tensor pipe 44 %), 4096 x 64 tokens 280 -> 196 us. Nothing is rounded to fp16 between chunks: the operands of the block products (a G, T - I, a V, U, P)
 // are halves and all sums are fp32, so the result is nearer to the recurrence in float64 (relative error at 128 tokens 4.3e-4 instead of 5.0e-4).
 //
 // Keys far from unit length would leave the halves' range: a G and P grow with the ratio of two keys' lengths, U falls with its key's square. Where |k_s|

@@ -1110,7 +1110,7 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     const bool gelu = p.epilogue == EPI_GELU_FP4 || p.epilogue == EPI_GELU_I8;
     const bool gelu_plain = !gelu || (p.act_scale <= 700.0f && (p.n % 32) == 0 && (p.epilogue == EPI_GELU_FP4 ? (p.next_nvec == 1 && p.d_i8 == nullptr) : p.next_nvec <= 1));
     const int rk = p.rank == 4 && (p.rows_per_member % 16) == 0 ? 4 : ((p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1)) ? 1 : (p.rank > 0 ? 2 : 0));
-    // CTA pairs pay where the mainloop is longer than the epilogue. Measured at 65536 x 512 (us, single
+    // CTA pairs pay where the mainloop is longer than the epilogue. Measured at 65536 x 512, before the pairs' copies moved to their K steps (us, single
     // CTAs -> pairs): fp32 / half / residual epilogues, rank 1: K 512 33.9 -> 35.9, 25.6 -> 27.0, 29.0 -> 29.8; K 1024 42.7 -> 38.2,
     // 33.1 -> 30.2, 36.1 -> 33.1; K 4096 107 -> 80, 96 -> 70, 98 -> 74. Rank 4 with the last two: K 1024 37.2 -> 39.2, 43.3 -> 45.4, K 1536
     // 46.8 -> 43.3, 49.5 -> 47.4. GELU epilogues, whose math takes as long as K 1536: K 1536 52.7 -> 54.6, K 2048 63.8 -> 59.9, K 4096 105 -> 82.
@@ -1118,8 +1118,9 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     const int pair_k = gelu ? 2048 : (p.rank > 1 && p.epilogue != EPI_F32 ? 1536 : 1024);
     // Those are figures of many waves. In a few, whole waves of the larger tiles and the drain of their two epilogues decide: 10218 x 384 x 2240 took
     // 15.1 us with single CTAs and 25.0 with pairs, 7668 x 576 x 2880 21.7 and 26.6. So the two are compared by what they cost in waves, in us: K blocks of 256
-    // at 0.44 and 0.6, epilogues of a sub-tile at 1.3 (GELU 1.9; 60 % more with the longer rank terms), 3 for starting a pair. Over 315 shapes of 0.5
-    // to 16 k rows, 64 to 4096 columns and K 1024 to 4096 the choice costs 0.2 % on average against the better of the two (by K and one tile per pair alone 6 %).
+    // at 0.44 and 0.6, epilogues of a sub-tile at 1.3 (GELU 1.9; 60 % more with the longer rank terms), 3 for starting a pair. Over 330 shapes of 0.5
+    // to 16 k rows, 64 to 4096 columns and K 1024 to 4096 the choice costs 0.3 % on average against the better of the two and 16 % at most (GELU at K 1984, where
+    // pairs pay by now; single CTAs throughout 2.4 %, pairs 37 %).
     auto waves_us = [&](long long t, int slots, float block, float epi) {
         const float nk = block * static_cast<float>((p.k + BK - 1) / BK);
         return nk + static_cast<float>((t + slots - 1) / slots - 1) * std::max(nk, epi) + epi;

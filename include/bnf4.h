@@ -269,8 +269,8 @@ typedef struct bnf4_efla_desc {
                     tokens: the closed form of the whole sequence instead); for head widths above 32 other than 64 with no HBM state, an fp16 state, up to
                     1024 tokens (beyond 128 only if out lies apart from q, k and v) and "efla_chunked" on,
                     the closed form of the whole sequence (nothing rounded to fp16 between tokens); the generic kernel otherwise. */
-    int qkv_f16; /* 1: q, k, v are IEEE halves and ld_qkv counts halves (chunked kernel only; 16-byte aligned rows) */
-    int out_f16; /* 1: out is IEEE halves and ld_out counts halves (chunked kernel only; 16-byte aligned rows) */
+    int qkv_f16; /* 1: q, k, v are IEEE halves and ld_qkv counts halves (heads of 64, AUTO or CHUNKED; 16-byte aligned rows) */
+    int out_f16; /* 1: out is IEEE halves and ld_out counts halves (as qkv_f16; 16-byte aligned rows) */
 } bnf4_efla_desc;
 #define BNF4_EFLA_AUTO 0
 #define BNF4_EFLA_GENERIC 1   /* any head_dim up to 2048, state in registers (and in HBM between calls), per-token fp16 rounding */
