@@ -231,13 +231,20 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
-// Two values at a time with packed fp32 instructions (each half rounds like the scalar instruction, so the biased results
-// equal gelu_q8_fast's). `back` receives the rounded integers as floats. The boundary test is done on squares and as a
-// running maximum: a value is safe iff d^2 + tol < 1/4 (stricter than |d| < 1/2 - tol for the same tol = 2e-6 (1 + |x act_scale|));
-// `worst` accumulates max(d^2 + 2e-6 |x act_scale|) over the caller's group, to be compared once with kGeluSafe.
-constexpr float kGeluSafe = 0.25f - 2e-6f;
-__device__ __forceinline__ void gelu_q8_fast2(float x0, float x1, float act_scale, bool lower_clamp, float& worst, float& t0, float& t1,
-                                              float& back0, float& back1) {
+// max(|a|, |b|, c) where a NaN is the largest of all
+__device__ __forceinline__ float fmax3_abs_nan(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(c));
+    return r;
+}
+// Two values at a time with packed fp32 instructions, before the clamp: t = rounded values still biased, back = the rounded integers as floats, and
+// `worst` = the largest distance to the nearest integer so far (NaN for a value that is no number). The caller takes gelu_q8_exact where !(worst <
+// gelu_q8_safe(act_scale)), and clamps where |back| passes 127, both rare: per value that leaves 7.5 instructions and two of the special-function unit, 10 with the
+// clamp and a tolerance that grows with |x|. No value of |x| > 6 needs a tolerance: x / (1 + e^(2u)) is below half an ulp of x there (and tanhf +-1), so both
+// forms round the same product; with one for them too (2e-6 |x act_scale|) four times as many values took the slow path, enough to hold up every other tile of the
+// GEMM epilogue that calls this.
+__device__ __forceinline__ float gelu_q8_safe(float act_scale) { return 0.5f - fmaf(fabsf(act_scale), 1.2e-5f, 2e-6f); }  // 2e-6 (1 + 6 act_scale) off a boundary
+__device__ __forceinline__ void gelu_q8_fast2(float x0, float x1, float act_scale, float& worst, float& t0, float& t1, float& back0, float& back1) {
     const float kB = 2.0f * 0.7978845608028654f * 1.4426950408889634f;  // 2 c log2(e)
     const float kA = kB * 0.044715f;
     const float2 x = make_float2(x0, x1);
@@ -245,25 +252,23 @@ __device__ __forceinline__ void gelu_q8_fast2(float x0, float x1, float act_scal
     float e0, e1, r0, r1;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(u2.x));
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(u2.y));
-    const float2 ep = __fadd2_rn(make_float2(e0, e1), make_float2(1.0f, 1.0f));
+    const float2 ep = __ffma2_rn(make_float2(e0, e1), make_float2(-1.0f, -1.0f), make_float2(-1.0f, -1.0f));  // -(1 + e^(2u))
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(ep.x));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(ep.y));
     const float2 xs = __fmul2_rn(x, make_float2(act_scale, act_scale));
-    const float2 nxs = __fmul2_rn(x, make_float2(-act_scale, -act_scale));
-    float2 f = __ffma2_rn(nxs, make_float2(r0, r1), xs);
-    f.x = fminf(f.x, 127.0f);
-    f.y = fminf(f.y, 127.0f);
-    if (lower_clamp) {  // gelu(x) >= -0.17 |x|: only a huge act_scale can reach -127
-        f.x = fmaxf(f.x, -127.0f);
-        f.y = fmaxf(f.y, -127.0f);
-    }
+    const float2 f = __ffma2_rn(xs, make_float2(r0, r1), xs);
     const float2 t = __fadd2_rn(f, make_float2(kRoundBias, kRoundBias));
     const float2 back = __fadd2_rn(t, make_float2(-kRoundBias, -kRoundBias));
     const float2 d = __fadd2_rn(f, make_float2(-back.x, -back.y));
-    const float2 d2 = __fmul2_rn(d, d);
-    worst = fmax3(worst, fmaf(fabsf(xs.x), 2e-6f, d2.x), fmaf(fabsf(xs.y), 2e-6f, d2.y));
+    worst = fmax3_abs_nan(d.x, d.y, worst);
     t0 = t.x; t1 = t.y;
     back0 = back.x; back1 = back.y;
+}
+// the biased values of a group clamped to +-127
+template <int N>
+__device__ __forceinline__ void clamp_biased(float* tb) {
+#pragma unroll
+    for (int e = 0; e < N; ++e) tb[e] = fminf(fmaxf(tb[e], kRoundBias - 127.0f), kRoundBias + 127.0f);
 }
 __device__ __forceinline__ int gelu_q8_exact(float x, float act_scale) {
     return clip_int8(__float2int_rn(gelu_tanh(x) * act_scale));
@@ -278,6 +283,15 @@ static __device__ __noinline__ void gelu_q8_exact4(float x0, float x1, float x2,
         tb[e] = __int_as_float(q + kRoundBiasBits);
         fc[e] = static_cast<float>(q);
     }
+}
+// four values, biased and clamped; safe = gelu_q8_safe(act_scale)
+__device__ __forceinline__ void gelu_q8x4(const float (&x)[4], float act_scale, float safe, float (&tb)[4]) {
+    float worst = 0.0f, fc[4];
+    gelu_q8_fast2(x[0], x[1], act_scale, worst, tb[0], tb[1], fc[0], fc[1]);
+    gelu_q8_fast2(x[2], x[3], act_scale, worst, tb[2], tb[3], fc[2], fc[3]);
+    const float am = fmax3(fmax3(0.0f, fabsf(fc[0]), fabsf(fc[1])), fabsf(fc[2]), fabsf(fc[3]));
+    if (!(worst < safe)) gelu_q8_exact4(x[0], x[1], x[2], x[3], act_scale, tb, fc);
+    else if (am > 127.0f) clamp_biased<4>(tb);
 }
 __device__ __forceinline__ int gelu_q8(float x, float act_scale) {
     bool ok = true;
@@ -393,7 +407,7 @@ __device__ __forceinline__ void quant_block16(const int (&w)[4], float row_scale
 // ---------------------------------------------------------------------------------------------
 constexpr int kQuantLutCodeBytes = 128 * 128;
 // A compact per-block table follows the first one, meant to be copied to shared memory: for every amax one 8-byte
-// entry {fl(1 / decoded scale) as fp32 bits, scale byte}. With it the codes need no per-element look-up (e2m1x8_int below).
+// entry {1 / decoded scale as fp32 bits, scale byte}. With it the codes need no per-element look-up (e2m1x8_table below).
 constexpr int kQuantBlockTabOffset = kQuantLutCodeBytes + 128;
 constexpr int kQuantBlockTabBytes = 128 * 8;
 constexpr int kQuantLutBytes = kQuantBlockTabOffset + kQuantBlockTabBytes;
@@ -428,12 +442,7 @@ __device__ __forceinline__ void quant_block16_lut(const int (&a)[16], const uint
 // multiple of 1/4) lands on it exactly, and any other quotient is at least 2^-6 away from every boundary (n is an integer,
 // the scale has four significant bits), so the conversion instruction rounds as the division would have.
 constexpr float kCodeSnap = 3072.0f;
-__device__ __forceinline__ uint32_t e2m1x8_int(const float* n, float r) {
-    float2 q[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        q[i] = __fadd2_rn(__ffma2_rn(make_float2(n[2 * i], n[2 * i + 1]), make_float2(r, r), make_float2(kCodeSnap, kCodeSnap)),
-                          make_float2(-kCodeSnap, -kCodeSnap));
+__device__ __forceinline__ uint32_t e2m1x8_pack(const float2 (&q)[4]) {
     uint32_t out;
     asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
         "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
@@ -445,7 +454,22 @@ __device__ __forceinline__ uint32_t e2m1x8_int(const float* n, float r) {
         : "f"(q[0].x), "f"(q[0].y), "f"(q[1].x), "f"(q[1].y), "f"(q[2].x), "f"(q[2].y), "f"(q[3].x), "f"(q[3].y));
     return out;
 }
-// The same for values still biased by kRoundBias (bit pattern = kRoundBiasBits + n).
+__device__ __forceinline__ uint32_t e2m1x8_int(const float* n, float r) {
+    float2 q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        q[i] = __fadd2_rn(__ffma2_rn(make_float2(n[2 * i], n[2 * i + 1]), make_float2(r, r), make_float2(kCodeSnap, kCodeSnap)),
+                          make_float2(-kCodeSnap, -kCodeSnap));
+    return e2m1x8_pack(q);
+}
+// The same under the reciprocal of the table of get_quant_lut(), which is chosen so that the plain product n * r converts as the quotient does, for
+// values still biased by kRoundBias (bit pattern = kRoundBiasBits + n) or already integers.
+__device__ __forceinline__ uint32_t e2m1x8_table(const float* n, float r) {
+    float2 q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = __fmul2_rn(make_float2(n[2 * i], n[2 * i + 1]), make_float2(r, r));
+    return e2m1x8_pack(q);
+}
 __device__ __forceinline__ uint32_t e2m1x8_biased(const float* tb, float r) {
     float n[8];
 #pragma unroll
@@ -454,7 +478,7 @@ __device__ __forceinline__ uint32_t e2m1x8_biased(const float* tb, float r) {
         n[i] = u.x;
         n[i + 1] = u.y;
     }
-    return e2m1x8_int(n, r);
+    return e2m1x8_table(n, r);
 }
 
 // Host twin of ue4m3_encode (used to build the table).

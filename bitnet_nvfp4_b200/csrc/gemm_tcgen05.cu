@@ -415,6 +415,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     __ldg(reinterpret_cast<const uint2*>(args.lut + kQuantBlockTabOffset) + ew * 32 + lane);
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
         }
+        // RK 4 with FP4 output: the vectors of the next projection, fetched a tile ahead like the factors (loads where they are used left the warps waiting: 65536 x 8192
+        // x 2048 with four of them 883 -> 878 us), and a place where the rows' sums are turned round (128-byte atomics instead of sixteen sectors each: 787 us).
+        constexpr bool R4 = RK == 4, kStageNext = R4 && EPI == EPI_GELU_FP4;
+        int4* next_sh = reinterpret_cast<int4*>(smem_gen + oSmemEpi + kQuantBlockTabBytes + ew * 640);  // [4][32] bytes, then [32][4] sums
         // Perturbation context of one tile: this thread's row (projections t, sign, pair) and this thread's element of the A factor
         // of the warp's first pair for the tile's columns. It is fetched one tile ahead so that the global-load latency hides
         // behind the previous tile's epilogue. A warp whose 32 rows reach into the next pair (members that are no multiple of the tile
@@ -423,6 +427,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             int member;
             int tr[4];    // raw integers: converted to float only when the tile is processed, so that nothing waits
             int aval[4];  // on these loads earlier;  aval[r] = A[pair of the warp's first row][col0 + lane][r]
+            int next_b;   // RK 4: this thread's word of the pair's vectors of the next projection: vector lane / 8, columns col0 + 4 (lane % 8) ..
         };
         const int row_in_tile = q * 32 + lane;
         // Tile coordinates advance by additions (tiles are walked in steps of gridDim.x): no division per tile.
@@ -493,10 +498,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             }
             const int first = __shfl_sync(0xffffffffu, cx.member, 0) >> 1;
             if (col0_ + lane < p.n) load_a(first, col0_ + lane, cx.aval);
+            if constexpr (kStageNext) {  // (n is a multiple of 32)
+                if (col0_ < p.n && (lane >> 3) < p.next_nvec)
+                    cx.next_b = *reinterpret_cast<const int*>(p.next_tvec + static_cast<size_t>(first) * p.next_tvec_pair_stride + static_cast<size_t>(lane >> 3) * p.n + col0_ + 4 * (lane & 7));
+            }
         };
         // The common case (rank 1, tiles inside one member) with as few instructions as possible: this phase sits on the serial
         // path of every tile.
-        constexpr bool R4 = RK == 4, R1 = RK == 1, R0 = RK == 0;
+        constexpr bool R1 = RK == 1, R0 = RK == 0;
         const bool fast_ctx = R1 || (RK == 2 && p.rank == 1 && tile_uniform_member);
         const int* t_row = !R0 && p.rank > 0 ? p.lora_t + static_cast<size_t>(row_in_tile) * p.t_stride : nullptr;
         auto fetch_fast = [&](const TileIdx& t, bool valid, LoraCtx& cx) {
@@ -554,6 +563,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         LoraCtx nxt;
         nxt.tr[1] = nxt.tr[2] = nxt.tr[3] = 0;
         nxt.aval[1] = nxt.aval[2] = nxt.aval[3] = 0;
+        nxt.next_b = 0;
         if constexpr (R0) nxt.member = 0;
         else if (R1 || fast_ctx) fetch_fast(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles, nxt);
         else fetch_ctx(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles, nxt);
@@ -588,6 +598,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
                     if (r < p.rank) loraA_sh[r * 32 + lane] = static_cast<float>(nxt.aval[r]);
+                if constexpr (kStageNext) reinterpret_cast<int*>(next_sh)[lane] = nxt.next_b;
                 __syncwarp();
                 fetch_ctx(nxt_t, more, nxt);
             }
@@ -814,11 +825,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 }
                 // One 16-element scale block at a time: its 16 values take the fast evaluation in one straight-line stretch (no
                 // branch between groups, so the scheduler interleaves them); a group with a value too close to a rounding
-                // boundary is flagged and redone with the tanhf form (about one group in a thousand). tb holds the rounded
-                // values still biased by 1.5 * 2^23: the low byte of the bit pattern is the int8.
-                const bool lower_clamp = !R1 && p.act_scale > 700.0f;  // gelu(x) >= -0.17 |x|: only a huge act_scale reaches -127 (those calls run the general instance)
+                // boundary is flagged and redone with the tanhf form (about one group in ten thousand), and a block that saturates is clamped. tb holds the
+                // rounded values still biased by 1.5 * 2^23: the low byte of the bit pattern is the int8.
+                // What bounds this: issue slots (about 20 per value, the special-function unit's 2.5 of them take it 65 % of the time). 262144 x 1024 x 512 rank 1 272 -> 249 us,
+                // 65536 x 8192 x 2048 rank 4 943 -> 787, 4096 x 1024 x 512 without a rank term 9.9 -> 7.5, with the clamp and the |x| dependent tolerance
+                // taken out of the common path and the codes' products unsnapped. One test per 8 or 16 values spills (254 -> 257, 264).
                 // entry address from the bit pattern of (amax + kRoundBias): (bits - kRoundBiasBits) * 8, folded into one constant
                 const uint32_t tab_c = smem_base + oSmemEpi - (static_cast<uint32_t>(kRoundBiasBits) << 3);
+                const float safe = gelu_q8_safe(p.act_scale);
                 int w[8];
                 uint32_t sfv[2] = {0u, 0u}, codes[4] = {0u, 0u, 0u, 0u};
                 int4 nb0 = make_int4(0, 0, 0, 0), nb1 = nb0;  // R1: the next projection's vector
@@ -826,7 +840,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 for (int blk = 0; blk < 2; ++blk) {
                     float tb[16];
                     float am = 0.0f;  // max |value| of the block
-                    uint32_t bad = 0;
                     // (requested behind the second block's math: 262144 x 1024 x 512 277.9 us with the loads where they are used, 273 in front of both
                     // blocks, 281 in front of the accumulator wait, 271 here)
                     if constexpr (R1 && EPI == EPI_GELU_FP4) {
@@ -836,15 +849,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                             nb1 = __ldg(bv + 1);
                         }
                     }
+                    float n16[16];  // R1: the integers as floats (the other instances have no registers for them: 250 instead of 201 us at 131072 x 1024 x 512 rank 4)
+                    uint32_t bad = 0;
 #pragma unroll
                     for (int g = 0; g < 4; ++g) {
-                        const int j = 16 * blk + 4 * g;
                         float worst = 0.0f;
-                        float fc[4];  // the rounded integers as floats
-                        gelu_q8_fast2(v[j], v[j + 1], p.act_scale, lower_clamp, worst, tb[4 * g], tb[4 * g + 1], fc[0], fc[1]);
-                        gelu_q8_fast2(v[j + 2], v[j + 3], p.act_scale, lower_clamp, worst, tb[4 * g + 2], tb[4 * g + 3], fc[2], fc[3]);
-                        bad |= worst < kGeluSafe ? 0u : (1u << g);
-                        am = fmax3(fmax3(am, fabsf(fc[0]), fabsf(fc[1])), fabsf(fc[2]), fabsf(fc[3]));
+#pragma unroll
+                        for (int e = 4 * g; e < 4 * g + 4; e += 2) {
+                            float fc[2];
+                            gelu_q8_fast2(v[16 * blk + e], v[16 * blk + e + 1], p.act_scale, worst, tb[e], tb[e + 1], fc[0], fc[1]);
+                            am = fmax3(am, fabsf(fc[0]), fabsf(fc[1]));
+                            n16[e] = fc[0];
+                            n16[e + 1] = fc[1];
+                        }
+                        bad |= worst < safe ? 0u : (1u << g);
                     }
                     if (bad != 0) {
 #pragma unroll
@@ -854,12 +872,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                                 float tbx[4], fcx[4];
                                 gelu_q8_exact4(v[j], v[j + 1], v[j + 2], v[j + 3], p.act_scale, tbx, fcx);
 #pragma unroll
-                                for (int e = 0; e < 4; ++e) tb[4 * g + e] = tbx[e];
+                                for (int e = 0; e < 4; ++e) {
+                                    tb[4 * g + e] = tbx[e];
+                                    n16[4 * g + e] = fcx[e];
+                                }
                             }
                         }
                         am = 0.0f;
 #pragma unroll
                         for (int e = 0; e < 16; ++e) am = fmaxf(am, fabsf(tb[e] - kRoundBias));
+                    }
+                    if (am > 127.0f) {
+                        clamp_biased<16>(tb);
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) n16[e] = tb[e] - kRoundBias;
+                        am = 127.0f;
                     }
 #pragma unroll
                     for (int g = 0; g < 4; ++g)
@@ -867,12 +894,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                                                                       __byte_perm(__float_as_uint(tb[4 * g + 2]), __float_as_uint(tb[4 * g + 3]), 0x0040), 0x5410));
                     if constexpr (EPI == EPI_GELU_FP4) {
                         // {1 / scale, scale byte} of the block from the table; the codes from the conversion instruction
-                        // applied to n / scale (e2m1x8_int)
+                        // applied to n / scale (e2m1x8_table)
                         uint32_t rbits, sbyte;
                         asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(rbits), "=r"(sbyte) : "r"((__float_as_uint(am + kRoundBias) << 3) + tab_c));
                         sfv[blk] = sbyte;
-                        codes[2 * blk] = e2m1x8_biased(tb, __uint_as_float(rbits));
-                        codes[2 * blk + 1] = e2m1x8_biased(tb + 8, __uint_as_float(rbits));
+                        codes[2 * blk] = R1 ? e2m1x8_table(n16, __uint_as_float(rbits)) : e2m1x8_biased(tb, __uint_as_float(rbits));
+                        codes[2 * blk + 1] = R1 ? e2m1x8_table(n16 + 8, __uint_as_float(rbits)) : e2m1x8_biased(tb + 8, __uint_as_float(rbits));
                     }
                 }
                 if (!(R1 && EPI == EPI_GELU_FP4) && row_ok && p.d_i8 != nullptr) {  // (the rank-1 FP4 instance writes no int8 copy)
@@ -893,7 +920,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                         const int kb = col0 >> 4;
                         *reinterpret_cast<uint16_t*>(p.d_sf + sf_offset(static_cast<int>(row), kb, sf_k_atoms(p.n))) =
                             static_cast<uint16_t>(s0 | (s1 << 8));
-                        if (R1 || p.next_nvec > 0) {  // (the rank-1 FP4 instance always feeds one projection)
+                        if (!kStageNext && (R1 || p.next_nvec > 0)) {  // (the rank-1 FP4 instance always feeds one projection)
                             const int8_t* tv = p.next_tvec + static_cast<size_t>(pair) * p.next_tvec_pair_stride + col0;
                             const int nv_ = R1 ? 1 : p.next_nvec;  // (the rank-1 instance runs with at most one projection)
                             for (int vv = 0; vv < nv_; ++vv) {
@@ -904,6 +931,34 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                                 a = __dp4a(w[4], b1.x, a); a = __dp4a(w[5], b1.y, a); a = __dp4a(w[6], b1.z, a); a = __dp4a(w[7], b1.w, a);
                                 atomicAdd(p.next_t + static_cast<size_t>(row) * p.next_nvec + vv, a);
                             }
+                        }
+                    }
+                    if constexpr (kStageNext) {  // (vectors that are not there are zeros; rows past m take part up to the store)
+                        int a4[4];
+#pragma unroll
+                        for (int vv = 0; vv < 4; ++vv) {
+                            const int4 b0 = next_sh[2 * vv], b1 = next_sh[2 * vv + 1];
+                            int a = 0;
+                            a = __dp4a(w[0], b0.x, a); a = __dp4a(w[1], b0.y, a); a = __dp4a(w[2], b0.z, a); a = __dp4a(w[3], b0.w, a);
+                            a = __dp4a(w[4], b1.x, a); a = __dp4a(w[5], b1.y, a); a = __dp4a(w[6], b1.z, a); a = __dp4a(w[7], b1.w, a);
+                            a4[vv] = a;
+                        }
+                        if (p.next_nvec == 4) {
+                            int* sums = reinterpret_cast<int*>(next_sh + 8);
+                            reinterpret_cast<int4*>(sums)[lane] = make_int4(a4[0], a4[1], a4[2], a4[3]);
+                            __syncwarp();
+                            int* t = p.next_t + (static_cast<size_t>(m0) + q * 32) * 4 + lane;
+                            if (m0 + BM <= p.m) {
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) atomicAdd(t + 32 * i, sums[32 * i + lane]);
+                            } else {
+                                for (int i = 0; i < 4; ++i)
+                                    if (m0 + q * 32 + 8 * i + (lane >> 2) < p.m) atomicAdd(t + 32 * i, sums[32 * i + lane]);
+                            }
+                        } else if (row_ok) {
+#pragma unroll
+                            for (int vv = 0; vv < 3; ++vv)
+                                if (vv < p.next_nvec) atomicAdd(p.next_t + static_cast<size_t>(row) * p.next_nvec + vv, a4[vv]);
                         }
                     }
                 }
@@ -1108,7 +1163,7 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     const int sms = multiprocessors(dev);
     if (sms <= 0) return BNF4_ERR_CUDA;
     const bool gelu = p.epilogue == EPI_GELU_FP4 || p.epilogue == EPI_GELU_I8;
-    const bool gelu_plain = !gelu || (p.act_scale <= 700.0f && (p.n % 32) == 0 && (p.epilogue == EPI_GELU_FP4 ? (p.next_nvec == 1 && p.d_i8 == nullptr) : p.next_nvec <= 1));
+    const bool gelu_plain = !gelu || ((p.n % 32) == 0 && (p.epilogue == EPI_GELU_FP4 ? (p.next_nvec == 1 && p.d_i8 == nullptr) : p.next_nvec <= 1));
     const int rk = p.rank == 4 && (p.rows_per_member % 16) == 0 ? 4 : ((p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1)) ? 1 : (p.rank > 0 ? 2 : 0));
     // CTA pairs pay where the mainloop is longer than the epilogue. Measured at 65536 x 512, before the pairs' copies moved to their K steps (us, single
     // CTAs -> pairs): fp32 / half / residual epilogues, rank 1: K 512 33.9 -> 35.9, 25.6 -> 27.0, 29.0 -> 29.8; K 1024 42.7 -> 38.2,

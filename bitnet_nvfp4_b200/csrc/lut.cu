@@ -1,5 +1,6 @@
 // Host-built lookup table of the NVFP4 block quantiser for int8 inputs (see quant_block16_lut in common.cuh).
 
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -28,7 +29,15 @@ const uint8_t* get_quant_lut() {
         if (sf == 0.0f) { sq = 0x38u; sf = 1.0f; }
         h[kQuantLutCodeBytes + amax] = static_cast<uint8_t>(sq);
         for (int a = 0; a < 128; ++a) h[amax * 128 + a] = static_cast<uint8_t>(e2m1_encode(static_cast<float>(a) / sf) & 7u);
-        const float rcp = 1.0f / sf;
+        // A quotient that lies on a rounding boundary of e2m1 must not leave it by the reciprocal's rounding: the first value from fl(1 / scale) downwards
+        // under which every |n| <= amax converts as n / scale does (fl(1 / scale) itself but for the scale 15, one ulp below for that).
+        float rcp = 1.0f / sf;
+        auto converts = [&](float r) {
+            for (int a = 0; a <= amax; ++a)
+                if (e2m1_encode(static_cast<float>(a) * r) != e2m1_encode(static_cast<float>(a) / sf)) return false;
+            return true;
+        };
+        for (int i = 0; i < 4 && !converts(rcp); ++i) rcp = nextafterf(rcp, 0.0f);
         uint32_t rcp_bits;
         memcpy(&rcp_bits, &rcp, 4);
         uint8_t* entry = h.data() + kQuantBlockTabOffset + amax * 8;

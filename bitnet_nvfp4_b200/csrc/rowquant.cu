@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(256) rowquant_kernel(const RowQuantParams p, c
 //   * bytes become floats with one byte-permute and one subtraction, and floats become bytes with a byte-permute;
 //   * rint() is an addition of M (round-to-nearest-even, like cvt.rni), clip8(rint(x)) = rint(clamp(x, +-127));
 //   * the block maximum is a float max; its bit pattern addresses a 1 KB shared-memory table of {1 / scale, scale byte},
-//     and the sixteen codes come from the conversion instruction applied to n * (1 / scale) (e2m1x8_int);
+//     and the sixteen codes come from the conversion instruction applied to n * (1 / scale) (e2m1x8_table);
 // the table is loaded once by a persistent CTA that then walks rows with a grid stride.
 // Requirements (checked by the host; otherwise rowquant_kernel runs): 16-byte aligned rows, cols_in == cols_out <= 2048.
 // ------------------------------------------------------------------------------------------------
@@ -429,6 +429,7 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
     const uint32_t tab_c = static_cast<uint32_t>(__cvta_generic_to_shared(tab_s)) - (static_cast<uint32_t>(kRoundBiasBits) << 3);
     const float M = kRoundBias;
     constexpr bool kNorm = (FE == FE_ADD_ABSMEAN || FE == FE_POS_GELU_ABSMEAN || FE == FE_ABSMEAN);
+    const float gelu_safe = gelu_q8_safe(p.act_scale);
 
     const int lane = threadIdx.x & 31;
     const int nblk = p.cols_out >> 4;
@@ -523,12 +524,8 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                 for (int q = 0; q < 4; ++q) {
                     float x[4] = {f4[q].x, f4[q].y, f4[q].z, f4[q].w};
                     if (p.act_mode == 3) {
-                        float worst = 0.0f, tb[4], fc[4];
-                        gelu_q8_fast2(x[0], x[1], p.act_scale, true, worst, tb[0], tb[1], fc[0], fc[1]);
-                        gelu_q8_fast2(x[2], x[3], p.act_scale, true, worst, tb[2], tb[3], fc[2], fc[3]);
-                        // (`worst` does not see a NaN, the sum does; a select per value cost the other modes 2 % as well)
-                        const float any_nan = (x[0] + x[1]) + (x[2] + x[3]);
-                        if (!(worst < kGeluSafe) || any_nan != any_nan) gelu_q8_exact4(x[0], x[1], x[2], x[3], p.act_scale, tb, fc);
+                        float tb[4];
+                        gelu_q8x4(x, p.act_scale, gelu_safe, tb);
 #pragma unroll
                         for (int j = 0; j < 4; ++j) vf[i][4 * q + j] = tb[j] - M;
                     } else {
@@ -621,16 +618,10 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
 #pragma unroll
                         for (int j = 0; j < 4; ++j) pv[j] = fmaf(ns, pnf[j], pv[j]);
                     }
-                    float x[4], tb[4], fc[4];
+                    float x[4], tb[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) x[j] = ff[j] + pv[j];
-                    float worst = 0.0f;  // packed evaluation, two values per call; one boundary test per four
-                    gelu_q8_fast2(x[0], x[1], p.act_scale, true, worst, tb[0], tb[1], fc[0], fc[1]);
-                    gelu_q8_fast2(x[2], x[3], p.act_scale, true, worst, tb[2], tb[3], fc[2], fc[3]);
-                    if (!(worst < kGeluSafe)) {
-                        float fcx[4];
-                        gelu_q8_exact4(x[0], x[1], x[2], x[3], p.act_scale, tb, fcx);
-                    }
+                    gelu_q8x4(x, p.act_scale, gelu_safe, tb);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) vf[i][4 * q + j] = tb[j] - M;
                     resid[q] = biased4_to_bytes(tb[0], tb[1], tb[2], tb[3]);
@@ -735,8 +726,8 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                     lo = e2m1x8_biased(tq, rs);
                     hi = e2m1x8_biased(tq + 8, rs);
                 } else {  // the values are integers already
-                    lo = e2m1x8_int(vf[i], rs);
-                    hi = e2m1x8_int(vf[i] + 8, rs);
+                    lo = e2m1x8_table(vf[i], rs);
+                    hi = e2m1x8_table(vf[i] + 8, rs);
                 }
                 *reinterpret_cast<uint2*>(p.out_codes + (static_cast<size_t>(row) * p.cols_out + k0) / 2) = make_uint2(lo, hi);
             }
