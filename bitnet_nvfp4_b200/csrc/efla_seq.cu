@@ -17,18 +17,19 @@
 // makes the state NaN, the sequence is cut off (as if it ended there) and the rows behind it are NaN; a v that is no number is taken out
 // and its column is NaN from its token on; in q it only meets its own row.
 //
-// One CTA of 16 warps per (sequence, head), two or four where units leave SMs idle (each does steps 1 to 4 and a share of step 5):
-//   1. norms of q and k and the per-token scalars (one warp per two rows at a time),
-//   2. G and X = Q^ K^^T over 64-column blocks of K and Q (fp32 -> two halves -> operand tiles, double-buffered): six tcgen05 products of 128 x 128 per
-//      16 columns accumulate in tensor memory while the next block is converted and the one after it is on its way,
+// One CTA per (sequence, head), two or four where units leave SMs idle (each does steps 1 to 4 and a share of step 5); sixteen warps that work, one that issues the
+// products, one that loads:
+//   1. G and X = Q^ K^^T over 32-column blocks of K and Q: TMA into four slots, two groups of eight warps convert blocks in turn (fp32 -> two halves, rows scaled by powers of
+//      two, squared norms on the way), six tcgen05 products of 128 x 128 per 16 columns accumulate in tensor memory, where the left operands lie too,
+//   2. the per-token scalars; 1 / |q| and 1 / |k| reach G and X when they are read,
 //   3. L and X into shared memory, inverses of the 16 x 16 diagonal blocks of I + L, L = diag(a) strict(G), by forward substitution in fp32,
-//   4. P~ by block back substitution from the right with mma.sync, one warp per 16-row block (rows are independent, no barriers),
-//   5. y = P~ V over 64-column tiles of V (tcgen05, V's columns contiguous); a tile leaves while the next one's product runs.
+//   4. P~ by block back substitution from the right with mma.sync, one warp per 16-row block (rows are independent, no barriers), into tensor memory,
+//   5. y = P~ V over 64-column tiles of V (tcgen05, V's columns contiguous): eight warps convert tiles while the other eight take finished ones.
 // No sum depends on which units share a launch.
-// What bounds it: trips through registers and shared memory between block-wide barriers (conversions of 64 columns at a time; one CTA per SM); the input and output
-// of a unit of 128 x 512 alone take 45 k cycles of an SM's share of DRAM. 1024 sequences of 128 tokens, one head of 512: 0.434 ms (0.56 with the products of steps
-// 2 and 5 on mma.sync, 17.6 token by token); 32 sequences 34 us, of 16 tokens 19 (40 and 22 with mma.sync and clusters of four that split rows). Two rows at a time
-// in step 1, and loads two blocks ahead in steps 2 and 5, are 450 -> 430 us of it.
+// What bounds it: DRAM in steps 1 and 5 (29 and 26 k of 66 k cycles for a unit of 128 x 512; its input and output alone are 45 k of an SM's share), the chain of steps 3 and 4 in
+// between. 1024 sequences of 128 tokens, one head of 512: 277 us; 32 sequences 27, of 16 tokens 18. The way there from 436 us: q and k read once and not for their norms
+// first, loads that need no L1 lines (behind 200 KB of shared memory 28 KB of L1 held 60 % of the loads back) 436 -> 318; groups of eight warps instead of barriers of sixteen
+// 318 -> 305; left operands in tensor memory 305 -> 277. Prefetches of the next unit into L2 (cp.async.bulk.prefetch, 11 bytes a cycle and SM) cost more than they hide.
 
 #include <algorithm>
 #include <atomic>
@@ -46,31 +47,38 @@ namespace {
 
 constexpr int kSeqMaxT = 128;
 constexpr int kSeqThreads = 512;
+constexpr int kSqThreads = kSeqThreads + 64;       // efla_seq_kernel: sixteen warps that work, one that issues the products of steps 1 and 5, one the loads
 constexpr int kSqStride = 72;                      // halves per row of the K / Q / V blocks: conflict-free ldmatrix rows
 constexpr int kSqTile = kSeqMaxT * kSqStride * 2;  // bytes of one 128 x 64 block of halves
-constexpr int kSqStage = 4 * kSqTile;              // K hi, K mid, Q hi, Q mid
 constexpr int kSqLStride = 136;                    // halves per row of L hi / L mid
-constexpr int kSqXStride = 140;                    // floats per row of X; the row then holds P~ hi (272 bytes) and P~ mid
-constexpr int kSqPMid = 272;                       // byte offset of P~ mid inside a row
+constexpr int kSqXStride = 140;                    // floats per row of X (efla_seq_kernel), whose blocks P~'s replace; of the matrix of efla_long_kernel, P~ hi and mid
+constexpr int kSqPMid = 272;                       // byte offset of P~ mid inside a row of the latter
 constexpr int kSqTStride = 24;                     // halves per row of a diagonal block's inverse
-constexpr int kSqDiag = 2 * kSqStage;                            // fp32 diagonal blocks of L [8][16][17]
+// Shared memory of efla_seq_kernel. Step 1: K hi and K mid (64 columns, two halves of 32 in turn), behind them four slots of 32 columns of K and Q as they come
+// from memory. Steps 3 and 4: L, X, the diagonal blocks and their inverses. Step 5: V hi and mid of two tiles, a finished tile of y, the odd tiles of V as they come. The even ones,
+// the first of them from the start, have a place of their own.
+constexpr int kSqUTile = kSeqMaxT * 128;                         // an operand tile: 128 rows x 64 halves, or 32 floats, 128B swizzle
+constexpr int kSqRaw = 2 * kSqUTile;
+constexpr int kSqX = 2 * kSeqMaxT * kSqLStride * 2;
+constexpr int kSqDiag = kSqX + kSeqMaxT * kSqXStride * 4;        // fp32 diagonal blocks of L [8][16][17]
 constexpr int kSqInv = kSqDiag + 8 * 16 * 17 * 4;                // their inverses, hi and mid [2][8][16][kSqTStride]
-constexpr int kSqScal = kSqInv + 2 * 8 * 16 * kSqTStride * 2;    // q scale, k scale, a, b [4][128] floats
-constexpr int kSqRed = kSqScal + 4 * kSeqMaxT * 4;               // reduction scratch [2][16] + broadcast
-constexpr int kSqPart = kSqRed + 256;                            // squared norms of the tokens [2][128] floats
-constexpr int kSqBad = kSqPart + 2 * kSeqMaxT * 4;               // first token of each of a tile's 64 columns whose v is no number, two tiles
+constexpr int kSqOut = 4 * kSqUTile;                             // 128 rows of 64 floats
+constexpr int kSqV1 = 8 * kSqUTile, kSqV0 = 10 * kSqUTile;       // tiles of V: odd, even
+constexpr int kSqScal = 12 * kSqUTile;                           // q factor, k factor, a, b [4][128] floats (first: largest values of the first columns)
+constexpr int kSqScale = kSqScal + 4 * kSeqMaxT * 4;             // powers of two that scale the rows of q and k [2][128] floats
+constexpr int kSqRed = kSqScale + 2 * kSeqMaxT * 4;              // reduction scratch [2][8], factors of two tiles of y, bad tokens [4]
+constexpr int kSqPart = kSqRed + 256;                            // squared norms of q and k, four shares [4][2][128] floats
+constexpr int kSqBad = kSqPart + 8 * kSeqMaxT * 4;               // first token of each of a tile's 64 columns whose v is no number, two tiles
 constexpr int kSqBar = kSqBad + 2 * 64 * 4;                      // mbarriers, tensor memory slot
-constexpr int kSqOut = kSqBar + 64;                              // a finished tile of y: 128 rows of 64 floats
-constexpr int kSqSmem = kSqOut + kSeqMaxT * 64 * 4 + 1024;       // (and room to align the tiles)
-// tcgen05 operands: tiles of 128 rows x 64 halves, 128B swizzle. Step 2: K hi, K mid, Q hi, Q mid at each stage; step 5: P~ hi and mid (tokens 0-63, 64-127) in
-// stage 0, V hi and mid of two column tiles in stage 1.
-constexpr int kSqUTile = kSeqMaxT * 128;
-static_assert(4 * kSqUTile <= kSqStage && kSqStage % 1024 == 0, "operand tiles");
-constexpr int kSqTmemCols = 256;  // G | X, then two tiles of y
+constexpr int kSqSmem = kSqBar + 256 + 1024;                     // (and room to align the tiles)
+static_assert(kSqRaw + 8 * kSqUTile <= kSqV0 && kSqInv + 2 * 8 * 16 * kSqTStride * 2 <= kSqV0 && kSqSmem <= 232448, "regions");
+// Tensor memory: G | X, then two tiles of y; behind them the left operands, which reach the products from here (from shared memory their reads, 4 KB for 64 cycles
+// like the right operands', took step 1 to the limit of its bandwidth): K hi, K mid, Q hi, Q mid of two halves, then P~ hi and mid.
+constexpr int kSqTmemCols = 512;
+constexpr int kSqTA = 256;
 constexpr uint32_t kSqIdesc = (1u << 4) | (static_cast<uint32_t>(kSeqMaxT >> 4) << 24);                        // fp16 x fp16 -> fp32, M 128
 constexpr uint32_t kSqIdescY = kSqIdesc | (1u << 16) | (64u >> 3 << 17);  // N 64, B with columns contiguous
-static_assert(2 * kSeqMaxT * kSqLStride * 2 <= kSqStage && kSeqMaxT * kSqXStride * 4 <= kSqStage && 4 * kSqTile <= kSqStage, "overlaid regions");
-static_assert(kSqDiag % 16 == 0 && kSqInv % 16 == 0 && kSqScal % 16 == 0, "16-byte aligned regions");
+static_assert(kSqX % 16 == 0 && kSqDiag % 16 == 0 && kSqInv % 16 == 0 && kSqScal % 16 == 0, "16-byte aligned regions");
 constexpr float kSqUp = 256.0f;                    // power-of-two scale of every normalised operand
 
 // x0, x1 -> packed (hi, hi) and (mid, mid) halves with x = hi + mid to 22 bits
@@ -117,6 +125,13 @@ __device__ __forceinline__ float seq_infinite_norm(float kss, const float* row, 
     for (int i = lane; i < hd; i += 32) bad = bad || !(fabsf(row[i]) <= FLT_MAX);
     return __any_sync(0xffffffffu, bad) ? NAN : kss;
 }
+// (one thread)
+__device__ __forceinline__ float seq_infinite_norm(float kss, const float* row, int hd) {
+    if (kss != INFINITY) return kss;
+    for (int i = 0; i < hd; ++i)
+        if (!(fabsf(row[i]) <= FLT_MAX)) return NAN;
+    return kss;
+}
 __device__ __forceinline__ uint32_t seq_abs_bits(const float4& x) {  // ordered like the magnitudes, infinities and NaN above all numbers
     const uint32_t m = 0x7fffffffu;
     return max(max(__float_as_uint(x.x) & m, __float_as_uint(x.y) & m), max(__float_as_uint(x.z) & m, __float_as_uint(x.w) & m));
@@ -151,9 +166,11 @@ __device__ __forceinline__ void seq_invert_diagonal(const float* Ld, __half* inv
     }
 }
 
-// One warp: rows 16 i .. 16 i + 15 of P with P (I + L) = X by block columns from the right; X in registers, L (two halves) at the start of
+// One warp: rows 16 i .. 16 i + 15 of P with P (I + L) = X by block columns from the right; L (two halves) at the start of
 // shared memory, the diagonal blocks' inverses at inv_off; P (two halves, scaled by kSqUp) at mat_off (prow: the same place).
-__device__ __forceinline__ void seq_solve_rows(uint32_t sm0, uint32_t mat_off, uint8_t* prow, uint32_t inv_off, int i, int lane, const float (&xr)[8][2][4]) {
+// X comes from get_x(j, n, e). PSTEP, PMID: bytes from a block's halves to the next block's, and to its mid halves.
+template <int PSTEP, int PMID, class GetX>
+__device__ __forceinline__ void seq_solve_rows(uint32_t sm0, uint32_t mat_off, uint8_t* prow, uint32_t inv_off, int i, int lane, GetX get_x) {
     const int g = lane >> 2, tq = lane & 3;
     const uint32_t p_addr = sm0 + mat_off + static_cast<uint32_t>((i * 16 + (lane & 15)) * (kSqXStride * 4) + (lane >> 4) * 16);
     const uint32_t l_addr = sm0 + static_cast<uint32_t>(((lane >> 3 & 1) * 8 + (lane & 7)) * kSqLStride + (lane >> 4) * 8) * 2u;
@@ -170,8 +187,8 @@ __device__ __forceinline__ void seq_solve_rows(uint32_t sm0, uint32_t mat_off, u
             for (int e = 0; e < 4; ++e) s[n][e] = c[n][e] = 0.0f;
         for (int k = j + 1; k <= i; ++k) {
             uint32_t ph[4], pm[4], lh[4], lm[4];
-            ldmatrix_x4(ph, p_addr + k * 32);
-            ldmatrix_x4(pm, p_addr + kSqPMid + k * 32);
+            ldmatrix_x4(ph, p_addr + k * PSTEP);
+            ldmatrix_x4(pm, p_addr + PMID + k * PSTEP);
             ldmatrix_x4_trans(lh, l_addr + k * (16 * kSqLStride * 2) + j * 32);
             ldmatrix_x4_trans(lm, l_addr + kLMid + k * (16 * kSqLStride * 2) + j * 32);
 #pragma unroll
@@ -187,7 +204,7 @@ __device__ __forceinline__ void seq_solve_rows(uint32_t sm0, uint32_t mat_off, u
         for (int n = 0; n < 2; ++n) {
             float z[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) z[e] = (xr[j][n][e] - (s[n][e] + c[n][e]) * down) * kSqUp;
+            for (int e = 0; e < 4; ++e) z[e] = (get_x(j, n, e) - (s[n][e] + c[n][e]) * down) * kSqUp;
             sq_split(z[0], z[1], zh[2 * n], zm[2 * n]);
             sq_split(z[2], z[3], zh[2 * n + 1], zm[2 * n + 1]);
         }
@@ -200,20 +217,34 @@ __device__ __forceinline__ void seq_solve_rows(uint32_t sm0, uint32_t mat_off, u
             mma_f16_16816(o, zh, th[2 * n], th[2 * n + 1]);
             mma_f16_16816(oc, zh, tm[2 * n], tm[2 * n + 1]);
             mma_f16_16816(oc, zm, th[2 * n], th[2 * n + 1]);
-            const int c0 = j * 16 + n * 8 + 2 * tq;
+            const int c0 = j * PSTEP + (n * 8 + 2 * tq) * 2;
 #pragma unroll
             for (int hr = 0; hr < 2; ++hr) {
                 uint32_t hi, mid;
                 sq_split((o[2 * hr] + oc[2 * hr]) * (1.0f / kSqUp), (o[2 * hr + 1] + oc[2 * hr + 1]) * (1.0f / kSqUp), hi, mid);
-                uint8_t* d = prow + (i * 16 + g + 8 * hr) * (kSqXStride * 4) + c0 * 2;
+                uint8_t* d = prow + (i * 16 + g + 8 * hr) * (kSqXStride * 4) + c0;
                 *reinterpret_cast<uint32_t*>(d) = hi;
-                *reinterpret_cast<uint32_t*>(d + kSqPMid) = mid;
+                *reinterpret_cast<uint32_t*>(d + PMID) = mid;
             }
         }
         __syncwarp();
     }
 }
 
+__device__ __forceinline__ void sq_tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+                 "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void sq_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// A from tensor memory: lane = row, two halves per column
+__device__ __forceinline__ void sq_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 __device__ __forceinline__ void sq_tmem_ld16(uint32_t taddr, float (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -224,8 +255,9 @@ __device__ __forceinline__ void sq_tmem_ld16(uint32_t taddr, float (&r)[16]) {
 }
 
 // cs CTAs share a unit: each does steps 1 to 4 (the same sums) and its share of the column tiles of step 5. meet: they form a cluster, and none writes
-// before all have read q and k, where the output may lie.
-__global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaParams p, const int cs, const int meet) {
+// before all have read q and k, where the output may lie. across: it may lie on v, on other columns.
+__global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                                                                 const __grid_constant__ CUtensorMap map_v, const EflaParams p, const int cs, const int meet, const int across) {
     pdl_wait();
     extern __shared__ uint8_t sm_raw[];
     uint8_t* sm = sm_raw + ((1024u - (smem_u32(sm_raw) & 1023u)) & 1023u);
@@ -252,62 +284,214 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     float* red = reinterpret_cast<float*>(sm + kSqRed);
     int* red_bad = reinterpret_cast<int*>(red + 48);  // [4]
     float* part = reinterpret_cast<float*>(sm + kSqPart);
-    const uint32_t bar0 = sm0 + kSqBar;  // the products that read stage b (step 2) / form tile b of y (step 5) are done: two barriers each
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + kSqBar + 32);
+    // mbarriers: slots of K and Q filled / read (four each), halves of the operands complete / multiplied (two each), tiles of V filled / read (two each), operands of V
+    // complete, tiles of y complete / read (two each)
+    const uint32_t bar0 = sm0 + kSqBar, bar_raw = bar0, bar_read = bar0 + 32, bar_op = bar0 + 64, bar_mul = bar0 + 80, bar_v = bar0 + 96, bar_vread = bar0 + 112, bar_vop = bar0 + 128, bar_y = bar0 + 144,
+                   bar_drain = bar0 + 160;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + kSqBar + 192);
+    constexpr int kGroup = kSeqThreads / 64;  // warps of one of the two groups that share steps 1 and 5
     if (tid == 0) {
-        for (int b = 0; b < 4; ++b) mbar_init(bar0 + 8 * b, 1);
+        for (int b = 0; b < 4; ++b) { mbar_init(bar_raw + 8 * b, 1); mbar_init(bar_read + 8 * b, kGroup); }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(bar_op + 8 * b, kGroup);
+            mbar_init(bar_mul + 8 * b, 1);
+            mbar_init(bar_v + 8 * b, 1);
+            mbar_init(bar_vread + 8 * b, kGroup);
+            mbar_init(bar_vop + 8 * b, kGroup);
+            mbar_init(bar_y + 8 * b, 1);
+            mbar_init(bar_drain + 8 * b, kGroup);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) {
-        tmem_alloc(bar0 + 32, kSqTmemCols);
+    if (warp == 16) {
+        tmem_alloc(bar0 + 192, kSqTmemCols);
         tmem_relinquish();
     }
     bool ok = true;  // no wait of this thread has expired; behind one that has there are no others, and what the thread would write stays unwritten
 
-    // ---------------- 1. norms and scalars ----------------
-    for (int t0 = 2 * warp; t0 < kSeqMaxT; t0 += 32) {  // two rows of each at a time: twice the loads in flight (a row's trip to DRAM paced this step)
-        float ss[2][2] = {};  // [row][q, k]
-        if (t0 < T) {
-            const int other = t0 + 1 < T ? 1 : 0;
-            const float4* q4 = reinterpret_cast<const float4*>(qg + static_cast<size_t>(t0) * p.ld_qkv);
-            const float4* k4 = reinterpret_cast<const float4*>(kg + static_cast<size_t>(t0) * p.ld_qkv);
-            const int next = other * (p.ld_qkv >> 2);
-#pragma unroll 4
-            for (int i = lane; i < (hd >> 2); i += 32) {
-                const float4 x[2][2] = {{q4[i], k4[i]}, {q4[i + next], k4[i + next]}};
-#pragma unroll
-                for (int r = 0; r < 2; ++r)
-#pragma unroll
-                    for (int m = 0; m < 2; ++m) {
-                        ss[r][m] = fmaf(x[r][m].x, x[r][m].x, ss[r][m]);
-                        ss[r][m] = fmaf(x[r][m].y, x[r][m].y, ss[r][m]);
-                        ss[r][m] = fmaf(x[r][m].z, x[r][m].z, ss[r][m]);
-                        ss[r][m] = fmaf(x[r][m].w, x[r][m].w, ss[r][m]);
-                    }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int t = t0 + r;
-            const float qss = warp_sum_f(ss[r][0]);
-            float kss = warp_sum_f(ss[r][1]);
-            if (t < T) kss = seq_infinite_norm(kss, kg + static_cast<size_t>(t) * p.ld_qkv, hd, lane);
-            if (lane == 0) { part[t] = t < T ? qss : 0.0f; part[kSeqMaxT + t] = t < T ? kss : 0.0f; }
-        }
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+
+    // ---------------- 1. G and X of rows scaled by powers of two, squared norms on the way ----------------
+    // 32 columns at a time: a warp loads (TMA), two groups of eight convert them in turn (thread = sixteen columns of a row of K and of Q), one issues the products.
+    const int nh = hd >> 5, group = warp >> 3, quad = warp & 3, ch = (warp >> 2) & 1;
+    const int t_row = 32 * quad + lane;  // this thread's row, and its lane of tensor memory
+    const uint32_t t_lane = tmem + (static_cast<uint32_t>(32 * quad) << 16);
+    const int swz = t_row & 7;
+    float* scale_sh = reinterpret_cast<float*>(sm + kSqScale);
+    auto workers_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kSeqThreads) : "memory"); };
+    auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(2 + group), "n"(kSeqThreads / 2) : "memory"); };
+    const int x0 = h * hd, y0 = static_cast<int>(row0);
+    auto put_split = [&](uint8_t* at, const float4& x, float s, int mid_off) {
+        uint2 hi, mid;
+        sq_split(x.x * s, x.y * s, hi.x, mid.x);
+        sq_split(x.z * s, x.w * s, hi.y, mid.y);
+        *reinterpret_cast<uint2*>(at) = hi;
+        *reinterpret_cast<uint2*>(at + mid_off) = mid;
+    };
+    auto arrive = [&](uint32_t bar) {  // this warp's share of an operand is in shared memory
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar);
+    };
+    auto abs4 = [](const float4& x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); };
+    auto sumsq = [](float s, const float4& x) {
+        s = fmaf(x.x, x.x, s); s = fmaf(x.y, x.y, s); s = fmaf(x.z, x.z, s);
+        return fmaf(x.w, x.w, s);
+    };
+    int v_loads = 0;
+    auto load_v = [&](int l) {  // (the loading warp) the CTA's l-th tile of V: two boxes of 32 columns, or the one that is left
+        const uint32_t at = sm0 + ((l & 1) ? kSqV1 : kSqV0);
+        const int c = (ct0 + l) * 64;
+        if (elect_one()) {
+            const bool two = c + 32 < hd;
+            mbar_expect_tx(bar_v + 8 * (l & 1), (two ? 2 : 1) * kSqUTile);
+            tma_load_2d(at, &map_v, x0 + c, y0, bar_v + 8 * (l & 1));
+            if (two) tma_load_2d(at + kSqUTile, &map_v, x0 + c + 32, y0, bar_v + 8 * (l & 1));
+        }
+        __syncwarp();
+        ++v_loads;
+    };
+    // The scale of a row is taken from its first 32 columns (largest value just below 2^8), so that q and k are read once; a row that leaves the range of
+    // halves later on, or has only zeros there, sends the whole unit through a second pass with scales from whole rows.
+    auto norm2 = [&](int m, int t) { return (part[m * kSeqMaxT + t] + part[(2 + m) * kSeqMaxT + t]) + (part[(4 + m) * kSeqMaxT + t] + part[(6 + m) * kSeqMaxT + t]); };
+    int loads = 0;  // blocks of K and Q that the loading warp has asked for
+    for (int pass = 0;; ++pass) {
+        const int it0 = pass * nh;  // blocks before this pass: the barriers' phases go on
+        if (warp < 16) {
+            float ss[2] = {0.0f, 0.0f}, sc[2];  // k, q
+            for (int hb = group; hb < nh; hb += 2) {
+                const int it = it0 + hb, slot = it & 3, half = it & 1;
+                ok = ok && mbar_wait(bar_raw + 8 * slot, static_cast<uint32_t>(it >> 2) & 1u, 26);
+                const uint8_t* raw = sm + kSqRaw + slot * (2 * kSqUTile) + t_row * 128;
+                float4 x[2][4];
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        x[m][j] = t_row < T ? *reinterpret_cast<const float4*>(raw + m * kSqUTile + (((4 * ch + j) ^ swz) << 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (hb == group) {  // the scales, from the first block: the largest values of its columns 16 ch ..
+                    if (group == 0) {
+#pragma unroll
+                        for (int m = 0; m < 2; ++m) {
+                            float mx = fmaxf(fmaxf(abs4(x[m][0]), abs4(x[m][1])), fmaxf(abs4(x[m][2]), abs4(x[m][3])));
+                            if (pass > 0 && t_row < T) {
+                                const float* src = (m == 0 ? kg : qg) + static_cast<size_t>(t_row) * p.ld_qkv;
+                                for (int c = 32 + 16 * ch; c < hd; c += 32)
+                                    for (int j = 0; j < 4; ++j) mx = fmaxf(mx, abs4(*reinterpret_cast<const float4*>(src + c + 4 * j)));
+                            }
+                            qs_sh[(2 * m + ch) * kSeqMaxT + t_row] = mx;
+                        }
+                    }
+                    workers_sync();
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        sc[m] = sq_pow2_scale<8>(fmaxf(qs_sh[2 * m * kSeqMaxT + t_row], qs_sh[(2 * m + 1) * kSeqMaxT + t_row]));
+                        if (group == 0 && ch == 0) scale_sh[(1 - m) * kSeqMaxT + t_row] = sc[m];
+                    }
+                }
+                if (it >= 2) ok = ok && mbar_wait(bar_mul + 8 * half, static_cast<uint32_t>(it / 2 - 1) & 1u, 21);  // the half's last products have read it
+                __syncwarp();
+                tc_fence_after();
+                if (32 * quad < 16 * nb) {
+                    const uint32_t ta = t_lane + kSqTA + 64 * half + 8 * ch;
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        uint32_t hi[8], mid[8];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float4 y = x[m][j];
+                            ss[m] = sumsq(ss[m], y);
+                            sq_split(y.x * sc[m], y.y * sc[m], hi[2 * j], mid[2 * j]);
+                            sq_split(y.z * sc[m], y.w * sc[m], hi[2 * j + 1], mid[2 * j + 1]);
+                        }
+                        if (m == 0) {  // K is the right operand too
+                            uint8_t* row = sm + t_row * 128;
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) {
+                                const int at = ((4 * half + 2 * ch + j) ^ swz) << 4;
+                                *reinterpret_cast<uint4*>(row + at) = make_uint4(hi[4 * j], hi[4 * j + 1], hi[4 * j + 2], hi[4 * j + 3]);
+                                *reinterpret_cast<uint4*>(row + kSqUTile + at) = make_uint4(mid[4 * j], mid[4 * j + 1], mid[4 * j + 2], mid[4 * j + 3]);
+                            }
+                        }
+                        sq_tmem_st8(ta + 32 * m, hi);
+                        sq_tmem_st8(ta + 32 * m + 16, mid);
+                    }
+                    sq_tmem_st_wait();
+                }
+                tc_fence_before();
+                arrive(bar_op + 8 * half);
+                if (lane == 0) mbar_arrive(bar_read + 8 * slot);  // (behind the stores of what was read: released behind the loads alone, the slot was filled again under them)
+            }
+            part[((2 * group + ch) * 2 + 1) * kSeqMaxT + t_row] = ss[0];
+            part[(2 * group + ch) * 2 * kSeqMaxT + t_row] = ss[1];
+        } else if (warp == 16) {
+            // The products have a warp of their own: their issue waits for the tensor pipe (64 cycles each, 12 to a block), which held up the conversions
+            // of the warp that did both, and with it every barrier.
+            const uint64_t kh = smem_desc(sm0, 16, 1024, kLayoutSw128), km = smem_desc(sm0 + kSqUTile, 16, 1024, kLayoutSw128);
+            const uint32_t gram = kSqIdesc | (static_cast<uint32_t>(2 * nb) << 17);  // N 16 nb
+            for (int hb = 0; hb < nh; ++hb) {
+                const int it = it0 + hb, half = it & 1;
+                ok = ok && mbar_wait(bar_op + 8 * half, static_cast<uint32_t>(it / 2) & 1u, 24);
+                if (elect_one() && ok) {
+                    tc_fence_after();
+#pragma unroll
+                    for (int kk = 0; kk < 2; ++kk) {  // hi hi + hi mid + mid hi
+                        const uint64_t o = static_cast<uint64_t>(4 * half + 2 * kk);
+                        const uint32_t ta = tmem + kSqTA + 64 * half + 8 * kk, more = hb > 0 || kk > 0 ? 1u : 0u;
+                        sq_mma_ts(tmem, ta, kh + o, gram, more);
+                        sq_mma_ts(tmem + 128, ta + 32, kh + o, gram, more);
+                        sq_mma_ts(tmem, ta, km + o, gram, 1u);
+                        sq_mma_ts(tmem + 128, ta + 32, km + o, gram, 1u);
+                        sq_mma_ts(tmem, ta + 16, kh + o, gram, 1u);
+                        sq_mma_ts(tmem + 128, ta + 48, kh + o, gram, 1u);
+                    }
+                    tc_commit(bar_mul + 8 * half);
+                }
+                __syncwarp();
+            }
+        } else {
+            for (int hb = 0; hb < nh; ++hb) {
+                const int it = it0 + hb, slot = it & 3;
+                if (it >= 4) ok = ok && mbar_wait(bar_read + 8 * slot, static_cast<uint32_t>(it / 4 - 1) & 1u, 27);
+                if (!__all_sync(0xffffffffu, ok)) break;
+                if (elect_one()) {
+                    const uint32_t at = sm0 + kSqRaw + slot * (2 * kSqUTile);
+                    mbar_expect_tx(bar_raw + 8 * slot, 2 * kSqUTile);
+                    tma_load_2d(at, &map_k, x0 + 32 * hb, y0, bar_raw + 8 * slot);
+                    tma_load_2d(at + kSqUTile, &map_q, x0 + 32 * hb, y0, bar_raw + 8 * slot);
+                }
+                __syncwarp();
+                ++loads;
+                if (pass == 0 && hb == min(3, nh - 1)) load_v(0);
+            }
+        }
+        for (int it = max(0, it0 + nh - 2); it < it0 + nh; ++it) ok = ok && mbar_wait(bar_mul + 8 * (it & 1), static_cast<uint32_t>(it / 2) & 1u, 22);
+        tc_fence_after();
+        __syncthreads();  // (everyone has seen the products done before their operands' places are taken)
+        bool again = false;
+        if (pass == 0 && tid < T) {
+            auto leaves = [](float sum, float s) {  // a scaled value may be beyond 2^15, or all are too small
+                const float v = sum * s * s;
+                return sum > 0.0f && !(v >= 0.0625f && v <= 1073741824.0f);
+            };
+            again = leaves(norm2(0, tid), scale_sh[tid]) || leaves(norm2(1, tid), scale_sh[kSeqMaxT + tid]);
+        }
+        if (pass > 0 || __syncthreads_or(again) == 0) break;
+    }
+
+    // ---------------- 2. scalars of the tokens ----------------
     if (tid < kSeqMaxT) {
         const int t = tid;
         float a = 0.0f, b = 0.0f, kinv = 0.0f, qinv = 0.0f;
         if (t < T) {
             const float bias = efla_seq_bias(p, static_cast<unsigned>(seq));
-            seq_scalars(p, p.beta_raw[(row0 + t) * p.ld_beta] + bias, part[t], part[kSeqMaxT + t], qinv, kinv, a, b);
+            seq_scalars(p, p.beta_raw[(row0 + t) * p.ld_beta] + bias, norm2(0, t), seq_infinite_norm(norm2(1, t), kg + static_cast<size_t>(t) * p.ld_qkv, hd), qinv, kinv, a, b);
         }
-        qs_sh[t] = kSqUp * qinv;
-        ks_sh[t] = kSqUp * kinv;
+        qs_sh[t] = qinv / scale_sh[t];  // (powers of two: exact)
+        ks_sh[t] = kinv / scale_sh[kSeqMaxT + t];
         a_sh[t] = a;
         b_sh[t] = b;
         float m = b;
@@ -319,102 +503,19 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
     __syncthreads();
     const int Te = min(min(red_bad[0], red_bad[1]), min(red_bad[2], red_bad[3]));  // tokens before the first one that makes the state NaN
     if (Te < T) {
-        if (tid >= Te && tid < T) qs_sh[tid] = ks_sh[tid] = a_sh[tid] = b_sh[tid] = 0.0f;
+        if (tid >= Te && tid < T) a_sh[tid] = b_sh[tid] = 0.0f;
         __syncthreads();
     }
     const float bscale = sq_pow2_scale<6>(fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3])));  // b * bscale < 64: P~ below 2^14, also for V's sake
-
-    // ---------------- 2. G and X ----------------
-    // staging: thread = (16-byte piece of a 64-column row block, row); four rows of K and of Q per thread
-    const int piece = tid & 15, srow = tid >> 4;
-    const uint32_t s_at = static_cast<uint32_t>(srow) * 128u + ((static_cast<uint32_t>(piece >> 1) ^ static_cast<uint32_t>(srow & 7)) << 4) + (piece & 1) * 8u;  // (+ 32 rows: + 4096)
-    struct KQ { float4 k[4], q[4]; };
-    auto load_block = [&](KQ& x, int d0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int t = srow + 32 * i, c = d0 + 4 * piece;
-            x.k[i] = x.q[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (t < Te && c < hd) {
-                x.k[i] = *reinterpret_cast<const float4*>(kg + static_cast<size_t>(t) * p.ld_qkv + c);
-                x.q[i] = *reinterpret_cast<const float4*>(qg + static_cast<size_t>(t) * p.ld_qkv + c);
-            }
-        }
-    };
-    auto put_split = [&](uint8_t* at, const float4& x, float s, int mid_off) {
-        uint2 hi, mid;
-        sq_split(x.x * s, x.y * s, hi.x, mid.x);
-        sq_split(x.z * s, x.w * s, hi.y, mid.y);
-        *reinterpret_cast<uint2*>(at) = hi;
-        *reinterpret_cast<uint2*>(at + mid_off) = mid;
-    };
-    auto gram_block = [&](KQ& x, int db) {  // (the next block but one is requested when this one has left the registers)
-        const int buf = db & 1;
-        if (db >= 2) ok = ok && mbar_wait(bar0 + 8 * buf, static_cast<uint32_t>(db / 2 - 1) & 1u, 21);  // the stage's last products have read it
-        uint8_t* st = sm + buf * kSqStage + s_at;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            if (srow + 32 * i >= 16 * nb) break;
-            put_split(st + i * 4096, x.k[i], ks_sh[srow + 32 * i], kSqUTile);
-            put_split(st + i * 4096 + 2 * kSqUTile, x.q[i], qs_sh[srow + 32 * i], kSqUTile);
-        }
-        fence_async_smem();
-        if (db + 2 < nd) load_block(x, (db + 2) * 64);
-        __syncthreads();
-        if (warp == 0 && elect_one()) {
-            tc_fence_after();
-            const uint32_t s0 = sm0 + buf * kSqStage;
-            const uint64_t kh = smem_desc(s0, 16, 1024, kLayoutSw128), km = smem_desc(s0 + kSqUTile, 16, 1024, kLayoutSw128);
-            const uint64_t qh = smem_desc(s0 + 2 * kSqUTile, 16, 1024, kLayoutSw128), qm = smem_desc(s0 + 3 * kSqUTile, 16, 1024, kLayoutSw128);
-            const int nk = min(4, (hd - db * 64) >> 4);
-            const uint32_t gram = kSqIdesc | (static_cast<uint32_t>(2 * nb) << 17);  // N 16 nb
-            for (int kk = 0; kk < nk; ++kk) {  // hi hi + hi mid + mid hi
-                const uint64_t o = static_cast<uint64_t>(2 * kk);
-                const uint32_t more = db > 0 || kk > 0 ? 1u : 0u;
-                tc_mma_f16(tmem, kh + o, kh + o, gram, more);
-                tc_mma_f16(tmem + 128, qh + o, kh + o, gram, more);
-                tc_mma_f16(tmem, kh + o, km + o, gram, 1u);
-                tc_mma_f16(tmem + 128, qh + o, km + o, gram, 1u);
-                tc_mma_f16(tmem, km + o, kh + o, gram, 1u);
-                tc_mma_f16(tmem + 128, qm + o, kh + o, gram, 1u);
-            }
-            tc_commit(bar0 + 8 * buf);
-        }
-        __syncwarp();
-    };
-    {
-        KQ even, odd;
-        load_block(even, 0);
-        if (nd > 1) load_block(odd, 64);
-        for (int db = 0; db < nd; db += 2) {
-            gram_block(even, db);
-            if (db + 1 < nd) gram_block(odd, db + 1);
-        }
-    }
-    for (int db = max(0, nd - 2); db < nd; ++db) ok = ok && mbar_wait(bar0 + 8 * (db & 1), static_cast<uint32_t>(db / 2) & 1u, 22);
-    tc_fence_after();
-    __syncthreads();  // (everyone has seen the products done before their operands' places are taken)
     if (meet) cluster_sync();
-    struct VT { float4 v[4]; };
-    auto load_v = [&](VT& x, int c0) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int t = srow + 32 * i, c = c0 + 4 * piece;
-            x.v[i] = (t < Te && c < hd) ? *reinterpret_cast<const float4*>(vg + static_cast<size_t>(t) * p.ld_qkv + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-    };
-    VT v_even;
-    load_v(v_even, ct0 * 64);  // (on its way during steps 3 and 4)
-
-    // ---------------- 3. L (two halves, stage 0), its diagonal blocks (fp32), X (fp32, stage 1): a thread per row and 32 columns ----------------
+    // ---------------- 3. L (two halves), its diagonal blocks (fp32), X (fp32): a thread per row and 32 columns ----------------
     __half* Lh = reinterpret_cast<__half*>(sm);
-    float* X = reinterpret_cast<float*>(sm + kSqStage);
+    float* X = reinterpret_cast<float*>(sm + kSqX);
     float* Ld = reinterpret_cast<float*>(sm + kSqDiag);
-    const int quad = warp & 3, cg = warp >> 2;  // rows 32 quad .. of tensor memory, columns 32 cg ..
-    const int t_row = 32 * quad + lane;
-    const uint32_t t_lane = tmem + (static_cast<uint32_t>(32 * quad) << 16);
-    if (cg <= quad && 32 * quad < 16 * nb) {
-        const float gdown = 1.0f / (kSqUp * kSqUp);
-        const float at = a_sh[t_row];
+    const int cg = warp >> 2;  // columns 32 cg ..
+    if (cg <= quad && 32 * quad < 16 * nb) {  // (the seventeenth warp has no columns: cg 4)
+        const bool row_ok = t_row < Te;  // (behind the cut there may be values that are no numbers)
+        const float at = a_sh[t_row], gf = ks_sh[t_row], xf = qs_sh[t_row];
 #pragma unroll
         for (int hc = 0; hc < 2; ++hc) {  // sixteen columns at a time
             const int c0 = 32 * cg + 16 * hc;
@@ -426,8 +527,9 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
             uint32_t hi[8], mid[8];
 #pragma unroll
             for (int e = 0; e < 16; ++e) {
-                g[e] = c0 + e < t_row ? at * (g[e] * gdown) : 0.0f;
-                x[e] = c0 + e <= t_row ? x[e] * gdown : 0.0f;
+                const float f = ks_sh[c0 + e];
+                g[e] = row_ok && c0 + e < t_row ? at * (g[e] * gf * f) : 0.0f;
+                x[e] = row_ok && c0 + e <= t_row ? x[e] * xf * f : 0.0f;
             }
 #pragma unroll
             for (int e = 0; e < 8; ++e) sq_split(g[2 * e] * kSqUp, g[2 * e + 1] * kSqUp, hi[e], mid[e]);
@@ -454,148 +556,189 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_seq_kernel(const EflaPara
 
     // ---------------- 4. P~ M = X by block columns from the right; warp i owns rows 16 i .. 16 i + 15 ----------------
     const int g = lane >> 2, tq = lane & 3;
-    uint8_t* prow = sm + kSqStage;
+    uint8_t* prow = sm + kSqX;
     if (warp < nb) {
+        // P~'s blocks, two halves a value, take the place of X's as they are finished (32 bytes a row each: hi, mid)
         const int i = warp;
-        float xr[8][2][4];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            if (j <= i) {
-#pragma unroll
-                for (int n = 0; n < 2; ++n) {
-                    const float2 lo = *reinterpret_cast<const float2*>(X + (i * 16 + g) * kSqXStride + j * 16 + n * 8 + 2 * tq);
-                    const float2 hi = *reinterpret_cast<const float2*>(X + (i * 16 + g + 8) * kSqXStride + j * 16 + n * 8 + 2 * tq);
-                    xr[j][n][0] = lo.x; xr[j][n][1] = lo.y; xr[j][n][2] = hi.x; xr[j][n][3] = hi.y;
-                }
-            }
-        }
-        __syncwarp();  // the rows are in registers: P~ takes their place
-        seq_solve_rows(sm0, kSqStage, prow, kSqInv, i, lane, xr);
+        const float* xi = X + (i * 16 + g) * kSqXStride + 2 * tq;
+        seq_solve_rows<64, 32>(sm0, kSqX, prow, kSqInv, i, lane, [&](int j, int n, int e) { return xi[(e >> 1) * 8 * kSqXStride + j * 16 + n * 8 + (e & 1)]; });
     }
-    __syncthreads();  // L has been read: the operand tiles of P~ take its place
-    if (warp < nb) {
+    __syncthreads();  // P~ is complete
+    if (warp < 16 && 32 * quad < 16 * nb) {
         // the columns' factors b_s, scaled to at most 64, applied to the finished rows (exact powers of two aside, one more rounding); zeros above the diagonal
-        const int i = warp;
-        for (int idx = lane; idx < 16 * 16; idx += 32) {
-            const int t = i * 16 + (idx >> 4), c0 = (idx & 15) * 8;
-            uint32_t hi[4] = {0u, 0u, 0u, 0u}, mid[4] = {0u, 0u, 0u, 0u};
-            if (c0 < 16 * (i + 1)) {
-                const uint8_t* d = prow + t * (kSqXStride * 4) + c0 * 2;
-                const uint4 hv = *reinterpret_cast<const uint4*>(d), mv = *reinterpret_cast<const uint4*>(d + kSqPMid);
-                const uint32_t hw[4] = {hv.x, hv.y, hv.z, hv.w}, mw[4] = {mv.x, mv.y, mv.z, mv.w};
+        const uint32_t ta = t_lane + kSqTA;
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hw[e])), mf = __half22float2(*reinterpret_cast<const __half2*>(&mw[e]));
-                    sq_split((hf.x + mf.x) * (b_sh[c0 + 2 * e] * bscale), (hf.y + mf.y) * (b_sh[c0 + 2 * e + 1] * bscale), hi[e], mid[e]);
+        for (int jj = 0; jj < 2; ++jj) {
+            const int j = 2 * cg + jj;
+            if (j >= nb) break;
+            uint32_t hi[8], mid[8];
+            const uint4* d = reinterpret_cast<const uint4*>(prow + t_row * (kSqXStride * 4) + j * 64);
+            const float4* bs = reinterpret_cast<const float4*>(b_sh + 16 * j);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) hi[e] = mid[e] = 0u;
+            if (j <= t_row >> 4) {
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    const uint4 hv = d[v], mv = d[2 + v];
+                    const uint32_t hw[4] = {hv.x, hv.y, hv.z, hv.w}, mw[4] = {mv.x, mv.y, mv.z, mv.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 hf = __half22float2(*reinterpret_cast<const __half2*>(&hw[e])), mf = __half22float2(*reinterpret_cast<const __half2*>(&mw[e]));
+                        const float4 b4 = bs[2 * v + (e >> 1)];
+                        const float b0 = (e & 1) ? b4.z : b4.x, b1 = (e & 1) ? b4.w : b4.y;
+                        sq_split((hf.x + mf.x) * (b0 * bscale), (hf.y + mf.y) * (b1 * bscale), hi[4 * v + e], mid[4 * v + e]);
+                    }
                 }
             }
-            uint8_t* d = sm + (c0 >> 6) * kSqUTile + t * 128 + ((((c0 >> 3) & 7) ^ (t & 7)) << 4);
-            *reinterpret_cast<uint4*>(d) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(d + 2 * kSqUTile) = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+            __syncwarp();
+            sq_tmem_st8(ta + 8 * j, hi);
+            sq_tmem_st8(ta + 64 + 8 * j, mid);
         }
+        sq_tmem_st_wait();
     }
+    tc_fence_before();
+    fence_async_smem();
     __syncthreads();  // (also: the rows of P~ have been read, V's tiles take their place)
 
-    // ---------------- 5. y = P~ V, 64 columns at a time; a tile leaves while the next one's product runs ----------------
-    float* out = reinterpret_cast<float*>(sm + kSqOut);
-    // rows t of 256 bytes, 16-byte piece ^ t % 16: the column group's rows go in, whole rows of the output come out, both without bank conflicts
-    auto finish = [&](int l, float ds, bool tile_bad) {  // the CTA's l-th tile
-        ok = ok && mbar_wait(bar0 + 16 + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 23);
-        tc_fence_after();
-        float y[16];
-        sq_tmem_ld16(t_lane + (l & 1) * 64 + 16 * cg, y);
-        tmem_ld_wait();
-        tc_fence_before();
-        const int* bad_col = reinterpret_cast<const int*>(sm + kSqBad) + 64 * (l & 1);
+    // ---------------- 5. y = P~ V, 64 columns at a time; a tile leaves while the next ones are converted and multiplied ----------------
+    const bool wide = ((reinterpret_cast<uintptr_t>(p.out) & 15) | (p.ld_out & 3)) == 0;  // rows of y start at multiples of 16 bytes
+    float* ds_sh = red + 16;                                  // [2]: undoes the scales of P~ and of V
+    int* bad_sh = reinterpret_cast<int*>(red + 18);           // [2]: a v of the tile is no number
+    if (warp < kGroup) {
+        // eight warps convert V (thread = a 16-byte piece of eight rows) ..
+        const int piece = tid & 15, srow = tid >> 4;
+        constexpr int kRows = kSeqThreads / 32, kPer = kSeqMaxT / kRows;
+        for (int l = 0; l < nct; ++l) {
+            float4 v[kPer];
+            ok = ok && mbar_wait(bar_v + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 28);
+            const int c = (ct0 + l) * 64 + 4 * piece;
+            const uint8_t* raw = sm + ((l & 1) ? kSqV1 : kSqV0) + (piece >> 3) * kSqUTile + srow * 128 + (((piece & 7) ^ (srow & 7)) << 4);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            y[e] *= ds;
-            if (tile_bad || Te < T)
-                if (t_row >= Te || (tile_bad && t_row >= bad_col[16 * cg + e])) y[e] = NAN;
-        }
+            for (int i = 0; i < kPer; ++i)
+                v[i] = srow + kRows * i < Te && c < hd ? *reinterpret_cast<const float4*>(raw + i * (kRows * 128)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            // the tile's own power-of-two scale keeps both halves of its values in range
+            uint32_t m = 0;
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-            *reinterpret_cast<float4*>(out + t_row * 64 + (((4 * cg + e) ^ (t_row & 15)) << 2)) = make_float4(y[4 * e], y[4 * e + 1], y[4 * e + 2], y[4 * e + 3]);
-        __syncthreads();
-        const int c = (ct0 + l) * 64 + 2 * lane;
-        for (int t = warp; t < T; t += 16)
-            if (ok && c < hd) *reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float2*>(out + t * 64 + (((lane >> 1) ^ (t & 15)) << 2) + 2 * (lane & 1));
-    };
-    float ds_prev = 0.0f;
-    bool bad_prev = false;
-    auto y_tile = [&](VT& x, int l) {
-        // the tile's own power-of-two scale keeps both halves of its values in range
-        uint32_t m = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) m = max(m, seq_abs_bits(x.v[i]));
-        m = __reduce_max_sync(0xffffffffu, m);
-        uint32_t* redb = reinterpret_cast<uint32_t*>(red) + 16 * (l & 1);
-        if (lane == 0) redb[warp] = m;
-        __syncthreads();
-        m = __reduce_max_sync(0xffffffffu, redb[lane & 15]);
-        const bool tile_bad = m >= kSeqNonFinite;
-        if (tile_bad) {
-            int* bad_col = reinterpret_cast<int*>(sm + kSqBad) + 64 * (l & 1);
-            if (tid < 64) bad_col[tid] = T;
-            __syncthreads();
-            m = 0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                auto clear = [&](float& x, int e) {
-                    if (!(fabsf(x) <= FLT_MAX)) {
-                        atomicMin(bad_col + 4 * piece + e, srow + 32 * i);
-                        x = 0.0f;
-                    }
-                };
-                clear(x.v[i].x, 0); clear(x.v[i].y, 1); clear(x.v[i].z, 2); clear(x.v[i].w, 3);
-                m = max(m, seq_abs_bits(x.v[i]));
-            }
+            for (int i = 0; i < kPer; ++i) m = max(m, seq_abs_bits(v[i]));
             m = __reduce_max_sync(0xffffffffu, m);
-            if (lane == 0) redb[warp] = m;  // (read by everyone before the barrier above)
-            __syncthreads();
-            m = __reduce_max_sync(0xffffffffu, redb[lane & 15]);
-        }
-        const float vs = sq_pow2_scale<15>(__uint_as_float(m));
-        uint8_t* st = sm + kSqStage + (l & 1) * (2 * kSqUTile) + s_at;  // (its last product is done: finish has waited for it)
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (srow + 32 * i < 16 * nb) put_split(st + i * 4096, x.v[i], vs, kSqUTile);
-        fence_async_smem();
-        if (l + 2 < nct) load_v(x, (ct0 + l + 2) * 64);
-        tc_fence_before();
-        __syncthreads();
-        if (warp == 0 && elect_one()) {
-            tc_fence_after();
-            const uint64_t ph = smem_desc(sm0, 16, 1024, kLayoutSw128), pm = smem_desc(sm0 + 2 * kSqUTile, 16, 1024, kLayoutSw128);
-            const uint32_t v0 = sm0 + kSqStage + (l & 1) * (2 * kSqUTile);
-            const uint64_t vh = smem_desc(v0, 1024, 1024, kLayoutSw128), vm = smem_desc(v0 + kSqUTile, 1024, 1024, kLayoutSw128);
-            const uint32_t d = tmem + (l & 1) * 64;
-            for (int kk = 0; kk < nb; ++kk) {  // sixteen tokens: 32 bytes of a row of P~, 16 rows of V
-                const uint64_t a = static_cast<uint64_t>((kk >> 2) * (kSqUTile >> 4) + (kk & 3) * 2), b = static_cast<uint64_t>(kk * (2048 >> 4));
-                tc_mma_f16(d, ph + a, vh + b, kSqIdescY, kk > 0 ? 1u : 0u);
-                tc_mma_f16(d, ph + a, vm + b, kSqIdescY, 1u);
-                tc_mma_f16(d, pm + a, vh + b, kSqIdescY, 1u);
+            uint32_t* redb = reinterpret_cast<uint32_t*>(red) + 8 * (l & 1);
+            if (lane == 0) {
+                redb[warp] = m;
+                mbar_arrive(bar_vread + 8 * (l & 1));  // (the tile has been read: its values are in m)
             }
-            tc_commit(bar0 + 16 + 8 * (l & 1));
+            if (l >= 2) ok = ok && mbar_wait(bar_drain + 8 * (l & 1), static_cast<uint32_t>(l / 2 - 1) & 1u, 27);  // the tile before the last has left its accumulator (and its product the operands)
+            group_sync();
+            m = __reduce_max_sync(0xffffffffu, redb[lane & 7]);
+            const bool tile_bad = m >= kSeqNonFinite;
+            if (tile_bad) {
+                int* bad_col = reinterpret_cast<int*>(sm + kSqBad) + 64 * (l & 1);
+                if (tid < 64) bad_col[tid] = T;
+                group_sync();
+                m = 0;
+#pragma unroll
+                for (int i = 0; i < kPer; ++i) {
+                    auto clear = [&](float& x, int e) {
+                        if (!(fabsf(x) <= FLT_MAX)) {
+                            atomicMin(bad_col + 4 * piece + e, srow + kRows * i);
+                            x = 0.0f;
+                        }
+                    };
+                    clear(v[i].x, 0); clear(v[i].y, 1); clear(v[i].z, 2); clear(v[i].w, 3);
+                    m = max(m, seq_abs_bits(v[i]));
+                }
+                m = __reduce_max_sync(0xffffffffu, m);
+                if (lane == 0) redb[warp] = m;  // (read by everyone before the barrier above)
+                group_sync();
+                m = __reduce_max_sync(0xffffffffu, redb[lane & 7]);
+            }
+            const float vs = sq_pow2_scale<15>(__uint_as_float(m));
+            if (tid == 0) {
+                ds_sh[l & 1] = 1.0f / kSqUp / bscale / vs;  // (P~'s scales are 2^8 and b's)
+                bad_sh[l & 1] = tile_bad;
+            }
+            uint8_t* st = sm + (l & 1) * (2 * kSqUTile) + srow * 128 + (((piece >> 1) ^ (srow & 7)) << 4) + (piece & 1) * 8;
+#pragma unroll
+            for (int i = 0; i < kPer; ++i)
+                if (srow + kRows * i < 16 * nb) put_split(st + i * (kRows * 128), v[i], vs, kSqUTile);
+            arrive(bar_vop + 8 * (l & 1));
         }
-        __syncwarp();
-        if (l > 0) finish(l - 1, ds_prev, bad_prev);
-        ds_prev = 1.0f / kSqUp / bscale / vs;  // undoes the scales of P~ (2^8 and b's) and of V
-        bad_prev = tile_bad;
-    };
-    {
-        VT v_odd;
-        if (nct > 1) load_v(v_odd, (ct0 + 1) * 64);
-        for (int l = 0; l < nct; l += 2) {
-            y_tile(v_even, l);
-            if (l + 1 < nct) y_tile(v_odd, l + 1);
+    } else if (warp < 16) {
+        // .. and eight take the tiles of y: rows t of 256 bytes, 16-byte piece ^ t % 16: a row's 32 columns go in, whole rows of the output come out, both without bank conflicts
+        float* out = reinterpret_cast<float*>(sm + kSqOut);
+        const int half = ch, gtid = tid - 32 * kGroup;
+        for (int l = 0; l < nct; ++l) {
+            ok = ok && mbar_wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 29);
+            const float ds = ds_sh[l & 1];
+            const bool tile_bad = bad_sh[l & 1] != 0;
+            ok = ok && mbar_wait(bar_y + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 23);
+            __syncwarp();
+            tc_fence_after();
+            uint32_t acc[32];
+            tmem_ld32(t_lane + (l & 1) * 64 + 32 * half, acc);
+            tmem_ld_wait();
+            tc_fence_before();
+            float y[32];
+            const int* bad_col = reinterpret_cast<const int*>(sm + kSqBad) + 64 * (l & 1);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+                y[e] = __uint_as_float(acc[e]) * ds;
+                if (tile_bad || Te < T)
+                    if (t_row >= Te || (tile_bad && t_row >= bad_col[32 * half + e])) y[e] = NAN;
+            }
+            if (l > 0) group_sync();  // the tile before has left `out`
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                *reinterpret_cast<float4*>(out + t_row * 64 + (((8 * half + e) ^ (t_row & 15)) << 2)) = make_float4(y[4 * e], y[4 * e + 1], y[4 * e + 2], y[4 * e + 3]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_drain + 8 * (l & 1));
+            group_sync();
+            if (across) {  // y may lie on other columns of v: it leaves when the next three tiles have been read or are here
+                if (l + 2 < nct) ok = ok && mbar_wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2 + 1) & 1u, 29);
+                if (l + 3 < nct) ok = ok && mbar_wait(bar_v + 8 * ((l + 3) & 1), static_cast<uint32_t>((l + 3) / 2) & 1u, 28);
+            }
+            if (wide) {
+                const int piece = gtid & 15, c = (ct0 + l) * 64 + 4 * piece;
+#pragma unroll 4
+                for (int t = gtid >> 4; t < T; t += kSeqThreads / 32)
+                    if (ok && c < hd) *reinterpret_cast<float4*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float4*>(out + t * 64 + ((piece ^ (t & 15)) << 2));
+            } else {
+                const int c = (ct0 + l) * 64 + 2 * lane;
+                for (int t = warp - kGroup; t < T; t += kGroup)
+                    if (ok && c < hd) *reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float2*>(out + t * 64 + (((lane >> 1) ^ (t & 15)) << 2) + 2 * (lane & 1));
+            }
         }
+    } else if (warp == 16) {
+        for (int l = 0; l < nct; ++l) {
+            ok = ok && mbar_wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 25);
+            if (elect_one() && ok) {
+                tc_fence_after();
+                const uint32_t at = sm0 + (l & 1) * (2 * kSqUTile), d = tmem + (l & 1) * 64, ta = tmem + kSqTA;
+                const uint64_t vh = smem_desc(at, 1024, 1024, kLayoutSw128), vm = smem_desc(at + kSqUTile, 1024, 1024, kLayoutSw128);
+                for (int kk = 0; kk < nb; ++kk) {  // sixteen tokens: 8 columns of P~, 16 rows of V
+                    const uint64_t b = static_cast<uint64_t>(kk * (2048 >> 4));
+                    sq_mma_ts(d, ta + 8 * kk, vh + b, kSqIdescY, kk > 0 ? 1u : 0u);
+                    sq_mma_ts(d, ta + 8 * kk, vm + b, kSqIdescY, 1u);
+                    sq_mma_ts(d, ta + 64 + 8 * kk, vh + b, kSqIdescY, 1u);
+                }
+                tc_commit(bar_y + 8 * (l & 1));
+            }
+            __syncwarp();
+        }
+    } else {
+        for (int l = 1; l < nct; ++l) {
+            if (l >= 2) ok = ok && mbar_wait(bar_vread + 8 * (l & 1), static_cast<uint32_t>(l / 2 - 1) & 1u, 29);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            load_v(l);
+        }
+        // none of the copies may be on its way when the CTA leaves (they have all been waited for unless a wait expired)
+        for (int s = 0; s < 4; ++s)
+            if (loads > s) mbar_wait(bar_raw + 8 * s, static_cast<uint32_t>((loads - 1 - s) / 4) & 1u, 26);
+        for (int s = 0; s < 2; ++s)
+            if (v_loads > s) mbar_wait(bar_v + 8 * s, static_cast<uint32_t>((v_loads - 1 - s) / 2) & 1u, 28);
     }
-    __syncthreads();  // (the tile before it has left)
-    finish(nct - 1, ds_prev, bad_prev);
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) {
+    if (warp == 16) {
         tc_fence_after();
         tmem_dealloc(tmem, kSqTmemCols);
     }
@@ -878,14 +1021,8 @@ __global__ void __launch_bounds__(kSeqThreads, 1) efla_long_kernel(const EflaPar
         seq_invert_diagonal(reinterpret_cast<const float*>(sm + kLgDiag), reinterpret_cast<__half*>(sm + kLgInv), 8, warp, lane);
         __syncthreads();
         if (warp < 8) {
-            float xr[8][2][4];
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-#pragma unroll
-                for (int n = 0; n < 2; ++n)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) xr[j][n][e] = j == warp && n * 8 + 2 * tq + (e & 1) == g + 8 * (e >> 1) ? 1.0f : 0.0f;
-            seq_solve_rows(sm0, kLgMat, sm + kLgMat, kLgInv, warp, lane, xr);
+            seq_solve_rows<32, kSqPMid>(sm0, kLgMat, sm + kLgMat, kLgInv, warp, lane,
+                                        [&](int j, int n, int e) { return j == warp && n * 8 + 2 * tq + (e & 1) == g + 8 * (e >> 1) ? 1.0f : 0.0f; });
         }
         __syncthreads();
     };
@@ -975,17 +1112,25 @@ int efla_seq_launch(const EflaParams& p, cudaStream_t stream) {
         if (dev < 64) configured[dev].store(true, std::memory_order_relaxed);
     }
     // Few units leave SMs idle: two or four CTAs each take a share of a unit's column tiles, as long as all run at once (the sums before them are done by
-    // each). One head of 512, 128 tokens: 32 sequences 45 us with one CTA each, 34 with four; 70 sequences 45 with one, 39 with two. Where the output lies on q or k, the CTAs of
+    // each). One head of 512, 128 tokens: 32 sequences 34.7 us with one CTA each, 27.2 with four; 70 sequences 35.3 with one, 30.3 with two; 32 of 16 tokens 24.4 and 18.2. Where the output lies on q or k, the CTAs of
     // a unit are a cluster; fours of them fit all SMs of a chip only in part (a processing cluster of 18 SMs holds four).
     const int sms = multiprocessors(dev), nd = (p.hidden / p.heads + 63) >> 6;
     if (sms <= 0) return BNF4_ERR_CUDA;
     const bool meet = seq_overlap(p, p.q) != SEQ_APART || seq_overlap(p, p.k) != SEQ_APART;
     const int cs = seq_overlap(p, p.v) == SEQ_ACROSS ? 1 : units * 4 <= (meet ? sms * 7 / 8 : sms) && nd >= 4 ? 4 : units * 2 <= sms && nd >= 2 ? 2 : 1;
     const bool early = p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems;
+    const int across = seq_overlap(p, p.v) == SEQ_ACROSS;
+    CUtensorMap maps[3];  // boxes of 128 tokens and 32 columns
+    const void* in[3] = {p.q, p.k, p.v};
+    for (int i = 0; i < 3; ++i) {
+        const int rc2 = make_map_2d(&maps[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, in[i], static_cast<uint64_t>(p.hidden), static_cast<uint64_t>(p.seqs) * static_cast<uint64_t>(p.T),
+                                    static_cast<uint64_t>(p.ld_qkv) * 4, 32, kSeqMaxT, "scan inputs");
+        if (rc2) return rc2;
+    }
     if (cs > 1 && meet) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(static_cast<unsigned>(units * cs));
-        cfg.blockDim = dim3(kSeqThreads);
+        cfg.blockDim = dim3(kSqThreads);
         cfg.dynamicSmemBytes = kSqSmem;
         cfg.stream = stream;
         cudaLaunchAttribute attr[2];
@@ -996,9 +1141,9 @@ int efla_seq_launch(const EflaParams& p, cudaStream_t stream) {
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = early ? 2 : 1;
-        cudaLaunchKernelEx(&cfg, efla_seq_kernel, p, cs, 1);  // errors surface in check_launch
+        cudaLaunchKernelEx(&cfg, efla_seq_kernel, maps[0], maps[1], maps[2], p, cs, 1, across);  // errors surface in check_launch
     } else {
-        launch_pdl_if(early, efla_seq_kernel, static_cast<unsigned>(units * cs), kSeqThreads, kSqSmem, stream, p, cs, 0);
+        launch_pdl_if(early, efla_seq_kernel, static_cast<unsigned>(units * cs), kSqThreads, kSqSmem, stream, maps[0], maps[1], maps[2], p, cs, 0, across);
     }
     return check_launch("efla_seq_kernel");
 }
