@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(1024) ce_step_kernel(const float* __restrict__
 // order, the group adds its chains in order, the mean adds the groups in double. Every loss is a function of the logits alone: grid and
 // member count only say which warps compute the row losses. (1024 pairs rank losses that differ in the last place: another order of these
 // sums moves some across each other and with them the update.)
-// Grid (16 split, members), split 1, 2 or 4: `split` blocks share a group, `split` warps a chain. Member counters (zero before the launch, zero
+// Grid (16 split, members), split 1, 2, 4 or 8: `split` blocks share a group, `split` warps a chain. Member counters (zero before the launch, zero
 // again after it): the member's last block forms the mean; without them split is 1, partial[member * 16 + group] holds the groups'
 // sums and ce_finalize_kernel follows. With split > 1 partial holds the chains' sums, 128 per member.
 constexpr int kCeChunks = 16;
@@ -885,9 +885,10 @@ int get_scratch(size_t floats, float** out) {
 
 int cross_entropy_launch(const float* logits, int ld, const float* bias, const int8_t* bias_noise, float sigma, const uint8_t* targets, int vocab, int members,
                          int rows_per_member, float* partial, unsigned* counters, float* loss_mean, cudaStream_t st) {
-    // few members (a validation pass has one): more blocks per member as long as the SMs are not filled and a warp keeps eight rows. Same bits.
+    // few members (a validation pass has one): more blocks per member as long as the SMs are not filled and a warp keeps four rows. Same bits. One member of
+    // 4096 rows, end of its whole pass: 63.5 us with at most four, 61.6 with eight; of 16384 rows 164 and 150.
     int split = 1;
-    while (counters != nullptr && split < 4 && members * kCeChunks * split < 2 * 148 && rows_per_member >= 2 * split * 1024) split *= 2;
+    while (counters != nullptr && split < 8 && members * kCeChunks * split < 2 * 148 && rows_per_member >= 2 * split * 512) split *= 2;
     const dim3 grid(kCeChunks * split, members);
     const bool early = static_cast<long long>(members) * rows_per_member * vocab <= kPdlStreamElems;
     const bool vec = (vocab % 4) == 0 && (ld % 4) == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0 &&

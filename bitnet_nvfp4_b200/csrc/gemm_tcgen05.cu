@@ -103,6 +103,10 @@ struct KernelArgs {
     int total_tiles;
     int ks_wrap;  // K blocks after which A starts again and B2 follows B (0: no second operand)
     int n_tiles;  // tiles along N (of 256 columns in the pair instances); blockIdx.x = m_tile * n_tiles + n_tile (N fastest: CTAs that share A rows run together)
+    // A CTA's (or pair's) first tile and the way to its next one without a division: four of them stood between the predecessor's end and the first load (800
+    // cycles; a GEMM of one tile behind another 4.7 -> 4.3 us).
+    uint32_t tile_magic;  // ceil(2^32 / n_tiles): exact quotients for the few hundred CTAs (0: one tile along N)
+    int step_n, step_m;   // CTAs (pairs) of the grid % and / n_tiles
 };
 
 // Persistent kernel: one CTA per SM walks the tile list (tile = m_tile * n_tiles + n_tile, N fastest so that
@@ -151,6 +155,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
     if constexpr (PAIR) rank = cluster_rank();
     // the tiles this CTA (or pair) walks: unit, unit + units, ..
     const unsigned unit = PAIR ? blockIdx.x >> 1 : blockIdx.x, units = PAIR ? gridDim.x >> 1 : gridDim.x;
+    const int first_m = static_cast<int>(args.tile_magic == 0 ? unit : __umulhi(unit, args.tile_magic)), first_n = static_cast<int>(unit) - first_m * args.n_tiles;
 
     if (threadIdx.x == 64) {  // the tensor maps come from the parameter area: fetch them before the predecessor has finished
         asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_a)) : "memory");
@@ -190,8 +195,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             int kc = 0, s = 0;
             uint32_t empty_parity = 1;
             bool ok = true;
+            int mt = first_m, nt = first_n;
             for (unsigned tile = unit; tile < static_cast<unsigned>(total_tiles) && ok; tile += units) {
-                const int mt = static_cast<int>(tile / static_cast<unsigned>(args.n_tiles)), nt = static_cast<int>(tile - static_cast<unsigned>(mt) * static_cast<unsigned>(args.n_tiles));
                 const bool two = nt * 256 + 128 < p.n;  // the second half has columns
                 // each CTA holds half of the B rows of the pair's MMA: 128 of 256, or 64 of 128
                 const int my = mt * 256 + static_cast<int>(rank) * BM, ny = nt * 256 + static_cast<int>(rank) * (two ? 128 : 64);
@@ -217,6 +222,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     __syncwarp();
                     if (++s == kStages) { s = 0; empty_parity ^= 1u; }
                 }
+                nt += args.step_n;
+                mt += args.step_m;
+                if (nt >= args.n_tiles) { nt -= args.n_tiles; ++mt; }
             }
             // the last stages' releases arrive from the leading CTA: wait for them, so that none is in flight towards a CTA that has left
             for (int i = 0; i < min(kc, kStages) && ok; ++i) {
@@ -238,8 +246,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             uint32_t full_parity = 0, kc = 0, odd = 0;
             uint32_t empty_par = 0, used = 0;  // per accumulator block (bit): parity of the drain to wait for next; whether it was used before
             bool ok = rank == 0;
+            int nt = first_n;
             for (unsigned tile = unit; tile < static_cast<unsigned>(total_tiles) && ok; tile += units, odd ^= 1u) {
-                const int nt = static_cast<int>(tile % static_cast<unsigned>(args.n_tiles));
                 const bool two = nt * 256 + 128 < p.n;
                 // both CTAs' epilogues must have drained the blocks
                 for (uint32_t b = odd; b <= odd + (two ? 1u : 0u) && ok; ++b) {
@@ -280,6 +288,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     __syncwarp();
                     if (++s == kStages) { s = 0; full_parity ^= 1u; }
                 }
+                nt += args.step_n;
+                if (nt >= args.n_tiles) nt -= args.n_tiles;
             }
         }
     } else if (warp == 0) {
@@ -290,9 +300,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             int s = 0;
             uint32_t empty_parity = 1;  // parity of the phase that precedes the first completion: the first pass does not wait
             bool ok = true;
-            const int step_n = static_cast<int>(gridDim.x % static_cast<unsigned>(args.n_tiles)), step_m = static_cast<int>(gridDim.x / static_cast<unsigned>(args.n_tiles));
-            int m_tile = static_cast<int>(blockIdx.x / static_cast<unsigned>(args.n_tiles)) - step_m;
-            int n_tile = static_cast<int>(blockIdx.x % static_cast<unsigned>(args.n_tiles)) - step_n;
+            const int step_n = args.step_n, step_m = args.step_m;
+            int m_tile = first_m - step_m;
+            int n_tile = first_n - step_n;
             for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
                 n_tile += step_n;
                 m_tile += step_m;
@@ -431,7 +441,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         };
         const int row_in_tile = q * 32 + lane;
         // Tile coordinates advance by additions (tiles are walked in steps of gridDim.x): no division per tile.
-        const int step_n = static_cast<int>(units % static_cast<unsigned>(args.n_tiles)), step_m = static_cast<int>(units / static_cast<unsigned>(args.n_tiles));
+        const int step_n = args.step_n, step_m = args.step_m;
         // m_tile counts 128-row tiles (of a pair's tile: this CTA's), n_tile 128-column tiles; the halves of a pair's tile follow each other.
         // PAIR: `odd` = parity of the tile, `last` = no further half follows in this tile.
         struct TileIdx { int m_tile, n_tile, odd; bool last; };
@@ -522,7 +532,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             }
             if (col0_ + lane < p.n) cx.aval[0] = __ldg(p.lora_A + static_cast<size_t>(trk_member >> 1) * p.lora_A_pair_stride + col0_ + lane);
         };
-        TileIdx cur_t{static_cast<int>(unit / static_cast<unsigned>(args.n_tiles)), static_cast<int>(unit % static_cast<unsigned>(args.n_tiles)), 0, true};
+        TileIdx cur_t{first_m, first_n, 0, true};
         if constexpr (PAIR) {
             cur_t.m_tile = 2 * cur_t.m_tile + static_cast<int>(rank);
             first_half(cur_t, cur_t.n_tile);
@@ -538,7 +548,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         bool have_cur = false, have_nxt = false;
         auto issue_res_load = [&](const TileIdx& t, bool valid) {
             const int col0_ = t.n_tile * BN + c * 32;
-            have_nxt = valid && col0_ < p.n;
+            have_nxt = valid && col0_ < p.n && (!R0 || t.m_tile * BM + q * 32 < p.m);
             if (!have_nxt) return;
             rb_last = rb_last == 2 ? 0 : rb_last + 1;
             if (lane == 0) {
@@ -579,7 +589,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             const long long row = static_cast<long long>(m0) + row_in_tile;
             const bool row_ok = R1 || row < p.m;  // (the rank-1 instance runs with m a multiple of the tile height)
             const int col0 = n0 + c * 32;
-            const bool chunk_ok = col0 < p.n;  // warp-uniform
+            // warp-uniform: the warp's part of the tile lies in the matrix (rows: the few of a token step; with a rank term the test cost ragged members 2 %)
+            const bool chunk_ok = col0 < p.n && (!R0 || m0 + q * 32 < p.m);
 
             const int member = nxt.member, pair = member >> 1;
             float tr[4] = {R0 ? 0.0f : static_cast<float>(nxt.tr[0]), 0.0f, 0.0f, 0.0f};
@@ -621,6 +632,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 }
             }
 
+            // C, too, is requested before the wait (a 32 x 512 x 512 product added to another 5.4 -> 5.0 us; the instances with a rank term have no registers for it)
+            constexpr bool kEarlyC = EPI == EPI_F32 && R0 && !PAIR && !B2;
+            float4 c_early[kEarlyC ? 8 : 1];
+            bool c_vec = false;
+            if constexpr (kEarlyC) {
+                if (p.beta != 0.0f && row_ok && col0 + 32 <= p.n) {
+                    const float* crow = p.c + static_cast<size_t>(row) * p.ldc + col0;
+                    c_vec = (reinterpret_cast<uintptr_t>(crow) & 15) == 0;
+                    if (c_vec)
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) c_early[j] = reinterpret_cast<const float4*>(crow)[j];
+                }
+            }
+
             ok = mbar_wait(bar_acc_full + 8 * buf, PAIR ? (pfull >> buf) & 1u : (it >> 1) & 1, 3);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -648,10 +673,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             }
             if (!R1 && p.beta != 0.0f && row_ok) {
                 const float* crow = p.c + static_cast<size_t>(row) * p.ldc + col0;
-                if (col0 + 32 <= p.n && (reinterpret_cast<uintptr_t>(crow) & 15) == 0) {
+                if (kEarlyC ? c_vec : col0 + 32 <= p.n && (reinterpret_cast<uintptr_t>(crow) & 15) == 0) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float4 c4 = reinterpret_cast<const float4*>(crow)[j];
+                        const float4 c4 = kEarlyC ? c_early[kEarlyC ? j : 0] : reinterpret_cast<const float4*>(crow)[j];
                         v[4 * j] = fmaf(p.beta, c4.x, v[4 * j]);
                         v[4 * j + 1] = fmaf(p.beta, c4.y, v[4 * j + 1]);
                         v[4 * j + 2] = fmaf(p.beta, c4.z, v[4 * j + 2]);
@@ -1153,6 +1178,13 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     } else {
         md = ma;  // unused
     }
+    // (also called for the tiles of a pair)
+    auto set_tiles = [&](int n_tiles, unsigned units) {
+        args.n_tiles = n_tiles;
+        args.tile_magic = n_tiles == 1 ? 0u : static_cast<uint32_t>(((1ull << 32) + static_cast<unsigned>(n_tiles) - 1) / static_cast<unsigned>(n_tiles));
+        args.step_n = static_cast<int>(units % static_cast<unsigned>(n_tiles));
+        args.step_m = static_cast<int>(units / static_cast<unsigned>(n_tiles));
+    };
     args.n_tiles = (p.n + BN - 1) / BN;
     const long long tiles = static_cast<long long>(args.n_tiles) * ((p.m + BM - 1) / BM);
     if (tiles > 0x7fffffffLL) return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: too many tiles");
@@ -1203,9 +1235,9 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
         if (!rc) rc = make_map_2d(&msf.sfa, CU_TENSOR_MAP_DATA_TYPE_UINT32, p.sfa, 128, static_cast<uint64_t>((p.m + 127) / 128) * args.k_atoms, 512, 128, 4, "A scales", CU_TENSOR_MAP_SWIZZLE_NONE);
         if (!rc) rc = make_map_2d(&msf.sfb, CU_TENSOR_MAP_DATA_TYPE_UINT32, p.sfb, 128, static_cast<uint64_t>((p.n + 127) / 128) * args.k_atoms, 512, 128, 4, "B scales", CU_TENSOR_MAP_SWIZZLE_NONE);
         if (rc) return rc;
-        args.n_tiles = (p.n + 255) / 256;
         args.total_tiles = static_cast<int>(pair_tiles);
         const dim3 grid(2 * static_cast<unsigned>(std::min<long long>(pair_tiles, sms / 2)), 1, 1);
+        set_tiles((p.n + 255) / 256, grid.x / 2);
         return with_epilogue([&](auto epi) -> int {
             constexpr int E = decltype(epi)::value;
             auto run = [&](auto r) { return launch_t<E, decltype(r)::value, true, false>(ma, mb, md, msf, args, grid, dev, stream); };
@@ -1214,6 +1246,7 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     }
     if (gemm_panel_applies(p, rk, sms)) return gemm_panel_launch(p, rk, ma, mb, md, args.group_magic, sms, dev, stream);
     const dim3 grid(static_cast<unsigned>(std::min<long long>(tiles, sms)), 1, 1);
+    set_tiles(args.n_tiles, grid.x);
     if (p.b2 != nullptr) {
         if (p.sfb2 == nullptr || (p.b2_rows % 128) != 0 || p.b2_rows < p.n || p.rows_per_member <= 0 || (p.rows_per_member % BM) != 0 || p.rank > 0)
             return set_error(BNF4_ERR_INVALID, "gemm_nvfp4: the second operand needs member rows and b2_rows in multiples of 128 and takes no rank term");
