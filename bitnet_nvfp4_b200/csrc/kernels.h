@@ -32,7 +32,8 @@ struct RowQuantParams : bnf4_rowquant_desc {
     int32_t* zero_t = nullptr;  // FE_ADD_ABSMEAN: clears [rows][zero_n] words, the projections the GEMM after next accumulates with atomics
     int zero_n = 0;
     int pad_sf = 0;              // also clears the padding of the scale array (rows to 128, columns to 64)
-    int batch = 1;   // set by the launch: rows a warp quantises before it takes their projections together
+    int wide_ok = 0;  // set by the dispatch: the fp32 (or fp16) rows and the position table can be read 32 bytes at a time
+    int batch = 1;    // set by the launch: rows a warp quantises before it takes their projections together
 };
 int rowquant_dispatch(int front_end, RowQuantParams p, cudaStream_t stream);
 

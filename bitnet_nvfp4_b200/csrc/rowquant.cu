@@ -312,6 +312,28 @@ __device__ __forceinline__ uint2 lds_u64(uint32_t saddr) {
     asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(saddr));
     return v;
 }
+// Eight of a lane's sixteen fp32 values (or its sixteen halves). The lanes' values lie 64 bytes apart, so that a load instruction touches
+// sixteen lines whatever its width, and a line is asked for by two or four of them: 32-byte loads halve both. They pass by L1, which the tables'
+// lines then keep; 16-byte loads (rows off a 32-byte boundary: wide = false) need their lines there until the last quarter is read, which a
+// streaming load does not promise. 16-byte streaming -> 16-byte plain -> 32-byte -> 32-byte past L1, us: fp32 rows 16384 x 512
+// 10.3 -> 9.4 -> 9.0 -> 8.9; + position / GELU 262144 x 512 219 -> 218 -> 191 -> 192, 65536 x 2048 with 16 projections 343 -> 318 -> 304 -> 287.
+__device__ __forceinline__ void load8(const void* src, bool wide, uint4& a, uint4& b) {
+    if (wide) {
+        asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                     : "l"(src));
+    } else {
+        a = *reinterpret_cast<const uint4*>(src);
+        b = *(reinterpret_cast<const uint4*>(src) + 1);
+    }
+}
+__device__ __forceinline__ float4 as_float4(const uint4& v) { return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)); }
+__device__ __forceinline__ void load8(const float* src, bool wide, float4& a, float4& b) {
+    uint4 ua, ub;
+    load8(static_cast<const void*>(src), wide, ua, ub);
+    a = as_float4(ua);
+    b = as_float4(ub);
+}
 // Element ownership as in rowquant_kernel: lane l owns the 16-element scale blocks l, l + 32, ... (NB of them).
 // NV = upper bound of p.nvec this instance handles (4 or kMaxTVec): the projection loops carry no tests beyond it.
 // BATCH (more than four projections): a 16-byte load per block and vector, one dp4a per four bytes, a warp reduction (8 cycles) per sum and
@@ -415,10 +437,25 @@ __device__ __forceinline__ void project_rows(const RowQuantParams& p, const int4
     }
 }
 
+// Which instances keep a row's bytes, not its sixteen floats per block, until the norm is known, and how many blocks of them share an SM.
+// Rows of more than 512 columns hold 32 or 64 floats a lane: with them in registers too few warps are resident to cover the latency of the
+// loads, without them the bytes are widened a second time. 65536 rows, us:
+//   floats kept -> bytes kept, 2 / 3 blocks an SM: int8 rows, 2048 columns, 16 projections 153 -> 136 / 140, 4 projections 126 -> 99 / 100,
+//     1024 columns 55 -> 53 / 52; + position / GELU, 1024 columns 137 -> 122 / 124, 2048 columns, 16 projections 344 -> 347 / 393;
+//     + branch, 2048 columns, 4 projections 160 -> 165 / 148, 1024 columns, 1 projection 67 -> 70 / 71
+//   floats kept, 2 / 3 blocks: + position / GELU, 2048 columns, 4 projections 257 / 261 (one block: 294, with 16-byte loads); fp32 rows of 2048
+//     columns 191 / 154 (one block: 191)
+template <int FE, int NB, int NV>
+constexpr bool kKeepBytes = NB > 1 && (FE == FE_ABSMEAN || (FE == FE_POS_GELU_ABSMEAN && NB <= 2) || (FE == FE_ADD_ABSMEAN && NB > 2 && NV <= 4));
+template <int FE, int NB, int NV>
+constexpr int kFastCtas = NB <= 1 ? 4 : kKeepBytes<FE, NB, NV> ? (FE == FE_ADD_ABSMEAN ? 3 : 2) : (FE == FE_ACT && NB > 2) ? 3 : (NB <= 2 || NV > 4 || FE == FE_POS_GELU_ABSMEAN) ? 2 : 1;
+
+// MODEL: powers of two for rows per member, columns and positions, 32-byte aligned rows, one or four projections: no test or division for any of it
+// (the 32-byte rule: 262144 x 512 + position / GELU 198 -> 191 us).
 // ZERO: the MODEL instance that also clears p.zero_t, for launches of up to kPdlStreamElems elements; larger ones have a memset in front (the test
 // and the store cost the default model's instance 4 %, 0.6 of 14.4 ms a step, the memsets 0.1 ms).
 template <int FE, int NB, int NV, bool MODEL = false, bool ZERO = !MODEL>
-__global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1))) rowquant_fast_kernel(const RowQuantParams p, const uint8_t* __restrict__ lut) {
+__global__ void __launch_bounds__(256, kFastCtas<FE, NB, NV>) rowquant_fast_kernel(const RowQuantParams p, const uint8_t* __restrict__ lut) {
     pdl_trigger();
     __shared__ __align__(16) uint2 tab_s[128];  // per amax: {bits of fl(1 / scale), scale byte}
     if (threadIdx.x < 128) tab_s[threadIdx.x] = __ldg(reinterpret_cast<const uint2*>(lut + kQuantBlockTabOffset) + threadIdx.x);
@@ -429,7 +466,9 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
     const uint32_t tab_c = static_cast<uint32_t>(__cvta_generic_to_shared(tab_s)) - (static_cast<uint32_t>(kRoundBiasBits) << 3);
     const float M = kRoundBias;
     constexpr bool kNorm = (FE == FE_ADD_ABSMEAN || FE == FE_POS_GELU_ABSMEAN || FE == FE_ABSMEAN);
+    constexpr bool PACK = kKeepBytes<FE, NB, NV>;
     const float gelu_safe = gelu_q8_safe(p.act_scale);
+    const bool wide = MODEL || p.wide_ok;
 
     const int lane = threadIdx.x & 31;
     const int nblk = p.cols_out >> 4;
@@ -481,8 +520,8 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
         }
 
         // ---------------- stage 1: integer values of the row as floats ----------------
-        float vf[NB][16];
-        uint32_t raw_w[FE == FE_INT8 ? NB : 1][4];  // FE_INT8: the row's bytes
+        float vf[PACK ? 1 : NB][16];
+        uint32_t raw_w[FE == FE_INT8 || PACK ? NB : 1][4];  // the row's bytes (FE_INT8, PACK)
         uint32_t sum_abs = 0;  // sum of |value| over this lane's elements (exact integer)
         int tok = 0;
         float a_r[4] = {0.f, 0.f, 0.f, 0.f};
@@ -501,8 +540,10 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
             const int kb = lane + 32 * i;
             const int k0 = kb << 4;
             if (kb >= nblk) {
+                if constexpr (!PACK) {
 #pragma unroll
-                for (int e = 0; e < 16; ++e) vf[i][e] = 0.0f;
+                    for (int e = 0; e < 16; ++e) vf[i][e] = 0.0f;
+                }
                 continue;
             }
             if constexpr (FE == FE_INT8) {
@@ -519,7 +560,14 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                 const float* src = p.in_f32 + static_cast<size_t>(row) * p.ld_in + k0;
                 float4 f4[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) f4[q] = __ldcs(reinterpret_cast<const float4*>(src) + q);
+                for (int q = 0; q < 4; q += 2) {
+                    if constexpr (NB == 2) {  // the one instance that streaming loads suit: 65536 x 1024 71.8 us, 74.0 with the 32-byte ones
+                        f4[q] = __ldcs(reinterpret_cast<const float4*>(src) + q);
+                        f4[q + 1] = __ldcs(reinterpret_cast<const float4*>(src) + q + 1);
+                    } else {
+                        load8(src + 4 * q, wide, f4[q], f4[q + 1]);
+                    }
+                }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     float x[4] = {f4[q].x, f4[q].y, f4[q].z, f4[q].w};
@@ -544,7 +592,8 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                 const uint32_t rw[4] = {static_cast<uint32_t>(raw.x), static_cast<uint32_t>(raw.y), static_cast<uint32_t>(raw.z), static_cast<uint32_t>(raw.w)};
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    bytes4_to_float(rw[q], &vf[i][4 * q]);
+                    if constexpr (PACK) raw_w[i][q] = rw[q];
+                    else bytes4_to_float(rw[q], &vf[i][4 * q]);
                     sum_abs += abs_sum_bytes4(rw[q]);
                 }
             } else if constexpr (FE == FE_ADD_ABSMEAN) {
@@ -555,7 +604,8 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                 float4 y4[4];
                 if (MODEL || p.in_f16) {  // the branch output as IEEE halves (exact widening)
                     const uint4* yh = reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(p.in_f32) + static_cast<size_t>(row) * p.ld_in + k0);
-                    const uint4 h0 = __ldcs(yh), h1 = __ldcs(yh + 1);
+                    uint4 h0, h1;
+                    load8(yh, wide, h0, h1);
                     const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
@@ -564,7 +614,7 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                     }
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) y4[q] = __ldcs(reinterpret_cast<const float4*>(yr + k0 + 4 * q));
+                    for (int q = 0; q < 4; q += 2) load8(yr + k0 + 4 * q, wide, y4[q], y4[q + 1]);
                 }
                 uint32_t upd[4];
 #pragma unroll
@@ -580,11 +630,14 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                         const float2 sm = __fadd2_rn(tr, make_float2(oldf[j], oldf[j + 1]));
                         tb[j] = fminf(fmaxf(sm.x, M - 127.0f), M + 127.0f);
                         tb[j + 1] = fminf(fmaxf(sm.y, M - 127.0f), M + 127.0f);
-                        const float2 vv = __fadd2_rn(make_float2(tb[j], tb[j + 1]), make_float2(-M, -M));
-                        vf[i][4 * q + j] = vv.x;
-                        vf[i][4 * q + j + 1] = vv.y;
+                        if constexpr (!PACK) {
+                            const float2 vv = __fadd2_rn(make_float2(tb[j], tb[j + 1]), make_float2(-M, -M));
+                            vf[i][4 * q + j] = vv.x;
+                            vf[i][4 * q + j + 1] = vv.y;
+                        }
                     }
                     upd[q] = biased4_to_bytes(tb[0], tb[1], tb[2], tb[3]);
+                    if constexpr (PACK) raw_w[i][q] = upd[q];
                     sum_abs += abs_sum_bytes4(upd[q]);
                 }
                 *reinterpret_cast<int4*>(xr + k0) = make_int4(static_cast<int>(upd[0]), static_cast<int>(upd[1]), static_cast<int>(upd[2]), static_cast<int>(upd[3]));
@@ -605,11 +658,13 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                 }
                 float4 f4[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) f4[q] = __ldcs(reinterpret_cast<const float4*>(src + k0 + 4 * q));
+                for (int q = 0; q < 4; q += 2) load8(src + k0 + 4 * q, wide, f4[q], f4[q + 1]);
+                float4 pos4[2];
                 uint32_t resid[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const float4 p4 = *reinterpret_cast<const float4*>(pos + k0 + 4 * q);
+                    if (!(q & 1)) load8(pos + k0 + 4 * q, wide, pos4[0], pos4[1]);
+                    const float4 p4 = pos4[q & 1];
                     const float ff[4] = {f4[q].x, f4[q].y, f4[q].z, f4[q].w};
                     float pv[4] = {p4.x, p4.y, p4.z, p4.w};
                     if (has_pn) {
@@ -622,9 +677,12 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
 #pragma unroll
                     for (int j = 0; j < 4; ++j) x[j] = ff[j] + pv[j];
                     gelu_q8x4(x, p.act_scale, gelu_safe, tb);
+                    if constexpr (!PACK) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) vf[i][4 * q + j] = tb[j] - M;
+                        for (int j = 0; j < 4; ++j) vf[i][4 * q + j] = tb[j] - M;
+                    }
                     resid[q] = biased4_to_bytes(tb[0], tb[1], tb[2], tb[3]);
+                    if constexpr (PACK) raw_w[i][q] = resid[q];
                     sum_abs += abs_sum_bytes4(resid[q]);
                 }
                 // residual stream = the pre-norm values
@@ -692,17 +750,25 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
             if (active) {
                 float tq[16];
                 float am = 0.0f;
+                float un[16];
+                const float* v16 = un;
+                if constexpr (PACK) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) bytes4_to_float(raw_w[i][q], un + 4 * q);
+                } else {
+                    v16 = vf[i];
+                }
                 if (kNorm && inv > 1.0f) {  // same for the whole row; only then can |v| * inv pass 127
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
-                        const float n = fminf(fmaxf(__fmul_rn(vf[i][e], inv), -127.0f), 127.0f);
+                        const float n = fminf(fmaxf(__fmul_rn(v16[e], inv), -127.0f), 127.0f);
                         am = fmaxf(am, fabsf(n));
                         tq[e] = n + M;
                     }
                 } else {
 #pragma unroll
                     for (int e = 0; e < 16; e += 2) {  // packed fp32 pairs: each half rounds like the scalar instruction
-                        float2 n = make_float2(vf[i][e], vf[i][e + 1]);
+                        float2 n = make_float2(v16[e], v16[e + 1]);
                         if constexpr (kNorm) n = __fmul2_rn(n, make_float2(inv, inv));
                         am = fmax3(am, fabsf(n.x), fabsf(n.y));
                         const float2 t2 = __fadd2_rn(n, make_float2(M, M));
@@ -726,8 +792,8 @@ __global__ void __launch_bounds__(256, (NB <= 1 ? 4 : (NB <= 2 || NV > 4 ? 2 : 1
                     lo = e2m1x8_biased(tq, rs);
                     hi = e2m1x8_biased(tq + 8, rs);
                 } else {  // the values are integers already
-                    lo = e2m1x8_table(vf[i], rs);
-                    hi = e2m1x8_table(vf[i] + 8, rs);
+                    lo = e2m1x8_table(v16, rs);
+                    hi = e2m1x8_table(v16 + 8, rs);
                 }
                 *reinterpret_cast<uint2*>(p.out_codes + (static_cast<size_t>(row) * p.cols_out + k0) / 2) = make_uint2(lo, hi);
             }
@@ -869,7 +935,7 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
             };
             // the batched driver's calls at hidden <= 512: see MODEL above
             auto pow2 = [](long long v) { return v > 0 && (v & (v - 1)) == 0; };
-            bool model = nblk <= 32 && (FE == FE_ADD_ABSMEAN || FE == FE_ABSMEAN || FE == FE_POS_GELU_ABSMEAN) && pow2(p.cols_in) && pow2(p.rows_per_member) &&
+            bool model = p.wide_ok && nblk <= 32 && (FE == FE_ADD_ABSMEAN || FE == FE_ABSMEAN || FE == FE_POS_GELU_ABSMEAN) && pow2(p.cols_in) && pow2(p.rows_per_member) &&
                          p.out_q == nullptr && (p.nvec == 1 || p.nvec == 4) && p.tvec != nullptr && p.t_out != nullptr && al16(p.t_out);
             if (FE == FE_ADD_ABSMEAN) model = model && p.in_f16 != 0;
             if (FE == FE_POS_GELU_ABSMEAN) model = model && pow2(p.pos_mod) && (p.gather_rows <= 0 || pow2(p.row_mod));
@@ -926,6 +992,10 @@ int rowquant_dispatch(int fe, RowQuantParams p, cudaStream_t stream) {
             p.vec_ok = aligned16(p.in_f32, static_cast<long long>(p.ld_in) * 4) ? 1 : 0; break;
         default: p.vec_ok = 1; break;
     }
+    // 32-byte loads: fp32 rows (or halves), and the position table's
+    const long long in_bytes = p.in_f16 ? 2 : 4;
+    p.wide_ok = (reinterpret_cast<uintptr_t>(p.in_f32) & 31) == 0 && ((p.ld_in * in_bytes) & 31) == 0 &&
+                (fe != FE_POS_GELU_ABSMEAN || ((reinterpret_cast<uintptr_t>(p.pos) & 31) == 0 && (p.cols_in & 7) == 0));
     p.vec_ok_q = (p.out_q != nullptr && aligned16(p.out_q, p.ld_q)) ? 1 : 0;
     if (fe == FE_ADD_ABSMEAN || fe == FE_POS_GELU_ABSMEAN) {
         if (!aligned16(p.inout_i8, p.cols_in))
