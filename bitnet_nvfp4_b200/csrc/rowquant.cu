@@ -443,12 +443,12 @@ __device__ __forceinline__ void project_rows(const RowQuantParams& p, const int4
 //   floats kept -> bytes kept, 2 / 3 blocks an SM: int8 rows, 2048 columns, 16 projections 153 -> 136 / 140, 4 projections 126 -> 99 / 100,
 //     1024 columns 55 -> 53 / 52; + position / GELU, 1024 columns 137 -> 122 / 124, 2048 columns, 16 projections 344 -> 347 / 393;
 //     + branch, 2048 columns, 4 projections 160 -> 165 / 148, 1024 columns, 1 projection 67 -> 70 / 71
-//   floats kept, 2 / 3 blocks: + position / GELU, 2048 columns, 4 projections 257 / 261 (one block: 294, with 16-byte loads); fp32 rows of 2048
-//     columns 191 / 154 (one block: 191)
+//   floats kept, 2 / 3 blocks: + position / GELU, 2048 columns, 4 projections 257 / 261 (one block: 294, with 16-byte loads).
+//     fp32 rows past 1024 columns stay at one block: three take 65536 x 2048 from 186 to 154, but 4000 x 1984 from 16 to 20
 template <int FE, int NB, int NV>
 constexpr bool kKeepBytes = NB > 1 && (FE == FE_ABSMEAN || (FE == FE_POS_GELU_ABSMEAN && NB <= 2) || (FE == FE_ADD_ABSMEAN && NB > 2 && NV <= 4));
 template <int FE, int NB, int NV>
-constexpr int kFastCtas = NB <= 1 ? 4 : kKeepBytes<FE, NB, NV> ? (FE == FE_ADD_ABSMEAN ? 3 : 2) : (FE == FE_ACT && NB > 2) ? 3 : (NB <= 2 || NV > 4 || FE == FE_POS_GELU_ABSMEAN) ? 2 : 1;
+constexpr int kFastCtas = NB <= 1 ? 4 : kKeepBytes<FE, NB, NV> ? (FE == FE_ADD_ABSMEAN ? 3 : 2) : (NB <= 2 || NV > 4 || FE == FE_POS_GELU_ABSMEAN) ? 2 : 1;
 
 // MODEL: powers of two for rows per member, columns and positions, 32-byte aligned rows, one or four projections: no test or division for any of it
 // (the 32-byte rule: 262144 x 512 + position / GELU 198 -> 191 us).
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(256, kFastCtas<FE, NB, NV>) rowquant_fast_kern
                 float4 f4[4];
 #pragma unroll
                 for (int q = 0; q < 4; q += 2) {
-                    if constexpr (NB == 2) {  // the one instance that streaming loads suit: 65536 x 1024 71.8 us, 74.0 with the 32-byte ones
+                    if constexpr (NB >= 2) {  // streaming loads suit these: 65536 x 1024 71.8 us, 74.0 with the 32-byte ones; 4000 x 1984 from DRAM 16.0, 19.5
                         f4[q] = __ldcs(reinterpret_cast<const float4*>(src) + q);
                         f4[q + 1] = __ldcs(reinterpret_cast<const float4*>(src) + q + 1);
                     } else {
