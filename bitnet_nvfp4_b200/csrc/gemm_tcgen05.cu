@@ -113,11 +113,14 @@ struct KernelArgs {
 // CTAs working at the same time share rows of A through L2). Three roles run concurrently on different tiles:
 // the producer prefetches operands up to kStages k-blocks ahead, the MMA warp fills one of two TMEM
 // accumulators while the sixteen epilogue warps drain the other one.
-// RK: 4 = the instance for rank-4 perturbation terms whose pairs start at multiples of 32 rows;
-// 1 = the instance for the batched driver's common case (rank 1, no C operand, every 128-row tile inside one member), which carries
-// none of the general paths; 0 = no rank term at all, 2 = every other one. (262144 x 1024 x 512 with GELU to FP4, no rank term: 303 us as a case
-// of the general instance, which spills, 256 us.)
-// B2: the instance with a second B operand (no rank term); the others carry no tests for one (rank 2 with GELU to FP4 446 -> 412 us).
+// RK: the form of the rank term. 0 = none; 1 = the batched driver's common case (rank 1, no C operand, every 128-row tile inside one member), which
+// carries none of the general paths; 3 and 5 = rank 2 and 4 whose pairs start at multiples of 32 rows, so that a warp's rows share a pair; 2 and 4 =
+// every other one of rank 1 and 2, 3 and 4, with zeros for a factor that is not there. The number of products is thereby known to the compiler: one
+// instance that tested the rank inside the loop over the columns spilled 90 bytes and more. Figures, one such instance -> these, us: 88800 x 320 x 320 rank 2 residual 44 -> 32,
+// 88800 x 961 x 320 rank 2 halves 69 -> 52, 88800 x 960 x 320 GELU to FP4 rank 2 141 -> 106, rank 3 with members of 1100 rows 152 -> 132, 65536 x 512 x 2048 rank 2
+// residual 65 -> 46, 16384 x 512 x 512 rank 3 fp32 11.9 -> 10.8. Without forms 3 and 5 those of rank 2 and 4 lose 2 to 12 % (33.5, 54, 119). Dearer: 16384 x 4096 x 4096
+// rank 3 fp32, 132 -> 134, where the products with a zero count. (262144 x 1024 x 512 with GELU to FP4 and no rank term: 303 us as a case of a general instance, 256 us.)
+// B2: the instance with a second B operand (no rank term); the others carry no tests for one (a rank-2 term with GELU to FP4 446 -> 412 us).
 // PAIR: the instance for operands with many K blocks. On the in-order pipe a scale copy costs about 44 cycles and an M 128 x N 128 MMA
 // 64 (measured, one CTA): 8 copies and 4 MMAs per 256-element K block of a 128 x 128 tile take 560 cycles before any operand
 // traffic, 860 with it. A CTA pair (cta_group::2) on a 256 x 256 tile needs 12 copies and 4 MMAs of N 256 for four times the work; the
@@ -425,9 +428,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     __ldg(reinterpret_cast<const uint2*>(args.lut + kQuantBlockTabOffset) + ew * 32 + lane);
             asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");
         }
-        // RK 4 with FP4 output: the vectors of the next projection, fetched a tile ahead like the factors (loads where they are used left the warps waiting: 65536 x 8192
+        // RK 2 and up with FP4 output: the vectors of the next projection, fetched a tile ahead like the factors (loads where they are used left the warps waiting: 65536 x 8192
         // x 2048 with four of them 883 -> 878 us), and a place where the rows' sums are turned round (128-byte atomics instead of sixteen sectors each: 787 us).
-        constexpr bool R4 = RK == 4, kStageNext = R4 && EPI == EPI_GELU_FP4;
+        constexpr bool kInside = RK == 3 || RK == 5, kStageNext = RK >= 2 && EPI == EPI_GELU_FP4;
+        constexpr int kTerms = RK >= 4 ? 4 : 2;  // products of the rank term (factors that are not there are zeros)
         int4* next_sh = reinterpret_cast<int4*>(smem_gen + oSmemEpi + kQuantBlockTabBytes + ew * 640);  // [4][32] bytes, then [32][4] sums
         // Perturbation context of one tile: this thread's row (projections t, sign, pair) and this thread's element of the A factor
         // of the warp's first pair for the tile's columns. It is fetched one tile ahead so that the global-load latency hides
@@ -437,7 +441,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             int member;
             int tr[4];    // raw integers: converted to float only when the tile is processed, so that nothing waits
             int aval[4];  // on these loads earlier;  aval[r] = A[pair of the warp's first row][col0 + lane][r]
-            int next_b;   // RK 4: this thread's word of the pair's vectors of the next projection: vector lane / 8, columns col0 + 4 (lane % 8) ..
+            int next_b;   // RK 2 and up: this thread's word of the pair's vectors of the next projection: vector lane / 8, columns col0 + 4 (lane % 8) ..
         };
         const int row_in_tile = q * 32 + lane;
         // Tile coordinates advance by additions (tiles are walked in steps of gridDim.x): no division per tile.
@@ -470,7 +474,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         auto has_rows = [&](const TileIdx& t) { return t.m_tile < m_end && t.m_tile * BM < p.m; };
         // Members are visited in ascending order, so when tiles never straddle members (rows_per_member a multiple of the
         // tile height) the member of the next tile is tracked with comparisons instead of a division per row.
-        const bool tile_uniform_member = p.rows_per_member > 0 && (p.rows_per_member % BM) == 0;
         int trk_member = static_cast<int>(opaque_zero());  // (the pair's vectors are loaded read-only: their addresses depend on this)
         long long trk_end = p.rows_per_member;  // first row of member trk_member + 1
         const uint32_t group_magic = args.group_magic;  // ceil(2^32 / group_cols): exact quotients for columns below 65536
@@ -479,14 +482,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             const unsigned e = __umulhi(row, args.rpm_magic);
             return static_cast<int>(row - e * static_cast<unsigned>(p.rows_per_member) >= static_cast<unsigned>(p.rows_per_member) ? e + 1 : e);
         };
+        const int terms = kInside ? kTerms : p.rank;
         auto load_a = [&](int pr, int n, int (&aval)[4]) {
-            const int8_t* Ag = p.lora_A + static_cast<size_t>(pr) * p.lora_A_pair_stride + static_cast<size_t>(n) * p.rank;
-            aval[0] = Ag[0];
-            if (p.rank > 1) {
-                aval[1] = Ag[1];
-                if (p.rank > 2) aval[2] = Ag[2];
-                if (p.rank > 3) aval[3] = Ag[3];
-            }
+            const int8_t* Ag = p.lora_A + static_cast<size_t>(pr) * p.lora_A_pair_stride + static_cast<size_t>(n) * terms;
+#pragma unroll
+            for (int r = 0; r < kTerms; ++r) aval[r] = r < terms ? Ag[r] : 0;
         };
         auto fetch_ctx = [&](const TileIdx& t, bool valid, LoraCtx& cx) {
             cx.member = 0;
@@ -498,13 +498,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             cx.member = member_of(static_cast<unsigned>(min(row_, p.m - 1)));  // (rows past m are never stored)
             if (row_ < p.m && col0_ < p.n) {
                 const int g = p.group_cols > 0 ? static_cast<int>(__umulhi(static_cast<uint32_t>(col0_), group_magic)) : 0;
-                const int* tp = p.lora_t + static_cast<size_t>(row_) * p.t_stride + g * p.rank;
-                cx.tr[0] = tp[0];
-                if (p.rank > 1) {
-                    cx.tr[1] = tp[1];
-                    if (p.rank > 2) cx.tr[2] = tp[2];
-                    if (p.rank > 3) cx.tr[3] = tp[3];
-                }
+                const int* tp = p.lora_t + static_cast<size_t>(row_) * p.t_stride + g * terms;
+#pragma unroll
+                for (int r = 0; r < kTerms; ++r)
+                    if (r < terms) cx.tr[r] = tp[r];
             }
             const int first = __shfl_sync(0xffffffffu, cx.member, 0) >> 1;
             if (col0_ + lane < p.n) load_a(first, col0_ + lane, cx.aval);
@@ -516,7 +513,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         // The common case (rank 1, tiles inside one member) with as few instructions as possible: this phase sits on the serial
         // path of every tile.
         constexpr bool R1 = RK == 1, R0 = RK == 0;
-        const bool fast_ctx = R1 || (RK == 2 && p.rank == 1 && tile_uniform_member);
         const int* t_row = !R0 && p.rank > 0 ? p.lora_t + static_cast<size_t>(row_in_tile) * p.t_stride : nullptr;
         auto fetch_fast = [&](const TileIdx& t, bool valid, LoraCtx& cx) {
             cx.member = 0;
@@ -575,7 +571,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
         nxt.aval[1] = nxt.aval[2] = nxt.aval[3] = 0;
         nxt.next_b = 0;
         if constexpr (R0) nxt.member = 0;
-        else if (R1 || fast_ctx) fetch_fast(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles, nxt);
+        else if (R1) fetch_fast(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles, nxt);
         else fetch_ctx(cur_t, PAIR ? has_rows(cur_t) : static_cast<int>(blockIdx.x) < total_tiles, nxt);
         uint32_t pfull = 0;  // PAIR: parities of the completions to wait for (bit per accumulator block)
         uint32_t acc_empty_bar = bar_acc_empty;
@@ -596,7 +592,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             float tr[4] = {R0 ? 0.0f : static_cast<float>(nxt.tr[0]), 0.0f, 0.0f, 0.0f};
             float* loraA_sh = reinterpret_cast<float*>(smem_gen + oSmemLora) + ew * 4 * 32;  // this warp's [4][32]
             if (R0) {
-            } else if (R1 || fast_ctx) {
+            } else if (R1) {
                 __syncwarp();  // the previous tile's reads are done
                 loraA_sh[lane] = static_cast<float>(nxt.aval[0]);
                 __syncwarp();
@@ -607,8 +603,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                 tr[3] = static_cast<float>(nxt.tr[3]);
                 __syncwarp();  // the previous tile's reads are done
 #pragma unroll
-                for (int r = 0; r < 4; ++r)
-                    if (r < p.rank) loraA_sh[r * 32 + lane] = static_cast<float>(nxt.aval[r]);
+                for (int r = 0; r < kTerms; ++r) loraA_sh[r * 32 + lane] = static_cast<float>(nxt.aval[r]);
                 if constexpr (kStageNext) reinterpret_cast<int*>(next_sh)[lane] = nxt.next_b;
                 __syncwarp();
                 fetch_ctx(nxt_t, more, nxt);
@@ -702,9 +697,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
             } else if constexpr (!R0) {
                 // sum_r t[r]*A[n][r] is an integer below 2^24: float products and sums are exact. Rows of another pair (and rows past m)
                 // take part with a zero factor.
-                const int pair_hi = R4 ? 0 : __shfl_sync(0xffffffffu, pair, 31);  // (the rank-4 instance runs with 32 rows inside one pair)
-                for (int pr = R4 ? 0 : __shfl_sync(0xffffffffu, pair, 0);; ++pr) {
-                    const float ls = R4 || pair == pr ? lsign : 0.0f;
+                const int pair_hi = kInside ? 0 : __shfl_sync(0xffffffffu, pair, 31);
+                for (int pr = kInside ? 0 : __shfl_sync(0xffffffffu, pair, 0);; ++pr) {
+                    const float ls = kInside || pair == pr ? lsign : 0.0f;
                     const float2 ls2 = make_float2(ls, ls);
                     const float2 t0 = make_float2(tr[0], tr[0]), t1 = make_float2(tr[1], tr[1]), t2 = make_float2(tr[2], tr[2]), t3 = make_float2(tr[3], tr[3]);
 #pragma unroll
@@ -716,23 +711,18 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                             lo = __ffma2_rn(tt, make_float2(a.x, a.y), lo);
                             hi = __ffma2_rn(tt, make_float2(a.z, a.w), hi);
                         };
-                        if constexpr (R4) { add(t1, 1); add(t2, 2); add(t3, 3); }
-                        else {
-                            if (p.rank > 1) add(t1, 1);
-                            if (p.rank > 2) add(t2, 2);
-                            if (p.rank > 3) add(t3, 3);
-                        }
+                        add(t1, 1);
+                        if constexpr (kTerms > 2) { add(t2, 2); add(t3, 3); }
                         lo = __ffma2_rn(ls2, lo, make_float2(v[4 * j + 0], v[4 * j + 1]));
                         hi = __ffma2_rn(ls2, hi, make_float2(v[4 * j + 2], v[4 * j + 3]));
                         v[4 * j + 0] = lo.x; v[4 * j + 1] = lo.y; v[4 * j + 2] = hi.x; v[4 * j + 3] = hi.y;
                     }
-                    if (R4 || pr >= pair_hi) break;
+                    if (kInside || pr >= pair_hi) break;
                     __syncwarp();  // the next pair's factor takes the place of this one's
                     int av[4] = {0, 0, 0, 0};
                     if (col0 + lane < p.n) load_a(pr + 1, col0 + lane, av);
 #pragma unroll
-                    for (int r = 0; r < 4; ++r)
-                        if (r < p.rank) loraA_sh[r * 32 + lane] = static_cast<float>(av[r]);
+                    for (int r = 0; r < kTerms; ++r) loraA_sh[r * 32 + lane] = static_cast<float>(av[r]);
                     __syncwarp();
                 }
             }
@@ -939,13 +929,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                     }
                 }
                 if constexpr (EPI == EPI_GELU_FP4) {
+                    const bool one_pair = kInside || !kStageNext || __shfl_sync(0xffffffffu, pair, 0) == __shfl_sync(0xffffffffu, pair, 31);
                     if (row_ok) {
                         const uint32_t s0 = sfv[0], s1 = sfv[1], lo0 = codes[0], hi0 = codes[1], lo1 = codes[2], hi1 = codes[3];
                         *reinterpret_cast<uint4*>(p.d_codes + (static_cast<size_t>(row) * p.n + col0) / 2) = make_uint4(lo0, hi0, lo1, hi1);
                         const int kb = col0 >> 4;
                         *reinterpret_cast<uint16_t*>(p.d_sf + sf_offset(static_cast<int>(row), kb, sf_k_atoms(p.n))) =
                             static_cast<uint16_t>(s0 | (s1 << 8));
-                        if (!kStageNext && (R1 || p.next_nvec > 0)) {  // (the rank-1 FP4 instance always feeds one projection)
+                        if ((!kStageNext || !one_pair) && (R1 || p.next_nvec > 0)) {  // (the rank-1 FP4 instance always feeds one projection)
                             const int8_t* tv = p.next_tvec + static_cast<size_t>(pair) * p.next_tvec_pair_stride + col0;
                             const int nv_ = R1 ? 1 : p.next_nvec;  // (the rank-1 instance runs with at most one projection)
                             for (int vv = 0; vv < nv_; ++vv) {
@@ -958,31 +949,32 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_nvfp4_kernel(const __grid_co
                             }
                         }
                     }
-                    if constexpr (kStageNext) {  // (vectors that are not there are zeros; rows past m take part up to the store)
-                        int a4[4];
+                    if (kStageNext && one_pair) {  // (vectors that are not there are zeros; rows past m take part up to the store)
+                        int a4[kTerms];
 #pragma unroll
-                        for (int vv = 0; vv < 4; ++vv) {
+                        for (int vv = 0; vv < kTerms; ++vv) {
                             const int4 b0 = next_sh[2 * vv], b1 = next_sh[2 * vv + 1];
                             int a = 0;
                             a = __dp4a(w[0], b0.x, a); a = __dp4a(w[1], b0.y, a); a = __dp4a(w[2], b0.z, a); a = __dp4a(w[3], b0.w, a);
                             a = __dp4a(w[4], b1.x, a); a = __dp4a(w[5], b1.y, a); a = __dp4a(w[6], b1.z, a); a = __dp4a(w[7], b1.w, a);
                             a4[vv] = a;
                         }
-                        if (p.next_nvec == 4) {
+                        if (p.next_nvec == kTerms) {
                             int* sums = reinterpret_cast<int*>(next_sh + 8);
-                            reinterpret_cast<int4*>(sums)[lane] = make_int4(a4[0], a4[1], a4[2], a4[3]);
+                            if constexpr (kTerms == 2) reinterpret_cast<int2*>(sums)[lane] = make_int2(a4[0], a4[1]);
+                            else reinterpret_cast<int4*>(sums)[lane] = make_int4(a4[0], a4[1], a4[kTerms - 2], a4[kTerms - 1]);
                             __syncwarp();
-                            int* t = p.next_t + (static_cast<size_t>(m0) + q * 32) * 4 + lane;
+                            int* t = p.next_t + (static_cast<size_t>(m0) + q * 32) * kTerms + lane;
                             if (m0 + BM <= p.m) {
 #pragma unroll
-                                for (int i = 0; i < 4; ++i) atomicAdd(t + 32 * i, sums[32 * i + lane]);
+                                for (int i = 0; i < kTerms; ++i) atomicAdd(t + 32 * i, sums[32 * i + lane]);
                             } else {
-                                for (int i = 0; i < 4; ++i)
-                                    if (m0 + q * 32 + 8 * i + (lane >> 2) < p.m) atomicAdd(t + 32 * i, sums[32 * i + lane]);
+                                for (int i = 0; i < kTerms; ++i)
+                                    if (m0 + q * 32 + (32 * i + lane) / kTerms < p.m) atomicAdd(t + 32 * i, sums[32 * i + lane]);
                             }
                         } else if (row_ok) {
 #pragma unroll
-                            for (int vv = 0; vv < 3; ++vv)
+                            for (int vv = 0; vv < kTerms - 1; ++vv)
                                 if (vv < p.next_nvec) atomicAdd(p.next_t + static_cast<size_t>(row) * p.next_nvec + vv, a4[vv]);
                         }
                     }
@@ -1196,7 +1188,9 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
     if (sms <= 0) return BNF4_ERR_CUDA;
     const bool gelu = p.epilogue == EPI_GELU_FP4 || p.epilogue == EPI_GELU_I8;
     const bool gelu_plain = !gelu || ((p.n % 32) == 0 && (p.epilogue == EPI_GELU_FP4 ? (p.next_nvec == 1 && p.d_i8 == nullptr) : p.next_nvec <= 1));
-    const int rk = p.rank == 4 && (p.rows_per_member % 16) == 0 ? 4 : ((p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1)) ? 1 : (p.rank > 0 ? 2 : 0));
+    const bool plain = p.rank == 1 && p.beta == 0.0f && p.rows_per_member > 0 && (p.rows_per_member % BM) == 0 && (p.m % BM) == 0 && gelu_plain && (p.epilogue != EPI_F16 || p.n - p.n_f16 <= 1);
+    const int rk = p.rank == 0 ? 0 : plain ? 1 : p.rank <= 2 && (p.epilogue != EPI_GELU_FP4 || p.next_nvec <= 2) ? 2 : 4;
+    const int form = (p.rank == 2 || p.rank == 4) && rk == p.rank && (p.rows_per_member % 16) == 0 ? rk + 1 : rk;  // 32 rows lie in one pair
     // CTA pairs pay where the mainloop is longer than the epilogue. Measured at 65536 x 512, before the pairs' copies moved to their K steps (us, single
     // CTAs -> pairs): fp32 / half / residual epilogues, rank 1: K 512 33.9 -> 35.9, 25.6 -> 27.0, 29.0 -> 29.8; K 1024 42.7 -> 38.2,
     // 33.1 -> 30.2, 36.1 -> 33.1; K 4096 107 -> 80, 96 -> 70, 98 -> 74. Rank 4 with the last two: K 1024 37.2 -> 39.2, 43.3 -> 45.4, K 1536
@@ -1217,7 +1211,14 @@ int gemm_nvfp4_launch(const GemmParams& p, cudaStream_t stream) {
                       3.0f + waves_us(pair_tiles, std::max(1, sms / 2), 0.6f, 2.0f * epi_us) < waves_us(tiles, sms, 0.44f, epi_us);
     // the epilogue and the form of the rank term are template arguments
     auto with_rank = [&](auto run) -> int {
-        return rk == 4 ? run(std::integral_constant<int, 4>()) : rk == 1 ? run(std::integral_constant<int, 1>()) : rk == 2 ? run(std::integral_constant<int, 2>()) : run(std::integral_constant<int, 0>());
+        switch (form) {
+            case 0: return run(std::integral_constant<int, 0>());
+            case 1: return run(std::integral_constant<int, 1>());
+            case 2: return run(std::integral_constant<int, 2>());
+            case 3: return run(std::integral_constant<int, 3>());
+            case 4: return run(std::integral_constant<int, 4>());
+        }
+        return run(std::integral_constant<int, 5>());
     };
     auto with_epilogue = [&](auto run) -> int {
         switch (p.epilogue) {
