@@ -442,13 +442,14 @@ __device__ __forceinline__ void project_rows(const RowQuantParams& p, const int4
 // loads, without them the bytes are widened a second time. 65536 rows, us:
 //   floats kept -> bytes kept, 2 / 3 blocks an SM: int8 rows, 2048 columns, 16 projections 153 -> 136 / 140, 4 projections 126 -> 99 / 100,
 //     1024 columns 55 -> 53 / 52; + position / GELU, 1024 columns 137 -> 122 / 124, 2048 columns, 16 projections 344 -> 347 / 393;
-//     + branch, 2048 columns, 4 projections 160 -> 165 / 148, 1024 columns, 1 projection 67 -> 70 / 71
+//     + branch, 1024 columns, 1 projection 67 -> 70 / 71, 2048 columns, 4 projections 160 -> 165 / 148, but 4000 such rows 17.8 -> 19.6
 //   floats kept, 2 / 3 blocks: + position / GELU, 2048 columns, 4 projections 257 / 261 (one block: 294, with 16-byte loads).
-//     fp32 rows past 1024 columns stay at one block: three take 65536 x 2048 from 186 to 154, but 4000 x 1984 from 16 to 20
+//     fp32 rows past 1024 columns stay at one block: three take 65536 x 2048 from 186 to 154, but 4000 x 1984 from 16 to 20.
+// Dearer: 1500 rows of 2048 bytes 5.7 -> 6.1 (4000: 13.7 -> 12.7), 1500 x 768 + position / GELU 7.7 -> 8.1 (65536 x 1024: 139 -> 114).
 template <int FE, int NB, int NV>
-constexpr bool kKeepBytes = NB > 1 && (FE == FE_ABSMEAN || (FE == FE_POS_GELU_ABSMEAN && NB <= 2) || (FE == FE_ADD_ABSMEAN && NB > 2 && NV <= 4));
+constexpr bool kKeepBytes = NB > 1 && (FE == FE_ABSMEAN || (FE == FE_POS_GELU_ABSMEAN && NB <= 2));
 template <int FE, int NB, int NV>
-constexpr int kFastCtas = NB <= 1 ? 4 : kKeepBytes<FE, NB, NV> ? (FE == FE_ADD_ABSMEAN ? 3 : 2) : (NB <= 2 || NV > 4 || FE == FE_POS_GELU_ABSMEAN) ? 2 : 1;
+constexpr int kFastCtas = NB <= 1 ? 4 : kKeepBytes<FE, NB, NV> ? 2 : (NB <= 2 || NV > 4 || FE == FE_POS_GELU_ABSMEAN) ? 2 : 1;
 
 // MODEL: powers of two for rows per member, columns and positions, 32-byte aligned rows, one or four projections: no test or division for any of it
 // (the 32-byte rule: 262144 x 512 + position / GELU 198 -> 191 us).
@@ -605,7 +606,12 @@ __global__ void __launch_bounds__(256, kFastCtas<FE, NB, NV>) rowquant_fast_kern
                 if (MODEL || p.in_f16) {  // the branch output as IEEE halves (exact widening)
                     const uint4* yh = reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(p.in_f32) + static_cast<size_t>(row) * p.ld_in + k0);
                     uint4 h0, h1;
-                    load8(yh, wide, h0, h1);
+                    if constexpr (NB > 2) {  // (as below)
+                        h0 = __ldcs(yh);
+                        h1 = __ldcs(yh + 1);
+                    } else {
+                        load8(yh, wide, h0, h1);
+                    }
                     const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
@@ -614,7 +620,14 @@ __global__ void __launch_bounds__(256, kFastCtas<FE, NB, NV>) rowquant_fast_kern
                     }
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 4; q += 2) load8(yr + k0 + 4 * q, wide, y4[q], y4[q + 1]);
+                    for (int q = 0; q < 4; q += 2) {
+                        if constexpr (NB > 2) {  // streaming loads: 4000 x 2048 from DRAM 14.9 us, 15.3 with the 32-byte ones (halves, 4 projections: 17.8, 20.6)
+                            y4[q] = __ldcs(reinterpret_cast<const float4*>(yr + k0 + 4 * q));
+                            y4[q + 1] = __ldcs(reinterpret_cast<const float4*>(yr + k0 + 4 * q) + 1);
+                        } else {
+                            load8(yr + k0 + 4 * q, wide, y4[q], y4[q + 1]);
+                        }
+                    }
                 }
                 uint32_t upd[4];
 #pragma unroll
