@@ -689,13 +689,13 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
 #pragma unroll
             for (int e = 0; e < 8; ++e)
                 *reinterpret_cast<float4*>(out + t_row * 64 + (((8 * half + e) ^ (t_row & 15)) << 2)) = make_float4(y[4 * e], y[4 * e + 1], y[4 * e + 2], y[4 * e + 3]);
+            // across: y may lie on other columns of v and leaves when the next three tiles have been read or are here. The last of them is waited for in front of this
+            // arrival: without it no warp reads that tile, so that the copy after next, which would complete the same barrier once more, cannot pass the wait.
+            if (across && l + 3 < nct) ok = ok && mbar_wait(bar_v + 8 * ((l + 3) & 1), static_cast<uint32_t>((l + 3) / 2) & 1u, 28);
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_drain + 8 * (l & 1));
             group_sync();
-            if (across) {  // y may lie on other columns of v: it leaves when the next three tiles have been read or are here
-                if (l + 2 < nct) ok = ok && mbar_wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2 + 1) & 1u, 29);
-                if (l + 3 < nct) ok = ok && mbar_wait(bar_v + 8 * ((l + 3) & 1), static_cast<uint32_t>((l + 3) / 2) & 1u, 28);
-            }
+            if (across && l + 2 < nct) ok = ok && mbar_wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2 + 1) & 1u, 29);
             if (wide) {
                 const int piece = gtid & 15, c = (ct0 + l) * 64 + 4 * piece;
 #pragma unroll 4

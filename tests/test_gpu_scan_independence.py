@@ -54,6 +54,32 @@ def test_closed_form_in_place(H, hidden, heads, seqs, T, where):
     assert torch.equal(rows, apart) and torch.equal(buffers, apart)
 
 
+# wide rows (q | k | v | room), and rows of v alone that are narrower than two outputs, so that a row of y ends on the next row of v
+@pytest.mark.parametrize("ld,shift", [(2048, 6), (2048, 64), (2048, 100), (2048, 128), (2048, 192), (2048, -8), (2048, -100), (576, 96), (640, 160)])
+@pytest.mark.parametrize("seqs,T", [(1, 128), (1, 33), (200, 128)])
+def test_closed_form_across_v(H, ld, shift, seqs, T):
+    """One head of eight column tiles whose output lies on other columns of v."""
+    import torch
+    hidden = 512
+    if ld < 2 * hidden and seqs > 1:
+        pytest.skip("a sequence's last row lies on the next sequence")
+    rng = np.random.default_rng(1000 + T + shift)
+    qkv = [torch.from_numpy((rng.standard_normal((seqs * T + 1, ld)) * 0.3).astype(np.float32)).cuda() for _ in range(3)]
+    beta = torch.from_numpy(rng.standard_normal(seqs * T).astype(np.float32)).cuda()
+
+    def scan(v, out, ld_out):
+        H.efla_scan(state=None, state_fp16=1, q=qkv[0], k=qkv[1], v=v, beta_raw=beta, ld_qkv=ld, ld_beta=1, beta_bias=-2.0, seqs_per_bias=1, hidden=hidden, heads=1, seqs=seqs, T=T,
+                    method=1, eps=1e-6, out=out, ld_out=ld_out, variant=0)
+        assert H.device_error() == 0
+
+    first = 512 if ld >= 2 * hidden else 0  # column of v
+    apart = torch.empty(seqs * T, hidden, device="cuda")
+    scan(qkv[2][:, first:], apart, hidden)
+    out = qkv[2].view(-1)[first + shift:]
+    scan(qkv[2][:, first:], out, ld)
+    assert torch.equal(torch.as_strided(out, (seqs * T, hidden), (ld, 1)), apart)
+
+
 @pytest.mark.parametrize("hidden,heads,method", [(96, 1, 1), (512, 8, 1), (128, 4, 0)])
 def test_other_scans(H, hidden, heads, method):
     """One CTA (128-token blocks) or one warp per unit, whatever their number."""
