@@ -45,6 +45,10 @@ namespace bnf4 {
 
 namespace {
 
+// How the output lies to q, k or v: apart from it (also in other columns of the same rows), exactly in its place, in the same rows and by less than its width to
+// the right, or in some other way.
+enum SeqOverlap { SEQ_APART, SEQ_SAME, SEQ_RIGHT, SEQ_ACROSS };
+
 constexpr int kSeqMaxT = 128;
 constexpr int kSeqThreads = 512;
 constexpr int kSqThreads = kSeqThreads + 64;       // efla_seq_kernel: sixteen warps that work, one that issues the products of steps 1 and 5, one the loads
@@ -255,7 +259,7 @@ __device__ __forceinline__ void sq_tmem_ld16(uint32_t taddr, float (&r)[16]) {
 }
 
 // cs CTAs share a unit: each does steps 1 to 4 (the same sums) and its share of the column tiles of step 5. meet: they form a cluster, and none writes
-// before all have read q and k, where the output may lie. across: it may lie on v, on other columns.
+// before all have read q and k, where the output may lie. across: it may lie on v, on other columns (SeqOverlap).
 __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                                                                  const __grid_constant__ CUtensorMap map_v, const EflaParams p, const int cs, const int meet, const int across) {
     pdl_wait();
@@ -341,10 +345,12 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
         s = fmaf(x.x, x.x, s); s = fmaf(x.y, x.y, s); s = fmaf(x.z, x.z, s);
         return fmaf(x.w, x.w, s);
     };
+    // An output to the right of v is formed from the last column tile to the first: a tile then lies on columns that have been read, however far to the right.
+    auto tile_col = [&](int l) { return (ct0 + (across == SEQ_RIGHT ? nct - 1 - l : l)) * 64; };
     int v_loads = 0;
     auto load_v = [&](int l) {  // (the loading warp) the CTA's l-th tile of V: two boxes of 32 columns, or the one that is left
         const uint32_t at = sm0 + ((l & 1) ? kSqV1 : kSqV0);
-        const int c = (ct0 + l) * 64;
+        const int c = tile_col(l);
         if (elect_one()) {
             const bool two = c + 32 < hd;
             mbar_expect_tx(bar_v + 8 * (l & 1), (two ? 2 : 1) * kSqUTile);
@@ -611,7 +617,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
         for (int l = 0; l < nct; ++l) {
             float4 v[kPer];
             ok = ok && mbar_wait(bar_v + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 28);
-            const int c = (ct0 + l) * 64 + 4 * piece;
+            const int c = tile_col(l) + 4 * piece;
             const uint8_t* raw = sm + ((l & 1) ? kSqV1 : kSqV0) + (piece >> 3) * kSqUTile + srow * 128 + (((piece & 7) ^ (srow & 7)) << 4);
 #pragma unroll
             for (int i = 0; i < kPer; ++i)
@@ -689,20 +695,20 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
 #pragma unroll
             for (int e = 0; e < 8; ++e)
                 *reinterpret_cast<float4*>(out + t_row * 64 + (((8 * half + e) ^ (t_row & 15)) << 2)) = make_float4(y[4 * e], y[4 * e + 1], y[4 * e + 2], y[4 * e + 3]);
-            // across: y may lie on other columns of v and leaves when the next three tiles have been read or are here. The last of them is waited for in front of this
+            // SEQ_ACROSS: y may lie on other columns of v and leaves when the next three tiles have been read or are here. The last of them is waited for in front of this
             // arrival: without it no warp reads that tile, so that the copy after next, which would complete the same barrier once more, cannot pass the wait.
-            if (across && l + 3 < nct) ok = ok && mbar_wait(bar_v + 8 * ((l + 3) & 1), static_cast<uint32_t>((l + 3) / 2) & 1u, 28);
+            if (across == SEQ_ACROSS && l + 3 < nct) ok = ok && mbar_wait(bar_v + 8 * ((l + 3) & 1), static_cast<uint32_t>((l + 3) / 2) & 1u, 28);
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_drain + 8 * (l & 1));
             group_sync();
-            if (across && l + 2 < nct) ok = ok && mbar_wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2 + 1) & 1u, 29);
+            if (across == SEQ_ACROSS && l + 2 < nct) ok = ok && mbar_wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2 + 1) & 1u, 29);
             if (wide) {
-                const int piece = gtid & 15, c = (ct0 + l) * 64 + 4 * piece;
+                const int piece = gtid & 15, c = tile_col(l) + 4 * piece;
 #pragma unroll 4
                 for (int t = gtid >> 4; t < T; t += kSeqThreads / 32)
                     if (ok && c < hd) *reinterpret_cast<float4*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float4*>(out + t * 64 + ((piece ^ (t & 15)) << 2));
             } else {
-                const int c = (ct0 + l) * 64 + 2 * lane;
+                const int c = tile_col(l) + 2 * lane;
                 for (int t = warp - kGroup; t < T; t += kGroup)
                     if (ok && c < hd) *reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float2*>(out + t * 64 + (((lane >> 1) ^ (t & 15)) << 2) + 2 * (lane & 1));
             }
@@ -1063,8 +1069,6 @@ static bool seq_ranges_apart(const EflaParams& p, const void* in) {
     const char *o = static_cast<const char*>(p.out), *a = static_cast<const char*>(in);
     return o >= a + (last * p.ld_qkv + p.hidden) * sizeof(float) || a >= o + (last * p.ld_out + p.hidden) * sizeof(float);
 }
-// How the output lies to q, k or v: apart from it (also in other columns of the same rows), exactly in its place, or in some other way.
-enum SeqOverlap { SEQ_APART, SEQ_SAME, SEQ_ACROSS };
 static SeqOverlap seq_overlap(const EflaParams& p, const void* in) {
     if (seq_ranges_apart(p, in)) return SEQ_APART;
     if (p.ld_out != p.ld_qkv) return SEQ_ACROSS;
@@ -1072,7 +1076,7 @@ static SeqOverlap seq_overlap(const EflaParams& p, const void* in) {
     const long long row = static_cast<long long>(p.ld_qkv) * sizeof(float), width = static_cast<long long>(p.hidden) * sizeof(float);
     if (row < 2 * width) return SEQ_ACROSS;
     const long long d = ((static_cast<long long>(reinterpret_cast<intptr_t>(p.out)) - static_cast<long long>(reinterpret_cast<intptr_t>(in))) % row + row) % row;
-    return d >= width && row - d >= width ? SEQ_APART : SEQ_ACROSS;
+    return d < width ? SEQ_RIGHT : row - d < width ? SEQ_ACROSS : SEQ_APART;
 }
 
 // The closed form's work per token grows with the sequence, the per-token kernel's does not, but the latter spreads a unit over several SMs. One head of
@@ -1117,9 +1121,9 @@ int efla_seq_launch(const EflaParams& p, cudaStream_t stream) {
     const int sms = multiprocessors(dev), nd = (p.hidden / p.heads + 63) >> 6;
     if (sms <= 0) return BNF4_ERR_CUDA;
     const bool meet = seq_overlap(p, p.q) != SEQ_APART || seq_overlap(p, p.k) != SEQ_APART;
-    const int cs = seq_overlap(p, p.v) == SEQ_ACROSS ? 1 : units * 4 <= (meet ? sms * 7 / 8 : sms) && nd >= 4 ? 4 : units * 2 <= sms && nd >= 2 ? 2 : 1;
+    const SeqOverlap across = seq_overlap(p, p.v);
+    const int cs = across == SEQ_RIGHT || across == SEQ_ACROSS ? 1 : units * 4 <= (meet ? sms * 7 / 8 : sms) && nd >= 4 ? 4 : units * 2 <= sms && nd >= 2 ? 2 : 1;
     const bool early = p.seqs * static_cast<long long>(p.T) * p.hidden <= kPdlStreamElems;
-    const int across = seq_overlap(p, p.v) == SEQ_ACROSS;
     CUtensorMap maps[3];  // boxes of 128 tokens and 32 columns
     const void* in[3] = {p.q, p.k, p.v};
     for (int i = 0; i < 3; ++i) {
@@ -1141,9 +1145,9 @@ int efla_seq_launch(const EflaParams& p, cudaStream_t stream) {
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = early ? 2 : 1;
-        cudaLaunchKernelEx(&cfg, efla_seq_kernel, maps[0], maps[1], maps[2], p, cs, 1, across);  // errors surface in check_launch
+        cudaLaunchKernelEx(&cfg, efla_seq_kernel, maps[0], maps[1], maps[2], p, cs, 1, static_cast<int>(across));  // errors surface in check_launch
     } else {
-        launch_pdl_if(early, efla_seq_kernel, static_cast<unsigned>(units * cs), kSqThreads, kSqSmem, stream, maps[0], maps[1], maps[2], p, cs, 0, across);
+        launch_pdl_if(early, efla_seq_kernel, static_cast<unsigned>(units * cs), kSqThreads, kSqSmem, stream, maps[0], maps[1], maps[2], p, cs, 0, static_cast<int>(across));
     }
     return check_launch("efla_seq_kernel");
 }

@@ -55,7 +55,7 @@ def test_closed_form_in_place(H, hidden, heads, seqs, T, where):
 
 
 # wide rows (q | k | v | room), and rows of v alone that are narrower than two outputs, so that a row of y ends on the next row of v
-@pytest.mark.parametrize("ld,shift", [(2048, 6), (2048, 64), (2048, 100), (2048, 128), (2048, 192), (2048, -8), (2048, -100), (576, 96), (640, 160)])
+@pytest.mark.parametrize("ld,shift", [(2048, 6), (2048, 64), (2048, 100), (2048, 128), (2048, 192), (2048, 256), (2048, 450), (2048, -8), (2048, -100), (576, 96), (640, 160)])
 @pytest.mark.parametrize("seqs,T", [(1, 128), (1, 33), (200, 128)])
 def test_closed_form_across_v(H, ld, shift, seqs, T):
     """One head of eight column tiles whose output lies on other columns of v."""
