@@ -287,6 +287,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
     float* b_sh = a_sh + kSeqMaxT;
     float* red = reinterpret_cast<float*>(sm + kSqRed);
     int* red_bad = reinterpret_cast<int*>(red + 48);  // [4]
+    volatile int* stop = reinterpret_cast<volatile int*>(red + 52);
     float* part = reinterpret_cast<float*>(sm + kSqPart);
     // mbarriers: slots of K and Q filled / read (four each), halves of the operands complete / multiplied (two each), tiles of V filled / read (two each), operands of V
     // complete, tiles of y complete / read (two each)
@@ -295,6 +296,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(sm + kSqBar + 192);
     constexpr int kGroup = kSeqThreads / 64;  // warps of one of the two groups that share steps 1 and 5
     if (tid == 0) {
+        *stop = 0;
         for (int b = 0; b < 4; ++b) { mbar_init(bar_raw + 8 * b, 1); mbar_init(bar_read + 8 * b, kGroup); }
         for (int b = 0; b < 2; ++b) {
             mbar_init(bar_op + 8 * b, kGroup);
@@ -311,7 +313,15 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
         tmem_alloc(bar0 + 192, kSqTmemCols);
         tmem_relinquish();
     }
-    bool ok = true;  // no wait of this thread has expired; behind one that has there are no others, and what the thread would write stays unwritten
+    // No wait of this thread has expired; behind one that has there are no others. `stop` tells the other threads: what follows an expired wait, whichever warp's, may
+    // rest on operands that never came, and stays unwritten. (It is set in front of the arrivals that lead there, and read behind them.)
+    bool ok = true;
+    auto wait = [&](uint32_t bar, uint32_t parity, int code) {
+        if (ok && !mbar_wait(bar, parity, code)) {
+            ok = false;
+            *stop = 1;
+        }
+    };
 
     tc_fence_before();
     __syncthreads();
@@ -370,7 +380,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
             float ss[2] = {0.0f, 0.0f}, sc[2];  // k, q
             for (int hb = group; hb < nh; hb += 2) {
                 const int it = it0 + hb, slot = it & 3, half = it & 1;
-                ok = ok && mbar_wait(bar_raw + 8 * slot, static_cast<uint32_t>(it >> 2) & 1u, 26);
+                wait(bar_raw + 8 * slot, static_cast<uint32_t>(it >> 2) & 1u, 26);
                 const uint8_t* raw = sm + kSqRaw + slot * (2 * kSqUTile) + t_row * 128;
                 float4 x[2][4];
 #pragma unroll
@@ -398,7 +408,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
                         if (group == 0 && ch == 0) scale_sh[(1 - m) * kSeqMaxT + t_row] = sc[m];
                     }
                 }
-                if (it >= 2) ok = ok && mbar_wait(bar_mul + 8 * half, static_cast<uint32_t>(it / 2 - 1) & 1u, 21);  // the half's last products have read it
+                if (it >= 2) wait(bar_mul + 8 * half, static_cast<uint32_t>(it / 2 - 1) & 1u, 21);  // the half's last products have read it
                 __syncwarp();
                 tc_fence_after();
                 if (32 * quad < 16 * nb) {
@@ -440,7 +450,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
             const uint32_t gram = kSqIdesc | (static_cast<uint32_t>(2 * nb) << 17);  // N 16 nb
             for (int hb = 0; hb < nh; ++hb) {
                 const int it = it0 + hb, half = it & 1;
-                ok = ok && mbar_wait(bar_op + 8 * half, static_cast<uint32_t>(it / 2) & 1u, 24);
+                wait(bar_op + 8 * half, static_cast<uint32_t>(it / 2) & 1u, 24);
                 if (elect_one() && ok) {
                     tc_fence_after();
 #pragma unroll
@@ -461,7 +471,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
         } else {
             for (int hb = 0; hb < nh; ++hb) {
                 const int it = it0 + hb, slot = it & 3;
-                if (it >= 4) ok = ok && mbar_wait(bar_read + 8 * slot, static_cast<uint32_t>(it / 4 - 1) & 1u, 27);
+                if (it >= 4) wait(bar_read + 8 * slot, static_cast<uint32_t>(it / 4 - 1) & 1u, 27);
                 if (!__all_sync(0xffffffffu, ok)) break;
                 if (elect_one()) {
                     const uint32_t at = sm0 + kSqRaw + slot * (2 * kSqUTile);
@@ -474,7 +484,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
                 if (pass == 0 && hb == min(3, nh - 1)) load_v(0);
             }
         }
-        for (int it = max(0, it0 + nh - 2); it < it0 + nh; ++it) ok = ok && mbar_wait(bar_mul + 8 * (it & 1), static_cast<uint32_t>(it / 2) & 1u, 22);
+        for (int it = max(0, it0 + nh - 2); it < it0 + nh; ++it) wait(bar_mul + 8 * (it & 1), static_cast<uint32_t>(it / 2) & 1u, 22);
         tc_fence_after();
         __syncthreads();  // (everyone has seen the products done before their operands' places are taken)
         bool again = false;
@@ -616,7 +626,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
         constexpr int kRows = kSeqThreads / 32, kPer = kSeqMaxT / kRows;
         for (int l = 0; l < nct; ++l) {
             float4 v[kPer];
-            ok = ok && mbar_wait(bar_v + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 28);
+            wait(bar_v + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 28);
             const int c = tile_col(l) + 4 * piece;
             const uint8_t* raw = sm + ((l & 1) ? kSqV1 : kSqV0) + (piece >> 3) * kSqUTile + srow * 128 + (((piece & 7) ^ (srow & 7)) << 4);
 #pragma unroll
@@ -632,7 +642,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
                 redb[warp] = m;
                 mbar_arrive(bar_vread + 8 * (l & 1));  // (the tile has been read: its values are in m)
             }
-            if (l >= 2) ok = ok && mbar_wait(bar_drain + 8 * (l & 1), static_cast<uint32_t>(l / 2 - 1) & 1u, 27);  // the tile before the last has left its accumulator (and its product the operands)
+            if (l >= 2) wait(bar_drain + 8 * (l & 1), static_cast<uint32_t>(l / 2 - 1) & 1u, 27);  // the tile before the last has left its accumulator (and its product the operands)
             group_sync();
             m = __reduce_max_sync(0xffffffffu, redb[lane & 7]);
             const bool tile_bad = m >= kSeqNonFinite;
@@ -673,10 +683,10 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
         float* out = reinterpret_cast<float*>(sm + kSqOut);
         const int half = ch, gtid = tid - 32 * kGroup;
         for (int l = 0; l < nct; ++l) {
-            ok = ok && mbar_wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 29);
+            wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 29);
             const float ds = ds_sh[l & 1];
             const bool tile_bad = bad_sh[l & 1] != 0;
-            ok = ok && mbar_wait(bar_y + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 23);
+            wait(bar_y + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 23);
             __syncwarp();
             tc_fence_after();
             uint32_t acc[32];
@@ -697,25 +707,26 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
                 *reinterpret_cast<float4*>(out + t_row * 64 + (((8 * half + e) ^ (t_row & 15)) << 2)) = make_float4(y[4 * e], y[4 * e + 1], y[4 * e + 2], y[4 * e + 3]);
             // SEQ_ACROSS: y may lie on other columns of v and leaves when the next three tiles have been read or are here. The last of them is waited for in front of this
             // arrival: without it no warp reads that tile, so that the copy after next, which would complete the same barrier once more, cannot pass the wait.
-            if (across == SEQ_ACROSS && l + 3 < nct) ok = ok && mbar_wait(bar_v + 8 * ((l + 3) & 1), static_cast<uint32_t>((l + 3) / 2) & 1u, 28);
+            if (across == SEQ_ACROSS && l + 3 < nct) wait(bar_v + 8 * ((l + 3) & 1), static_cast<uint32_t>((l + 3) / 2) & 1u, 28);
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_drain + 8 * (l & 1));
+            if (across == SEQ_ACROSS && l + 2 < nct) wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2 + 1) & 1u, 29);
             group_sync();
-            if (across == SEQ_ACROSS && l + 2 < nct) ok = ok && mbar_wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2 + 1) & 1u, 29);
+            const bool write = *stop == 0;  // (no way out of the loop: threads that read it before and after it is set would part at the barriers)
             if (wide) {
                 const int piece = gtid & 15, c = tile_col(l) + 4 * piece;
 #pragma unroll 4
                 for (int t = gtid >> 4; t < T; t += kSeqThreads / 32)
-                    if (ok && c < hd) *reinterpret_cast<float4*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float4*>(out + t * 64 + ((piece ^ (t & 15)) << 2));
+                    if (write && c < hd) *reinterpret_cast<float4*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float4*>(out + t * 64 + ((piece ^ (t & 15)) << 2));
             } else {
                 const int c = tile_col(l) + 2 * lane;
                 for (int t = warp - kGroup; t < T; t += kGroup)
-                    if (ok && c < hd) *reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float2*>(out + t * 64 + (((lane >> 1) ^ (t & 15)) << 2) + 2 * (lane & 1));
+                    if (write && c < hd) *reinterpret_cast<float2*>(og + static_cast<size_t>(t) * p.ld_out + c) = *reinterpret_cast<const float2*>(out + t * 64 + (((lane >> 1) ^ (t & 15)) << 2) + 2 * (lane & 1));
             }
         }
     } else if (warp == 16) {
         for (int l = 0; l < nct; ++l) {
-            ok = ok && mbar_wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 25);
+            wait(bar_vop + 8 * (l & 1), static_cast<uint32_t>(l / 2) & 1u, 25);
             if (elect_one() && ok) {
                 tc_fence_after();
                 const uint32_t at = sm0 + (l & 1) * (2 * kSqUTile), d = tmem + (l & 1) * 64, ta = tmem + kSqTA;
@@ -732,7 +743,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
         }
     } else {
         for (int l = 1; l < nct; ++l) {
-            if (l >= 2) ok = ok && mbar_wait(bar_vread + 8 * (l & 1), static_cast<uint32_t>(l / 2 - 1) & 1u, 29);
+            if (l >= 2) wait(bar_vread + 8 * (l & 1), static_cast<uint32_t>(l / 2 - 1) & 1u, 29);
             if (!__all_sync(0xffffffffu, ok)) break;
             load_v(l);
         }
