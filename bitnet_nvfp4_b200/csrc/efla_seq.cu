@@ -489,9 +489,10 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
         __syncthreads();  // (everyone has seen the products done before their operands' places are taken)
         bool again = false;
         if (pass == 0 && tid < T) {
-            auto leaves = [](float sum, float s) {  // a scaled value may be beyond 2^15, or all are too small
+            // A scaled value may be beyond 2^15, or all are too small. Squares of values below 2^-75 are lost: these stay below 2^15 under scales of up to 2^90.
+            auto leaves = [](float sum, float s) {
                 const float v = sum * s * s;
-                return sum > 0.0f && !(v >= 0.0625f && v <= 1073741824.0f);
+                return sum > 0.0f ? !(v >= 0.0625f && v <= 1073741824.0f) : s > 0x1p90f;
             };
             again = leaves(norm2(0, tid), scale_sh[tid]) || leaves(norm2(1, tid), scale_sh[kSeqMaxT + tid]);
         }

@@ -25,7 +25,8 @@ def recurrence(q, k, v, logit, method, eps):
 
 @pytest.mark.parametrize("method", [1, 0])
 @pytest.mark.parametrize("T,hd,kind", [(128, 512, "plain"), (1, 64 + 32, "plain"), (17, 160, "plain"), (113, 288, "plain"), (40, 512, "grow"), (128, 96, "grow"), (40, 320, "shrink"),
-                                       (33, 512, "zero first"), (50, 224, "zero rows"), (64, 512, "large"), (64, 512, "small"), (128, 128, "one row")])
+                                       (33, 512, "zero first"), (50, 224, "zero rows"), (64, 512, "large"), (64, 512, "small"), (128, 128, "one row"),
+                                       (64, 512, "tiny q"), (64, 512, "tiny k"), (40, 96, "tiny q"), (40, 96, "tiny k"), (33, 512, "tinier first"), (33, 512, "tiny")])
 def test_scales(T, hd, kind, method):
     import torch
     from bitnet_nvfp4_b200 import host
@@ -47,6 +48,18 @@ def test_scales(T, hd, kind, method):
         q, k = q * 1e15, k * 1e15
     elif kind == "small":
         q, k = q * 1e-5, k * 1e-17
+    elif kind == "tiny q":  # squares that underflow, behind a scale of 2^107
+        q[:, 1::4] *= 1e-24
+        q[:, 1::4, :32] *= 1e-6
+    elif kind == "tiny k":
+        k[:, ::3] *= 1e-24
+        k[:, ::3, :32] *= 1e-6
+    elif kind == "tinier first":
+        q[:, 1::4, :32] *= 1e-30
+        k[:, ::3, :32] *= 1e-30
+    elif kind == "tiny":
+        q[:, 1::4] *= 1e-36
+        k[:, ::3] *= 1e-36
     elif kind == "one row":
         q[1, 100, 70] = 3e4  # (out of the range of the first columns' scale)
         k[2, 64, 127] = -7e5
