@@ -9,8 +9,8 @@
 // multiplies it with V: 2 T^2 hd multiply-adds per sequence instead of the 3 T hd^2 of the state form (six times fewer at
 // T = 128, hd = 512), every input read once, no state, no scratch.
 //
-// Precision: every operand is split into two fp16 terms (x = hi + mid, 22 significant bits; rows are normalised and scaled by powers of
-// two first so that neither term under- or overflows) and the products hi hi + hi mid + mid hi accumulate in fp32. Nothing is
+// Precision: every operand is split into two fp16 terms (x = hi + mid, 22 significant bits; rows of q and k are scaled by powers of
+// two first, to a norm of 2^6 or more and values below 2^15, so that neither term under- or overflows) and the products hi hi + hi mid + mid hi accumulate in fp32. Nothing is
 // rounded to fp16 between tokens, so the result lies closer to exact arithmetic than the per-token form's fp16 state.
 //
 // Values that are no numbers stay where the recurrence has them, although 0 x NaN is NaN in a contraction: from the first token on whose k or beta
@@ -489,10 +489,11 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
         __syncthreads();  // (everyone has seen the products done before their operands' places are taken)
         bool again = false;
         if (pass == 0 && tid < T) {
-            // A scaled value may be beyond 2^15, or all are too small. Squares of values below 2^-75 are lost: these stay below 2^15 under scales of up to 2^90.
+            // A scaled value may be beyond 2^15, or the row is below 2^6, where the mid halves run out of bits (first columns that are not zero make it 2^7 at least). Squares of
+            // values below 2^-75 are lost: these stay below 2^15 under scales of up to 2^90.
             auto leaves = [](float sum, float s) {
                 const float v = sum * s * s;
-                return sum > 0.0f ? !(v >= 0.0625f && v <= 1073741824.0f) : s > 0x1p90f;
+                return sum > 0.0f ? !(v >= 4096.0f && v <= 1073741824.0f) : s > 0x1p90f;
             };
             again = leaves(norm2(0, tid), scale_sh[tid]) || leaves(norm2(1, tid), scale_sh[kSeqMaxT + tid]);
         }

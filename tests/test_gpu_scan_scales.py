@@ -74,6 +74,31 @@ def test_scales(T, hd, kind, method):
     assert (err <= 2.0 ** -17 * want.abs().amax((1, 2))).all(), (err / want.abs().amax((1, 2))).tolist()
 
 
+@pytest.mark.parametrize("norm", [0.01, 0.26, 0.9, 20.0])
+@pytest.mark.parametrize("T,hd", [(33, 512), (128, 256), (64, 96), (50, 224)])
+def test_zeros_first_cost_no_bits(T, hd, norm):
+    """Rows whose first 32 columns are zero are off by what the same rows with these columns last are off by: the products are the same, their
+    sums begin at another column. (Seen: within 5e-5 of each other; 1.5 to 1.8 times as much where rows of norm 0.26 were left unscaled.)"""
+    import torch
+    from bitnet_nvfp4_b200 import host
+    seqs = 24
+    g = torch.Generator(device="cuda").manual_seed(T + hd)
+    q, k, v = (torch.randn(seqs, T, hd, device="cuda", generator=g) for _ in range(3))
+    for x in (q, k):
+        x[..., hd - 32:] = 0
+        x *= norm / x.norm(dim=-1, keepdim=True)
+    logit = torch.randn(seqs, T, device="cuda", generator=g)
+    want = recurrence(q, k, v, logit, 1, 1e-6)
+    err = []
+    for shift in (0, 32):
+        qkv = torch.cat([q.roll(shift, -1), k.roll(shift, -1), v], -1).reshape(seqs * T, 3 * hd).contiguous()
+        out = torch.empty(seqs * T, hd, device="cuda")
+        host.efla_scan(state=None, state_fp16=1, q=qkv, k=qkv[:, hd:], v=qkv[:, 2 * hd:], beta_raw=logit.reshape(-1), ld_qkv=3 * hd, ld_beta=1, beta_bias=0.0, seqs_per_bias=1,
+                       hidden=hd, heads=1, seqs=seqs, T=T, method=1, eps=1e-6, out=out, ld_out=hd, variant=0, qkv_f16=0, out_f16=0)
+        err.append(float((out.reshape(seqs, T, hd).double() - want).norm()))
+    assert err[1] <= 1.01 * err[0], err
+
+
 def test_values_that_are_no_numbers_behind_the_first_columns():
     """An infinite q meets its own row, an infinite k cuts the sequence, a norm that overflows leaves the state alone; rows of other sequences keep their bits."""
     import torch
