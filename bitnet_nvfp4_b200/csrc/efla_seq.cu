@@ -33,6 +33,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include <cfloat>
 #include <cmath>
 
@@ -258,6 +259,26 @@ __device__ __forceinline__ void sq_tmem_ld16(uint32_t taddr, float (&r)[16]) {
         : "memory");
 }
 
+// The largest values of the rows of q and k [2][128], a warp (of sixteen) per row
+__device__ __forceinline__ void seq_row_maxima(const float* qg, const float* kg, int ld, int T, int hd, float* out) {
+    const int lane = threadIdx.x & 31;
+    for (int t = threadIdx.x >> 5; t < T; t += kSeqThreads / 32) {
+        float m[2] = {0.0f, 0.0f};
+        const float *qr = qg + static_cast<size_t>(t) * ld, *kr = kg + static_cast<size_t>(t) * ld;
+#pragma unroll 4
+        for (int c = 4 * lane; c < hd; c += 128) {
+            const float4 x = *reinterpret_cast<const float4*>(qr + c), y = *reinterpret_cast<const float4*>(kr + c);
+            m[0] = fmaxf(m[0], fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
+            m[1] = fmaxf(m[1], fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w))));
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t bits = __reduce_max_sync(0xffffffffu, __float_as_uint(m[i]));
+            if (lane == 0) out[i * kSeqMaxT + t] = __uint_as_float(bits);
+        }
+    }
+}
+
 // cs CTAs share a unit: each does steps 1 to 4 (the same sums) and its share of the column tiles of step 5. meet: they form a cluster, and none writes
 // before all have read q and k, where the output may lie. across: it may lie on v, on other columns (SeqOverlap).
 __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -371,11 +392,14 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
         ++v_loads;
     };
     // The scale of a row is taken from its first 32 columns (largest value just below 2^8), so that q and k are read once; a row that leaves the range of
-    // halves later on, or has only zeros there, sends the whole unit through a second pass with scales from whole rows.
+    // halves later on, or has only zeros there, sends the whole unit through a second pass with scales from whole rows. One head of 512, a row of every unit being
+    // such: 1024 x 128 tokens 277 -> 403 us, 32 x 128 26.4 -> 41.8, 1024 x 33 180 -> 249 (with a thread per row for the largest values 508, 56.7, 295). The passes are
+    // two instances of one body: tests for the pass inside it cost 0.8 us of 17.9 at one token.
     auto norm2 = [&](int m, int t) { return (part[m * kSeqMaxT + t] + part[(2 + m) * kSeqMaxT + t]) + (part[(4 + m) * kSeqMaxT + t] + part[(6 + m) * kSeqMaxT + t]); };
     int loads = 0;  // blocks of K and Q that the loading warp has asked for
-    for (int pass = 0;; ++pass) {
-        const int it0 = pass * nh;  // blocks before this pass: the barriers' phases go on
+    auto step1 = [&](auto second) {  // does a row leave the range?
+        constexpr bool kSecond = decltype(second)::value;
+        const int it0 = kSecond ? nh : 0;  // blocks before this pass: the barriers' phases go on
         if (warp < 16) {
             float ss[2] = {0.0f, 0.0f}, sc[2];  // k, q
             for (int hb = group; hb < nh; hb += 2) {
@@ -393,11 +417,7 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
 #pragma unroll
                         for (int m = 0; m < 2; ++m) {
                             float mx = fmaxf(fmaxf(abs4(x[m][0]), abs4(x[m][1])), fmaxf(abs4(x[m][2]), abs4(x[m][3])));
-                            if (pass > 0 && t_row < T) {
-                                const float* src = (m == 0 ? kg : qg) + static_cast<size_t>(t_row) * p.ld_qkv;
-                                for (int c = 32 + 16 * ch; c < hd; c += 32)
-                                    for (int j = 0; j < 4; ++j) mx = fmaxf(mx, abs4(*reinterpret_cast<const float4*>(src + c + 4 * j)));
-                            }
+                            if (kSecond && t_row < T) mx = fmaxf(mx, scale_sh[(1 - m) * kSeqMaxT + t_row]);
                             qs_sh[(2 * m + ch) * kSeqMaxT + t_row] = mx;
                         }
                     }
@@ -481,14 +501,14 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
                 }
                 __syncwarp();
                 ++loads;
-                if (pass == 0 && hb == min(3, nh - 1)) load_v(0);
+                if (!kSecond && hb == min(3, nh - 1)) load_v(0);
             }
         }
         for (int it = max(0, it0 + nh - 2); it < it0 + nh; ++it) wait(bar_mul + 8 * (it & 1), static_cast<uint32_t>(it / 2) & 1u, 22);
         tc_fence_after();
         __syncthreads();  // (everyone has seen the products done before their operands' places are taken)
         bool again = false;
-        if (pass == 0 && tid < T) {
+        if (!kSecond && tid < T) {
             // A scaled value may be beyond 2^15, or the row is below 2^6, where the mid halves run out of bits (first columns that are not zero make it 2^7 at least). Squares of
             // values below 2^-75 are lost: these stay below 2^15 under scales of up to 2^90.
             auto leaves = [](float sum, float s) {
@@ -497,7 +517,14 @@ __global__ void __launch_bounds__(kSqThreads, 1) efla_seq_kernel(const __grid_co
             };
             again = leaves(norm2(0, tid), scale_sh[tid]) || leaves(norm2(1, tid), scale_sh[kSeqMaxT + tid]);
         }
-        if (pass > 0 || __syncthreads_or(again) == 0) break;
+        return !kSecond && __syncthreads_or(again) != 0;
+    };
+    if (step1(std::false_type())) {
+        if (warp < 16) {
+            seq_row_maxima(qg, kg, p.ld_qkv, T, hd, scale_sh);
+            workers_sync();
+        }
+        step1(std::true_type());
     }
 
     // ---------------- 2. scalars of the tokens ----------------
