@@ -413,6 +413,7 @@ constexpr int kQuantBlockTabBytes = 128 * 8;
 constexpr int kQuantLutBytes = kQuantBlockTabOffset + kQuantBlockTabBytes;
 // Device pointer to the table of the current device (allocated and filled on first use); nullptr + error on failure.
 const uint8_t* get_quant_lut();
+bool fill_quant_lut(uint8_t* table);  // on the host, kQuantLutBytes
 
 __device__ __forceinline__ void quant_block16_lut(const int (&a)[16], const uint8_t* __restrict__ lut, uint32_t& sf_byte,
                                                   uint32_t& code_lo, uint32_t& code_hi) {

@@ -15,13 +15,8 @@ std::mutex g_lut_mu;
 uint8_t* g_lut[64] = {};
 }  // namespace
 
-const uint8_t* get_quant_lut() {
-    int dev = 0;
-    if (check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return nullptr;
-    if (dev < 0 || dev >= 64) { set_error(BNF4_ERR_INVALID, "device index %d out of range", dev); return nullptr; }
-    std::lock_guard<std::mutex> lock(g_lut_mu);
-    if (g_lut[dev] != nullptr) return g_lut[dev];
-    std::vector<uint8_t> h(kQuantLutBytes, 0);
+// false: no reciprocal next to fl(1 / scale) converts every value of some block as the division does, and the table must not be used
+bool fill_quant_lut(uint8_t* h) {
     for (int amax = 0; amax < 128; ++amax) {
         const float scale = amax > 0 ? static_cast<float>(amax) / 6.0f : 1.0f;
         uint32_t sq = ue4m3_encode_host(scale);
@@ -38,12 +33,24 @@ const uint8_t* get_quant_lut() {
             return true;
         };
         for (int i = 0; i < 4 && !converts(rcp); ++i) rcp = nextafterf(rcp, 0.0f);
+        if (!converts(rcp)) return false;
         uint32_t rcp_bits;
         memcpy(&rcp_bits, &rcp, 4);
-        uint8_t* entry = h.data() + kQuantBlockTabOffset + amax * 8;
+        uint8_t* entry = h + kQuantBlockTabOffset + amax * 8;
         memcpy(entry, &rcp_bits, 4);
         memcpy(entry + 4, &sq, 4);
     }
+    return true;
+}
+
+const uint8_t* get_quant_lut() {
+    int dev = 0;
+    if (check_cuda(cudaGetDevice(&dev), "cudaGetDevice")) return nullptr;
+    if (dev < 0 || dev >= 64) { set_error(BNF4_ERR_INVALID, "device index %d out of range", dev); return nullptr; }
+    std::lock_guard<std::mutex> lock(g_lut_mu);
+    if (g_lut[dev] != nullptr) return g_lut[dev];
+    std::vector<uint8_t> h(kQuantLutBytes, 0);
+    if (!fill_quant_lut(h.data())) { set_error(BNF4_ERR_INVALID, "quantiser table: a scale without an exact reciprocal"); return nullptr; }
     uint8_t* d = nullptr;
     if (check_cuda(cudaMalloc(&d, kQuantLutBytes), "cudaMalloc(quant lut)")) return nullptr;
     if (check_cuda(cudaMemcpy(d, h.data(), kQuantLutBytes, cudaMemcpyHostToDevice), "cudaMemcpy(quant lut)")) {
