@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -317,8 +318,14 @@ __device__ __forceinline__ uint2 lds_u64(uint32_t saddr) {
 // lines then keep; 16-byte loads (rows off a 32-byte boundary: wide = false) need their lines there until the last quarter is read, which a
 // streaming load does not promise. 16-byte streaming -> 16-byte plain -> 32-byte -> 32-byte past L1, us: fp32 rows 16384 x 512
 // 10.3 -> 9.4 -> 9.0 -> 8.9; + position / GELU 262144 x 512 219 -> 218 -> 191 -> 192, 65536 x 2048 with 16 projections 343 -> 318 -> 304 -> 287.
+// FIRST: their lines are the first to leave L2, as a streaming load's are (kFirstToo).
+template <bool FIRST = false>
 __device__ __forceinline__ void load8(const void* src, bool wide, uint4& a, uint4& b) {
-    if (wide) {
+    if (wide && FIRST) {
+        asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                     : "l"(src));
+    } else if (wide) {
         asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                      : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
                      : "l"(src));
@@ -328,9 +335,10 @@ __device__ __forceinline__ void load8(const void* src, bool wide, uint4& a, uint
     }
 }
 __device__ __forceinline__ float4 as_float4(const uint4& v) { return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w)); }
+template <bool FIRST = false>
 __device__ __forceinline__ void load8(const float* src, bool wide, float4& a, float4& b) {
     uint4 ua, ub;
-    load8(static_cast<const void*>(src), wide, ua, ub);
+    load8<FIRST>(static_cast<const void*>(src), wide, ua, ub);
     a = as_float4(ua);
     b = as_float4(ub);
 }
@@ -451,11 +459,18 @@ constexpr bool kKeepBytes = NB > 1 && (FE == FE_ABSMEAN || (FE == FE_POS_GELU_AB
 template <int FE, int NB, int NV>
 constexpr int kFastCtas = NB <= 1 ? 4 : kKeepBytes<FE, NB, NV> ? 2 : (NB <= 2 || NV > 4 || FE == FE_POS_GELU_ABSMEAN) ? 2 : 1;
 
+// Rows that are read once and that L2 could hold leave it first, or they push out what is read again (the residual stream, the codes). Halves always do: 65536 x 512
+// 31.1 -> 28.9 us, 32000 x 1024 36.8 -> 32.6, 1048576 x 512 450 both. fp32 rows have instances of their own for it, FIRST, from 40 MB on, with the residual add up to
+// 128 MB (L2 holds 126): 32000 x 512 activation 18.2 -> 17.6 us, + branch 21.5 -> 19.0, 16384 x 1024 + branch 24.4 -> 21.2; but 16384 x 512 activation 9.9 -> 10.7,
+// 262144 x 512 + branch 140 -> 162. (16-byte streaming loads: 29.4, 34.8, 455; 18.0, 20.4, 22.0; 10.8, 149.)
+template <int FE, int NB>
+constexpr bool kFirstToo = (FE == FE_ACT && NB == 1) || (FE == FE_ADD_ABSMEAN && NB <= 2);
+
 // MODEL: powers of two for rows per member, columns and positions, 32-byte aligned rows, one or four projections: no test or division for any of it
 // (the 32-byte rule: 262144 x 512 + position / GELU 198 -> 191 us).
 // ZERO: the MODEL instance that also clears p.zero_t, for launches of up to kPdlStreamElems elements; larger ones have a memset in front (the test
 // and the store cost the default model's instance 4 %, 0.6 of 14.4 ms a step, the memsets 0.1 ms).
-template <int FE, int NB, int NV, bool MODEL = false, bool ZERO = !MODEL>
+template <int FE, int NB, int NV, bool MODEL = false, bool ZERO = !MODEL, bool FIRST = false>
 __global__ void __launch_bounds__(256, kFastCtas<FE, NB, NV>) rowquant_fast_kernel(const RowQuantParams p, const uint8_t* __restrict__ lut) {
     pdl_trigger();
     __shared__ __align__(16) uint2 tab_s[128];  // per amax: {bits of fl(1 / scale), scale byte}
@@ -566,7 +581,7 @@ __global__ void __launch_bounds__(256, kFastCtas<FE, NB, NV>) rowquant_fast_kern
                         f4[q] = __ldcs(reinterpret_cast<const float4*>(src) + q);
                         f4[q + 1] = __ldcs(reinterpret_cast<const float4*>(src) + q + 1);
                     } else {
-                        load8(src + 4 * q, wide, f4[q], f4[q + 1]);
+                        load8<FIRST>(src + 4 * q, wide, f4[q], f4[q + 1]);
                     }
                 }
 #pragma unroll
@@ -610,7 +625,7 @@ __global__ void __launch_bounds__(256, kFastCtas<FE, NB, NV>) rowquant_fast_kern
                         h0 = __ldcs(yh);
                         h1 = __ldcs(yh + 1);
                     } else {
-                        load8(yh, wide, h0, h1);
+                        load8<true>(yh, wide, h0, h1);
                     }
                     const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
 #pragma unroll
@@ -625,7 +640,7 @@ __global__ void __launch_bounds__(256, kFastCtas<FE, NB, NV>) rowquant_fast_kern
                             y4[q] = __ldcs(reinterpret_cast<const float4*>(yr + k0 + 4 * q));
                             y4[q + 1] = __ldcs(reinterpret_cast<const float4*>(yr + k0 + 4 * q) + 1);
                         } else {
-                            load8(yr + k0 + 4 * q, wide, y4[q], y4[q + 1]);
+                            load8<FIRST>(yr + k0 + 4 * q, wide, y4[q], y4[q + 1]);
                         }
                     }
                 }
@@ -889,7 +904,7 @@ __global__ void __launch_bounds__(256, kFastCtas<FE, NB, NV>) rowquant_fast_kern
 }
 
 // CTAs of a fast-kernel instance that fit one SM, per device (0 = not looked up yet)
-template <int FE, int NB, int NV, bool MODEL = false, bool ZERO = !MODEL>
+template <int FE, int NB, int NV, bool MODEL = false, bool ZERO = !MODEL, bool FIRST = false>
 std::atomic<int> resident_ctas[64] = {};
 
 template <int FE>
@@ -967,15 +982,18 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
                     return check_launch("rowquant_fast_kernel");
                 }
             }
-            if (p.nvec <= 4) {
-                if (nblk <= 32) rc = run(rowquant_fast_kernel<FE, 1, 4>, resident_ctas<FE, 1, 4>);
-                else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, 4>, resident_ctas<FE, 2, 4>);
-                else rc = run(rowquant_fast_kernel<FE, 4, 4>, resident_ctas<FE, 4, 4>);
-            } else {
-                if (nblk <= 32) rc = run(rowquant_fast_kernel<FE, 1, kMaxTVec>, resident_ctas<FE, 1, kMaxTVec>, batch_smem(1), batch_rows(1));
-                else if (nblk <= 64) rc = run(rowquant_fast_kernel<FE, 2, kMaxTVec>, resident_ctas<FE, 2, kMaxTVec>, batch_smem(2), batch_rows(2));
-                else rc = run(rowquant_fast_kernel<FE, 4, kMaxTVec>, resident_ctas<FE, 4, kMaxTVec>, batch_smem(4), batch_rows(4));
-            }
+            const long long row_bytes = 4LL * p.rows * p.cols_out;
+            const bool first = !p.in_f16 && row_bytes >= (40LL << 20) && (FE == FE_ACT || row_bytes <= (128LL << 20));  // (kFirstToo)
+            auto run_nv = [&](auto nb, auto nv) -> int {
+                constexpr int NB = decltype(nb)::value, NV = decltype(nv)::value;
+                constexpr int smem = NV > 4 ? batch_smem(NB) : 0, batch = NV > 4 ? batch_rows(NB) : 1;
+                if constexpr (kFirstToo<FE, NB>) {
+                    if (first) return run(rowquant_fast_kernel<FE, NB, NV, false, true, true>, resident_ctas<FE, NB, NV, false, true, true>, smem, batch);
+                }
+                return run(rowquant_fast_kernel<FE, NB, NV>, resident_ctas<FE, NB, NV>, smem, batch);
+            };
+            auto run_nb = [&](auto nb) -> int { return p.nvec <= 4 ? run_nv(nb, std::integral_constant<int, 4>()) : run_nv(nb, std::integral_constant<int, kMaxTVec>()); };
+            rc = nblk <= 32 ? run_nb(std::integral_constant<int, 1>()) : nblk <= 64 ? run_nb(std::integral_constant<int, 2>()) : run_nb(std::integral_constant<int, 4>());
             if (rc) return rc;
             return check_launch("rowquant_fast_kernel");
         }

@@ -67,3 +67,28 @@ def test_rows_on_every_boundary(fe, cols, rpm, nvec):
         fast = run(host.FE_ABSMEAN, in_i8=x, norm_scale=40.0)
         assert all(torch.equal(a, b) for a, b in zip(ref, fast))
         assert all(torch.equal(a, b) for a, b in zip(ref, (codes, sf, t)))
+
+
+@pytest.mark.parametrize("cols,rpm", [(512, 5376), (1024, 2688)])
+@pytest.mark.parametrize("nvec", [1, 16])
+@pytest.mark.parametrize("fe", ["act", "add"])
+def test_rows_that_fill_much_of_l2(fe, cols, rpm, nvec):
+    """fp32 rows of 40 MB and more give the bytes of their halves."""
+    import torch
+    from bitnet_nvfp4_b200 import host
+    g = torch.Generator(device="cuda").manual_seed(cols + nvec)
+    x0 = torch.randint(-127, 128, (4 * rpm, cols), device="cuda", generator=g).to(torch.int8)
+    f = torch.randn(4 * rpm, cols, device="cuda", generator=g) * 30
+    tvec = torch.randint(-127, 128, (2, nvec, cols), device="cuda", generator=g).to(torch.int8)
+
+    def run(pairs):
+        rows, part = 2 * rpm * len(pairs), slice(2 * rpm * pairs[0], 2 * rpm * (pairs[-1] + 1))
+        codes, sf = (torch.zeros(b, dtype=torch.uint8, device="cuda") for b in (host.matrix_bytes(rows, cols), host.sf_bytes(rows, cols)))
+        t, x, y = torch.zeros(rows, nvec, dtype=torch.int32, device="cuda"), x0[part].clone(), f[part].clone()
+        kw = dict(in_f32=y, act_mode=3, act_scale=0.9) if fe == "act" else dict(in_f32=y, add_scale=1.0, norm_scale=40.0, inout_i8=x)
+        host.rowquant(host.FE_ACT if fe == "act" else host.FE_ADD_ABSMEAN, rows=rows, cols_in=cols, cols_out=cols, rows_per_member=rpm, out_codes=codes, out_sf=sf,
+                      ld_in=cols, tvec=tvec[pairs[0]:].contiguous(), tvec_pair_stride=nvec * cols, nvec=nvec, t_out=t, **kw)
+        return codes, sf, t, x
+
+    for whole, a, b in zip(run([0, 1]), run([0]), run([1])):
+        assert torch.equal(whole, torch.cat([a, b]))
