@@ -316,7 +316,7 @@ __device__ __forceinline__ uint2 lds_u64(uint32_t saddr) {
 // Eight of a lane's sixteen fp32 values (or its sixteen halves). The lanes' values lie 64 bytes apart, so that a load instruction touches
 // sixteen lines whatever its width, and a line is asked for by two or four of them: 32-byte loads halve both. They pass by L1, which the tables'
 // lines then keep; 16-byte loads (rows off a 32-byte boundary: wide = false) need their lines there until the last quarter is read, which a
-// streaming load does not promise. 16-byte streaming -> 16-byte plain -> 32-byte -> 32-byte past L1, us: fp32 rows 16384 x 512
+// streaming load does not promise. 16-byte streaming -> 16-byte plain -> 32-byte -> 32-byte past L1, us: fp32 rows in L2, 16384 x 512
 // 10.3 -> 9.4 -> 9.0 -> 8.9; + position / GELU 262144 x 512 219 -> 218 -> 191 -> 192, 65536 x 2048 with 16 projections 343 -> 318 -> 304 -> 287.
 // FIRST: their lines are the first to leave L2, as a streaming load's are (kFirstToo).
 template <bool FIRST = false>
@@ -459,12 +459,14 @@ constexpr bool kKeepBytes = NB > 1 && (FE == FE_ABSMEAN || (FE == FE_POS_GELU_AB
 template <int FE, int NB, int NV>
 constexpr int kFastCtas = NB <= 1 ? 4 : kKeepBytes<FE, NB, NV> ? 2 : (NB <= 2 || NV > 4 || FE == FE_POS_GELU_ABSMEAN) ? 2 : 1;
 
-// Rows that are read once and that L2 could hold leave it first, or they push out what is read again (the residual stream, the codes). Halves always do: 65536 x 512
-// 31.1 -> 28.9 us, 32000 x 1024 36.8 -> 32.6, 1048576 x 512 450 both. fp32 rows have instances of their own for it, FIRST, from 40 MB on, with the residual add up to
-// 128 MB (L2 holds 126): 32000 x 512 activation 18.2 -> 17.6 us, + branch 21.5 -> 19.0, 16384 x 1024 + branch 24.4 -> 21.2; but 16384 x 512 activation 9.9 -> 10.7,
-// 262144 x 512 + branch 140 -> 162. (16-byte streaming loads: 29.4, 34.8, 455; 18.0, 20.4, 22.0; 10.8, 149.)
+// Rows that are read once leave L2 first, or they push out what is read again (the residual stream, the codes). 16-byte streaming loads -> 32-byte -> 32-byte, first to leave, us:
+//   halves, + branch: 65536 x 512 29.4 -> 31.1 -> 28.9, 32000 x 1024 34.8 -> 36.8 -> 32.6, 1048576 x 512 455 -> 450 -> 450;
+//   fp32 rows, activation, from DRAM: 16384 x 512 10.7 -> 10.7 -> 10.5, with four projections 12.4 -> 13.2 -> 12.0, 8000 x 512 with four 8.2 -> 9.1 -> 7.9; from L2 16384 x 512
+//     10.5 -> 9.9 -> 9.9, two buffers in turn 10.8 -> 9.9 -> 10.7; a GEMM behind 16384 x 512 that are new each time 21.8 -> 20.8 for both.
+// fp32 rows of the residual add have instances of their own for it, FIRST, from 40 to 128 MB (L2 holds 126): 32000 x 512 20.4 -> 21.5 -> 19.0, 12000 x 1024 17.1 -> 19.6 -> 16.6,
+// 65536 x 512 35.4 -> 38.3 -> 33.3; but 262144 x 512 149 -> 140 -> 162.
 template <int FE, int NB>
-constexpr bool kFirstToo = (FE == FE_ACT && NB == 1) || (FE == FE_ADD_ABSMEAN && NB <= 2);
+constexpr bool kFirstToo = FE == FE_ADD_ABSMEAN && NB <= 2;
 
 // MODEL: powers of two for rows per member, columns and positions, 32-byte aligned rows, one or four projections: no test or division for any of it
 // (the 32-byte rule: 262144 x 512 + position / GELU 198 -> 191 us).
@@ -581,7 +583,7 @@ __global__ void __launch_bounds__(256, kFastCtas<FE, NB, NV>) rowquant_fast_kern
                         f4[q] = __ldcs(reinterpret_cast<const float4*>(src) + q);
                         f4[q + 1] = __ldcs(reinterpret_cast<const float4*>(src) + q + 1);
                     } else {
-                        load8<FIRST>(src + 4 * q, wide, f4[q], f4[q + 1]);
+                        load8<true>(src + 4 * q, wide, f4[q], f4[q + 1]);
                     }
                 }
 #pragma unroll
@@ -983,7 +985,7 @@ int launch(const RowQuantParams& p, cudaStream_t stream) {
                 }
             }
             const long long row_bytes = 4LL * p.rows * p.cols_out;
-            const bool first = !p.in_f16 && row_bytes >= (40LL << 20) && (FE == FE_ACT || row_bytes <= (128LL << 20));  // (kFirstToo)
+            const bool first = !p.in_f16 && row_bytes >= (40LL << 20) && row_bytes <= (128LL << 20);  // (kFirstToo)
             auto run_nv = [&](auto nb, auto nv) -> int {
                 constexpr int NB = decltype(nb)::value, NV = decltype(nv)::value;
                 constexpr int smem = NV > 4 ? batch_smem(NB) : 0, batch = NV > 4 ? batch_rows(NB) : 1;
