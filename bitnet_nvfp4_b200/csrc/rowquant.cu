@@ -453,7 +453,9 @@ __device__ __forceinline__ void project_rows(const RowQuantParams& p, const int4
 //     + branch, 1024 columns, 1 projection 67 -> 70 / 71, 2048 columns, 4 projections 160 -> 165 / 148, but 4000 such rows 17.8 -> 19.6
 //   floats kept, 2 / 3 blocks: + position / GELU, 2048 columns, 4 projections 257 / 261 (one block: 294, with 16-byte loads).
 //     fp32 rows past 1024 columns stay at one block: three take 65536 x 2048 from 186 to 154, but 4000 x 1984 from 16 to 20.
-// Dearer: 1500 rows of 2048 bytes 5.7 -> 6.1 (4000: 13.7 -> 12.7), 1500 x 768 + position / GELU 7.7 -> 8.1 (65536 x 1024: 139 -> 114).
+// 1500 / 4000 / 16384 / 65536 rows behind another kernel: 2048 bytes 6.3 -> 5.9, 9.5 -> 8.7, 28 -> 20, 95 -> 68; 768 + position / GELU 8.5 -> 8.0, 13.6 -> 12.1,
+// 37.5 -> 33.7, 135 -> 109. Dearer: launches of 1000 to 2300 rows behind one another (4.5 -> 4.8, 6.6 -> 7.0: the next launch starts in the room that the smaller register
+// count leaves), and + position / GELU with four projections 200 rows 7.7 -> 8.0, 4700 x 1024 from DRAM 15.2 -> 16.9 (from L2 14.8 both).
 template <int FE, int NB, int NV>
 constexpr bool kKeepBytes = NB > 1 && (FE == FE_ABSMEAN || (FE == FE_POS_GELU_ABSMEAN && NB <= 2));
 template <int FE, int NB, int NV>
