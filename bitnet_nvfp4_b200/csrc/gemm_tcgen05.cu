@@ -118,8 +118,8 @@ struct KernelArgs {
 // every other one of rank 1 and 2, 3 and 4, with zeros for a factor that is not there. The number of products is thereby known to the compiler: one
 // instance tested the rank inside the loop over the columns (and spilled: 88 and 114 bytes with FP4 output, 4 to 28 with the others). Figures, one such instance -> these, us: 88800 x 320 x 320 rank 2 residual 44 -> 32,
 // 88800 x 961 x 320 rank 2 halves 69 -> 52, 88800 x 960 x 320 GELU to FP4 rank 2 141 -> 106, rank 3 with members of 1100 rows 152 -> 132, 65536 x 512 x 2048 rank 2
-// residual 65 -> 46, 16384 x 512 x 512 rank 3 fp32 11.9 -> 10.8. Without forms 3 and 5 those of rank 2 and 4 lose 2 to 12 % (33.5, 54, 119). Dearer: 16384 x 4096 x 4096
-// rank 3 fp32, 132 -> 135, where the products with a zero count (rank 3 with the other epilogues there 150 -> 144, 125 -> 121, 154 -> 146). (262144 x 1024 x 512 with GELU to FP4 and no rank term: 303 us as a case of a general instance, 256 us.)
+// residual 65 -> 46, 16384 x 512 x 512 rank 3 fp32 11.9 -> 10.8. Without forms 3 and 5 those of rank 2 and 4 lose 2 to 12 % (33.5, 54, 119). 16384 x 4096 x 4096 rank 3 fp32
+// stands at 132 to 150 with either (one build's runs differ by 5 % there; an instance of three products gave nothing), the other epilogues gain: 150 -> 144, 125 -> 121, 154 -> 146. (262144 x 1024 x 512 with GELU to FP4 and no rank term: 303 us as a case of a general instance, 256 us.)
 // B2: the instance with a second B operand (no rank term); the others carry no tests for one (a rank-2 term with GELU to FP4 446 -> 412 us).
 // PAIR: the instance for operands with many K blocks. On the in-order pipe a scale copy costs about 44 cycles and an M 128 x N 128 MMA
 // 64 (measured, one CTA): 8 copies and 4 MMAs per 256-element K block of a 128 x 128 tile take 560 cycles before any operand
